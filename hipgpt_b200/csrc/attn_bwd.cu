@@ -1,4 +1,5 @@
-// Attention backward: dQ, dK, dV from dO, Q, K, V and either the stored probabilities or nothing
+// Attention backward, head dimensions other than 32 and 64 (those run on the tensor pipe, attn_bwd_tc.cu) and unaligned planes:
+// dQ, dK, dV from dO, Q, K, V and either the stored probabilities or nothing
 // more (the probabilities are then recomputed from row maxima and sums that this file forms itself).
 //
 // Replaces multihead_attention_backward_kernel behind launch_multihead_attention_backward
@@ -239,6 +240,8 @@ int launch_mha_backward(const float *g, const float *q, const float *k, const fl
     const int D = E / H;
     if (D > kBwdMaxD) return fail(HIPGPT_ERR_UNSUPPORTED, "attention backward: head_dim %d exceeds %d", D, kBwdMaxD);
     if (B == 0 || S == 0) return HIPGPT_OK;
+    if (mha_backward_tc_supports(g, q, k, v, probs, dq, dk, dv, B, S, E, H))
+        return launch_mha_backward_tc(g, q, k, v, probs, dq, dk, dv, B, S, E, H, causal, st);
 #define HIPGPT_BWD(DP) (causal ? launch_bwd_cfg<DP, true>(g, q, k, v, probs, dq, dk, dv, scratch, B, S, E, H, st) \
                                : launch_bwd_cfg<DP, false>(g, q, k, v, probs, dq, dk, dv, scratch, B, S, E, H, st))
     if (D <= 32) return HIPGPT_BWD(32);

@@ -94,6 +94,13 @@ int bf16_status_fetch(int *status);
 size_t mha_backward_scratch_bytes(int B, int H, int S);
 int launch_mha_backward(const float *g, const float *q, const float *k, const float *v, const float *probs,
                         float *dq, float *dk, float *dv, float *scratch, int B, int S, int E, int H, int causal, cudaStream_t st);
+// the same on the tensor pipe, head_dim 32 / 64 (attn_bwd_tc.cu)
+bool mha_backward_tc_supports(const void *g, const void *q, const void *k, const void *v, const void *probs, const void *dq, const void *dk,
+                              const void *dv, int B, int S, int E, int H);
+int launch_mha_backward_tc(const float *g, const float *q, const float *k, const float *v, const float *probs, float *dq, float *dk, float *dv,
+                           int B, int S, int E, int H, int causal, cudaStream_t st);
+int mha_backward_tc_status_fetch(int *status);
+void mha_backward_tc_release();
 // the launchers either side of attention (layer_ops.cu)
 int launch_matmul_exact(const float *A, const float *B, const float *bias, float *C, int M, int N, int K, cudaStream_t st);
 // The same product on the tensor pipe with fp32-grade (not bit-identical) results (gemm_tc.cu); its status word and scratch.

@@ -149,6 +149,9 @@ HIPGPT_API int hipgpt_attention_weighted_sum(const float *d_softmax, const float
  *   d_scratch      hipgpt_mha_backward_scratch_bytes(B, H, S) bytes (2 B H S floats)
  * No atomics: a key row's gradients add its queries in ascending order, so results are reproducible run to
  * run (the reference's atomicAdd order is not); they agree with the reference's arithmetic to rounding.
+ * head_dim 32 and 64 run on the tensor pipe with fp32 accuracy over the whole fp32 range (every operand as the sum of three
+ * bf16 numbers, six products per product); the operands' images live in a buffer of the library (per device and stream,
+ * at most eight; hipgpt_release_workspace() frees them; a captured call gets a buffer of its graph).
  * hipgpt_mha_backward_planes is the launcher's own view (three stacked planes in d_qkv and d_grad_qkv) with
  * the scratch kept in a buffer of the library, which grows with cudaMalloc to the largest call per device.
  */
@@ -364,7 +367,8 @@ HIPGPT_API int hipgpt_probe_fma(float *d_sink, int blocks, int iters, double *fl
  * Device-side status of the tensor-core kernels (no counterpart in the reference).  Their
  * waits on hardware barriers are bounded; a block whose wait runs out stores nothing and records
  * which wait it was: 1..8 for the split-TF32 kernel, 100 + site for the bf16 kernel, 300 + site
- * for the tiled fp32 kernel, 400 + site for the whole-head kernel, 900 + site for the test hook
+ * for the tiled fp32 kernel, 400 + site for the whole-head kernel, 500 + site for the tensor-core projections,
+ * 600 + site for the attention backward, 900 + site for the test hook
  * hipgpt_debug_wait_expiry.  This call waits for the whole
  * device (cudaDeviceSynchronize), stores the status word in *status and clears it.  0 means every
  * launch since the last call completed normally.  Callers of the device-pointer entry points

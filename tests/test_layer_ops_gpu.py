@@ -254,6 +254,45 @@ def test_attention_backward_matches_oracle(shape, causal, stored):
     assert np.array_equal(again, got)                      # no atomics: the same bits on every run and entry point
 
 
+@pytest.mark.parametrize("shape", [(1, 2, 63, 32), (1, 2, 64, 64), (2, 1, 65, 64), (1, 3, 127, 32), (1, 1, 128, 64), (1, 2, 129, 64), (1, 1, 450, 32), (65, 8, 128, 64)])
+@pytest.mark.parametrize("causal,stored", [(False, True), (True, False), (False, False)])
+def test_attention_backward_tensor_kernels_at_tile_edges(shape, causal, stored):
+    """head_dim 32 / 64: tiles of 64 keys or queries, blocks of 128 rows, sequence lengths at and beside both, odd lengths (the
+    stored probabilities then have no 16-byte rows), one and several groups of batches (the last shape)."""
+    B, H, S, D = shape
+    E = H * D
+    qkv = synth.qkv_planes(820 + S, B, S, E)
+    g = synth.normal(821 + S, (B * S, E))
+    probs = ob.mha(qkv, B, S, E, H, causal=causal, want_probs=True)[1] if stored else None
+    want = ob.mha_backward(g, qkv, probs, B, S, E, H, causal=causal, fma=True)
+    got = _run_backward(g, qkv, probs, B, S, E, H, causal)
+    assert float(np.abs(got - want).max()) <= 4e-6 * max(1.0, float(np.abs(want).max()))
+    st = C.c_int(-1)
+    _capi.check(_capi.lib().hipgpt_kernel_status(C.byref(st)))
+    assert st.value == 0
+
+
+def test_attention_backward_of_any_magnitude_and_captured_into_a_graph():
+    B, H, S, D = 2, 2, 96, 64
+    E = H * D
+    qkv = synth.qkv_planes(830, B, S, E).reshape(3, B * S, E)
+    qkv[0] *= np.float32(1e-6); qkv[1] *= np.float32(1e6); qkv[2] *= np.float32(3e8)
+    g = synth.normal(831, (B * S, E)) * np.float32(2e-9)
+    want = ob.mha_backward(g, qkv, None, B, S, E, H, fma=True).reshape(3, -1)
+    got = _run_backward(g, qkv, None, B, S, E, H, False).reshape(3, -1)
+    for w, o in zip(want, got):
+        assert float(np.abs(o - w).max()) <= 1e-5 * float(np.abs(w).max())
+    dg, dq, dout = dev(g), dev(qkv), torch.full((3, B * S, E), float("nan"), device="cuda")
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        _capi.check(_capi.lib().hipgpt_mha_backward_planes(dg.data_ptr(), dq.data_ptr(), None, dout.data_ptr(), B, S, E, H, 0, _st()))
+    for _ in range(2):
+        dout.fill_(float("nan"))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert np.array_equal(dout.cpu().numpy().reshape(3, -1), got)
+
+
 def test_attention_backward_reference_named_launcher():
     raw = C.CDLL(_capi.lib_path())
     fn = getattr(raw, _capi.CXX_LAUNCHERS["launch_multihead_attention_backward"])
