@@ -1,0 +1,812 @@
+// Greedy generation with HipGPT's model shape, KV-cache form, by clusters of sixteen blocks (sm_100a).
+//
+// The same arithmetic as the launches of gpt_decode.cu, bit for bit: matmuls accumulate 16 segments of the inner dimension k
+// ascending with fused multiply-add and add the partial sums in order, layer norms are 32 lane-strided sums joined by a butterfly,
+// the attention is split over the context as attn_decode.cu splits it and merged in its order.
+//
+// What bounds a token step is a chain of small products: 4 per layer, each needing all of the one before it, with a few KB of
+// activations between them and 30 MB of weights beside them.  As 52 launches a step of the default model took 320 us, nearly all
+// of it launch gaps, L2 round trips and weights fetched only when a kernel had started.  Here one launch runs all steps, and
+// sequences, which do not depend on one another, are dealt out to clusters:
+//   * A cluster owns `rows` sequences and runs every layer for them.  A block owns a sixteenth of the columns of every matrix.
+//     The activations are replicated: each block keeps whole rows in its shared memory, and the block that finishes four columns
+//     stores them into all sixteen with st.async, which counts the bytes on the receiver's mbarrier.  A hop from product to product
+//     is therefore one such store and one barrier inside the block: no barrier over the cluster, nothing through L2.
+//   * A block's weights are laid out once in the order in which a step reads them and arrive through a ring in shared memory by
+//     bulk copies that run up to a layer ahead of the arithmetic; they do not depend on activations, so nothing waits for them.
+//   * Warp s owns segment s of the inner dimension (lanes: columns), so a layer norm needs no barrier either: every warp forms
+//     the row's statistics and normalises the part that it multiplies.
+//   * Keys and values of older positions are asked for before the projection of the new one is formed.
+//   * The logits are formed where an id is picked from them: not at prompt positions before the last.
+// Buffers are received into once per layer (or step); a sender can be at most one product ahead of the slowest receiver, because
+// each product needs the columns of all blocks, so a buffer is never overwritten while it is read.
+// Waits on mbarriers are bounded: on expiry the block raises a flag that cuts its later waits short and sets the error word; the
+// steps then run out without waiting.
+//
+// Measured at the default model (E=256 L=8 H=8 V=5000), batch 8: 90 us per step (the replayed graph: 318), batch 1: 75 (256).  A
+// step is 42 products of about 450 ns each: multiply-adds 20 %, layer norms 10 %, adding up and storing 15 %, arrival of the
+// others' columns 25 %, attention 30 %.  Sizes are template parameters because the chain is bound by the instructions of single
+// warps: with sizes read from the plan a step took 143 us.
+#include "gpt_cluster.cuh"
+#include "tc_primitives.cuh"
+
+#include <math.h>
+
+namespace hipgpt {
+namespace {
+
+constexpr int kThreads = 512;
+constexpr int kWarps = 16;
+constexpr int kMostSlots = 24;
+constexpr int kSmemMost = 232448 - 1024;
+constexpr int kAhead = 4;                        // key / value rows per lane asked for ahead of the projection
+
+__device__ __forceinline__ uint32_t peer_addr(uint32_t addr, int rank)
+{
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+// 16 or 8 bytes into a block of the cluster, counted on the mbarrier there
+__device__ __forceinline__ void send4(uint32_t addr, uint32_t bar, float4 v)
+{
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
+                 ::"r"(addr), "r"(__float_as_uint(v.x)), "r"(__float_as_uint(v.y)), "r"(__float_as_uint(v.z)), "r"(__float_as_uint(v.w)), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void send2(uint32_t addr, uint32_t bar, uint32_t x, uint32_t y)
+{
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];" ::"r"(addr), "r"(x), "r"(y), "r"(bar) : "memory");
+}
+
+// The polling part of a wait, out of line: the kernel's code should stay in the instruction cache.
+__device__ __noinline__ void cluster_wait_slow(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int *err)
+{
+    if (!mbar_wait(bar, parity)) {
+        *abort_flag = 1;
+        atomicExch(err, 1);
+    }
+}
+
+struct Part {
+    float m, l;
+    float4 o;
+};
+// as in attn_decode.cu
+__device__ __forceinline__ void merge_part(Part &a, float m2, float l2, const float4 &o2)
+{
+    const float mn = fmaxf(a.m, m2);
+    const float a1 = ex2_approx(a.m - mn), a2 = ex2_approx(m2 - mn);
+    a.l = a.l * a1 + l2 * a2;
+    a.o.x = a.o.x * a1 + o2.x * a2;
+    a.o.y = a.o.y * a1 + o2.y * a2;
+    a.o.z = a.o.z * a1 + o2.z * a2;
+    a.o.w = a.o.w * a1 + o2.w * a2;
+    a.m = mn;
+}
+
+template <int J>
+struct Job { static constexpr int value = J; };
+template <int E, int R>
+struct Width { static constexpr int kE = E, kR = R; };
+
+// Shared memory of a block, in floats from the start: what has a size known to the compiler first.  Rows of activations are padded
+// by four floats: the rows that a warp reads side by side then lie in different banks.
+template <int E, int R>
+struct Lay {
+    static constexpr int F = 4 * E;
+    static constexpr int es = E + 4, qs = 3 * E + 4, fs = F + 4;         // row strides
+    static constexpr int seg = cluster_job_of(kJobQkv, E, 16).klp + 4;   // of a warp's own segment
+    static constexpr int xb = 0, xa = xb + R * es, qkv = xa + R * es, ff = qkv + R * qs, aw = ff + R * fs, part = aw + kWarps * R * seg;
+    static constexpr int part_stride = R * 16 * 64;
+    static constexpr int unit = part + 2 * part_stride, amax = unit + 4 * 4 * 32 * 8, fixed = (amax + 32 * R * 2 + 3) & ~3;
+    static constexpr int slot_bytes()
+    {
+        int most = 0;
+        for (int i = 0; i < kJobs; ++i) { const int b = cluster_job_of(i, E, 64 * 64).chunk_bytes(); most = b > most ? b : most; }
+        return (most + 127) & ~127;
+    }
+    static constexpr int kSlot = slot_bytes();
+};
+// ... then the attention records and the chunk table, then the ring.
+struct Rest { int table, ring, slots, total; };
+template <int E, int R>
+Rest rest_of(int H, int D, int ns, int all_chunks)
+{
+    using L = Lay<E, R>;
+    Rest r;
+    r.table = L::fixed + ((R * H * ns * (D + 4) + 3) & ~3);
+    r.ring = (r.table + 2 * all_chunks + 31) & ~31;
+    r.slots = (kSmemMost - 4 * r.ring) / L::kSlot;
+    if (r.slots > kMostSlots) r.slots = kMostSlots;
+    if (r.slots < 0) r.slots = 0;
+    r.total = 4 * r.ring + r.slots * L::kSlot;
+    return r;
+}
+
+template <int E, int R>
+__global__ void __launch_bounds__(kThreads, 1)
+cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_constant__ ClusterArgs a, const __grid_constant__ Rest lay)
+{
+    using C = Lay<E, R>;
+    constexpr int F = 4 * E;
+    extern __shared__ __align__(128) float sm[];
+    __shared__ uint64_t full[kMostSlots];
+    __shared__ uint64_t hop[6];                      // qkv, attention records, xa, ff, xb, first maxima
+    __shared__ float2 stats[R];                      // a row's mean and 1 / sqrt(variance + eps)
+    __shared__ int next_id[R];
+    __shared__ volatile int abort_flag;
+    enum { kQkv, kRec, kXa, kFf, kXb, kAm };
+
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    int rank;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    const int row0 = (int)(blockIdx.x / kClusterBlocks) * R;
+    const int rows = min(R, a.B - row0);             // sequences of this cluster
+    const int V = a.V, H = a.H, D = E / H, ns = a.ns;
+    const int rstride = D + 4;
+
+    float *xb = sm + C::xb, *xa = sm + C::xa, *qkv = sm + C::qkv, *ff = sm + C::ff, *rec = sm + C::fixed, *part = sm + C::part;
+    float *aw = sm + C::aw + warp * (R * C::seg);    // this warp's own segment of the activations
+    uint32_t *amax = reinterpret_cast<uint32_t *>(sm + C::amax);
+    uint2 *table = reinterpret_cast<uint2 *>(sm + lay.table);
+    uint8_t *ring = reinterpret_cast<uint8_t *>(sm + lay.ring);
+    auto tx = [&](int i) {
+        return (uint32_t)(rows * (i == kQkv ? 12 * E : i == kRec ? H * ns * (D + 2) * 4 : i == kFf ? 4 * F : i == kAm ? 32 * 8 : 4 * E));
+    };
+
+    for (int i = tid; i < lay.table; i += kThreads) sm[i] = 0.0f;         // rows that the cluster does not have stay zero
+    for (int i = tid; i < plan.all_chunks; i += kThreads) table[i] = a.table[i];
+    if (tid == 0) {
+        abort_flag = 0;
+        for (int i = 0; i < lay.slots; ++i) mbar_init(&full[i], 1);
+        for (int i = 0; i < 6; ++i) { mbar_init(&hop[i], 1); mbar_arrive_expect_tx(&hop[i], tx(i)); }
+    }
+    __syncthreads();
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+
+    auto wait = [&](uint64_t *bar, uint32_t parity) {
+        if (mbar_test(bar, parity) || abort_flag) return;
+        cluster_wait_slow(bar, parity, &abort_flag, a.err);
+    };
+    // what a hop delivers is complete; one thread opens the barrier's next phase
+    uint32_t hop_phase = 0;                          // a bit per hop
+    auto receive = [&](int i) {
+        wait(&hop[i], (hop_phase >> i) & 1u);
+        hop_phase ^= 1u << i;
+        if (tid == kThreads - 1) mbar_arrive_expect_tx(&hop[i], tx(i));
+    };
+    // an address of this block -> the same place in four of the blocks (those this thread stores into)
+    const int dq = tid & 3;
+    uint32_t peer[4];
+#pragma unroll
+    for (int d = 0; d < 4; ++d) peer[d] = peer_addr(smem_u32(sm), 4 * dq + d) - smem_u32(sm);
+
+    // ---- the weights: the lanes of the last warp keep the ring full, in the order in which the steps consume it ----
+    const uint8_t *share = a.stream + (size_t)rank * plan.block_bytes;
+    int f_step = 0, f_pos = 0, f_slot = 0;           // the next chunk: its step, its place in the step, its slot
+    auto step_chunks = [&](int step) { return a.p0 + step >= a.n_prompt - 1 ? plan.all_chunks : plan.layer_chunks; };     // an id is picked there
+    auto fetch = [&](int n) {                        // the next n <= 16 chunks (as long as there are any), a lane each
+        const int len = step_chunks(f_step);
+        int pos = f_pos + lane, slot = f_slot + lane;
+        const bool wraps = pos >= len;
+        if (wraps) pos -= len;
+        if (slot >= lay.slots) slot -= lay.slots;
+        if (lane < n && f_step + (wraps ? 1 : 0) < a.nsteps) {
+            const uint2 t = table[pos];
+            mbar_arrive_expect_tx(&full[slot], t.y);
+            bulk_load(ring + slot * C::kSlot, share + t.x, t.y, &full[slot]);
+        }
+        f_pos += n;
+        if (f_pos >= len) { f_pos -= len; ++f_step; }
+        f_slot += n;
+        if (f_slot >= lay.slots) f_slot -= lay.slots;
+    };
+    if (warp == kWarps - 1)
+#pragma unroll 1
+        for (int i = 0; i < lay.slots; ++i) fetch(1);
+    int slot0 = 0;                                   // slot of the next product's first chunk
+    uint32_t slot_par = 0;                           // parity of the ring's round there
+    int flip = 0;                                    // buffer of partial sums
+
+    // a row's statistics by one warp: 32 lane-strided sums joined by a butterfly, nothing contracted
+    auto row_stats = [&](const float *row, float2 *out) {
+        float v[E / 32];
+        float s = 0.0f, q = 0.0f;
+#pragma unroll
+        for (int i = 0; i < E / 32; ++i) v[i] = row[lane + 32 * i];
+#pragma unroll
+        for (int i = 0; i < E / 32; ++i) s = __fadd_rn(s, v[i]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s = __fadd_rn(s, __shfl_xor_sync(0xffffffffu, s, o));
+        // a division by a power of two is a multiplication
+        const float mean = (E & (E - 1)) == 0 ? __fmul_rn(s, 1.0f / E) : __fdiv_rn(s, (float)E);
+#pragma unroll
+        for (int i = 0; i < E / 32; ++i) {
+            const float d = __fsub_rn(v[i], mean);
+            q = __fadd_rn(q, __fmul_rn(d, d));
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) q = __fadd_rn(q, __shfl_xor_sync(0xffffffffu, q, o));
+        const float var = (E & (E - 1)) == 0 ? __fmul_rn(q, 1.0f / E) : __fdiv_rn(q, (float)E);
+        if (lane == 0) *out = make_float2(mean, __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(var, 1e-5f))));
+    };
+
+    auto add4 = [](float4 x, float4 y) { return make_float4(__fadd_rn(x.x, y.x), __fadd_rn(x.y, y.y), __fadd_rn(x.z, y.z), __fadd_rn(x.w, y.w)); };
+    // One product's multiply-adds: this warp's segment of the inner dimension, all columns of the part.  The activations: rows at
+    // `src` in shared memory, normalised first where the job says so; kJobO takes this warp's own segment.  Leaves the partial sums
+    // in part + flip * part_stride and ends with a barrier of the block.  Lanes: up to 16 columns: (column, row of a pair); more:
+    // columns lane, lane + 32, all rows.  Returns the part's bias for the columns that this thread finishes.
+    auto product = [&](auto jn, const float *src) {
+        constexpr int J = decltype(jn)::value;
+        constexpr ClusterJob jb = cluster_job_of(J, E, 64 * 64);          // (the output projection's cut depends on V in its parts only)
+        constexpr int pw = jb.width, klen = jb.klen, klp = jb.klp, sh = jb.seg_shift, nch = jb.chunks();
+        constexpr int stride = J == kJobF2 ? C::fs : C::es;
+        int slot = slot0 + (warp >> sh);
+        uint32_t par = slot_par;
+        if (slot >= lay.slots) { slot -= lay.slots; par ^= 1u; }
+        const float *chunk = reinterpret_cast<const float *>(ring + slot * C::kSlot);
+        const int in_chunk = warp & ((1 << sh) - 1);
+        const float4 *w4 = reinterpret_cast<const float4 *>(chunk + in_chunk * (klp * pw));
+        const float *as = aw;
+        constexpr bool kOwn = jb.ln || J == kJobO || (klen & 3) != 0;     // the activations are (copied) in this warp's own segment
+        constexpr int astride = kOwn ? C::seg : stride;
+        if constexpr (jb.ln != 0) {
+            if (warp < rows) row_stats(src + warp * stride, &stats[warp]);
+            __syncthreads();
+        }
+        wait(&full[slot], par);
+        if constexpr (jb.ln != 0) {
+            const float *gm = chunk + jb.weight_floats() + in_chunk * klp, *bt = gm + (klp << sh);
+#pragma unroll
+            for (int t = 0; t < (R * klp + 31) / 32; ++t) {
+                const int i = lane + 32 * t, r = i / klp, k = i % klp;
+                if (i < R * klp) {
+                    const float2 st = stats[r];
+                    aw[r * C::seg + k] = k < klen ? __fadd_rn(__fmul_rn(__fmul_rn(gm[k], __fsub_rn(src[r * stride + warp * klen + k], st.x)), st.y), bt[k]) : 0.0f;
+                }
+            }
+            __syncwarp();
+        } else if constexpr (kOwn && J != kJobO) {
+#pragma unroll
+            for (int t = 0; t < (R * klp + 31) / 32; ++t) {
+                const int i = lane + 32 * t, r = i / klp, k = i % klp;
+                if (i < R * klp) aw[r * C::seg + k] = k < klen ? src[r * stride + warp * klen + k] : 0.0f;
+            }
+            __syncwarp();
+        } else if constexpr (!kOwn) {
+            as = src + warp * klen;
+        }
+        float *dst = part + flip * C::part_stride + warp * pw;
+        if constexpr (pw <= 16) {
+            constexpr int RH = (R + 1) / 2;          // rows of a lane: r0, r0 + 2
+            const int c = lane & 15, r0 = R > 1 ? lane >> 4 : 0;
+            const float4 *wp = w4 + (pw < 16 ? min(c, pw - 1) : c);
+            float acc[RH];
+#pragma unroll
+            for (int r = 0; r < RH; ++r) acc[r] = 0.0f;
+#pragma unroll 8
+            for (int k = 0; k < klp / 4; ++k) {
+                const float4 w = wp[k * pw];
+#pragma unroll
+                for (int r = 0; r < RH; ++r) {
+                    const float4 x = *reinterpret_cast<const float4 *>(as + (r0 + 2 * r) * astride + 4 * k);
+                    acc[r] = fmaf(x.x, w.x, acc[r]);
+                    acc[r] = fmaf(x.y, w.y, acc[r]);
+                    acc[r] = fmaf(x.z, w.z, acc[r]);
+                    acc[r] = fmaf(x.w, w.w, acc[r]);
+                }
+            }
+            if (c < pw && (R > 1 || lane < 16))
+#pragma unroll
+                for (int r = 0; r < RH; ++r) dst[(r0 + 2 * r) * 16 * pw + c] = acc[r];
+        } else {
+            constexpr int NC = (pw + 31) / 32;       // 1 or 2 columns per lane
+            float acc[NC][R];
+#pragma unroll
+            for (int n = 0; n < NC; ++n)
+#pragma unroll
+                for (int r = 0; r < R; ++r) acc[n][r] = 0.0f;
+            const float4 *wp = w4 + (pw < 32 ? min(lane, pw - 1) : lane), *wq = w4 + (pw < 64 ? min(lane + 32, pw - 1) : lane + 32);
+#pragma unroll 4
+            for (int k = 0; k < klp / 4; ++k) {
+                float4 w[NC];
+                w[0] = wp[k * pw];
+                if constexpr (NC > 1) w[1] = wq[k * pw];
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const float4 x = *reinterpret_cast<const float4 *>(as + r * astride + 4 * k);
+#pragma unroll
+                    for (int n = 0; n < NC; ++n) acc[n][r] = fmaf(x.x, w[n].x, acc[n][r]);
+#pragma unroll
+                    for (int n = 0; n < NC; ++n) acc[n][r] = fmaf(x.y, w[n].y, acc[n][r]);
+#pragma unroll
+                    for (int n = 0; n < NC; ++n) acc[n][r] = fmaf(x.z, w[n].z, acc[n][r]);
+#pragma unroll
+                    for (int n = 0; n < NC; ++n) acc[n][r] = fmaf(x.w, w[n].w, acc[n][r]);
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+#pragma unroll
+                for (int n = 0; n < NC; ++n)
+                    if (32 * (n + 1) <= pw || lane + 32 * n < pw) dst[r * 16 * pw + lane + 32 * n] = acc[n][r];
+        }
+        float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
+        if constexpr (J != kJobVoc) {
+            // the first chunk has landed: warp 0 waited for it; another warp may not have, and asks again
+            if (tid < pw * R) {
+                wait(&full[slot0], slot_par);
+                bias = *reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(ring + slot0 * C::kSlot) + jb.weight_floats() + jb.ln_floats() + 4 * (tid / (4 * R)));
+            }
+        }
+        __syncthreads();                             // the partial sums are there; the chunks may be overwritten
+        if (warp == kWarps - 1) fetch(nch);
+        slot0 += nch;
+        if (slot0 >= lay.slots) { slot0 -= lay.slots; slot_par ^= 1u; }
+        return bias;
+    };
+    // Finishes part `pt` of a product: a thread adds up four columns of a row (partial sums in ascending order) and stores them
+    // into four of the sixteen blocks; the threads of the other receivers form the same sums, which is cheaper than handing them over.
+    auto finish = [&](auto jn, int pt, float4 bias, int layer, int p) {
+        constexpr int J = decltype(jn)::value;
+        constexpr ClusterJob jb = cluster_job_of(J, E, 64 * 64);
+        constexpr int pw = jb.width, stride = J == kJobQkv ? C::qs : J == kJobF1 ? C::fs : C::es;
+        constexpr int buf = J == kJobQkv ? C::qkv : J == kJobO ? C::xa : J == kJobF1 ? C::ff : C::xb;
+        constexpr int res = J == kJobO ? C::xb : C::xa;
+        constexpr int h = J == kJobQkv ? kQkv : J == kJobO ? kXa : J == kJobF1 ? kFf : kXb;
+        const int r = (tid >> 2) & (R - 1), g = tid / (4 * R), n = rank * jb.nc + pt * pw + 4 * g;
+        // the block's last columns may lie past its share (the last part) or past the matrix
+        if (g < pw / 4 && r < rows && pt * pw + 4 * g < jb.nc && n < jb.n) {
+            const float *ps = part + flip * C::part_stride + r * 16 * pw + 4 * g;
+            float4 v = *reinterpret_cast<const float4 *>(ps);
+#pragma unroll
+            for (int s = 1; s < 16; ++s) v = add4(v, *reinterpret_cast<const float4 *>(ps + s * pw));
+            v = add4(v, bias);
+            if constexpr (J == kJobF1) v = make_float4(fmaxf(0.0f, v.x), fmaxf(0.0f, v.y), fmaxf(0.0f, v.z), fmaxf(0.0f, v.w));
+            if constexpr (J == kJobO || J == kJobF2) v = add4(*reinterpret_cast<const float4 *>(sm + res + r * stride + n), v);
+            const uint32_t to = smem_u32(sm + buf + r * stride + n), bar = smem_u32(&hop[h]);
+#pragma unroll
+            for (int d = 0; d < 4; ++d) send4(to + peer[d], bar + peer[d], v);
+            if constexpr (J == kJobQkv) {
+                if (dq == (rank >> 2) && n >= E) {   // keys and values, for the later positions
+                    float *cache = (n < 2 * E ? a.kc : a.vc) + (size_t)layer * a.layer_stride + ((size_t)(row0 + r) * a.S + p) * E;
+                    *reinterpret_cast<float4 *>(cache + (n < 2 * E ? n - E : n - 2 * E)) = v;
+                }
+            }
+        }
+        flip ^= 1;
+    };
+
+    // ---- the attention of one position: units of (row, head, split), four warps each, dealt out over the blocks' warp groups.
+    //      A key's head is read by LPK lanes (4 numbers each), as in attn_decode.cu ----
+    constexpr int W4 = 4;
+    const int lpk_log = D <= 32 ? 3 : 4, LPK = 1 << lpk_log, KPW = 32 >> lpk_log;
+    const int slot4 = warp >> 2, w4i = warp & 3, lik = lane & (LPK - 1), kg = lane >> lpk_log;
+    const bool act = lik * 4 < D;
+    const float qscale = (1.0f / sqrtf((float)D)) * kLog2e;
+    const int units = rows * H * ns;
+    float *merge_s = sm + C::unit + slot4 * (W4 * 32 * 8);
+    struct Unit { int split, now, rec, mem; };       // its split; offsets of its head in qkv, of its record, of its row and head in a layer's cache
+    auto make_unit = [&](int u) {
+        const int split = u % ns, bh = u / ns, h = bh % H, r = bh / H;
+        return Unit{split, r * C::qs + h * D + lik * 4, u * rstride, (row0 + r) * a.S * E + h * D + lik * 4};
+    };
+    const int u0 = rank + kClusterBlocks * slot4;
+    const Unit first_unit = make_unit(min(u0, units - 1));
+    int per = 0;                                     // positions of a split at this step
+    float4 k4[kAhead], v4[kAhead];                   // rows of a unit that earlier steps wrote
+    auto ask = [&](const Unit &un, int layer, int p, int it0) {
+        const int j0 = un.split * per + (it0 * W4 + w4i) * KPW + kg, k1 = act ? min(p, un.split * per + per) : 0;
+        const size_t at = (size_t)layer * a.layer_stride + (size_t)un.mem + (size_t)j0 * E;
+        const float *kp = a.kc + at, *vp = a.vc + at;
+#pragma unroll
+        for (int it = 0; it < kAhead; ++it) {
+            k4[it] = v4[it] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (j0 + it * W4 * KPW < k1) {
+                k4[it] = __ldcg(reinterpret_cast<const float4 *>(kp + it * W4 * KPW * E));
+                v4[it] = __ldcg(reinterpret_cast<const float4 *>(vp + it * W4 * KPW * E));
+            }
+        }
+    };
+    auto attend = [&](int layer, int p) {
+#pragma unroll 1
+        for (int u = u0; u < units; u += 4 * kClusterBlocks) {
+            const Unit un = u == u0 ? first_unit : make_unit(u);
+            const int k0 = un.split * per, k1 = min(p + 1, k0 + per);
+            if (u != u0) ask(un, layer, p, 0);       // the first unit's rows were asked for ahead
+            const float *now = qkv + un.now;         // this position's query, key and value
+            float4 q4 = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (act) {
+                q4 = *reinterpret_cast<const float4 *>(now);
+                q4.x *= qscale; q4.y *= qscale; q4.z *= qscale; q4.w *= qscale;
+            }
+            Part acc{-1e30f, 0.0f, make_float4(0.f, 0.f, 0.f, 0.f)};
+            const int step = W4 * KPW;
+#pragma unroll 1
+            for (int it0 = 0; k0 + it0 * step < k1; it0 += kAhead) {
+                if (it0 > 0) ask(un, layer, p, it0);
+                const int j0 = k0 + (it0 * W4 + w4i) * KPW + kg;
+                const int own = p < k1 ? p - j0 : -1;                      // where this position's own row is among them
+                float s[kAhead];
+#pragma unroll
+                for (int it = 0; it < kAhead; ++it) {
+                    if (own == it * step && act) {
+                        k4[it] = *reinterpret_cast<const float4 *>(now + E);
+                        v4[it] = *reinterpret_cast<const float4 *>(now + 2 * E);
+                    }
+                    float x = q4.x * k4[it].x;
+                    x = fmaf(q4.y, k4[it].y, x);
+                    x = fmaf(q4.z, k4[it].z, x);
+                    s[it] = fmaf(q4.w, k4[it].w, x);
+                }
+#pragma unroll
+                for (int o = 1; o < 8; o <<= 1)
+#pragma unroll
+                    for (int it = 0; it < kAhead; ++it) s[it] += __shfl_xor_sync(0xffffffffu, s[it], o);
+                if (LPK > 8)
+#pragma unroll
+                    for (int it = 0; it < kAhead; ++it) s[it] += __shfl_xor_sync(0xffffffffu, s[it], 8);
+#pragma unroll
+                for (int it = 0; it < kAhead; ++it) {
+                    if (k0 + (it0 + it) * step >= k1) break;               // no lane of the four warps has a row there
+                    const float x = j0 + it * step < k1 ? s[it] : -INFINITY;
+                    const float mn = fmaxf(acc.m, x);
+                    const float alpha = ex2_approx(acc.m - mn), pr = ex2_approx(x - mn);
+                    acc.l = fmaf(acc.l, alpha, pr);
+                    acc.o.x = fmaf(pr, v4[it].x, acc.o.x * alpha);
+                    acc.o.y = fmaf(pr, v4[it].y, acc.o.y * alpha);
+                    acc.o.z = fmaf(pr, v4[it].z, acc.o.z * alpha);
+                    acc.o.w = fmaf(pr, v4[it].w, acc.o.w * alpha);
+                    acc.m = mn;
+                }
+            }
+#pragma unroll
+            for (int o = 8; o < 32; o <<= 1) {
+                if (o < LPK) continue;
+                const float m2 = __shfl_xor_sync(0xffffffffu, acc.m, o);
+                const float l2 = __shfl_xor_sync(0xffffffffu, acc.l, o);
+                float4 o2;
+                o2.x = __shfl_xor_sync(0xffffffffu, acc.o.x, o);
+                o2.y = __shfl_xor_sync(0xffffffffu, acc.o.y, o);
+                o2.z = __shfl_xor_sync(0xffffffffu, acc.o.z, o);
+                o2.w = __shfl_xor_sync(0xffffffffu, acc.o.w, o);
+                merge_part(acc, m2, l2, o2);
+            }
+            if (kg == 0) {
+                float *d = merge_s + (w4i * 32 + lik) * 8;
+                *reinterpret_cast<float4 *>(d) = acc.o;
+                *reinterpret_cast<float2 *>(d + 4) = make_float2(acc.m, acc.l);
+            }
+            asm volatile("bar.sync %0, 128;" ::"r"(1 + slot4) : "memory");
+            // each of the four warps merges the columns of its lanes' `lik`; its key groups serve different receivers
+            const float *m0 = merge_s + lik * 8;
+            Part t;
+            t.o = *reinterpret_cast<const float4 *>(m0);
+            t.m = m0[4]; t.l = m0[5];
+#pragma unroll
+            for (int w = 1; w < W4; ++w) {
+                const float4 o2 = *reinterpret_cast<const float4 *>(m0 + w * 256);
+                const float2 ml = *reinterpret_cast<const float2 *>(m0 + w * 256 + 4);
+                merge_part(t, ml.x, ml.y, o2);
+            }
+            const uint32_t dst = smem_u32(rec + un.rec), bar = smem_u32(&hop[kRec]);
+#pragma unroll 1
+            for (int d = kg; d < 4; d += KPW) {
+                const uint32_t pb = peer_addr(bar, 4 * w4i + d), pd = peer_addr(dst, 4 * w4i + d);
+                if (act) send4(pd + lik * 16, pb, t.o);
+                if (lik == 0) send2(pd + D * 4, pb, __float_as_uint(t.m), __float_as_uint(t.l));
+            }
+            if (u + 4 * kClusterBlocks < units) asm volatile("bar.sync %0, 128;" ::"r"(1 + slot4) : "memory");
+        }
+    };
+    // this warp's segment of the attention output from the records of all splits (attn_decode.cu's decode_combine_kernel)
+    constexpr int o_klen = E / 16;
+    auto combine = [&]() {
+#pragma unroll
+        for (int t = 0; t < (R * o_klen + 31) / 32; ++t) {
+            const int i = lane + 32 * t, r = i / o_klen, e = warp * o_klen + i % o_klen;
+            if (i < R * o_klen && r < rows) {
+                const int h = D == 32 ? e >> 5 : D == 64 ? e >> 6 : e / D, d = e - h * D;
+                const float *rc = rec + (r * H + h) * ns * rstride;
+                float M = -1e30f, Lsum = 0.0f, acc = 0.0f;
+                if (ns <= 8) {                       // all loads in flight at once
+                    float2 ml[8];
+                    float os[8];
+#pragma unroll
+                    for (int s = 0; s < 8; ++s) {
+                        if (s >= ns) break;
+                        ml[s] = *reinterpret_cast<const float2 *>(rc + s * rstride + D);
+                        os[s] = rc[s * rstride + d];
+                    }
+#pragma unroll
+                    for (int s = 0; s < 8; ++s) { if (s >= ns) break; M = fmaxf(M, ml[s].x); }
+#pragma unroll
+                    for (int s = 0; s < 8; ++s) {
+                        if (s >= ns) break;
+                        const float x = ex2_approx(ml[s].x - M);
+                        Lsum += ml[s].y * x;
+                        acc += os[s] * x;
+                    }
+                } else {
+#pragma unroll 1
+                    for (int s = 0; s < ns; ++s) M = fmaxf(M, rc[s * rstride + D]);
+#pragma unroll 1
+                    for (int s = 0; s < ns; ++s) {
+                        const float x = ex2_approx(rc[s * rstride + D] - M);
+                        Lsum += rc[s * rstride + D + 1] * x;
+                        acc += rc[s * rstride + d] * x;
+                    }
+                }
+                aw[r * C::seg + i % o_klen] = acc * (1.0f / fmaxf(Lsum, 1e-20f));
+            }
+        }
+        if constexpr ((o_klen & 3) != 0) {           // the padding of the segment
+            if (lane < R * 4 && (o_klen & ~3) + (lane & 3) >= o_klen) aw[(lane >> 2) * C::seg + (o_klen & ~3) + (lane & 3)] = 0.0f;
+        }
+        __syncwarp();
+    };
+    auto embed = [&](int p, int r, int id) {
+        const bool ok = id >= 0 && id < V;
+        if (tid < E) xb[r * C::es + tid] = ok ? __fadd_rn(a.tok[(size_t)id * E + tid], a.pos[(size_t)p * E + tid]) : 0.0f;
+    };
+    static_assert(E <= kThreads && E % 32 == 0, "");
+
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+        if (r < rows) embed(a.p0, r, a.p0 < a.n_prompt ? a.prompts[(size_t)(row0 + r) * a.n_prompt + a.p0] : a.ids[row0 + r]);
+    __syncthreads();
+#pragma unroll 1
+    for (int step = 0; step < a.nsteps; ++step) {
+        const int p = a.p0 + step;
+        per = (p + ns) / ns;
+#pragma unroll 1
+        for (int l = 0; l < a.L; ++l) {
+            ask(first_unit, l, p, 0);
+            if (l > 0) receive(kXb);
+#pragma unroll 1
+            for (int pt = 0; pt < cluster_job_of(kJobQkv, E, 0).parts; ++pt) finish(Job<kJobQkv>(), pt, product(Job<kJobQkv>(), xb), l, p);
+            receive(kQkv);
+            attend(l, p);
+            receive(kRec);
+            combine();
+#pragma unroll 1
+            for (int pt = 0; pt < cluster_job_of(kJobO, E, 0).parts; ++pt) finish(Job<kJobO>(), pt, product(Job<kJobO>(), nullptr), 0, 0);
+            receive(kXa);
+#pragma unroll 1
+            for (int pt = 0; pt < cluster_job_of(kJobF1, E, 0).parts; ++pt) finish(Job<kJobF1>(), pt, product(Job<kJobF1>(), xa), 0, 0);
+            receive(kFf);
+#pragma unroll 1
+            for (int pt = 0; pt < cluster_job_of(kJobF2, E, 0).parts; ++pt) finish(Job<kJobF2>(), pt, product(Job<kJobF2>(), ff), 0, 0);
+        }
+        receive(kXb);
+        const bool head = p >= a.n_prompt - 1, last = step + 1 == a.nsteps;
+        if (head) {
+            // thread = (row, column of the part); columns ascend from part to part, so a thread keeps its first maximum
+            float best = -INFINITY;
+            int bi = 0x7fffffff;
+            const int hr = tid >> 6, hc = tid & 63;
+            constexpr int pw = cluster_job_of(kJobVoc, E, 64 * 64).width;
+#pragma unroll 1
+            for (int pt = 0; pt < plan.voc.parts; ++pt) {
+                product(Job<kJobVoc>(), xb);
+                const int n = rank * plan.voc.nc + pt * pw + hc;
+                if (hr < rows && hc < pw && pt * pw + hc < plan.voc.nc && n < V) {
+                    const float *pp = part + flip * C::part_stride + hr * 16 * pw + hc;
+                    float v = pp[0];
+#pragma unroll
+                    for (int s = 1; s < 16; ++s) v = __fadd_rn(v, pp[s * pw]);
+                    if (last) a.logits[(size_t)(row0 + hr) * V + n] = v;
+                    if (v > best || bi == 0x7fffffff) { best = v; bi = n; }
+                }
+                flip ^= 1;
+            }
+            auto better = [&](float ov, int oi) {
+                if (oi != 0x7fffffff && (bi == 0x7fffffff || ov > best || (ov == best && oi < bi))) { best = ov; bi = oi; }
+            };
+            auto butterfly = [&]() {
+#pragma unroll 1
+                for (int o = 16; o > 0; o >>= 1) {
+                    const float ov = __shfl_xor_sync(0xffffffffu, best, o);
+                    const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+                    better(ov, oi);
+                }
+            };
+            if (hr < rows) {
+                butterfly();
+                if (lane < kClusterBlocks) {
+                    const uint32_t dst = smem_u32(amax + (hr * 32 + rank * 2 + (warp & 1)) * 2);
+                    send2(peer_addr(dst, lane), peer_addr(smem_u32(&hop[kAm]), lane), __float_as_uint(best), (uint32_t)bi);
+                }
+            }
+            asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+            receive(kAm);
+            if (warp < rows) {
+                best = __uint_as_float(amax[(warp * 32 + lane) * 2]);
+                bi = (int)amax[(warp * 32 + lane) * 2 + 1];
+                butterfly();
+                if (lane == 0) {
+                    next_id[warp] = bi;
+                    if (rank == 0) {
+                        a.ids[row0 + warp] = bi;
+                        const int col = p - (a.n_prompt - 1);
+                        if (col < a.n_new) a.out_ids[(size_t)(row0 + warp) * a.n_new + col] = bi;
+                    }
+                }
+            }
+            __syncthreads();
+        } else {
+            __syncthreads();                         // every warp is done with xb
+            asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+        }
+        if (!last)
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                if (r < rows) embed(p + 1, r, p + 1 < a.n_prompt ? a.prompts[(size_t)(row0 + r) * a.n_prompt + p + 1] : next_id[r]);
+        // the keys and values of this position reach the other blocks before the next one is attended to; the barrier also keeps a
+        // block from leaving while others still store into it
+        asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+        __syncthreads();
+    }
+    if (abort_flag) {                                // let copies in flight land before the shared memory is given back
+        const long long t0 = clock64();
+        while (clock64() - t0 < 4000000) {}
+    }
+}
+
+// One chunk per block of this grid: (chunk, owner).  Columns and inner indices past the matrix (or the owner's share) are zeros.
+__global__ void __launch_bounds__(256)
+cluster_pack_kernel(const ClusterJob j, int pt, const float *__restrict__ w, const float *__restrict__ bias, const float *__restrict__ gamma,
+                    const float *__restrict__ beta, uint8_t *dst, size_t block_bytes)
+{
+    const int pw = j.width, ch = blockIdx.x, owner = blockIdx.y;
+    const int first = owner * j.nc + pt * pw, end = min(j.n, (owner + 1) * j.nc), segs = 1 << j.seg_shift;
+    float *d = reinterpret_cast<float *>(dst + (size_t)owner * block_bytes + (size_t)ch * j.chunk_bytes());
+    for (int i = threadIdx.x; i < j.weight_floats(); i += blockDim.x) {
+        const int u = i & 3, c = (i >> 2) % pw, k4 = (i >> 2) / pw % (j.klp >> 2), s = (i >> 2) / pw / (j.klp >> 2);
+        const int k = 4 * k4 + u;
+        d[i] = (first + c < end && k < j.klen) ? w[(size_t)((ch * segs + s) * j.klen + k) * j.n + first + c] : 0.0f;
+    }
+    d += j.weight_floats();
+    if (j.ln)
+        for (int i = threadIdx.x; i < segs * j.klp; i += blockDim.x) {
+            const int s = i / j.klp, k = i % j.klp, at = (ch * segs + s) * j.klen + k;
+            d[i] = k < j.klen ? gamma[at] : 0.0f;
+            d[segs * j.klp + i] = k < j.klen ? beta[at] : 0.0f;
+        }
+    d += j.ln_floats();
+    for (int i = threadIdx.x; i < pw; i += blockDim.x) d[i] = (bias && first + i < end) ? bias[first + i] : 0.0f;
+}
+
+// A launch of `clusters` clusters of sixteen blocks
+struct ClusterLaunch {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    ClusterLaunch(int clusters, size_t smem, cudaStream_t st)
+    {
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = kClusterBlocks;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.gridDim = dim3((unsigned)(clusters * kClusterBlocks));
+        cfg.blockDim = dim3(kThreads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+    }
+};
+
+template <int E, int R>
+cudaError_t prepare_kernel()
+{
+    auto kern = cluster_steps_kernel<E, R>;
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMost);
+}
+
+// `f.template operator()<E, R>()` for the shape; -1 where there is no kernel for it
+template <int R, typename F>
+int with_width(int E, F f)
+{
+    switch (E) {
+#define HIPGPT_CLUSTER(W) case W: return f(Width<W, R>());
+    HIPGPT_CLUSTER(128) HIPGPT_CLUSTER(160) HIPGPT_CLUSTER(192) HIPGPT_CLUSTER(224) HIPGPT_CLUSTER(256) HIPGPT_CLUSTER(288)
+    HIPGPT_CLUSTER(320) HIPGPT_CLUSTER(352) HIPGPT_CLUSTER(384)
+#undef HIPGPT_CLUSTER
+    default: return -1;
+    }
+}
+template <typename F>
+int with_kernel(int E, int rows, F f) { return rows == 1 ? with_width<1>(E, f) : with_width<2>(E, f); }
+
+}  // namespace
+
+ClusterPlan cluster_plan(int V, int S, int E, int L, int H, int F)
+{
+    ClusterPlan p = {};
+    const int D = E / H;
+    if (D % 4 != 0 || D > 64 || F != 4 * E) return p;
+    // the output projection's parts have the width the kernel is compiled for; the vocabulary decides how many there are
+    p.voc = cluster_job_of(kJobVoc, E, 64 * 64);
+    p.voc.n = V;
+    p.voc.nc = 4 * ((V + 63) / 64);
+    p.voc.parts = (p.voc.nc + p.voc.width - 1) / p.voc.width;
+    for (int i = 0; i < kJobs; ++i) {
+        const ClusterJob j = i == kJobVoc ? p.voc : cluster_job_of(i, E, V);
+        const int times = i == kJobVoc ? 1 : L;
+        p.block_bytes += (size_t)times * j.parts * j.chunks() * j.chunk_bytes();
+        p.all_chunks += times * j.parts * j.chunks();
+        if (i == kJobF2) p.layer_chunks = p.all_chunks;
+    }
+    if (p.all_chunks > 1024 || p.block_bytes > 0xffffffffu || (long long)S * E > 1 << 24) return p;
+    // how many clusters of sixteen blocks, one block per SM, the GPU holds at the same time
+    const int rc = with_kernel(E, 2, [&](auto w) {
+        if (prepare_kernel<decltype(w)::kE, decltype(w)::kR>() != cudaSuccess) return 1;
+        ClusterLaunch l(1, kSmemMost, nullptr);
+        return cudaOccupancyMaxActiveClusters(&p.clusters_most, cluster_steps_kernel<decltype(w)::kE, decltype(w)::kR>, &l.cfg) == cudaSuccess ? 0 : 1;
+    });
+    if (rc > 0) cudaGetLastError();
+    p.ok = rc == 0 && p.clusters_most > 0;
+    return p;
+}
+
+void cluster_table(const ClusterPlan &p, int E, int L, uint2 *table)
+{
+    unsigned off = 0;
+    auto job = [&](const ClusterJob &j) {
+        for (int i = 0; i < j.parts * j.chunks(); ++i) {
+            *table++ = make_uint2(off, (unsigned)j.chunk_bytes());
+            off += (unsigned)j.chunk_bytes();
+        }
+    };
+    for (int l = 0; l < L; ++l)
+        for (int i = kJobQkv; i <= kJobF2; ++i) job(cluster_job_of(i, E, 0));
+    job(p.voc);
+}
+
+int cluster_pack(const ClusterPlan &p, int E, const ClusterLayerWeights *layers, int L, const float *wout, uint8_t *dst, cudaStream_t st)
+{
+    size_t off = 0;
+    auto job = [&](const ClusterJob &j, const float *w, const float *bias, const float *gamma, const float *beta) {
+        for (int pt = 0; pt < j.parts; ++pt) {
+            cluster_pack_kernel<<<dim3(j.chunks(), kClusterBlocks), 256, 0, st>>>(j, pt, w, bias, gamma, beta, dst + off, p.block_bytes);
+            off += (size_t)j.chunks() * j.chunk_bytes();
+        }
+    };
+    for (int l = 0; l < L; ++l) {
+        const ClusterLayerWeights &w = layers[l];
+        job(cluster_job_of(kJobQkv, E, 0), w.wqkv, w.bqkv, w.g1, w.be1);
+        job(cluster_job_of(kJobO, E, 0), w.wo, w.bo, nullptr, nullptr);
+        job(cluster_job_of(kJobF1, E, 0), w.w1, w.b1, w.g2, w.be2);
+        job(cluster_job_of(kJobF2, E, 0), w.w2, w.b2, nullptr, nullptr);
+    }
+    job(p.voc, wout, nullptr, nullptr, nullptr);
+    return check_launch("cluster_pack_kernel");
+}
+
+// One sequence per cluster while every cluster is resident, then two; larger batches take the launches, whose matmuls share a
+// weight among eight rows.  The ring has to hold a part (sixteen chunks at most) and more.
+int cluster_rows(const ClusterPlan &p, int B, int E, int H, int ns)
+{
+    if (!p.ok) return 0;
+    const int rows = B <= p.clusters_most ? 1 : (B + 1) / 2 <= p.clusters_most ? 2 : 0;
+    if (rows == 0) return 0;
+    const int slots = with_kernel(E, rows, [&](auto w) { return rest_of<decltype(w)::kE, decltype(w)::kR>(H, E / H, ns, p.all_chunks).slots; });
+    return slots >= 9 ? rows : 0;
+}
+
+int launch_cluster_steps(const ClusterPlan &p, const ClusterArgs &a, int E, int rows, cudaStream_t st)
+{
+    return with_kernel(E, rows, [&](auto w) {
+        constexpr int kE = decltype(w)::kE, kR = decltype(w)::kR;
+        const Rest lay = rest_of<kE, kR>(a.H, kE / a.H, a.ns, p.all_chunks);
+        cudaError_t e = prepare_kernel<kE, kR>();
+        if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "cluster_steps_kernel attributes: %s", cudaGetErrorString(e));
+        ClusterLaunch l((a.B + rows - 1) / rows, (size_t)lay.total, st);
+        e = cudaLaunchKernelEx(&l.cfg, cluster_steps_kernel<kE, kR>, p, a, lay);
+        if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "cluster_steps_kernel launch: %s", cudaGetErrorString(e));
+        return HIPGPT_OK;
+    });
+}
+
+}  // namespace hipgpt

@@ -19,6 +19,7 @@
 // layer-norm sums are 32 lane-strided partial sums joined by a butterfly; nothing else is
 // contracted (explicit __fmul_rn / __fadd_rn), divisions and square roots are IEEE.
 #include "attn_common.cuh"
+#include "gpt_cluster.cuh"
 
 #include <math.h>
 #include <stdlib.h>
@@ -235,9 +236,7 @@ __global__ void advance_pos_kernel(int *pos_ptr)
     *pos_ptr += 1;
 }
 
-struct LayerW {
-    const float *wqkv, *wo, *w1, *w2, *bqkv, *bo, *b1, *b2, *g1, *be1, *g2, *be2;
-};
+using LayerW = ClusterLayerWeights;
 
 // ------------------------------------------------------------------------------------------------
 // The persistent form: ONE cooperative launch runs `nsteps` token positions.  A step of the graph
@@ -562,6 +561,10 @@ struct GptDecoder {
     bool persistent_ok = false;                      // head_dim, shared memory and co-residency allow it
     int grid_blocks = 0;
     size_t fused_smem = 0;
+    // the cluster form (gpt_cluster.cu): the weights once more, as the sixteen blocks' shares
+    ClusterPlan plan = {};
+    uint8_t *d_shares = nullptr;
+    uint2 *d_table = nullptr;
     cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};   // start, prompt done, all done
     // test hook (hipgpt_gpt_debug_stall_barrier): the next persistent call starts with an arrival counter
     // that can never complete and this wait limit, so that the barrier's give-up path runs
@@ -737,6 +740,16 @@ int hipgpt_gpt_create(hipgpt_gpt **out, const float *h_weights, int V, int S, in
         TRY(cudaMalloc(&g->d_err, sizeof(int)));
         TRY(cudaMemsetAsync(g->d_err, 0, sizeof(int), g->stream));
     }
+    g->plan = cluster_plan(V, S, E, L, H, F);
+    if (g->plan.ok) {
+        TRY(cudaMalloc(&g->d_shares, g->plan.block_bytes * kClusterBlocks));
+        const int rc = cluster_pack(g->plan, E, g->lw.data(), L, g->wout, g->d_shares, g->stream);
+        if (rc != HIPGPT_OK) return bail(rc);
+        std::vector<uint2> table(g->plan.all_chunks);
+        cluster_table(g->plan, E, L, table.data());
+        TRY(cudaMalloc(&g->d_table, table.size() * sizeof(uint2)));
+        TRY(cudaMemcpy(g->d_table, table.data(), table.size() * sizeof(uint2), cudaMemcpyHostToDevice));
+    }
     TRY(cudaStreamSynchronize(g->stream));
 #undef TRY
     *out = reinterpret_cast<hipgpt_gpt *>(g);
@@ -765,7 +778,9 @@ int hipgpt_gpt_generate(hipgpt_gpt *handle, const int *h_prompts, int B, int n_p
         g->prompt_cap = B * n_prompt;
     }
     const bool persistent = g->mode == HIPGPT_GPT_MODE_PERSISTENT && g->persistent_ok;
-    int rc = persistent ? HIPGPT_OK : build_graph(*g, B, n_prompt, n_new);
+    const int ns = decode_splits(B, g->H, g->E / g->H, g->S);
+    const int cluster = persistent ? 0 : cluster_rows(g->plan, B, g->E, g->H, ns);     // sequences per cluster, 0: the graph
+    int rc = persistent || cluster ? HIPGPT_OK : build_graph(*g, B, n_prompt, n_new);
     if (rc != HIPGPT_OK) return rc;
     CUDA_OK(cudaMemcpyAsync(g->d_prompts, h_prompts, (size_t)B * n_prompt * sizeof(int), cudaMemcpyHostToDevice, g->stream));
     CUDA_OK(cudaMemsetAsync(g->d_pos, 0, sizeof(int), g->stream));
@@ -780,7 +795,7 @@ int hipgpt_gpt_generate(hipgpt_gpt *handle, const int *h_prompts, int B, int n_p
         a.kc = g->d_kc; a.vc = g->d_vc; a.layer_stride = (size_t)g->max_batch * g->S * g->E;
         a.x = g->d_x; a.q = g->d_q; a.att = g->d_att; a.ff = g->d_ff; a.logits = g->d_logits; a.scratch = g->d_scratch;
         a.ids = g->d_ids; a.out_ids = g->d_out; a.pos_ptr = g->d_pos; a.prompts = g->d_prompts;
-        a.B = B; a.n_prompt = n_prompt; a.n_new = n_new; a.ns = decode_splits(B, g->H, g->E / g->H, g->S);
+        a.B = B; a.n_prompt = n_prompt; a.n_new = n_new; a.ns = ns;
         a.bar = g->d_bar; a.cnt = g->d_cnt; a.err = g->d_err;
         a.bar_limit = kBarrierLimitCycles;
         if (g->stall_next) {
@@ -798,6 +813,19 @@ int hipgpt_gpt_generate(hipgpt_gpt *handle, const int *h_prompts, int B, int n_p
         a.nsteps = n_new - 1;
         if (a.nsteps > 0)
             CUDA_OK(cudaLaunchCooperativeKernel((const void *)gpt_steps_kernel, dim3(g->grid_blocks), dim3(32 * kSeg), params, g->fused_smem, g->stream));
+    } else if (cluster) {
+        ClusterArgs a{};
+        a.tok = g->tok; a.pos = g->pos; a.stream = g->d_shares; a.table = g->d_table;
+        a.kc = g->d_kc; a.vc = g->d_vc; a.layer_stride = (size_t)g->max_batch * g->S * g->E;
+        a.logits = g->d_logits; a.ids = g->d_ids; a.out_ids = g->d_out; a.err = g->d_err; a.prompts = g->d_prompts;
+        a.V = g->V; a.S = g->S; a.L = g->L; a.H = g->H;
+        a.B = B; a.n_prompt = n_prompt; a.n_new = n_new; a.ns = ns;
+        a.nsteps = n_prompt;
+        if ((rc = launch_cluster_steps(g->plan, a, g->E, cluster, g->stream)) != HIPGPT_OK) return rc;
+        CUDA_OK(cudaEventRecord(e1, g->stream));
+        a.p0 = n_prompt;
+        a.nsteps = n_new - 1;
+        if (a.nsteps > 0 && (rc = launch_cluster_steps(g->plan, a, g->E, cluster, g->stream)) != HIPGPT_OK) return rc;
     } else {
         for (int p = 0; p < n_prompt; ++p) CUDA_OK(cudaGraphLaunch(g->graph, g->stream));
         CUDA_OK(cudaEventRecord(e1, g->stream));
@@ -808,14 +836,14 @@ int hipgpt_gpt_generate(hipgpt_gpt *handle, const int *h_prompts, int B, int n_p
     if (h_logits_last)
         CUDA_OK(cudaMemcpyAsync(h_logits_last, g->d_logits, (size_t)B * g->V * sizeof(float), cudaMemcpyDeviceToHost, g->stream));
     int h_err = 0;
-    if (persistent) CUDA_OK(cudaMemcpyAsync(&h_err, g->d_err, sizeof(int), cudaMemcpyDeviceToHost, g->stream));
+    if (persistent || cluster) CUDA_OK(cudaMemcpyAsync(&h_err, g->d_err, sizeof(int), cudaMemcpyDeviceToHost, g->stream));
     CUDA_OK(cudaStreamSynchronize(g->stream));
     if (h_err) {
         cudaMemsetAsync(g->d_err, 0, sizeof(int), g->stream);
         cudaMemsetAsync(g->d_bar, 0, 2 * sizeof(unsigned), g->stream);
         cudaMemsetAsync(g->d_cnt, 0, (size_t)g->max_batch * g->H * sizeof(unsigned), g->stream);
         cudaStreamSynchronize(g->stream);
-        rc = fail(HIPGPT_ERR_CUDA, "persistent generation kernel: a wait at the grid barrier ran out");
+        rc = fail(HIPGPT_ERR_CUDA, persistent ? "persistent generation kernel: a wait at the grid barrier ran out" : "generation kernel: a wait inside a cluster ran out");
     }
     float a = 0.f, b = 0.f;
     cudaEventElapsedTime(&a, e0, e1);
@@ -862,6 +890,8 @@ void hipgpt_gpt_destroy(hipgpt_gpt *handle)
     if (g->d_bar) cudaFree(g->d_bar);
     if (g->d_cnt) cudaFree(g->d_cnt);
     if (g->d_err) cudaFree(g->d_err);
+    if (g->d_shares) cudaFree(g->d_shares);
+    if (g->d_table) cudaFree(g->d_table);
     for (cudaEvent_t ev : g->ev) if (ev) cudaEventDestroy(ev);
     if (g->stream) cudaStreamDestroy(g->stream);
     delete g;

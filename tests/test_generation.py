@@ -137,3 +137,26 @@ def test_gpu_generation_forms_agree_and_a_handle_serves_many_requests():
             got[mode] = logits
         assert float(np.abs(got[generation.MODE_PERSISTENT] - got[generation.MODE_GRAPH]).max()) <= 1e-5
     dec.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cfg,B,n_prompt,n_new", [
+    (dict(V=131, S=40, E=128, L=2, H=4, F=512), 1, 3, 20),          # one cluster, fewer columns than blocks times four
+    (dict(V=777, S=64, E=160, L=2, H=5, F=640), 3, 1, 30),          # segments of 10 inner indices: padded
+    (dict(V=1000, S=300, E=256, L=1, H=4, F=1024), 9, 5, 40),       # head_dim 64, two sequences per cluster, one left over
+    (dict(V=1371, S=96, E=384, L=1, H=12, F=1536), 2, 4, 24),       # products in several parts
+    (dict(V=300, S=700, E=128, L=1, H=2, F=512), 2, 300, 60),       # contexts of more rows than a lane asks for ahead
+    (dict(V=200, S=40, E=128, L=1, H=4, F=512), 15, 2, 10),         # a batch for the replayed graph
+    (dict(V=200, S=40, E=128, L=1, H=4, F=256), 2, 2, 10)])         # a feed-forward width for the replayed graph
+def test_gpu_generation_by_clusters_at_its_edges(cfg, B, n_prompt, n_new):
+    pytest.importorskip("torch")
+    from hipgpt_b200 import generation
+    w = synth.gpt_weights(31, **cfg, std=0.08)
+    prompts = synth.token_ids(32, (B, n_prompt), cfg["V"])
+    ref_ids, ref_logits = ob.gpt_generate(w, **cfg, prompts=prompts, n_new=n_new, fma=True)
+    dec = generation.GptDecoder(w, **cfg, max_batch=B)
+    for _ in range(2):
+        ids, logits, _, _ = dec.generate(prompts, n_new)
+        assert np.array_equal(ids, ref_ids)
+        assert float(np.abs(logits - ref_logits).max()) <= 1e-4
+    dec.close()
