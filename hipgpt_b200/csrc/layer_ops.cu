@@ -7,113 +7,128 @@
 //                   dimension (src/hip_kernels.cpp:69-154).  One accumulator per output, terms added
 //                   k ascending with fused multiply-add, the bias added once at the end: the
 //                   summation order of the reference kernel, hence bit-identical to its arithmetic.
-//                   Register-tiled (each thread 64 outputs), operands staged through shared memory.
+//                   Register-tiled, operands staged through shared memory.
 //   layer norm      src/hip_kernels.cpp:757-848: mean, variance about the mean, 1/sqrt(var + 1e-5),
 //                   gamma (x - mean) inv + beta.  One warp per row; the reference reduces in 64-lane
 //                   waves, so sums agree to rounding (about 1e-7), not bitwise.
 //   dropout         src/hip_kernels.cpp:944-970 with the generator at :24-42: the mask is a pure function
 //                   of the element index; restated in integer arithmetic, bit-identical.
 //   add, ReLU, embedding lookup   src/hip_kernels.cpp:721-730, :248-258, :537-599; bit-identical.
-#include "attn_common.cuh"
+#include "tc_primitives.cuh"
 
 #include <math.h>
 
 namespace hipgpt {
 namespace {
 
-constexpr int kGemmThreads = 256;
 constexpr int kBK = 16;
 
-// C tile of BM x BN per block, 16 x 16 threads, TM x TN outputs per thread.  A thread's rows are
-// contiguous (ty * TM ...), its columns come in groups of four, 64 apart (tx * 4 + 64 j), so that the
-// shared-memory reads of a warp are either broadcasts (A) or 256 contiguous bytes (B).
-template <int BM, int BN>
-__global__ void __launch_bounds__(kGemmThreads)
-matmul_exact_kernel(const float *A, const float *__restrict__ B, const float *__restrict__ bias,
-                    float *C, int M, int N, int K)          // A and C may be the same buffer (see the launcher)
+// A tile is 8 TM x 16 TN outputs, 128 threads of TM x TN; TM and TN are chosen per call so that the tiles fill the SMs evenly
+// (launch_matmul_tiles).
+// Two bounds: the FFMA pipe, TM TN clocks per inner index and warp, and the return path of shared memory, which hands a warp 128
+// bytes per clock whether lanes ask for the same words or not: 4 (TM + TN) clocks for the four warps of an SM's quarters.  8 x 8
+// outputs per thread are bound by the second; 8 x 16 (and 7 x 16) leave it at three quarters of the first.  The rest is kept out
+// of the issue slots: multiply-adds run on pairs of columns (fma.rn.f32x2, one instruction for two roundings), and both operands
+// come by 16-byte asynchronous copies, three stages, A untransposed (a thread reads four inner indices of a row at once).
+// Registers alone (the same multiply-adds without loads) reach 61 TFLOP/s; here 54 at 16384 x 512 x 1536 (one inner index after
+// another in 128 x 128 tiles, operands through registers: 47.7).  With 8192 rows: 256 -> 768 columns 80 -> 66 us, 256 -> 256 35 -> 27,
+// 256 -> 1024 105 -> 84, 1024 -> 256 125 -> 91.
+constexpr int kTileThreads = 128;
+constexpr int kTileStages = 3;
+template <int TM, int TN>
+struct TileCfg {
+    static constexpr int BM = 8 * TM, BN = 16 * TN;
+    static constexpr int AStride = kBK + 4;                              // floats between rows of A in shared memory
+    static constexpr int kStageFloats = BM * AStride + kBK * BN;
+    static constexpr size_t kSmem = (size_t)kTileStages * kStageFloats * 4;
+};
+template <int TM, int TN>
+__global__ void __launch_bounds__(kTileThreads, TM * TN > 64 ? 2 : 3)
+matmul_tile_kernel(const float *A, const float *__restrict__ B, const float *__restrict__ bias, float *C,     // A and C may be one buffer
+                   int M, int N, int K, int col_tiles)
 {
-    constexpr int TM = BM / 16, TN = BN / 16, NJ = TN / 4;
-    constexpr int A4 = (BM * kBK / 4) / kGemmThreads;      // float4 loads of A per thread and tile
-    constexpr int B4 = (kBK * BN / 4) / kGemmThreads;
-    __shared__ __align__(16) float As[2][kBK][BM + 4];     // transposed: As[k][m]
-    __shared__ __align__(16) float Bs[2][kBK][BN];
+    using T = TileCfg<TM, TN>;
+    constexpr int BM = T::BM, BN = T::BN;
+    extern __shared__ __align__(16) float tile_s[];                      // [stage][A: BM rows of 16 | B: 16 rows of BN]
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    const int row0 = blockIdx.y * BM, col0 = blockIdx.x * BN;
+    // column tile fastest: blocks that run side by side share rows of A
+    const int row0 = (int)(blockIdx.x / col_tiles) * BM, col0 = (int)(blockIdx.x % col_tiles) * BN;
 
-    float acc[TM][TN];
+    float2 acc[TM][TN / 2];
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = 0.0f;
-
-    float4 ra[A4], rb[B4];
-    auto fetch = [&](int k0) {
-#pragma unroll
-        for (int i = 0; i < A4; ++i) {
-            const int f = tid + i * kGemmThreads;            // float4 index inside the A tile: 4 per row
-            const int r = row0 + (f >> 2), k = k0 + (f & 3) * 4;
-            ra[i] = (r < M && k < N) ? *reinterpret_cast<const float4 *>(A + (size_t)r * N + k) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-#pragma unroll
-        for (int i = 0; i < B4; ++i) {
-            const int f = tid + i * kGemmThreads;            // BN / 4 per row
-            const int k = k0 + f / (BN / 4), c = col0 + (f % (BN / 4)) * 4;
-            rb[i] = (k < N && c < K) ? *reinterpret_cast<const float4 *>(B + (size_t)k * K + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-    };
-    auto stash = [&](int buf) {
-#pragma unroll
-        for (int i = 0; i < A4; ++i) {
-            const int f = tid + i * kGemmThreads;
-            const int m = f >> 2, k = (f & 3) * 4;
-            As[buf][k][m] = ra[i].x; As[buf][k + 1][m] = ra[i].y; As[buf][k + 2][m] = ra[i].z; As[buf][k + 3][m] = ra[i].w;
-        }
-#pragma unroll
-        for (int i = 0; i < B4; ++i) {
-            const int f = tid + i * kGemmThreads;
-            *reinterpret_cast<float4 *>(&Bs[buf][f / (BN / 4)][(f % (BN / 4)) * 4]) = rb[i];
-        }
-    };
+        for (int j = 0; j < TN / 2; ++j) acc[i][j] = make_float2(0.0f, 0.0f);
 
     const int ntiles = (N + kBK - 1) / kBK;
-    fetch(0);
-    stash(0);
-    __syncthreads();
+    auto copy = [&](int t) {
+        if (t < ntiles) {
+            float *as = tile_s + (t % kTileStages) * T::kStageFloats, *bs = as + BM * T::AStride;
+            const int k0 = t * kBK;
+#pragma unroll
+            for (int i = 0; i < (BM * 4 + kTileThreads - 1) / kTileThreads; ++i) {
+                const int f = tid + i * kTileThreads, m = f >> 2, k = (f & 3) * 4;
+                const bool in = row0 + m < M && k0 + k < N;
+                if (BM * 4 % kTileThreads == 0 || f < BM * 4) cp_async16(as + m * T::AStride + k, A + (in ? (size_t)(row0 + m) * N + k0 + k : 0), in);
+            }
+#pragma unroll
+            for (int i = 0; i < kBK * BN / 4 / kTileThreads; ++i) {
+                const int f = tid + i * kTileThreads, kr = f / (BN / 4), cc = (f % (BN / 4)) * 4;
+                const bool in = k0 + kr < N && col0 + cc < K;
+                cp_async16(bs + kr * BN + cc, B + (in ? (size_t)(k0 + kr) * K + col0 + cc : 0), in);
+            }
+        }
+        cp_async_commit();
+    };
+    copy(0);
+    copy(1);
     for (int t = 0; t < ntiles; ++t) {
-        const int buf = t & 1;
-        if (t + 1 < ntiles) fetch((t + 1) * kBK);            // global loads in flight during the products
+        cp_async_wait_1();                                   // tile t is there (this thread's part)
+        __syncthreads();                                     // everybody's part; and everybody is done with tile t - 1
+        copy(t + 2);
+        const float *as = tile_s + (t % kTileStages) * T::kStageFloats + ty * TM * T::AStride;
+        const float *bs = tile_s + (t % kTileStages) * T::kStageFloats + BM * T::AStride + tx * 4;
+        float2 b[2][TN / 2];
+        auto load_b = [&](int k) {
+#pragma unroll
+            for (int j = 0; j < TN / 4; ++j) *reinterpret_cast<float4 *>(&b[k & 1][2 * j]) = *reinterpret_cast<const float4 *>(bs + k * BN + 64 * j);
+        };
+        float a[TM][4];
+        auto load_a = [&](int i, int k) { *reinterpret_cast<float4 *>(a[i]) = *reinterpret_cast<const float4 *>(as + i * T::AStride + k); };
+#pragma unroll
+        for (int i = 0; i < TM; ++i) load_a(i, 0);
+        load_b(0);
 #pragma unroll
         for (int k = 0; k < kBK; ++k) {
-            float a[TM], b[TN];
+            if (k + 1 < kBK) load_b(k + 1);
+            float2 aa[TM];
 #pragma unroll
-            for (int i = 0; i < TM; i += 4)
-                *reinterpret_cast<float4 *>(&a[i]) = *reinterpret_cast<const float4 *>(&As[buf][k][ty * TM + i]);
+            for (int i = 0; i < TM; ++i) aa[i] = make_float2(a[i][k & 3], a[i][k & 3]);
+            if ((k & 3) == 3 && k + 1 < kBK)
 #pragma unroll
-            for (int j = 0; j < NJ; ++j)
-                *reinterpret_cast<float4 *>(&b[4 * j]) = *reinterpret_cast<const float4 *>(&Bs[buf][k][tx * 4 + 64 * j]);
+                for (int i = 0; i < TM; ++i) load_a(i, k + 1);
 #pragma unroll
-            for (int i = 0; i < TM; ++i)
+            for (int j = 0; j < TN / 2; ++j)
 #pragma unroll
-                for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+                for (int i = 0; i < TM; ++i) acc[i][j] = ffma2(aa[i], b[k & 1][j], acc[i][j]);
         }
-        if (t + 1 < ntiles) {
-            stash(buf ^ 1);                                  // the other buffer was last read two tiles ago
-            __syncthreads();
-        }
+    }
+    float4 bb[TN / 4];
+#pragma unroll
+    for (int j = 0; j < TN / 4; ++j) {
+        const int c = col0 + tx * 4 + 64 * j;
+        bb[j] = (bias && c < K) ? *reinterpret_cast<const float4 *>(bias + c) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
         const int r = row0 + ty * TM + i;
         if (r >= M) continue;
 #pragma unroll
-        for (int j = 0; j < NJ; ++j) {
+        for (int j = 0; j < TN / 4; ++j) {
             const int c = col0 + tx * 4 + 64 * j;
             if (c >= K) continue;                            // K % 4 == 0 on this path: a group of four is in or out
-            float4 v = make_float4(acc[i][4 * j], acc[i][4 * j + 1], acc[i][4 * j + 2], acc[i][4 * j + 3]);
-            if (bias) {
-                const float4 bb = *reinterpret_cast<const float4 *>(bias + c);
-                v.x += bb.x; v.y += bb.y; v.z += bb.z; v.w += bb.w;
-            }
+            float4 v = make_float4(acc[i][2 * j].x, acc[i][2 * j].y, acc[i][2 * j + 1].x, acc[i][2 * j + 1].y);
+            if (bias) { v.x += bb[j].x; v.y += bb[j].y; v.z += bb[j].z; v.w += bb[j].w; }
             *reinterpret_cast<float4 *>(C + (size_t)r * K + c) = v;
         }
     }
@@ -246,6 +261,39 @@ bool overlap(const void *a, size_t na, const void *b, size_t nb)
 
 }  // namespace
 
+// The tile of a product.  In place (C over A) a block must own whole rows: it stores after its last read.  Cost: clocks per inner index of the SM with the most tiles (a tile's own bound, see above; an SM with a
+// single block of four warps hides less latency, about a fifth), the larger tile among equals.
+struct TileChoice {
+    void (*kernel)(const float *, const float *, const float *, float *, int, int, int, int);
+    int tm, tn;
+    size_t smem;
+};
+template <int TM, int TN>
+TileChoice tile_choice() { return {matmul_tile_kernel<TM, TN>, TM, TN, TileCfg<TM, TN>::kSmem}; }
+
+static int launch_matmul_tiles(const float *A, const float *B, const float *bias, float *C, int M, int N, int K, bool whole_rows, cudaStream_t st)
+{
+    static const TileChoice choices[] = {tile_choice<8, 16>(), tile_choice<7, 16>(), tile_choice<6, 16>(), tile_choice<5, 16>(), tile_choice<8, 8>(), tile_choice<7, 8>(),
+                                         tile_choice<6, 8>(), tile_choice<5, 8>(), tile_choice<4, 8>(), tile_choice<3, 8>(), tile_choice<4, 4>(), tile_choice<2, 4>()};
+    constexpr int kSms = 148;
+    const TileChoice *best = nullptr;
+    double best_cost = 0.0;
+    long long best_tiles = 0;
+    for (const TileChoice &c : choices) {
+        if (whole_rows && K > 16 * c.tn) continue;
+        const long long tiles = (long long)((M + 8 * c.tm - 1) / (8 * c.tm)) * ((K + 16 * c.tn - 1) / (16 * c.tn));
+        const long long per_sm = (tiles + kSms - 1) / kSms;
+        const int fma = c.tm * c.tn, loads = 4 * (c.tm + c.tn), clocks = fma > loads ? fma : loads;
+        const double cost = (double)per_sm * clocks * (per_sm == 1 ? 1.2 : 1.0);
+        if (!best || cost < best_cost) { best = &c; best_cost = cost; best_tiles = tiles; }
+    }
+    if (best_tiles > 2147483647LL) return fail(HIPGPT_ERR_BAD_ARG, "matmul: %lld tiles are too many", best_tiles);
+    const cudaError_t e = cudaFuncSetAttribute(best->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)best->smem);
+    if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+    best->kernel<<<(unsigned)best_tiles, kTileThreads, best->smem, st>>>(A, B, bias, C, M, N, K, (K + 16 * best->tn - 1) / (16 * best->tn));
+    return check_launch("matmul_tile_kernel");
+}
+
 int launch_matmul_exact(const float *A, const float *B, const float *bias, float *C, int M, int N, int K, cudaStream_t st)
 {
     if (M == 0 || K == 0) return HIPGPT_OK;
@@ -255,17 +303,8 @@ int launch_matmul_exact(const float *A, const float *B, const float *bias, float
     // HipGPT's layer projects in place (src/transformer_layer.cpp:220 passes the same buffer as A and C).  That is
     // safe when one block holds whole rows of C: it reads its rows of A completely before it stores.
     const bool alias = overlap(A, (size_t)M * N * 4, C, (size_t)M * K * 4);
-    if (vec && K <= 256) {
-        const dim3 grid(1, (M + 63) / 64);
-        matmul_exact_kernel<64, 256><<<grid, kGemmThreads, 0, st>>>(A, B, bias, C, M, N, K);
-        return check_launch("matmul_exact_kernel");
-    }
-    if (alias) return fail(HIPGPT_ERR_UNSUPPORTED, "matmul in place needs an output of at most 256 columns, a multiple of 4 (K=%d)", K);
-    if (vec) {
-        const dim3 grid((K + 127) / 128, (M + 127) / 128);
-        matmul_exact_kernel<128, 128><<<grid, kGemmThreads, 0, st>>>(A, B, bias, C, M, N, K);
-        return check_launch("matmul_exact_kernel");
-    }
+    if (alias && (!vec || K > 256)) return fail(HIPGPT_ERR_UNSUPPORTED, "matmul in place needs an output of at most 256 columns, a multiple of 4 (K=%d)", K);
+    if (vec) return launch_matmul_tiles(A, B, bias, C, M, N, K, alias, st);
     const long long n = (long long)M * K;
     matmul_plain_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(A, B, bias, C, M, N, K);
     return check_launch("matmul_plain_kernel");

@@ -39,6 +39,29 @@ def test_matmul_is_bit_identical_to_the_reference_order(M, N, K, bias):
     assert np.array_equal(dC.cpu().numpy(), want)
 
 
+@pytest.mark.parametrize("M,K", [(8903, 388), (7123, 388), (6222, 388), (4747, 132), (4194, 132), (3556, 132), (5922, 68), (4739, 4), (1805, 132),
+                                 (2374, 68), (2371, 4), (1, 20)])
+def test_matmul_tiles_are_bit_identical_to_the_reference_order(M, K):
+    """One shape for every tile the exact matmul chooses from, with rows and columns left over, an inner dimension that is no
+    multiple of a tile's depth, and (for 256 columns at most) the same product in place."""
+    lib = _capi.lib()
+    N = 36
+    A, W, b = synth.normal(4, (M, N)), synth.normal(5, (N, K), 0.1), synth.normal(6, (K,))
+    want = ob.matmul(A, W, b, M, N, K, fma=True)
+    dA, dW, db, dC = dev(A), dev(W), dev(b), torch.full((M, K), float("nan"), device="cuda")
+    _capi.check(lib.hipgpt_matmul(dA.data_ptr(), dW.data_ptr(), db.data_ptr(), dC.data_ptr(), M, N, K, _st()))
+    torch.cuda.synchronize()
+    assert np.array_equal(dC.cpu().numpy(), want)
+    if K <= 256:                                        # square in place
+        W2 = synth.normal(7, (K, K), 0.1)
+        A2 = synth.normal(8, (M, K))
+        want = ob.matmul(A2, W2, b, M, K, K, fma=True)
+        dA2, dW2 = dev(A2), dev(W2)
+        _capi.check(lib.hipgpt_matmul(dA2.data_ptr(), dW2.data_ptr(), db.data_ptr(), dA2.data_ptr(), M, K, K, _st()))
+        torch.cuda.synchronize()
+        assert np.array_equal(dA2.cpu().numpy(), want)
+
+
 @pytest.mark.parametrize("M,N,K,bias", [(8192, 256, 768, True), (300, 256, 768, True), (64, 1024, 256, True), (257, 256, 1024, False), (130, 64, 5000, False),
                                         (33, 100, 20, True), (5, 7, 3, False), (1, 256, 256, True), (129, 65, 129, True)])
 def test_tensor_core_matmul_is_fp32_grade(M, N, K, bias):
