@@ -18,6 +18,8 @@
 
 #include <math.h>
 
+#include <initializer_list>
+
 namespace hipgpt {
 namespace {
 
@@ -54,6 +56,8 @@ matmul_tile_kernel(const float *A, const float *__restrict__ B, const float *__r
     // column tile fastest: blocks that run side by side share rows of A
     const int row0 = (int)(blockIdx.x / col_tiles) * BM, col0 = (int)(blockIdx.x % col_tiles) * BN;
 
+    dependency_wait();                                       // overlapped launch: nothing is read before the kernel before this one has completed
+    dependents_may_start();
     float2 acc[TM][TN / 2];
 #pragma unroll
     for (int i = 0; i < TM; ++i)
@@ -146,55 +150,65 @@ __global__ void matmul_plain_kernel(const float *__restrict__ A, const float *__
     C[idx] = bias ? s + bias[c] : s;
 }
 
+// The kernels below are passes over memory of a few microseconds: 16-byte accesses where the pointers allow, and overlapped
+// launches, so that a kernel's blocks are placed while the kernel before it drains (without: about a microsecond between two).
+
 // One warp per row.  Sums: lane l adds elements l, l + 32, ... ascending, then a butterfly over the lanes.
 // Separately rounded multiplies and adds (no contraction), IEEE division and square root: the CPU oracle
-// built without contraction reproduces every bit.
+// built without contraction reproduces every bit.  NV > 0: the row (E <= 32 NV) stays in registers between the three sweeps.
+template <int NV>
 __global__ void layer_norm_rows_kernel(const float *x, float *y, const float *__restrict__ g,
                                        const float *__restrict__ b, int rows, int E)
 {
+    dependency_wait();
+    dependents_may_start();
     const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (row >= rows) return;
     const float *xr = x + (size_t)row * E;
-    float s = 0.0f;
-    for (int e = lane; e < E; e += 32) s = __fadd_rn(s, xr[e]);
+    float *yr = y + (size_t)row * E;
+    float v[NV > 0 ? NV : 1];
+    float s = 0.0f, q = 0.0f;
+    if constexpr (NV > 0) {
+#pragma unroll
+        for (int i = 0; i < NV; ++i) v[i] = lane + 32 * i < E ? xr[lane + 32 * i] : 0.0f;
+#pragma unroll
+        for (int i = 0; i < NV; ++i) s = lane + 32 * i < E ? __fadd_rn(s, v[i]) : s;
+    } else {
+        for (int e = lane; e < E; e += 32) s = __fadd_rn(s, xr[e]);
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s = __fadd_rn(s, __shfl_xor_sync(0xffffffffu, s, o));
     const float mean = __fdiv_rn(s, (float)E);
-    float v = 0.0f;
-    for (int e = lane; e < E; e += 32) {
-        const float d = __fsub_rn(xr[e], mean);
-        v = __fadd_rn(v, __fmul_rn(d, d));
+    if constexpr (NV > 0) {
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            v[i] = __fsub_rn(v[i], mean);
+            q = lane + 32 * i < E ? __fadd_rn(q, __fmul_rn(v[i], v[i])) : q;
+        }
+    } else {
+        for (int e = lane; e < E; e += 32) {
+            const float d = __fsub_rn(xr[e], mean);
+            q = __fadd_rn(q, __fmul_rn(d, d));
+        }
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, o));
-    const float inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(v, (float)E), 1e-5f)));
-    float *yr = y + (size_t)row * E;
-    for (int e = lane; e < E; e += 32)
-        yr[e] = __fadd_rn(__fmul_rn(__fmul_rn(g[e], __fsub_rn(xr[e], mean)), inv), b[e]);
+    for (int o = 16; o > 0; o >>= 1) q = __fadd_rn(q, __shfl_xor_sync(0xffffffffu, q, o));
+    const float inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(q, (float)E), 1e-5f)));
+    if constexpr (NV > 0) {
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            const int e = lane + 32 * i;
+            if (e < E) yr[e] = __fadd_rn(__fmul_rn(__fmul_rn(__ldg(g + e), v[i]), inv), __ldg(b + e));
+        }
+    } else {
+        for (int e = lane; e < E; e += 32)
+            yr[e] = __fadd_rn(__fmul_rn(__fmul_rn(g[e], __fsub_rn(xr[e], mean)), inv), b[e]);
+    }
 }
 
 // The reference seeds a xorwow state from the element index, its 256-thread block and its thread
 // (a = idx + 1, b = block + 1, c = thread + 1, d = idx * block + 1) and draws once: only a and d reach
 // that first draw.  u = (t + 1) / 2^32; the element is dropped when u < p, else divided by (1 - p).
-__global__ void dropout_index_kernel(const float *in, float *out, float *__restrict__ mask, float p, unsigned n)   // in == out allowed
-{
-    const unsigned idx = blockIdx.x * 256u + threadIdx.x;
-    if (idx >= n) return;
-    const unsigned s = idx + 1u;
-    unsigned t = idx * blockIdx.x + 1u;
-    t ^= t >> 2;
-    t ^= t << 1;
-    t ^= s ^ (s << 4);
-    const float u = __fdiv_rn((float)(t + 1u), 4294967296.0f);
-    const bool drop = u < p;
-    out[idx] = drop ? 0.0f : __fdiv_rn(in[idx], __fsub_rn(1.0f, p));
-    if (mask) mask[idx] = drop ? 0.0f : 1.0f;
-}
-
-// out = residual + dropout(in): the sub-layer tail of the reference's block (dropout in place, then the residual
-// add, src/transformer_layer.cpp:242-244 and :250-252) in one pass over memory instead of three.  The same generator,
-// the same division, the same addition: bit-identical to hipgpt_dropout followed by hipgpt_add_inplace.  Four
-// consecutive elements per thread when the count and the pointers allow 16-byte accesses.
 __device__ __forceinline__ bool dropped(unsigned idx, float p)
 {
     const unsigned s = idx + 1u;
@@ -202,55 +216,99 @@ __device__ __forceinline__ bool dropped(unsigned idx, float p)
     t ^= t >> 2;
     t ^= t << 1;
     t ^= s ^ (s << 4);
-    return __fdiv_rn((float)(t + 1u), 4294967296.0f) < p;
+    return __fmul_rn((float)(t + 1u), 2.3283064365386963e-10f) < p;       // / 2^32: exact
 }
 
+// out = dropout(in), or out = residual + dropout(in): the sub-layer tail of the reference's block (dropout in place, then
+// the residual add, src/transformer_layer.cpp:242-244 and :250-252) in one pass over memory instead of three, bit-identical to
+// hipgpt_dropout followed by hipgpt_add_inplace.  Four consecutive elements per thread when the count and the pointers allow
+// 16-byte accesses.
+template <bool RESIDUAL>
 __global__ void __launch_bounds__(256)
-dropout_residual_kernel(const float *in, const float *residual, float *out, float *__restrict__ mask, float p, unsigned n, int vec)   // out may be in or residual
+dropout_kernel(const float *in, const float *residual, float *out, float *__restrict__ mask, float p, unsigned n, int vec)   // out may be in or residual
 {
+    dependency_wait();
+    dependents_may_start();
     const float keep = __fsub_rn(1.0f, p);
     if (vec) {
         const unsigned i4 = (blockIdx.x * 256u + threadIdx.x) * 4u;
         if (i4 >= n) return;
-        const float4 x = *reinterpret_cast<const float4 *>(in + i4), r = *reinterpret_cast<const float4 *>(residual + i4);
+        const float4 x = *reinterpret_cast<const float4 *>(in + i4);
+        float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (RESIDUAL) r = *reinterpret_cast<const float4 *>(residual + i4);
         const bool d0 = dropped(i4, p), d1 = dropped(i4 + 1u, p), d2 = dropped(i4 + 2u, p), d3 = dropped(i4 + 3u, p);
         float4 o;
-        o.x = __fadd_rn(r.x, d0 ? 0.0f : __fdiv_rn(x.x, keep));
-        o.y = __fadd_rn(r.y, d1 ? 0.0f : __fdiv_rn(x.y, keep));
-        o.z = __fadd_rn(r.z, d2 ? 0.0f : __fdiv_rn(x.z, keep));
-        o.w = __fadd_rn(r.w, d3 ? 0.0f : __fdiv_rn(x.w, keep));
+        o.x = d0 ? 0.0f : __fdiv_rn(x.x, keep);
+        o.y = d1 ? 0.0f : __fdiv_rn(x.y, keep);
+        o.z = d2 ? 0.0f : __fdiv_rn(x.z, keep);
+        o.w = d3 ? 0.0f : __fdiv_rn(x.w, keep);
+        if (RESIDUAL) { o.x = __fadd_rn(r.x, o.x); o.y = __fadd_rn(r.y, o.y); o.z = __fadd_rn(r.z, o.z); o.w = __fadd_rn(r.w, o.w); }
         *reinterpret_cast<float4 *>(out + i4) = o;
         if (mask) *reinterpret_cast<float4 *>(mask + i4) = make_float4(d0 ? 0.f : 1.f, d1 ? 0.f : 1.f, d2 ? 0.f : 1.f, d3 ? 0.f : 1.f);
     } else {
         const unsigned idx = blockIdx.x * 256u + threadIdx.x;
         if (idx >= n) return;
         const bool d = dropped(idx, p);
-        out[idx] = __fadd_rn(residual[idx], d ? 0.0f : __fdiv_rn(in[idx], keep));
+        const float o = d ? 0.0f : __fdiv_rn(in[idx], keep);
+        out[idx] = RESIDUAL ? __fadd_rn(residual[idx], o) : o;
         if (mask) mask[idx] = d ? 0.0f : 1.0f;
     }
 }
 
-__global__ void add_inplace_kernel(float *__restrict__ a, const float *__restrict__ b, long long n)
+// a = a + b, or a = max(0, a); `n4` groups of four elements, then the rest one by one
+template <bool ADD>
+__global__ void __launch_bounds__(256)
+pass_kernel(float *a, const float *__restrict__ b, long long n4, long long n)
 {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) a[i] = __fadd_rn(a[i], b[i]);
+    dependency_wait();
+    dependents_may_start();
+    const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+    if (i < n4) {
+        float4 x = reinterpret_cast<const float4 *>(a)[i];
+        if (ADD) {
+            const float4 y = __ldg(reinterpret_cast<const float4 *>(b) + i);
+            x = make_float4(__fadd_rn(x.x, y.x), __fadd_rn(x.y, y.y), __fadd_rn(x.z, y.z), __fadd_rn(x.w, y.w));
+        } else {
+            x = make_float4(fmaxf(0.0f, x.x), fmaxf(0.0f, x.y), fmaxf(0.0f, x.z), fmaxf(0.0f, x.w));
+        }
+        reinterpret_cast<float4 *>(a)[i] = x;
+    } else {
+        const long long e = 4 * n4 + (i - n4);
+        if (e < n) a[e] = ADD ? __fadd_rn(a[e], b[e]) : fmaxf(0.0f, a[e]);
+    }
 }
 
-__global__ void relu_kernel(float *a, long long n)
+// out[t][e] = tok[id_t][e] + pos[t mod S][e]; an id outside [0, V) gives a row of zeros.  VEC: four elements per thread.
+template <bool VEC>
+__global__ void __launch_bounds__(256)
+embedding_kernel(const int *__restrict__ ids, const float *__restrict__ tok, const float *__restrict__ pos,
+                 float *__restrict__ out, long long T, int S, int V, int E)
 {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) a[i] = fmaxf(0.0f, a[i]);
-}
-
-// out[t][e] = tok[id_t][e] + pos[t mod S][e]; an id outside [0, V) gives a row of zeros.
-__global__ void embedding_kernel(const int *__restrict__ ids, const float *__restrict__ tok, const float *__restrict__ pos,
-                                 float *__restrict__ out, long long T, int S, int V, int E)
-{
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    dependency_wait();
+    dependents_may_start();
+    constexpr int W = VEC ? 4 : 1;
+    const long long i = ((long long)blockIdx.x * 256 + threadIdx.x) * W;
     if (i >= T * E) return;
     const long long t = i / E;
     const int e = (int)(i % E), id = ids[t];
-    out[i] = (id < 0 || id >= V) ? 0.0f : __fadd_rn(tok[(size_t)id * E + e], pos[(size_t)(t % S) * E + e]);
+    const bool ok = id >= 0 && id < V;
+    if constexpr (VEC) {
+        float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (ok) {
+            const float4 x = __ldg(reinterpret_cast<const float4 *>(tok + (size_t)id * E + e)), y = __ldg(reinterpret_cast<const float4 *>(pos + (size_t)(t % S) * E + e));
+            o = make_float4(__fadd_rn(x.x, y.x), __fadd_rn(x.y, y.y), __fadd_rn(x.z, y.z), __fadd_rn(x.w, y.w));
+        }
+        *reinterpret_cast<float4 *>(out + i) = o;
+    } else {
+        out[i] = ok ? __fadd_rn(tok[(size_t)id * E + e], pos[(size_t)(t % S) * E + e]) : 0.0f;
+    }
+}
+
+bool aligned16(std::initializer_list<const void *> ps)
+{
+    uintptr_t all = 0;
+    for (const void *p : ps) all |= reinterpret_cast<uintptr_t>(p);
+    return (all & 15) == 0;
 }
 
 bool overlap(const void *a, size_t na, const void *b, size_t nb)
@@ -288,10 +346,11 @@ static int launch_matmul_tiles(const float *A, const float *B, const float *bias
         if (!best || cost < best_cost) { best = &c; best_cost = cost; best_tiles = tiles; }
     }
     if (best_tiles > 2147483647LL) return fail(HIPGPT_ERR_BAD_ARG, "matmul: %lld tiles are too many", best_tiles);
-    const cudaError_t e = cudaFuncSetAttribute(best->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)best->smem);
-    if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-    best->kernel<<<(unsigned)best_tiles, kTileThreads, best->smem, st>>>(A, B, bias, C, M, N, K, (K + 16 * best->tn - 1) / (16 * best->tn));
-    return check_launch("matmul_tile_kernel");
+    cudaError_t e = cudaFuncSetAttribute(best->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)best->smem);
+    if (e == cudaSuccess)
+        e = launch_overlapped(best->kernel, dim3((unsigned)best_tiles), dim3(kTileThreads), best->smem, st, A, B, bias, C, M, N, K, (K + 16 * best->tn - 1) / (16 * best->tn));
+    if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "matmul_tile_kernel: %s", cudaGetErrorString(e));
+    return HIPGPT_OK;
 }
 
 int launch_matmul_exact(const float *A, const float *B, const float *bias, float *C, int M, int N, int K, cudaStream_t st)
@@ -310,52 +369,58 @@ int launch_matmul_exact(const float *A, const float *B, const float *bias, float
     return check_launch("matmul_plain_kernel");
 }
 
+namespace {
+int launched(cudaError_t e, const char *what) { return e == cudaSuccess ? HIPGPT_OK : fail(HIPGPT_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e)); }
+}  // namespace
+
 int launch_layer_norm_rows(const float *x, float *y, const float *g, const float *b, int rows, int E, cudaStream_t st)
 {
     if (rows == 0 || E == 0) return HIPGPT_OK;
-    layer_norm_rows_kernel<<<(rows + 7) / 8, 256, 0, st>>>(x, y, g, b, rows, E);
-    return check_launch("layer_norm_rows_kernel");
+    const auto kern = E <= 128 ? layer_norm_rows_kernel<4> : E <= 256 ? layer_norm_rows_kernel<8> : E <= 512 ? layer_norm_rows_kernel<16>
+                      : E <= 1024 ? layer_norm_rows_kernel<32> : layer_norm_rows_kernel<0>;
+    return launched(launch_overlapped(kern, dim3((unsigned)((rows + 7) / 8)), dim3(256), 0, st, x, y, g, b, rows, E), "layer_norm_rows_kernel");
 }
 
 int launch_dropout_index(const float *in, float *out, float *mask, float p, long long n, cudaStream_t st)
 {
     if (n == 0) return HIPGPT_OK;
     if (n > 0xffffffffLL) return fail(HIPGPT_ERR_BAD_ARG, "dropout over %lld elements: the reference's index is 32 bits wide", n);
-    dropout_index_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(in, out, mask, p, (unsigned)n);
-    return check_launch("dropout_index_kernel");
+    const int vec = n % 4 == 0 && aligned16({in, out, mask});
+    return launched(launch_overlapped(dropout_kernel<false>, dim3((unsigned)(((vec ? n / 4 : n) + 255) / 256)), dim3(256), 0, st, in, (const float *)nullptr, out, mask, p,
+                                      (unsigned)n, vec), "dropout_kernel");
 }
 
 int launch_dropout_residual(const float *in, const float *residual, float *out, float *mask, float p, long long n, cudaStream_t st)
 {
     if (n == 0) return HIPGPT_OK;
     if (n > 0xffffffffLL) return fail(HIPGPT_ERR_BAD_ARG, "dropout over %lld elements: the reference's index is 32 bits wide", n);
-    const uintptr_t all = reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(residual) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(mask);
-    const int vec = (n % 4 == 0) && (all & 15) == 0;
-    const long long threads = vec ? n / 4 : n;
-    dropout_residual_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(in, residual, out, mask, p, (unsigned)n, vec);
-    return check_launch("dropout_residual_kernel");
+    const int vec = n % 4 == 0 && aligned16({in, residual, out, mask});
+    return launched(launch_overlapped(dropout_kernel<true>, dim3((unsigned)(((vec ? n / 4 : n) + 255) / 256)), dim3(256), 0, st, in, residual, out, mask, p, (unsigned)n, vec),
+                    "dropout_kernel");
 }
 
 int launch_add_inplace_n(float *a, const float *b, long long n, cudaStream_t st)
 {
     if (n == 0) return HIPGPT_OK;
-    add_inplace_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(a, b, n);
-    return check_launch("add_inplace_kernel");
+    const long long n4 = aligned16({a, b}) ? n / 4 : 0, threads = n4 + (n - 4 * n4);
+    return launched(launch_overlapped(pass_kernel<true>, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, st, a, b, n4, n), "add_inplace");
 }
 
 int launch_relu_n(float *a, long long n, cudaStream_t st)
 {
     if (n == 0) return HIPGPT_OK;
-    relu_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(a, n);
-    return check_launch("relu_kernel");
+    const long long n4 = aligned16({a}) ? n / 4 : 0, threads = n4 + (n - 4 * n4);
+    return launched(launch_overlapped(pass_kernel<false>, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, st, a, (const float *)nullptr, n4, n), "relu");
 }
 
 int launch_embedding_rows(const int *ids, const float *tok, const float *pos, float *out, int B, int S, int V, int E, cudaStream_t st)
 {
     const long long n = (long long)B * S * E;
     if (n == 0) return HIPGPT_OK;
-    embedding_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(ids, tok, pos, out, (long long)B * S, S, V, E);
-    return check_launch("embedding_kernel");
+    const bool vec = E % 4 == 0 && aligned16({tok, pos, out});
+    const long long threads = vec ? n / 4 : n;
+    return launched(launch_overlapped(vec ? embedding_kernel<true> : embedding_kernel<false>, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, st, ids, tok, pos, out,
+                                      (long long)B * S, S, V, E), "embedding_kernel");
 }
 
 }  // namespace hipgpt
