@@ -87,6 +87,8 @@ bwd_pack_kernel(const float *__restrict__ q, const float *__restrict__ k, const 
                 uint8_t *__restrict__ img, size_t img_bytes, int S, int Spad, int E, int H, int tasks)
 {
     constexpr int PARTS = D / 32;
+    dependency_wait();
+    dependents_may_start();
     const int task = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (task >= tasks) return;
     const int part = task % PARTS, rb = (task / PARTS) % (Spad / 8), bh = task / PARTS / (Spad / 8);
@@ -700,9 +702,8 @@ int launch_cfg(const float *g, const float *q, const float *k, const float *v, c
         const size_t off = (size_t)b0 * S * E;
         const float *p = STORED ? probs + (size_t)b0 * H * S * S : nullptr;
         const int tasks = nb * H * (Spad / 8) * (D / 32);
-        bwd_pack_kernel<D><<<dim3((unsigned)((tasks + 7) / 8), 4), 256, 0, st>>>(q + off, k + off, v + off, g + off, img, img_bytes, S, Spad, E, H, tasks);
-        rc = check_launch("bwd_pack_kernel");
-        if (rc != HIPGPT_OK) return rc;
+        e = launch_overlapped(bwd_pack_kernel<D>, dim3((unsigned)((tasks + 7) / 8), 4), dim3(256), 0, st, q + off, k + off, v + off, g + off, img, img_bytes, S, Spad, E, H, tasks);
+        if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "bwd_pack_kernel launch: %s", cudaGetErrorString(e));
         const dim3 grid((unsigned)(nb * H * nblk));
         e = launch_overlapped(rows, grid, dim3(kThreads), rows_smem, st, (const uint8_t *)img, img_bytes, p, dq + off, lse, w, S, Spad, E, H, nblk, c);
         if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "bwd_rows_kernel launch: %s", cudaGetErrorString(e));

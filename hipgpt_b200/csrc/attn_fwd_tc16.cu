@@ -168,6 +168,9 @@ kv_pack_kernel(const float *__restrict__ K, const float *__restrict__ V, float *
     using C = Tc16Cfg<D>;
     constexpr int PPR = C::PPR, RPT = kPackThreads / PPR, NP = kKeys / RPT;      // rows covered per pass, pieces per thread
     __shared__ float red[2][kPackThreads / 32];
+    // overlapped launch; the wait comes first, because the attention kernel reads Q before its own wait: it may only come in once
+    // the kernel before this one has completed
+    dependency_wait();
     dependents_may_start();                          // the attention kernel's blocks may come in as this grid's blocks leave
     const int kt = blockIdx.x, bh = blockIdx.y;
     const int b = bh / H, h = bh % H;
@@ -755,9 +758,15 @@ int launch_tc16_cfg(const float *q, const float *k, const float *v, float *out, 
             e = cudaStreamWaitEvent(side, attended[g & 1], 0);               // the group that used this buffer has been attended to
             if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "event hand-off: %s", cudaGetErrorString(e));
         }
-        kv_pack_kernel<D><<<dim3((unsigned)ntk, (unsigned)(nb * H)), kPackThreads, 0, ps>>>(k + off, v + off, tmax, buf, buf + kbytes, S, E, H, ntk, ntiles);
-        rc = check_launch("kv_pack_kernel");
-        if (rc != HIPGPT_OK) return rc;
+        const dim3 pgrid((unsigned)ntk, (unsigned)(nb * H));
+        if (overlap) {                               // on the second stream, behind an event
+            kv_pack_kernel<D><<<pgrid, kPackThreads, 0, ps>>>(k + off, v + off, tmax, buf, buf + kbytes, S, E, H, ntk, ntiles);
+            rc = check_launch("kv_pack_kernel");
+            if (rc != HIPGPT_OK) return rc;
+        } else {
+            e = launch_overlapped(kv_pack_kernel<D>, pgrid, dim3(kPackThreads), 0, ps, k + off, v + off, tmax, buf, buf + kbytes, S, E, H, ntk, ntiles);
+            if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "kv_pack_kernel launch: %s", cudaGetErrorString(e));
+        }
         if (overlap) {
             e = cudaEventRecord(packed[g & 1], side);
             if (e == cudaSuccess) e = cudaStreamWaitEvent(st, packed[g & 1], 0);

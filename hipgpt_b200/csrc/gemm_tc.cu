@@ -85,6 +85,8 @@ __global__ void __launch_bounds__(256) gemm_amax_kernel(const float *__restrict_
 // With ln_g / ln_b given, the row is layer-normalised first (mean and variance over its N values, eps 1e-5, times gamma
 // plus beta: launch_layer_norm_forward, src/hip_kernels.cpp:757-848, to rounding), so that LN + projection of the
 // reference's block (src/transformer_layer.cpp:240-241, 246-247) need no pass over memory of their own.
+// NV > 0: the row (at most 256 NV values) stays in registers from its one read to the stores; 0: it is read again for every sweep.
+template <int NV>
 __global__ void __launch_bounds__(128) gemm_pack_a_kernel(const float *__restrict__ A, uint8_t *__restrict__ img, float *__restrict__ row_inv,
                                                            int M, int N, int KT, const float *__restrict__ ln_g, const float *__restrict__ ln_b)
 {
@@ -107,31 +109,44 @@ __global__ void __launch_bounds__(128) gemm_pack_a_kernel(const float *__restric
         }
     };
     const int depth = KT * kTK;
+    float held[NV > 0 ? NV : 1][8];
+    if constexpr (NV > 0) {
+#pragma unroll
+        for (int i = 0; i < NV; ++i) raw8(lane * 8 + 256 * i, held[i]);          // (past N: zeros)
+    }
+    // f(k0, values) for this lane's runs of eight
+    auto sweep = [&](auto f) {
+        if constexpr (NV > 0) {
+#pragma unroll
+            for (int i = 0; i < NV; ++i) f(lane * 8 + 256 * i, held[i]);
+        } else {
+            for (int k0 = lane * 8; k0 < depth; k0 += 256) {
+                float v[8];
+                raw8(k0, v);
+                f(k0, v);
+            }
+        }
+    };
     float mean = 0.0f, rstd = 1.0f;
     if (ln_g) {
         float sum = 0.0f;
-        for (int k0 = lane * 8; k0 < depth; k0 += 256) {
-            float v[8];
-            raw8(k0, v);
+        sweep([&](int, float (&v)[8]) {
 #pragma unroll
             for (int j = 0; j < 8; ++j) sum += v[j];             // values past N are zeros
-        }
+        });
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
         mean = sum / (float)N;
         float var = 0.0f;
-        for (int k0 = lane * 8; k0 < depth; k0 += 256) {
-            float v[8];
-            raw8(k0, v);
+        sweep([&](int k0, float (&v)[8]) {
 #pragma unroll
             for (int j = 0; j < 8; ++j) { const float d = (k0 + j < N) ? v[j] - mean : 0.0f; var = fmaf(d, d, var); }
-        }
+        });
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) var += __shfl_xor_sync(0xffffffffu, var, o);
         rstd = 1.0f / sqrtf(var / (float)N + 1e-5f);
     }
-    auto load8 = [&](int k0, float (&v)[8]) {
-        raw8(k0, v);
+    auto normalised = [&](int k0, float (&v)[8]) {
         if (ln_g) {
 #pragma unroll
             for (int j = 0; j < 8; ++j)
@@ -139,20 +154,19 @@ __global__ void __launch_bounds__(128) gemm_pack_a_kernel(const float *__restric
         }
     };
     float amax = 0.0f;
-    for (int k0 = lane * 8; k0 < depth; k0 += 256) {
-        float v[8];
-        load8(k0, v);
+    sweep([&](int k0, float (&v)[8]) {
+        normalised(k0, v);                                       // (held in registers: normalised in place)
 #pragma unroll
         for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(v[j]));
-    }
+    });
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
     const float s = pow2_scale(amax);
     if (lane == 0) row_inv[m] = pow2_inverse(s);
     const int mt = m / kTM, r = m % kTM;
-    for (int k0 = lane * 8; k0 < depth; k0 += 256) {             // the row is read again: it is in L1 / L2
-        float v[8];
-        load8(k0, v);
+    sweep([&](int k0, float (&v)[8]) {
+        if (NV > 0 && k0 >= depth) return;
+        if constexpr (NV == 0) normalised(k0, v);
         uint32_t hi[4], lo[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -165,7 +179,7 @@ __global__ void __launch_bounds__(128) gemm_pack_a_kernel(const float *__restric
         uint8_t *stage = img + ((size_t)mt * KT + kt) * kAStage;
         *reinterpret_cast<uint4 *>(stage + sw128(r, c)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
         *reinterpret_cast<uint4 *>(stage + kABlk + sw128(r, c)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-    }
+    });
 }
 
 // One block per 8 reduction rows of a (64-deep slice kt, 128-column tile nt) of B [N][K] (N inner, K the output width).
@@ -459,18 +473,13 @@ int pack_b(const float *B, int N, int K, uint8_t *bimg, float *b_amax, cudaStrea
 
 // A -> its stage images, then the product kernel, with B's images given
 int pack_a_and_multiply(const float *A, const uint8_t *bimg, const float *b_amax, const float *bias, float *C, int M, int N, int K,
-                        uint8_t *aimg, float *row_inv, bool first_is_plain, int dev, cudaStream_t st, const float *ln_g = nullptr, const float *ln_b = nullptr)
+                        uint8_t *aimg, float *row_inv, int dev, cudaStream_t st, const float *ln_g = nullptr, const float *ln_b = nullptr)
 {
     const int MT = (M + kTM - 1) / kTM, NT = (K + kTN - 1) / kTN, KT = (N + kTK - 1) / kTK;
     cudaError_t e;
-    if (first_is_plain) {
-        // nothing of this call precedes the pack kernel: a plain launch, so that the product kernel, which waits for the
-        // pack kernel only, is ordered after everything before the call (the kernel's own wait then returns at once)
-        gemm_pack_a_kernel<<<(unsigned)(MT * kTM / 4), 128, 0, st>>>(A, aimg, row_inv, M, N, KT, ln_g, ln_b);
-    } else {
-        e = launch_overlapped(gemm_pack_a_kernel, dim3((unsigned)(MT * kTM / 4)), dim3(128), 0, st, A, aimg, row_inv, M, N, KT, ln_g, ln_b);
-        if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "gemm_pack_a_kernel launch: %s", cudaGetErrorString(e));
-    }
+    const auto pack = KT <= 4 ? gemm_pack_a_kernel<1> : KT <= 8 ? gemm_pack_a_kernel<2> : KT <= 16 ? gemm_pack_a_kernel<4> : KT <= 32 ? gemm_pack_a_kernel<8> : gemm_pack_a_kernel<0>;
+    e = launch_overlapped(pack, dim3((unsigned)(MT * kTM / 4)), dim3(128), 0, st, A, aimg, row_inv, M, N, KT, ln_g, ln_b);
+    if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "gemm_pack_a_kernel launch: %s", cudaGetErrorString(e));
     int rc = check_launch("gemm_pack_a_kernel");
     if (rc != HIPGPT_OK) return rc;
     int sms = 0;
@@ -504,7 +513,7 @@ int launch_matmul_tc(const float *A, const float *B, const float *bias, float *C
     rc = set_gemm_attr();
     if (rc == HIPGPT_OK) rc = pack_b(B, N, K, bimg, b_amax, st);
     if (rc != HIPGPT_OK) return rc;
-    return pack_a_and_multiply(A, bimg, b_amax, bias, C, M, N, K, aimg, row_inv, false, dev, st, ln_g, ln_b);
+    return pack_a_and_multiply(A, bimg, b_amax, bias, C, M, N, K, aimg, row_inv, dev, st, ln_g, ln_b);
 }
 
 // ---- a right-hand side packed once (the weights of a layer) and used by many products ---------------------------
@@ -552,7 +561,7 @@ int launch_matmul_tc_prepared(const float *A, const PackedB *b, const float *bia
     if (rc != HIPGPT_OK) return rc;
     rc = set_gemm_attr();
     if (rc != HIPGPT_OK) return rc;
-    return pack_a_and_multiply(A, b->bimg, b->b_amax, bias, C, M, N, K, scratch, reinterpret_cast<float *>(scratch + abytes), true, dev, st, ln_g, ln_b);
+    return pack_a_and_multiply(A, b->bimg, b->b_amax, bias, C, M, N, K, scratch, reinterpret_cast<float *>(scratch + abytes), dev, st, ln_g, ln_b);
 }
 
 }  // namespace hipgpt
