@@ -20,8 +20,9 @@ int check_launch(const char *what);
 // have let their dependents go.  Such a kernel must execute dependency_wait() before its first access to global
 // memory; the wait returns when the kernel before it has completed and its writes are visible.
 // HIPGPT_NO_OVERLAPPED_LAUNCH=1 launches the plain way.
+// `cluster` > 1: that many consecutive blocks form a cluster.
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_overlapped(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args)
+inline cudaError_t launch_overlapped_clusters(void (*kern)(KArgs...), int cluster, dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args)
 {
     static const bool plain = [] { const char *e = getenv("HIPGPT_NO_OVERLAPPED_LAUNCH"); return e && *e && *e != '0'; }();
     cudaLaunchConfig_t cfg = {};
@@ -29,12 +30,26 @@ inline cudaError_t launch_overlapped(void (*kern)(KArgs...), dim3 grid, dim3 blo
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    unsigned n = 0;
+    if (!plain) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = (unsigned)cluster;
+        attr[n].val.clusterDim.y = 1;
+        attr[n++].val.clusterDim.z = 1;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = plain ? 0 : 1;
+    cfg.numAttrs = n;
     return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_overlapped(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args)
+{
+    return launch_overlapped_clusters(kern, 1, grid, block, smem, st, args...);
 }
 
 #ifdef __CUDACC__

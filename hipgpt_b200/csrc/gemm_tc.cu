@@ -228,6 +228,17 @@ __device__ __noinline__ void gemm_wait_slow(uint64_t *bar, uint32_t parity, int 
     }
 }
 
+// KS > 1: the slices of a tile are shared by the KS blocks of a cluster (each one tile, no second one), for products with too few
+// tiles for the SMs: a block fetches 64 KB per slice at what L2 gives one SM, about 80 GB/s, so 32 slices on 44 SMs took 25 us.
+// The blocks' partial sums meet in shared memory: the tile's columns are dealt out in pieces of 32, every block stores what it
+// has of the others' pieces into their (now idle) operand stages and adds up its own, in rank order.
+constexpr int kMostSplit = 4;
+__device__ __forceinline__ void cluster_sync()
+{
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
+template <int KS>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_tc_kernel(const uint8_t *__restrict__ aimg, const uint8_t *__restrict__ bimg, const float *__restrict__ row_inv, const float *__restrict__ b_amax,
                const float *__restrict__ bias, float *__restrict__ C, int M, int K, int KT, int NT, int ntiles)
@@ -258,6 +269,9 @@ gemm_tc_kernel(const uint8_t *__restrict__ aimg, const uint8_t *__restrict__ bim
     // The block takes output tiles blockIdx.x, + gridDim.x, ... (column tile fastest: blocks that run side by side share
     // the rows of A).  Stages are counted through all tiles (g), accumulators alternate between two halves of TMEM, so
     // the copies of the next tile and its products run while the four epilogue warps drain the tile before it.
+    int rank = 0;
+    if constexpr (KS > 1) asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    const int kt0 = rank * KT / KS, kt1 = (rank + 1) * KT / KS, first = (int)blockIdx.x / KS, stride = (int)gridDim.x / KS;
 
     if (warp == 4) {
         // ---- producer: whole stages by bulk copies ----
@@ -268,9 +282,9 @@ gemm_tc_kernel(const uint8_t *__restrict__ aimg, const uint8_t *__restrict__ bim
         tc_fence_before();
         __syncthreads();                              // TMEM allocated
         int g = 0;
-        for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+        for (int t = first; t < ntiles; t += stride) {
             const int nt = t % NT, mt = t / NT;
-            for (int kt = 0; kt < KT; ++kt, ++g) {
+            for (int kt = kt0; kt < kt1; ++kt, ++g) {
                 const int s = g % kStages;
                 if (g >= kStages) wait(&empty[s], (uint32_t)((g / kStages - 1) & 1), 2);     // the products that read the stage have completed
                 if (lane == 0) {
@@ -285,6 +299,7 @@ gemm_tc_kernel(const uint8_t *__restrict__ aimg, const uint8_t *__restrict__ bim
             }
         }
         __syncwarp();
+        if constexpr (KS > 1) { cluster_sync(); cluster_sync(); }
         tc_fence_before();
         __syncthreads();                              // the last output has been read from TMEM
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base_slot), "r"(kTmemCols) : "memory");
@@ -299,11 +314,11 @@ gemm_tc_kernel(const uint8_t *__restrict__ aimg, const uint8_t *__restrict__ bim
         constexpr uint32_t id_wide = idesc_f16(kTM, 2 * kTN) | (1u << 16);       // A_hi x [B_hi | B_lo], B N-major
         constexpr uint32_t id_half = idesc_f16(kTM, kTN) | (1u << 16);           // A_lo x B_hi
         int g = 0, i = 0;
-        for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++i) {
+        for (int t = first; t < ntiles; t += stride, ++i) {
             const uint32_t acc = tmem + (uint32_t)((i & 1) * 2 * kTN);
             if (i >= 2) wait(&acc_empty[i & 1], (uint32_t)((i / 2 - 1) & 1), 4);             // the epilogue has read this half's previous tile
             tc_fence_after();
-            for (int kt = 0; kt < KT; ++kt, ++g) {
+            for (int kt = kt0; kt < kt1; ++kt, ++g) {
                 const int s = g % kStages;
                 wait(&full[s], (uint32_t)((g / kStages) & 1), 1);
                 tc_fence_after();
@@ -313,7 +328,7 @@ gemm_tc_kernel(const uint8_t *__restrict__ aimg, const uint8_t *__restrict__ bim
                 const uint64_t db = make_desc(smem_u32(b_s + s * kBStage), kGroupStride, 128, 0);
 #pragma unroll
                 for (int k = 0; k < kTK / 16; ++k)    // 16 deep = 32 bytes of an A row = two groups of B
-                    if (elect_one()) mma_h_ss(acc, da_hi + (uint64_t)(2 * k), db + (uint64_t)(k * 2 * (kGroupStride >> 4)), id_wide, (kt | k) ? 1u : 0u);
+                    if (elect_one()) mma_h_ss(acc, da_hi + (uint64_t)(2 * k), db + (uint64_t)(k * 2 * (kGroupStride >> 4)), id_wide, (kt > kt0 || k) ? 1u : 0u);
 #pragma unroll
                 for (int k = 0; k < kTK / 16; ++k)
                     if (elect_one()) mma_h_ss(acc + kTN, da_lo + (uint64_t)(2 * k), db + (uint64_t)(k * 2 * (kGroupStride >> 4)), id_half, 1u);
@@ -322,6 +337,7 @@ gemm_tc_kernel(const uint8_t *__restrict__ aimg, const uint8_t *__restrict__ bim
             if (elect_one()) tc_commit(&acc_full[i & 1]);
         }
         __syncwarp();
+        if constexpr (KS > 1) { cluster_sync(); cluster_sync(); }
         tc_fence_before();
         __syncthreads();
         return;
@@ -334,7 +350,7 @@ gemm_tc_kernel(const uint8_t *__restrict__ aimg, const uint8_t *__restrict__ bim
     const float b_inv = pow2_inverse(pow2_scale(__ldg(b_amax)));
     const bool vec = (K & 3) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0;
     int i = 0;
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++i) {
+    for (int t = first; t < ntiles; t += stride, ++i) {
         const int nt = t % NT, mt = t / NT;
         const int r = warp * 32 + lane, m = mt * kTM + r;
         const uint32_t lane_base = tmem_base_slot + ((uint32_t)(warp * 32) << 16) + (uint32_t)((i & 1) * 2 * kTN);
@@ -347,12 +363,54 @@ gemm_tc_kernel(const uint8_t *__restrict__ aimg, const uint8_t *__restrict__ bim
         // r * 128 + ((c ^ (r & 7)) * 16)) so that a store instruction writes four rows of 128 contiguous bytes instead
         // of 32 rows of 16
         uint8_t *tb = reinterpret_cast<uint8_t *>(epi[warp]);
+        // (KS > 1) piece c of the columns belongs to block c * KS / 4; what block q has of it lies in the owner's stages, q's place
+        // among the others first: [place][piece of the owner's (at most 2)][column / 4][row] of 16 bytes
+        auto parked = [&](int q, int owner, int c) {
+            const int place = q < owner ? q : q - 1, lc = c - (owner * 4 + KS - 1) / KS;
+            return (uint32_t)((place * 2 + lc) * (8 * kTM * 16) + r * 16);
+        };
+        if constexpr (KS > 1) {
+            cluster_sync();                           // every block of the cluster is done with its operand stages
+#pragma unroll 1
+            for (int c = 0; c < 4; ++c) {
+                const int owner = c * KS / 4;
+                if (owner == rank) continue;
+                float a[32], b[32];
+                tmem_ld32(lane_base + 32 * c, a);
+                tmem_ld32(lane_base + kTN + 32 * c, b);
+                tmem_wait_ld();
+                uint32_t dst;
+                asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(smem_u32(base) + parked(rank, owner, c)), "r"(owner));
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(dst + j * (kTM * 16)), "f"(a[4 * j] + b[4 * j]), "f"(a[4 * j + 1] + b[4 * j + 1]),
+                                 "f"(a[4 * j + 2] + b[4 * j + 2]), "f"(a[4 * j + 3] + b[4 * j + 3]) : "memory");
+            }
+            cluster_sync();
+        }
 #pragma unroll 1
         for (int c0 = 0; c0 < kTN; c0 += 32) {
+            if (KS > 1 && (c0 / 32) * KS / 4 != rank) continue;
             float a[32], b[32];
             tmem_ld32(lane_base + c0, a);             // A_hi B_hi
             tmem_ld32(lane_base + kTN + c0, b);       // the correction terms
             tmem_wait_ld();
+            if constexpr (KS > 1) {
+#pragma unroll
+                for (int x = 0; x < 32; ++x) { b[x] += a[x]; a[x] = 0.0f; }                  // b: this block's share
+#pragma unroll
+                for (int q = 0; q < KS; ++q) {
+                    const uint8_t *src = base + (q == rank ? 0 : parked(q, rank, c0 / 32));
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const float4 y = q == rank ? make_float4(b[4 * j], b[4 * j + 1], b[4 * j + 2], b[4 * j + 3])
+                                                   : *reinterpret_cast<const float4 *>(src + j * (kTM * 16));
+                        a[4 * j] += y.x; a[4 * j + 1] += y.y; a[4 * j + 2] += y.z; a[4 * j + 3] += y.w;
+                    }
+                }
+#pragma unroll
+                for (int x = 0; x < 32; ++x) b[x] = 0.0f;
+            }
             if (c_base + c0 >= K) continue;           // warp-uniform: a tile past the last column
 #pragma unroll
             for (int j4 = 0; j4 < 8; ++j4) {
@@ -446,7 +504,9 @@ int set_gemm_attr()
 {
     static bool attr_set = false;
     if (!attr_set) {
-        const cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem);
+        cudaError_t e = cudaSuccess;
+        for (auto kern : {gemm_tc_kernel<1>, gemm_tc_kernel<2>, gemm_tc_kernel<3>, gemm_tc_kernel<4>})
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem);
         if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
         attr_set = true;
     }
@@ -486,9 +546,13 @@ int pack_a_and_multiply(const float *A, const uint8_t *bimg, const float *b_amax
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
     const long long ntiles = (long long)MT * NT;
     if (ntiles > 2147483647LL) return fail(HIPGPT_ERR_BAD_ARG, "%lld output tiles are too many", ntiles);
-    const unsigned grid = (unsigned)(ntiles < sms ? ntiles : sms);           // one block per SM, each takes tiles in turn
-    e = launch_overlapped(gemm_tc_kernel, dim3(grid), dim3(kGemmThreads), kGemmSmem, st, (const uint8_t *)aimg, bimg,
-                          (const float *)row_inv, b_amax, bias, C, M, K, KT, NT, (int)ntiles);
+    // too few tiles: the slices of a tile on up to four SMs, two slices each at least (below that the exchange costs what it saves)
+    int ks = 1;
+    while (ks < kMostSplit && ntiles * (ks + 1) <= sms && KT >= 2 * (ks + 1)) ++ks;
+    const unsigned grid = ks > 1 ? (unsigned)(ntiles * ks) : (unsigned)(ntiles < sms ? ntiles : sms);      // ks = 1: one block per SM, each takes tiles in turn
+    const auto kern = ks == 1 ? gemm_tc_kernel<1> : ks == 2 ? gemm_tc_kernel<2> : ks == 3 ? gemm_tc_kernel<3> : gemm_tc_kernel<4>;
+    e = launch_overlapped_clusters(kern, ks, dim3(grid), dim3(kGemmThreads), kGemmSmem, st, (const uint8_t *)aimg, bimg,
+                                   (const float *)row_inv, b_amax, bias, C, M, K, KT, NT, (int)ntiles);
     if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "gemm_tc_kernel launch: %s", cudaGetErrorString(e));
     return check_launch("gemm_tc_kernel");
 }
