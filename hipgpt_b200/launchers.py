@@ -21,8 +21,14 @@ def _ptr(t):
     return t.data_ptr()
 
 
+# the current stream's handle without the Stream object around it (3.2 us of host time per call)
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream():
-    return torch.cuda.current_stream().cuda_stream
+    if _raw_stream is None:
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(torch.cuda.current_device())
 
 
 def launch_multihead_attention(d_qkv, d_output, d_attn_probs, B: int, S: int, E: int, H: int, *, causal: bool = False):
