@@ -227,8 +227,10 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
 
     const int tid = threadIdx.x, lane = tid & 31;
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
-    const int bh = blockIdx.x / nblk;
-    const int blk = CAUSAL ? nblk - 1 - (int)(blockIdx.x % nblk) : (int)(blockIdx.x % nblk);      // the longest first
+    // with the mask the longest blocks of all heads come first; else a head's blocks run side by side
+    const int nbh = (int)gridDim.x / nblk;
+    const int bh = CAUSAL ? (int)blockIdx.x % nbh : (int)blockIdx.x / nblk;
+    const int blk = CAUSAL ? nblk - 1 - (int)blockIdx.x / nbh : (int)blockIdx.x % nblk;
     const int b = bh / H, h = bh % H, q0 = blk * kLanes;
     const int kend = CAUSAL ? min(S, q0 + kLanes) : S;
     const int nk = (kend + kTile - 1) / kTile;       // key tiles of a sweep
@@ -514,7 +516,8 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
 
     const int tid = threadIdx.x, lane = tid & 31;
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
-    const int bh = blockIdx.x / nblk, blk = blockIdx.x % nblk;           // with the mask the first key block is the longest
+    const int nbh = (int)gridDim.x / nblk;           // with the mask the first key block of a head is the longest
+    const int bh = CAUSAL ? (int)blockIdx.x % nbh : (int)blockIdx.x / nblk, blk = CAUSAL ? (int)blockIdx.x / nbh : (int)blockIdx.x % nblk;
     const int b = bh / H, h = bh % H, k0 = blk * kLanes;
     const int t0 = CAUSAL ? k0 / kTile : 0;          // the first query that sees key j is query j
     const int total = (S + kTile - 1) / kTile - t0;
