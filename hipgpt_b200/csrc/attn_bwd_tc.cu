@@ -20,8 +20,8 @@
 //                     dV += P^T dO, dK += ds^T Q, queries ascending.
 // Nothing is added atomically: each output has one owner and a fixed order, results are the same bits on every run.
 //
-// Eight worker warps (two per TMEM lane quarter, each 32 of the tile's 64 columns) and one issuing warp, which also fetches.  Two
-// score buffers in TMEM: the products of tile i + 1 run while the workers are at tile i.  Every wait is bounded: on expiry the
+// Eight worker warps (two per TMEM lane quarter, each 32 of the tile's 64 columns) and two issuing warps, which also fetch and
+// issue side by side.  Two score buffers in TMEM: the products of tile i + 1 run while the workers are at tile i.  Every wait is bounded: on expiry the
 // block raises a flag that cuts later waits short, records a status code, skips its stores, frees its TMEM and returns.
 #include "stream_workspace.hpp"
 #include "tc_primitives.cuh"
@@ -34,7 +34,7 @@ namespace {
 constexpr int kLanes = 128;            // rows (or keys) per block = TMEM lanes
 constexpr int kTile = 64;              // columns per tile
 constexpr int kWorkerWarps = 8;
-constexpr int kThreads = kWorkerWarps * 32 + 32;
+constexpr int kThreads = kWorkerWarps * 32 + 64;
 constexpr uint32_t kTmemCols = 512;
 
 __device__ int g_bwd_status = 0;
@@ -128,21 +128,21 @@ __device__ __forceinline__ void issue_scores(uint32_t d_tmem, uint32_t a_smem, u
         }
 }
 
-// acc[tmem] (128 x D) = A B over the 64 rows of B's image, read N-major; A: three pieces in TMEM, the piece `p` of the columns
+// acc[tmem] (128 x D) = A B over rows [16 KS0, 16 KS1) of B's image, read N-major; A: three pieces in TMEM, the piece `p` of the columns
 // [32 hf, 32 hf + 32) packed in 16 columns at a_col(p, hf).  WIDE: acc is 2 D columns, the second half collects the products with
 // B's mid and lo pieces (wider instructions, fewer of them).  The small products come first: the tensor core truncates where
 // it adds to its accumulator, so the accumulator should be small while they are added, and it starts anew for every tile (the
 // workers add the tiles up in registers).  One accumulator over all tiles was 10 times farther from float64 at S = 777.
-template <int D, bool WIDE, typename ACol>
+template <int D, bool WIDE, int KS0, int KS1, typename ACol>
 __device__ __forceinline__ void issue_accumulate(uint32_t acc, ACol a_col, uint32_t b_smem)
 {
     const uint64_t b = make_desc(b_smem, Img<D>::kBlock, 128, 0);
     constexpr uint32_t id1 = idesc_bf16(D, 1), id2 = idesc_bf16(2 * D, 1);
     auto product = [&](int pa, int pb, int d, uint32_t id, bool fresh) {
 #pragma unroll
-        for (int ks = 0; ks < kTile / 16; ++ks) {
+        for (int ks = KS0; ks < KS1; ++ks) {
             const uint64_t bk = b + (uint64_t)(ks * 2 * (Img<D>::kBlock >> 4) + pb * (Img<D>::kPiece >> 4));
-            if (elect_one()) mma_h_ts(acc + d, a_col(pa, ks >> 1) + (ks & 1) * 8, bk, id, (fresh && ks == 0) ? 0u : 1u);
+            if (elect_one()) mma_h_ts(acc + d, a_col(pa, ks >> 1) + (ks & 1) * 8, bk, id, (fresh && ks == KS0) ? 0u : 1u);
         }
     };
     if (WIDE) {
@@ -208,7 +208,7 @@ struct RowsCfg {
     static constexpr int kResident = 2 * 2 * Img<D>::kTileBytes;         // Q and dO, 128 rows each
     static constexpr int kStage = STORED ? kWorkerWarps * 4096 : 0;      // per warp 32 rows x 32 probabilities on their way to their rows
     static constexpr size_t kSmem = (size_t)kResident + (kKStages + kVStages) * Img<D>::kTileBytes + kStage;
-    static constexpr uint32_t kColAcc = 4 * kTile;                       // after two buffers of S and dP
+    static constexpr uint32_t kColAcc = 4 * kTile;                       // after two buffers of S and dP: two accumulators of 2 D columns
 };
 
 template <int D, bool CAUSAL, bool STORED>
@@ -241,7 +241,7 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         mbar_init(&res_full, 1);
         for (int i = 0; i < C::kKStages; ++i) mbar_init(&k_full[i], 1);
         for (int i = 0; i < C::kVStages; ++i) mbar_init(&v_full[i], 1);
-        for (int i = 0; i < 2; ++i) { mbar_init(&sd_full[i], 1); mbar_init(&ready[i], kWorkerWarps); mbar_init(&acc_done[i], 1); }
+        for (int i = 0; i < 2; ++i) { mbar_init(&sd_full[i], STORED ? 1 : 2); mbar_init(&ready[i], kWorkerWarps); mbar_init(&acc_done[i], 2); }      // (commits: one per issuing warp)
     }
     if (warp == kWorkerWarps) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)), "r"(kTmemCols) : "memory");
@@ -258,7 +258,9 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         bwd_wait_slow(bar, parity, site, &abort_flag);
     };
 
-    if (warp == kWorkerWarps) {
+    if (warp >= kWorkerWarps) {
+        // the first issuing warp has K: S = Q K^T and half of the accumulation; the second V: dP = dO V^T and the other half
+        const bool first = warp == kWorkerWarps;
         const uint8_t *q_img = img + (size_t)bh * Spad * (Img<D>::kBlock / 8) + (size_t)q0 * (Img<D>::kBlock / 8);
         const uint8_t *k_img = img + img_bytes + (size_t)bh * Spad * (Img<D>::kBlock / 8);
         const uint8_t *v_img = k_img + img_bytes, *g_img = q_img + 3 * img_bytes;
@@ -282,24 +284,29 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
             }
             __syncwarp();
         };
-        if (lane == 0) {
-            mbar_arrive_expect_tx(&res_full, 4 * TB);
-            bulk_load(q_s, q_img, 2 * TB, &res_full);
-            bulk_load(g_s, g_img, 2 * TB, &res_full);
+        if (first) {
+            if (lane == 0) {
+                mbar_arrive_expect_tx(&res_full, 4 * TB);
+                bulk_load(q_s, q_img, 2 * TB, &res_full);
+                bulk_load(g_s, g_img, 2 * TB, &res_full);
+            }
+            __syncwarp();
+            for (int i = 0; i < C::kKStages; ++i) fetch_k(k_first + i);
+        } else {
+            for (int i = 0; i < C::kVStages; ++i) fetch_v(i);
         }
-        __syncwarp();
-        for (int i = 0; i < C::kVStages; ++i) fetch_v(i);
-        for (int i = 0; i < C::kKStages; ++i) fetch_k(k_first + i);
         auto issue_sd = [&](int i) {
             const uint32_t d = tmem + (uint32_t)((i & 1) * 2 * kTile);
-            if (!STORED) {
+            if (first) {
+                if (STORED) return;
                 wait(&k_full[k_slot(i)], k_phase(i), 2);
                 tc_fence_after();
                 issue_scores<D>(d, smem_u32(q_s), smem_u32(k_s + k_slot(i) * TB));
+            } else {
+                wait(&v_full[i % C::kVStages], (uint32_t)((i / C::kVStages) & 1), 3);
+                tc_fence_after();
+                issue_scores<D>(d + kTile, smem_u32(g_s), smem_u32(v_s + (i % C::kVStages) * TB));
             }
-            wait(&v_full[i % C::kVStages], (uint32_t)((i / C::kVStages) & 1), 3);
-            tc_fence_after();
-            issue_scores<D>(d + kTile, smem_u32(g_s), smem_u32(v_s + (i % C::kVStages) * TB));
             if (elect_one()) tc_commit(&sd_full[i & 1]);
         };
         wait(&res_full, 0, 1);
@@ -309,26 +316,28 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
             // the buffer of scores i + 1 is free once the workers (first sweep) or the accumulation (second) have read it
             if (i - 1 >= nk) {
                 wait(&acc_done[(i - 1) & 1], (uint32_t)(((i - 1 - nk) >> 1) & 1), 6);
-                fetch_k(i - 1 + C::kKStages);
+                if (first) fetch_k(i - 1 + C::kKStages);
             }
             if (i + 1 < total) issue_sd(i + 1);
             wait(&ready[i & 1], (uint32_t)((i >> 1) & 1), 5);
             tc_fence_after();
-            fetch_v(i + C::kVStages);                // the scores of tile i have been read, so the products that read V have completed
+            if (!first) fetch_v(i + C::kVStages);    // the scores of tile i have been read, so the products that read V have completed
             if (i < nk) {
-                if (!STORED) fetch_k(i + C::kKStages);
+                if (!STORED && first) fetch_k(i + C::kKStages);
             } else {
-                if (STORED) { wait(&k_full[k_slot(i)], k_phase(i), 2); tc_fence_after(); }
-                const uint32_t s0 = tmem + (uint32_t)((i & 1) * 2 * kTile);
+                wait(&k_full[k_slot(i)], k_phase(i), 2);
+                tc_fence_after();
+                const uint32_t s0 = tmem + (uint32_t)((i & 1) * 2 * kTile), kt = smem_u32(k_s + k_slot(i) * TB);
                 auto a_col = [&](int p, int hf) { return p == 2 ? s0 + kTile + 32 * hf : s0 + 32 * hf + 16 * p; };
-                issue_accumulate<D, true>(tmem + C::kColAcc, a_col, smem_u32(k_s + k_slot(i) * TB));
+                if (first) issue_accumulate<D, true, 0, 2>(tmem + C::kColAcc, a_col, kt);
+                else issue_accumulate<D, true, 2, 4>(tmem + C::kColAcc + 2 * D, a_col, kt);
                 if (elect_one()) tc_commit(&acc_done[i & 1]);
             }
         }
         __syncwarp();
         tc_fence_before();
         __syncthreads();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
+        if (first) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
         return;
     }
 
@@ -350,7 +359,11 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
     float4 pf[8];
     auto fetch_p = [&](int i) {
         const int j0 = (i % nk) * kTile + hf * 32;
-        if (vec) {
+        if (vec && q0 + wq * 32 + 32 <= S && j0 + 32 <= S) {
+            const float *src = p_rows + (size_t)(lane >> 3) * S + j0 + (lane & 7) * 4;
+#pragma unroll
+            for (int u = 0; u < 8; ++u, src += 4 * S) pf[u] = __ldg(reinterpret_cast<const float4 *>(src));
+        } else if (vec) {
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
                 const int r = u * 4 + (lane >> 3), j = j0 + (lane & 7) * 4;
@@ -393,6 +406,7 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         wait(&acc_done[i & 1], (uint32_t)(((i - nk) >> 1) & 1), 6);
         tc_fence_after();
         add_tile<D, true>(lane_base + C::kColAcc, hf, o);
+        add_tile<D, true>(lane_base + C::kColAcc + 2 * D, hf, o);
     };
     if (STORED) fetch_p(0);
     for (int i = 0; i < total; ++i) {
@@ -526,7 +540,7 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         abort_flag = 0;
         mbar_init(&res_full, 1);
         for (int i = 0; i < C::kStages; ++i) mbar_init(&full[i], 1);
-        for (int i = 0; i < 2; ++i) { mbar_init(&sd_full[i], 1); mbar_init(&ready[i], kWorkerWarps); mbar_init(&acc_done[i], 1); }
+        for (int i = 0; i < 2; ++i) { mbar_init(&sd_full[i], STORED ? 1 : 2); mbar_init(&ready[i], kWorkerWarps); mbar_init(&acc_done[i], 2); }      // (commits: one per issuing warp)
     }
     if (warp == kWorkerWarps) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)), "r"(kTmemCols) : "memory");
@@ -543,7 +557,9 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         bwd_wait_slow(bar, parity, site, &abort_flag);
     };
 
-    if (warp == kWorkerWarps) {
+    if (warp >= kWorkerWarps) {
+        // the first issuing warp: S^T = K Q^T and dV; the second: dP^T = V dO^T and dK
+        const bool first = warp == kWorkerWarps;
         const uint8_t *q_img = img + (size_t)bh * Spad * (Img<D>::kBlock / 8);
         const uint8_t *k_img = q_img + img_bytes + (size_t)k0 * (Img<D>::kBlock / 8), *v_img = k_img + img_bytes, *g_img = q_img + 3 * img_bytes;
         auto fetch = [&](int i) {
@@ -556,19 +572,22 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
             }
             __syncwarp();
         };
-        if (lane == 0) {
-            mbar_arrive_expect_tx(&res_full, 4 * TB);
-            bulk_load(k_s, k_img, 2 * TB, &res_full);
-            bulk_load(v_s, v_img, 2 * TB, &res_full);
+        if (first) {
+            if (lane == 0) {
+                mbar_arrive_expect_tx(&res_full, 4 * TB);
+                bulk_load(k_s, k_img, 2 * TB, &res_full);
+                bulk_load(v_s, v_img, 2 * TB, &res_full);
+            }
+            __syncwarp();
+            for (int i = 0; i < C::kStages; ++i) fetch(i);
         }
-        __syncwarp();
-        for (int i = 0; i < C::kStages; ++i) fetch(i);
         auto issue_sd = [&](int i) {
+            if (STORED && first) return;
             const uint32_t d = tmem + (uint32_t)(i & 1) * C::kBuf, t = smem_u32(t_s + (i % C::kStages) * 2 * TB);
             wait(&full[i % C::kStages], (uint32_t)((i / C::kStages) & 1), 12);
             tc_fence_after();
-            if (!STORED) issue_scores<D>(d, smem_u32(k_s), t);
-            issue_scores<D>(d + kTile, smem_u32(v_s), t + TB);
+            if (first) issue_scores<D>(d, smem_u32(k_s), t);
+            else issue_scores<D>(d + kTile, smem_u32(v_s), t + TB);
             if (elect_one()) tc_commit(&sd_full[i & 1]);
         };
         wait(&res_full, 0, 11);
@@ -577,22 +596,23 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         for (int i = 0; i < total; ++i) {
             if (i >= 1) {                            // tile i - 1 has been accumulated: its stage and its buffer are free
                 wait(&acc_done[(i - 1) & 1], (uint32_t)(((i - 1) >> 1) & 1), 16);
-                fetch(i - 1 + C::kStages);
+                if (first) fetch(i - 1 + C::kStages);
             }
             if (i + 1 < total) issue_sd(i + 1);
+            if (STORED && first) wait(&full[i % C::kStages], (uint32_t)((i / C::kStages) & 1), 12);
             wait(&ready[i & 1], (uint32_t)((i >> 1) & 1), 15);
             tc_fence_after();
             const uint32_t s0 = tmem + (uint32_t)(i & 1) * C::kBuf, t = smem_u32(t_s + (i % C::kStages) * 2 * TB);
             auto p_col = [&](int p, int hf) { return p == 2 ? s0 + kTile + 32 * hf : s0 + 32 * hf + 16 * p; };
             auto ds_col = [&](int p, int hf) { return p == 0 ? s0 + kTile + 32 * hf + 16 : s0 + 2 * kTile + 32 * hf + 16 * (p - 1); };
-            issue_accumulate<D, C::kWide>(tmem + C::kColV, p_col, t + TB);
-            issue_accumulate<D, C::kWide>(tmem + C::kColK, ds_col, t);
+            if (first) issue_accumulate<D, C::kWide, 0, 4>(tmem + C::kColV, p_col, t + TB);
+            else issue_accumulate<D, C::kWide, 0, 4>(tmem + C::kColK, ds_col, t);
             if (elect_one()) tc_commit(&acc_done[i & 1]);
         }
         __syncwarp();
         tc_fence_before();
         __syncthreads();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
+        if (first) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
         return;
     }
 
@@ -610,9 +630,16 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
     float pn[32];                                    // stored probabilities of the tile ahead: a query's are contiguous over the keys (lanes)
     auto fetch_p = [&](int i) {
         const int qb = (t0 + i) * kTile + hf * 32;
-        const float *src = P + ((size_t)bh * S + qb) * S + key;
+        // a lane past S reads its neighbour's key (its results go nowhere): no load depends on the lane, and in a full tile none
+        // on the query either (loads behind conditions took 3500 cycles per tile to issue)
+        const float *src = P + ((size_t)bh * S + qb) * S + min(key, S - 1);
+        if (qb + 32 <= S) {
 #pragma unroll
-        for (int x = 0; x < 32; ++x) pn[x] = (qb + x < S && key < S) ? __ldg(src + (size_t)x * S) : 0.0f;
+            for (int x = 0; x < 32; ++x, src += S) pn[x] = __ldg(src);
+        } else {
+#pragma unroll
+            for (int x = 0; x < 32; ++x, src += S) pn[x] = qb + x < S ? __ldg(src) : 0.0f;
+        }
     };
     float ok[D / 2], ov[D / 2];
 #pragma unroll

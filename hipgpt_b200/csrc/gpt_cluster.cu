@@ -237,7 +237,9 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
     // `src` in shared memory, normalised first where the job says so; kJobO takes this warp's own segment.  Leaves the partial sums
     // in part + flip * part_stride and ends with a barrier of the block.  Lanes: up to 16 columns: (column, row of a pair); more:
     // columns lane, lane + 32, all rows.  Returns the part's bias for the columns that this thread finishes.
-    auto product = [&](auto jn, const float *src) {
+    // `arrival` waits for the activations.  Before it the weights of this lane go to registers (where there are at most 64): they
+    // have been in the ring for long, and reading them takes the shared memory's return path about as long as a hop takes.
+    auto product = [&](auto jn, const float *src, auto arrival) {
         constexpr int J = decltype(jn)::value;
         constexpr ClusterJob jb = cluster_job_of(J, E, 64 * 64);          // (the output projection's cut depends on V in its parts only)
         constexpr int pw = jb.width, klen = jb.klen, klp = jb.klp, sh = jb.seg_shift, nch = jb.chunks();
@@ -251,11 +253,25 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
         const float *as = aw;
         constexpr bool kOwn = jb.ln || J == kJobO || (klen & 3) != 0;     // the activations are (copied) in this warp's own segment
         constexpr int astride = kOwn ? C::seg : stride;
+        constexpr int NC = pw <= 16 ? 1 : (pw + 31) / 32;                // columns per lane
+        constexpr bool kEarly = J != kJobQkv && J != kJobVoc && NC * klp <= 64;
+        const int wc0 = pw <= 16 ? (pw < 16 ? min(lane & 15, pw - 1) : lane & 15) : (pw < 32 ? min(lane, pw - 1) : lane);
+        const float4 *wp = w4 + wc0, *wq = w4 + (pw < 64 ? min(lane + 32, pw - 1) : lane + 32);
+        float4 held[kEarly ? NC * klp / 4 : 1];
+        if constexpr (kEarly) {
+            wait(&full[slot], par);
+#pragma unroll
+            for (int k = 0; k < klp / 4; ++k) {
+                held[NC * k] = wp[k * pw];
+                if constexpr (NC > 1) held[NC * k + 1] = wq[k * pw];
+            }
+        }
+        arrival();
         if constexpr (jb.ln != 0) {
             if (warp < rows) row_stats(src + warp * stride, &stats[warp]);
             __syncthreads();
         }
-        wait(&full[slot], par);
+        if constexpr (!kEarly) wait(&full[slot], par);
         if constexpr (jb.ln != 0) {
             const float *gm = chunk + jb.weight_floats() + in_chunk * klp, *bt = gm + (klp << sh);
 #pragma unroll
@@ -281,13 +297,12 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
         if constexpr (pw <= 16) {
             constexpr int RH = (R + 1) / 2;          // rows of a lane: r0, r0 + 2
             const int c = lane & 15, r0 = R > 1 ? lane >> 4 : 0;
-            const float4 *wp = w4 + (pw < 16 ? min(c, pw - 1) : c);
             float acc[RH];
 #pragma unroll
             for (int r = 0; r < RH; ++r) acc[r] = 0.0f;
-#pragma unroll 8
+#pragma unroll (kEarly ? klp / 4 : 8)
             for (int k = 0; k < klp / 4; ++k) {
-                const float4 w = wp[k * pw];
+                const float4 w = kEarly ? held[k] : wp[k * pw];
 #pragma unroll
                 for (int r = 0; r < RH; ++r) {
                     const float4 x = *reinterpret_cast<const float4 *>(as + (r0 + 2 * r) * astride + 4 * k);
@@ -301,18 +316,16 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
 #pragma unroll
                 for (int r = 0; r < RH; ++r) dst[(r0 + 2 * r) * 16 * pw + c] = acc[r];
         } else {
-            constexpr int NC = (pw + 31) / 32;       // 1 or 2 columns per lane
             float acc[NC][R];
 #pragma unroll
             for (int n = 0; n < NC; ++n)
 #pragma unroll
                 for (int r = 0; r < R; ++r) acc[n][r] = 0.0f;
-            const float4 *wp = w4 + (pw < 32 ? min(lane, pw - 1) : lane), *wq = w4 + (pw < 64 ? min(lane + 32, pw - 1) : lane + 32);
-#pragma unroll 4
+#pragma unroll (kEarly ? klp / 4 : 4)
             for (int k = 0; k < klp / 4; ++k) {
                 float4 w[NC];
-                w[0] = wp[k * pw];
-                if constexpr (NC > 1) w[1] = wq[k * pw];
+                w[0] = kEarly ? held[NC * k] : wp[k * pw];
+                if constexpr (NC > 1) w[1] = kEarly ? held[NC * k + 1] : wq[k * pw];
 #pragma unroll
                 for (int r = 0; r < R; ++r) {
                     const float4 x = *reinterpret_cast<const float4 *>(as + r * astride + 4 * k);
@@ -414,7 +427,7 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
         for (int u = u0; u < units; u += 4 * kClusterBlocks) {
             const Unit un = u == u0 ? first_unit : make_unit(u);
             const int k0 = un.split * per, k1 = min(p + 1, k0 + per);
-            if (u != u0) ask(un, layer, p, 0);       // the first unit's rows were asked for ahead
+            if (u != u0) ask(un, layer, p, 0);       // the first unit's rows were asked for ahead (the next one's too: spills, 105 us per step)
             const float *now = qkv + un.now;         // this position's query, key and value
             float4 q4 = make_float4(0.f, 0.f, 0.f, 0.f);
             if (act) {
@@ -563,21 +576,20 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
 #pragma unroll 1
         for (int l = 0; l < a.L; ++l) {
             ask(first_unit, l, p, 0);
-            if (l > 0) receive(kXb);
 #pragma unroll 1
-            for (int pt = 0; pt < cluster_job_of(kJobQkv, E, 0).parts; ++pt) finish(Job<kJobQkv>(), pt, product(Job<kJobQkv>(), xb), l, p);
+            for (int pt = 0; pt < cluster_job_of(kJobQkv, E, 0).parts; ++pt)
+                finish(Job<kJobQkv>(), pt, product(Job<kJobQkv>(), xb, [&] { if (pt == 0 && l > 0) receive(kXb); }), l, p);
             receive(kQkv);
             attend(l, p);
-            receive(kRec);
-            combine();
 #pragma unroll 1
-            for (int pt = 0; pt < cluster_job_of(kJobO, E, 0).parts; ++pt) finish(Job<kJobO>(), pt, product(Job<kJobO>(), nullptr), 0, 0);
-            receive(kXa);
+            for (int pt = 0; pt < cluster_job_of(kJobO, E, 0).parts; ++pt)
+                finish(Job<kJobO>(), pt, product(Job<kJobO>(), nullptr, [&] { if (pt == 0) { receive(kRec); combine(); } }), 0, 0);
 #pragma unroll 1
-            for (int pt = 0; pt < cluster_job_of(kJobF1, E, 0).parts; ++pt) finish(Job<kJobF1>(), pt, product(Job<kJobF1>(), xa), 0, 0);
-            receive(kFf);
+            for (int pt = 0; pt < cluster_job_of(kJobF1, E, 0).parts; ++pt)
+                finish(Job<kJobF1>(), pt, product(Job<kJobF1>(), xa, [&] { if (pt == 0) receive(kXa); }), 0, 0);
 #pragma unroll 1
-            for (int pt = 0; pt < cluster_job_of(kJobF2, E, 0).parts; ++pt) finish(Job<kJobF2>(), pt, product(Job<kJobF2>(), ff), 0, 0);
+            for (int pt = 0; pt < cluster_job_of(kJobF2, E, 0).parts; ++pt)
+                finish(Job<kJobF2>(), pt, product(Job<kJobF2>(), ff, [&] { if (pt == 0) receive(kFf); }), 0, 0);
         }
         receive(kXb);
         const bool head = p >= a.n_prompt - 1, last = step + 1 == a.nsteps;
@@ -589,7 +601,7 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
             constexpr int pw = cluster_job_of(kJobVoc, E, 64 * 64).width;
 #pragma unroll 1
             for (int pt = 0; pt < plan.voc.parts; ++pt) {
-                product(Job<kJobVoc>(), xb);
+                product(Job<kJobVoc>(), xb, [] {});
                 const int n = rank * plan.voc.nc + pt * pw + hc;
                 if (hr < rows && hc < pw && pt * pw + hc < plan.voc.nc && n < V) {
                     const float *pp = part + flip * C::part_stride + hr * 16 * pw + hc;

@@ -11,24 +11,26 @@ import torch
 from . import _capi
 
 
+_FLOAT32 = torch.float32
+
+
 def _ptr(t):
-    if t is None:
-        return None
-    if isinstance(t, int):
+    if t is None or isinstance(t, int):
         return t
-    if not (t.is_cuda and t.dtype == torch.float32 and t.is_contiguous()):
+    if not (t.is_cuda and t.dtype is _FLOAT32 and t.is_contiguous()):
         raise ValueError("expected a contiguous CUDA float32 tensor")
     return t.data_ptr()
 
 
 # the current stream's handle without the Stream object around it (3.2 us of host time per call)
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_current_device = torch.cuda.current_device
 
 
 def _stream():
     if _raw_stream is None:
         return torch.cuda.current_stream().cuda_stream
-    return _raw_stream(torch.cuda.current_device())
+    return _raw_stream(_current_device())
 
 
 def launch_multihead_attention(d_qkv, d_output, d_attn_probs, B: int, S: int, E: int, H: int, *, causal: bool = False):
