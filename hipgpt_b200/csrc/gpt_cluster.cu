@@ -23,10 +23,9 @@
 // Waits on mbarriers are bounded: on expiry the block raises a flag that cuts its later waits short and sets the error word; the
 // steps then run out without waiting.
 //
-// Measured at the default model (E=256 L=8 H=8 V=5000), batch 8: 90 us per step (the replayed graph: 318), batch 1: 75 (256).  A
-// step is 42 products of about 450 ns each: multiply-adds 20 %, layer norms 10 %, adding up and storing 15 %, arrival of the
-// others' columns 25 %, attention 30 %.  Sizes are template parameters because the chain is bound by the instructions of single
-// warps: with sizes read from the plan a step took 143 us.
+// Measured at the default model (E=256 L=8 H=8 V=5000), batch 8: 87 us per step (the replayed graph: 318), batch 1: 73 (256).  A
+// step is 42 products of about 450 ns each, attention two fifths of a layer.  Sizes are template parameters because the chain is
+// bound by the instructions of single warps: with sizes read from the plan a step took 143 us.
 #include "gpt_cluster.cuh"
 #include "tc_primitives.cuh"
 

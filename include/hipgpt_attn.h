@@ -299,7 +299,7 @@ HIPGPT_API int hipgpt_gpt_create_from_run(hipgpt_gpt **out, const char *json_pat
  *     prompt positions, a second one the remaining tokens; the phases of a step follow one another inside the
  *     kernel, separated by a bounded barrier over the grid (one block per SM).  If a wait at that barrier runs
  *     out, hipgpt_gpt_generate returns HIPGPT_ERR_CUDA and the handle stays usable.  Measured no faster than the
- *     graph on B200 (335 against 327 us per step of 8 tokens; the clusters: 90).
+ *     graph on B200 (335 against 327 us per step of 8 tokens; the clusters: 87).
  */
 #define HIPGPT_GPT_MODE_GRAPH 0
 #define HIPGPT_GPT_MODE_PERSISTENT 1
