@@ -75,18 +75,19 @@ __device__ __forceinline__ void merge_part(Part &a, float m2, float l2, const fl
 {
     const float mn = fmaxf(a.m, m2);
     const float a1 = ex2_approx(a.m - mn), a2 = ex2_approx(m2 - mn);
-    a.l = a.l * a1 + l2 * a2;
-    a.o.x = a.o.x * a1 + o2.x * a2;
-    a.o.y = a.o.y * a1 + o2.y * a2;
-    a.o.z = a.o.z * a1 + o2.z * a2;
-    a.o.w = a.o.w * a1 + o2.w * a2;
+    // (the contraction written out: the compiler may choose either product for the multiply-add, and the bits should be the launches')
+    a.l = fmaf(a.l, a1, __fmul_rn(l2, a2));
+    a.o.x = fmaf(a.o.x, a1, __fmul_rn(o2.x, a2));
+    a.o.y = fmaf(a.o.y, a1, __fmul_rn(o2.y, a2));
+    a.o.z = fmaf(a.o.z, a1, __fmul_rn(o2.z, a2));
+    a.o.w = fmaf(a.o.w, a1, __fmul_rn(o2.w, a2));
     a.m = mn;
 }
 
 template <int J>
 struct Job { static constexpr int value = J; };
-template <int E, int R>
-struct Width { static constexpr int kE = E, kR = R; };
+template <int E, int R, int VW>
+struct Width { static constexpr int kE = E, kR = R, kVW = VW; };
 
 // Shared memory of a block, in floats from the start: what has a size known to the compiler first.  Rows of activations are padded
 // by four floats: the rows that a warp reads side by side then lie in different banks.
@@ -97,7 +98,7 @@ struct Lay {
     static constexpr int seg = cluster_job_of(kJobQkv, E, 16).klp + 4;   // of a warp's own segment
     static constexpr int xb = 0, xa = xb + R * es, qkv = xa + R * es, ff = qkv + R * qs, aw = ff + R * fs, part = aw + kWarps * R * seg;
     static constexpr int part_stride = R * 16 * 64;
-    static constexpr int unit = part + 2 * part_stride, amax = unit + 4 * 4 * 32 * 8, fixed = (amax + 32 * R * 2 + 3) & ~3;
+    static constexpr int unit = part + 2 * part_stride, amax = unit + 8 * 4 * 16 * 8, fixed = (amax + 32 * R * 2 + 3) & ~3;
     static constexpr int slot_bytes()
     {
         int most = 0;
@@ -122,7 +123,7 @@ Rest rest_of(int H, int D, int ns, int all_chunks)
     return r;
 }
 
-template <int E, int R>
+template <int E, int R, int VW>
 __global__ void __launch_bounds__(kThreads, 1)
 cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_constant__ ClusterArgs a, const __grid_constant__ Rest lay)
 {
@@ -390,126 +391,147 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
         flip ^= 1;
     };
 
-    // ---- the attention of one position: units of (row, head, split), four warps each, dealt out over the blocks' warp groups.
-    //      A key's head is read by LPK lanes (4 numbers each), as in attn_decode.cu ----
-    constexpr int W4 = 4;
-    const int lpk_log = D <= 32 ? 3 : 4, LPK = 1 << lpk_log, KPW = 32 >> lpk_log;
-    const int slot4 = warp >> 2, w4i = warp & 3, lik = lane & (LPK - 1), kg = lane >> lpk_log;
-    const bool act = lik * 4 < D;
+    // ---- the attention of one position: units of (row, head, split), dealt out over the blocks' warp groups.  attn_decode.cu gives a
+    //      unit four warps; here a warp stands for VW of them, whose arithmetic it interleaves: two where the units of the cluster
+    //      outnumber its groups of four warps (a second round costs more than the doubled work of a warp that is bound by latency).
+    //      A key's head is read by LPK lanes (4 numbers each) ----
+    constexpr int W4 = 4, GW = W4 / VW, GROUPS = kWarps / GW, AHEAD = kAhead / VW;
+    const bool narrow = D <= 32;                     // LPK = 8, else 16: the code exists for both, so that lanes and strides are constants
+    const int group = warp / GW, wg = warp % GW;
     const float qscale = (1.0f / sqrtf((float)D)) * kLog2e;
     const int units = rows * H * ns;
-    float *merge_s = sm + C::unit + slot4 * (W4 * 32 * 8);
+    float *merge_s = sm + C::unit + group * (W4 * 16 * 8);
     struct Unit { int split, now, rec, mem; };       // its split; offsets of its head in qkv, of its record, of its row and head in a layer's cache
     auto make_unit = [&](int u) {
         const int split = u % ns, bh = u / ns, h = bh % H, r = bh / H;
-        return Unit{split, r * C::qs + h * D + lik * 4, u * rstride, (row0 + r) * a.S * E + h * D + lik * 4};
+        return Unit{split, r * C::qs + h * D, u * rstride, (row0 + r) * a.S * E + h * D};
     };
-    const int u0 = rank + kClusterBlocks * slot4;
+    const int u0 = rank + kClusterBlocks * group;
     const Unit first_unit = make_unit(min(u0, units - 1));
     int per = 0;                                     // positions of a split at this step
-    float4 k4[kAhead], v4[kAhead];                   // rows of a unit that earlier steps wrote
-    auto ask = [&](const Unit &un, int layer, int p, int it0) {
-        const int j0 = un.split * per + (it0 * W4 + w4i) * KPW + kg, k1 = act ? min(p, un.split * per + per) : 0;
-        const size_t at = (size_t)layer * a.layer_stride + (size_t)un.mem + (size_t)j0 * E;
+    float4 k4[VW][AHEAD], v4[VW][AHEAD];             // rows of a unit that earlier steps wrote
+    auto ask = [&](auto lpk, const Unit &un, int layer, int p, int it0) {
+        constexpr int LPK = decltype(lpk)::value, KPW = 32 / LPK;
+        const int lik = lane % LPK, kg = lane / LPK;
+        const bool act = lik * 4 < D;
+        const int j0 = un.split * per + (it0 * W4 + wg * VW) * KPW + kg, k1 = act ? min(p, un.split * per + per) : 0;
+        const size_t at = (size_t)layer * a.layer_stride + (size_t)(un.mem + lik * 4) + (size_t)j0 * E;
         const float *kp = a.kc + at, *vp = a.vc + at;
 #pragma unroll
-        for (int it = 0; it < kAhead; ++it) {
-            k4[it] = v4[it] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (j0 + it * W4 * KPW < k1) {
-                k4[it] = __ldcg(reinterpret_cast<const float4 *>(kp + it * W4 * KPW * E));
-                v4[it] = __ldcg(reinterpret_cast<const float4 *>(vp + it * W4 * KPW * E));
+        for (int w = 0; w < VW; ++w)
+#pragma unroll
+            for (int it = 0; it < AHEAD; ++it) {
+                const int j = (it * W4 + w) * KPW;
+                k4[w][it] = v4[w][it] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (j0 + j < k1) {
+                    k4[w][it] = __ldcg(reinterpret_cast<const float4 *>(kp + j * E));
+                    v4[w][it] = __ldcg(reinterpret_cast<const float4 *>(vp + j * E));
+                }
             }
-        }
     };
-    auto attend = [&](int layer, int p) {
+    auto attend = [&](auto lpk, int layer, int p) {
+        constexpr int LPK = decltype(lpk)::value, KPW = 32 / LPK;
+        const int lik = lane % LPK, kg = lane / LPK;
+        const bool act = lik * 4 < D;
 #pragma unroll 1
-        for (int u = u0; u < units; u += 4 * kClusterBlocks) {
+        for (int u = u0; u < units; u += GROUPS * kClusterBlocks) {
             const Unit un = u == u0 ? first_unit : make_unit(u);
             const int k0 = un.split * per, k1 = min(p + 1, k0 + per);
-            if (u != u0) ask(un, layer, p, 0);       // the first unit's rows were asked for ahead (the next one's too: spills, 105 us per step)
-            const float *now = qkv + un.now;         // this position's query, key and value
+            if (u != u0) ask(lpk, un, layer, p, 0);       // the first unit's rows were asked for ahead (the next one's too: spills, 105 us per step)
+            const float *now = qkv + un.now + lik * 4;         // this position's query, key and value
             float4 q4 = make_float4(0.f, 0.f, 0.f, 0.f);
             if (act) {
                 q4 = *reinterpret_cast<const float4 *>(now);
                 q4.x *= qscale; q4.y *= qscale; q4.z *= qscale; q4.w *= qscale;
             }
-            Part acc{-1e30f, 0.0f, make_float4(0.f, 0.f, 0.f, 0.f)};
-            const int step = W4 * KPW;
-#pragma unroll 1
-            for (int it0 = 0; k0 + it0 * step < k1; it0 += kAhead) {
-                if (it0 > 0) ask(un, layer, p, it0);
-                const int j0 = k0 + (it0 * W4 + w4i) * KPW + kg;
-                const int own = p < k1 ? p - j0 : -1;                      // where this position's own row is among them
-                float s[kAhead];
+            Part acc[VW];
 #pragma unroll
-                for (int it = 0; it < kAhead; ++it) {
-                    if (own == it * step && act) {
-                        k4[it] = *reinterpret_cast<const float4 *>(now + E);
-                        v4[it] = *reinterpret_cast<const float4 *>(now + 2 * E);
+            for (int w = 0; w < VW; ++w) acc[w] = Part{-1e30f, 0.0f, make_float4(0.f, 0.f, 0.f, 0.f)};
+            constexpr int step = W4 * KPW;
+#pragma unroll 1
+            for (int it0 = 0; k0 + it0 * step < k1; it0 += AHEAD) {
+                if (it0 > 0) ask(lpk, un, layer, p, it0);
+                const int j0 = k0 + (it0 * W4 + wg * VW) * KPW + kg;
+                const int own = p < k1 && act ? p - j0 : -1;               // where this position's own row is among them
+                float s[VW][AHEAD];
+#pragma unroll
+                for (int w = 0; w < VW; ++w) {
+#pragma unroll
+                    for (int it = 0; it < AHEAD; ++it) {
+                        if (own == it * step + w * KPW) {
+                            k4[w][it] = *reinterpret_cast<const float4 *>(now + E);
+                            v4[w][it] = *reinterpret_cast<const float4 *>(now + 2 * E);
+                        }
+                        float x = q4.x * k4[w][it].x;
+                        x = fmaf(q4.y, k4[w][it].y, x);
+                        x = fmaf(q4.z, k4[w][it].z, x);
+                        s[w][it] = fmaf(q4.w, k4[w][it].w, x);
                     }
-                    float x = q4.x * k4[it].x;
-                    x = fmaf(q4.y, k4[it].y, x);
-                    x = fmaf(q4.z, k4[it].z, x);
-                    s[it] = fmaf(q4.w, k4[it].w, x);
                 }
 #pragma unroll
-                for (int o = 1; o < 8; o <<= 1)
+                for (int o = 1; o < LPK; o <<= 1)
 #pragma unroll
-                    for (int it = 0; it < kAhead; ++it) s[it] += __shfl_xor_sync(0xffffffffu, s[it], o);
-                if (LPK > 8)
+                    for (int i = 0; i < VW * AHEAD; ++i) s[i / AHEAD][i % AHEAD] += __shfl_xor_sync(0xffffffffu, s[i / AHEAD][i % AHEAD], o);
 #pragma unroll
-                    for (int it = 0; it < kAhead; ++it) s[it] += __shfl_xor_sync(0xffffffffu, s[it], 8);
-#pragma unroll
-                for (int it = 0; it < kAhead; ++it) {
+                for (int it = 0; it < AHEAD; ++it) {
                     if (k0 + (it0 + it) * step >= k1) break;               // no lane of the four warps has a row there
-                    const float x = j0 + it * step < k1 ? s[it] : -INFINITY;
-                    const float mn = fmaxf(acc.m, x);
-                    const float alpha = ex2_approx(acc.m - mn), pr = ex2_approx(x - mn);
-                    acc.l = fmaf(acc.l, alpha, pr);
-                    acc.o.x = fmaf(pr, v4[it].x, acc.o.x * alpha);
-                    acc.o.y = fmaf(pr, v4[it].y, acc.o.y * alpha);
-                    acc.o.z = fmaf(pr, v4[it].z, acc.o.z * alpha);
-                    acc.o.w = fmaf(pr, v4[it].w, acc.o.w * alpha);
-                    acc.m = mn;
+#pragma unroll
+                    for (int w = 0; w < VW; ++w) {
+                        Part &t = acc[w];
+                        const float x = j0 + it * step + w * KPW < k1 ? s[w][it] : -INFINITY;
+                        const float mn = fmaxf(t.m, x);
+                        const float alpha = ex2_approx(t.m - mn), pr = ex2_approx(x - mn);
+                        t.l = fmaf(t.l, alpha, pr);
+                        t.o.x = fmaf(pr, v4[w][it].x, t.o.x * alpha);
+                        t.o.y = fmaf(pr, v4[w][it].y, t.o.y * alpha);
+                        t.o.z = fmaf(pr, v4[w][it].z, t.o.z * alpha);
+                        t.o.w = fmaf(pr, v4[w][it].w, t.o.w * alpha);
+                        t.m = mn;
+                    }
                 }
             }
 #pragma unroll
-            for (int o = 8; o < 32; o <<= 1) {
-                if (o < LPK) continue;
-                const float m2 = __shfl_xor_sync(0xffffffffu, acc.m, o);
-                const float l2 = __shfl_xor_sync(0xffffffffu, acc.l, o);
-                float4 o2;
-                o2.x = __shfl_xor_sync(0xffffffffu, acc.o.x, o);
-                o2.y = __shfl_xor_sync(0xffffffffu, acc.o.y, o);
-                o2.z = __shfl_xor_sync(0xffffffffu, acc.o.z, o);
-                o2.w = __shfl_xor_sync(0xffffffffu, acc.o.w, o);
-                merge_part(acc, m2, l2, o2);
+            for (int o = LPK; o < 32; o <<= 1) {
+#pragma unroll
+                for (int w = 0; w < VW; ++w) {
+                    const float m2 = __shfl_xor_sync(0xffffffffu, acc[w].m, o);
+                    const float l2 = __shfl_xor_sync(0xffffffffu, acc[w].l, o);
+                    float4 o2;
+                    o2.x = __shfl_xor_sync(0xffffffffu, acc[w].o.x, o);
+                    o2.y = __shfl_xor_sync(0xffffffffu, acc[w].o.y, o);
+                    o2.z = __shfl_xor_sync(0xffffffffu, acc[w].o.z, o);
+                    o2.w = __shfl_xor_sync(0xffffffffu, acc[w].o.w, o);
+                    merge_part(acc[w], m2, l2, o2);
+                }
             }
             if (kg == 0) {
-                float *d = merge_s + (w4i * 32 + lik) * 8;
-                *reinterpret_cast<float4 *>(d) = acc.o;
-                *reinterpret_cast<float2 *>(d + 4) = make_float2(acc.m, acc.l);
+#pragma unroll
+                for (int w = 0; w < VW; ++w) {
+                    float *d = merge_s + ((wg * VW + w) * 16 + lik) * 8;
+                    *reinterpret_cast<float4 *>(d) = acc[w].o;
+                    *reinterpret_cast<float2 *>(d + 4) = make_float2(acc[w].m, acc[w].l);
+                }
             }
-            asm volatile("bar.sync %0, 128;" ::"r"(1 + slot4) : "memory");
-            // each of the four warps merges the columns of its lanes' `lik`; its key groups serve different receivers
+            asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(32 * GW) : "memory");
+            // each of the group's warps merges the columns of its lanes' `lik`; its key groups serve different receivers
             const float *m0 = merge_s + lik * 8;
             Part t;
             t.o = *reinterpret_cast<const float4 *>(m0);
             t.m = m0[4]; t.l = m0[5];
 #pragma unroll
             for (int w = 1; w < W4; ++w) {
-                const float4 o2 = *reinterpret_cast<const float4 *>(m0 + w * 256);
-                const float2 ml = *reinterpret_cast<const float2 *>(m0 + w * 256 + 4);
+                const float4 o2 = *reinterpret_cast<const float4 *>(m0 + w * 128);
+                const float2 ml = *reinterpret_cast<const float2 *>(m0 + w * 128 + 4);
                 merge_part(t, ml.x, ml.y, o2);
             }
             const uint32_t dst = smem_u32(rec + un.rec), bar = smem_u32(&hop[kRec]);
 #pragma unroll 1
-            for (int d = kg; d < 4; d += KPW) {
-                const uint32_t pb = peer_addr(bar, 4 * w4i + d), pd = peer_addr(dst, 4 * w4i + d);
+            for (int d = kg; d < 4 * VW; d += KPW) {
+                const uint32_t pb = peer_addr(bar, 4 * VW * wg + d), pd = peer_addr(dst, 4 * VW * wg + d);
                 if (act) send4(pd + lik * 16, pb, t.o);
                 if (lik == 0) send2(pd + D * 4, pb, __float_as_uint(t.m), __float_as_uint(t.l));
             }
-            if (u + 4 * kClusterBlocks < units) asm volatile("bar.sync %0, 128;" ::"r"(1 + slot4) : "memory");
+            if (u + GROUPS * kClusterBlocks < units) asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(32 * GW) : "memory");
         }
     };
     // this warp's segment of the attention output from the records of all splits (attn_decode.cu's decode_combine_kernel)
@@ -574,12 +596,12 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
         per = (p + ns) / ns;
 #pragma unroll 1
         for (int l = 0; l < a.L; ++l) {
-            ask(first_unit, l, p, 0);
+            if (narrow) ask(Job<8>(), first_unit, l, p, 0); else ask(Job<16>(), first_unit, l, p, 0);
 #pragma unroll 1
             for (int pt = 0; pt < cluster_job_of(kJobQkv, E, 0).parts; ++pt)
                 finish(Job<kJobQkv>(), pt, product(Job<kJobQkv>(), xb, [&] { if (pt == 0 && l > 0) receive(kXb); }), l, p);
             receive(kQkv);
-            attend(l, p);
+            if (narrow) attend(Job<8>(), l, p); else attend(Job<16>(), l, p);
 #pragma unroll 1
             for (int pt = 0; pt < cluster_job_of(kJobO, E, 0).parts; ++pt)
                 finish(Job<kJobO>(), pt, product(Job<kJobO>(), nullptr, [&] { if (pt == 0) { receive(kRec); combine(); } }), 0, 0);
@@ -707,28 +729,33 @@ struct ClusterLaunch {
     }
 };
 
-template <int E, int R>
+template <int E, int R, int VW>
 cudaError_t prepare_kernel()
 {
-    auto kern = cluster_steps_kernel<E, R>;
+    auto kern = cluster_steps_kernel<E, R, VW>;
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     return e != cudaSuccess ? e : cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMost);
 }
 
-// `f.template operator()<E, R>()` for the shape; -1 where there is no kernel for it
-template <int R, typename F>
+// f(Width<E, R, VW>()) for the shape; -1 where there is no kernel for it
+template <int R, int VW, typename F>
 int with_width(int E, F f)
 {
     switch (E) {
-#define HIPGPT_CLUSTER(W) case W: return f(Width<W, R>());
+#define HIPGPT_CLUSTER(W) case W: return f(Width<W, R, VW>());
     HIPGPT_CLUSTER(128) HIPGPT_CLUSTER(160) HIPGPT_CLUSTER(192) HIPGPT_CLUSTER(224) HIPGPT_CLUSTER(256) HIPGPT_CLUSTER(288)
     HIPGPT_CLUSTER(320) HIPGPT_CLUSTER(352) HIPGPT_CLUSTER(384)
 #undef HIPGPT_CLUSTER
     default: return -1;
     }
 }
+// `units`: (row, head, split) of a cluster.  Sixteen blocks have 64 groups of four warps.
 template <typename F>
-int with_kernel(int E, int rows, F f) { return rows == 1 ? with_width<1>(E, f) : with_width<2>(E, f); }
+int with_kernel(int E, int rows, int units, F f)
+{
+    if (rows == 1) return units <= 64 ? with_width<1, 1>(E, f) : with_width<1, 2>(E, f);
+    return units <= 64 ? with_width<2, 1>(E, f) : with_width<2, 2>(E, f);
+}
 
 }  // namespace
 
@@ -751,10 +778,11 @@ ClusterPlan cluster_plan(int V, int S, int E, int L, int H, int F)
     }
     if (p.all_chunks > 1024 || p.block_bytes > 0xffffffffu || (long long)S * E > 1 << 24) return p;
     // how many clusters of sixteen blocks, one block per SM, the GPU holds at the same time
-    const int rc = with_kernel(E, 2, [&](auto w) {
-        if (prepare_kernel<decltype(w)::kE, decltype(w)::kR>() != cudaSuccess) return 1;
+    const int rc = with_kernel(E, 2, 1, [&](auto w) {
+        using W = decltype(w);
+        if (prepare_kernel<W::kE, W::kR, W::kVW>() != cudaSuccess) return 1;
         ClusterLaunch l(1, kSmemMost, nullptr);
-        return cudaOccupancyMaxActiveClusters(&p.clusters_most, cluster_steps_kernel<decltype(w)::kE, decltype(w)::kR>, &l.cfg) == cudaSuccess ? 0 : 1;
+        return cudaOccupancyMaxActiveClusters(&p.clusters_most, cluster_steps_kernel<W::kE, W::kR, W::kVW>, &l.cfg) == cudaSuccess ? 0 : 1;
     });
     if (rc > 0) cudaGetLastError();
     p.ok = rc == 0 && p.clusters_most > 0;
@@ -802,19 +830,19 @@ int cluster_rows(const ClusterPlan &p, int B, int E, int H, int ns)
     if (!p.ok) return 0;
     const int rows = B <= p.clusters_most ? 1 : (B + 1) / 2 <= p.clusters_most ? 2 : 0;
     if (rows == 0) return 0;
-    const int slots = with_kernel(E, rows, [&](auto w) { return rest_of<decltype(w)::kE, decltype(w)::kR>(H, E / H, ns, p.all_chunks).slots; });
+    const int slots = with_kernel(E, rows, rows * H * ns, [&](auto w) { return rest_of<decltype(w)::kE, decltype(w)::kR>(H, E / H, ns, p.all_chunks).slots; });
     return slots >= 9 ? rows : 0;
 }
 
 int launch_cluster_steps(const ClusterPlan &p, const ClusterArgs &a, int E, int rows, cudaStream_t st)
 {
-    return with_kernel(E, rows, [&](auto w) {
-        constexpr int kE = decltype(w)::kE, kR = decltype(w)::kR;
+    return with_kernel(E, rows, rows * a.H * a.ns, [&](auto w) {
+        constexpr int kE = decltype(w)::kE, kR = decltype(w)::kR, kVW = decltype(w)::kVW;
         const Rest lay = rest_of<kE, kR>(a.H, kE / a.H, a.ns, p.all_chunks);
-        cudaError_t e = prepare_kernel<kE, kR>();
+        cudaError_t e = prepare_kernel<kE, kR, kVW>();
         if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "cluster_steps_kernel attributes: %s", cudaGetErrorString(e));
         ClusterLaunch l((a.B + rows - 1) / rows, (size_t)lay.total, st);
-        e = cudaLaunchKernelEx(&l.cfg, cluster_steps_kernel<kE, kR>, p, a, lay);
+        e = cudaLaunchKernelEx(&l.cfg, cluster_steps_kernel<kE, kR, kVW>, p, a, lay);
         if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "cluster_steps_kernel launch: %s", cudaGetErrorString(e));
         return HIPGPT_OK;
     });
