@@ -23,8 +23,8 @@
 // Waits on mbarriers are bounded: on expiry the block raises a flag that cuts its later waits short and sets the error word; the
 // steps then run out without waiting.
 //
-// Measured at the default model (E=256 L=8 H=8 V=5000), batch 8: 87 us per step (the replayed graph: 318), batch 1: 73 (256).  A
-// step is 42 products of about 450 ns each, attention two fifths of a layer.  Sizes are template parameters because the chain is
+// Measured at the default model (E=256 L=8 H=8 V=5000), batch 8: 73 us per step (the replayed graph: 318), batch 1: 68 (256).  A
+// step is 42 products of 400 - 450 ns each, attention a third of a layer.  Sizes are template parameters because the chain is
 // bound by the instructions of single warps: with sizes read from the plan a step took 143 us.
 #include "gpt_cluster.cuh"
 #include "tc_primitives.cuh"
@@ -86,8 +86,8 @@ __device__ __forceinline__ void merge_part(Part &a, float m2, float l2, const fl
 
 template <int J>
 struct Job { static constexpr int value = J; };
-template <int E, int R, int VW>
-struct Width { static constexpr int kE = E, kR = R, kVW = VW; };
+template <int E, int D, int R, int VW>
+struct Width { static constexpr int kE = E, kD = D, kR = R, kVW = VW; };
 
 // Shared memory of a block, in floats from the start: what has a size known to the compiler first.  Rows of activations are padded
 // by four floats: the rows that a warp reads side by side then lie in different banks.
@@ -123,7 +123,7 @@ Rest rest_of(int H, int D, int ns, int all_chunks)
     return r;
 }
 
-template <int E, int R, int VW>
+template <int E, int D, int R, int VW>
 __global__ void __launch_bounds__(kThreads, 1)
 cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_constant__ ClusterArgs a, const __grid_constant__ Rest lay)
 {
@@ -143,8 +143,8 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
     asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
     const int row0 = (int)(blockIdx.x / kClusterBlocks) * R;
     const int rows = min(R, a.B - row0);             // sequences of this cluster
-    const int V = a.V, H = a.H, D = E / H, ns = a.ns;
-    const int rstride = D + 4;
+    constexpr int H = E / D, rstride = D + 4;
+    const int V = a.V, ns = a.ns;
 
     float *xb = sm + C::xb, *xa = sm + C::xa, *qkv = sm + C::qkv, *ff = sm + C::ff, *rec = sm + C::fixed, *part = sm + C::part;
     float *aw = sm + C::aw + warp * (R * C::seg);    // this warp's own segment of the activations
@@ -396,8 +396,8 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
     //      outnumber its groups of four warps (a second round costs more than the doubled work of a warp that is bound by latency).
     //      A key's head is read by LPK lanes (4 numbers each) ----
     constexpr int W4 = 4, GW = W4 / VW, GROUPS = kWarps / GW, AHEAD = kAhead / VW;
-    const bool narrow = D <= 32;                     // LPK = 8, else 16: the code exists for both, so that lanes and strides are constants
-    const int group = warp / GW, wg = warp % GW;
+    constexpr int LPK = D / 4, KPW = 32 / LPK;
+    const int group = warp / GW, wg = warp % GW, lik = lane % LPK, kg = lane / LPK;
     const float qscale = (1.0f / sqrtf((float)D)) * kLog2e;
     const int units = rows * H * ns;
     float *merge_s = sm + C::unit + group * (W4 * 16 * 8);
@@ -410,11 +410,8 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
     const Unit first_unit = make_unit(min(u0, units - 1));
     int per = 0;                                     // positions of a split at this step
     float4 k4[VW][AHEAD], v4[VW][AHEAD];             // rows of a unit that earlier steps wrote
-    auto ask = [&](auto lpk, const Unit &un, int layer, int p, int it0) {
-        constexpr int LPK = decltype(lpk)::value, KPW = 32 / LPK;
-        const int lik = lane % LPK, kg = lane / LPK;
-        const bool act = lik * 4 < D;
-        const int j0 = un.split * per + (it0 * W4 + wg * VW) * KPW + kg, k1 = act ? min(p, un.split * per + per) : 0;
+    auto ask = [&](const Unit &un, int layer, int p, int it0) {
+        const int j0 = un.split * per + (it0 * W4 + wg * VW) * KPW + kg, k1 = min(p, un.split * per + per);
         const size_t at = (size_t)layer * a.layer_stride + (size_t)(un.mem + lik * 4) + (size_t)j0 * E;
         const float *kp = a.kc + at, *vp = a.vc + at;
 #pragma unroll
@@ -429,30 +426,24 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
                 }
             }
     };
-    auto attend = [&](auto lpk, int layer, int p) {
-        constexpr int LPK = decltype(lpk)::value, KPW = 32 / LPK;
-        const int lik = lane % LPK, kg = lane / LPK;
-        const bool act = lik * 4 < D;
+    auto attend = [&](int layer, int p) {
 #pragma unroll 1
         for (int u = u0; u < units; u += GROUPS * kClusterBlocks) {
             const Unit un = u == u0 ? first_unit : make_unit(u);
             const int k0 = un.split * per, k1 = min(p + 1, k0 + per);
-            if (u != u0) ask(lpk, un, layer, p, 0);       // the first unit's rows were asked for ahead (the next one's too: spills, 105 us per step)
+            if (u != u0) ask(un, layer, p, 0);       // the first unit's rows were asked for ahead (the next one's too: spills, 105 us per step)
             const float *now = qkv + un.now + lik * 4;         // this position's query, key and value
-            float4 q4 = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (act) {
-                q4 = *reinterpret_cast<const float4 *>(now);
-                q4.x *= qscale; q4.y *= qscale; q4.z *= qscale; q4.w *= qscale;
-            }
+            float4 q4 = *reinterpret_cast<const float4 *>(now);
+            q4.x *= qscale; q4.y *= qscale; q4.z *= qscale; q4.w *= qscale;
             Part acc[VW];
 #pragma unroll
             for (int w = 0; w < VW; ++w) acc[w] = Part{-1e30f, 0.0f, make_float4(0.f, 0.f, 0.f, 0.f)};
             constexpr int step = W4 * KPW;
 #pragma unroll 1
             for (int it0 = 0; k0 + it0 * step < k1; it0 += AHEAD) {
-                if (it0 > 0) ask(lpk, un, layer, p, it0);
+                if (it0 > 0) ask(un, layer, p, it0);
                 const int j0 = k0 + (it0 * W4 + wg * VW) * KPW + kg;
-                const int own = p < k1 && act ? p - j0 : -1;               // where this position's own row is among them
+                const int own = p < k1 ? p - j0 : -1;               // where this position's own row is among them
                 float s[VW][AHEAD];
 #pragma unroll
                 for (int w = 0; w < VW; ++w) {
@@ -528,7 +519,7 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
 #pragma unroll 1
             for (int d = kg; d < 4 * VW; d += KPW) {
                 const uint32_t pb = peer_addr(bar, 4 * VW * wg + d), pd = peer_addr(dst, 4 * VW * wg + d);
-                if (act) send4(pd + lik * 16, pb, t.o);
+                send4(pd + lik * 16, pb, t.o);
                 if (lik == 0) send2(pd + D * 4, pb, __float_as_uint(t.m), __float_as_uint(t.l));
             }
             if (u + GROUPS * kClusterBlocks < units) asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(32 * GW) : "memory");
@@ -541,7 +532,7 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
         for (int t = 0; t < (R * o_klen + 31) / 32; ++t) {
             const int i = lane + 32 * t, r = i / o_klen, e = warp * o_klen + i % o_klen;
             if (i < R * o_klen && r < rows) {
-                const int h = D == 32 ? e >> 5 : D == 64 ? e >> 6 : e / D, d = e - h * D;
+                const int h = e / D, d = e % D;
                 const float *rc = rec + (r * H + h) * ns * rstride;
                 float M = -1e30f, Lsum = 0.0f, acc = 0.0f;
                 if (ns <= 8) {                       // all loads in flight at once
@@ -596,12 +587,12 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
         per = (p + ns) / ns;
 #pragma unroll 1
         for (int l = 0; l < a.L; ++l) {
-            if (narrow) ask(Job<8>(), first_unit, l, p, 0); else ask(Job<16>(), first_unit, l, p, 0);
+            ask(first_unit, l, p, 0);
 #pragma unroll 1
             for (int pt = 0; pt < cluster_job_of(kJobQkv, E, 0).parts; ++pt)
                 finish(Job<kJobQkv>(), pt, product(Job<kJobQkv>(), xb, [&] { if (pt == 0 && l > 0) receive(kXb); }), l, p);
             receive(kQkv);
-            if (narrow) attend(Job<8>(), l, p); else attend(Job<16>(), l, p);
+            attend(l, p);
 #pragma unroll 1
             for (int pt = 0; pt < cluster_job_of(kJobO, E, 0).parts; ++pt)
                 finish(Job<kJobO>(), pt, product(Job<kJobO>(), nullptr, [&] { if (pt == 0) { receive(kRec); combine(); } }), 0, 0);
@@ -729,32 +720,33 @@ struct ClusterLaunch {
     }
 };
 
-template <int E, int R, int VW>
+template <int E, int D, int R, int VW>
 cudaError_t prepare_kernel()
 {
-    auto kern = cluster_steps_kernel<E, R, VW>;
+    auto kern = cluster_steps_kernel<E, D, R, VW>;
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     return e != cudaSuccess ? e : cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMost);
 }
 
-// f(Width<E, R, VW>()) for the shape; -1 where there is no kernel for it
+// f(Width<E, D, R, VW>()) for the shape; -1 where there is no kernel for it
 template <int R, int VW, typename F>
-int with_width(int E, F f)
+int with_width(int E, int D, F f)
 {
-    switch (E) {
-#define HIPGPT_CLUSTER(W) case W: return f(Width<W, R, VW>());
-    HIPGPT_CLUSTER(128) HIPGPT_CLUSTER(160) HIPGPT_CLUSTER(192) HIPGPT_CLUSTER(224) HIPGPT_CLUSTER(256) HIPGPT_CLUSTER(288)
-    HIPGPT_CLUSTER(320) HIPGPT_CLUSTER(352) HIPGPT_CLUSTER(384)
+    switch (E * 1000 + D) {
+#define HIPGPT_CLUSTER(W, HD) case W * 1000 + HD: return f(Width<W, HD, R, VW>());
+    HIPGPT_CLUSTER(128, 32) HIPGPT_CLUSTER(160, 32) HIPGPT_CLUSTER(192, 32) HIPGPT_CLUSTER(224, 32) HIPGPT_CLUSTER(256, 32) HIPGPT_CLUSTER(288, 32)
+    HIPGPT_CLUSTER(320, 32) HIPGPT_CLUSTER(352, 32) HIPGPT_CLUSTER(384, 32)
+    HIPGPT_CLUSTER(128, 64) HIPGPT_CLUSTER(192, 64) HIPGPT_CLUSTER(256, 64) HIPGPT_CLUSTER(320, 64) HIPGPT_CLUSTER(384, 64)
 #undef HIPGPT_CLUSTER
     default: return -1;
     }
 }
 // `units`: (row, head, split) of a cluster.  Sixteen blocks have 64 groups of four warps.
 template <typename F>
-int with_kernel(int E, int rows, int units, F f)
+int with_kernel(int E, int D, int rows, int units, F f)
 {
-    if (rows == 1) return units <= 64 ? with_width<1, 1>(E, f) : with_width<1, 2>(E, f);
-    return units <= 64 ? with_width<2, 1>(E, f) : with_width<2, 2>(E, f);
+    if (rows == 1) return units <= 64 ? with_width<1, 1>(E, D, f) : with_width<1, 2>(E, D, f);
+    return units <= 64 ? with_width<2, 1>(E, D, f) : with_width<2, 2>(E, D, f);
 }
 
 }  // namespace
@@ -763,7 +755,7 @@ ClusterPlan cluster_plan(int V, int S, int E, int L, int H, int F)
 {
     ClusterPlan p = {};
     const int D = E / H;
-    if (D % 4 != 0 || D > 64 || F != 4 * E) return p;
+    if ((D != 32 && D != 64) || F != 4 * E) return p;
     // the output projection's parts have the width the kernel is compiled for; the vocabulary decides how many there are
     p.voc = cluster_job_of(kJobVoc, E, 64 * 64);
     p.voc.n = V;
@@ -778,11 +770,11 @@ ClusterPlan cluster_plan(int V, int S, int E, int L, int H, int F)
     }
     if (p.all_chunks > 1024 || p.block_bytes > 0xffffffffu || (long long)S * E > 1 << 24) return p;
     // how many clusters of sixteen blocks, one block per SM, the GPU holds at the same time
-    const int rc = with_kernel(E, 2, 1, [&](auto w) {
+    const int rc = with_kernel(E, D, 2, 1, [&](auto w) {
         using W = decltype(w);
-        if (prepare_kernel<W::kE, W::kR, W::kVW>() != cudaSuccess) return 1;
+        if (prepare_kernel<W::kE, W::kD, W::kR, W::kVW>() != cudaSuccess) return 1;
         ClusterLaunch l(1, kSmemMost, nullptr);
-        return cudaOccupancyMaxActiveClusters(&p.clusters_most, cluster_steps_kernel<W::kE, W::kR, W::kVW>, &l.cfg) == cudaSuccess ? 0 : 1;
+        return cudaOccupancyMaxActiveClusters(&p.clusters_most, cluster_steps_kernel<W::kE, W::kD, W::kR, W::kVW>, &l.cfg) == cudaSuccess ? 0 : 1;
     });
     if (rc > 0) cudaGetLastError();
     p.ok = rc == 0 && p.clusters_most > 0;
@@ -830,19 +822,19 @@ int cluster_rows(const ClusterPlan &p, int B, int E, int H, int ns)
     if (!p.ok) return 0;
     const int rows = B <= p.clusters_most ? 1 : (B + 1) / 2 <= p.clusters_most ? 2 : 0;
     if (rows == 0) return 0;
-    const int slots = with_kernel(E, rows, rows * H * ns, [&](auto w) { return rest_of<decltype(w)::kE, decltype(w)::kR>(H, E / H, ns, p.all_chunks).slots; });
+    const int slots = with_kernel(E, E / H, rows, rows * H * ns, [&](auto w) { return rest_of<decltype(w)::kE, decltype(w)::kR>(H, E / H, ns, p.all_chunks).slots; });
     return slots >= 9 ? rows : 0;
 }
 
 int launch_cluster_steps(const ClusterPlan &p, const ClusterArgs &a, int E, int rows, cudaStream_t st)
 {
-    return with_kernel(E, rows, rows * a.H * a.ns, [&](auto w) {
-        constexpr int kE = decltype(w)::kE, kR = decltype(w)::kR, kVW = decltype(w)::kVW;
+    return with_kernel(E, E / a.H, rows, rows * a.H * a.ns, [&](auto w) {
+        constexpr int kE = decltype(w)::kE, kD = decltype(w)::kD, kR = decltype(w)::kR, kVW = decltype(w)::kVW;
         const Rest lay = rest_of<kE, kR>(a.H, kE / a.H, a.ns, p.all_chunks);
-        cudaError_t e = prepare_kernel<kE, kR, kVW>();
+        cudaError_t e = prepare_kernel<kE, kD, kR, kVW>();
         if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "cluster_steps_kernel attributes: %s", cudaGetErrorString(e));
         ClusterLaunch l((a.B + rows - 1) / rows, (size_t)lay.total, st);
-        e = cudaLaunchKernelEx(&l.cfg, cluster_steps_kernel<kE, kR, kVW>, p, a, lay);
+        e = cudaLaunchKernelEx(&l.cfg, cluster_steps_kernel<kE, kD, kR, kVW>, p, a, lay);
         if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "cluster_steps_kernel launch: %s", cudaGetErrorString(e));
         return HIPGPT_OK;
     });
