@@ -32,7 +32,9 @@
 // query tile share its output columns.  One issuing warp issues the copies and every Q K^T, the other two the
 // P V products of one query tile each, in a fixed order, so results do not depend on timing.
 // Probabilities (when asked for): a row's sum is known once all its tiles have been through the exponentials;
-// the workers then read P_hi + P_lo back from TMEM, divide by the sum and store [B][H][S][S]: no second Q K^T.
+// the workers then read P_hi + P_lo back from TMEM, divide by the sum and store [B][H][S][S] by TMA: no second Q K^T.
+// At B=32 H=8 S=256 unmasked 30.2 us (36.2 with stores through the workers' registers, the next head's Q and K fetched
+// only after them), causal 25.4 (30.4); a store phase of 128 KB takes 2.5 us on all SMs at once, which is what HBM takes.
 // Every wait is bounded: on expiry the block raises a flag that cuts all later waits short, records a
 // site code for hipgpt_kernel_status, skips its stores, frees its TMEM and returns.
 #include "tc_primitives.cuh"
@@ -51,7 +53,10 @@ constexpr int kHeadThreads = kHeadWorkers + 32 * kHeadIssuers;
 constexpr uint32_t kTileBytes = kTile * 128;     // one [128][128 byte] operand block
 constexpr uint32_t kOffQraw = 0, kOffKraw = 2 * kTileBytes, kOffVraw = 4 * kTileBytes;
 constexpr uint32_t kOffQ16 = 6 * kTileBytes, kOffK16 = 8 * kTileBytes, kOffV16 = 10 * kTileBytes;
+// probabilities on their way out: 4 KB per worker warp, in the raw V tiles (read once, at the start of a head) and behind the operands
+constexpr uint32_t kOffStage = 12 * kTileBytes, kStageWarp = 4096;
 constexpr uint32_t kHeadSmemBytes = 12 * kTileBytes;
+constexpr uint32_t kStageBytes = (kHeadWorkers / 32) * kStageWarp - 2 * kTileBytes;
 constexpr uint32_t kColO = 384;                  // after three buffers of 128 columns
 constexpr float kPShift = 8.0f;                  // P carries a factor 2^8: small probabilities stay normal fp16 numbers
 constexpr long long kHeadCycleLimit = 1LL << 28; // per wait, about 0.14 s
@@ -125,14 +130,33 @@ __device__ __forceinline__ void chunk_zero(uint32_t addr)
     tmem_st16_u32(addr + 16, z);
 }
 
+// Two values from their packed fp16 halves hi (exact) and lo; the sums are rounded once, as float adds.
+__device__ __forceinline__ float2 f16_sum(float hi, float lo)
+{
+    const __half2 h = *reinterpret_cast<const __half2 *>(&hi);
+    float2 r = make_float2(__low2float(h), __high2float(h));
+    asm("{.reg .b16 a, b; mov.b32 {a, b}, %2; add.rn.f32.f16 %0, a, %0; add.rn.f32.f16 %1, b, %1;}" : "+f"(r.x), "+f"(r.y) : "r"(__float_as_uint(lo)));
+    return r;
+}
+
+__device__ __forceinline__ void tma_store_3d(const void *tensor_map, const void *smem_src, int c0, int c1, int c2)
+{
+    asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%1, %2, %3}], [%4];"
+                 ::"l"(reinterpret_cast<uint64_t>(tensor_map)), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(smem_src)) : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+// Until this thread's stores have read shared memory.
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+
 struct HeadMaps {
     CUtensorMap q, k, v;
+    CUtensorMap p;                               // the probabilities, [BH][S][S], in boxes of 32 x 32
     CUtensorMap q32;                             // Q in boxes of 32 rows (a causal head's first query tile, below)
 };
 
-template <bool CAUSAL, bool PROBS>
+template <bool CAUSAL, bool PROBS, bool RING>
 __global__ void __launch_bounds__(kHeadThreads, 1)
-mha_head_kernel(const __grid_constant__ HeadMaps maps, float *__restrict__ O, float *__restrict__ P, int S, int E, int H, int BH, float cscale)
+mha_head_kernel(const __grid_constant__ HeadMaps maps, float *__restrict__ O, float *__restrict__ P, int S, int E, int H, int BH, float cscale, int p_mapped)
 {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *base = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -142,20 +166,21 @@ mha_head_kernel(const __grid_constant__ HeadMaps maps, float *__restrict__ O, fl
     uint8_t *v_16 = base + kOffV16;              // [V_hi | V_lo] (64 columns) fp16, N-major without swizzle: 8 keys x 8 columns
                                                  // form one 128-byte core matrix, column blocks 128 bytes apart, key groups 1024
     __shared__ uint64_t ld_q[2], ld_k[2], ld_v[2], cv_q[2], cv_k[2], cv_v[2];
-    __shared__ uint64_t s_full[3], p_full[4], o_done[2], xm[2], xs[2], epi_done, vx, pr_done, b0_free;
+    __shared__ uint64_t s_full[3], p_full[4], o_done[2], xm[2], xs[2], epi_done, vx, pr_read[3], b_free[3];
     __shared__ uint32_t tmem_base_slot;
     __shared__ volatile int abort_flag;
     __shared__ float xmax[2][2][2][kTile];       // [head parity][query tile][slot][row]
     __shared__ float xsum[2][2][2][kTile];
     __shared__ float vmaxw[2][4];                // [head parity][warp of the V group]
-    __shared__ float s_vinv[2];                  // 1 / (V's power-of-two scale), by head parity
+    __shared__ float s_vinv[4];                  // 1 / (V's power-of-two scale), by head mod 4 (found one head ahead)
     __shared__ unsigned s_amax[2];               // bit patterns of max |Q| and max |K| of the current head
 
     const int tid = threadIdx.x, lane = tid & 31;
     // the warp's number, read from one lane so that the compiler knows it (and the role, tile and buffer numbers
     // that follow from it) to be the same for the whole warp: descriptors then live in uniform registers
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
-    const int nq = S > kTile ? 2 : 1;            // query tiles = key tiles of a head
+    // query tiles = key tiles of a head (the host launches the forms without RING for two tiles, the causal one with it for one)
+    const int nq = !RING ? 2 : CAUSAL ? 1 : S > kTile ? 2 : 1;
     // A causal head of two tiles has two diagonal score tiles, (q0, k0) and (q1, k1), where a warp's work grows with its
     // rows: the warp of TMEM lanes 96-127 sweeps four 32-column chunks, that of lanes 0-31 one.  A warp's number fixes
     // both its lanes and its scheduler (warp mod 4), so one scheduler would get 4 + 4 + 4 chunks of exponentials per
@@ -163,10 +188,18 @@ mha_head_kernel(const __grid_constant__ HeadMaps maps, float *__restrict__ O, fl
     // 32 in reverse order (tile row r in lanes of group 3 - r / 32): the copies place them so, and every place that
     // turns a lane of that tile into a row (mask, output row, probabilities) turns it back.  9 chunks per scheduler.
     const bool flip0 = CAUSAL && nq == 2;
+    // Which buffer a score tile goes into, and how many tiles that buffer has held before it.  RING: the tiles of all the block's
+    // heads in sequence (four per head, one with a single query tile) go through the three buffers, and the groups of workers
+    // that own them, in turn: a group that owns two tiles of one head owns one of the next two, and a head's first tiles start
+    // while the last ones of the head before are still being stored.  Otherwise tile t of every head goes into buffer t, an
+    // unmasked head's fourth into the first buffer again.
+    auto ring_no = [&](int it, int t) { return (nq == 1 ? it : 4 * it) + t; };
+    auto buf_of = [&](int it, int t) { return RING ? ring_no(it, t) % 3 : t == 3 ? 0 : t; };
+    auto use_of = [&](int it, int t) { return ring_no(it, t) / 3; };
 
     // site codes: 1 Q/K/V landed, 2 operand converted, 3 S ready, 4 P written, 5 output complete,
     // 6 row maxima exchanged, 7 row sums exchanged, 8 previous head's output read, 9 V maximum exchanged,
-    // 10 probabilities of the first tile read back, 11 first product of an unmasked head complete
+    // 10 probabilities of a tile read back, 11 a buffer's product complete (unmasked)
     // (the kernel's instructions are fetched cold by every SM, so the code is kept small: the polling loop of a
     // wait exists once, out of line, behind a one-instruction test that is all an already completed phase costs)
     auto wait = [&](uint64_t *bar, uint32_t parity, int site) {
@@ -229,8 +262,7 @@ mha_head_kernel(const __grid_constant__ HeadMaps maps, float *__restrict__ O, fl
                 for (int i = 0; i < 4; ++i) mbar_init(&p_full[i], 4);
                 mbar_init(&epi_done, kHeadWorkers / 32);
                 mbar_init(&vx, 4);
-                mbar_init(&pr_done, 4);
-                mbar_init(&b0_free, 1);
+                for (int i = 0; i < 3; ++i) { mbar_init(&pr_read[i], 4); mbar_init(&b_free[i], 1); }
             }
             __syncwarp();
             asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)), "r"(512) : "memory");
@@ -275,7 +307,7 @@ mha_head_kernel(const __grid_constant__ HeadMaps maps, float *__restrict__ O, fl
                     if (elect_one()) mma_ss(d, dq + (uint64_t)(ks * 2), dk + (uint64_t)(ks * 2), id_qk_t, 1u);
                 if (elect_one()) tc_commit(&s_full[buf]);
             };
-            const int nfirst = nq == 1 ? 1 : 3;      // tiles whose buffers are free at the start of a head
+            const int nfirst = nq == 1 ? 1 : 3;      // tiles issued before V's conversion is waited for
             int it = 0;
 #pragma unroll 1
             for (int hd = blockIdx.x; hd < BH; hd += gridDim.x, ++it) {
@@ -283,26 +315,31 @@ mha_head_kernel(const __grid_constant__ HeadMaps maps, float *__restrict__ O, fl
                 const int next = hd + (int)gridDim.x;
                 const bool has_next = next < BH;
                 // ---- Q K^T of every tile whose buffer is free ---------------------------------------
-                // (with the probabilities stored, the workers read P back from these buffers until their output is out,
-                // and stage them in the Q and K areas of shared memory, so this head's Q and K are fetched only now)
-                if (PROBS && it > 0) {
-                    wait(&epi_done, ppar, 8);
-                    load_qk(hd);
-                }
-                // tile t: causal (q0,k0) (q1,k0) (q1,k1), unmasked (q0,k0) (q0,k1) (q1,k0), into buffer t.  A buffer still
-                // holds the previous head's P until the P V products that read it have completed: the first buffer is
-                // read by query tile 0 only in a causal head, every other case waits for both accumulators.
-#pragma unroll 1
-                for (int t = 0; t < nfirst; ++t) {
-                    const int q = CAUSAL ? (t > 0) : (t >> 1), k = CAUSAL ? (t > 1) : (t & 1);
-                    if (it > 0) {
+                // tile t: causal (q0,k0) (q1,k0) (q1,k1), unmasked (q0,k0) (q0,k1) (q1,k0) (q1,k1).  A buffer still holds the P
+                // of the tile before until the P V product that reads it has completed (RING: that product; otherwise the first
+                // buffer is read by query tile 0 only in a causal head, every other case waits for both accumulators) and, with
+                // the probabilities stored, until its workers have read it back.
+                auto issue_tile = [&](int t) {
+                    const int q = CAUSAL ? (t > 0) : (t >> 1), k = CAUSAL ? (t > 1) : (t & 1), buf = buf_of(it, t);
+                    if (RING) {
+                        const int use = use_of(it, t);
+                        if (use > 0) {
+                            wait(&b_free[buf], (uint32_t)((use - 1) & 1), 11);
+                            if (PROBS) wait(&pr_read[buf], (uint32_t)((use - 1) & 1), 10);
+                        }
+                    } else if (it > 0) {
                         if (t == 0) wait(&o_done[0], ppar, 5);
                         if (nq == 2 && t == (CAUSAL ? 1 : 0)) wait(&o_done[1], ppar, 5);
+                        if (PROBS) wait(&pr_read[buf], ppar, 10);
                     }
                     wait(&cv_k[k], par, 2);
                     wait(&cv_q[q], par, 2);
                     tc_fence_after();
-                    issue_qk(q, k, t);
+                    issue_qk(q, k, buf);
+                };
+#pragma unroll 1
+                for (int t = 0; t < nfirst; ++t) {
+                    issue_tile(t);
                     // The next head's tiles are asked into L2 now: this head's operands have landed, so the memory system is
                     // idle, and the copies that fetch them once this head's Q K^T products have completed (all SMs within the
                     // same microsecond again) then hit L2.
@@ -329,27 +366,35 @@ mha_head_kernel(const __grid_constant__ HeadMaps maps, float *__restrict__ O, fl
                     if (over || (flush > 3.8e-6f && (aq + ak) > 8.0f * aq * ak)) atomicOr(&g_head_notice, 1);
                 }
                 __syncwarp();
+                // the raw Q and K tiles and their fp16 copies are free once every Q K^T has completed
+                auto wait_qk = [&](int t) {
+                    if (RING) wait(&s_full[buf_of(it, t)], (uint32_t)(use_of(it, t) & 1), 3);
+                    else wait(&s_full[t], par, 3);
+                };
                 const bool tail_qk = !CAUSAL && nq == 2;    // the fourth tile's Q K^T comes after the first P V product
-                if (has_next && !tail_qk && !PROBS) {
-                    // the raw Q and K tiles and their fp16 copies are free once every Q K^T has completed
-                    wait(&s_full[0], par, 3);
-                    if (nq == 2) { wait(&s_full[1], par, 3); wait(&s_full[2], par, 3); }
+                if (has_next && !tail_qk) {
+                    wait_qk(0);
+                    if (nq == 2) { wait_qk(1); wait_qk(2); }
                     load_qk(next);
                 }
-                wait(&cv_v[0], par, 2);
-                if (nq == 2) wait(&cv_v[1], par, 2);
-                if (has_next) load_v(next);              // the raw V tiles have been read
+                if (!PROBS) {
+                    wait(&cv_v[0], par, 2);
+                    if (nq == 2) wait(&cv_v[1], par, 2);
+                    if (has_next) load_v(next);          // the raw V tiles have been read
+                }
                 if (tail_qk) {
-                    // (q1, k1) into the first buffer, once the product that reads (q0, k0)'s P from it has completed;
-                    // with the probabilities stored its workers must also have read that P back
-                    wait(&b0_free, par, 11);
-                    if (PROBS) wait(&pr_done, par, 10);
-                    tc_fence_after();
-                    issue_qk(1, 1, 0);
-                    if (has_next && !PROBS) {
-                        wait(&s_full[0], 1u, 3);         // second completion of this barrier in this head
-                        wait(&s_full[1], par, 3);
-                        wait(&s_full[2], par, 3);
+                    if (RING) {
+                        issue_tile(3);
+                    } else {
+                        wait(&b_free[0], par, 11);
+                        tc_fence_after();
+                        issue_qk(1, 1, 0);
+                    }
+                    if (has_next) {
+                        if (RING) wait_qk(3);
+                        else wait(&s_full[0], 1u, 3);    // second completion of this barrier in this head
+                        wait_qk(1);
+                        wait_qk(2);
                         load_qk(next);
                     }
                 }
@@ -369,13 +414,17 @@ mha_head_kernel(const __grid_constant__ HeadMaps maps, float *__restrict__ O, fl
 #pragma unroll 1
             for (int hd = blockIdx.x; hd < BH; hd += gridDim.x, ++it) {
                 const uint32_t par = (uint32_t)(it & 1);
-                if (it > 0) wait(&epi_done, (uint32_t)((it - 1) & 1), 8);     // the previous head's output has left TMEM
+                if (it > 0) {
+                    wait(&epi_done, (uint32_t)((it - 1) & 1), 8);        // the previous head's output has left TMEM
+                    if (PROBS && q == 0) load_v(hd);     // ... and its probabilities have left the raw V tiles
+                }
 #pragma unroll 1
                 for (int j = 0; j < npv; ++j) {
                     const uint32_t pj = j ? pj1 : pj0;
-                    const int k = pj & 1, buf = (pj >> 1) & 3, ptile = (pj >> 3) & 3;
+                    const int k = pj & 1, t = (pj >> 3) & 3, buf = RING ? buf_of(it, t) : (pj >> 1) & 3;
                     wait(&cv_v[k], par, 2);
-                    wait(&p_full[ptile], par, 4);
+                    // (RING: by buffer; with one query tile the workers may be two heads ahead of this product)
+                    wait(&p_full[RING ? buf : t], RING ? (uint32_t)(use_of(it, t) & 1) : par, 4);
                     tc_fence_after();
                     // keys 32c .. 32c+31 of the tile: P_hi in columns [32c, 32c+16) of the buffer, P_lo in [32c+16, 32c+32)
                     const uint32_t a0 = tmem + (uint32_t)(buf * kTile);
@@ -388,8 +437,12 @@ mha_head_kernel(const __grid_constant__ HeadMaps maps, float *__restrict__ O, fl
 #pragma unroll
                     for (int ks = 0; ks < 8; ++ks)
                         if (ks < nks && elect_one()) mma_h_ts(d + 32, a0 + (uint32_t)(32 * (ks >> 1) + 8 * (ks & 1) + 16), dv + (uint64_t)(ks * 128), id_pv_b, 1u);
-                    // an unmasked head's fourth score tile goes into the first buffer once this product has read it
-                    if (!CAUSAL && nq == 2 && q == 0 && j == 0 && elect_one()) tc_commit(&b0_free);
+                    // the buffer's next tile waits for this product alone
+                    if (RING) {
+                        if (elect_one()) tc_commit(&b_free[buf]);
+                    } else if (!CAUSAL && nq == 2 && q == 0 && j == 0) {
+                        if (elect_one()) tc_commit(&b_free[0]);
+                    }
                 }
                 if (elect_one()) tc_commit(&o_done[q]);
             }
@@ -412,30 +465,30 @@ mha_head_kernel(const __grid_constant__ HeadMaps maps, float *__restrict__ O, fl
 
     // The score tiles this group owns, packed: bit 0 query tile, 1 key tile, 2-3 S/P buffer, 4-5 index of the
     // p_full barrier, 6 slot in the exchange with the group that holds the other key tile of the same rows,
-    // 7 whether there is such a group, 8-9 parity of s_full[buffer] (0: the head's parity, 1: always 0, 2: always 1).
+    // 7 whether there is such a group, 8-9 parity of s_full[buffer] (0: the head's parity, 1: always 0, 2: always 1;
+    // RING: the group's own count of tiles).
+    // `turn`: the first of the head's tiles that this group owns.  RING: one less from head to head, the buffer stays the group's.
     auto mk = [](int q, int k, int buf, int ptile, int slot, int paired, int sp) {
         return (uint32_t)(q | (k << 1) | (buf << 2) | (ptile << 4) | (slot << 6) | (paired << 7) | (sp << 8));
     };
-    uint32_t job0 = 0, job1 = 0;
-    int njobs = 0;
-    if (nq == 1) {
-        if (grp == 0) { job0 = mk(0, 0, 0, 0, 0, 0, 0); njobs = 1; }
-    } else if (CAUSAL) {
-        njobs = 1;
-        job0 = grp == 0 ? mk(0, 0, 0, 0, 0, 0, 0) : grp == 1 ? mk(1, 0, 1, 1, 0, 1, 0) : mk(1, 1, 2, 2, 1, 1, 0);
-    } else {
+    int turn = grp, fills = 0;
+    auto job_of = [&](int ji) {
+        if (RING) {
+            const int t = ji ? 3 : turn;
+            return (CAUSAL || nq == 1) ? mk(0, 0, grp, grp, 0, 0, 0) : mk(t >> 1, t & 1, grp, grp, t & 1, 1, 0);
+        }
+        if (CAUSAL) return grp == 0 ? mk(0, 0, 0, 0, 0, 0, 0) : grp == 1 ? mk(1, 0, 1, 1, 0, 1, 0) : mk(1, 1, 2, 2, 1, 1, 0);
         // s_full[0] completes twice per head here: first for (q0, k0), then for (q1, k1)
-        njobs = grp == 0 ? 2 : 1;
-        job0 = grp == 0 ? mk(0, 0, 0, 0, 0, 1, 1) : grp == 1 ? mk(0, 1, 1, 1, 1, 1, 0) : mk(1, 0, 2, 2, 0, 1, 0);
-        job1 = mk(1, 1, 0, 3, 1, 1, 2);
-    }
+        if (ji) return mk(1, 1, 0, 3, 1, 1, 2);
+        return grp == 0 ? mk(0, 0, 0, 0, 0, 1, 1) : grp == 1 ? mk(0, 1, 1, 1, 1, 1, 0) : mk(1, 0, 2, 2, 0, 1, 0);
+    };
 
     // ---- conversion of K (group 0) or Q (group 1) for the head this block takes `itn`-th: thread = one row of each tile ----
-    auto convert_kq = [&](int itn) {
+    auto convert_kq = [&](int itn, int which) {      // which: 0 K, 1 Q
         const uint32_t parn = (uint32_t)(itn & 1);
         // K: [K_hi | K_lo];  Q: [Q_lo | Q].  hi = the 11 leading bits (exact in fp16), lo = x - hi.
-        uint8_t *raw = grp == 0 ? k_raw : q_raw, *dst16 = grp == 0 ? k_16 : q_16;
-        uint64_t *ld = grp == 0 ? ld_k : ld_q, *cv = grp == 0 ? cv_k : cv_q;
+        uint8_t *raw = which == 0 ? k_raw : q_raw, *dst16 = which == 0 ? k_16 : q_16;
+        uint64_t *ld = which == 0 ? ld_k : ld_q, *cv = which == 0 ? cv_k : cv_q;
         float amax = 0.0f;
         for (int t = 0; t < nq; ++t) {
             wait(&ld[t], parn, 1);
@@ -452,7 +505,7 @@ mha_head_kernel(const __grid_constant__ HeadMaps maps, float *__restrict__ O, fl
                                          fmaxf(fmaxf(fabsf(c4.x), fabsf(c4.y)), fmaxf(fabsf(c4.z), fabsf(c4.w)))));
                 const uint4 lo = make_uint4(pack_f16(a.x - ah.x, a.y - ah.y), pack_f16(a.z - ah.z, a.w - ah.w),
                                             pack_f16(c4.x - ch.x, c4.y - ch.y), pack_f16(c4.z - ch.z, c4.w - ch.w));
-                if (grp == 0) {
+                if (which == 0) {
                     *reinterpret_cast<uint4 *>(dst + sw128(rloc, pc)) =
                         make_uint4(pack_f16(ah.x, ah.y), pack_f16(ah.z, ah.w), pack_f16(ch.x, ch.y), pack_f16(ch.z, ch.w));
                     *reinterpret_cast<uint4 *>(dst + sw128(rloc, 4 + pc)) = lo;
@@ -466,13 +519,13 @@ mha_head_kernel(const __grid_constant__ HeadMaps maps, float *__restrict__ O, fl
                 // a NaN compares false everywhere: its bit pattern is what reaches the range test
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-                if (lane == 0) atomicMax(&s_amax[grp == 0 ? 1 : 0], __float_as_uint(amax));
+                if (lane == 0) atomicMax(&s_amax[which == 0 ? 1 : 0], __float_as_uint(amax));
             }
             proxy_fence();                       // generic-proxy writes -> visible to the tensor core
             arrive(&cv[t]);
         }
     };
-    if (grp < 2 && (int)blockIdx.x < BH) convert_kq(0);
+    if (grp < 2 && (int)blockIdx.x < BH) convert_kq(0, grp);
 
     int it = 0;
     float v_sc = 1.0f;                               // group 2: V's scale for the head about to be converted,
@@ -480,6 +533,8 @@ mha_head_kernel(const __grid_constant__ HeadMaps maps, float *__restrict__ O, fl
     for (int hd = blockIdx.x; hd < BH; hd += gridDim.x, ++it) {
         const uint32_t par = (uint32_t)(it & 1);
         const int b = hd / H, h = hd % H;
+        const bool has_next = hd + (int)gridDim.x < BH;
+        const int njobs = nq == 1 ? (turn == 0) : (!CAUSAL && turn == 0) ? 2 : 1;
 
         // ---- conversion of V (group 2): scaled by a power of two so that the head's largest magnitude lies in
         // [2^14, 2^15), then [V_hi | V_lo], before the group turns to its score tile.  (Placed between the
@@ -515,7 +570,7 @@ mha_head_kernel(const __grid_constant__ HeadMaps maps, float *__restrict__ O, fl
                 sc = __uint_as_float((uint32_t)(127 + sh) << 23);
                 inv = __uint_as_float((uint32_t)(127 - sh) << 23);
             }
-            if (tid == 2 * kTile) s_vinv[parn] = inv;
+            if ((tid & (kTile - 1)) == 0) s_vinv[itn & 3] = inv;
             return sc;
         };
         auto convert_v = [&](float sc) {
@@ -548,7 +603,11 @@ mha_head_kernel(const __grid_constant__ HeadMaps maps, float *__restrict__ O, fl
         };
         // (Letting the conversion wait until the group has swept its score tile for the row maxima, so that the group at
         // the other end of the exchange is not held up by it, measured slower: 15.42 against 15.30 us.)
-        if (grp == 2) {
+        // With the probabilities stored the raw V arrives late (its tiles are the probabilities' staging area).  Causal heads
+        // after the first then convert it behind the exponentials; unmasked ones cannot: the fourth score tile waits for a
+        // product with V, and this group's exponentials for that tile's maxima.
+        const bool v_late = PROBS && CAUSAL && nq == 2 && it > 0;
+        if (turn == 2 && !v_late) {
             if (!v_scale_known) v_sc = v_scale(it);
             v_scale_known = false;
             convert_v(v_sc);
@@ -561,10 +620,10 @@ mha_head_kernel(const __grid_constant__ HeadMaps maps, float *__restrict__ O, fl
         // columns [32c, 32c+16), its P_lo to [32c+16, 32c+32), so a chunk is rewritten where it was read.
         // The probabilities of one tile, normalised: P_hi + P_lo read back from TMEM, divided by the row's sum over all
         // of its tiles (P carries a factor 2^8, and so does the sum).  A worker holds a row, so its own stores would be
-        // 16-byte pieces S floats apart; the warp turns each 32 x 32 chunk through shared memory instead and stores four
-        // rows of 128 contiguous bytes per instruction.  The scratch is the first tile of the raw Q (group 0), of the fp16
-        // Q (group 1) or of the raw K (group 2): free once the products that read them have completed, which the caller
-        // has made sure of.  Chunks that no row of the warp sees are zeros.
+        // pieces of a row S floats apart (32 bytes per lane and instruction: 1.0 us per 32 columns of two tiles, against
+        // 0.3 for the arithmetic).  The warp lays each 32 x 32 chunk into its staging area in the 128-byte swizzle instead and one
+        // lane hands it to a TMA store, which clips it to the head's rows and columns; the next chunk is read and normalised
+        // meanwhile.  Chunks that no row of the warp sees are zeros, staged once.
         auto store_probs = [&](uint32_t job, float l_total) {
             const int q = job & 1, k = (job >> 1) & 1, buf = (job >> 2) & 3;
             const uint32_t s_addr = lane_base + (uint32_t)(buf * kTile);
@@ -574,67 +633,72 @@ mha_head_kernel(const __grid_constant__ HeadMaps maps, float *__restrict__ O, fl
             const int nwarp = diag ? min(ncols, eq * 32 + 32) : ncols;
             const int nch = (nwarp + 31) >> 5;
             const int wrow0 = q * kTile + eq * 32;              // first row of this warp
+            // a causal head's first query tile has no second key tile: those columns are zeros too
+            const int nout = CAUSAL && q == 0 ? S : ncols;
             const float inv = 1.0f / fmaxf(l_total, 1e-20f);
-            uint8_t *tb = (grp == 0 ? q_raw : grp == 1 ? q_16 : k_raw) + wq * 4096;   // [32 rows][128 bytes], 16-byte chunks swizzled by the row
-            float *pw = P + ((size_t)hd * S + wrow0) * (size_t)S + (size_t)k * kTile;
-            const bool vec = (S & 3) == 0;                      // then every group of four columns is 16-byte aligned
+            uint8_t *tb = warp < 8 ? v_raw + warp * kStageWarp : base + kOffStage + (warp - 8) * kStageWarp;
+            if (warp < 8) {                                     // the raw V has been read
+                wait(&cv_v[0], par, 2);
+                if (nq == 2) wait(&cv_v[1], par, 2);
+            }
+            if (wrow0 >= S) return;
+            bool zeroed = false;
+            const bool pairs = (S & 1) == 0 && (reinterpret_cast<uintptr_t>(P) & 7) == 0;
 #pragma unroll 1
-            for (int c = 0; c < 4; ++c) {
-                const int nleft = ncols - c * 32;               // columns of this chunk that exist
-                if (nleft <= 0) break;
-                if (c < nch) {
+            for (int c = 0; c * 32 < nout; ++c) {
+                if (c < nch || !zeroed) {
                     float w[32];
-                    tmem_ld32(s_addr + c * 32, w);              // 16 words of packed P_hi, then 16 of packed P_lo
-                    tmem_wait_ld();
+                    if (c < nch) {
+                        tmem_ld32(s_addr + c * 32, w);          // 16 words of packed P_hi, then 16 of packed P_lo
+                        tmem_wait_ld();
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) w[j] = 0.0f;
+                        zeroed = true;
+                    }
+                    float4 o[8];
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
-                        float o[4];
-#pragma unroll
-                        for (int i = 0; i < 2; ++i) {
-                            const __half2 hh = *reinterpret_cast<const __half2 *>(&w[2 * j + i]), ll = *reinterpret_cast<const __half2 *>(&w[16 + 2 * j + i]);
-                            o[2 * i] = (__low2float(hh) + __low2float(ll)) * inv;
-                            o[2 * i + 1] = (__high2float(hh) + __high2float(ll)) * inv;
-                        }
-                        *reinterpret_cast<float4 *>(tb + lane * 128 + ((j ^ (lane & 7)) << 4)) = make_float4(o[0], o[1], o[2], o[3]);
+                        const float2 a = f16_sum(w[2 * j], w[16 + 2 * j]), a2 = f16_sum(w[2 * j + 1], w[16 + 2 * j + 1]);
+                        o[j] = make_float4(a.x * inv, a.y * inv, a2.x * inv, a2.y * inv);
                     }
+                    if (p_mapped && lane == 0) bulk_wait_read();    // the chunk before has left
+                    __syncwarp();
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) *reinterpret_cast<float4 *>(tb + sw128(lane, j)) = o[j];
+                    if (p_mapped) proxy_fence();
+                    __syncwarp();
+                }
+                if (abort_flag) continue;
+                if (p_mapped) {
+                    if (lane == 0) tma_store_3d(&maps.p, tb, k * kTile + c * 32, wrow0, hd);
                 } else {
-#pragma unroll
-                    for (int j = 0; j < 8; ++j)
-                        *reinterpret_cast<float4 *>(tb + lane * 128 + ((j ^ (lane & 7)) << 4)) = make_float4(0.f, 0.f, 0.f, 0.f);
-                }
-                __syncwarp();
-                if (!abort_flag) {
-                    if (vec) {
-                        const int ch = lane & 7;                // 16-byte piece of a row
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) {
-                            const int rr = 4 * i + (lane >> 3);
-                            const float4 val = *reinterpret_cast<const float4 *>(tb + rr * 128 + ((ch ^ (rr & 7)) << 4));
-                            if (wrow0 + rr < S && 4 * ch < nleft) *reinterpret_cast<float4 *>(pw + (size_t)rr * S + c * 32 + 4 * ch) = val;
-                        }
-                    } else {
-                        for (int rr = 0; rr < 32 && wrow0 + rr < S; ++rr)
-                            if (lane < nleft)
-                                pw[(size_t)rr * S + c * 32 + lane] = *reinterpret_cast<const float *>(tb + rr * 128 + (((lane >> 2) ^ (rr & 7)) << 4) + (lane & 3) * 4);
+                    // rows that are not 16-byte aligned: pairs where S is even, else single elements
+                    float *pw = P + ((size_t)hd * S + wrow0) * (size_t)S + (size_t)(k * kTile + c * 32);
+                    const int nr = min(32, S - wrow0), left = S - (k * kTile + c * 32);
+                    if (pairs) {
+                        const int col = 2 * (lane & 15);
+                        if (col < left)
+#pragma unroll 4
+                            for (int rr = lane >> 4; rr < nr; rr += 2)
+                                *reinterpret_cast<float2 *>(pw + (size_t)rr * S + col) = *reinterpret_cast<const float2 *>(tb + sw128(rr, col >> 2) + (col & 3) * 4);
+                    } else if (lane < left) {
+#pragma unroll 4
+                        for (int rr = 0; rr < nr; ++rr) pw[(size_t)rr * S + lane] = *reinterpret_cast<const float *>(tb + sw128(rr, lane >> 2) + (lane & 3) * 4);
                     }
+                    __syncwarp();                               // the chunk is out before the next one is staged
                 }
-                __syncwarp();                                   // the chunk is out before the next one is staged
             }
-            // a causal head's first query tile has no second key tile: those columns are zeros
-            if (CAUSAL && q == 0 && k == 0 && !abort_flag)
-                for (int rr = 0; rr < 32 && wrow0 + rr < S; ++rr) {
-                    float *pr = P + ((size_t)hd * S + wrow0 + rr) * (size_t)S;
-                    if (vec) for (int col = kTile + 4 * lane; col < S; col += 128) *reinterpret_cast<float4 *>(pr + col) = make_float4(0.f, 0.f, 0.f, 0.f);
-                    else for (int col = kTile + lane; col < S; col += 32) pr[col] = 0.0f;
-                }
         };
         float lsum[2] = {0.0f, 0.0f};
 #pragma unroll 1
         for (int ji = 0; ji < njobs; ++ji) {
-            const uint32_t job = ji ? job1 : job0;
+            const uint32_t job = job_of(ji);
             const int q = job & 1, k = (job >> 1) & 1, buf = (job >> 2) & 3, ptile = (job >> 4) & 3, slot = (job >> 6) & 1;
             const bool paired = (job >> 7) & 1;
-            const uint32_t spar = ((job >> 8) & 3) == 0 ? par : ((job >> 8) & 3) - 1;   // parity of s_full[buf] for this tile
+            // parity of s_full[buf] for this tile
+            const uint32_t spar = RING ? (uint32_t)(fills & 1) : ((job >> 8) & 3) == 0 ? par : ((job >> 8) & 3) - 1;
+            if (RING) ++fills;
             const uint32_t s_addr = lane_base + (uint32_t)(buf * kTile);
             const int ncols = min(kTile, S - k * kTile);                      // keys of this tile that exist
             const bool diag = CAUSAL && q == k;
@@ -679,38 +743,52 @@ mha_head_kernel(const __grid_constant__ HeadMaps maps, float *__restrict__ O, fl
                 xsum[par][q][slot][rloc] = ps;
                 arrive(&xs[q]);
             }
-            if (ji) lsum[1] = ps; else lsum[0] = ps;
-            if (PROBS && !CAUSAL && njobs == 2 && ji == 0) {
-                // this tile's buffer is taken by the group's second tile: its probabilities leave now
+            // (RING: the sum is completed here, not at the output: the other groups may be in the next head by then)
+            if (paired && (RING || PROBS)) {
                 wait(&xs[q], par, 7);
-                store_probs(job, ps + xsum[par][q][slot ^ 1][rloc]);
+                ps += xsum[par][q][slot ^ 1][rloc];
+            }
+            if (ji) lsum[1] = ps; else lsum[0] = ps;
+            if (v_late && turn == 2) convert_v(v_scale(it));
+            if (PROBS) {
+                store_probs(job, ps);
                 tc_fence_before();
-                arrive(&pr_done);
+                arrive(&pr_read[buf]);
             }
         }
         // the next head's K and Q have landed by now (their copies were issued when this head's Q K^T had
         // completed): converting them here lets its Q K^T run while this head's output is stored
-        if (!PROBS && grp < 2 && hd + (int)gridDim.x < BH) convert_kq(it + 1);
-        if (!PROBS && grp == 2 && hd + (int)gridDim.x < BH) {
+        // (RING, two query tiles: both by the group that owns the second tile, the others have two tiles or a late one; one query
+        // tile: by the two groups without one)
+        if (has_next) {
+            if (!RING) {
+                if (grp < 2) convert_kq(it + 1, grp);
+            } else if (nq == 1) {
+                if (turn > 0) convert_kq(it + 1, turn - 1);
+            } else if (turn == 1) {
+#pragma unroll 1
+                for (int which = 0; which < 2; ++which) convert_kq(it + 1, which);
+            }
+        }
+        if (!PROBS && has_next && turn == (RING ? 0 : 2)) {      // the group that converts V for the next head
             v_sc = v_scale(it + 1);                  // the next head's raw V has landed (its copies were issued when this head's V had been converted)
             v_scale_known = true;
         }
         // ---- output: (P_hi V_hi + corrections) / (l * V's scale); the groups of a query tile share its columns ----
 #pragma unroll 1
         for (int ji = 0; ji < njobs; ++ji) {
-            const uint32_t job = ji ? job1 : job0;
+            const uint32_t job = job_of(ji);
             const int q = job & 1, slot = (job >> 6) & 1;
             const bool paired = (job >> 7) & 1;
             const int c0 = paired ? 16 * slot : 0, nc = paired ? 16 : 32;
             float l = ji ? lsum[1] : lsum[0];
-            if (paired) {
+            if (paired && !RING && !PROBS) {
                 wait(&xs[q], par, 7);
                 l += xsum[par][q][slot ^ 1][rloc];
             }
             wait(&o_done[q], par, 5);                    // every product of this head issued so far has completed
             tc_fence_after();
-            if (PROBS && !(!CAUSAL && njobs == 2 && ji == 0)) store_probs(job, l);
-            const float inv = (1.0f / fmaxf(l, 1e-20f)) * s_vinv[par];
+            const float inv = (1.0f / fmaxf(l, 1e-20f)) * s_vinv[it & 3];
             const int row = q * kTile + ((flip0 && q == 0) ? 3 - wq : wq) * 32 + lane;
             const bool store = !abort_flag && row < S;
             float4 *dst = reinterpret_cast<float4 *>(O + ((size_t)b * S + (row < S ? row : 0)) * (size_t)E + (size_t)h * 32);
@@ -729,22 +807,24 @@ mha_head_kernel(const __grid_constant__ HeadMaps maps, float *__restrict__ O, fl
                 }
             }
         }
+        if (njobs == 0) wait(&o_done[0], par, 5);        // nothing to read, but no further ahead than the groups that have
+        if (PROBS && p_mapped && lane == 0) bulk_wait_read();    // the next head's V may land on the staging area
         tc_fence_before();
         arrive(&epi_done);
-        // with the probabilities stored, shared memory of this head served as their staging area until now
-        if (PROBS && grp < 2 && hd + (int)gridDim.x < BH) convert_kq(it + 1);
+        if (RING) turn = turn == 0 ? 2 : turn - 1;
     }
+    if (PROBS && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     tc_fence_before();
     __syncthreads();
 }
 
 // ---- host side: tensor maps and the launch ---------------------------------------------------------
 
-template <bool CAUSAL, bool PROBS>
-int launch_head_cfg(const HeadMaps &maps, float *out, float *probs, int B, int S, int E, int H, cudaStream_t st)
+template <bool CAUSAL, bool PROBS, bool RING>
+int launch_head_cfg(const HeadMaps &maps, float *out, float *probs, int p_mapped, int B, int S, int E, int H, cudaStream_t st)
 {
-    auto kern = mha_head_kernel<CAUSAL, PROBS>;
-    const size_t smem = kHeadSmemBytes + 1024;
+    auto kern = mha_head_kernel<CAUSAL, PROBS, RING>;
+    const size_t smem = kHeadSmemBytes + (PROBS ? kStageBytes : 0) + 1024;
     static bool attr_set = false;                    // per instantiation; setting it twice is harmless
     if (!attr_set) {
         const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -758,7 +838,7 @@ int launch_head_cfg(const HeadMaps &maps, float *out, float *probs, int B, int S
     if (bh > 2147483647LL) return fail(HIPGPT_ERR_BAD_ARG, "%lld (batch, head) pairs are too many", bh);
     const unsigned grid = (unsigned)(bh < sms ? bh : sms);
     const float cscale = (1.0f / sqrtf(32.0f)) * kLog2e;
-    const cudaError_t le = launch_overlapped(kern, dim3(grid), dim3(kHeadThreads), smem, st, maps, out, probs, S, E, H, (int)bh, cscale);
+    const cudaError_t le = launch_overlapped(kern, dim3(grid), dim3(kHeadThreads), smem, st, maps, out, probs, S, E, H, (int)bh, cscale, p_mapped);
     if (le != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "mha_head_kernel launch: %s", cudaGetErrorString(le));
     return check_launch("mha_head_kernel");
 }
@@ -784,8 +864,23 @@ int launch_mha_head(const float *q, const float *k, const float *v, float *out, 
     if (rc == HIPGPT_OK) rc = tma_plane_map(&maps.k, k, B, S, E, kTile, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc == HIPGPT_OK) rc = tma_plane_map(&maps.v, v, B, S, E, kTile, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc != HIPGPT_OK) return rc;
-    if (probs) return causal ? launch_head_cfg<true, true>(maps, out, probs, B, S, E, H, st) : launch_head_cfg<false, true>(maps, out, probs, B, S, E, H, st);
-    return causal ? launch_head_cfg<true, false>(maps, out, nullptr, B, S, E, H, st) : launch_head_cfg<false, false>(maps, out, nullptr, B, S, E, H, st);
+    // rows of probabilities that TMA can address: the store by TMA; else element by element
+    const int p_mapped = probs && (S & 3) == 0 && (reinterpret_cast<uintptr_t>(probs) & 15) == 0;
+    if (p_mapped) {
+        rc = tma_plane_map(&maps.p, probs, B * H, S, S, 32, CU_TENSOR_MAP_SWIZZLE_128B);
+        if (rc != HIPGPT_OK) return rc;
+    }
+    // The ring where it is the faster order: a single query tile (three heads in flight instead of one: 27.5 -> 25.6 us at B=64 H=16
+    // S=100 unmasked), and unmasked heads whose probabilities are stored (30.8 -> 30.2 us at B=32 H=8 S=256, 52.6 -> 49.7 at B=40 H=12
+    // S=200).  Unmasked without them it is the slower one (21.7 against 21.0 us): the next head's first two tiles both
+    // need groups that are still busy with this head's output.
+    auto go = [&](auto kernel_of) { return kernel_of(maps, out, probs, p_mapped, B, S, E, H, st); };
+    if (S <= kTile) {
+        if (probs) return causal ? go(launch_head_cfg<true, true, true>) : go(launch_head_cfg<false, true, true>);
+        return causal ? go(launch_head_cfg<true, false, true>) : go(launch_head_cfg<false, false, true>);
+    }
+    if (probs) return causal ? go(launch_head_cfg<true, true, false>) : go(launch_head_cfg<false, true, true>);
+    return causal ? go(launch_head_cfg<true, false, false>) : go(launch_head_cfg<false, false, false>);
 }
 
 // Reads and clears a status word of this file.

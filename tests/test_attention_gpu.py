@@ -49,6 +49,21 @@ def test_mha_matches_oracle(shape, causal, want_probs):
             assert np.all(np.triu(probs, 1) == 0.0)
 
 
+@pytest.mark.parametrize("S", [1, 6, 31, 100, 128, 129, 198, 231, 256])
+@pytest.mark.parametrize("causal", [False, True])
+def test_whole_head_kernel_many_heads_per_block(S, causal):
+    """Several heads in sequence per block (more heads than three times the SMs): one query tile and two, rows of probabilities
+    stored by TMA (S a multiple of four), in pairs and element by element."""
+    B, H, D = 60, 8, 32
+    E = H * D
+    qkv = synth.qkv_planes(70 + S, B, S, E)
+    ref_out, ref_probs = ob.mha(qkv, B, S, E, H, causal=causal, want_probs=True)
+    out, probs = gpu_mha(qkv, B, S, E, H, causal, True)
+    plain, _ = gpu_mha(qkv, B, S, E, H, causal, False)
+    assert _maxerr(out, ref_out) <= TOL and _maxerr(probs, ref_probs) <= TOL
+    np.testing.assert_array_equal(out, plain)
+
+
 @pytest.mark.parametrize("warps", [1, 2, 4])
 @pytest.mark.parametrize("D", [32, 64, 128])
 @pytest.mark.parametrize("causal", [False, True])
