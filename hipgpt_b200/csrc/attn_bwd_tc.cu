@@ -195,9 +195,17 @@ __device__ __forceinline__ void add_tile(uint32_t acc, int hf, float (&o)[D / 2]
 template <int D>
 __device__ __forceinline__ void store_out(const float (&o)[D / 2], int hf, float scale, float *dst)
 {
+    dst += hf * (D / 2);
+    if ((reinterpret_cast<uintptr_t>(dst) & 31) == 0) {          // rows are whole 32-byte sectors apart: one store per sector
 #pragma unroll
-    for (int c = 0; c < D / 2; c += 4)
-        *reinterpret_cast<float4 *>(dst + hf * (D / 2) + c) = make_float4(o[c] * scale, o[c + 1] * scale, o[c + 2] * scale, o[c + 3] * scale);
+        for (int c = 0; c < D / 2; c += 8)
+            asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst + c), "f"(o[c] * scale), "f"(o[c + 1] * scale), "f"(o[c + 2] * scale),
+                         "f"(o[c + 3] * scale), "f"(o[c + 4] * scale), "f"(o[c + 5] * scale), "f"(o[c + 6] * scale), "f"(o[c + 7] * scale) : "memory");
+    } else {
+#pragma unroll
+        for (int c = 0; c < D / 2; c += 4)
+            *reinterpret_cast<float4 *>(dst + c) = make_float4(o[c] * scale, o[c + 1] * scale, o[c + 2] * scale, o[c + 3] * scale);
+    }
 }
 
 // ---- rows: log-sum-exp, w, dQ --------------------------------------------------------------------------
@@ -248,6 +256,7 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     dependency_wait();
+    dependents_may_start();                          // the columns' blocks take the SMs that run out of rows, up to where they need w
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -286,8 +295,8 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         };
         if (first) {
             if (lane == 0) {
-                mbar_arrive_expect_tx(&res_full, 4 * TB);
-                bulk_load(q_s, q_img, 2 * TB, &res_full);
+                mbar_arrive_expect_tx(&res_full, (STORED ? 2 : 4) * TB);
+                if (!STORED) bulk_load(q_s, q_img, 2 * TB, &res_full);
                 bulk_load(g_s, g_img, 2 * TB, &res_full);
             }
             __syncwarp();
@@ -546,7 +555,8 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)), "r"(kTmemCols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    dependency_wait();
+    // No wait for the kernel before yet: the probabilities and the images are older than that one (it waited for the
+    // packing before it let this one start); the workers wait for it where they first read w and lse.
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -574,8 +584,8 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         };
         if (first) {
             if (lane == 0) {
-                mbar_arrive_expect_tx(&res_full, 4 * TB);
-                bulk_load(k_s, k_img, 2 * TB, &res_full);
+                mbar_arrive_expect_tx(&res_full, (STORED ? 2 : 4) * TB);
+                if (!STORED) bulk_load(k_s, k_img, 2 * TB, &res_full);
                 bulk_load(v_s, v_img, 2 * TB, &res_full);
             }
             __syncwarp();
@@ -651,6 +661,7 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         add_tile<D, C::kWide>(lane_base + C::kColK, hf, ok);
     };
     if (STORED) fetch_p(0);
+    dependency_wait();
     for (int i = 0; i < total; ++i) {
         const uint32_t s_addr = lane_base + (uint32_t)(i & 1) * C::kBuf + hf * 32, dp_addr = s_addr + kTile, room = s_addr + 2 * kTile;
         const int qb = (t0 + i) * kTile + hf * 32;
