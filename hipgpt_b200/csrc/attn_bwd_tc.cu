@@ -25,8 +25,10 @@
 // block raises a flag that cuts later waits short, records a status code, skips its stores, frees its TMEM and returns.
 #include "stream_workspace.hpp"
 #include "tc_primitives.cuh"
+#include "tma_host.cuh"
 
 #include <math.h>
+#include <type_traits>
 
 namespace hipgpt {
 namespace {
@@ -209,26 +211,38 @@ __device__ __forceinline__ void store_out(const float (&o)[D / 2], int hf, float
 }
 
 // ---- rows: log-sum-exp, w, dQ --------------------------------------------------------------------------
-template <int D, bool STORED>
+// STORED: where the probabilities come from.  0: formed again from Q and K.  1: the caller's, one tile ahead through registers
+// (rows that TMA cannot address: S not a multiple of four).  2: the caller's, by TMA into a ring of tiles: a tile of
+// the first sweep took 1.2 us, which was the latency of the loads one tile ahead; no registers and no turning are needed
+// either (B=32 H=8 S=256 D=32: 109.9 -> 102.5 us, B=2 H=16 S=1024 D=64: 258 -> 212).
+constexpr int kPTile = kLanes * kTile * 4;           // bytes of a tile of probabilities
+template <int STORED>
+using PMap = std::conditional_t<STORED == 2, CUtensorMap, int>;
+template <int D>
+constexpr int kPStages = D == 32 ? 3 : 2;
+
+template <int D, int STORED>
 struct RowsCfg {
-    static constexpr int kKStages = D == 32 ? 4 : (STORED ? 2 : 3);      // what 227 KB hold beside Q, dO and the staged probabilities
+    static constexpr int kKStages = D == 32 ? 4 : (STORED ? 2 : 3);      // what 227 KB hold beside Q, dO and the probabilities
     static constexpr int kVStages = D == 32 ? 4 : 2;
-    static constexpr int kResident = 2 * 2 * Img<D>::kTileBytes;         // Q and dO, 128 rows each
-    static constexpr int kStage = STORED ? kWorkerWarps * 4096 : 0;      // per warp 32 rows x 32 probabilities on their way to their rows
-    static constexpr size_t kSmem = (size_t)kResident + (kKStages + kVStages) * Img<D>::kTileBytes + kStage;
+    static constexpr int kResident = (STORED ? 1 : 2) * 2 * Img<D>::kTileBytes;      // dO and, to form P again, Q: 128 rows each
+    // 1: per warp 32 rows x 32 probabilities on their way to their rows
+    static constexpr int kStage = STORED == 2 ? kPStages<D> * kPTile : STORED == 1 ? kWorkerWarps * 4096 : 0;
+    static constexpr size_t kSmem = (STORED == 2 ? 1024 : 0) + (size_t)kResident + (kKStages + kVStages) * Img<D>::kTileBytes + kStage;
     static constexpr uint32_t kColAcc = 4 * kTile;                       // after two buffers of S and dP: two accumulators of 2 D columns
 };
 
-template <int D, bool CAUSAL, bool STORED>
+template <int D, bool CAUSAL, int STORED>
 __global__ void __launch_bounds__(kThreads, 1)
 bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *__restrict__ P, float *__restrict__ dQ,
-                float *__restrict__ lse_out, float *__restrict__ w_out, int S, int Spad, int E, int H, int nblk, float c)
+                float *__restrict__ lse_out, float *__restrict__ w_out, int S, int Spad, int E, int H, int nblk, float c, const __grid_constant__ PMap<STORED> p_map)
 {
     using C = RowsCfg<D, STORED>;
     constexpr int TB = Img<D>::kTileBytes;
-    extern __shared__ __align__(128) uint8_t smem[];
-    uint8_t *q_s = smem, *g_s = q_s + 2 * TB, *k_s = g_s + 2 * TB, *v_s = k_s + C::kKStages * TB, *p_s = v_s + C::kVStages * TB;
-    __shared__ uint64_t res_full, k_full[C::kKStages], v_full[C::kVStages], sd_full[2], ready[2], acc_done[2];
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    uint8_t *p_s = STORED == 2 ? reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023) : smem_raw;
+    uint8_t *q_s = p_s + C::kStage, *g_s = q_s + (STORED ? 0 : 2 * TB), *k_s = g_s + 2 * TB, *v_s = k_s + C::kKStages * TB;
+    __shared__ uint64_t res_full, k_full[C::kKStages], v_full[C::kVStages], sd_full[2], ready[2], acc_done[2], p_full[STORED == 2 ? kPStages<D> : 1];
     __shared__ float comb[2][STORED ? 1 : 3][kLanes];           // w and, where P is formed again, maximum and sum of each half row
     __shared__ uint32_t tmem_base_slot;
     __shared__ volatile int abort_flag;
@@ -249,6 +263,7 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         mbar_init(&res_full, 1);
         for (int i = 0; i < C::kKStages; ++i) mbar_init(&k_full[i], 1);
         for (int i = 0; i < C::kVStages; ++i) mbar_init(&v_full[i], 1);
+        if (STORED == 2) for (int i = 0; i < kPStages<D>; ++i) mbar_init(&p_full[i], 1);
         for (int i = 0; i < 2; ++i) { mbar_init(&sd_full[i], STORED ? 1 : 2); mbar_init(&ready[i], kWorkerWarps); mbar_init(&acc_done[i], 2); }      // (commits: one per issuing warp)
     }
     if (warp == kWorkerWarps) {
@@ -261,7 +276,7 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_base_slot;
-    // site codes: 1 resident operands, 2 K tile, 3 V tile, 4 scores, 5 workers at a tile, 6 accumulation
+    // site codes: 1 resident operands, 2 K tile, 3 V tile, 4 scores, 5 workers at a tile, 6 accumulation, 7 probabilities
     auto wait = [&](uint64_t *bar, uint32_t parity, int site) {
         if (abort_flag || mbar_test(bar, parity)) return;
         bwd_wait_slow(bar, parity, site, &abort_flag);
@@ -293,6 +308,17 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
             }
             __syncwarp();
         };
+        // 128 rows x 64 probabilities in two boxes of 32 columns (rows and columns past S arrive as zeros)
+        auto fetch_p = [&](int i) {
+            if (lane == 0 && i < total) {
+                uint64_t *bar = &p_full[i % kPStages<D>];
+                uint8_t *dst = p_s + (i % kPStages<D>) * kPTile;
+                mbar_arrive_expect_tx(bar, kPTile);
+                tma_load_3d(dst, &p_map, (i % nk) * kTile, q0, bh, bar);
+                tma_load_3d(dst + kPTile / 2, &p_map, (i % nk) * kTile + 32, q0, bh, bar);
+            }
+            __syncwarp();
+        };
         if (first) {
             if (lane == 0) {
                 mbar_arrive_expect_tx(&res_full, (STORED ? 2 : 4) * TB);
@@ -300,6 +326,7 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
                 bulk_load(g_s, g_img, 2 * TB, &res_full);
             }
             __syncwarp();
+            if (STORED == 2) for (int i = 0; i < kPStages<D>; ++i) fetch_p(i);
             for (int i = 0; i < C::kKStages; ++i) fetch_k(k_first + i);
         } else {
             for (int i = 0; i < C::kVStages; ++i) fetch_v(i);
@@ -330,6 +357,7 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
             if (i + 1 < total) issue_sd(i + 1);
             wait(&ready[i & 1], (uint32_t)((i >> 1) & 1), 5);
             tc_fence_after();
+            if (STORED == 2 && first) fetch_p(i + kPStages<D>);      // the workers have read tile i of the probabilities
             if (!first) fetch_v(i + C::kVStages);    // the scores of tile i have been read, so the products that read V have completed
             if (i < nk) {
                 if (!STORED && first) fetch_k(i + C::kKStages);
@@ -360,51 +388,38 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         __syncwarp();
         if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
     };
-    // The stored probabilities of this warp's 32 rows x 32 columns: read with whole lines (eight lanes per row), turned to
-    // their rows through shared memory (16-byte pieces, permuted by the row: no bank conflicts).
-    const bool vec = STORED && (S & 3) == 0;         // (the pointer is 16-byte aligned)
-    uint8_t *turn = p_s + warp * 4096;
-    const float *p_rows = STORED ? P + ((size_t)bh * S + q0 + wq * 32) * S : nullptr;
-    float4 pf[8];
+    // The stored probabilities of this thread's row.  1: a warp reads 32 rows x 32 columns a row per load, and turns them to their
+    // rows through shared memory (16-byte pieces, permuted by the row: no bank conflicts).
+    const float *p_rows = STORED == 1 ? P + ((size_t)bh * S + q0 + wq * 32) * S : nullptr;
+    float pf[STORED == 1 ? 32 : 1];
     auto fetch_p = [&](int i) {
         const int j0 = (i % nk) * kTile + hf * 32;
-        if (vec && q0 + wq * 32 + 32 <= S && j0 + 32 <= S) {
-            const float *src = p_rows + (size_t)(lane >> 3) * S + j0 + (lane & 7) * 4;
+        // (a lane past S reads its neighbour's column: dP is zero there, and ds is set to zero)
+        const float *src = p_rows + min(j0 + lane, S - 1);
+        if (q0 + wq * 32 + 32 <= S) {
 #pragma unroll
-            for (int u = 0; u < 8; ++u, src += 4 * S) pf[u] = __ldg(reinterpret_cast<const float4 *>(src));
-        } else if (vec) {
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int r = u * 4 + (lane >> 3), j = j0 + (lane & 7) * 4;
-                pf[u] = (q0 + wq * 32 + r < S && j < S) ? __ldg(reinterpret_cast<const float4 *>(p_rows + (size_t)r * S + j)) : make_float4(0.f, 0.f, 0.f, 0.f);
-            }
+            for (int r = 0; r < 32; ++r, src += S) pf[STORED == 1 ? r : 0] = __ldg(src);
         } else {
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                float *e = reinterpret_cast<float *>(&pf[u]);
-#pragma unroll
-                for (int x = 0; x < 4; ++x) {
-                    const int r = u * 4 + x;
-                    e[x] = (q0 + wq * 32 + r < S && j0 + lane < S) ? __ldg(p_rows + (size_t)r * S + j0 + lane) : 0.0f;
-                }
-            }
+            for (int r = 0; r < 32; ++r, src += S) pf[STORED == 1 ? r : 0] = q0 + wq * 32 + r < S ? __ldg(src) : 0.0f;
         }
     };
-    auto turn_p = [&](float (&p)[32]) {
-        __syncwarp();
-        if (vec) {
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int r = u * 4 + (lane >> 3);
-                *reinterpret_cast<float4 *>(turn + sw128(r, lane & 7)) = pf[u];
-            }
+    auto take_p = [&](int i, float (&p)[32]) {
+        const uint8_t *src = p_s + (i % kPStages<D>) * kPTile + hf * (kPTile / 2);
+        int r0 = rloc;
+        if (STORED == 2) {
+            wait(&p_full[i % kPStages<D>], (uint32_t)((i / kPStages<D>) & 1), 7);
         } else {
+            uint8_t *turn = p_s + warp * 4096;
+            __syncwarp();
 #pragma unroll
-            for (int r = 0; r < 32; ++r) *reinterpret_cast<float *>(turn + sw128(r, lane >> 2) + (lane & 3) * 4) = reinterpret_cast<const float *>(&pf[r >> 2])[r & 3];
+            for (int r = 0; r < 32; ++r) *reinterpret_cast<float *>(turn + sw128(r, lane >> 2) + (lane & 3) * 4) = pf[STORED == 1 ? r : 0];
+            __syncwarp();
+            src = turn;
+            r0 = lane;
         }
-        __syncwarp();
 #pragma unroll
-        for (int ch = 0; ch < 8; ++ch) *reinterpret_cast<float4 *>(&p[ch * 4]) = *reinterpret_cast<const float4 *>(turn + sw128(lane, ch));
+        for (int ch = 0; ch < 8; ++ch) *reinterpret_cast<float4 *>(&p[ch * 4]) = *reinterpret_cast<const float4 *>(src + sw128(r0, ch));
     };
 
     float m = -INFINITY, l = 0.0f, w = 0.0f, lse = 0.0f;
@@ -417,7 +432,7 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         add_tile<D, true>(lane_base + C::kColAcc, hf, o);
         add_tile<D, true>(lane_base + C::kColAcc + 2 * D, hf, o);
     };
-    if (STORED) fetch_p(0);
+    if (STORED == 1) fetch_p(0);
     for (int i = 0; i < total; ++i) {
         const uint32_t s_addr = lane_base + (uint32_t)((i & 1) * 2 * kTile) + hf * 32, dp_addr = s_addr + kTile;
         const int j0 = (i % nk) * kTile + hf * 32;
@@ -446,8 +461,8 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
             }
         }
         if (STORED) {
-            turn_p(s);
-            if (i + 1 < total) fetch_p(i + 1);       // in flight during this tile
+            take_p(i, s);
+            if (STORED == 1 && i + 1 < total) fetch_p(i + 1);       // in flight during this tile
         }
         wait(&sd_full[i & 1], (uint32_t)((i >> 1) & 1), 4);
         tc_fence_after();
@@ -514,26 +529,28 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
 }
 
 // ---- columns: dK, dV -----------------------------------------------------------------------------------
-template <int D>
+template <int D, int STORED>
 struct ColsCfg {
     static constexpr int kStages = D == 32 ? 4 : 2;                      // (Q, dO) tile pairs
-    static constexpr int kResident = 2 * 2 * Img<D>::kTileBytes;         // K and V, 128 rows each
-    static constexpr size_t kSmem = (size_t)kResident + kStages * 2 * Img<D>::kTileBytes;
+    static constexpr int kResident = (STORED ? 1 : 2) * 2 * Img<D>::kTileBytes;      // V and, to form P again, K: 128 rows each
+    static constexpr int kStage = STORED == 2 ? kPStages<D> * kPTile : 0;
+    static constexpr size_t kSmem = (STORED == 2 ? 1024 : 0) + (size_t)kResident + kStages * 2 * Img<D>::kTileBytes + kStage;
     static constexpr uint32_t kBuf = 3 * kTile;                          // S^T, dP^T and room: six pieces take 192 columns
     static constexpr uint32_t kColV = 2 * kBuf, kColK = kColV + 64;
     static constexpr bool kWide = D == 32;                               // 64 columns per accumulator
 };
 
-template <int D, bool CAUSAL, bool STORED>
+template <int D, bool CAUSAL, int STORED>
 __global__ void __launch_bounds__(kThreads, 1)
 bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *__restrict__ P, float *__restrict__ dK, float *__restrict__ dV,
-                const float *__restrict__ lse_in, const float *__restrict__ w_in, int S, int Spad, int E, int H, int nblk, float c)
+                const float *__restrict__ lse_in, const float *__restrict__ w_in, int S, int Spad, int E, int H, int nblk, float c, const __grid_constant__ PMap<STORED> p_map)
 {
-    using C = ColsCfg<D>;
+    using C = ColsCfg<D, STORED>;
     constexpr int TB = Img<D>::kTileBytes;
-    extern __shared__ __align__(128) uint8_t smem[];
-    uint8_t *k_s = smem, *v_s = k_s + 2 * TB, *t_s = v_s + 2 * TB;       // t_s: [stage][Q tile | dO tile]
-    __shared__ uint64_t res_full, full[C::kStages], sd_full[2], ready[2], acc_done[2];
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    uint8_t *p_s = STORED == 2 ? reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023) : smem_raw;
+    uint8_t *k_s = p_s + C::kStage, *v_s = k_s + (STORED ? 0 : 2 * TB), *t_s = v_s + 2 * TB;     // t_s: [stage][Q tile | dO tile]
+    __shared__ uint64_t res_full, full[C::kStages], sd_full[2], ready[2], acc_done[2], p_full[STORED == 2 ? kPStages<D> : 1];
     __shared__ uint32_t tmem_base_slot;
     __shared__ volatile int abort_flag;
 
@@ -549,6 +566,7 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         abort_flag = 0;
         mbar_init(&res_full, 1);
         for (int i = 0; i < C::kStages; ++i) mbar_init(&full[i], 1);
+        if (STORED == 2) for (int i = 0; i < kPStages<D>; ++i) mbar_init(&p_full[i], 1);
         for (int i = 0; i < 2; ++i) { mbar_init(&sd_full[i], STORED ? 1 : 2); mbar_init(&ready[i], kWorkerWarps); mbar_init(&acc_done[i], 2); }      // (commits: one per issuing warp)
     }
     if (warp == kWorkerWarps) {
@@ -561,7 +579,7 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_base_slot;
-    // site codes: 11 resident operands, 12 tile pair, 14 scores, 15 workers at a tile, 16 accumulation
+    // site codes: 11 resident operands, 12 tile pair, 14 scores, 15 workers at a tile, 16 accumulation, 17 probabilities
     auto wait = [&](uint64_t *bar, uint32_t parity, int site) {
         if (abort_flag || mbar_test(bar, parity)) return;
         bwd_wait_slow(bar, parity, site, &abort_flag);
@@ -582,6 +600,16 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
             }
             __syncwarp();
         };
+        // 64 queries x 128 probabilities in four boxes of 32 columns (a box per lane quarter)
+        auto fetch_p = [&](int i) {
+            if (lane == 0 && i < total) {
+                uint64_t *bar = &p_full[i % kPStages<D>];
+                uint8_t *dst = p_s + (i % kPStages<D>) * kPTile;
+                mbar_arrive_expect_tx(bar, kPTile);
+                for (int u = 0; u < 4; ++u) tma_load_3d(dst + u * (kPTile / 4), &p_map, k0 + 32 * u, (t0 + i) * kTile, bh, bar);
+            }
+            __syncwarp();
+        };
         if (first) {
             if (lane == 0) {
                 mbar_arrive_expect_tx(&res_full, (STORED ? 2 : 4) * TB);
@@ -589,7 +617,14 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
                 bulk_load(v_s, v_img, 2 * TB, &res_full);
             }
             __syncwarp();
-            for (int i = 0; i < C::kStages; ++i) fetch(i);
+            if (STORED == 2) {
+                for (int i = 0; i < C::kStages; ++i) {
+                    fetch(i);
+                    if (i < kPStages<D>) fetch_p(i);
+                }
+            } else {
+                for (int i = 0; i < C::kStages; ++i) fetch(i);
+            }
         }
         auto issue_sd = [&](int i) {
             if (STORED && first) return;
@@ -612,6 +647,7 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
             if (STORED && first) wait(&full[i % C::kStages], (uint32_t)((i / C::kStages) & 1), 12);
             wait(&ready[i & 1], (uint32_t)((i >> 1) & 1), 15);
             tc_fence_after();
+            if (STORED == 2 && first) fetch_p(i + kPStages<D>);      // the workers have read tile i of the probabilities
             const uint32_t s0 = tmem + (uint32_t)(i & 1) * C::kBuf, t = smem_u32(t_s + (i % C::kStages) * 2 * TB);
             auto p_col = [&](int p, int hf) { return p == 2 ? s0 + kTile + 32 * hf : s0 + 32 * hf + 16 * p; };
             auto ds_col = [&](int p, int hf) { return p == 0 ? s0 + kTile + 32 * hf + 16 : s0 + 2 * kTile + 32 * hf + 16 * (p - 1); };
@@ -637,7 +673,7 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
     };
     const float *wrow = w_in + (size_t)bh * Spad, *lrow = lse_in + (size_t)bh * Spad;
-    float pn[32];                                    // stored probabilities of the tile ahead: a query's are contiguous over the keys (lanes)
+    float pn[STORED == 1 ? 32 : 1];                  // stored probabilities of the tile ahead: a query's are contiguous over the keys (lanes)
     auto fetch_p = [&](int i) {
         const int qb = (t0 + i) * kTile + hf * 32;
         // a lane past S reads its neighbour's key (its results go nowhere): no load depends on the lane, and in a full tile none
@@ -645,10 +681,10 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         const float *src = P + ((size_t)bh * S + qb) * S + min(key, S - 1);
         if (qb + 32 <= S) {
 #pragma unroll
-            for (int x = 0; x < 32; ++x, src += S) pn[x] = __ldg(src);
+            for (int x = 0; x < 32; ++x, src += S) pn[STORED == 1 ? x : 0] = __ldg(src);
         } else {
 #pragma unroll
-            for (int x = 0; x < 32; ++x, src += S) pn[x] = qb + x < S ? __ldg(src) : 0.0f;
+            for (int x = 0; x < 32; ++x, src += S) pn[STORED == 1 ? x : 0] = qb + x < S ? __ldg(src) : 0.0f;
         }
     };
     float ok[D / 2], ov[D / 2];
@@ -660,17 +696,23 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         add_tile<D, C::kWide>(lane_base + C::kColV, hf, ov);
         add_tile<D, C::kWide>(lane_base + C::kColK, hf, ok);
     };
-    if (STORED) fetch_p(0);
+    if (STORED == 1) fetch_p(0);
     dependency_wait();
     for (int i = 0; i < total; ++i) {
         const uint32_t s_addr = lane_base + (uint32_t)(i & 1) * C::kBuf + hf * 32, dp_addr = s_addr + kTile, room = s_addr + 2 * kTile;
         const int qb = (t0 + i) * kTile + hf * 32;
         const bool mask = CAUSAL && qb < k0 + wq * 32 + 31;              // some lane of the warp has a key after some query
         float p[32], d[32];
-        if (STORED) {
+        if (STORED == 1) {
 #pragma unroll
-            for (int x = 0; x < 32; ++x) p[x] = pn[x];
+            for (int x = 0; x < 32; ++x) p[x] = pn[STORED == 1 ? x : 0];
             if (i + 1 < total) fetch_p(i + 1);       // in flight during this tile
+        }
+        if (STORED == 2) {
+            wait(&p_full[i % kPStages<D>], (uint32_t)((i / kPStages<D>) & 1), 17);
+            const uint8_t *src = p_s + (i % kPStages<D>) * kPTile + wq * (kPTile / 4) + (lane & 3) * 4;
+#pragma unroll
+            for (int x = 0; x < 32; ++x) p[x] = *reinterpret_cast<const float *>(src + sw128(hf * 32 + x, lane >> 2));
         }
         wait(&sd_full[i & 1], (uint32_t)((i >> 1) & 1), 14);
         tc_fence_after();
@@ -714,13 +756,13 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
 
 StreamWorkspace g_bwd_ws;
 
-template <int D, bool CAUSAL, bool STORED>
+template <int D, bool CAUSAL, int STORED>
 int launch_cfg(const float *g, const float *q, const float *k, const float *v, const float *probs, float *dq, float *dk, float *dv,
                int B, int S, int E, int H, cudaStream_t st)
 {
     auto rows = bwd_rows_kernel<D, CAUSAL, STORED>;
     auto cols = bwd_cols_kernel<D, CAUSAL, STORED>;
-    constexpr size_t rows_smem = RowsCfg<D, STORED>::kSmem, cols_smem = ColsCfg<D>::kSmem;
+    constexpr size_t rows_smem = RowsCfg<D, STORED>::kSmem, cols_smem = ColsCfg<D, STORED>::kSmem;
     static_assert(rows_smem + (STORED ? 1 : 3) * 2 * kLanes * 4 + 256 <= 232448 && cols_smem + 256 <= 232448, "shared memory of a block");
     cudaError_t e = cudaFuncSetAttribute(rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(cols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cols_smem);
@@ -745,11 +787,17 @@ int launch_cfg(const float *g, const float *q, const float *k, const float *v, c
         const int tasks = nb * H * (Spad / 8) * (D / 32);
         e = launch_overlapped(bwd_pack_kernel<D>, dim3((unsigned)((tasks + 7) / 8), 4), dim3(256), 0, st, q + off, k + off, v + off, g + off, img, img_bytes, S, Spad, E, H, tasks);
         if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "bwd_pack_kernel launch: %s", cudaGetErrorString(e));
+        PMap<STORED> rows_map = {}, cols_map = {};
+        if constexpr (STORED == 2) {
+            rc = tma_plane_map(&rows_map, p, nb * H, S, S, kLanes, CU_TENSOR_MAP_SWIZZLE_128B);
+            if (rc == HIPGPT_OK) rc = tma_plane_map(&cols_map, p, nb * H, S, S, kTile, CU_TENSOR_MAP_SWIZZLE_128B);
+            if (rc != HIPGPT_OK) return rc;
+        }
         const dim3 grid((unsigned)(nb * H * nblk));
-        e = launch_overlapped(rows, grid, dim3(kThreads), rows_smem, st, (const uint8_t *)img, img_bytes, p, dq + off, lse, w, S, Spad, E, H, nblk, c);
+        e = launch_overlapped(rows, grid, dim3(kThreads), rows_smem, st, (const uint8_t *)img, img_bytes, p, dq + off, lse, w, S, Spad, E, H, nblk, c, rows_map);
         if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "bwd_rows_kernel launch: %s", cudaGetErrorString(e));
         e = launch_overlapped(cols, grid, dim3(kThreads), cols_smem, st, (const uint8_t *)img, img_bytes, p, dk + off, dv + off, (const float *)lse,
-                              (const float *)w, S, Spad, E, H, nblk, c);
+                              (const float *)w, S, Spad, E, H, nblk, c, cols_map);
         if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "bwd_cols_kernel launch: %s", cudaGetErrorString(e));
     }
     return HIPGPT_OK;
@@ -772,16 +820,13 @@ bool mha_backward_tc_supports(const void *g, const void *q, const void *k, const
 int launch_mha_backward_tc(const float *g, const float *q, const float *k, const float *v, const float *probs, float *dq, float *dk, float *dv,
                            int B, int S, int E, int H, int causal, cudaStream_t st)
 {
-    switch ((E / H == 64 ? 4 : 0) | (causal ? 2 : 0) | (probs ? 1 : 0)) {
-    case 0: return launch_cfg<32, false, false>(g, q, k, v, probs, dq, dk, dv, B, S, E, H, st);
-    case 1: return launch_cfg<32, false, true>(g, q, k, v, probs, dq, dk, dv, B, S, E, H, st);
-    case 2: return launch_cfg<32, true, false>(g, q, k, v, probs, dq, dk, dv, B, S, E, H, st);
-    case 3: return launch_cfg<32, true, true>(g, q, k, v, probs, dq, dk, dv, B, S, E, H, st);
-    case 4: return launch_cfg<64, false, false>(g, q, k, v, probs, dq, dk, dv, B, S, E, H, st);
-    case 5: return launch_cfg<64, false, true>(g, q, k, v, probs, dq, dk, dv, B, S, E, H, st);
-    case 6: return launch_cfg<64, true, false>(g, q, k, v, probs, dq, dk, dv, B, S, E, H, st);
-    default: return launch_cfg<64, true, true>(g, q, k, v, probs, dq, dk, dv, B, S, E, H, st);
-    }
+    // probabilities whose rows TMA can address (the pointer is 16-byte aligned)
+    const int stored = !probs ? 0 : (S & 3) == 0 && tma_encode_fn() != nullptr ? 2 : 1;
+    auto go = [&](auto launch) { return launch(g, q, k, v, probs, dq, dk, dv, B, S, E, H, st); };
+    auto pick = [&](auto l0, auto l1, auto l2) { return stored == 0 ? go(l0) : stored == 1 ? go(l1) : go(l2); };
+    if (E / H == 64)
+        return causal ? pick(launch_cfg<64, true, 0>, launch_cfg<64, true, 1>, launch_cfg<64, true, 2>) : pick(launch_cfg<64, false, 0>, launch_cfg<64, false, 1>, launch_cfg<64, false, 2>);
+    return causal ? pick(launch_cfg<32, true, 0>, launch_cfg<32, true, 1>, launch_cfg<32, true, 2>) : pick(launch_cfg<32, false, 0>, launch_cfg<32, false, 1>, launch_cfg<32, false, 2>);
 }
 
 void mha_backward_tc_release() { g_bwd_ws.release(); }

@@ -296,6 +296,21 @@ def test_attention_backward_tensor_kernels_at_tile_edges(shape, causal, stored):
     assert st.value == 0
 
 
+@pytest.mark.parametrize("shape", [(1, 1, 4, 32), (1, 2, 132, 32), (1, 1, 451, 32), (2, 1, 452, 32), (1, 2, 388, 64)])
+@pytest.mark.parametrize("causal", [False, True])
+def test_attention_backward_ring_of_stored_probabilities(shape, causal):
+    """The stored probabilities through a ring of two or three tiles: fewer tiles than the ring and several rounds of it, rows
+    and columns that end inside a box, and (an odd length) the path without it."""
+    B, H, S, D = shape
+    E = H * D
+    qkv = synth.qkv_planes(840 + S, B, S, E)
+    g = synth.normal(841 + S, (B * S, E))
+    probs = ob.mha(qkv, B, S, E, H, causal=causal, want_probs=True)[1]
+    want = ob.mha_backward(g, qkv, probs, B, S, E, H, causal=causal, fma=True)
+    got = _run_backward(g, qkv, probs, B, S, E, H, causal)
+    assert float(np.abs(got - want).max()) <= 4e-6 * max(1.0, float(np.abs(want).max()))
+
+
 def test_attention_backward_of_any_magnitude_and_captured_into_a_graph():
     B, H, S, D = 2, 2, 96, 64
     E = H * D
