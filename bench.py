@@ -354,7 +354,7 @@ def decode_leg():
     return {"metric": "greedy_decode_tokens_per_s", "value": B * n_new / ((ms_prompt + ms_decode) * 1e-3), "unit": "tok/s",
             "steady_state_tokens_per_s": B * (n_new - 1) / (ms_decode * 1e-3), "us_per_step": ms_decode / (n_new - 1) * 1e3,
             "ids_equal_cpu_oracle": bool(np.array_equal(ids, ref_ids)),
-            "driver": "one CUDA graph of 52 launches per step",
+            "driver": "one launch for all steps: a cluster of blocks per rows of the batch (one CUDA graph of 52 launches per step for models outside its sizes)",
             "persistent_form": {"value": B * n_new / ((msp_prompt + msp_decode) * 1e-3), "us_per_step": msp_decode / (n_new - 1) * 1e3,
                            "ids_equal_cpu_oracle": bool(np.array_equal(ids_p, ref_ids))},
             "cpu_oracle_tokens_per_s": B * n_new / t_cpu, "cpu_threads": os.cpu_count(),

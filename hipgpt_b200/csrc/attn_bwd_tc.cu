@@ -194,19 +194,25 @@ __device__ __forceinline__ void add_tile(uint32_t acc, int hf, float (&o)[D / 2]
     }
 }
 
+// A warp's 32 rows x D / 2 results leave in whole lines: through shared memory (boxes of 32 x 32, 16-byte pieces permuted by the row; at head_dim
+// 32 the two warps of a quarter share one), then a row of 128 bytes per eight lanes.  A thread's own stores touched 32 lines
+// each (1.2 us at the end of a 10.7 us block of columns).  dst: the head's first column of the warp's first row.
 template <int D>
-__device__ __forceinline__ void store_out(const float (&o)[D / 2], int hf, float scale, float *dst)
+__device__ __forceinline__ void store_out(const float (&o)[D / 2], int warp, int lane, float scale, uint8_t *stage, float *dst, int E, int nrows, bool off)
 {
-    dst += hf * (D / 2);
-    if ((reinterpret_cast<uintptr_t>(dst) & 31) == 0) {          // rows are whole 32-byte sectors apart: one store per sector
+    const int wq = warp & 3, hf = warp >> 2;
+    uint8_t *box = stage + (D == 64 ? warp : wq) * 4096;
 #pragma unroll
-        for (int c = 0; c < D / 2; c += 8)
-            asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst + c), "f"(o[c] * scale), "f"(o[c + 1] * scale), "f"(o[c + 2] * scale),
-                         "f"(o[c + 3] * scale), "f"(o[c + 4] * scale), "f"(o[c + 5] * scale), "f"(o[c + 6] * scale), "f"(o[c + 7] * scale) : "memory");
-    } else {
+    for (int c = 0; c < D / 8; ++c)
+        *reinterpret_cast<float4 *>(box + sw128(lane, D == 64 ? c : hf * 4 + c)) = make_float4(o[4 * c] * scale, o[4 * c + 1] * scale, o[4 * c + 2] * scale, o[4 * c + 3] * scale);
+    if (D == 64) __syncwarp();
+    else asm volatile("bar.sync %0, 64;" ::"r"(2 + wq) : "memory");
+    constexpr int kRows = D == 64 ? 32 : 16;
 #pragma unroll
-        for (int c = 0; c < D / 2; c += 4)
-            *reinterpret_cast<float4 *>(dst + c) = make_float4(o[c] * scale, o[c + 1] * scale, o[c + 2] * scale, o[c + 3] * scale);
+    for (int i = 0; i < kRows / 4; ++i) {
+        const int r = (D == 64 ? 0 : hf * 16) + 4 * i + (lane >> 3);
+        const float4 v = *reinterpret_cast<const float4 *>(box + sw128(r, lane & 7));
+        if (r < nrows && !off) *reinterpret_cast<float4 *>(dst + (size_t)r * E + (D == 64 ? hf * 32 : 0) + (lane & 7) * 4) = v;
     }
 }
 
@@ -523,7 +529,9 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         }
     }
     add_dq(total - 1);
-    if (row < S && !abort_flag) store_out<D>(o, hf, c, dQ + ((size_t)b * S + row) * E + (size_t)h * D);
+    // (through the K tiles' memory: the last product has read it)
+    const int row0 = q0 + wq * 32;
+    store_out<D>(o, warp, lane, c, k_s, dQ + ((size_t)b * S + row0) * E + (size_t)h * D, E, S - row0, abort_flag);
     tc_fence_before();
     __syncthreads();
 }
@@ -745,11 +753,11 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         arrive(&ready[i & 1]);
     }
     add_dkv(total - 1);
-    if (key < S && !abort_flag) {
-        const size_t dst = ((size_t)b * S + key) * E + (size_t)h * D;
-        store_out<D>(ov, hf, 1.0f, dV + dst);
-        store_out<D>(ok, hf, c, dK + dst);
-    }
+    // (through the tiles' memory: the last products have read it)
+    const int row0 = k0 + wq * 32;
+    const size_t dst = ((size_t)b * S + row0) * E + (size_t)h * D;
+    store_out<D>(ov, warp, lane, 1.0f, t_s, dV + dst, E, S - row0, abort_flag);
+    store_out<D>(ok, warp, lane, c, t_s + TB * 2, dK + dst, E, S - row0, abort_flag);
     tc_fence_before();
     __syncthreads();
 }
