@@ -546,6 +546,10 @@ struct ColsCfg {
     static constexpr uint32_t kBuf = 3 * kTile;                          // S^T, dP^T and room: six pieces take 192 columns
     static constexpr uint32_t kColV = 2 * kBuf, kColK = kColV + 64;
     static constexpr bool kWide = D == 32;                               // 64 columns per accumulator
+    // w and lse by bulk copy, tiles ahead, or by the workers' loads: those stand between the scores and ds (0.3 us per tile of 1.4, 1.4 in
+    // a block's first at D = 32 with stored probabilities: 100.7 -> 97.8 us at B=32 H=8 S=256), but where the rest of a tile is short
+    // and a block has a tile or two the copy's longer way costs more (D = 32 without them, S = 64: 17.1 against 17.5 us)
+    static constexpr bool kRowsAhead = STORED != 0 || D == 64;
 };
 
 template <int D, bool CAUSAL, int STORED>
@@ -558,7 +562,8 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *p_s = STORED == 2 ? reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023) : smem_raw;
     uint8_t *k_s = p_s + C::kStage, *v_s = k_s + (STORED ? 0 : 2 * TB), *t_s = v_s + 2 * TB;     // t_s: [stage][Q tile | dO tile]
-    __shared__ uint64_t res_full, full[C::kStages], sd_full[2], ready[2], acc_done[2], p_full[STORED == 2 ? kPStages<D> : 1];
+    __shared__ __align__(16) float rows_s[C::kStages][2][kTile];         // w and, to form P again, lse of a tile's queries
+    __shared__ uint64_t res_full, full[C::kStages], w_full[C::kStages], sd_full[2], ready[2], acc_done[2], p_full[STORED == 2 ? kPStages<D> : 1];
     __shared__ uint32_t tmem_base_slot;
     __shared__ volatile int abort_flag;
 
@@ -573,7 +578,7 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
     if (tid == 0) {
         abort_flag = 0;
         mbar_init(&res_full, 1);
-        for (int i = 0; i < C::kStages; ++i) mbar_init(&full[i], 1);
+        for (int i = 0; i < C::kStages; ++i) { mbar_init(&full[i], 1); mbar_init(&w_full[i], 1); }
         if (STORED == 2) for (int i = 0; i < kPStages<D>; ++i) mbar_init(&p_full[i], 1);
         for (int i = 0; i < 2; ++i) { mbar_init(&sd_full[i], STORED ? 1 : 2); mbar_init(&ready[i], kWorkerWarps); mbar_init(&acc_done[i], 2); }      // (commits: one per issuing warp)
     }
@@ -582,12 +587,12 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     // No wait for the kernel before yet: the probabilities and the images are older than that one (it waited for the
-    // packing before it let this one start); the workers wait for it where they first read w and lse.
+    // packing before it let this one start); who reads w and lse waits for it.
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_base_slot;
-    // site codes: 11 resident operands, 12 tile pair, 14 scores, 15 workers at a tile, 16 accumulation, 17 probabilities
+    // site codes: 11 resident operands, 12 tile pair, 14 scores, 15 workers at a tile, 16 accumulation, 17 probabilities, 18 w and lse
     auto wait = [&](uint64_t *bar, uint32_t parity, int site) {
         if (abort_flag || mbar_test(bar, parity)) return;
         bwd_wait_slow(bar, parity, site, &abort_flag);
@@ -634,6 +639,16 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
                 for (int i = 0; i < C::kStages; ++i) fetch(i);
             }
         }
+        auto fetch_w = [&](int i) {
+            if (lane == 0 && i < total) {
+                uint64_t *bar = &w_full[i % C::kStages];
+                const size_t at = (size_t)bh * Spad + (size_t)(t0 + i) * kTile;
+                mbar_arrive_expect_tx(bar, (STORED ? 1 : 2) * kTile * 4);
+                bulk_load(rows_s[i % C::kStages][0], w_in + at, kTile * 4, bar);
+                if (!STORED) bulk_load(rows_s[i % C::kStages][1], lse_in + at, kTile * 4, bar);
+            }
+            __syncwarp();
+        };
         auto issue_sd = [&](int i) {
             if (STORED && first) return;
             const uint32_t d = tmem + (uint32_t)(i & 1) * C::kBuf, t = smem_u32(t_s + (i % C::kStages) * 2 * TB);
@@ -646,6 +661,10 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         wait(&res_full, 0, 11);
         tc_fence_after();
         issue_sd(0);
+        if (!first && C::kRowsAhead) {
+            dependency_wait();
+            for (int i = 0; i < C::kStages; ++i) fetch_w(i);
+        }
         for (int i = 0; i < total; ++i) {
             if (i >= 1) {                            // tile i - 1 has been accumulated: its stage and its buffer are free
                 wait(&acc_done[(i - 1) & 1], (uint32_t)(((i - 1) >> 1) & 1), 16);
@@ -656,6 +675,7 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
             wait(&ready[i & 1], (uint32_t)((i >> 1) & 1), 15);
             tc_fence_after();
             if (STORED == 2 && first) fetch_p(i + kPStages<D>);      // the workers have read tile i of the probabilities
+            if (!first && C::kRowsAhead) fetch_w(i + C::kStages);                     // ... and its w and lse
             const uint32_t s0 = tmem + (uint32_t)(i & 1) * C::kBuf, t = smem_u32(t_s + (i % C::kStages) * 2 * TB);
             auto p_col = [&](int p, int hf) { return p == 2 ? s0 + kTile + 32 * hf : s0 + 32 * hf + 16 * p; };
             auto ds_col = [&](int p, int hf) { return p == 0 ? s0 + kTile + 32 * hf + 16 : s0 + 2 * kTile + 32 * hf + 16 * (p - 1); };
@@ -680,7 +700,6 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         __syncwarp();
         if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
     };
-    const float *wrow = w_in + (size_t)bh * Spad, *lrow = lse_in + (size_t)bh * Spad;
     float pn[STORED == 1 ? 32 : 1];                  // stored probabilities of the tile ahead: a query's are contiguous over the keys (lanes)
     auto fetch_p = [&](int i) {
         const int qb = (t0 + i) * kTile + hf * 32;
@@ -705,10 +724,12 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         add_tile<D, C::kWide>(lane_base + C::kColK, hf, ok);
     };
     if (STORED == 1) fetch_p(0);
-    dependency_wait();
+    if (!C::kRowsAhead) dependency_wait();
     for (int i = 0; i < total; ++i) {
         const uint32_t s_addr = lane_base + (uint32_t)(i & 1) * C::kBuf + hf * 32, dp_addr = s_addr + kTile, room = s_addr + 2 * kTile;
         const int qb = (t0 + i) * kTile + hf * 32;
+        const size_t at = (size_t)bh * Spad + qb;
+        const float *wrow = C::kRowsAhead ? rows_s[i % C::kStages][0] + hf * 32 : w_in + at, *lrow = C::kRowsAhead ? rows_s[i % C::kStages][1] + hf * 32 : lse_in + at;
         const bool mask = CAUSAL && qb < k0 + wq * 32 + 31;              // some lane of the warp has a key after some query
         float p[32], d[32];
         if (STORED == 1) {
@@ -727,10 +748,11 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         if (!STORED) tmem_ld32(s_addr, p);
         tmem_ld32(dp_addr, d);
         tmem_wait_ld();
+        if (C::kRowsAhead) wait(&w_full[i % C::kStages], (uint32_t)((i / C::kStages) & 1), 18);
         if (!STORED) {
 #pragma unroll
             for (int x = 0; x < 32; x += 4) {
-                const float4 ls = __ldg(reinterpret_cast<const float4 *>(lrow + qb + x));       // rows past S: a probability of 0
+                const float4 ls = *reinterpret_cast<const float4 *>(lrow + x);       // rows past S: a probability of 0
                 float2 a = ffma2(make_float2(p[x], p[x + 1]), make_float2(cl2, cl2), make_float2(-ls.x, -ls.y));
                 float2 e = ffma2(make_float2(p[x + 2], p[x + 3]), make_float2(cl2, cl2), make_float2(-ls.z, -ls.w));
                 p[x] = ex2_approx(a.x); p[x + 1] = ex2_approx(a.y); p[x + 2] = ex2_approx(e.x); p[x + 3] = ex2_approx(e.y);
@@ -742,7 +764,7 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         }
 #pragma unroll
         for (int x = 0; x < 32; x += 4) {
-            const float4 w4 = __ldg(reinterpret_cast<const float4 *>(wrow + qb + x));
+            const float4 w4 = *reinterpret_cast<const float4 *>(wrow + x);
             d[x] = p[x] * (d[x] - w4.x); d[x + 1] = p[x + 1] * (d[x + 1] - w4.y);
             d[x + 2] = p[x + 2] * (d[x + 2] - w4.z); d[x + 3] = p[x + 3] * (d[x + 3] - w4.w);
         }
@@ -771,7 +793,7 @@ int launch_cfg(const float *g, const float *q, const float *k, const float *v, c
     auto rows = bwd_rows_kernel<D, CAUSAL, STORED>;
     auto cols = bwd_cols_kernel<D, CAUSAL, STORED>;
     constexpr size_t rows_smem = RowsCfg<D, STORED>::kSmem, cols_smem = ColsCfg<D, STORED>::kSmem;
-    static_assert(rows_smem + (STORED ? 1 : 3) * 2 * kLanes * 4 + 256 <= 232448 && cols_smem + 256 <= 232448, "shared memory of a block");
+    static_assert(rows_smem + (STORED ? 1 : 3) * 2 * kLanes * 4 + 256 <= 232448 && cols_smem + ColsCfg<D, STORED>::kStages * 2 * kTile * 4 + 512 <= 232448, "shared memory of a block");
     cudaError_t e = cudaFuncSetAttribute(rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(cols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cols_smem);
     if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
