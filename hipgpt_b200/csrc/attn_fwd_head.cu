@@ -139,6 +139,11 @@ __device__ __forceinline__ float2 f16_sum(float hi, float lo)
     return r;
 }
 
+__device__ __forceinline__ void store_sector(float *dst, float a, float b, float c, float d, float e, float f, float g, float h)
+{
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "f"(a), "f"(b), "f"(c), "f"(d), "f"(e), "f"(f), "f"(g), "f"(h) : "memory");
+}
+
 __device__ __forceinline__ void tma_store_3d(const void *tensor_map, const void *smem_src, int c0, int c1, int c2)
 {
     asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%1, %2, %3}], [%4];"
@@ -791,7 +796,8 @@ mha_head_kernel(const __grid_constant__ HeadMaps maps, float *__restrict__ O, fl
             const float inv = (1.0f / fmaxf(l, 1e-20f)) * s_vinv[it & 3];
             const int row = q * kTile + ((flip0 && q == 0) ? 3 - wq : wq) * 32 + lane;
             const bool store = !abort_flag && row < S;
-            float4 *dst = reinterpret_cast<float4 *>(O + ((size_t)b * S + (row < S ? row : 0)) * (size_t)E + (size_t)h * 32);
+            float *dst = O + ((size_t)b * S + (row < S ? row : 0)) * (size_t)E + (size_t)h * 32;
+            const bool o_sectors = (reinterpret_cast<uintptr_t>(O) & 31) == 0;   // (a head's columns are 128 bytes, rows a multiple of that)
             const uint32_t o_addr = lane_base + kColO + (uint32_t)(q * 64);
 #pragma unroll 1
             for (int cc = c0; cc < c0 + nc; cc += 16) {
@@ -799,11 +805,15 @@ mha_head_kernel(const __grid_constant__ HeadMaps maps, float *__restrict__ O, fl
                 tmem_ld16(o_addr + cc, a);
                 tmem_ld16(o_addr + 32 + cc, c2);
                 tmem_wait_ld();
-                if (store) {
+                float o[16];
 #pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        dst[(cc >> 2) + j] = make_float4((a[4 * j] + c2[4 * j]) * inv, (a[4 * j + 1] + c2[4 * j + 1]) * inv,
-                                                         (a[4 * j + 2] + c2[4 * j + 2]) * inv, (a[4 * j + 3] + c2[4 * j + 3]) * inv);
+                for (int j = 0; j < 16; ++j) o[j] = (a[j] + c2[j]) * inv;
+                if (store && o_sectors) {
+                    store_sector(dst + cc, o[0], o[1], o[2], o[3], o[4], o[5], o[6], o[7]);
+                    store_sector(dst + cc + 8, o[8], o[9], o[10], o[11], o[12], o[13], o[14], o[15]);
+                } else if (store) {
+#pragma unroll
+                    for (int j = 0; j < 16; j += 4) *reinterpret_cast<float4 *>(dst + cc + j) = make_float4(o[j], o[j + 1], o[j + 2], o[j + 3]);
                 }
             }
         }
