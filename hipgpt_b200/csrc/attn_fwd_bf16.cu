@@ -339,20 +339,27 @@ mha_bf16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant_
         wait(&o_done[(nt - 1) % kStages], phn(nt - 1, kStages), 3);
         tc_fence_after();
         const float inv = 1.0f / fmaxf(l, 1e-20f);
-        const bool store = !abort_flag && row < S;
-        uint4 *dst = reinterpret_cast<uint4 *>(O + (tok0 + (row < S ? row : 0)) * (size_t)E + hcol);
+        // The output leaves in whole lines, turned through the Q tile (the last Q K^T has read it): a thread's own 16-byte
+        // stores touched 32 lines per instruction.
+        uint8_t *ob = q_s + wq * 4096;
 #pragma unroll
         for (int hh = 0; hh < D / 32; ++hh) {
             float a[32];
             tmem_ld32(o_addr + hh * 32, a);
             tmem_wait_ld();
-            if (store) {
 #pragma unroll
-                for (int c = 0; c < 4; ++c)
-                    dst[hh * 4 + c] = make_uint4(pack_bf16(a[c * 8 + 0] * inv, a[c * 8 + 1] * inv), pack_bf16(a[c * 8 + 2] * inv, a[c * 8 + 3] * inv),
-                                                 pack_bf16(a[c * 8 + 4] * inv, a[c * 8 + 5] * inv), pack_bf16(a[c * 8 + 6] * inv, a[c * 8 + 7] * inv));
-            }
+            for (int c = 0; c < 4; ++c)
+                *reinterpret_cast<uint4 *>(ob + sw128(lane, hh * 4 + c)) =
+                    make_uint4(pack_bf16(a[c * 8 + 0] * inv, a[c * 8 + 1] * inv), pack_bf16(a[c * 8 + 2] * inv, a[c * 8 + 3] * inv),
+                               pack_bf16(a[c * 8 + 4] * inv, a[c * 8 + 5] * inv), pack_bf16(a[c * 8 + 6] * inv, a[c * 8 + 7] * inv));
         }
+        __syncwarp();
+        const int row0 = row - lane;
+        __nv_bfloat16 *dst = O + (tok0 + row0) * (size_t)E + hcol + (lane & 7) * 8;
+        const bool store = !abort_flag;
+#pragma unroll
+        for (int r = lane >> 3; r < 32; r += 4)
+            if (store && row0 + r < S) *reinterpret_cast<uint4 *>(dst + (size_t)r * E) = *reinterpret_cast<const uint4 *>(ob + sw128(r, lane & 7));
     }
     tc_fence_before();
     __syncthreads();

@@ -139,11 +139,6 @@ __device__ __forceinline__ float2 f16_sum(float hi, float lo)
     return r;
 }
 
-__device__ __forceinline__ void store_sector(float *dst, float a, float b, float c, float d, float e, float f, float g, float h)
-{
-    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "f"(a), "f"(b), "f"(c), "f"(d), "f"(e), "f"(f), "f"(g), "f"(h) : "memory");
-}
-
 __device__ __forceinline__ void tma_store_3d(const void *tensor_map, const void *smem_src, int c0, int c1, int c2)
 {
     asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%1, %2, %3}], [%4];"
