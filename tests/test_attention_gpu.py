@@ -64,6 +64,23 @@ def test_whole_head_kernel_many_heads_per_block(S, causal):
     np.testing.assert_array_equal(out, plain)
 
 
+@pytest.mark.parametrize("S", [40, 200, 300])
+def test_output_aligned_to_16_bytes_only(S):
+    """head_dim 32: an output whose rows are not whole 32-byte sectors, probabilities that are not 16-byte aligned."""
+    from hipgpt_b200 import launchers
+    B, H, D = 2, 3, 32
+    E = H * D
+    qkv = synth.qkv_planes(50 + S, B, S, E)
+    ref_out, ref_probs = ob.mha(qkv, B, S, E, H, causal=True, want_probs=True)
+    buf, pbuf = torch.full((B * S * E + 8,), float("nan"), device="cuda"), torch.full((B * H * S * S + 8,), float("nan"), device="cuda")
+    for p_at in (0, 1):
+        out, probs = buf[4:4 + B * S * E], pbuf[p_at:p_at + B * H * S * S]
+        launchers.launch_multihead_attention(dev(qkv), out, probs, B, S, E, H, causal=True)
+        assert _maxerr(out.cpu().numpy().reshape(-1), ref_out.reshape(-1)) <= TOL
+        assert _maxerr(probs.cpu().numpy().reshape(-1), ref_probs.reshape(-1)) <= TOL
+    assert torch.isnan(buf[:4]).all() and torch.isnan(buf[-4:]).all() and torch.isnan(pbuf[-7:]).all()
+
+
 @pytest.mark.parametrize("warps", [1, 2, 4])
 @pytest.mark.parametrize("D", [32, 64, 128])
 @pytest.mark.parametrize("causal", [False, True])
