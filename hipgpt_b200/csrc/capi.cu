@@ -1,7 +1,7 @@
 // C ABI of the attention library: argument checks, dispatch, the host-buffer call and the
 // per-thread error text.  Declarations and the reference interfaces they replace are in
 // include/hipgpt_attn.h.
-#include "attn_common.cuh"
+#include "stream_workspace.hpp"
 
 #include <stdarg.h>
 #include <stdio.h>
@@ -135,6 +135,8 @@ struct Workspace {
     int device = -1;
 };
 Workspace g_ws;
+
+StreamWorkspace g_bwd_rows_ws;                       // hipgpt_mha_backward_planes
 
 }  // namespace
 }  // namespace hipgpt
@@ -317,6 +319,7 @@ void hipgpt_release_workspace(void)
     tc16_release_scratch();
     gemm_tc_release_scratch();
     mha_backward_tc_release();
+    g_bwd_rows_ws.release();
     std::lock_guard<std::mutex> lock(g_ws.mu);
     if (g_ws.dev) cudaFree(g_ws.dev);
     for (int i = 0; i < Workspace::kStreams; ++i) if (g_ws.streams[i]) { cudaStreamDestroy(g_ws.streams[i]); g_ws.streams[i] = nullptr; }
@@ -404,8 +407,8 @@ int hipgpt_mha_backward(const float *d_grad_out, const float *d_q, const float *
                                static_cast<cudaStream_t>(stream));
 }
 
-// The reference's launcher has no scratch argument (include/hip_kernels.h:59-62): its drop-in form keeps the row
-// sums in a buffer of the library that grows to the largest call on the current device.
+// The reference's launcher has no scratch argument (include/hip_kernels.h:59-62): in its drop-in form the kernels that need the
+// row sums get them from a workspace of the library.  Those of the tensor pipe have none.
 int hipgpt_mha_backward_planes(const float *d_grad_out, const float *d_qkv, const float *d_probs, float *d_grad_qkv,
                                int B, int S, int E, int H, int causal, void *stream)
 {
@@ -413,29 +416,16 @@ int hipgpt_mha_backward_planes(const float *d_grad_out, const float *d_qkv, cons
     if (H <= 0 || E % H != 0) return fail(HIPGPT_ERR_BAD_ARG, "Bad MHA config: E=%d H=%d", E, H);
     if (B == 0 || S == 0 || E == 0) return HIPGPT_OK;
     if (!d_grad_out || !d_qkv || !d_grad_qkv) return fail(HIPGPT_ERR_NULL, "grad_out, qkv and grad_qkv must not be NULL");
-    static std::mutex mu;
-    static float *buf[64] = {};
-    static size_t cap[64] = {};
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess || dev < 0 || dev >= 64) return fail(HIPGPT_ERR_CUDA, "cudaGetDevice: %s", cudaGetErrorString(e));
-    const size_t need = mha_backward_scratch_bytes(B, H, S);
-    float *scratch;
-    {
-        std::lock_guard<std::mutex> lock(mu);
-        if (cap[dev] < need) {
-            if (buf[dev]) cudaFree(buf[dev]);
-            buf[dev] = nullptr;
-            cap[dev] = 0;
-            e = cudaMalloc(&buf[dev], need);
-            if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "cudaMalloc(%zu): %s", need, cudaGetErrorString(e));
-            cap[dev] = need;
-        }
-        scratch = buf[dev];
-    }
     const size_t plane = (size_t)B * S * E;
-    return launch_mha_backward(d_grad_out, d_qkv, d_qkv + plane, d_qkv + 2 * plane, d_probs, d_grad_qkv, d_grad_qkv + plane,
-                               d_grad_qkv + 2 * plane, scratch, B, S, E, H, causal, static_cast<cudaStream_t>(stream));
+    const float *k = d_qkv + plane, *v = k + plane;
+    float *dk = d_grad_qkv + plane, *dv = dk + plane;
+    const cudaStream_t st = static_cast<cudaStream_t>(stream);
+    StreamWorkspace::Lease scratch;
+    if (!mha_backward_tc_supports(d_grad_out, d_qkv, k, v, d_probs, d_grad_qkv, dk, dv, B, S, E, H)) {
+        const int rc = g_bwd_rows_ws.enter(st, mha_backward_scratch_bytes(B, H, S), &scratch);
+        if (rc != HIPGPT_OK) return rc;
+    }
+    return launch_mha_backward(d_grad_out, d_qkv, k, v, d_probs, d_grad_qkv, dk, dv, reinterpret_cast<float *>(scratch.get()), B, S, E, H, causal, st);
 }
 
 int hipgpt_shard_range(int B, int world, int rank, int *b_begin, int *b_end)

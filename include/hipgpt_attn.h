@@ -152,8 +152,8 @@ HIPGPT_API int hipgpt_attention_weighted_sum(const float *d_softmax, const float
  * head_dim 32 and 64 run on the tensor pipe with fp32 accuracy over the whole fp32 range (every operand as the sum of three
  * bf16 numbers, six products per product); the operands' images live in a buffer of the library (per device and stream,
  * at most eight; hipgpt_release_workspace() frees them; a captured call gets a buffer of its graph).
- * hipgpt_mha_backward_planes is the launcher's own view (three stacked planes in d_qkv and d_grad_qkv) with
- * the scratch kept in a buffer of the library, which grows with cudaMalloc to the largest call per device.
+ * hipgpt_mha_backward_planes is the launcher's own view (three stacked planes in d_qkv and d_grad_qkv): the scratch, which
+ * only the kernels of the other head dimensions use, comes from a buffer of the library of the same kind.
  */
 HIPGPT_API size_t hipgpt_mha_backward_scratch_bytes(int B, int H, int S);
 HIPGPT_API int hipgpt_mha_backward(const float *d_grad_out, const float *d_q, const float *d_k, const float *d_v, const float *d_probs,
