@@ -25,12 +25,10 @@
 //                        while the products of the next one run.
 // Rows, columns and depth beyond the matrices are zeros in the images; stores are bounded by M and K.
 // Every wait is bounded: on expiry the block records a status code, skips its stores, frees its TMEM and returns.
+#include "stream_workspace.hpp"
 #include "tc_primitives.cuh"
 
 #include <math.h>
-
-#include <mutex>
-#include <vector>
 
 namespace hipgpt {
 namespace {
@@ -453,36 +451,7 @@ gemm_tc_kernel(const uint8_t *__restrict__ aimg, const uint8_t *__restrict__ bim
     __syncthreads();
 }
 
-// The packed operands of a call live in a buffer of the library, one per device and stream; it grows to the largest call.
-struct GemmScratch {
-    std::mutex mu;
-    struct Entry { int dev; cudaStream_t st; uint8_t *buf; size_t cap; };
-    std::vector<Entry> entries;
-    int get(int dev, cudaStream_t st, size_t need, uint8_t **out)
-    {
-        std::lock_guard<std::mutex> lock(mu);
-        Entry *e = nullptr;
-        for (auto &x : entries) if (x.dev == dev && x.st == st) e = &x;
-        if (!e) { entries.push_back({dev, st, nullptr, 0}); e = &entries.back(); }
-        if (e->cap < need) {
-            if (e->buf) cudaFree(e->buf);            // waits for the kernels that read it
-            e->buf = nullptr;
-            e->cap = 0;
-            const cudaError_t err = cudaMalloc(&e->buf, need);
-            if (err != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "cudaMalloc(%zu) for the packed operands: %s", need, cudaGetErrorString(err));
-            e->cap = need;
-        }
-        *out = e->buf;
-        return HIPGPT_OK;
-    }
-    void release()
-    {
-        std::lock_guard<std::mutex> lock(mu);
-        for (auto &x : entries) if (x.buf) cudaFree(x.buf);
-        entries.clear();
-    }
-};
-GemmScratch g_gemm;
+StreamWorkspace g_gemm;                              // the packed operands of a call
 
 }  // namespace
 
@@ -569,10 +538,10 @@ int launch_matmul_tc(const float *A, const float *B, const float *bias, float *C
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "cudaGetDevice: %s", cudaGetErrorString(e));
     const size_t abytes = (size_t)MT * KT * kAStage, bbytes = (size_t)NT * KT * kBStage, rbytes = ((size_t)MT * kTM * sizeof(float) + 255) & ~(size_t)255;
-    uint8_t *scratch = nullptr;
-    int rc = g_gemm.get(dev, st, abytes + bbytes + rbytes + 256, &scratch);
+    StreamWorkspace::Lease ws;
+    int rc = g_gemm.enter(st, abytes + bbytes + rbytes + 256, &ws);
     if (rc != HIPGPT_OK) return rc;
-    uint8_t *aimg = scratch, *bimg = scratch + abytes;
+    uint8_t *scratch = ws.get(), *aimg = scratch, *bimg = scratch + abytes;
     float *row_inv = reinterpret_cast<float *>(scratch + abytes + bbytes), *b_amax = reinterpret_cast<float *>(scratch + abytes + bbytes + rbytes);
     rc = set_gemm_attr();
     if (rc == HIPGPT_OK) rc = pack_b(B, N, K, bimg, b_amax, st);
@@ -620,9 +589,10 @@ int launch_matmul_tc_prepared(const float *A, const PackedB *b, const float *bia
     if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "cudaGetDevice: %s", cudaGetErrorString(e));
     if (dev != b->dev) return fail(HIPGPT_ERR_BAD_ARG, "the right-hand side was packed on device %d, the current device is %d", b->dev, dev);
     const size_t abytes = (size_t)MT * KT * kAStage, rbytes = ((size_t)MT * kTM * sizeof(float) + 255) & ~(size_t)255;
-    uint8_t *scratch = nullptr;
-    int rc = g_gemm.get(dev, st, abytes + rbytes, &scratch);
+    StreamWorkspace::Lease ws;
+    int rc = g_gemm.enter(st, abytes + rbytes, &ws);
     if (rc != HIPGPT_OK) return rc;
+    uint8_t *scratch = ws.get();
     rc = set_gemm_attr();
     if (rc != HIPGPT_OK) return rc;
     return pack_a_and_multiply(A, b->bimg, b->b_amax, bias, C, M, N, K, scratch, reinterpret_cast<float *>(scratch + abytes), dev, st, ln_g, ln_b);

@@ -175,7 +175,8 @@ HIPGPT_API int hipgpt_mha_backward_planes(const float *d_grad_out, const float *
  *                            power-of-two scaling (per row of A, one for B), three products per product, fp32
  *                            accumulation: 1e-5 on unit-scale data instead of identical bits, several times the
  *                            rate.  Not in place.  The packed operands live in a buffer of the library (per device
- *                            and stream; hipgpt_release_workspace() frees it).
+ *                            and stream, at most eight; hipgpt_release_workspace() frees them; a captured call gets a
+ *                            buffer of its graph).
  *   hipgpt_matmul_tc_prepare / _prepared / _release
  *                            the same with the right-hand side (a layer's weights) packed once: prepare() allocates
  *                            device memory for B's packed form and fills it (asynchronously on `stream`; B may be
