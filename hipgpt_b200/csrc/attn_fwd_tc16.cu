@@ -35,13 +35,11 @@
 //   A warp stages its 32 query rows with whole-line reads (D / 4 lanes per row), all in flight at once.
 // Every wait is bounded: on expiry the block raises a flag that cuts all later waits short,
 // records a status code, skips its stores, frees its TMEM and returns.
+#include "stream_workspace.hpp"
 #include "tc_primitives.cuh"
 
 #include <math.h>
 #include <stdlib.h>
-
-#include <mutex>
-#include <vector>
 
 namespace hipgpt {
 namespace {
@@ -677,59 +675,7 @@ mha_tc16_kernel(const uint8_t *__restrict__ kimg, const uint8_t *__restrict__ vi
     __syncthreads();
 }
 
-// The packed operands of a call live in a buffer of the library, one per device and stream (a call's kernels read it
-// after the call has returned; calls on different streams must not share it).  It grows to the largest call.
-struct PackScratch {
-    std::mutex mu;
-    // side: the stream on which the groups after the first are packed while the group before them is attended to;
-    // entered: the caller's stream has reached the call; packed[i], attended[i]: buffer i has been written / read
-    struct Entry { int dev; cudaStream_t st; uint8_t *buf; size_t cap; cudaStream_t side; cudaEvent_t entered, packed[2], attended[2]; };
-    std::vector<Entry> entries;
-    int get(int dev, cudaStream_t st, size_t need, uint8_t **out, Entry **entry = nullptr)
-    {
-        std::lock_guard<std::mutex> lock(mu);
-        Entry *e = nullptr;
-        for (auto &x : entries) if (x.dev == dev && x.st == st) e = &x;
-        if (!e) { entries.push_back({dev, st, nullptr, 0, nullptr, nullptr, {nullptr, nullptr}, {nullptr, nullptr}}); e = &entries.back(); }
-        if (entry) {
-            *entry = e;                              // entries are only appended, and only under the lock: take care below
-            if (!e->side) {
-                cudaError_t err = cudaStreamCreateWithFlags(&e->side, cudaStreamNonBlocking);
-                if (err == cudaSuccess) err = cudaEventCreateWithFlags(&e->entered, cudaEventDisableTiming);
-                for (int i = 0; i < 2 && err == cudaSuccess; ++i) {
-                    err = cudaEventCreateWithFlags(&e->packed[i], cudaEventDisableTiming);
-                    if (err == cudaSuccess) err = cudaEventCreateWithFlags(&e->attended[i], cudaEventDisableTiming);
-                }
-                if (err != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "stream or event for the packing: %s", cudaGetErrorString(err));
-            }
-        }
-        if (e->cap < need) {
-            if (e->buf) cudaFree(e->buf);        // waits for the kernels that read it
-            e->buf = nullptr;
-            e->cap = 0;
-            const cudaError_t err = cudaMalloc(&e->buf, need);
-            if (err != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "cudaMalloc(%zu) for the packed K and V: %s", need, cudaGetErrorString(err));
-            e->cap = need;
-        }
-        *out = e->buf;
-        return HIPGPT_OK;
-    }
-    void release()
-    {
-        std::lock_guard<std::mutex> lock(mu);
-        for (auto &x : entries) {
-            if (x.buf) cudaFree(x.buf);
-            if (x.side) cudaStreamDestroy(x.side);
-            if (x.entered) cudaEventDestroy(x.entered);
-            for (int i = 0; i < 2; ++i) {
-                if (x.packed[i]) cudaEventDestroy(x.packed[i]);
-                if (x.attended[i]) cudaEventDestroy(x.attended[i]);
-            }
-        }
-        entries.clear();
-    }
-};
-PackScratch g_pack;
+StreamWorkspace g_pack;                              // the packed operands of a group of batches (two groups)
 
 template <int D, bool CAUSAL, bool PROBS>
 int launch_tc16_cfg(const float *q, const float *k, const float *v, float *out, float *probs, int B, int S, int E, int H, cudaStream_t st)
@@ -755,31 +701,25 @@ int launch_tc16_cfg(const float *q, const float *k, const float *v, float *out, 
     // a group each (the same footprint in L2), events in both directions.  Measured at B=64 H=16 S=2048 head_dim 64:
     // unmasked 292 -> 309 TFLOP/s; causal 256 -> 249 (half-size groups leave the causal kernel, whose blocks differ in
     // length, a longer tail per launch, and 128 - 192 MB of buffers do not help either: 252 - 254).  So it is the default
-    // for unmasked calls only; HIPGPT_PACK_OVERLAP=0 / 1 forces it off / on for both.
+    // for unmasked calls only; HIPGPT_PACK_OVERLAP=0 / 1 forces it off / on for both.  A call that is captured stays on its stream.
     static const int overlap_env = [] { const char *e = getenv("HIPGPT_PACK_OVERLAP"); return (!e || !*e) ? -1 : (*e != '0' ? 1 : 0); }();
-    const bool overlap = (overlap_env < 0 ? !CAUSAL : overlap_env == 1) && B > gb && gb >= 2;
+    const bool overlap = (overlap_env < 0 ? !CAUSAL : overlap_env == 1) && B > gb && gb >= 2 && !being_captured(st);
     if (overlap) gb = gb / 2;
     if (gb > B) gb = B;
     while (gb * H > 65535) --gb;                     // grid.y of the pack kernel
     if (gb < 1) return fail(HIPGPT_ERR_BAD_ARG, "%d heads are too many", H);
     if (gb * H * (long long)nqblk > 2147483647LL) return fail(HIPGPT_ERR_BAD_ARG, "grid of %lld blocks is too large", gb * H * (long long)nqblk);
-    int dev = 0;
-    e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "cudaGetDevice: %s", cudaGetErrorString(e));
     const size_t kbytes = (size_t)gb * H * ntk * C::kK16Stage, vbytes = (size_t)gb * H * ntk * C::kV16Stage;
     const size_t gtiles = (size_t)gb * H * ntk;
     const size_t one = (kbytes + vbytes + 2 * gtiles * sizeof(float) + 1023) & ~(size_t)1023;      // one buffer: K images, V images, the tiles' maxima
-    uint8_t *scratch = nullptr;
-    PackScratch::Entry *ent = nullptr;
-    int rc = g_pack.get(dev, st, overlap ? 2 * one : one, &scratch, overlap ? &ent : nullptr);
+    StreamWorkspace::Lease ws;
+    int rc = g_pack.enter(st, overlap ? 2 * one : one, &ws, overlap);
     if (rc != HIPGPT_OK) return rc;
-    cudaStream_t side = nullptr;
-    cudaEvent_t entered = nullptr, packed[2] = {nullptr, nullptr}, attended[2] = {nullptr, nullptr};
-    if (overlap) {                                   // copies: the vector of entries may move
-        side = ent->side; entered = ent->entered;
-        for (int i = 0; i < 2; ++i) { packed[i] = ent->packed[i]; attended[i] = ent->attended[i]; }
-        e = cudaEventRecord(entered, st);            // K and V are valid from here on, and earlier calls have read the buffers
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(side, entered, 0);
+    uint8_t *scratch = ws.get();
+    const StreamWorkspace::Side &side = ws.side();   // done[i], taken[i]: buffer i has been packed, attended to
+    if (overlap) {
+        e = cudaEventRecord(side.entered, st);       // K and V are valid from here on, and earlier calls have read the buffers
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(side.stream, side.entered, 0);
         if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "event hand-off: %s", cudaGetErrorString(e));
     }
     const float qscale = (1.0f / sqrtf((float)D)) * kLog2e;
@@ -790,9 +730,9 @@ int launch_tc16_cfg(const float *q, const float *k, const float *v, float *out, 
         const int ntiles = nb * H * ntk;
         uint8_t *buf = scratch + (overlap ? (size_t)(g & 1) * one : 0);
         float *tmax = reinterpret_cast<float *>(buf + kbytes + vbytes);      // [2][group's tiles]: largest |K|, |V| of every tile
-        const cudaStream_t ps = overlap ? side : st;
+        const cudaStream_t ps = overlap ? side.stream : st;
         if (overlap && g >= 2) {
-            e = cudaStreamWaitEvent(side, attended[g & 1], 0);               // the group that used this buffer has been attended to
+            e = cudaStreamWaitEvent(side.stream, side.taken[g & 1], 0);    // the group that used this buffer has been attended to
             if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "event hand-off: %s", cudaGetErrorString(e));
         }
         const dim3 pgrid((unsigned)ntk, (unsigned)(nb * H));
@@ -805,8 +745,8 @@ int launch_tc16_cfg(const float *q, const float *k, const float *v, float *out, 
             if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "kv_pack_kernel launch: %s", cudaGetErrorString(e));
         }
         if (overlap) {
-            e = cudaEventRecord(packed[g & 1], side);
-            if (e == cudaSuccess) e = cudaStreamWaitEvent(st, packed[g & 1], 0);
+            e = cudaEventRecord(side.done[g & 1], side.stream);
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(st, side.done[g & 1], 0);
             if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "event hand-off: %s", cudaGetErrorString(e));
         }
         // (one stream:) the attention kernel's blocks start, and stage their query rows, while the pack kernel's last blocks run
@@ -816,7 +756,7 @@ int launch_tc16_cfg(const float *q, const float *k, const float *v, float *out, 
         rc = check_launch("mha_tc16_kernel");
         if (rc != HIPGPT_OK) return rc;
         if (overlap) {
-            e = cudaEventRecord(attended[g & 1], st);
+            e = cudaEventRecord(side.taken[g & 1], st);
             if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "event hand-off: %s", cudaGetErrorString(e));
         }
     }

@@ -81,7 +81,8 @@ HIPGPT_API int hipgpt_mha_forward(const float *d_q, const float *d_k, const floa
  * number of warps per thread block (0 = default); for HIPGPT_ALGO_TENSOR one of HIPGPT_TENSOR_*.
  * Every kernel holds 1e-5 on unit-scale data.  TILED scales its operands into fp16's range by exact powers of two
  * (per query row, per 64-key tile of K and of V) and keeps that accuracy for any fp32 magnitude; it keeps the fp16
- * images of K and V in a buffer of the library (per device and stream; hipgpt_release_workspace() frees it).
+ * images of K and V in a buffer of the library (per device and stream, at most eight; hipgpt_release_workspace()
+ * frees them; a captured call gets a buffer of its graph).
  * WHOLE_HEAD keeps the accuracy while Q and K stay within fp16's range (about 1e-4 .. 6e4; it rescales V by a
  * power of two per head, so V may have any magnitude); outside it its correction terms saturate or are flushed,
  * the result falls to plain TF32 grade (~3e-4 relative), and the launch raises the flag that
