@@ -1,5 +1,7 @@
 """The library's own device buffers (one per device and stream): calls captured into a graph, streams and threads side by
 side, buffers that grow, are evicted or released while graphs and other streams still use theirs."""
+import threading
+
 import pytest
 
 from hipgpt_b200 import _capi
@@ -76,3 +78,139 @@ def test_backwards_of_two_streams_have_their_own_row_sums():
     for i in range(2):
         for r in range(8):
             assert torch.equal(got[i][r], want[i])
+
+
+class _Backward:
+    """dQ, dK, dV with the probabilities formed again; head_dim 64: the tensor pipe's images, 16: row sums."""
+
+    def __init__(self, seed, size, D):
+        self.shape = B, H, S, D = size, 4, 192, D
+        self.inputs = _rand(seed, B * S, H * D), _rand(seed + 1, 3, B * S, H * D)
+
+    def empty(self):
+        return torch.full_like(self.inputs[1], float("nan"))
+
+    def run(self, out, stream):
+        g, qkv = self.inputs
+        B, H, S, D = self.shape
+        _capi.check(_capi.lib().hipgpt_mha_backward_planes(g.data_ptr(), qkv.data_ptr(), None, out.data_ptr(), B, S, H * D, H, 1, stream))
+
+
+class _Matmul:
+    def __init__(self, seed, size):
+        self.shape = M, N, K = 300 * size, 320, 256
+        self.inputs = _rand(seed, M, N), _rand(seed + 1, N, K)
+
+    def empty(self):
+        return torch.full((self.shape[0], self.shape[2]), float("nan"), device="cuda")
+
+    def run(self, out, stream):
+        a, w = self.inputs
+        _capi.check(_capi.lib().hipgpt_matmul_tc(a.data_ptr(), w.data_ptr(), None, out.data_ptr(), *self.shape, stream))
+
+
+class _Attention:
+    """The tiled kernel's packed K and V; `groups`: cut into groups of batches, packed on a second stream (unmasked)."""
+
+    def __init__(self, seed, size, groups):
+        self.shape, self.groups = (size, 16, 128, 64), groups       # 0.5 MB of images per batch
+        B, H, S, D = self.shape
+        self.inputs = _rand(seed, 3, B * S, H * D)
+
+    def empty(self):
+        B, H, S, D = self.shape
+        return torch.full((B * S, H * D), float("nan"), device="cuda")
+
+    def run(self, out, stream):
+        B, H, S, D = self.shape
+        _capi.check(_capi.lib().hipgpt_mha_forward_planes(self.inputs.data_ptr(), out.data_ptr(), None, B, S, H * D, H, int(not self.groups), stream))
+
+
+KINDS = {"attention": lambda seed, size: _Attention(seed, size, False), "attention_groups": lambda seed, size: _Attention(seed, size, True),
+         "backward": lambda seed, size: _Backward(seed, size, 64), "backward_rows": lambda seed, size: _Backward(seed, size, 16), "matmul": _Matmul}
+
+
+@pytest.fixture(autouse=True)
+def _groups(request, monkeypatch):
+    if "attention_groups" in request.node.name:
+        monkeypatch.setenv("HIPGPT_PACK_GROUP_MB", "1")             # two batches
+
+
+def _expected(job):
+    out = job.empty()
+    job.run(out, _st())
+    torch.cuda.synchronize()
+    assert bool(torch.isfinite(out).all())
+    return out
+
+
+@pytest.mark.parametrize("kind", KINDS)
+def test_a_graph_keeps_its_buffer_when_later_calls_grow_or_release_theirs(kind):
+    lib = _capi.lib()
+    small, big = KINDS[kind](10, 2), KINDS[kind](20, 24)
+    want, want_big = _expected(small), _expected(big)
+    stream = torch.cuda.Stream()
+    lib.hipgpt_release_workspace()
+    before, out, out_big = small.empty(), small.empty(), big.empty()
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    small.run(before, stream.cuda_stream)                   # the stream's buffer, in the size of the captured call
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        small.run(out, torch.cuda.current_stream().cuda_stream)
+    big.run(out_big, stream.cuda_stream)                    # grows it
+    torch.cuda.synchronize()
+    assert torch.equal(before, want) and torch.equal(out_big, want_big)
+    for _ in range(2):
+        lib.hipgpt_release_workspace()
+        out.fill_(float("nan"))
+        torch.cuda.synchronize()
+        with torch.cuda.stream(stream):
+            graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("kind", KINDS)
+def test_threads_that_share_a_stream_and_grow_its_buffer(kind):
+    jobs = [KINDS[kind](100 + 10 * i, size) for i, size in enumerate((1, 3, 7, 20))]
+    want = [_expected(j) for j in jobs]
+    _capi.lib().hipgpt_release_workspace()
+    stream = torch.cuda.Stream()
+    outs = [[j.empty() for _ in range(6)] for j in jobs]
+    torch.cuda.synchronize()
+    failed = []
+
+    def work(i):
+        try:
+            for out in outs[i]:
+                jobs[i].run(out, stream.cuda_stream)
+        except Exception as e:                              # noqa: BLE001
+            failed.append(e)
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(jobs))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not failed
+    for i, w in enumerate(want):
+        assert all(torch.equal(out, w) for out in outs[i])
+
+
+@pytest.mark.parametrize("kind", KINDS)
+def test_more_streams_than_buffers(kind):
+    """Twelve streams in turn, eight buffers: the ninth stream takes the buffer that was used longest ago."""
+    jobs = [KINDS[kind](200 + 10 * i, 6 + 2 * (i % 3)) for i in range(3)]
+    want = [_expected(j) for j in jobs]
+    _capi.lib().hipgpt_release_workspace()
+    streams = [torch.cuda.Stream() for _ in range(12)]
+    outs = [[jobs[(i + r) % 3].empty() for i in range(12)] for r in range(3)]
+    torch.cuda.synchronize()
+    for r in range(3):
+        for i, s in enumerate(streams):
+            jobs[(i + r) % 3].run(outs[r][i], s.cuda_stream)
+    torch.cuda.synchronize()
+    for r in range(3):
+        for i in range(12):
+            assert torch.equal(outs[r][i], want[(i + r) % 3])
