@@ -8,6 +8,18 @@
 
 namespace hipgpt {
 
+// While it lives the calling thread may allocate, free and create although some stream is being captured (in the strictest mode a
+// capture forbids that to every thread, and one that tries ends the capture): for calls on streams outside the capture.
+class OutsideCapture {
+public:
+    OutsideCapture() { cudaThreadExchangeStreamCaptureMode(&mode_); }
+    ~OutsideCapture() { cudaThreadExchangeStreamCaptureMode(&mode_); }
+    OutsideCapture(const OutsideCapture &) = delete;
+    OutsideCapture &operator=(const OutsideCapture &) = delete;
+private:
+    cudaStreamCaptureMode mode_ = cudaStreamCaptureModeRelaxed;
+};
+
 inline bool being_captured(cudaStream_t st)
 {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -66,6 +78,7 @@ public:
         Entry *mine = nullptr;
         for (Entry &x : entries_) if (x.dev == dev && x.id == id) mine = &x;
         if (!mine) {
+            const OutsideCapture outside;
             if (entries_.size() >= kMostEntries) {
                 size_t oldest = 0;
                 for (size_t i = 1; i < entries_.size(); ++i) if (entries_[i].used < entries_[oldest].used) oldest = i;
@@ -77,6 +90,7 @@ public:
         }
         mine->used = ++clock_;
         if (mine->cap < need) {
+            const OutsideCapture outside;
             if (mine->buf) cudaFree(mine->buf);
             mine->buf = nullptr;
             mine->cap = 0;
@@ -96,6 +110,7 @@ public:
     void release()
     {
         std::lock_guard<std::mutex> lock(mu_);
+        const OutsideCapture outside;
         for (Entry &x : entries_) give_back(x);
         entries_.clear();
     }
@@ -106,6 +121,8 @@ private:
 
     static cudaError_t make_side(Side &s)
     {
+        if (s.taken[1]) return cudaSuccess;          // (the last to be made)
+        const OutsideCapture outside;
         cudaError_t e = s.stream ? cudaSuccess : cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking);
         for (cudaEvent_t *ev : {&s.entered, &s.done[0], &s.done[1], &s.taken[0], &s.taken[1]})
             if (e == cudaSuccess && !*ev) e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
@@ -113,10 +130,14 @@ private:
     }
     static void give_back(Entry &x)
     {
+        int dev = x.dev;                             // an entry of another device is freed, and waited for, there
+        cudaGetDevice(&dev);
+        if (dev != x.dev) cudaSetDevice(x.dev);
         if (x.buf) cudaFree(x.buf);
         if (x.side.stream) cudaStreamDestroy(x.side.stream);
         for (cudaEvent_t ev : {x.side.entered, x.side.done[0], x.side.done[1], x.side.taken[0], x.side.taken[1]})
             if (ev) cudaEventDestroy(ev);
+        if (dev != x.dev) cudaSetDevice(dev);
     }
 
     std::mutex mu_;

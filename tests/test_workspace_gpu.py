@@ -214,3 +214,22 @@ def test_more_streams_than_buffers(kind):
     for r in range(3):
         for i in range(12):
             assert torch.equal(outs[r][i], want[(i + r) % 3])
+
+
+@pytest.mark.parametrize("kind", KINDS)
+def test_a_buffer_grows_on_one_stream_while_another_is_captured(kind):
+    """Capture in its strictest mode forbids cudaMalloc to every thread; a growing call on a stream outside the capture has to do
+    it all the same, and must not end the capture."""
+    job = KINDS[kind](300, 3)
+    want = _expected(job)
+    _capi.lib().hipgpt_release_workspace()
+    other, x, out = torch.cuda.Stream(), torch.zeros(1000, device="cuda"), job.empty()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, capture_error_mode="global"):
+        x += 1.0
+        job.run(out, other.cuda_stream)
+        x += 1.0
+    graph.replay()
+    torch.cuda.synchronize()
+    assert bool((x == 2.0).all()) and torch.equal(out, want)
