@@ -73,6 +73,7 @@ SIGNATURES = {
     "hipgpt_set_full_range": (_i, [_i]),
     "hipgpt_debug_wait_expiry": (_i, [_vp, _i, C.c_longlong, _vp]),
     "hipgpt_gpt_debug_stall_barrier": (_i, [_vp, C.c_longlong]),
+    "hipgpt_gpt_debug_cluster_rows": (_i, [_vp, _i, _i]),
     "hipgpt_last_error": (C.c_char_p, []),
     "hipgpt_version": (_i, []),
 }

@@ -817,11 +817,15 @@ int cluster_pack(const ClusterPlan &p, int E, const ClusterLayerWeights *layers,
 
 // One sequence per cluster while every cluster is resident, then two; larger batches take the launches, whose matmuls share a
 // weight among eight rows.  The ring has to hold a part (sixteen chunks at most) and more.
-int cluster_rows(const ClusterPlan &p, int B, int E, int H, int ns)
+// `positions` of the longest context: a cluster reads its sequences' keys and values with sixteen SMs, the launches theirs with all,
+// so where few clusters have long contexts the launches are ahead.  us per position of a whole run, cluster / launches (two layers): E = 256,
+// 2 sequences: 77 / 111 at 16384, 154 / 143 at 32768; 8: 134 / 189, 249 / 253; 14: 130 / 231, 241 / 340.  E = 128, 2: 78 / 89 at 32768,
+// 155 / 113 at 65536; 8: 131 / 150, 244 / 213.  The line lies between: positions x E x (sequences per cluster) / clusters = 3 x 2^20.
+int cluster_rows(const ClusterPlan &p, int B, int E, int H, int ns, int positions)
 {
     if (!p.ok) return 0;
     const int rows = B <= p.clusters_most ? 1 : (B + 1) / 2 <= p.clusters_most ? 2 : 0;
-    if (rows == 0) return 0;
+    if (rows == 0 || (long long)positions * E * rows > (3LL << 20) * ((B + rows - 1) / rows)) return 0;
     const int slots = with_kernel(E, E / H, rows, rows * H * ns, [&](auto w) { return rest_of<decltype(w)::kE, decltype(w)::kR>(H, E / H, ns, p.all_chunks).slots; });
     return slots >= 9 ? rows : 0;
 }

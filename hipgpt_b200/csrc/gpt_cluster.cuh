@@ -73,8 +73,8 @@ ClusterPlan cluster_plan(int V, int S, int E, int L, int H, int F);
 // Lays the weights (checkpoint order, device memory) out as the blocks' shares: dst [16][plan.block_bytes]; and the chunk table.
 int cluster_pack(const ClusterPlan &p, int E, const ClusterLayerWeights *layers, int L, const float *wout, uint8_t *dst, cudaStream_t st);
 void cluster_table(const ClusterPlan &p, int E, int L, uint2 *table);
-// Sequences per cluster for a batch, 0 where the batch does not fit.
-int cluster_rows(const ClusterPlan &p, int B, int E, int H, int ns);
+// Sequences per cluster for a batch with contexts of up to `positions`, 0 where the launches are to run.
+int cluster_rows(const ClusterPlan &p, int B, int E, int H, int ns, int positions);
 int launch_cluster_steps(const ClusterPlan &p, const ClusterArgs &a, int E, int rows, cudaStream_t st);
 
 }  // namespace hipgpt

@@ -650,6 +650,37 @@ int build_graph(GptDecoder &g, int B, int n_prompt, int n_new)
     return HIPGPT_OK;
 }
 
+// The cluster form's copy of the weights and its chunk table.  Where the device has no room for it the handle goes on without that form.
+int make_shares(GptDecoder &g)
+{
+    if (!g.plan.ok || g.d_shares) return HIPGPT_OK;
+    std::vector<uint2> table(g.plan.all_chunks);
+    cluster_table(g.plan, g.E, g.L, table.data());
+    auto drop = [&] {
+        cudaFree(g.d_shares);
+        cudaFree(g.d_table);
+        g.d_shares = nullptr;
+        g.d_table = nullptr;
+    };
+    if (cudaMalloc(&g.d_shares, g.plan.block_bytes * kClusterBlocks) != cudaSuccess || cudaMalloc(&g.d_table, table.size() * sizeof(uint2)) != cudaSuccess) {
+        cudaGetLastError();
+        drop();
+        g.plan.ok = false;
+        return HIPGPT_OK;
+    }
+    int rc = cluster_pack(g.plan, g.E, g.lw.data(), g.L, g.wout, g.d_shares, g.stream);
+    const cudaError_t e = cudaMemcpyAsync(g.d_table, table.data(), table.size() * sizeof(uint2), cudaMemcpyHostToDevice, g.stream);
+    if (rc == HIPGPT_OK && e != cudaSuccess) rc = fail(HIPGPT_ERR_CUDA, "copy of the chunk table: %s", cudaGetErrorString(e));
+    if (rc != HIPGPT_OK) drop();
+    return rc;
+}
+
+// Sequences per cluster for a request, 0: the graph
+int request_rows(const GptDecoder &g, int B, int positions)
+{
+    return cluster_rows(g.plan, B, g.E, g.H, decode_splits(B, g.H, g.E / g.H, g.S), positions);
+}
+
 }  // namespace
 }  // namespace hipgpt
 
@@ -741,14 +772,9 @@ int hipgpt_gpt_create(hipgpt_gpt **out, const float *h_weights, int V, int S, in
         TRY(cudaMemsetAsync(g->d_err, 0, sizeof(int), g->stream));
     }
     g->plan = cluster_plan(V, S, E, L, H, F);
-    if (g->plan.ok) {
-        TRY(cudaMalloc(&g->d_shares, g->plan.block_bytes * kClusterBlocks));
-        const int rc = cluster_pack(g->plan, E, g->lw.data(), L, g->wout, g->d_shares, g->stream);
+    if (max_batch <= 2 * g->plan.clusters_most) {    // else with the first batch that takes the cluster form
+        const int rc = make_shares(*g);
         if (rc != HIPGPT_OK) return bail(rc);
-        std::vector<uint2> table(g->plan.all_chunks);
-        cluster_table(g->plan, E, L, table.data());
-        TRY(cudaMalloc(&g->d_table, table.size() * sizeof(uint2)));
-        TRY(cudaMemcpy(g->d_table, table.data(), table.size() * sizeof(uint2), cudaMemcpyHostToDevice));
     }
     TRY(cudaStreamSynchronize(g->stream));
 #undef TRY
@@ -779,8 +805,11 @@ int hipgpt_gpt_generate(hipgpt_gpt *handle, const int *h_prompts, int B, int n_p
     }
     const bool persistent = g->mode == HIPGPT_GPT_MODE_PERSISTENT && g->persistent_ok;
     const int ns = decode_splits(B, g->H, g->E / g->H, g->S);
-    const int cluster = persistent ? 0 : cluster_rows(g->plan, B, g->E, g->H, ns);     // sequences per cluster, 0: the graph
-    int rc = persistent || cluster ? HIPGPT_OK : build_graph(*g, B, n_prompt, n_new);
+    int cluster = persistent ? 0 : request_rows(*g, B, n_prompt + n_new - 1);
+    int rc = cluster ? make_shares(*g) : HIPGPT_OK;
+    if (rc != HIPGPT_OK) return rc;
+    if (!g->plan.ok) cluster = 0;
+    if (!persistent && !cluster) rc = build_graph(*g, B, n_prompt, n_new);
     if (rc != HIPGPT_OK) return rc;
     CUDA_OK(cudaMemcpyAsync(g->d_prompts, h_prompts, (size_t)B * n_prompt * sizeof(int), cudaMemcpyHostToDevice, g->stream));
     CUDA_OK(cudaMemsetAsync(g->d_pos, 0, sizeof(int), g->stream));
@@ -862,6 +891,14 @@ int hipgpt_gpt_set_mode(hipgpt_gpt *handle, int mode)
         return fail(HIPGPT_ERR_UNSUPPORTED, "persistent form needs head_dim %% 4 == 0, head_dim <= 128 and cooperative launch");
     g->mode = mode;
     return HIPGPT_OK;
+}
+
+int hipgpt_gpt_debug_cluster_rows(hipgpt_gpt *handle, int B, int positions)
+{
+    const GptDecoder *g = reinterpret_cast<GptDecoder *>(handle);
+    if (!g) return fail(HIPGPT_ERR_NULL, "handle must not be NULL");
+    if (B <= 0 || B > g->max_batch || positions <= 0 || positions > g->S) return fail(HIPGPT_ERR_BAD_ARG, "bad request: B=%d (max %d) positions=%d S=%d", B, g->max_batch, positions, g->S);
+    return request_rows(*g, B, positions);
 }
 
 int hipgpt_gpt_debug_stall_barrier(hipgpt_gpt *handle, long long limit_cycles)

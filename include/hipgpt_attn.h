@@ -403,9 +403,12 @@ HIPGPT_API int hipgpt_set_full_range(int on);
  *   hipgpt_gpt_debug_stall_barrier  makes the NEXT persistent-mode hipgpt_gpt_generate call start with a
  *       grid-barrier counter that cannot complete and a wait limit of `limit_cycles`: every block gives up
  *       at its first barrier, the call returns HIPGPT_ERR_CUDA, and the handle stays usable.
+ *   hipgpt_gpt_debug_cluster_rows  the sequences per cluster with which the default form would run a batch of B up to
+ *       `positions` positions, 0: it would replay the graph (negative: an error code).
  */
 HIPGPT_API int hipgpt_debug_wait_expiry(float *d_canary, int n, long long limit_cycles, void *stream);
 HIPGPT_API int hipgpt_gpt_debug_stall_barrier(hipgpt_gpt *g, long long limit_cycles);
+HIPGPT_API int hipgpt_gpt_debug_cluster_rows(hipgpt_gpt *g, int B, int positions);
 
 /* Text of the calling thread's most recent failure ("" if none). */
 HIPGPT_API const char *hipgpt_last_error(void);

@@ -146,6 +146,7 @@ def test_gpu_generation_forms_agree_and_a_handle_serves_many_requests():
     (dict(V=1000, S=300, E=256, L=1, H=4, F=1024), 9, 5, 40),       # head_dim 64, two sequences per cluster, one left over
     (dict(V=1371, S=96, E=384, L=1, H=12, F=1536), 2, 4, 24),       # products in several parts
     (dict(V=300, S=700, E=128, L=1, H=2, F=512), 2, 300, 60),       # contexts of more rows than a lane asks for ahead
+    (dict(V=200, S=2100, E=128, L=1, H=4, F=512), 2, 2060, 40),     # a long context, several rounds of a unit
     (dict(V=200, S=40, E=128, L=1, H=4, F=512), 15, 2, 10),         # a batch for the replayed graph
     (dict(V=200, S=40, E=128, L=1, H=4, F=256), 2, 2, 10)])         # a feed-forward width for the replayed graph
 def test_gpu_generation_by_clusters_at_its_edges(cfg, B, n_prompt, n_new):
@@ -160,3 +161,45 @@ def test_gpu_generation_by_clusters_at_its_edges(cfg, B, n_prompt, n_new):
         assert np.array_equal(ids, ref_ids)
         assert float(np.abs(logits - ref_logits).max()) <= 1e-4
     dec.close()
+
+
+@pytest.mark.gpu
+def test_gpu_generation_by_clusters_ends_where_the_graph_is_ahead():
+    """Few sequences with long contexts, and batches that do not fit, replay the graph."""
+    pytest.importorskip("torch")
+    from hipgpt_b200 import _capi, generation
+    cfg = dict(V=64, S=32768, E=256, L=1, H=8, F=1024)
+    dec = generation.GptDecoder(synth.gpt_weights(5, **cfg), **cfg, max_batch=64)
+    rows = lambda B, positions: _capi.lib().hipgpt_gpt_debug_cluster_rows(dec._h, B, positions)      # noqa: E731
+    assert [rows(2, n) for n in (1, 16384, 24576, 24577, 32768)] == [1, 1, 1, 0, 0]
+    most = next(b for b in range(2, 65) if rows(b, 100) != 1) - 1
+    assert rows(most, 32768) == 1 and rows(2 * most, 32768) == 2 and rows(2 * most + 1, 100) == 0
+    assert rows(most + 1, 24576) == 2 and rows(most + 1, 32768) == (2 if (most + 2) // 2 * 3 >= 16 else 0)
+    assert rows(0, 5) == _capi.ERR_BAD_ARG and rows(65, 5) == _capi.ERR_BAD_ARG and rows(1, 32769) == _capi.ERR_BAD_ARG
+    dec.close()
+
+
+@pytest.mark.gpu
+def test_gpu_generation_lays_the_weights_out_again_only_for_batches_that_use_it():
+    torch = pytest.importorskip("torch")
+    from hipgpt_b200 import generation
+    cfg = dict(V=5000, S=64, E=256, L=4, H=8, F=1024)
+    w = synth.gpt_weights(6, **cfg)
+    weights = 4 * (12 * cfg["L"] * cfg["E"] ** 2 + cfg["E"] * cfg["V"])
+    prompts = {B: synth.token_ids(7, (B, 3), cfg["V"]) for B in (4, 40)}
+    free = lambda: torch.cuda.mem_get_info()[0]              # noqa: E731
+
+    def used(max_batch, *batches):
+        """Device memory that each batch's first request takes, and the ids."""
+        dec, out, ids = generation.GptDecoder(w, **cfg, max_batch=max_batch), [], []
+        for B in batches:
+            before = free()
+            ids.append(dec.generate(prompts[B], 5)[0])
+            out.append(before - free())
+        dec.close()
+        return out, ids
+    used(64, 4, 40)                                          # the kernels are loaded
+    (large, small), ids = used(64, 40, 4)
+    assert large < weights // 2 and small >= weights
+    (at_once,), again = used(4, 4)
+    assert at_once < weights // 2 and np.array_equal(ids[1], again[0]) and np.array_equal(ids[1], ids[0][:4])
