@@ -72,6 +72,7 @@ SIGNATURES = {
     "hipgpt_accuracy_notice": (_i, [C.POINTER(_i)]),
     "hipgpt_set_full_range": (_i, [_i]),
     "hipgpt_debug_wait_expiry": (_i, [_vp, _i, C.c_longlong, _vp]),
+    "hipgpt_debug_expire_wait": (_i, [_i, _i]),
     "hipgpt_gpt_debug_stall_barrier": (_i, [_vp, C.c_longlong]),
     "hipgpt_gpt_debug_cluster_rows": (_i, [_vp, _i, _i]),
     "hipgpt_last_error": (C.c_char_p, []),

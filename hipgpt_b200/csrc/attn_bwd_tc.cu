@@ -22,7 +22,8 @@
 //
 // Eight worker warps (two per TMEM lane quarter, each 32 of the tile's 64 columns) and two issuing warps, which also fetch and
 // issue side by side.  Two score buffers in TMEM: the products of tile i + 1 run while the workers are at tile i.  Every wait is bounded: on expiry the
-// block raises a flag that cuts later waits short, records a status code, skips its stores, frees its TMEM and returns.
+// block raises a flag that cuts later waits short, records a status code, skips its stores, lets what is on its way land, frees its
+// TMEM and returns.
 #include "stream_workspace.hpp"
 #include "tc_primitives.cuh"
 #include "tma_host.cuh"
@@ -41,12 +42,13 @@ constexpr uint32_t kTmemCols = 512;
 
 __device__ int g_bwd_status = 0;
 
-__device__ __noinline__ void bwd_wait_slow(uint64_t *bar, uint32_t parity, int site, volatile int *abort_flag)
+__device__ __noinline__ bool bwd_wait_slow(uint64_t *bar, uint32_t parity, int site, volatile int *abort_flag, int expire)
 {
-    if (!mbar_wait(bar, parity)) {
-        *abort_flag = 1;
-        atomicCAS(&g_bwd_status, 0, site);
-    }
+    if (!expires_now(expire, site) && mbar_wait(bar, parity)) return true;
+    *abort_flag = 1;
+    atomicCAS(&g_bwd_status, 0, site);
+    linger();
+    return false;
 }
 
 // Sizes of an operand image, in bytes.
@@ -241,7 +243,7 @@ struct RowsCfg {
 template <int D, bool CAUSAL, int STORED>
 __global__ void __launch_bounds__(kThreads, 1)
 bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *__restrict__ P, float *__restrict__ dQ,
-                float *__restrict__ lse_out, float *__restrict__ w_out, int S, int Spad, int E, int H, int nblk, float c, const __grid_constant__ PMap<STORED> p_map)
+                float *__restrict__ lse_out, float *__restrict__ w_out, int S, int Spad, int E, int H, int nblk, float c, const __grid_constant__ PMap<STORED> p_map, int expire)
 {
     using C = RowsCfg<D, STORED>;
     constexpr int TB = Img<D>::kTileBytes;
@@ -283,9 +285,12 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
     tc_fence_after();
     const uint32_t tmem = tmem_base_slot;
     // site codes: 1 resident operands, 2 K tile, 3 V tile, 4 scores, 5 workers at a tile, 6 accumulation, 7 probabilities
+    bool seen = true;                                // what this thread waited for last has come (for who asks for copies then)
     auto wait = [&](uint64_t *bar, uint32_t parity, int site) {
-        if (abort_flag || mbar_test(bar, parity)) return;
-        bwd_wait_slow(bar, parity, site, &abort_flag);
+        const int gone = abort_flag;                 // (before the test, and not in its way)
+        const bool done = mbar_test(bar, parity);
+        seen = !gone;
+        if (!gone && !done) seen = bwd_wait_slow(bar, parity, site, &abort_flag, expire);
     };
 
     if (warp >= kWorkerWarps) {
@@ -299,7 +304,7 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         auto k_slot = [&](int i) { return (i - k_first) % C::kKStages; };
         auto k_phase = [&](int i) { return (uint32_t)(((i - k_first) / C::kKStages) & 1); };
         auto fetch_k = [&](int i) {
-            if (lane == 0 && i < total) {
+            if (lane == 0 && i < total && seen) {
                 uint64_t *bar = &k_full[k_slot(i)];
                 mbar_arrive_expect_tx(bar, TB);
                 bulk_load(k_s + k_slot(i) * TB, k_img + (size_t)(i % nk) * TB, TB, bar);
@@ -307,7 +312,7 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
             __syncwarp();
         };
         auto fetch_v = [&](int i) {
-            if (lane == 0 && i < total) {
+            if (lane == 0 && i < total && seen) {
                 uint64_t *bar = &v_full[i % C::kVStages];
                 mbar_arrive_expect_tx(bar, TB);
                 bulk_load(v_s + (i % C::kVStages) * TB, v_img + (size_t)(i % nk) * TB, TB, bar);
@@ -316,7 +321,7 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         };
         // 128 rows x 64 probabilities in two boxes of 32 columns (rows and columns past S arrive as zeros)
         auto fetch_p = [&](int i) {
-            if (lane == 0 && i < total) {
+            if (lane == 0 && i < total && seen) {
                 uint64_t *bar = &p_full[i % kPStages<D>];
                 uint8_t *dst = p_s + (i % kPStages<D>) * kPTile;
                 mbar_arrive_expect_tx(bar, kPTile);
@@ -378,6 +383,7 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
             }
         }
         __syncwarp();
+        if (abort_flag) linger();
         tc_fence_before();
         __syncthreads();
         if (first) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
@@ -555,7 +561,7 @@ struct ColsCfg {
 template <int D, bool CAUSAL, int STORED>
 __global__ void __launch_bounds__(kThreads, 1)
 bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *__restrict__ P, float *__restrict__ dK, float *__restrict__ dV,
-                const float *__restrict__ lse_in, const float *__restrict__ w_in, int S, int Spad, int E, int H, int nblk, float c, const __grid_constant__ PMap<STORED> p_map)
+                const float *__restrict__ lse_in, const float *__restrict__ w_in, int S, int Spad, int E, int H, int nblk, float c, const __grid_constant__ PMap<STORED> p_map, int expire)
 {
     using C = ColsCfg<D, STORED>;
     constexpr int TB = Img<D>::kTileBytes;
@@ -593,9 +599,12 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
     tc_fence_after();
     const uint32_t tmem = tmem_base_slot;
     // site codes: 11 resident operands, 12 tile pair, 14 scores, 15 workers at a tile, 16 accumulation, 17 probabilities, 18 w and lse
+    bool seen = true;                                // what this thread waited for last has come (for who asks for copies then)
     auto wait = [&](uint64_t *bar, uint32_t parity, int site) {
-        if (abort_flag || mbar_test(bar, parity)) return;
-        bwd_wait_slow(bar, parity, site, &abort_flag);
+        const int gone = abort_flag;                 // (before the test, and not in its way)
+        const bool done = mbar_test(bar, parity);
+        seen = !gone;
+        if (!gone && !done) seen = bwd_wait_slow(bar, parity, site, &abort_flag, expire);
     };
 
     if (warp >= kWorkerWarps) {
@@ -604,7 +613,7 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         const uint8_t *q_img = img + (size_t)bh * Spad * (Img<D>::kBlock / 8);
         const uint8_t *k_img = q_img + img_bytes + (size_t)k0 * (Img<D>::kBlock / 8), *v_img = k_img + img_bytes, *g_img = q_img + 3 * img_bytes;
         auto fetch = [&](int i) {
-            if (lane == 0 && i < total) {
+            if (lane == 0 && i < total && seen) {
                 uint64_t *bar = &full[i % C::kStages];
                 uint8_t *dst = t_s + (i % C::kStages) * 2 * TB;
                 mbar_arrive_expect_tx(bar, 2 * TB);
@@ -615,7 +624,7 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         };
         // 64 queries x 128 probabilities in four boxes of 32 columns (a box per lane quarter)
         auto fetch_p = [&](int i) {
-            if (lane == 0 && i < total) {
+            if (lane == 0 && i < total && seen) {
                 uint64_t *bar = &p_full[i % kPStages<D>];
                 uint8_t *dst = p_s + (i % kPStages<D>) * kPTile;
                 mbar_arrive_expect_tx(bar, kPTile);
@@ -640,7 +649,7 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
             }
         }
         auto fetch_w = [&](int i) {
-            if (lane == 0 && i < total) {
+            if (lane == 0 && i < total && seen) {
                 uint64_t *bar = &w_full[i % C::kStages];
                 const size_t at = (size_t)bh * Spad + (size_t)(t0 + i) * kTile;
                 mbar_arrive_expect_tx(bar, (STORED ? 1 : 2) * kTile * 4);
@@ -684,6 +693,7 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
             if (elect_one()) tc_commit(&acc_done[i & 1]);
         }
         __syncwarp();
+        if (abort_flag) linger();
         tc_fence_before();
         __syncthreads();
         if (first) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
@@ -810,6 +820,7 @@ int launch_cfg(const float *g, const float *q, const float *k, const float *v, c
     uint8_t *img = ws.get();
     float *lse = reinterpret_cast<float *>(img + 4 * img_bytes), *w = lse + stat;
     const float c = 1.0f / sqrtf((float)D);
+    const int expire = take_expiry(600);
     for (long long b0 = 0; b0 < B; b0 += gb) {
         const int nb = (int)(B - b0 < gb ? B - b0 : gb);
         const size_t off = (size_t)b0 * S * E;
@@ -824,10 +835,10 @@ int launch_cfg(const float *g, const float *q, const float *k, const float *v, c
             if (rc != HIPGPT_OK) return rc;
         }
         const dim3 grid((unsigned)(nb * H * nblk));
-        e = launch_overlapped(rows, grid, dim3(kThreads), rows_smem, st, (const uint8_t *)img, img_bytes, p, dq + off, lse, w, S, Spad, E, H, nblk, c, rows_map);
+        e = launch_overlapped(rows, grid, dim3(kThreads), rows_smem, st, (const uint8_t *)img, img_bytes, p, dq + off, lse, w, S, Spad, E, H, nblk, c, rows_map, (expire & 255) <= 10 ? expire : 0);
         if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "bwd_rows_kernel launch: %s", cudaGetErrorString(e));
         e = launch_overlapped(cols, grid, dim3(kThreads), cols_smem, st, (const uint8_t *)img, img_bytes, p, dk + off, dv + off, (const float *)lse,
-                              (const float *)w, S, Spad, E, H, nblk, c, cols_map);
+                              (const float *)w, S, Spad, E, H, nblk, c, cols_map, (expire & 255) > 10 ? expire : 0);
         if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "bwd_cols_kernel launch: %s", cudaGetErrorString(e));
     }
     return HIPGPT_OK;

@@ -12,6 +12,9 @@ namespace hipgpt {
 
 // Records the calling thread's failure text and returns `code` (host side, capi.cu).
 int fail(int code, const char *fmt, ...);
+// hipgpt_debug_expire_wait: (block << 8 | site) for the calling thread's next launch of the kernels whose status codes start at `family`,
+// 0 where nothing was asked for.  Asking clears it.
+int take_expiry(int family);
 // Checks the launch that was just enqueued; HIPGPT_OK or HIPGPT_ERR_CUDA.
 int check_launch(const char *what);
 

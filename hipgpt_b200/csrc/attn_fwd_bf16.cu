@@ -79,12 +79,13 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi)
 // +3 % at S = 1024, -2 % at S = 2048, not kept.)
 
 // The polling part of a bounded wait; on expiry the block's abort flag is raised and the site recorded.
-__device__ __noinline__ void bf16_wait_slow(uint64_t *bar, uint32_t parity, int site, volatile int *abort_flag)
+__device__ __noinline__ bool bf16_wait_slow(uint64_t *bar, uint32_t parity, int site, volatile int *abort_flag)
 {
-    if (!mbar_wait(bar, parity)) {
-        *abort_flag = 1;
-        atomicCAS(&g_bf16_status, 0, site);
-    }
+    if (mbar_wait(bar, parity)) return true;
+    *abort_flag = 1;
+    atomicCAS(&g_bf16_status, 0, site);
+    linger();
+    return false;
 }
 
 template <int D>
@@ -139,9 +140,12 @@ mha_bf16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant_
     // site codes in the status word: 1 S ready, 2 O complete (rescale), 3 O complete (end), 4 K tile landed,
     // 5 P written, 6 V tile landed, 7 K stage free, 8 V stage free, 9 Q tile landed
     // (the polling loop exists once, out of line: an already completed phase costs one test)
+    bool seen = true;                                // what this thread waited for last has come (for who asks for copies then)
     auto wait = [&](uint64_t *bar, uint32_t parity, int site) {
-        if (abort_flag || mbar_test(bar, parity)) return;
-        bf16_wait_slow(bar, parity, site, &abort_flag);
+        const int gone = abort_flag;                 // (before the test, and not in its way)
+        const bool done = mbar_test(bar, parity);
+        seen = !gone;
+        if (!gone && !done) seen = bf16_wait_slow(bar, parity, site, &abort_flag);
     };
     // one arrival for the whole warp: every lane's writes are ordered before it by the warp barrier
     auto arrive = [&](uint64_t *bar) {
@@ -159,7 +163,7 @@ mha_bf16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant_
             asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
         }
         auto copy_tile = [&](const CUtensorMap *map, uint8_t *ring, uint64_t *full, int u) {
-            if (lane == 0 && u < nt) {
+            if (lane == 0 && u < nt && seen) {
                 mbar_arrive_expect_tx(&full[u % kStages], (uint32_t)TILE);
                 tma_load_3d(ring + (u % kStages) * TILE, map, (int)hcol, u * kKeys, b, &full[u % kStages]);
             }
@@ -230,6 +234,7 @@ mha_bf16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant_
             }
         }
         __syncwarp();
+        if (abort_flag) linger();
         tc_fence_before();
         __syncthreads();                             // the workers have read the output
         if (qk_role) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");

@@ -66,12 +66,13 @@ __device__ int g_head_status = 0;                // first wait site that ran out
 __device__ int g_head_notice = 0;                // bit 0: Q or K left the range in which the fp16 correction terms are exact
 
 // The polling part of a bounded wait; on expiry the block's abort flag is raised and the site recorded.
-__device__ __noinline__ void head_wait_slow(uint64_t *bar, uint32_t parity, int site, volatile int *abort_flag)
+__device__ __noinline__ bool head_wait_slow(uint64_t *bar, uint32_t parity, int site, volatile int *abort_flag)
 {
-    if (!mbar_wait_for(bar, parity, kHeadCycleLimit, kHeadPollLimit)) {
-        *abort_flag = 1;
-        atomicCAS(&g_head_status, 0, site);
-    }
+    if (mbar_wait_for(bar, parity, kHeadCycleLimit, kHeadPollLimit)) return true;
+    *abort_flag = 1;
+    atomicCAS(&g_head_status, 0, site);
+    linger();
+    return false;
 }
 
 // Largest score of one 32-column chunk; columns from `nvalid` on (counted from the tile's first column) are hidden.
@@ -202,9 +203,12 @@ mha_head_kernel(const __grid_constant__ HeadMaps maps, float *__restrict__ O, fl
     // 10 probabilities of a tile read back, 11 a buffer's product complete (unmasked)
     // (the kernel's instructions are fetched cold by every SM, so the code is kept small: the polling loop of a
     // wait exists once, out of line, behind a one-instruction test that is all an already completed phase costs)
+    bool seen = true;                                // what this thread waited for last has come (for who asks for copies then)
     auto wait = [&](uint64_t *bar, uint32_t parity, int site) {
-        if (abort_flag || mbar_test(bar, parity)) return;
-        head_wait_slow(bar, parity, site, &abort_flag);
+        const int gone = abort_flag;                 // (before the test, and not in its way)
+        const bool done = mbar_test(bar, parity);
+        seen = !gone;
+        if (!gone && !done) seen = head_wait_slow(bar, parity, site, &abort_flag);
     };
     auto arrive = [&](uint64_t *bar) {           // one arrival per warp, after every lane's writes
         __syncwarp();
@@ -222,7 +226,7 @@ mha_head_kernel(const __grid_constant__ HeadMaps maps, float *__restrict__ O, fl
         // accumulator is written by one warp only, in a fixed order: results do not depend on timing.
         const int role = warp - kHeadWorkers / 32;
         auto load_qk = [&](int hd) {
-            if (lane == 0) {
+            if (lane == 0 && seen) {
                 const int b = hd / H, c0 = (hd % H) * 32;
                 for (int t = 0; t < nq; ++t) {
                     mbar_arrive_expect_tx(&ld_k[t], kTileBytes);
@@ -239,7 +243,7 @@ mha_head_kernel(const __grid_constant__ HeadMaps maps, float *__restrict__ O, fl
             __syncwarp();
         };
         auto load_v = [&](int hd) {
-            if (lane == 0) {
+            if (lane == 0 && seen) {
                 const int b = hd / H, c0 = (hd % H) * 32;
                 for (int t = 0; t < nq; ++t) {
                     mbar_arrive_expect_tx(&ld_v[t], kTileBytes);
@@ -448,6 +452,7 @@ mha_head_kernel(const __grid_constant__ HeadMaps maps, float *__restrict__ O, fl
             }
         }
         __syncwarp();
+        if (abort_flag) linger();
         tc_fence_before();
         __syncthreads();                             // the workers have read their last output
         if (role == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");

@@ -124,7 +124,7 @@ mha_tc_kernel(const float *__restrict__ Q, const float *__restrict__ K, const fl
     // 5 P written, 6 V staged, 7 K buffer free (producer), 8 V buffer free (producer)
     auto wait = [&](uint64_t *bar, uint32_t parity, int site) {
         if (abort_flag) return;
-        if (!mbar_wait(bar, parity)) { abort_flag = 1; atomicCAS(&g_tc_status, 0, site); }
+        if (!mbar_wait(bar, parity)) { abort_flag = 1; atomicCAS(&g_tc_status, 0, site); linger(); }
     };
     auto arrive = [&](uint64_t *bar) {
         asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -189,6 +189,7 @@ mha_tc_kernel(const float *__restrict__ Q, const float *__restrict__ K, const fl
             }
         }
         __syncwarp();
+        if (abort_flag) linger();
         tc_fence_before();
         __syncthreads();                         // the workers have collected the last O_ext
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(C::kTmemCols) : "memory");

@@ -75,12 +75,13 @@ __device__ int g_tc16_status = 0;
 __device__ int g_tc16_notice = 0;                // never raised by this kernel: its operands are scaled into fp16's range
 
 // The polling part of a bounded wait; on expiry the block's abort flag is raised and the site recorded.
-__device__ __noinline__ void tc16_wait_slow(uint64_t *bar, uint32_t parity, int site, volatile int *abort_flag)
+__device__ __noinline__ bool tc16_wait_slow(uint64_t *bar, uint32_t parity, int site, volatile int *abort_flag)
 {
-    if (!mbar_wait(bar, parity)) {
-        *abort_flag = 1;
-        atomicCAS(&g_tc16_status, 0, site);
-    }
+    if (mbar_wait(bar, parity)) return true;
+    *abort_flag = 1;
+    atomicCAS(&g_tc16_status, 0, site);
+    linger();
+    return false;
 }
 
 // Largest of 32 scores; columns from `nvalid` on (counted from the chunk's first column `col0`) are hidden.
@@ -285,9 +286,12 @@ mha_tc16_kernel(const uint8_t *__restrict__ kimg, const uint8_t *__restrict__ vi
     // site codes in the status word: 1 S ready, 2 O complete (rescale), 3 O complete (end), 4 K stage landed,
     // 5 P written, 6 V stage landed, 7 K stage free, 8 V stage free
     // (the polling loop exists once, out of line: an already completed phase costs one test)
+    bool seen = true;                                // what this thread waited for last has come (for who asks for copies then)
     auto wait = [&](uint64_t *bar, uint32_t parity, int site) {
-        if (abort_flag || mbar_test(bar, parity)) return;
-        tc16_wait_slow(bar, parity, site, &abort_flag);
+        const int gone = abort_flag;                 // (before the test, and not in its way)
+        const bool done = mbar_test(bar, parity);
+        seen = !gone;
+        if (!gone && !done) seen = tc16_wait_slow(bar, parity, site, &abort_flag);
     };
     // one arrival for the whole warp: every lane's writes are ordered before it by the warp barrier
     auto arrive = [&](uint64_t *bar) {
@@ -314,7 +318,7 @@ mha_tc16_kernel(const uint8_t *__restrict__ kimg, const uint8_t *__restrict__ vi
         }
         // one lane asks for a whole packed stage (u counts staged K tiles: the second sweep reads the tiles again)
         auto copy_k = [&](int u) {
-            if (lane == 0 && u < nk) {
+            if (lane == 0 && u < nk && seen) {
                 const int kt = u < nt ? u : u - nt;
                 mbar_arrive_expect_tx(&k_full[u % KST], (uint32_t)C::kK16Stage);
                 bulk_load(k_16 + (u % KST) * C::kK16Stage, kimg + ((size_t)bh * ntk + kt) * C::kK16Stage, (uint32_t)C::kK16Stage, &k_full[u % KST]);
@@ -322,7 +326,7 @@ mha_tc16_kernel(const uint8_t *__restrict__ kimg, const uint8_t *__restrict__ vi
             __syncwarp();
         };
         auto copy_v = [&](int u) {
-            if (lane == 0 && u < nt) {
+            if (lane == 0 && u < nt && seen) {
                 mbar_arrive_expect_tx(&v_full[u % VST], (uint32_t)C::kV16Stage);
                 bulk_load(v_16 + (u % VST) * C::kV16Stage, vimg + ((size_t)bh * ntk + u) * C::kV16Stage, (uint32_t)C::kV16Stage, &v_full[u % VST]);
             }
@@ -399,6 +403,7 @@ mha_tc16_kernel(const uint8_t *__restrict__ kimg, const uint8_t *__restrict__ vi
             }
         }
         __syncwarp();
+        if (abort_flag) linger();
         tc_fence_before();
         __syncthreads();                             // the workers have read the output
         if (qk_role) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");

@@ -16,6 +16,14 @@ namespace hipgpt {
 
 namespace {
 thread_local char g_err[512] = "";
+thread_local int g_expire_family = 0, g_expire = 0;
+}
+
+int take_expiry(int family)
+{
+    if (g_expire_family != family) return 0;
+    g_expire_family = 0;
+    return g_expire;
 }
 
 int fail(int code, const char *fmt, ...)
@@ -437,6 +445,15 @@ int hipgpt_shard_range(int B, int world, int rank, int *b_begin, int *b_end)
     const int base = B / world, extra = B % world;
     *b_begin = rank * base + (rank < extra ? rank : extra);
     *b_end = *b_begin + base + (rank < extra ? 1 : 0);
+    return HIPGPT_OK;
+}
+
+int hipgpt_debug_expire_wait(int code, int block)
+{
+    const int family = code / 100 * 100, site = code % 100;
+    if ((family != 500 && family != 600) || site == 0 || block < 0 || block >= 1 << 22) return fail(HIPGPT_ERR_BAD_ARG, "no wait has code %d, or block %d", code, block);
+    g_expire_family = family;
+    g_expire = block << 8 | site;
     return HIPGPT_OK;
 }
 

@@ -24,7 +24,8 @@
 //                        output row = TMEM lane) add the halves, take the scales out, add the bias and store one tile
 //                        while the products of the next one run.
 // Rows, columns and depth beyond the matrices are zeros in the images; stores are bounded by M and K.
-// Every wait is bounded: on expiry the block records a status code, skips its stores, frees its TMEM and returns.
+// Every wait is bounded: on expiry the block records a status code, skips its stores, lets what is on its way land, frees its TMEM
+// and returns.
 #include "stream_workspace.hpp"
 #include "tc_primitives.cuh"
 
@@ -218,12 +219,13 @@ __global__ void __launch_bounds__(128) gemm_pack_b_kernel(const float *__restric
     }
 }
 
-__device__ __noinline__ void gemm_wait_slow(uint64_t *bar, uint32_t parity, int site, volatile int *abort_flag)
+__device__ __noinline__ bool gemm_wait_slow(uint64_t *bar, uint32_t parity, int site, volatile int *abort_flag, int expire)
 {
-    if (!mbar_wait(bar, parity)) {
-        *abort_flag = 1;
-        atomicCAS(&g_gemm_status, 0, site);
-    }
+    if (!expires_now(expire, site) && mbar_wait(bar, parity)) return true;
+    *abort_flag = 1;
+    atomicCAS(&g_gemm_status, 0, site);
+    linger();
+    return false;
 }
 
 // KS > 1: the slices of a tile are shared by the KS blocks of a cluster (each one tile, no second one), for products with too few
@@ -239,7 +241,7 @@ __device__ __forceinline__ void cluster_sync()
 template <int KS>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_tc_kernel(const uint8_t *__restrict__ aimg, const uint8_t *__restrict__ bimg, const float *__restrict__ row_inv, const float *__restrict__ b_amax,
-               const float *__restrict__ bias, float *__restrict__ C, int M, int K, int KT, int NT, int ntiles)
+               const float *__restrict__ bias, float *__restrict__ C, int M, int K, int KT, int NT, int ntiles, int expire)
 {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *base = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -260,9 +262,12 @@ gemm_tc_kernel(const uint8_t *__restrict__ aimg, const uint8_t *__restrict__ bim
     }
     __syncthreads();
     // site codes in the status word: 1 stage landed, 2 stage free, 3 accumulator complete, 4 accumulator drained
+    bool seen = true;                                // what this thread waited for last has come (for who asks for copies then)
     auto wait = [&](uint64_t *bar, uint32_t parity, int site) {
-        if (abort_flag || mbar_test(bar, parity)) return;
-        gemm_wait_slow(bar, parity, site, &abort_flag);
+        const int gone = abort_flag;                 // (before the test, and not in its way)
+        const bool done = mbar_test(bar, parity);
+        seen = !gone;
+        if (!gone && !done) seen = gemm_wait_slow(bar, parity, site, &abort_flag, expire);
     };
     // The block takes output tiles blockIdx.x, + gridDim.x, ... (column tile fastest: blocks that run side by side share
     // the rows of A).  Stages are counted through all tiles (g), accumulators alternate between two halves of TMEM, so
@@ -285,7 +290,7 @@ gemm_tc_kernel(const uint8_t *__restrict__ aimg, const uint8_t *__restrict__ bim
             for (int kt = kt0; kt < kt1; ++kt, ++g) {
                 const int s = g % kStages;
                 if (g >= kStages) wait(&empty[s], (uint32_t)((g / kStages - 1) & 1), 2);     // the products that read the stage have completed
-                if (lane == 0) {
+                if (lane == 0 && seen) {
                     mbar_arrive_expect_tx(&full[s], (uint32_t)(kAStage + kBStage));
                     const uint8_t *asrc = aimg + ((size_t)mt * KT + kt) * kAStage, *bsrc = bimg + ((size_t)nt * KT + kt) * kBStage;
                     bulk_load(a_s + s * kAStage, asrc, kABlk, &full[s]);
@@ -297,6 +302,7 @@ gemm_tc_kernel(const uint8_t *__restrict__ aimg, const uint8_t *__restrict__ bim
             }
         }
         __syncwarp();
+        if (abort_flag) linger();
         if constexpr (KS > 1) { cluster_sync(); cluster_sync(); }
         tc_fence_before();
         __syncthreads();                              // the last output has been read from TMEM
@@ -335,6 +341,7 @@ gemm_tc_kernel(const uint8_t *__restrict__ aimg, const uint8_t *__restrict__ bim
             if (elect_one()) tc_commit(&acc_full[i & 1]);
         }
         __syncwarp();
+        if (abort_flag) linger();
         if constexpr (KS > 1) { cluster_sync(); cluster_sync(); }
         tc_fence_before();
         __syncthreads();
@@ -521,7 +528,7 @@ int pack_a_and_multiply(const float *A, const uint8_t *bimg, const float *b_amax
     const unsigned grid = ks > 1 ? (unsigned)(ntiles * ks) : (unsigned)(ntiles < sms ? ntiles : sms);      // ks = 1: one block per SM, each takes tiles in turn
     const auto kern = ks == 1 ? gemm_tc_kernel<1> : ks == 2 ? gemm_tc_kernel<2> : ks == 3 ? gemm_tc_kernel<3> : gemm_tc_kernel<4>;
     e = launch_overlapped_clusters(kern, ks, dim3(grid), dim3(kGemmThreads), kGemmSmem, st, (const uint8_t *)aimg, bimg,
-                                   (const float *)row_inv, b_amax, bias, C, M, K, KT, NT, (int)ntiles);
+                                   (const float *)row_inv, b_amax, bias, C, M, K, KT, NT, (int)ntiles, take_expiry(500));
     if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "gemm_tc_kernel launch: %s", cudaGetErrorString(e));
     return check_launch("gemm_tc_kernel");
 }

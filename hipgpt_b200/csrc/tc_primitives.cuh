@@ -57,6 +57,19 @@ __device__ __forceinline__ bool mbar_wait_for(uint64_t *bar, uint32_t parity, lo
 }
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity) { return mbar_wait_for(bar, parity, kCycleLimit, kSpinLimit); }
 
+// What a kernel does after a wait has run out.  No copy is asked for any more by a thread that has not seen its stage free: the
+// stage's barrier may still wait for the bytes of the copy before.  And shared memory and TMEM are not given back while copies and
+// products may be on their way to them: the thread whose wait ran out, and the warps that issue, once they have come to their end,
+// stay for longer than either can take (4 x 10^6 cycles, 2 ms).
+__device__ __forceinline__ void linger()
+{
+    const long long t0 = clock64();
+    while (clock64() - t0 < 4000000) {}
+}
+
+// Test hook (hipgpt_debug_expire_wait): whether the wait at `site` is to run out at once in this block.  0: none.
+__device__ __forceinline__ bool expires_now(int expire, int site) { return (expire & 255) == site && expire >> 8 == (int)blockIdx.x; }
+
 // One arrival that also announces `bytes` of asynchronous copies which will complete on this barrier.
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t *bar, uint32_t bytes)
 {

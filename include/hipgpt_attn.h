@@ -400,6 +400,9 @@ HIPGPT_API int hipgpt_set_full_range(int on);
  *       (bounded mbarrier wait, abort flag, status word, stores skipped) on a barrier at which nothing
  *       arrives, with a limit of `limit_cycles` SM cycles (at most 2^24, a few milliseconds).  Afterwards
  *       hipgpt_kernel_status() reports 907 and d_canary[0..n) is untouched.
+ *   hipgpt_debug_expire_wait  in the calling thread's next call of a tensor-core projection (code 501 ... 504) or of a tensor-core
+ *       backward (601 ... 618) the wait that hipgpt_kernel_status reports with this code runs out at once in block `block` of
+ *       each of the call's launches that has it, if it has to wait at all.
  *   hipgpt_gpt_debug_stall_barrier  makes the NEXT persistent-mode hipgpt_gpt_generate call start with a
  *       grid-barrier counter that cannot complete and a wait limit of `limit_cycles`: every block gives up
  *       at its first barrier, the call returns HIPGPT_ERR_CUDA, and the handle stays usable.
@@ -407,6 +410,7 @@ HIPGPT_API int hipgpt_set_full_range(int on);
  *       `positions` positions, 0: it would replay the graph (negative: an error code).
  */
 HIPGPT_API int hipgpt_debug_wait_expiry(float *d_canary, int n, long long limit_cycles, void *stream);
+HIPGPT_API int hipgpt_debug_expire_wait(int code, int block);
 HIPGPT_API int hipgpt_gpt_debug_stall_barrier(hipgpt_gpt *g, long long limit_cycles);
 HIPGPT_API int hipgpt_gpt_debug_cluster_rows(hipgpt_gpt *g, int B, int positions);
 

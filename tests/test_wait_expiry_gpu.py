@@ -54,3 +54,83 @@ def test_a_stalled_grid_barrier_ends_the_persistent_generation_call_with_an_erro
         dec.generate(prompts, 10)
     assert np.array_equal(dec.generate(prompts, 10)[0], want)                  # the handle stays usable
     dec.close()
+
+
+def _expired(code, block, call, *outs):
+    """The outputs of `call` with the wait of this code run out in one block, canaries where nothing was stored."""
+    for o in outs:
+        o.fill_(-7.0)
+    _capi.check(_capi.lib().hipgpt_debug_expire_wait(code, block))
+    call()
+    torch.cuda.synchronize()
+    assert _status() == code and _status() == 0
+    return [o.clone() for o in outs]
+
+
+@pytest.mark.parametrize("code,block", [(501, 0), (501, 147), (502, 3), (503, 5)])
+def test_an_expired_wait_of_a_projection_stores_none_of_the_blocks_tiles(code, block):
+    """20 x 20 tiles: a block has two or three, none of them may be stored; the others and the next call are as ever."""
+    M, N, K = 2560, 320, 2560
+    a, w = (torch.randn(*s, generator=torch.Generator(device="cuda").manual_seed(3), device="cuda") for s in ((M, N), (N, K)))
+    out = torch.empty(M, K, device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+    run = lambda: _capi.check(_capi.lib().hipgpt_matmul_tc(a.data_ptr(), w.data_ptr(), None, out.data_ptr(), M, N, K, st))      # noqa: E731
+    run()
+    want = out.clone()
+    got, = _expired(code, block, run, out)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    for t in range(400):
+        piece = (slice(t // 20 * 128, t // 20 * 128 + 128), slice(t % 20 * 128, t % 20 * 128 + 128))
+        if t % sms == block:
+            assert bool((got[piece] == -7.0).all()), t
+        else:
+            assert torch.equal(got[piece], want[piece]), t
+    run()
+    assert torch.equal(out, want) and _status() == 0
+    assert _capi.lib().hipgpt_debug_expire_wait(401, 0) == _capi.ERR_BAD_ARG
+
+
+BWD_SHAPE = B_, H_, S_ = 2, 2, 300
+
+
+def _backward(D, stored):
+    E = H_ * D
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    qkv, g = torch.randn(3, B_ * S_, E, generator=gen, device="cuda"), torch.randn(B_ * S_, E, generator=gen, device="cuda")
+    p, grad, st = None, torch.empty(3, B_ * S_, E, device="cuda"), torch.cuda.current_stream().cuda_stream
+    if stored:
+        p, out = torch.empty(B_, H_, S_, S_, device="cuda"), torch.empty(B_ * S_, E, device="cuda")
+        _capi.check(_capi.lib().hipgpt_mha_forward_planes(qkv.data_ptr(), out.data_ptr(), p.data_ptr(), B_, S_, E, H_, 0, st))
+    run = lambda: _capi.check(_capi.lib().hipgpt_mha_backward_planes(g.data_ptr(), qkv.data_ptr(), p.data_ptr() if stored else None,       # noqa: E731
+                                                                     grad.data_ptr(), B_, S_, E, H_, 0, st))
+    return run, grad, (qkv, g, p)
+
+
+def _blocks(x, D):
+    """Gradients [3][B S][E] as [3][B][block of 128 rows][H][row, D]."""
+    x = x.view(3, B_, S_, H_, D)
+    return [[x[i, :, j:j + 128].permute(0, 2, 1, 3) for j in range(0, S_, 128)] for i in range(3)]
+
+
+@pytest.mark.parametrize("D", [32, 64])
+@pytest.mark.parametrize("stored", [True, False])
+@pytest.mark.parametrize("code", [601, 604, 605, 606, 611, 614, 615, 616])
+def test_an_expired_wait_of_the_backward_stores_none_of_the_blocks_rows(D, stored, code):
+    """Block 1: the second 128 queries (dQ) or keys (dK, dV) of the first head."""
+    if stored and code == 614:
+        code = 617                                           # the stored probabilities come later than the scores
+    run, grad, keep = _backward(D, stored)
+    run()
+    want = grad.clone()
+    got, = _expired(code, 1, run, grad)
+    touched = (0,) if code < 610 else (1, 2)
+    for i in range(3):
+        for j, (g, w) in enumerate(zip(_blocks(got, D)[i], _blocks(want, D)[i])):
+            if i in touched and j == 1:
+                assert bool((g[0, 0] == -7.0).all())
+                g[0, 0] = w[0, 0]
+            if code < 610 and i > 0:
+                g[0, 0] = w[0, 0]                            # the first head's columns depend on the rows that were left out
+            assert torch.equal(g, w), (i, j)
+    run()
+    assert torch.equal(grad, want) and _status() == 0
