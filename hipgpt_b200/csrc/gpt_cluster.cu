@@ -20,8 +20,10 @@
 //   * The logits are formed where an id is picked from them: not at prompt positions before the last.
 // Buffers are received into once per layer (or step); a sender can be at most one product ahead of the slowest receiver, because
 // each product needs the columns of all blocks, so a buffer is never overwritten while it is read.
-// Waits on mbarriers are bounded: on expiry the block raises a flag that cuts its later waits short and sets the error word; the
-// steps then run out without waiting.
+// Waits on mbarriers are bounded: on expiry the block raises a flag that cuts its later waits short and sets the error word, goes on
+// without waiting to the end of the step (or of four layers) and sends nothing after it; the other blocks' waits then run
+// out too, and all meet at the barriers of the remaining steps and leave.  (A barrier whose phase has not been seen complete is not
+// opened again, and the bytes that nobody waits for stay within eight layers' worth, at most 90 KB each: an mbarrier counts 2^20.)
 //
 // Measured at the default model (E=256 L=8 H=8 V=5000), batch 8: 73 us per step (the replayed graph: 318), batch 1: 68 (256).  A
 // step is 42 products of 400 - 450 ns each, attention a third of a layer.  Sizes are template parameters because the chain is
@@ -38,6 +40,7 @@ constexpr int kThreads = 512;
 constexpr int kWarps = 16;
 constexpr int kMostSlots = 24;
 constexpr int kSmemMost = 232448 - 1024;
+constexpr int kLayersChecked = 4;                // layers between two looks at whether a wait has run out
 constexpr int kAhead = 4;                        // key / value rows per lane asked for ahead of the projection
 
 __device__ __forceinline__ uint32_t peer_addr(uint32_t addr, int rank)
@@ -57,13 +60,20 @@ __device__ __forceinline__ void send2(uint32_t addr, uint32_t bar, uint32_t x, u
     asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];" ::"r"(addr), "r"(x), "r"(y), "r"(bar) : "memory");
 }
 
-// The polling part of a wait, out of line: the kernel's code should stay in the instruction cache.
-__device__ __noinline__ void cluster_wait_slow(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int *err)
+// What the waits of a block share
+struct Waits {
+    volatile int gone;                               // a wait has run out: later ones are cut short
+    int *err;
+    long long limit;                                 // SM cycles
+    const uint64_t *expire;                          // test hook: the barrier whose wait runs out at once
+};
+// The polling part of a wait, out of line: the kernel's code should stay in the instruction cache.  1: it, or one before it, has run out.
+__device__ __noinline__ int cluster_wait_slow(uint64_t *bar, uint32_t parity, Waits *w)
 {
-    if (!mbar_wait(bar, parity)) {
-        *abort_flag = 1;
-        atomicExch(err, 1);
-    }
+    if (!w->gone && bar != w->expire && mbar_wait_for(bar, parity, w->limit, kSpinLimit)) return 0;
+    if (!w->gone) atomicExch(w->err, 1);
+    w->gone = 1;
+    return 1;
 }
 
 struct Part {
@@ -134,8 +144,9 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
     __shared__ uint64_t hop[6];                      // qkv, attention records, xa, ff, xb, first maxima
     __shared__ float2 stats[R];                      // a row's mean and 1 / sqrt(variance + eps)
     __shared__ int next_id[R];
-    __shared__ volatile int abort_flag;
+    __shared__ Waits waits;
     enum { kQkv, kRec, kXa, kFf, kXb, kAm };
+    static_assert(kRec == kHopRecords, "");
 
     const int tid = threadIdx.x, lane = tid & 31;
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
@@ -158,7 +169,10 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
     for (int i = tid; i < lay.table; i += kThreads) sm[i] = 0.0f;         // rows that the cluster does not have stay zero
     for (int i = tid; i < plan.all_chunks; i += kThreads) table[i] = a.table[i];
     if (tid == 0) {
-        abort_flag = 0;
+        waits.gone = 0;
+        waits.err = a.err;
+        waits.limit = a.wait_cycles;
+        waits.expire = blockIdx.x == 0 && a.expire_hop >= 0 ? &hop[a.expire_hop] : nullptr;
         for (int i = 0; i < lay.slots; ++i) mbar_init(&full[i], 1);
         for (int i = 0; i < 6; ++i) { mbar_init(&hop[i], 1); mbar_arrive_expect_tx(&hop[i], tx(i)); }
     }
@@ -166,15 +180,19 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
     asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 
     auto wait = [&](uint64_t *bar, uint32_t parity) {
-        if (mbar_test(bar, parity) || abort_flag) return;
-        cluster_wait_slow(bar, parity, &abort_flag, a.err);
+        if (!mbar_test(bar, parity)) cluster_wait_slow(bar, parity, &waits);
     };
     // what a hop delivers is complete; one thread opens the barrier's next phase
     uint32_t hop_phase = 0;                          // a bit per hop
     auto receive = [&](int i) {
-        wait(&hop[i], (hop_phase >> i) & 1u);
+        int gone = waits.gone;
+        if (!mbar_test(&hop[i], (hop_phase >> i) & 1u)) gone = cluster_wait_slow(&hop[i], (hop_phase >> i) & 1u, &waits);
         hop_phase ^= 1u << i;
-        if (tid == kThreads - 1) mbar_arrive_expect_tx(&hop[i], tx(i));
+        if (tid == kThreads - 1 && !gone) mbar_arrive_expect_tx(&hop[i], tx(i));
+    };
+    // after a wait that has run out: through the barriers of this step and those to come with the others
+    auto leave = [&](int step) {
+        for (; step < a.nsteps; ++step) asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
     };
     // an address of this block -> the same place in four of the blocks (those this thread stores into)
     const int dq = tid & 3;
@@ -192,7 +210,7 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
         const bool wraps = pos >= len;
         if (wraps) pos -= len;
         if (slot >= lay.slots) slot -= lay.slots;
-        if (lane < n && f_step + (wraps ? 1 : 0) < a.nsteps) {
+        if (lane < n && f_step + (wraps ? 1 : 0) < a.nsteps && !waits.gone) {           // (no copy onto one that nobody saw land)
             const uint2 t = table[pos];
             mbar_arrive_expect_tx(&full[slot], t.y);
             bulk_load(ring + slot * C::kSlot, share + t.x, t.y, &full[slot]);
@@ -587,6 +605,11 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
         per = (p + ns) / ns;
 #pragma unroll 1
         for (int l = 0; l < a.L; ++l) {
+            if (l > 0 && l % kLayersChecked == 0 && __syncthreads_or(waits.gone)) {
+                leave(step);
+                step = a.nsteps;
+                break;
+            }
             ask(first_unit, l, p, 0);
 #pragma unroll 1
             for (int pt = 0; pt < cluster_job_of(kJobQkv, E, 0).parts; ++pt)
@@ -603,6 +626,7 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
             for (int pt = 0; pt < cluster_job_of(kJobF2, E, 0).parts; ++pt)
                 finish(Job<kJobF2>(), pt, product(Job<kJobF2>(), ff, [&] { if (pt == 0) receive(kFf); }), 0, 0);
         }
+        if (step >= a.nsteps) break;
         receive(kXb);
         const bool head = p >= a.n_prompt - 1, last = step + 1 == a.nsteps;
         if (head) {
@@ -670,12 +694,12 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
         // the keys and values of this position reach the other blocks before the next one is attended to; the barrier also keeps a
         // block from leaving while others still store into it
         asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
-        __syncthreads();
+        if (__syncthreads_or(waits.gone)) {
+            leave(step + 1);
+            break;
+        }
     }
-    if (abort_flag) {                                // let copies in flight land before the shared memory is given back
-        const long long t0 = clock64();
-        while (clock64() - t0 < 4000000) {}
-    }
+    if (waits.gone) linger();
 }
 
 // One chunk per block of this grid: (chunk, owner).  Columns and inner indices past the matrix (or the owner's share) are zeros.

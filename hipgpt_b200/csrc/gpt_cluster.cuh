@@ -7,6 +7,8 @@
 namespace hipgpt {
 
 constexpr int kClusterBlocks = 16;
+constexpr long long kClusterWaitCycles = 1LL << 31;    // about a second
+constexpr int kHopRecords = 1;                         // the attention records among the kernel's hops
 
 // One matrix of the model, cut for the sixteen blocks: block c owns columns [c * nc, (c + 1) * nc) in parts of `width` columns, and
 // reads a part in chunks of 2^seg_shift of the sixteen segments of the inner dimension.  A segment of a part lies as
@@ -64,6 +66,8 @@ struct ClusterArgs {
     const int *prompts;
     int V, S, L, H, B, n_prompt, n_new, ns;
     int p0, nsteps;              // first position, number of positions
+    long long wait_cycles;       // limit of a wait
+    int expire_hop;              // test hook: the hop whose wait runs out at once in the first block, -1: none
 };
 
 struct ClusterLayerWeights { const float *wqkv, *wo, *w1, *w2, *bqkv, *bo, *b1, *b2, *g1, *be1, *g2, *be2; };

@@ -566,8 +566,8 @@ struct GptDecoder {
     uint8_t *d_shares = nullptr;
     uint2 *d_table = nullptr;
     cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};   // start, prompt done, all done
-    // test hook (hipgpt_gpt_debug_stall_barrier): the next persistent call starts with an arrival counter
-    // that can never complete and this wait limit, so that the barrier's give-up path runs
+    // test hook (hipgpt_gpt_debug_stall_barrier): with this wait limit the next persistent call starts with an arrival counter that can
+    // never complete, the next call by clusters with a wait of its first block that runs out, so that the give-up path runs
     bool stall_next = false;
     long long stall_limit = 0;
 };
@@ -849,9 +849,18 @@ int hipgpt_gpt_generate(hipgpt_gpt *handle, const int *h_prompts, int B, int n_p
         a.logits = g->d_logits; a.ids = g->d_ids; a.out_ids = g->d_out; a.err = g->d_err; a.prompts = g->d_prompts;
         a.V = g->V; a.S = g->S; a.L = g->L; a.H = g->H;
         a.B = B; a.n_prompt = n_prompt; a.n_new = n_new; a.ns = ns;
+        a.wait_cycles = kClusterWaitCycles;
+        a.expire_hop = -1;
+        if (g->stall_next) {
+            a.wait_cycles = g->stall_limit;
+            a.expire_hop = kHopRecords;
+            g->stall_next = false;
+        }
         a.nsteps = n_prompt;
         if ((rc = launch_cluster_steps(g->plan, a, g->E, cluster, g->stream)) != HIPGPT_OK) return rc;
         CUDA_OK(cudaEventRecord(e1, g->stream));
+        a.wait_cycles = kClusterWaitCycles;
+        a.expire_hop = -1;
         a.p0 = n_prompt;
         a.nsteps = n_new - 1;
         if (a.nsteps > 0 && (rc = launch_cluster_steps(g->plan, a, g->E, cluster, g->stream)) != HIPGPT_OK) return rc;
@@ -906,7 +915,7 @@ int hipgpt_gpt_debug_stall_barrier(hipgpt_gpt *handle, long long limit_cycles)
     GptDecoder *g = reinterpret_cast<GptDecoder *>(handle);
     if (!g) return fail(HIPGPT_ERR_NULL, "handle must not be NULL");
     if (limit_cycles <= 0 || limit_cycles > kBarrierLimitCycles) return fail(HIPGPT_ERR_BAD_ARG, "limit of %lld cycles out of range", limit_cycles);
-    if (!(g->mode == HIPGPT_GPT_MODE_PERSISTENT && g->persistent_ok)) return fail(HIPGPT_ERR_UNSUPPORTED, "the handle is not in the persistent mode");
+    if (!(g->mode == HIPGPT_GPT_MODE_PERSISTENT ? g->persistent_ok : g->plan.ok)) return fail(HIPGPT_ERR_UNSUPPORTED, "the handle's form has no waits of its own");
     g->stall_next = true;
     g->stall_limit = limit_cycles;
     return HIPGPT_OK;

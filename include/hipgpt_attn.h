@@ -403,9 +403,10 @@ HIPGPT_API int hipgpt_set_full_range(int on);
  *   hipgpt_debug_expire_wait  in the calling thread's next call of a tensor-core projection (code 501 ... 504) or of a tensor-core
  *       backward (601 ... 618) the wait that hipgpt_kernel_status reports with this code runs out at once in block `block` of
  *       each of the call's launches that has it, if it has to wait at all.
- *   hipgpt_gpt_debug_stall_barrier  makes the NEXT persistent-mode hipgpt_gpt_generate call start with a
- *       grid-barrier counter that cannot complete and a wait limit of `limit_cycles`: every block gives up
- *       at its first barrier, the call returns HIPGPT_ERR_CUDA, and the handle stays usable.
+ *   hipgpt_gpt_debug_stall_barrier  makes the NEXT hipgpt_gpt_generate call give up: in the persistent mode it starts with a
+ *       grid-barrier counter that cannot complete, and every block gives up at its first barrier; by clusters the first block's
+ *       first wait for other blocks' attention runs out at once, and the others' waits for what it then no longer sends.  Waits
+ *       are limited to `limit_cycles`, the call returns HIPGPT_ERR_CUDA, and the handle stays usable.
  *   hipgpt_gpt_debug_cluster_rows  the sequences per cluster with which the default form would run a batch of B up to
  *       `positions` positions, 0: it would replay the graph (negative: an error code).
  */

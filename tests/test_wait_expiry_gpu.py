@@ -56,6 +56,24 @@ def test_a_stalled_grid_barrier_ends_the_persistent_generation_call_with_an_erro
     dec.close()
 
 
+def test_stalled_clusters_end_the_generation_call_with_an_error():
+    """One block's wait runs out; it sends nothing after its layer, so the other blocks' waits run out too, and all leave."""
+    from hipgpt_b200.generation import GptDecoder
+    cfg = dict(V=131, S=64, E=128, L=3, H=4, F=512)
+    w = synth.gpt_weights(9, **cfg)
+    prompts = synth.token_ids(10, (9, 6), cfg["V"])
+    dec = GptDecoder(w, **cfg, max_batch=9)
+    assert _capi.lib().hipgpt_gpt_debug_cluster_rows(dec._h, 9, 20) > 0
+    want = dec.generate(prompts, 15)
+    for _ in range(2):
+        _capi.check(_capi.lib().hipgpt_gpt_debug_stall_barrier(dec._h, 400000))      # ~0.2 ms
+        with pytest.raises(_capi.HipGPTError, match="inside a cluster"):
+            dec.generate(prompts, 15)
+        again = dec.generate(prompts, 15)
+        assert np.array_equal(again[0], want[0]) and np.array_equal(again[1], want[1])    # the handle stays usable
+    dec.close()
+
+
 def _expired(code, block, call, *outs):
     """The outputs of `call` with the wait of this code run out in one block, canaries where nothing was stored."""
     for o in outs:
