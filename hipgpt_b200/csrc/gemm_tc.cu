@@ -25,7 +25,7 @@
 //                        while the products of the next one run.
 // Rows, columns and depth beyond the matrices are zeros in the images; stores are bounded by M and K.
 // Every wait is bounded: on expiry the block records a status code, skips its stores, lets what is on its way land, frees its TMEM
-// and returns.
+// and returns; the blocks that share its tile store none of it.
 #include "stream_workspace.hpp"
 #include "tc_primitives.cuh"
 
@@ -363,7 +363,7 @@ gemm_tc_kernel(const uint8_t *__restrict__ aimg, const uint8_t *__restrict__ bim
         wait(&acc_full[i & 1], (uint32_t)((i / 2) & 1), 3);
         tc_fence_after();
         const int c_base = nt * kTN;
-        const bool live = !abort_flag;
+        bool live = !abort_flag;
         // 32 columns at a time; the warp turns its 32 x 32 piece through shared memory (16-byte chunk c of row r at
         // r * 128 + ((c ^ (r & 7)) * 16)) so that a store instruction writes four rows of 128 contiguous bytes instead
         // of 32 rows of 16
@@ -375,7 +375,13 @@ gemm_tc_kernel(const uint8_t *__restrict__ aimg, const uint8_t *__restrict__ bim
             return (uint32_t)((place * 2 + lc) * (8 * kTM * 16) + r * 16);
         };
         if constexpr (KS > 1) {
-            cluster_sync();                           // every block of the cluster is done with its operand stages
+            cluster_sync();                           // every block of the cluster is done with its operand stages, and with its waits
+            // a tile whose sum is unfinished in one block is stored by none (the loads are used behind the exchange)
+            uint32_t gone[KS];
+#pragma unroll
+            for (int q = 0; q < KS; ++q)
+                asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %1, %2;\n\tld.shared::cluster.b32 %0, [a];\n\t}"
+                             : "=r"(gone[q]) : "r"(smem_u32(const_cast<const int *>(&abort_flag))), "r"(q) : "memory");
 #pragma unroll 1
             for (int c = 0; c < 4; ++c) {
                 const int owner = c * KS / 4;
@@ -391,6 +397,8 @@ gemm_tc_kernel(const uint8_t *__restrict__ aimg, const uint8_t *__restrict__ bim
                     asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(dst + j * (kTM * 16)), "f"(a[4 * j] + b[4 * j]), "f"(a[4 * j + 1] + b[4 * j + 1]),
                                  "f"(a[4 * j + 2] + b[4 * j + 2]), "f"(a[4 * j + 3] + b[4 * j + 3]) : "memory");
             }
+#pragma unroll
+            for (int q = 0; q < KS; ++q) live = live && gone[q] == 0;
             cluster_sync();
         }
 #pragma unroll 1

@@ -152,3 +152,24 @@ def test_an_expired_wait_of_the_backward_stores_none_of_the_blocks_rows(D, store
             assert torch.equal(g, w), (i, j)
     run()
     assert torch.equal(grad, want) and _status() == 0
+
+
+@pytest.mark.parametrize("code,block", [(501, 1), (503, 6), (501, 79)])
+def test_an_expired_wait_of_a_split_product_leaves_the_whole_tile_out(code, block):
+    """Four blocks of a cluster share a tile's slices and store a quarter of its columns each: none may, with one's sum unfinished."""
+    M, N, K = 1280, 1024, 256
+    a, w = (torch.randn(*s, generator=torch.Generator(device="cuda").manual_seed(5), device="cuda") for s in ((M, N), (N, K)))
+    out = torch.empty(M, K, device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+    run = lambda: _capi.check(_capi.lib().hipgpt_matmul_tc(a.data_ptr(), w.data_ptr(), None, out.data_ptr(), M, N, K, st))      # noqa: E731
+    run()
+    want = out.clone()
+    got, = _expired(code, block, run, out)
+    for t in range(20):
+        piece = (slice(t // 2 * 128, t // 2 * 128 + 128), slice(t % 2 * 128, t % 2 * 128 + 128))
+        if t == block // 4:
+            assert bool((got[piece] == -7.0).all())
+        else:
+            assert torch.equal(got[piece], want[piece]), t
+    run()
+    assert torch.equal(out, want) and _status() == 0
