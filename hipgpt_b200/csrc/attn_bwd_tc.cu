@@ -467,9 +467,11 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
                 w = (hf == 0 ? wa + wb : wb + wa) / fmaxf(l, 1e-30f);
                 lse = mn + log2f(fmaxf(l, 1e-30f));
             }
-            if (hf == 0 && !abort_flag) {            // rows past S: a probability of 0 for every key
-                if (!STORED) lse_out[(size_t)bh * Spad + row] = row < S ? lse : 1e30f;
-                w_out[(size_t)bh * Spad + row] = row < S ? w : 0.0f;
+            if (hf == 0) {                           // rows past S: a probability of 0 for every key
+                // after a wait that ran out: NaN, so that no block of columns makes a result of what the buffer held before
+                const bool lost = abort_flag;
+                if (!STORED) lse_out[(size_t)bh * Spad + row] = lost ? NAN : row < S ? lse : 1e30f;
+                w_out[(size_t)bh * Spad + row] = lost ? NAN : row < S ? w : 0.0f;
             }
         }
         if (STORED) {
