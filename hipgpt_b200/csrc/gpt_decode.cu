@@ -266,6 +266,7 @@ struct FusedArgs {
     int *err;
 };
 
+constexpr int kWidest = 6000;                                // largest E and F
 constexpr long long kBarrierLimitCycles = 4000000000LL;     // about two seconds
 
 __device__ __forceinline__ bool grid_barrier(const FusedArgs &a, unsigned &gen, int *ok_s)
@@ -697,7 +698,7 @@ long long hipgpt_gpt_weight_count(int V, int S, int E, int L, int H, int F)
 int hipgpt_gpt_create(hipgpt_gpt **out, const float *h_weights, int V, int S, int E, int L, int H, int F, int max_batch)
 {
     if (!out || !h_weights) return fail(HIPGPT_ERR_NULL, "out and h_weights must not be NULL");
-    if (V <= 0 || S <= 0 || E <= 0 || L <= 0 || H <= 0 || F <= 0 || E % H || max_batch <= 0 || E % 16 || F % 16 || F > 6000 || E > 6000)
+    if (V <= 0 || S <= 0 || E <= 0 || L <= 0 || H <= 0 || F <= 0 || E % H || max_batch <= 0 || E % 16 || F % 16 || F > kWidest || E > kWidest)
         return fail(HIPGPT_ERR_BAD_ARG, "bad model shape V=%d S=%d E=%d L=%d H=%d F=%d batch=%d", V, S, E, L, H, F, max_batch);
     GptDecoder *g = new (std::nothrow) GptDecoder();
     if (!g) return fail(HIPGPT_ERR_CUDA, "out of host memory");
@@ -745,10 +746,9 @@ int hipgpt_gpt_create(hipgpt_gpt **out, const float *h_weights, int V, int S, in
         }
     g->scratch_bytes = sb ? sb : 16;
     TRY(cudaMalloc(&g->d_scratch, g->scratch_bytes));
-    {
-        const int need = kRowsPerBlock * ((E > F ? E : F) + kSeg * 32) * (int)sizeof(float);   // activation rows of the widest matmul + partial sums
-        if (need > 48 * 1024) TRY(cudaFuncSetAttribute(matmul_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, need));
-    }
+    // activation rows of the widest matmul + partial sums; the limit is the kernel's, not the handle's: the widest shape that is accepted
+    constexpr int most_smem = kRowsPerBlock * (kWidest + kSeg * 32) * (int)sizeof(float);
+    TRY(cudaFuncSetAttribute(matmul_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most_smem));
     {
         // the persistent kernel: one block per SM, all resident at once (checked here, enforced by the cooperative launch)
         const int D = E / H;
@@ -758,7 +758,7 @@ int hipgpt_gpt_create(hipgpt_gpt **out, const float *h_weights, int V, int S, in
         TRY(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
         g->fused_smem = (size_t)kRowsPerBlock * ((E > F ? E : F) + kSeg * 32) * sizeof(float);
         if (g->fused_smem < 16 * 1024) g->fused_smem = 16 * 1024;      // the attention and first-maximum phases' scratch
-        TRY(cudaFuncSetAttribute(gpt_steps_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g->fused_smem));
+        TRY(cudaFuncSetAttribute(gpt_steps_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most_smem));
         TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gpt_steps_kernel, 32 * kSeg, g->fused_smem));
         g->persistent_ok = coop && per_sm >= 1 && D % 4 == 0 && D <= 128;
         g->grid_blocks = sms;

@@ -203,3 +203,21 @@ def test_gpu_generation_lays_the_weights_out_again_only_for_batches_that_use_it(
     assert large < weights // 2 and small >= weights
     (at_once,), again = used(4, 4)
     assert at_once < weights // 2 and np.array_equal(ids[1], again[0]) and np.array_equal(ids[1], ids[0][:4])
+
+
+@pytest.mark.gpu
+def test_gpu_generation_handles_of_different_widths_side_by_side():
+    """A narrower model's handle does not take shared memory away from a wider one's kernels."""
+    pytest.importorskip("torch")
+    from hipgpt_b200 import generation
+    wide, narrow = dict(V=90, S=24, E=64, L=1, H=2, F=4096), dict(V=90, S=24, E=64, L=1, H=2, F=1600)
+    w = synth.gpt_weights(41, **wide)
+    prompts = synth.token_ids(42, (2, 3), wide["V"])
+    want, _ = ob.gpt_generate(w, **wide, prompts=prompts, n_new=6, fma=True)
+    a = generation.GptDecoder(w, **wide, max_batch=2)
+    b = generation.GptDecoder(synth.gpt_weights(43, **narrow), **narrow, max_batch=2)
+    for mode in (generation.MODE_GRAPH, generation.MODE_PERSISTENT):
+        a.set_mode(mode)
+        assert np.array_equal(a.generate(prompts, 6)[0], want)
+    a.close()
+    b.close()
