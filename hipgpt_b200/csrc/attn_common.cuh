@@ -6,6 +6,8 @@
 #include <stdint.h>
 #include <stdlib.h>
 
+#include <atomic>
+
 #include "hipgpt_attn.h"
 
 namespace hipgpt {
@@ -53,6 +55,18 @@ template <typename... KArgs, typename... Args>
 inline cudaError_t launch_overlapped(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args)
 {
     return launch_overlapped_clusters(kern, 1, grid, block, smem, st, args...);
+}
+
+// A kernel's limit of dynamic shared memory belongs to the kernel on one device: set() runs at the first call on each.
+// `done`: a bit per device, one word per kernel (or set of kernels).
+template <typename Set>
+inline cudaError_t once_per_device(std::atomic<unsigned long long> &done, int dev, Set set)
+{
+    const unsigned long long bit = dev >= 0 && dev < 64 ? 1ull << dev : 0;
+    if (done.load(std::memory_order_acquire) & bit) return cudaSuccess;
+    const cudaError_t e = set();
+    if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+    return e;
 }
 
 #ifdef __CUDACC__

@@ -835,15 +835,12 @@ int launch_head_cfg(const HeadMaps &maps, float *out, float *probs, int p_mapped
 {
     auto kern = mha_head_kernel<CAUSAL, PROBS, RING>;
     const size_t smem = kHeadSmemBytes + (PROBS ? kStageBytes : 0) + 1024;
-    static bool attr_set = false;                    // per instantiation; setting it twice is harmless
-    if (!attr_set) {
-        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-        attr_set = true;
-    }
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
         sms = 148;
+    static std::atomic<unsigned long long> done{0};  // per instantiation
+    const cudaError_t e = once_per_device(done, dev, [&] { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); });
+    if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     const long long bh = (long long)B * H;
     if (bh > 2147483647LL) return fail(HIPGPT_ERR_BAD_ARG, "%lld (batch, head) pairs are too many", bh);
     const unsigned grid = (unsigned)(bh < sms ? bh : sms);

@@ -484,17 +484,16 @@ int gemm_tc_status_fetch(int *status)
 
 namespace {
 
-int set_gemm_attr()
+int set_gemm_attr(int dev)
 {
-    static bool attr_set = false;
-    if (!attr_set) {
-        cudaError_t e = cudaSuccess;
+    static std::atomic<unsigned long long> done{0};
+    const cudaError_t e = once_per_device(done, dev, [] {
+        cudaError_t r = cudaSuccess;
         for (auto kern : {gemm_tc_kernel<1>, gemm_tc_kernel<2>, gemm_tc_kernel<3>, gemm_tc_kernel<4>})
-            if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem);
-        if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-        attr_set = true;
-    }
-    return HIPGPT_OK;
+            if (r == cudaSuccess) r = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem);
+        return r;
+    });
+    return e == cudaSuccess ? HIPGPT_OK : fail(HIPGPT_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
 }
 
 // B -> its stage images and its largest magnitude (three launches on `st`; the first is a plain one, so everything
@@ -558,7 +557,7 @@ int launch_matmul_tc(const float *A, const float *B, const float *bias, float *C
     if (rc != HIPGPT_OK) return rc;
     uint8_t *scratch = ws.get(), *aimg = scratch, *bimg = scratch + abytes;
     float *row_inv = reinterpret_cast<float *>(scratch + abytes + bbytes), *b_amax = reinterpret_cast<float *>(scratch + abytes + bbytes + rbytes);
-    rc = set_gemm_attr();
+    rc = set_gemm_attr(dev);
     if (rc == HIPGPT_OK) rc = pack_b(B, N, K, bimg, b_amax, st);
     if (rc != HIPGPT_OK) return rc;
     return pack_a_and_multiply(A, bimg, b_amax, bias, C, M, N, K, aimg, row_inv, dev, st, ln_g, ln_b);
@@ -608,7 +607,7 @@ int launch_matmul_tc_prepared(const float *A, const PackedB *b, const float *bia
     int rc = g_gemm.enter(st, abytes + rbytes, &ws);
     if (rc != HIPGPT_OK) return rc;
     uint8_t *scratch = ws.get();
-    rc = set_gemm_attr();
+    rc = set_gemm_attr(dev);
     if (rc != HIPGPT_OK) return rc;
     return pack_a_and_multiply(A, b->bimg, b->b_amax, bias, C, M, N, K, scratch, reinterpret_cast<float *>(scratch + abytes), dev, st, ln_g, ln_b);
 }

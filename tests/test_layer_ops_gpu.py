@@ -145,6 +145,26 @@ def test_layer_norm_fused_into_the_tensor_core_projection(M, N, K):
     assert float((c1 - c3).abs().max()) <= 1e-5 * np.abs(want).max()
 
 
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs two GPUs")
+def test_kernels_with_large_shared_memory_on_a_second_device_of_the_process():
+    """A kernel's limit of dynamic shared memory is set per device; calls on one after the other, each on its own data."""
+    lib = _capi.lib()
+    M, N, K = 300, 256, 768
+    A, W = synth.normal(60, (M, N)), synth.normal(61, (N, K), 0.1)
+    B, H, S, D = 2, 4, 200, 32
+    qkv = synth.qkv_planes(62, B, S, H * D)
+    want_c, want_o = A.astype(np.float64) @ W.astype(np.float64), ob.mha(qkv, B, S, H * D, H, causal=True)[0]
+    for device in range(2):
+        with torch.cuda.device(device):
+            dA, dW, dq = dev(A), dev(W), dev(qkv)
+            c, o = torch.full((M, K), float("nan"), device="cuda"), torch.full((B * S, H * D), float("nan"), device="cuda")
+            _capi.check(lib.hipgpt_matmul_tc(dA.data_ptr(), dW.data_ptr(), None, c.data_ptr(), M, N, K, _st()))
+            _capi.check(lib.hipgpt_mha_forward_planes(dq.data_ptr(), o.data_ptr(), None, B, S, H * D, H, 1, _st()))
+            torch.cuda.synchronize()
+            assert np.abs(c.cpu().numpy() - want_c).max() <= 1e-5 * np.abs(want_c).max()
+            assert np.abs(o.cpu().numpy() - want_o).max() <= 1e-5
+
+
 def test_matmul_in_place_like_the_layers_output_projection():
     """src/transformer_layer.cpp:220 passes d_attn_output_ as both A and C."""
     lib = _capi.lib()
