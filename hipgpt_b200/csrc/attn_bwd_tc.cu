@@ -59,19 +59,6 @@ struct Img {
     static constexpr int kTileBytes = (kTile / 8) * kBlock;     // 64 rows
 };
 
-__host__ __device__ constexpr uint32_t idesc_bf16(int n, int b_n_major)
-{
-    // fp32 accumulator, bf16 A (K-major) and B, M = 128
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)b_n_major << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kLanes >> 4) << 24);
-}
-
-__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi)
-{
-    uint32_t r;
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
-    return r;
-}
-
 // Two fp32 numbers -> three words of two bf16 each whose sums are the numbers (to 2^-25 of them)
 __device__ __forceinline__ void cut3(float x, float y, uint32_t &h, uint32_t &m, uint32_t &l)
 {
@@ -121,7 +108,7 @@ template <int D>
 __device__ __forceinline__ void issue_scores(uint32_t d_tmem, uint32_t a_smem, uint32_t b_smem)
 {
     const uint64_t a = make_desc(a_smem, 128, Img<D>::kBlock, 0), b = make_desc(b_smem, 128, Img<D>::kBlock, 0);
-    constexpr uint32_t id = idesc_bf16(kTile, 0);
+    constexpr uint32_t id = idesc_bf16(kLanes, kTile, 0);
     constexpr int PA[6] = {0, 2, 1, 1, 0, 0}, PB[6] = {2, 0, 1, 0, 1, 0};        // small terms first
 #pragma unroll
     for (int p = 0; p < 6; ++p)
@@ -141,7 +128,7 @@ template <int D, bool WIDE, int KS0, int KS1, typename ACol>
 __device__ __forceinline__ void issue_accumulate(uint32_t acc, ACol a_col, uint32_t b_smem)
 {
     const uint64_t b = make_desc(b_smem, Img<D>::kBlock, 128, 0);
-    constexpr uint32_t id1 = idesc_bf16(D, 1), id2 = idesc_bf16(2 * D, 1);
+    constexpr uint32_t id1 = idesc_bf16(kLanes, D, 1), id2 = idesc_bf16(kLanes, 2 * D, 1);
     auto product = [&](int pa, int pb, int d, uint32_t id, bool fresh) {
 #pragma unroll
         for (int ks = KS0; ks < KS1; ++ks) {

@@ -85,6 +85,28 @@ __device__ __forceinline__ float ex2_approx(float x)
     return y;
 }
 
+// All threads of a cluster meet; what each has stored before, in shared memory of any of its blocks too, is visible behind it.
+__device__ __forceinline__ void cluster_sync() { asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory"); }
+
+// Part of an attention row: maximum (log2 domain), sum of exponentials and four columns of the output, both relative to the maximum.
+// Shared by the decode kernel and the forms of generation, whose results are the same bits.
+struct AttnPart {
+    float m, l;
+    float4 o;
+};
+__device__ __forceinline__ void merge_part(AttnPart &a, float m2, float l2, const float4 &o2)
+{
+    const float mn = fmaxf(a.m, m2);
+    const float a1 = ex2_approx(a.m - mn), a2 = ex2_approx(m2 - mn);
+    // (the contraction written out: the compiler may choose either product for the multiply-add)
+    a.l = fmaf(a.l, a1, __fmul_rn(l2, a2));
+    a.o.x = fmaf(a.o.x, a1, __fmul_rn(o2.x, a2));
+    a.o.y = fmaf(a.o.y, a1, __fmul_rn(o2.y, a2));
+    a.o.z = fmaf(a.o.z, a1, __fmul_rn(o2.z, a2));
+    a.o.w = fmaf(a.o.w, a1, __fmul_rn(o2.w, a2));
+    a.m = mn;
+}
+
 // 16-byte asynchronous global -> shared copy; `valid == false` writes zeros and reads nothing.
 __device__ __forceinline__ void cp_async16(void *smem_dst, const void *gmem_src, bool valid)
 {

@@ -24,25 +24,7 @@ constexpr int kMaxD = 512;
 
 __host__ __device__ inline int rec_stride(int D) { return ((D + 3) / 4) * 4 + 4; }
 
-struct Partial4 {
-    float m, l;
-    float4 o;
-};
-
-__device__ __forceinline__ void merge(Partial4 &a, float m2, float l2, const float4 &o2)
-{
-    const float mn = fmaxf(a.m, m2);
-    const float a1 = ex2_approx(a.m - mn), a2 = ex2_approx(m2 - mn);
-    a.l = a.l * a1 + l2 * a2;
-    a.o.x = a.o.x * a1 + o2.x * a2;
-    a.o.y = a.o.y * a1 + o2.y * a2;
-    a.o.z = a.o.z * a1 + o2.z * a2;
-    a.o.w = a.o.w * a1 + o2.w * a2;
-    a.m = mn;
-}
-
 // A cluster's partial results meet in the first block's shared memory; nothing else is read before every block has stored there.
-__device__ __forceinline__ void cluster_sync() { asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory"); }
 __device__ __forceinline__ uint32_t first_block(const void *p)
 {
     uint32_t r;
@@ -103,7 +85,7 @@ decode_split_vec_kernel(const float *__restrict__ q, const float *__restrict__ k
         q4 = __ldg(reinterpret_cast<const float4 *>(q + (size_t)b * E + col));
         q4.x *= qscale; q4.y *= qscale; q4.z *= qscale; q4.w *= qscale;
     }
-    Partial4 acc{-1e30f, 0.0f, make_float4(0.f, 0.f, 0.f, 0.f)};
+    AttnPart acc{-1e30f, 0.0f, make_float4(0.f, 0.f, 0.f, 0.f)};
     const int steps = (max(k1 - k0, 0) + kWarps * KPW - 1) / (kWarps * KPW);
     const float *kp = kc + (size_t)b * cap * E + col, *vp = vc + (size_t)b * cap * E + col;
     auto step = [&](const float4 &k4, const float4 &v4, bool valid) {
@@ -149,7 +131,7 @@ decode_split_vec_kernel(const float *__restrict__ q, const float *__restrict__ k
         o2.y = __shfl_xor_sync(0xffffffffu, acc.o.y, off);
         o2.z = __shfl_xor_sync(0xffffffffu, acc.o.z, off);
         o2.w = __shfl_xor_sync(0xffffffffu, acc.o.w, off);
-        merge(acc, m2, l2, o2);
+        merge_part(acc, m2, l2, o2);
     }
     if (kg == 0) {
         float *r = sm[warp][lik];
@@ -157,10 +139,10 @@ decode_split_vec_kernel(const float *__restrict__ q, const float *__restrict__ k
     }
     __syncthreads();
     if (warp == 0 && lane < LPK) {
-        Partial4 t{sm[0][lane][0], sm[0][lane][1], make_float4(sm[0][lane][2], sm[0][lane][3], sm[0][lane][4], sm[0][lane][5])};
+        AttnPart t{sm[0][lane][0], sm[0][lane][1], make_float4(sm[0][lane][2], sm[0][lane][3], sm[0][lane][4], sm[0][lane][5])};
 #pragma unroll
         for (int w = 1; w < kWarps; ++w)
-            merge(t, sm[w][lane][0], sm[w][lane][1], make_float4(sm[w][lane][2], sm[w][lane][3], sm[w][lane][4], sm[w][lane][5]));
+            merge_part(t, sm[w][lane][0], sm[w][lane][1], make_float4(sm[w][lane][2], sm[w][lane][3], sm[w][lane][4], sm[w][lane][5]));
         if (lane * 4 < D) {
             if (CLUSTER) {
                 const uint32_t rec = first_block(met[split]);

@@ -44,37 +44,6 @@ constexpr uint32_t kColX = 0, kColO = kBufs * kKeys, kTmemCols = 256;
 
 __device__ int g_bf16_status = 0;
 
-__host__ __device__ constexpr uint32_t idesc_bf16(int m, int n, int b_n_major)
-{
-    // fp32 accumulator, bf16 A and B, A K-major, B K- or N-major
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)b_n_major << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
-}
-
-__device__ __forceinline__ void mma_f16_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate)
-{
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate)
-{
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-}
-
-// two floats -> one word of two bf16 (round to nearest even), `lo` in the low half
-__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi)
-{
-    uint32_t r;
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
-    return r;
-}
-
 // (A cubic on the FMA pipe for a share of the exponentials, to relieve the special-function unit, was measured:
 // +3 % at S = 1024, -2 % at S = 2048, not kept.)
 
@@ -195,7 +164,7 @@ mha_bf16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant_
                 const uint64_t dk = make_desc(smem_u32(k_s + (t % kStages) * TILE), 16, 1024, 2);
 #pragma unroll
                 for (int k = 0; k < D / 16; ++k)         // 16 bf16 = 32 bytes per instruction
-                    if (elect_one()) mma_f16_ss(tmem + kColX + (t % kBufs) * kKeys, dq + (uint64_t)(k * 2), dk + (uint64_t)(k * 2), idesc_qk, k ? 1u : 0u);
+                    if (elect_one()) mma_h_ss(tmem + kColX + (t % kBufs) * kKeys, dq + (uint64_t)(k * 2), dk + (uint64_t)(k * 2), idesc_qk, k ? 1u : 0u);
                 if (elect_one()) tc_commit(&s_full[t % kStages]);    // S is ready, and this K stage may be refilled
             };
             wait(&q_full, 0, 9);
@@ -223,7 +192,7 @@ mha_bf16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant_
                 const uint64_t dv = make_desc(smem_u32(v_s + (t % kStages) * TILE), 1024, 1024, 2);
 #pragma unroll
                 for (int k = 0; k < kKeys / 16; ++k)
-                    if (elect_one()) mma_f16_ts(tmem + kColO, tmem + kColX + (t % kBufs) * kKeys + (uint32_t)(k * 8), dv + (uint64_t)(k * 128), idesc_pv,
+                    if (elect_one()) mma_h_ts(tmem + kColO, tmem + kColX + (t % kBufs) * kKeys + (uint32_t)(k * 8), dv + (uint64_t)(k * 128), idesc_pv,
                                                 (t == 0 && k == 0) ? 0u : 1u);
                 if (elect_one()) tc_commit(&o_done[t % kStages]);    // O is up to date; this V stage may be refilled, Q K^T may take the buffer
                 // P V(t-1) was issued a whole step ago: its stage takes V(t-1+4)

@@ -233,11 +233,6 @@ __device__ __noinline__ bool gemm_wait_slow(uint64_t *bar, uint32_t parity, int 
 // The blocks' partial sums meet in shared memory: the tile's columns are dealt out in pieces of 32, every block stores what it
 // has of the others' pieces into their (now idle) operand stages and adds up its own, in rank order.
 constexpr int kMostSplit = 4;
-__device__ __forceinline__ void cluster_sync()
-{
-    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
-}
-
 template <int KS>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_tc_kernel(const uint8_t *__restrict__ aimg, const uint8_t *__restrict__ bimg, const float *__restrict__ row_inv, const float *__restrict__ b_amax,

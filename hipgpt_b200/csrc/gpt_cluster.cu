@@ -76,24 +76,6 @@ __device__ __noinline__ int cluster_wait_slow(uint64_t *bar, uint32_t parity, Wa
     return 1;
 }
 
-struct Part {
-    float m, l;
-    float4 o;
-};
-// as in attn_decode.cu
-__device__ __forceinline__ void merge_part(Part &a, float m2, float l2, const float4 &o2)
-{
-    const float mn = fmaxf(a.m, m2);
-    const float a1 = ex2_approx(a.m - mn), a2 = ex2_approx(m2 - mn);
-    // (the contraction written out: the compiler may choose either product for the multiply-add, and the bits should be the launches')
-    a.l = fmaf(a.l, a1, __fmul_rn(l2, a2));
-    a.o.x = fmaf(a.o.x, a1, __fmul_rn(o2.x, a2));
-    a.o.y = fmaf(a.o.y, a1, __fmul_rn(o2.y, a2));
-    a.o.z = fmaf(a.o.z, a1, __fmul_rn(o2.z, a2));
-    a.o.w = fmaf(a.o.w, a1, __fmul_rn(o2.w, a2));
-    a.m = mn;
-}
-
 template <int J>
 struct Job { static constexpr int value = J; };
 template <int E, int D, int R, int VW>
@@ -177,7 +159,7 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
         for (int i = 0; i < 6; ++i) { mbar_init(&hop[i], 1); mbar_arrive_expect_tx(&hop[i], tx(i)); }
     }
     __syncthreads();
-    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+    cluster_sync();
 
     auto wait = [&](uint64_t *bar, uint32_t parity) {
         if (!mbar_test(bar, parity)) cluster_wait_slow(bar, parity, &waits);
@@ -192,7 +174,7 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
     };
     // after a wait that has run out: through the barriers of this step and those to come with the others
     auto leave = [&](int step) {
-        for (; step < a.nsteps; ++step) asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+        for (; step < a.nsteps; ++step) cluster_sync();
     };
     // an address of this block -> the same place in four of the blocks (those this thread stores into)
     const int dq = tid & 3;
@@ -453,9 +435,9 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
             const float *now = qkv + un.now + lik * 4;         // this position's query, key and value
             float4 q4 = *reinterpret_cast<const float4 *>(now);
             q4.x *= qscale; q4.y *= qscale; q4.z *= qscale; q4.w *= qscale;
-            Part acc[VW];
+            AttnPart acc[VW];
 #pragma unroll
-            for (int w = 0; w < VW; ++w) acc[w] = Part{-1e30f, 0.0f, make_float4(0.f, 0.f, 0.f, 0.f)};
+            for (int w = 0; w < VW; ++w) acc[w] = AttnPart{-1e30f, 0.0f, make_float4(0.f, 0.f, 0.f, 0.f)};
             constexpr int step = W4 * KPW;
 #pragma unroll 1
             for (int it0 = 0; k0 + it0 * step < k1; it0 += AHEAD) {
@@ -486,7 +468,7 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
                     if (k0 + (it0 + it) * step >= k1) break;               // no lane of the four warps has a row there
 #pragma unroll
                     for (int w = 0; w < VW; ++w) {
-                        Part &t = acc[w];
+                        AttnPart &t = acc[w];
                         const float x = j0 + it * step + w * KPW < k1 ? s[w][it] : -INFINITY;
                         const float mn = fmaxf(t.m, x);
                         const float alpha = ex2_approx(t.m - mn), pr = ex2_approx(x - mn);
@@ -524,7 +506,7 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
             asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(32 * GW) : "memory");
             // each of the group's warps merges the columns of its lanes' `lik`; its key groups serve different receivers
             const float *m0 = merge_s + lik * 8;
-            Part t;
+            AttnPart t;
             t.o = *reinterpret_cast<const float4 *>(m0);
             t.m = m0[4]; t.l = m0[5];
 #pragma unroll

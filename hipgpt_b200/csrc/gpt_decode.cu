@@ -34,22 +34,6 @@ namespace {
 constexpr int kRowsPerBlock = 8;     // activation rows a matmul block keeps in shared memory
 
 // running (max, sum, weighted V) of the split-context attention, as in attn_decode.cu
-struct Partial4f {
-    float m, l;
-    float4 o;
-};
-__device__ __forceinline__ void merge_partial(Partial4f &a, float m2, float l2, const float4 &o2)
-{
-    const float mn = fmaxf(a.m, m2);
-    const float a1 = ex2_approx(a.m - mn), a2 = ex2_approx(m2 - mn);
-    a.l = a.l * a1 + l2 * a2;
-    a.o.x = a.o.x * a1 + o2.x * a2;
-    a.o.y = a.o.y * a1 + o2.y * a2;
-    a.o.z = a.o.z * a1 + o2.z * a2;
-    a.o.w = a.o.w * a1 + o2.w * a2;
-    a.m = mn;
-}
-
 // x[b] = tok[id] + pos[p]; the id is the prompt's while p is inside it, afterwards the id picked
 // by the previous step.  p is read from device memory so that one captured step serves all.
 __global__ void embed_kernel(const int *__restrict__ prompts, int n_prompt, const int *__restrict__ ids,
@@ -323,7 +307,7 @@ __device__ __forceinline__ void attn_split_phase(const FusedArgs &a, const float
         const size_t col = (size_t)h * D + lik * 4;
         const int per = (ctx + ns - 1) / ns;
         const int k0 = split * per, k1 = min(ctx, k0 + per);
-        Partial4f acc{-1e30f, 0.0f, make_float4(0.f, 0.f, 0.f, 0.f)};
+        AttnPart acc{-1e30f, 0.0f, make_float4(0.f, 0.f, 0.f, 0.f)};
         if (live) {
             float4 q4 = make_float4(0.f, 0.f, 0.f, 0.f);
             if (act) {
@@ -365,7 +349,7 @@ __device__ __forceinline__ void attn_split_phase(const FusedArgs &a, const float
                 o2.y = __shfl_xor_sync(0xffffffffu, acc.o.y, off);
                 o2.z = __shfl_xor_sync(0xffffffffu, acc.o.z, off);
                 o2.w = __shfl_xor_sync(0xffffffffu, acc.o.w, off);
-                merge_partial(acc, m2, l2, o2);
+                merge_part(acc, m2, l2, o2);
             }
             if (kg == 0) {
                 float *r = smb + (warp * LPK + lik) * 6;
@@ -376,11 +360,11 @@ __device__ __forceinline__ void attn_split_phase(const FusedArgs &a, const float
         if (live && warp == 0) {
             if (lane < LPK) {
                 const float *r0 = smb + lane * 6;
-                Partial4f tt{r0[0], r0[1], make_float4(r0[2], r0[3], r0[4], r0[5])};
+                AttnPart tt{r0[0], r0[1], make_float4(r0[2], r0[3], r0[4], r0[5])};
 #pragma unroll
                 for (int w = 1; w < W4; ++w) {
                     const float *r = smb + (w * LPK + lane) * 6;
-                    merge_partial(tt, r[0], r[1], make_float4(r[2], r[3], r[4], r[5]));
+                    merge_part(tt, r[0], r[1], make_float4(r[2], r[3], r[4], r[5]));
                 }
                 if (lane * 4 < D) {
                     if (ns == 1) {

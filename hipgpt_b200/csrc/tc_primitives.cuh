@@ -164,14 +164,6 @@ __device__ __forceinline__ void tmem_ld16(uint32_t addr, float (&v)[16])
                  : "r"(addr) : "memory");
     v[0] = __uint_as_float(r0); v[1] = __uint_as_float(r1); v[2] = __uint_as_float(r2); v[3] = __uint_as_float(r3); v[4] = __uint_as_float(r4); v[5] = __uint_as_float(r5); v[6] = __uint_as_float(r6); v[7] = __uint_as_float(r7); v[8] = __uint_as_float(r8); v[9] = __uint_as_float(r9); v[10] = __uint_as_float(r10); v[11] = __uint_as_float(r11); v[12] = __uint_as_float(r12); v[13] = __uint_as_float(r13); v[14] = __uint_as_float(r14); v[15] = __uint_as_float(r15);
 }
-__device__ __forceinline__ void tmem_ld8(uint32_t addr, float (&v)[8])
-{
-    uint32_t r0, r1, r2, r3, r4, r5, r6, r7;
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3), "=r"(r4), "=r"(r5), "=r"(r6), "=r"(r7)
-                 : "r"(addr) : "memory");
-    v[0] = __uint_as_float(r0); v[1] = __uint_as_float(r1); v[2] = __uint_as_float(r2); v[3] = __uint_as_float(r3); v[4] = __uint_as_float(r4); v[5] = __uint_as_float(r5); v[6] = __uint_as_float(r6); v[7] = __uint_as_float(r7);
-}
 __device__ __forceinline__ void tmem_st16(uint32_t addr, const float (&v)[16])
 {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
@@ -239,7 +231,7 @@ __device__ __forceinline__ void store_split_nmajor(float *hi_blk, float *lo_blk,
     *reinterpret_cast<float4 *>(lo_blk + off) = make_float4(x.x - h.x, x.y - h.y, x.z - h.z, x.w - h.w);
 }
 
-// ---- fp16 products (kind::f16) used for the correction terms and the all-fp16 P V product ----
+// ---- 16-bit products (kind::f16: fp16 or bf16 by the instruction descriptor) ----
 
 // fp32 accumulator, fp16 A and B, both K-major
 __host__ __device__ constexpr uint32_t idesc_f16(int m, int n)
@@ -262,6 +254,19 @@ __device__ __forceinline__ void mma_h_ts(uint32_t d_tmem, uint32_t a_tmem, uint6
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
         ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+}
+
+// fp32 accumulator, bf16 A and B, A K-major, B K- or N-major
+__host__ __device__ constexpr uint32_t idesc_bf16(int m, int n, int b_n_major)
+{
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)b_n_major << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
+}
+// two floats -> one word of two bf16 (round to nearest even), `lo` in the low half
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi)
+{
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
 }
 
 // two floats -> one word of two fp16 (round to nearest, saturating), `lo` in the low half
