@@ -165,3 +165,13 @@ def test_reference_layer_and_model_resolve_their_forward_path_against_the_librar
                              "launch_multihead_attention_backward"):
                     assert _capi.CXX_LAUNCHERS[must] in wanted and _capi.CXX_LAUNCHERS[must] in exported
     assert os.path.exists(os.path.join(ROOT, "oracle", "_ref", "ref_model_run")), "run `make -C oracle` (or __graft_entry__.build())"
+
+
+def test_reference_arm_of_the_benchmark_claims_no_number():
+    """What runs there without the reference's own code is not the reference: the line says so."""
+    import json
+    import subprocess
+    import sys
+    r = subprocess.run([sys.executable, os.path.join(ROOT, "bench.py"), "--impl", "reference", "--steps", "2", "--warmup", "1"], capture_output=True, text=True, check=True)
+    line = json.loads(r.stdout)
+    assert line["impl"] == "reference" and line["unavailable"] and "value" not in line
