@@ -23,7 +23,7 @@
 // its issuer more than it costs the tensor pipe, and two warps issue side by side); both stay converged and elect
 // the issuing lane per instruction.  Each accumulator is written by one warp, in tile order.
 // Every wait is bounded: on expiry the block raises a flag that cuts all later waits short,
-// records a status code, skips its stores, frees its TMEM and returns.
+// records a status code, skips its stores, lets what is on its way land, frees its TMEM and returns.
 #include "tc_primitives.cuh"
 #include "tma_host.cuh"
 

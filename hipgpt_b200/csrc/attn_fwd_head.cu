@@ -33,10 +33,10 @@
 // P V products of one query tile each, in a fixed order, so results do not depend on timing.
 // Probabilities (when asked for): a row's sum is known once all its tiles have been through the exponentials;
 // the workers then read P_hi + P_lo back from TMEM, divide by the sum and store [B][H][S][S] by TMA: no second Q K^T.
-// At B=32 H=8 S=256 unmasked 30.2 us (36.2 with stores through the workers' registers, the next head's Q and K fetched
-// only after them), causal 25.4 (30.4); a store phase of 128 KB takes 2.5 us on all SMs at once, which is what HBM takes.
+// At B=32 H=8 S=256 unmasked 29.3 us (36.2 with stores through the workers' registers, the next head's Q and K fetched
+// only after them), causal 24.3 (30.4); a store phase of 128 KB takes 2.5 us on all SMs at once, which is what HBM takes.
 // Every wait is bounded: on expiry the block raises a flag that cuts all later waits short, records a
-// site code for hipgpt_kernel_status, skips its stores, frees its TMEM and returns.
+// site code for hipgpt_kernel_status, skips its stores, lets what is on its way land, frees its TMEM and returns.
 #include "tc_primitives.cuh"
 #include "tma_host.cuh"
 

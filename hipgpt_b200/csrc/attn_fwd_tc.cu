@@ -32,8 +32,8 @@
 // Hand-offs use mbarriers: tcgen05.commit signals the MMAs' completion, 128 arrivals signal
 // "next K staged" and "P written, V staged".  Two blocks per SM (head_dim 32) overlap one
 // block's softmax with the other's MMAs.  Every wait is bounded: on expiry the block raises a
-// flag that cuts all its later waits short, records a status code, skips its stores, frees
-// its TMEM and returns.  No probabilities are written by this kernel; callers that want them
+// flag that cuts all its later waits short, records a status code, skips its stores, lets what
+// is on its way land, frees its TMEM and returns.  No probabilities are written by this kernel; callers that want them
 // get the FFMA rows kernel.
 #include "tc_primitives.cuh"
 

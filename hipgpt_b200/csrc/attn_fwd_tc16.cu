@@ -34,7 +34,7 @@
 //   multiply-adds work on pairs of values per instruction (the sweeps are bound by the instructions they issue).
 //   A warp stages its 32 query rows with whole-line reads (D / 4 lanes per row), all in flight at once.
 // Every wait is bounded: on expiry the block raises a flag that cuts all later waits short,
-// records a status code, skips its stores, frees its TMEM and returns.
+// records a status code, skips its stores, lets what is on its way land, frees its TMEM and returns.
 #include "stream_workspace.hpp"
 #include "tc_primitives.cuh"
 
@@ -551,8 +551,8 @@ mha_tc16_kernel(const uint8_t *__restrict__ kimg, const uint8_t *__restrict__ vi
         const float linv = 1.0f / fmaxf(l, 1e-20f);  // for the probabilities
         const float inv = linv * vinv;
         // Rows of 64 floats leave in whole lines, turned through the V stages (free: the last P V product has completed): a thread's own
-        // 16-byte stores touched 32 lines per instruction, and the next block on the SM waited for them (B=16 H=8 S=1024 causal:
-        // 94.7 -> 90.5 us, B=16 H=12 S=500: 61.2 -> 54.2; whole sectors as below: 92.2, 55.1).  Rows of 32 floats: in whole sectors,
+        // 16-byte stores touched 32 lines per instruction, and the next block on the SM waited for them (in runs short enough for the full clock, B=16 H=8 S=1024
+        // causal: 94.7 -> 90.5 us, B=16 H=12 S=500: 61.2 -> 54.2; whole sectors as below: 92.2, 55.1).  Rows of 32 floats: in whole sectors,
         // a quarter of a row each (B=30 H=8 S=300: 30.9 -> 30.5; by lines 31.5).
         if constexpr (D == 64) {
             uint8_t *ob = v_16 + wq * (32 * D * 4);          // 16-byte chunk c of row r at r * 4 D + ((c ^ (r & 7)) << 4)

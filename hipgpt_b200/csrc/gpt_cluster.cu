@@ -25,7 +25,7 @@
 // out too, and all meet at the barriers of the remaining steps and leave.  (A barrier whose phase has not been seen complete is not
 // opened again, and the bytes that nobody waits for stay within eight layers' worth, at most 90 KB each: an mbarrier counts 2^20.)
 //
-// Measured at the default model (E=256 L=8 H=8 V=5000), batch 8: 73 us per step (the replayed graph: 318), batch 1: 68 (256).  A
+// Measured at the default model (E=256 L=8 H=8 V=5000), batch 8: 72 us per step (the replayed graph: 318), batch 1: 67 (256).  A
 // step is 42 products of 400 - 450 ns each, attention a third of a layer.  Sizes are template parameters because the chain is
 // bound by the instructions of single warps: with sizes read from the plan a step took 143 us.
 #include "gpt_cluster.cuh"

@@ -33,8 +33,9 @@ constexpr int kBK = 16;
 // of the issue slots: multiply-adds run on pairs of columns (fma.rn.f32x2, one instruction for two roundings), and both operands
 // come by 16-byte asynchronous copies, three stages, A untransposed (a thread reads four inner indices of a row at once).
 // Registers alone (the same multiply-adds without loads) reach 61 TFLOP/s; here 54 at 16384 x 512 x 1536 (one inner index after
-// another in 128 x 128 tiles, operands through registers: 47.7).  With 8192 rows: 256 -> 768 columns 80 -> 66 us, 256 -> 256 35 -> 27,
-// 256 -> 1024 105 -> 84, 1024 -> 256 125 -> 91.
+// another in 128 x 128 tiles, operands through registers: 47.7).  With 8192 rows: 256 -> 768 columns 80 -> 63 us, 256 -> 256 35 -> 27,
+// 256 -> 1024 105 -> 83, 1024 -> 256 125 -> 92; where a product of two tiles per SM follows itself its blocks come in beside the last one's
+// tiles, up to three to an SM: 34 and 130 us.
 constexpr int kTileThreads = 128;
 constexpr int kTileStages = 3;
 template <int TM, int TN>

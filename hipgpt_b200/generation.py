@@ -10,7 +10,7 @@ import numpy as np
 from . import _capi
 
 
-MODE_GRAPH = 0          # one step = a CUDA graph of 52 launches, replayed per token (default)
+MODE_GRAPH = 0          # default: one launch for all positions by clusters of blocks; a CUDA graph of 52 launches, replayed per token, where they do not fit
 MODE_PERSISTENT = 1     # one cooperative launch for a run of token steps, phases separated by a barrier over the grid
 
 

@@ -295,13 +295,13 @@ HIPGPT_API int hipgpt_gpt_create_from_run(hipgpt_gpt **out, const char *json_pat
 /*
  * Two modes of the same token step, same arithmetic and the same ids (extension, like the driver itself):
  *   HIPGPT_GPT_MODE_GRAPH (default): where the shape allows (embedding 128 ... 384 in steps of 32, feed-forward width four times
- *     that, head_dim 32 or 64, batches up to 14) clusters of sixteen blocks run all token positions of their sequences in
- *     one launch; elsewhere one step = 52 kernel launches captured once as a CUDA graph and replayed per token.
+ *     that, head_dim 32 or 64, batches up to 14, contexts short for the batch: 24576 positions for two sequences at E = 256)
+ *     clusters of sixteen blocks run all token positions of their sequences in one launch; elsewhere one step = 52 kernel launches captured once as a CUDA graph and replayed per token.
  *   HIPGPT_GPT_MODE_PERSISTENT (head_dim % 4 == 0 and head_dim <= 128): one cooperative launch runs all
  *     prompt positions, a second one the remaining tokens; the phases of a step follow one another inside the
- *     kernel, separated by a bounded barrier over the grid (one block per SM).  If a wait at that barrier runs
- *     out, hipgpt_gpt_generate returns HIPGPT_ERR_CUDA and the handle stays usable.  Measured no faster than the
- *     graph on B200 (335 against 327 us per step of 8 tokens; the clusters: 73).
+ *     kernel, separated by a bounded barrier over the grid (one block per SM).  Measured no faster than the
+ *     graph on B200 (336 against 318 us per step of 8 tokens; the clusters: 72).
+ * If a wait inside a kernel of either mode runs out, hipgpt_gpt_generate returns HIPGPT_ERR_CUDA and the handle stays usable.
  */
 #define HIPGPT_GPT_MODE_GRAPH 0
 #define HIPGPT_GPT_MODE_PERSISTENT 1
