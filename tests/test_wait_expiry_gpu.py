@@ -75,13 +75,18 @@ def test_stalled_clusters_end_the_generation_call_with_an_error():
 
 
 def _expired(code, block, call, *outs):
-    """The outputs of `call` with the wait of this code run out in one block, canaries where nothing was stored."""
-    for o in outs:
-        o.fill_(-7.0)
-    _capi.check(_capi.lib().hipgpt_debug_expire_wait(code, block))
-    call()
-    torch.cuda.synchronize()
-    assert _status() == code and _status() == 0
+    """The outputs of `call` with the wait of this code run out in one block, canaries where nothing was stored.  What is waited for
+    may have come before, so that nothing has to wait: then once more."""
+    for _ in range(20):
+        for o in outs:
+            o.fill_(-7.0)
+        _capi.check(_capi.lib().hipgpt_debug_expire_wait(code, block))
+        call()
+        torch.cuda.synchronize()
+        status = _status()
+        if status:
+            break
+    assert status == code and _status() == 0
     return [o.clone() for o in outs]
 
 
