@@ -20,9 +20,12 @@
 //   gemm_tc_kernel       one block per SM, 128 x 128 output tiles in turn: a producer warp fetches whole stages with bulk
 //                        copies (three stages of 64 KB in flight, running on into the next tile), an issuing warp forms
 //                        A_hi [B_hi | B_lo] (N = 256) and A_lo B_hi (N = 128, onto the second half) for every slice, 8
-//                        instructions per slice, into one of two accumulators of 256 TMEM columns; four warps (thread =
-//                        output row = TMEM lane) add the halves, take the scales out, add the bias and store one tile
-//                        while the products of the next one run.
+//                        instructions per slice, into one of two accumulators of 256 TMEM columns; eight warps (thread =
+//                        output row = TMEM lane; two share the columns of a row) add the halves, take the scales out, add
+//                        the bias and store one tile while the products of the next one run.
+// Where the time of a small product goes (1407 x 512 x 1536, marks in an instrumented copy, us after A's images are there): first
+// stage landed 0.8 (1.3 with B's part asked for only then), eight slices 4.0 (64 KB each at 64 bytes per clock and SM), last product 0.7, output
+// 1.5 (4.0 with four warps and the bias asked for piece by piece behind the products).
 // Rows, columns and depth beyond the matrices are zeros in the images; stores are bounded by M and K.
 // Every wait is bounded: on expiry the block records a status code, skips its stores, lets what is on its way land, frees its TMEM
 // and returns; the blocks that share its tile store none of it.
@@ -40,7 +43,8 @@ constexpr int kABlk = kTM * 128;                  // bytes of one block of an A 
 constexpr int kAStage = 2 * kABlk;                // [A_hi | A_lo]
 constexpr int kBStage = kTK * 2 * kTN * 2;        // 64 deep x [B_hi (128) | B_lo (128)] fp16
 constexpr int kGroupStride = 2 * kTN * 16;        // bytes between groups of 8 reduction rows of a B stage (32 column blocks of 128 bytes)
-constexpr int kGemmThreads = 192;                 // 4 epilogue warps, a producer warp, an issuing warp
+constexpr int kEpiWarps = 8;                      // two per quarter of the rows, each half of the columns
+constexpr int kGemmThreads = 32 * (kEpiWarps + 2);        // and a producer warp, an issuing warp
 constexpr int kTmemCols = 512;                    // two accumulators of [A_hi B_hi (128) | corrections (128)]
 constexpr size_t kGemmSmem = (size_t)kStages * (kAStage + kBStage) + 1024;
 
@@ -243,7 +247,7 @@ gemm_tc_kernel(const uint8_t *__restrict__ aimg, const uint8_t *__restrict__ bim
     uint8_t *a_s = base;                              // [stage][A_hi block | A_lo block]
     uint8_t *b_s = base + kStages * kAStage;          // [stage][64 deep][B_hi | B_lo]
     __shared__ uint64_t full[kStages], empty[kStages], acc_full[2], acc_empty[2];
-    __shared__ __align__(16) float epi[4][32 * 32];  // per epilogue warp: a 32 x 32 piece of the output on its way out
+    __shared__ __align__(16) float epi[kEpiWarps][32 * 32];  // per epilogue warp: a 32 x 32 piece of the output on its way out
     __shared__ uint32_t tmem_base_slot;
     __shared__ volatile int abort_flag;
 
@@ -253,7 +257,7 @@ gemm_tc_kernel(const uint8_t *__restrict__ aimg, const uint8_t *__restrict__ bim
     if (tid == 0) {
         abort_flag = 0;
         for (int i = 0; i < kStages; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
-        for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 4); }
+        for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], kEpiWarps); }
     }
     __syncthreads();
     // site codes in the status word: 1 stage landed, 2 stage free, 3 accumulator complete, 4 accumulator drained
@@ -271,12 +275,25 @@ gemm_tc_kernel(const uint8_t *__restrict__ aimg, const uint8_t *__restrict__ bim
     if constexpr (KS > 1) asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
     const int kt0 = rank * KT / KS, kt1 = (rank + 1) * KT / KS, first = (int)blockIdx.x / KS, stride = (int)gridDim.x / KS;
 
-    if (warp == 4) {
+    if (warp == kEpiWarps) {
         // ---- producer: whole stages by bulk copies ----
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)), "r"(kTmemCols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
         dependents_may_start();
-        dependency_wait();                            // the pack kernels have completed
+        // What the kernel that packs A does not write is asked for before it has completed: it let this kernel in behind its own wait, so
+        // B's images (and magnitude, and the bias) are older.
+        auto ask_b = [&](int s, int nt, int kt) {
+            mbar_arrive_expect_tx(&full[s], (uint32_t)(kAStage + kBStage));
+            const uint8_t *bsrc = bimg + ((size_t)nt * KT + kt) * kBStage;
+            bulk_load(b_s + s * kBStage, bsrc, kBStage / 2, &full[s]);
+            bulk_load(b_s + s * kBStage + kBStage / 2, bsrc + kBStage / 2, kBStage / 2, &full[s]);
+        };
+        int early = 0;
+        for (int t = first, kt = kt0; early < kStages && t < ntiles; ++early) {
+            if (lane == 0) ask_b(early, t % NT, kt);
+            if (++kt == kt1) { kt = kt0; t += stride; }
+        }
+        dependency_wait();                            // A's images are there
         tc_fence_before();
         __syncthreads();                              // TMEM allocated
         int g = 0;
@@ -286,12 +303,10 @@ gemm_tc_kernel(const uint8_t *__restrict__ aimg, const uint8_t *__restrict__ bim
                 const int s = g % kStages;
                 if (g >= kStages) wait(&empty[s], (uint32_t)((g / kStages - 1) & 1), 2);     // the products that read the stage have completed
                 if (lane == 0 && seen) {
-                    mbar_arrive_expect_tx(&full[s], (uint32_t)(kAStage + kBStage));
-                    const uint8_t *asrc = aimg + ((size_t)mt * KT + kt) * kAStage, *bsrc = bimg + ((size_t)nt * KT + kt) * kBStage;
+                    if (g >= early) ask_b(s, nt, kt);
+                    const uint8_t *asrc = aimg + ((size_t)mt * KT + kt) * kAStage;
                     bulk_load(a_s + s * kAStage, asrc, kABlk, &full[s]);
                     bulk_load(a_s + s * kAStage + kABlk, asrc + kABlk, kABlk, &full[s]);
-                    bulk_load(b_s + s * kBStage, bsrc, kBStage / 2, &full[s]);
-                    bulk_load(b_s + s * kBStage + kBStage / 2, bsrc + kBStage / 2, kBStage / 2, &full[s]);
                 }
                 __syncwarp();
             }
@@ -304,7 +319,7 @@ gemm_tc_kernel(const uint8_t *__restrict__ aimg, const uint8_t *__restrict__ bim
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base_slot), "r"(kTmemCols) : "memory");
         return;
     }
-    if (warp == 5) {
+    if (warp == kEpiWarps + 1) {
         // ---- issuing warp: stays converged, elects the lane per instruction ----
         tc_fence_before();
         __syncthreads();
@@ -349,12 +364,24 @@ gemm_tc_kernel(const uint8_t *__restrict__ aimg, const uint8_t *__restrict__ bim
     tc_fence_after();
     const float b_inv = pow2_inverse(pow2_scale(__ldg(b_amax)));
     const bool vec = (K & 3) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0;
+    const int quarter = warp & 3, half = warp >> 2;   // its rows; its pieces of 32 columns: half, half + 2
+    const int ch = lane & 7;                          // of a piece it stores columns 4 ch ... 4 ch + 3
     int i = 0;
     for (int t = first; t < ntiles; t += stride, ++i) {
         const int nt = t % NT, mt = t / NT;
-        const int r = warp * 32 + lane, m = mt * kTM + r;
-        const uint32_t lane_base = tmem_base_slot + ((uint32_t)(warp * 32) << 16) + (uint32_t)((i & 1) * 2 * kTN);
+        const int r = quarter * 32 + lane, m = mt * kTM + r;
+        const uint32_t lane_base = tmem_base_slot + ((uint32_t)(quarter * 32) << 16) + (uint32_t)((i & 1) * 2 * kTN);
         const float unscale = (m < M ? __ldg(row_inv + m) : 0.0f) * b_inv;
+        // the bias is on its way while the products run: asked for behind them, piece by piece, it cost 2.8 us per tile
+        float4 bias4[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
+        if (bias) {
+#pragma unroll
+            for (int p = 0; p < 2; ++p) {
+                const int col = nt * kTN + 32 * (half + 2 * p) + 4 * ch;
+                bias4[p] = make_float4(col < K ? __ldg(bias + col) : 0.0f, col + 1 < K ? __ldg(bias + col + 1) : 0.0f,
+                                       col + 2 < K ? __ldg(bias + col + 2) : 0.0f, col + 3 < K ? __ldg(bias + col + 3) : 0.0f);
+            }
+        }
         wait(&acc_full[i & 1], (uint32_t)((i / 2) & 1), 3);
         tc_fence_after();
         const int c_base = nt * kTN;
@@ -378,7 +405,7 @@ gemm_tc_kernel(const uint8_t *__restrict__ aimg, const uint8_t *__restrict__ bim
                 asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %1, %2;\n\tld.shared::cluster.b32 %0, [a];\n\t}"
                              : "=r"(gone[q]) : "r"(smem_u32(const_cast<const int *>(&abort_flag))), "r"(q) : "memory");
 #pragma unroll 1
-            for (int c = 0; c < 4; ++c) {
+            for (int c = half; c < 4; c += 2) {
                 const int owner = c * KS / 4;
                 if (owner == rank) continue;
                 float a[32], b[32];
@@ -396,8 +423,9 @@ gemm_tc_kernel(const uint8_t *__restrict__ aimg, const uint8_t *__restrict__ bim
             for (int q = 0; q < KS; ++q) live = live && gone[q] == 0;
             cluster_sync();
         }
-#pragma unroll 1
-        for (int c0 = 0; c0 < kTN; c0 += 32) {
+#pragma unroll (KS > 1 ? 1 : 2)
+        for (int p = 0; p < 2; ++p) {
+            const int c0 = 32 * (half + 2 * p);
             if (KS > 1 && (c0 / 32) * KS / 4 != rank) continue;
             float a[32], b[32];
             tmem_ld32(lane_base + c0, a);             // A_hi B_hi
@@ -424,20 +452,18 @@ gemm_tc_kernel(const uint8_t *__restrict__ aimg, const uint8_t *__restrict__ bim
             for (int j4 = 0; j4 < 8; ++j4) {
                 float o[4];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const int c = c_base + c0 + 4 * j4 + j;
-                    o[j] = (a[4 * j4 + j] + b[4 * j4 + j]) * unscale + ((bias && c < K) ? __ldg(bias + c) : 0.0f);
-                }
+                for (int j = 0; j < 4; ++j) o[j] = (a[4 * j4 + j] + b[4 * j4 + j]) * unscale;     // (a power of two)
                 *reinterpret_cast<float4 *>(tb + lane * 128 + ((j4 ^ (lane & 7)) << 4)) = make_float4(o[0], o[1], o[2], o[3]);
             }
             __syncwarp();
-            const int ch = lane & 7;
             const int col = c_base + c0 + 4 * ch;
+            const float4 bp = p ? bias4[1] : bias4[0];
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 const int rr = 4 * i + (lane >> 3);
-                const int mrow = mt * kTM + warp * 32 + rr;
-                const float4 val = *reinterpret_cast<const float4 *>(tb + rr * 128 + ((ch ^ (rr & 7)) << 4));
+                const int mrow = mt * kTM + quarter * 32 + rr;
+                float4 val = *reinterpret_cast<const float4 *>(tb + rr * 128 + ((ch ^ (rr & 7)) << 4));
+                val.x += bp.x; val.y += bp.y; val.z += bp.z; val.w += bp.w;
                 if (live && mrow < M) {
                     float *dst = C + (size_t)mrow * K + col;
                     if (vec && col + 4 <= K) {
