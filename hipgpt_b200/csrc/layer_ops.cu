@@ -18,6 +18,7 @@
 
 #include <math.h>
 
+#include <algorithm>
 #include <initializer_list>
 
 namespace hipgpt {
@@ -34,8 +35,7 @@ constexpr int kBK = 16;
 // come by 16-byte asynchronous copies, three stages, A untransposed (a thread reads four inner indices of a row at once).
 // Registers alone (the same multiply-adds without loads) reach 61 TFLOP/s; here 54 at 16384 x 512 x 1536 (one inner index after
 // another in 128 x 128 tiles, operands through registers: 47.7).  With 8192 rows: 256 -> 768 columns 80 -> 63 us, 256 -> 256 35 -> 27,
-// 256 -> 1024 105 -> 83, 1024 -> 256 125 -> 92; where a product of two tiles per SM follows itself its blocks come in beside the last one's
-// tiles, up to three to an SM: 34 and 130 us.
+// 256 -> 1024 105 -> 83, 1024 -> 256 125 -> 92.
 constexpr int kTileThreads = 128;
 constexpr int kTileStages = 3;
 template <int TM, int TN>
@@ -334,7 +334,7 @@ static int launch_matmul_tiles(const float *A, const float *B, const float *bias
 {
     static const TileChoice choices[] = {tile_choice<8, 16>(), tile_choice<7, 16>(), tile_choice<6, 16>(), tile_choice<5, 16>(), tile_choice<8, 8>(), tile_choice<7, 8>(),
                                          tile_choice<6, 8>(), tile_choice<5, 8>(), tile_choice<4, 8>(), tile_choice<3, 8>(), tile_choice<4, 4>(), tile_choice<2, 4>()};
-    constexpr int kSms = 148;
+    constexpr int kSms = 148, kSmSharedBytes = 228 * 1024;
     const TileChoice *best = nullptr;
     double best_cost = 0.0;
     long long best_tiles = 0;
@@ -347,9 +347,16 @@ static int launch_matmul_tiles(const float *A, const float *B, const float *bias
         if (!best || cost < best_cost) { best = &c; best_cost = cost; best_tiles = tiles; }
     }
     if (best_tiles > 2147483647LL) return fail(HIPGPT_ERR_BAD_ARG, "matmul: %lld tiles are too many", best_tiles);
-    cudaError_t e = cudaFuncSetAttribute(best->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)best->smem);
+    // Blocks of an overlapped launch come in beside the last tiles of the product before, up to as many on an SM as fit: where every SM is to have two (or
+    // three), a third (fourth) that fits leaves another SM with one.  So a block asks for so much shared memory that no more than that fit.
+    // Behind itself: 8192 x 256 x 256 34.3 -> 24.3 us, 8192 x 1024 x 256 130.7 -> 90.2, 5000 x 512 x 320 66.9 -> 46.4; a block of the model, where the products
+    // follow other kernels, 333.7 -> 323.8.  (One tile per SM, and many: nothing to even out.)
+    const long long per_sm = (best_tiles + kSms - 1) / kSms;
+    size_t smem = best->smem;
+    if (per_sm == 2 || per_sm == 3) smem = std::max(smem, (size_t)(((size_t)kSmSharedBytes / (size_t)(per_sm + 1) + 128) & ~(size_t)127));
+    cudaError_t e = cudaFuncSetAttribute(best->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max(best->smem, (size_t)kSmSharedBytes / 3 + 128));
     if (e == cudaSuccess)
-        e = launch_overlapped(best->kernel, dim3((unsigned)best_tiles), dim3(kTileThreads), best->smem, st, A, B, bias, C, M, N, K, (K + 16 * best->tn - 1) / (16 * best->tn));
+        e = launch_overlapped(best->kernel, dim3((unsigned)best_tiles), dim3(kTileThreads), smem, st, A, B, bias, C, M, N, K, (K + 16 * best->tn - 1) / (16 * best->tn));
     if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "matmul_tile_kernel: %s", cudaGetErrorString(e));
     return HIPGPT_OK;
 }
