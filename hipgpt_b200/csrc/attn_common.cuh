@@ -175,5 +175,8 @@ int launch_weighted_sum(const float *P, const float *V, float *out, int B, int S
 int launch_decode(const float *q, const float *kc, const float *vc, float *out, float *scratch,
                   int B, int H, int D, int ctx, int cap, int nsplit, cudaStream_t st, const int *pos_ptr = nullptr);
 int decode_splits(int B, int H, int D, int ctx);
+// `rows` query rows, per_seq consecutive positions of each sequence, the first of which sees ctx0 keys
+bool decode_rows_supports(int D, int nsplit);
+int launch_decode_rows(const float *q, const float *kc, const float *vc, float *out, int rows, int per_seq, int H, int D, int ctx0, int cap, int nsplit, cudaStream_t st);
 
 }  // namespace hipgpt

@@ -248,7 +248,124 @@ decode_combine_kernel(const float *__restrict__ scratch, float *__restrict__ out
     combine_splits(scratch + (size_t)bh * nsplit * rec_stride(D), rec_stride(D), out + (size_t)(bh / H) * H * D + (size_t)(bh % H) * D, D, nsplit, threadIdx.x, kThreads);
 }
 
+// Many positions of a sequence at once (a prompt): query row i is position i % per_seq of sequence i / per_seq, which sees ctx0 + i % per_seq
+// keys, cut into nsplit <= 8 splits.  The same arithmetic in the same order as decode_split_vec_kernel, so the same bits; a block does all splits
+// of a (row, head) and merges them in shared memory.  Clusters of nsplit blocks would do too, but contexts are short here: 960 x 5 blocks for 120 rows
+// and 8 heads took 15 us, this 10.5 (both by themselves, from a cold instruction cache).
+template <int LPK>
+__global__ void __launch_bounds__(kThreads)
+decode_rows_kernel(const float *__restrict__ q, const float *__restrict__ kc, const float *__restrict__ vc, float *__restrict__ out,
+                   int H, int D, int ctx0, int cap, int nsplit, float qscale, int per_seq)
+{
+    dependency_wait();
+    dependents_may_start();
+    constexpr int KPW = 32 / LPK;
+    __shared__ __align__(16) float sm[kClusterSplits][kWarps][LPK][8];
+    __shared__ __align__(16) float met[kClusterSplits][4 * LPK + 4];
+    const int row = blockIdx.x, h = blockIdx.y, b = row / per_seq, ctx = ctx0 + row % per_seq, E = H * D;
+    const int per = (ctx + nsplit - 1) / nsplit;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lik = lane % LPK, kg = lane / LPK;
+    const bool act = lik * 4 < D;
+    const size_t col = (size_t)h * D + lik * 4;
+    float4 q4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (act) {
+        q4 = __ldg(reinterpret_cast<const float4 *>(q + (size_t)row * E + col));
+        q4.x *= qscale; q4.y *= qscale; q4.z *= qscale; q4.w *= qscale;
+    }
+    const float *kp = kc + (size_t)b * cap * E + col, *vp = vc + (size_t)b * cap * E + col;
+    constexpr int AT_ONCE = 4;                     // splits whose rows are asked for together
+    for (int s0 = 0; s0 < nsplit; s0 += AT_ONCE) {
+        AttnPart acc[AT_ONCE];
+#pragma unroll
+        for (int s = 0; s < AT_ONCE; ++s) acc[s] = AttnPart{-1e30f, 0.0f, make_float4(0.f, 0.f, 0.f, 0.f)};
+        for (int it = 0; it < (per + kWarps * KPW - 1) / (kWarps * KPW); ++it) {
+            float4 k4[AT_ONCE], v4[AT_ONCE];
+            bool valid[AT_ONCE], any[AT_ONCE];
+#pragma unroll
+            for (int s = 0; s < AT_ONCE; ++s) {
+                const int k0 = (s0 + s) * per, k1 = s0 + s < nsplit ? min(ctx, k0 + per) : 0, j = k0 + (it * kWarps + warp) * KPW + kg;
+                valid[s] = j < k1;
+                any[s] = k0 + it * kWarps * KPW < k1;          // (the split's steps end with the last key of its warps)
+                k4[s] = v4[s] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (valid[s] && act) {
+                    k4[s] = __ldg(reinterpret_cast<const float4 *>(kp + (size_t)j * E));
+                    v4[s] = __ldg(reinterpret_cast<const float4 *>(vp + (size_t)j * E));
+                }
+            }
+#pragma unroll
+            for (int s = 0; s < AT_ONCE; ++s) {
+                if (!any[s]) continue;
+                float x = q4.x * k4[s].x;
+                x = fmaf(q4.y, k4[s].y, x);
+                x = fmaf(q4.z, k4[s].z, x);
+                x = fmaf(q4.w, k4[s].w, x);
+#pragma unroll
+                for (int off = 1; off < LPK; off <<= 1) x += __shfl_xor_sync(0xffffffffu, x, off);
+                if (!valid[s]) x = -INFINITY;
+                const float mn = fmaxf(acc[s].m, x);
+                const float alpha = ex2_approx(acc[s].m - mn), p = ex2_approx(x - mn);
+                acc[s].l = fmaf(acc[s].l, alpha, p);
+                acc[s].o.x = fmaf(p, v4[s].x, acc[s].o.x * alpha);
+                acc[s].o.y = fmaf(p, v4[s].y, acc[s].o.y * alpha);
+                acc[s].o.z = fmaf(p, v4[s].z, acc[s].o.z * alpha);
+                acc[s].o.w = fmaf(p, v4[s].w, acc[s].o.w * alpha);
+                acc[s].m = mn;
+            }
+        }
+#pragma unroll
+        for (int off = LPK; off < 32; off <<= 1)
+#pragma unroll
+            for (int s = 0; s < AT_ONCE; ++s) {
+                const float m2 = __shfl_xor_sync(0xffffffffu, acc[s].m, off);
+                const float l2 = __shfl_xor_sync(0xffffffffu, acc[s].l, off);
+                float4 o2;
+                o2.x = __shfl_xor_sync(0xffffffffu, acc[s].o.x, off);
+                o2.y = __shfl_xor_sync(0xffffffffu, acc[s].o.y, off);
+                o2.z = __shfl_xor_sync(0xffffffffu, acc[s].o.z, off);
+                o2.w = __shfl_xor_sync(0xffffffffu, acc[s].o.w, off);
+                merge_part(acc[s], m2, l2, o2);
+            }
+        if (kg == 0) {
+#pragma unroll
+            for (int s = 0; s < AT_ONCE; ++s)
+                if (s0 + s < nsplit) {
+                    float *r = sm[s0 + s][warp][lik];
+                    *reinterpret_cast<float4 *>(r) = acc[s].o;
+                    *reinterpret_cast<float2 *>(r + 4) = make_float2(acc[s].m, acc[s].l);
+                }
+        }
+    }
+    __syncthreads();
+    for (int s = warp * KPW + kg; s < nsplit; s += kWarps * KPW) {           // a group of LPK lanes per split
+        const float *r = sm[s][0][lik];
+        AttnPart t{r[4], r[5], *reinterpret_cast<const float4 *>(r)};
+#pragma unroll
+        for (int w = 1; w < kWarps; ++w) {
+            const float *rw = sm[s][w][lik];
+            merge_part(t, rw[4], rw[5], *reinterpret_cast<const float4 *>(rw));
+        }
+        *reinterpret_cast<float4 *>(&met[s][lik * 4]) = t.o;
+        if (lik == 0) { met[s][4 * LPK] = t.m; met[s][4 * LPK + 1] = t.l; }
+    }
+    __syncthreads();
+    if (nsplit == 1) {
+        if (threadIdx.x < D) out[(size_t)row * E + (size_t)h * D + threadIdx.x] = met[0][threadIdx.x] * (1.0f / fmaxf(met[0][4 * LPK + 1], 1e-20f));
+    } else if (warp == 0) {
+        combine_splits(&met[0][0], 4 * LPK + 4, out + (size_t)row * E + (size_t)h * D, D, nsplit, lane, 32);
+    }
+}
+
 }  // namespace
+
+// Query rows of `rows / per_seq` sequences, see decode_rows_kernel; for the shapes that decode_rows_supports allows.
+bool decode_rows_supports(int D, int nsplit) { return D % 4 == 0 && D <= 128 && nsplit <= kClusterSplits; }
+int launch_decode_rows(const float *q, const float *kc, const float *vc, float *out, int rows, int per_seq, int H, int D, int ctx0, int cap, int nsplit, cudaStream_t st)
+{
+    const float qscale = (1.0f / sqrtf((float)D)) * kLog2e;
+    const auto kern = D <= 32 ? decode_rows_kernel<8> : D <= 64 ? decode_rows_kernel<16> : decode_rows_kernel<32>;
+    const cudaError_t e = launch_overlapped(kern, dim3(rows, H), dim3(kThreads), 0, st, q, kc, vc, out, H, D, ctx0, cap, nsplit, qscale, per_seq);
+    return e == cudaSuccess ? HIPGPT_OK : fail(HIPGPT_ERR_CUDA, "decode_rows_kernel launch: %s", cudaGetErrorString(e));
+}
 
 // Splits of the context: enough thread blocks for two waves over 148 SMs, at least 32 keys each.
 int decode_splits(int B, int H, int D, int ctx)

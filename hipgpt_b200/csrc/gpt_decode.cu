@@ -25,6 +25,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <algorithm>
 #include <new>
 #include <vector>
 
@@ -38,16 +39,17 @@ constexpr int kRowsPerBlock = 8;     // activation rows a matmul block keeps in 
 // by the previous step.  p is read from device memory so that one captured step serves all.
 __global__ void embed_kernel(const int *__restrict__ prompts, int n_prompt, const int *__restrict__ ids,
                              const int *__restrict__ pos_ptr, const float *__restrict__ tok, const float *__restrict__ pos,
-                             float *__restrict__ x, int E, int V)
+                             float *__restrict__ x, int E, int V, int per_seq, int p0)
 {
     dependency_wait();                               // overlapped launch: nothing is read before the kernel before this one has completed
     dependents_may_start();
-    const int b = blockIdx.x;
-    const int p = *pos_ptr;
+    // a row per sequence, or per_seq consecutive prompt positions from p0 on of each
+    const int row = blockIdx.x, b = per_seq ? row / per_seq : row;
+    const int p = per_seq ? p0 + row % per_seq : *pos_ptr;
     const int id = p < n_prompt ? prompts[(size_t)b * n_prompt + p] : ids[b];
     const bool ok = id >= 0 && id < V;
     for (int e = threadIdx.x; e < E; e += blockDim.x)
-        x[(size_t)b * E + e] = ok ? __fadd_rn(tok[(size_t)id * E + e], pos[(size_t)p * E + e]) : 0.0f;
+        x[(size_t)row * E + e] = ok ? __fadd_rn(tok[(size_t)id * E + e], pos[(size_t)p * E + e]) : 0.0f;
 }
 
 // Layer norm of one row held in shared memory, by one warp, in place.  Sums are 32 lane-strided
@@ -82,6 +84,7 @@ struct MatmulOut {
     const int *pos_ptr;          // position of the scatter, read from the device ...
     int cap, E;
     int p_fixed;                 // ... or, when pos_ptr is NULL, given here
+    int per_seq;                 // > 0: the rows are per_seq consecutive positions from p_fixed on of each sequence
 };
 
 // y = relu?( LN?(A) * W + bias ) (+ res) for up to kRowsPerBlock rows.  A block owns 32 columns; its
@@ -107,37 +110,67 @@ __device__ __forceinline__ void matmul_rows_body(int bx, int by, float *a_s, con
     const int rows = min(kRowsPerBlock, M - m0);
     float *part = a_s + kRowsPerBlock * K;          // a_s: [rows][K] activations, then [kSeg][rows][32] partial sums
     const int seg = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int i = threadIdx.x; i < rows * K; i += blockDim.x)
-        a_s[i] = FUSED ? __ldcg(A + (size_t)(m0 + i / K) * lda + i % K) : A[(size_t)(m0 + i / K) * lda + i % K];
+    const int n = bx * 32 + lane;
+    const int klen = K / kSeg, k0 = seg * klen;
+    // weights sixteen rows at a time, asked for before the rows are staged (and then before the sixteen before them are used)
+    const float *wp = W + (size_t)k0 * N + n;
+    float w[16];
+    auto load_w = [&](int k) {
+#pragma unroll
+        for (int u = 0; u < 16; ++u) w[u] = n < N && k + u < klen ? __ldg(wp + (size_t)(k + u) * N) : 0.0f;
+    };
+    load_w(0);
+    // (K, lda and the handle's buffers allow 16 bytes at a time)
+    const int k4 = K >> 2, all = rows * k4;
+    auto four = [&](int i) {
+        const float4 *src = reinterpret_cast<const float4 *>(A + (size_t)(m0 + i / k4) * lda) + i % k4;
+        return FUSED ? __ldcg(src) : *src;
+    };
+    for (int i = threadIdx.x; i < all; i += 4 * blockDim.x) {
+        float4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (i + u * (int)blockDim.x < all) v[u] = four(i + u * blockDim.x);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (i + u * (int)blockDim.x < all) reinterpret_cast<float4 *>(a_s)[i + u * blockDim.x] = v[u];
+    }
     __syncthreads();
     if (ln_g) {
         if (seg < rows) layernorm_row(a_s + seg * K, ln_g, ln_b, K, lane);
         __syncthreads();
     }
-    const int n = bx * 32 + lane;
-    const int klen = K / kSeg, k0 = seg * klen;
     float acc[kRowsPerBlock];
 #pragma unroll
     for (int m = 0; m < kRowsPerBlock; ++m) acc[m] = 0.0f;
-    if (n < N) {
-        const float *wp = W + (size_t)k0 * N + n;
-        int k = 0;
+    const float *as = a_s + k0;
+    int k = 0;
+    if ((klen & 3) == 0) {
         for (; k + 16 <= klen; k += 16) {
-            float w[16];
+            float wk[16];
 #pragma unroll
-            for (int u = 0; u < 16; ++u) w[u] = __ldg(wp + (size_t)(k + u) * N);     // sixteen loads in flight
+            for (int u = 0; u < 16; ++u) wk[u] = w[u];
+            if (k + 16 < klen) load_w(k + 16);
 #pragma unroll
-            for (int u = 0; u < 16; ++u)
+            for (int u = 0; u < 16; u += 4)
+#pragma unroll
+                for (int m = 0; m < kRowsPerBlock; ++m) {            // (rows past the matrix: whatever lies there, and never stored)
+                    const float4 x = *reinterpret_cast<const float4 *>(as + m * K + k + u);
+                    acc[m] = fmaf(x.x, wk[u], acc[m]);
+                    acc[m] = fmaf(x.y, wk[u + 1], acc[m]);
+                    acc[m] = fmaf(x.z, wk[u + 2], acc[m]);
+                    acc[m] = fmaf(x.w, wk[u + 3], acc[m]);
+                }
+        }
+    }
+    for (; k < klen; k += 16) {
+        if (k > 0) load_w(k);
+#pragma unroll
+        for (int u = 0; u < 16; ++u)
+            if (k + u < klen)
 #pragma unroll
                 for (int m = 0; m < kRowsPerBlock; ++m)
-                    if (m < rows) acc[m] = fmaf(a_s[m * K + k0 + k + u], w[u], acc[m]);
-        }
-        for (; k < klen; ++k) {
-            const float w = __ldg(wp + (size_t)k * N);
-#pragma unroll
-            for (int m = 0; m < kRowsPerBlock; ++m)
-                if (m < rows) acc[m] = fmaf(a_s[m * K + k0 + k], w, acc[m]);
-        }
+                    if (m < rows) acc[m] = fmaf(as[m * K + k + u], w[u], acc[m]);
     }
 #pragma unroll
     for (int m = 0; m < kRowsPerBlock; ++m) part[(seg * kRowsPerBlock + m) * 32 + lane] = acc[m];
@@ -152,10 +185,11 @@ __device__ __forceinline__ void matmul_rows_body(int bx, int by, float *a_s, con
         if (relu) v = fmaxf(0.0f, v);
         const int row = m0 + m;
         if (o.q) {
-            const int p = o.pos_ptr ? *o.pos_ptr : o.p_fixed;
+            int p = o.pos_ptr ? *o.pos_ptr : o.p_fixed, b = row;
+            if (o.per_seq) { b = row / o.per_seq; p += row % o.per_seq; }
             if (n < o.E) o.q[(size_t)row * o.E + n] = v;
-            else if (n < 2 * o.E) o.kc[((size_t)row * o.cap + p) * o.E + (n - o.E)] = v;
-            else o.vc[((size_t)row * o.cap + p) * o.E + (n - 2 * o.E)] = v;
+            else if (n < 2 * o.E) o.kc[((size_t)b * o.cap + p) * o.E + (n - o.E)] = v;
+            else o.vc[((size_t)b * o.cap + p) * o.E + (n - 2 * o.E)] = v;
         } else {
             if (o.res) v = __fadd_rn(FUSED ? __ldcg(o.res + (size_t)row * o.ldo + n) : o.res[(size_t)row * o.ldo + n], v);
             o.out[(size_t)row * o.ldo + n] = v;
@@ -212,6 +246,8 @@ argmax_kernel(const float *__restrict__ logits, int V, int *__restrict__ ids_nex
         if (col >= 0 && col < n_new) out_ids[(size_t)b * n_new + col] = si[0];
     }
 }
+
+__global__ void set_pos_kernel(int *pos_ptr, int p) { *pos_ptr = p; }
 
 __global__ void advance_pos_kernel(int *pos_ptr)
 {
@@ -464,23 +500,23 @@ gpt_steps_kernel(const FusedArgs a)
         for (int l = 0; l < a.L; ++l) {
             const LayerW w = a.layers[l];
             float *kc = a.kc + (size_t)l * a.layer_stride, *vc = a.vc + (size_t)l * a.layer_stride;
-            const MatmulOut scatter{nullptr, 0, nullptr, a.q, kc, vc, nullptr, a.S, E, p};
+            const MatmulOut scatter{nullptr, 0, nullptr, a.q, kc, vc, nullptr, a.S, E, p, 0};
             matmul_phase(a.x, E, w.g1, w.be1, w.wqkv, w.bqkv, scatter, E, 3 * E, 0);
             if (!grid_barrier(a, gen, &ok_s)) return;
             if (D <= 32) attn_split_phase<8>(a, kc, vc, p + 1, dsm);
             else if (D <= 64) attn_split_phase<16>(a, kc, vc, p + 1, dsm);
             else attn_split_phase<32>(a, kc, vc, p + 1, dsm);
             if (!grid_barrier(a, gen, &ok_s)) return;
-            const MatmulOut to_x{a.x, E, a.x, nullptr, nullptr, nullptr, nullptr, 0, 0, 0};
+            const MatmulOut to_x{a.x, E, a.x, nullptr, nullptr, nullptr, nullptr, 0, 0, 0, 0};
             matmul_phase(a.att, E, nullptr, nullptr, w.wo, w.bo, to_x, E, E, 0);
             if (!grid_barrier(a, gen, &ok_s)) return;
-            const MatmulOut to_ff{a.ff, F, nullptr, nullptr, nullptr, nullptr, nullptr, 0, 0, 0};
+            const MatmulOut to_ff{a.ff, F, nullptr, nullptr, nullptr, nullptr, nullptr, 0, 0, 0, 0};
             matmul_phase(a.x, E, w.g2, w.be2, w.w1, w.b1, to_ff, E, F, 1);
             if (!grid_barrier(a, gen, &ok_s)) return;
             matmul_phase(a.ff, F, nullptr, nullptr, w.w2, w.b2, to_x, F, E, 0);
             if (!grid_barrier(a, gen, &ok_s)) return;
         }
-        const MatmulOut to_logits{a.logits, V, nullptr, nullptr, nullptr, nullptr, nullptr, 0, 0, 0};
+        const MatmulOut to_logits{a.logits, V, nullptr, nullptr, nullptr, nullptr, nullptr, 0, 0, 0, 0};
         matmul_phase(a.x, E, nullptr, nullptr, a.wout, nullptr, to_logits, E, V, 0);
         if (!grid_barrier(a, gen, &ok_s)) return;
         // first maximum of each row of the logits (lowest index wins ties)
@@ -534,6 +570,8 @@ struct GptDecoder {
     size_t scratch_bytes = 0;
     int *d_ids = nullptr, *d_out = nullptr, *d_pos = nullptr, *d_prompts = nullptr;
     int out_cap = 0, prompt_cap = 0;
+    float *d_pre = nullptr;                        // activations of many prompt positions (prompt_pass)
+    size_t pre_bytes = 0;
     cudaStream_t stream = nullptr;
     // one step of generation captured as a CUDA graph; valid for (graph_B, graph_n_prompt, graph_n_new)
     cudaGraphExec_t graph = nullptr;
@@ -582,7 +620,7 @@ int matmul(const GptDecoder &g, const float *A, int lda, const float *ln_g, cons
     return check_launch("matmul_rows_kernel");
 }
 
-MatmulOut plain_out(float *out, int ldo, const float *res) { return MatmulOut{out, ldo, res, nullptr, nullptr, nullptr, nullptr, 0, 0, 0}; }
+MatmulOut plain_out(float *out, int ldo, const float *res) { return MatmulOut{out, ldo, res, nullptr, nullptr, nullptr, nullptr, 0, 0, 0, 0}; }
 
 // One token position for all B sequences, every launch reading the position from g.d_pos: embed,
 // L x {LN+QKV projection scattered into q and the caches, split-context attention, output
@@ -593,7 +631,7 @@ int enqueue_step(GptDecoder &g, int B, int n_prompt, int n_new)
     // every launch of the step is an overlapped one (captured into the graph as programmatic dependencies): a kernel's
     // blocks are placed while the kernel before it drains and wait for it before their first read
     cudaError_t le = launch_overlapped(embed_kernel, dim3(B), dim3(128), 0, g.stream, (const int *)g.d_prompts, n_prompt, (const int *)g.d_ids, (const int *)g.d_pos,
-                                       (const float *)g.tok, (const float *)g.pos, g.d_x, E, V);
+                                       (const float *)g.tok, (const float *)g.pos, g.d_x, E, V, 0, 0);
     if (le != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "embed_kernel launch: %s", cudaGetErrorString(le));
     int rc = check_launch("embed_kernel");
     if (rc) return rc;
@@ -602,7 +640,7 @@ int enqueue_step(GptDecoder &g, int B, int n_prompt, int n_new)
         const LayerW &w = g.lw[l];
         float *kc = g.d_kc + (size_t)l * g.max_batch * g.S * E;
         float *vc = g.d_vc + (size_t)l * g.max_batch * g.S * E;
-        const MatmulOut scatter{nullptr, 0, nullptr, g.d_q, kc, vc, g.d_pos, g.S, E, 0};
+        const MatmulOut scatter{nullptr, 0, nullptr, g.d_q, kc, vc, g.d_pos, g.S, E, 0, 0};
         if ((rc = matmul(g, g.d_x, E, w.g1, w.be1, w.wqkv, w.bqkv, scatter, B, E, 3 * E, 0))) return rc;
         if ((rc = launch_decode(g.d_q, kc, vc, g.d_att, g.d_scratch, B, g.H, D, 1, g.S, ns, g.stream, g.d_pos))) return rc;
         if ((rc = matmul(g, g.d_att, E, nullptr, nullptr, w.wo, w.bo, plain_out(g.d_x, E, g.d_x), B, E, E, 0))) return rc;
@@ -616,6 +654,61 @@ int enqueue_step(GptDecoder &g, int B, int n_prompt, int n_new)
     le = launch_overlapped(advance_pos_kernel, dim3(1), dim3(1), 0, g.stream, g.d_pos);
     if (le != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "advance_pos_kernel launch: %s", cudaGetErrorString(le));
     return check_launch("advance_pos_kernel");
+}
+
+// The keys and values of prompt positions 0 ... n - 1 of all sequences, every position of a layer in the same launches: the arithmetic
+// of a step, row by row, so what follows is the same bits.  A step costs the same chain of products for one position as these launches do for
+// some hundred rows.  The default model, 8 x 15 positions: 330 us instead of 15 x 72 (the whole request of 143
+// positions 10450 -> 9760 us); E=192, four layers, 5 x 17 of 67 positions: 2200 -> 1825.  The steps are kept for fewer than kPassFrom positions.
+// The last layer ends with its keys and values, and no logits are formed.
+constexpr int kPassRows = 512;                       // most rows at a time (at least a position of every sequence)
+constexpr int kPassFrom = 4;
+int prompt_pass(GptDecoder &g, int B, int n_prompt, int n, int ns)
+{
+    const int E = g.E, F = g.F, D = g.E / g.H;
+    float *x = g.d_pre;
+    const int most = std::max(1, std::min(n, kPassRows / B));
+    float *q = x + (size_t)B * most * E, *att = q + (size_t)B * most * E, *ff = att + (size_t)B * most * E;
+    for (int p0 = 0; p0 < n; p0 += most) {
+        const int per_seq = std::min(most, n - p0), M = B * per_seq;
+        const cudaError_t le = launch_overlapped(embed_kernel, dim3(M), dim3(128), 0, g.stream, (const int *)g.d_prompts, n_prompt, (const int *)g.d_ids, (const int *)g.d_pos,
+                                                 (const float *)g.tok, (const float *)g.pos, x, E, g.V, per_seq, p0);
+        if (le != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "embed_kernel launch: %s", cudaGetErrorString(le));
+        int rc = check_launch("embed_kernel");
+        for (int l = 0; l < g.L && rc == HIPGPT_OK; ++l) {
+            const LayerW &w = g.lw[l];
+            float *kc = g.d_kc + (size_t)l * g.max_batch * g.S * E, *vc = g.d_vc + (size_t)l * g.max_batch * g.S * E;
+            const MatmulOut scatter{nullptr, 0, nullptr, q, kc, vc, nullptr, g.S, E, p0, per_seq};
+            rc = matmul(g, x, E, w.g1, w.be1, w.wqkv, w.bqkv, scatter, M, E, 3 * E, 0);
+            if (rc != HIPGPT_OK || l + 1 == g.L) break;
+            if ((rc = launch_decode_rows(q, kc, vc, att, M, per_seq, g.H, D, p0 + 1, g.S, ns, g.stream))) return rc;
+            if ((rc = matmul(g, att, E, nullptr, nullptr, w.wo, w.bo, plain_out(x, E, x), M, E, E, 0))) return rc;
+            if ((rc = matmul(g, x, E, w.g2, w.be2, w.w1, w.b1, plain_out(ff, F, nullptr), M, E, F, 1))) return rc;
+            rc = matmul(g, ff, F, nullptr, nullptr, w.w2, w.b2, plain_out(x, E, x), M, F, E, 0);
+        }
+        if (rc != HIPGPT_OK) return rc;
+    }
+    return HIPGPT_OK;
+}
+
+// Positions of a prompt that prompt_pass is to take (0: none), with the memory that it needs.
+int pass_positions(GptDecoder &g, int B, int n_prompt, int ns)
+{
+    const int n = n_prompt - 1, rows = B * std::max(1, std::min(n, kPassRows / B));
+    if (n < kPassFrom || g.H > 65535 || !decode_rows_supports(g.E / g.H, ns)) return 0;
+    const size_t need = (size_t)rows * (3 * g.E + g.F) * sizeof(float);
+    if (g.pre_bytes < need) {
+        if (g.d_pre) cudaFree(g.d_pre);
+        g.d_pre = nullptr;
+        g.pre_bytes = 0;
+        if (cudaMalloc(&g.d_pre, need) != cudaSuccess) {
+            cudaGetLastError();                      // the steps take the prompt
+            g.d_pre = nullptr;
+            return 0;
+        }
+        g.pre_bytes = need;
+    }
+    return n;
 }
 
 int build_graph(GptDecoder &g, int B, int n_prompt, int n_new)
@@ -795,12 +888,14 @@ int hipgpt_gpt_generate(hipgpt_gpt *handle, const int *h_prompts, int B, int n_p
     if (!g->plan.ok) cluster = 0;
     if (!persistent && !cluster) rc = build_graph(*g, B, n_prompt, n_new);
     if (rc != HIPGPT_OK) return rc;
+    const int pre = persistent ? 0 : pass_positions(*g, B, n_prompt, ns);
     CUDA_OK(cudaMemcpyAsync(g->d_prompts, h_prompts, (size_t)B * n_prompt * sizeof(int), cudaMemcpyHostToDevice, g->stream));
     CUDA_OK(cudaMemsetAsync(g->d_pos, 0, sizeof(int), g->stream));
     for (cudaEvent_t &ev : g->ev)
         if (!ev) CUDA_OK(cudaEventCreate(&ev));
     const cudaEvent_t e0 = g->ev[0], e1 = g->ev[1], e2 = g->ev[2];
     CUDA_OK(cudaEventRecord(e0, g->stream));
+    if (pre > 0 && (rc = prompt_pass(*g, B, n_prompt, pre, ns)) != HIPGPT_OK) return rc;
     if (persistent) {
         FusedArgs a{};
         a.tok = g->tok; a.pos = g->pos; a.wout = g->wout; a.layers = g->d_layers;
@@ -840,7 +935,8 @@ int hipgpt_gpt_generate(hipgpt_gpt *handle, const int *h_prompts, int B, int n_p
             a.expire_hop = kHopRecords;
             g->stall_next = false;
         }
-        a.nsteps = n_prompt;
+        a.p0 = pre;
+        a.nsteps = n_prompt - pre;
         if ((rc = launch_cluster_steps(g->plan, a, g->E, cluster, g->stream)) != HIPGPT_OK) return rc;
         CUDA_OK(cudaEventRecord(e1, g->stream));
         a.wait_cycles = kClusterWaitCycles;
@@ -849,7 +945,11 @@ int hipgpt_gpt_generate(hipgpt_gpt *handle, const int *h_prompts, int B, int n_p
         a.nsteps = n_new - 1;
         if (a.nsteps > 0 && (rc = launch_cluster_steps(g->plan, a, g->E, cluster, g->stream)) != HIPGPT_OK) return rc;
     } else {
-        for (int p = 0; p < n_prompt; ++p) CUDA_OK(cudaGraphLaunch(g->graph, g->stream));
+        if (pre > 0) {
+            set_pos_kernel<<<1, 1, 0, g->stream>>>(g->d_pos, pre);
+            if ((rc = check_launch("set_pos_kernel")) != HIPGPT_OK) return rc;
+        }
+        for (int p = pre; p < n_prompt; ++p) CUDA_OK(cudaGraphLaunch(g->graph, g->stream));
         CUDA_OK(cudaEventRecord(e1, g->stream));
         for (int i = 1; i < n_new; ++i) CUDA_OK(cudaGraphLaunch(g->graph, g->stream));
     }
@@ -909,7 +1009,7 @@ void hipgpt_gpt_destroy(hipgpt_gpt *handle)
 {
     GptDecoder *g = reinterpret_cast<GptDecoder *>(handle);
     if (!g) return;
-    float *bufs[] = {g->d_weights, g->d_kc, g->d_vc, g->d_x, g->d_h, g->d_qkv, g->d_q, g->d_att, g->d_ff, g->d_logits, g->d_scratch};
+    float *bufs[] = {g->d_weights, g->d_kc, g->d_vc, g->d_x, g->d_h, g->d_qkv, g->d_q, g->d_att, g->d_ff, g->d_logits, g->d_scratch, g->d_pre};
     for (float *b : bufs) if (b) cudaFree(b);
     if (g->graph) cudaGraphExecDestroy(g->graph);
     if (g->d_ids) cudaFree(g->d_ids);

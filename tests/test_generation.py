@@ -221,3 +221,24 @@ def test_gpu_generation_handles_of_different_widths_side_by_side():
         assert np.array_equal(a.generate(prompts, 6)[0], want)
     a.close()
     b.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cfg,B,n_prompt,n_new", [
+    (dict(V=90, S=24, E=64, L=2, H=4, F=128), 3, 5, 6),             # as few positions as are taken together; head_dim 16, one split
+    (dict(V=90, S=160, E=128, L=2, H=1, F=256), 2, 150, 4),         # head_dim 128, splits of more keys than a block's lanes hold
+    (dict(V=300, S=300, E=320, L=2, H=5, F=1280), 7, 80, 5),        # clusters; more rows than fit at a time
+    (dict(V=90, S=40, E=60 * 16, L=1, H=12, F=960), 1, 33, 3)])     # head_dim 80
+def test_gpu_generation_takes_the_positions_of_a_prompt_together(cfg, B, n_prompt, n_new):
+    pytest.importorskip("torch")
+    from hipgpt_b200 import generation
+    w = synth.gpt_weights(51, **cfg, std=0.08)
+    prompts = synth.token_ids(52, (B, n_prompt), cfg["V"])
+    ref_ids, ref_logits = ob.gpt_generate(w, **cfg, prompts=prompts, n_new=n_new, fma=True)
+    dec = generation.GptDecoder(w, **cfg, max_batch=B)
+    for n in (n_prompt, 4, n_prompt):                                # (the steps in between, on the same handle)
+        ids, logits, _, _ = dec.generate(prompts[:, :n], n_new)
+        if n == n_prompt:
+            assert np.array_equal(ids, ref_ids)
+            assert float(np.abs(logits - ref_logits).max()) <= 1e-4
+    dec.close()
