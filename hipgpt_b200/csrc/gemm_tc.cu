@@ -102,74 +102,101 @@ __global__ void __launch_bounds__(128) gemm_pack_a_kernel(const float *__restric
     const bool live = m < M;
     const float *row = A + (size_t)(live ? m : 0) * N;
     const bool vec = (N & 3) == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0;
-    auto raw8 = [&](int k0, float (&v)[8]) {
-        if (live && vec && k0 + 8 <= N) {
-            const float4 a = __ldg(reinterpret_cast<const float4 *>(row + k0)), b = __ldg(reinterpret_cast<const float4 *>(row + k0) + 1);
+    const bool ln_vec = ((reinterpret_cast<uintptr_t>(ln_g) | reinterpret_cast<uintptr_t>(ln_b)) & 15) == 0;
+    auto load8 = [&](const float *p, int k0, bool wide, float (&v)[8]) {          // values past N: zeros
+        if (wide && k0 + 8 <= N) {
+            const float4 a = __ldg(reinterpret_cast<const float4 *>(p + k0)), b = __ldg(reinterpret_cast<const float4 *>(p + k0) + 1);
             v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
         } else {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = (live && k0 + j < N) ? __ldg(row + k0 + j) : 0.0f;
+            for (int j = 0; j < 8; ++j) v[j] = k0 + j < N ? __ldg(p + k0 + j) : 0.0f;
+        }
+    };
+    auto raw8 = [&](int k0, float (&v)[8]) {
+        if (live) load8(row, k0, vec, v);
+        else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] = 0.0f;
         }
     };
     const int depth = KT * kTK;
-    float held[NV > 0 ? NV : 1][8];
+    // Gamma and beta come with the row, 16 bytes at a time, and wait in registers where the row is short: as 16 loads of 4 bytes per run of eight
+    // behind the statistics they made the two normalised packings of a block (1407 rows, E=512) 4 of its 86 us longer.  (Four warps to a long row: 82 -> 88.)
+    constexpr bool kHoldLn = NV > 0 && NV <= 2;
+    float held[NV > 0 ? NV : 1][8], gm[kHoldLn ? NV : 1][8], bt[kHoldLn ? NV : 1][8];
     if constexpr (NV > 0) {
 #pragma unroll
-        for (int i = 0; i < NV; ++i) raw8(lane * 8 + 256 * i, held[i]);          // (past N: zeros)
+        for (int i = 0; i < NV; ++i) raw8(lane * 8 + 256 * i, held[i]);
     }
-    // f(k0, values) for this lane's runs of eight
+    if constexpr (kHoldLn) {
+        if (ln_g) {
+#pragma unroll
+            for (int i = 0; i < NV; ++i) {
+                load8(ln_g, lane * 8 + 256 * i, ln_vec, gm[i]);
+                load8(ln_b, lane * 8 + 256 * i, ln_vec, bt[i]);
+            }
+        }
+    }
+    // f(i, k0, values) for this lane's runs of eight
     auto sweep = [&](auto f) {
         if constexpr (NV > 0) {
 #pragma unroll
-            for (int i = 0; i < NV; ++i) f(lane * 8 + 256 * i, held[i]);
+            for (int i = 0; i < NV; ++i) f(i, lane * 8 + 256 * i, held[i]);
         } else {
             for (int k0 = lane * 8; k0 < depth; k0 += 256) {
                 float v[8];
                 raw8(k0, v);
-                f(k0, v);
+                f(0, k0, v);
             }
         }
     };
+    auto over_row = [&](float x, auto op) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) x = op(x, __shfl_xor_sync(0xffffffffu, x, o));
+        return x;
+    };
+    auto add = [](float x, float y) { return x + y; };
     float mean = 0.0f, rstd = 1.0f;
     if (ln_g) {
         float sum = 0.0f;
-        sweep([&](int, float (&v)[8]) {
+        sweep([&](int, int, float (&v)[8]) {
 #pragma unroll
             for (int j = 0; j < 8; ++j) sum += v[j];             // values past N are zeros
         });
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-        mean = sum / (float)N;
+        mean = over_row(sum, add) / (float)N;
         float var = 0.0f;
-        sweep([&](int k0, float (&v)[8]) {
+        sweep([&](int, int k0, float (&v)[8]) {
 #pragma unroll
             for (int j = 0; j < 8; ++j) { const float d = (k0 + j < N) ? v[j] - mean : 0.0f; var = fmaf(d, d, var); }
         });
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) var += __shfl_xor_sync(0xffffffffu, var, o);
-        rstd = 1.0f / sqrtf(var / (float)N + 1e-5f);
+        rstd = 1.0f / sqrtf(over_row(var, add) / (float)N + 1e-5f);
     }
-    auto normalised = [&](int k0, float (&v)[8]) {
+    auto normalised = [&](int i, int k0, float (&v)[8]) {
         if (ln_g) {
+            float g8[8], b8[8];
+            if constexpr (!kHoldLn) {
+                load8(ln_g, k0, ln_vec, g8);
+                load8(ln_b, k0, ln_vec, b8);
+            }
 #pragma unroll
-            for (int j = 0; j < 8; ++j)
-                v[j] = (live && k0 + j < N) ? __ldg(ln_g + k0 + j) * (v[j] - mean) * rstd + __ldg(ln_b + k0 + j) : 0.0f;
+            for (int j = 0; j < 8; ++j) {
+                const float g = kHoldLn ? gm[i][j] : g8[j], b = kHoldLn ? bt[i][j] : b8[j];      // (zeros past N)
+                v[j] = live && k0 + j < N ? g * (v[j] - mean) * rstd + b : 0.0f;
+            }
         }
     };
     float amax = 0.0f;
-    sweep([&](int k0, float (&v)[8]) {
-        normalised(k0, v);                                       // (held in registers: normalised in place)
+    sweep([&](int i, int k0, float (&v)[8]) {
+        normalised(i, k0, v);                                    // (held in registers: normalised in place)
 #pragma unroll
         for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(v[j]));
     });
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    const float s = pow2_scale(amax);
+    const float s = pow2_scale(over_row(amax, [](float x, float y) { return fmaxf(x, y); }));
     if (lane == 0) row_inv[m] = pow2_inverse(s);
     const int mt = m / kTM, r = m % kTM;
-    sweep([&](int k0, float (&v)[8]) {
+    sweep([&](int i, int k0, float (&v)[8]) {
         if (NV > 0 && k0 >= depth) return;
-        if constexpr (NV == 0) normalised(k0, v);
+        if constexpr (NV == 0) normalised(i, k0, v);
         uint32_t hi[4], lo[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
