@@ -544,6 +544,31 @@ int set_gemm_attr(int dev)
     return e == cudaSuccess ? HIPGPT_OK : fail(HIPGPT_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
 }
 
+// How many clusters of `ks` blocks of the product kernel the device holds at the same time (a property of the device: asked for once on each)
+int clusters_at_once(int dev, int ks)
+{
+    static std::atomic<int> known[64][kMostSplit + 1];
+    std::atomic<int> *cell = dev >= 0 && dev < 64 ? &known[dev][ks] : nullptr;
+    if (cell && cell->load(std::memory_order_relaxed) > 0) return cell->load(std::memory_order_relaxed);
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)ks;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)(ks * 148));
+    cfg.blockDim = dim3(kGemmThreads);
+    cfg.dynamicSmemBytes = kGemmSmem;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, ks == 2 ? gemm_tc_kernel<2> : ks == 3 ? gemm_tc_kernel<3> : gemm_tc_kernel<4>, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    if (cell) cell->store(n, std::memory_order_relaxed);
+    return n;
+}
+
 // B -> its stage images and its largest magnitude (three launches on `st`; the first is a plain one, so everything
 // enqueued before has completed when the images are written)
 int pack_b(const float *B, int N, int K, uint8_t *bimg, float *b_amax, cudaStream_t st)
@@ -577,9 +602,11 @@ int pack_a_and_multiply(const float *A, const uint8_t *bimg, const float *b_amax
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
     const long long ntiles = (long long)MT * NT;
     if (ntiles > 2147483647LL) return fail(HIPGPT_ERR_BAD_ARG, "%lld output tiles are too many", ntiles);
-    // too few tiles: the slices of a tile on up to four SMs, two slices each at least (below that the exchange costs what it saves)
+    // Too few tiles: the slices of a tile on up to four SMs, two slices each at least (below that the exchange costs what it saves), and as many clusters at
+    // the same time as there are tiles: one that waits for another costs the whole product again (148 SMs in clusters of four are 33 clusters, not 37:
+    // 1152 x 2048 x 512, 36 tiles, 23.9 -> 17.7 us; 640 x 1024 x 896, 35 tiles, 17.7 -> 13.0).
     int ks = 1;
-    while (ks < kMostSplit && ntiles * (ks + 1) <= sms && KT >= 2 * (ks + 1)) ++ks;
+    while (ks < kMostSplit && ntiles * (ks + 1) <= sms && KT >= 2 * (ks + 1) && ntiles <= clusters_at_once(dev, ks + 1)) ++ks;
     const unsigned grid = ks > 1 ? (unsigned)(ntiles * ks) : (unsigned)(ntiles < sms ? ntiles : sms);      // ks = 1: one block per SM, each takes tiles in turn
     const auto kern = ks == 1 ? gemm_tc_kernel<1> : ks == 2 ? gemm_tc_kernel<2> : ks == 3 ? gemm_tc_kernel<3> : gemm_tc_kernel<4>;
     e = launch_overlapped_clusters(kern, ks, dim3(grid), dim3(kGemmThreads), kGemmSmem, st, (const uint8_t *)aimg, bimg,
