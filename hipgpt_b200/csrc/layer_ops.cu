@@ -355,14 +355,15 @@ static int launch_matmul_tiles(const float *A, const float *B, const float *bias
         if (!best || cost < best_cost) { best = &c; best_cost = cost; best_tiles = tiles; }
     }
     if (best_tiles > 2147483647LL) return fail(HIPGPT_ERR_BAD_ARG, "matmul: %lld tiles are too many", best_tiles);
-    // Blocks of an overlapped launch come in beside the last tiles of the product before, up to as many on an SM as fit: where every SM is to have two (or
-    // three), a third (fourth) that fits leaves another SM with one.  So a block asks for so much shared memory that no more than that fit.
-    // Behind itself: 8192 x 256 x 256 34.3 -> 24.3 us, 8192 x 1024 x 256 130.7 -> 90.2, 5000 x 512 x 320 66.9 -> 46.4; a block of the model, where the products
-    // follow other kernels, 333.7 -> 323.8.  (One tile per SM, and many: nothing to even out.)
+    // Blocks of an overlapped launch come in beside the last blocks of the kernel before, as many on an SM as fit, and so unevenly: where every SM is to
+    // have one, two or three, a further one that fits leaves another SM without.  So a block asks for so much shared memory that no more than that fit.
+    // Behind itself: 8192 x 256 x 256 34.3 -> 24.3 us, 8192 x 1024 x 256 130.7 -> 90.2, 5000 x 512 x 320 66.9 -> 46.4.  A block of the model, where the products
+    // follow other kernels: 8192 rows E=256 333.7 -> 322.4, sixteen others of 47 - 4807 rows 0.69 - 0.99 of their time, 0.82 in the mean (with the line at two:
+    // up to 1.26, where the kernel before has fewer blocks than fit).  More tiles per SM even out by themselves.
     const long long per_sm = (best_tiles + kSms - 1) / kSms;
     size_t smem = best->smem;
-    if (per_sm == 2 || per_sm == 3) smem = std::max(smem, (size_t)(((size_t)kSmSharedBytes / (size_t)(per_sm + 1) + 128) & ~(size_t)127));
-    cudaError_t e = cudaFuncSetAttribute(best->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max(best->smem, (size_t)kSmSharedBytes / 3 + 128));
+    if (per_sm <= 3) smem = std::max(smem, (size_t)(((size_t)kSmSharedBytes / (size_t)(per_sm + 1) + 128) & ~(size_t)127));
+    cudaError_t e = cudaFuncSetAttribute(best->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max(best->smem, (size_t)kSmSharedBytes / 2 + 128));
     if (e == cudaSuccess)
         e = launch_overlapped(best->kernel, dim3((unsigned)best_tiles), dim3(kTileThreads), smem, st, A, B, bias, C, M, N, K, (K + 16 * best->tn - 1) / (16 * best->tn));
     if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "matmul_tile_kernel: %s", cudaGetErrorString(e));
