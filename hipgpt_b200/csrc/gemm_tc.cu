@@ -605,8 +605,11 @@ int pack_a_and_multiply(const float *A, const uint8_t *bimg, const float *b_amax
     // Too few tiles: the slices of a tile on up to four SMs, two slices each at least (below that the exchange costs what it saves), and as many clusters at
     // the same time as there are tiles: one that waits for another costs the whole product again (148 SMs in clusters of four are 33 clusters, not 37:
     // 1152 x 2048 x 512, 36 tiles, 23.9 -> 17.7 us; 640 x 1024 x 896, 35 tiles, 17.7 -> 13.0).
+    // The last places are found only when the SMs come free in the right order (44 tiles in clusters of three, of which 45 fit: two waited, 7 us), so a product of
+    // few slices, which gains little by one block more, leaves a sixteenth of them: 1407 x 512 x 512 13.0 -> 10.0 us, a block of 1407 rows, E=512 81.9 -> 80.1, of 1380
+    // 80.2 -> 79.0.  With 16 slices and more the block more is worth it (leaving places there too: 80.8 and 79.2).
     int ks = 1;
-    while (ks < kMostSplit && ntiles * (ks + 1) <= sms && KT >= 2 * (ks + 1) && ntiles <= clusters_at_once(dev, ks + 1)) ++ks;
+    while (ks < kMostSplit && ntiles * (ks + 1) <= sms && KT >= 2 * (ks + 1) && ntiles * 16 <= (KT < 16 ? 15LL : 16LL) * clusters_at_once(dev, ks + 1)) ++ks;
     const unsigned grid = ks > 1 ? (unsigned)(ntiles * ks) : (unsigned)(ntiles < sms ? ntiles : sms);      // ks = 1: one block per SM, each takes tiles in turn
     const auto kern = ks == 1 ? gemm_tc_kernel<1> : ks == 2 ? gemm_tc_kernel<2> : ks == 3 ? gemm_tc_kernel<3> : gemm_tc_kernel<4>;
     e = launch_overlapped_clusters(kern, ks, dim3(grid), dim3(kGemmThreads), kGemmSmem, st, (const uint8_t *)aimg, bimg,
