@@ -166,6 +166,21 @@ mha_head_kernel(const __grid_constant__ HeadMaps maps, float *__restrict__ O, fl
     uint8_t *k_16 = base + kOffK16;              // per key tile:   rows of [K_hi (32) | K_lo (32)]
     uint8_t *v_16 = base + kOffV16;              // [V_hi | V_lo] (64 columns) fp16, N-major without swizzle: 8 keys x 8 columns
                                                  // form one 128-byte core matrix, column blocks 128 bytes apart, key groups 1024
+    // A wait tests a phase's parity, so it also passes while the phase before the one it means is still open.  Every wait for phase n
+    // therefore comes after something that implies the end of phase n - 1, and phase n + 1 cannot end before it.  Without RING that
+    // something is the same warp's wait for phase n - 1, or the waits of the one issuing warp, which takes tiles and copies in order.
+    // RING, one query tile: nobody enters head it before o_done of head it - 1, which implies every phase of that head.  During head it a group
+    // asks for phases of head it + 1 only after it has seen this head's: ld_q and ld_k behind s_full (the product needed both converted), ld_v
+    // and vx behind cv_v.  Head it + 1's own phases cannot end without the conversions that follow these waits.
+    // RING, two query tiles (probabilities stored; group n holds tile n, the first group tile 3 too):
+    //   ld_q, ld_k  the converting group has seen s_full of tile 1, hence cv_k[0] (tiles are issued in order); the next head's ld_k[0] then follows
+    //               all of this head's products, which implies the other three.
+    //   xm, xs [0]  the first group waited for the head before's as the second; the second, then the third, has seen xm[1] and xs[1], where the first
+    //               group arrives after its waits for [0].
+    //   xm, xs [1]  the third group waited for the head before's as the first; the first reaches its tile 3 only after tiles 1 and 2 were issued
+    //               into buffers that the head before's tiles 2 and 3 had left (pr_read).
+    //   p_full      tile 3's follows tile 2's in its issuing warp, which by xm[1] implies tile 0's in the same buffer.
+    //   o_done      the product of the head after follows epi_done, that is every group's waits for this head.
     __shared__ uint64_t ld_q[2], ld_k[2], ld_v[2], cv_q[2], cv_k[2], cv_v[2];
     __shared__ uint64_t s_full[3], p_full[4], o_done[2], xm[2], xs[2], epi_done, vx, pr_read[3], b_free[3];
     __shared__ uint32_t tmem_base_slot;
@@ -769,13 +784,18 @@ mha_head_kernel(const __grid_constant__ HeadMaps maps, float *__restrict__ O, fl
             if (!RING) {
                 if (grp < 2) convert_kq(it + 1, grp);
             } else if (nq == 1) {
-                if (turn > 0) convert_kq(it + 1, turn - 1);
+                if (turn > 0) {
+                    // (this group had no part in converting what it now waits for: that this head's Q and K have landed it learns from their product)
+                    wait(&s_full[buf_of(it, 0)], (uint32_t)(use_of(it, 0) & 1), 3);
+                    convert_kq(it + 1, turn - 1);
+                }
             } else if (turn == 1) {
 #pragma unroll 1
                 for (int which = 0; which < 2; ++which) convert_kq(it + 1, which);
             }
         }
         if (!PROBS && has_next && turn == (RING ? 0 : 2)) {      // the group that converts V for the next head
+            if (RING) wait(&cv_v[0], par, 2);        // (another group converted this head's V: that it has landed is known once that is done)
             v_sc = v_scale(it + 1);                  // the next head's raw V has landed (its copies were issued when this head's V had been converted)
             v_scale_known = true;
         }
@@ -819,6 +839,7 @@ mha_head_kernel(const __grid_constant__ HeadMaps maps, float *__restrict__ O, fl
         }
         if (njobs == 0) wait(&o_done[0], par, 5);        // nothing to read, but no further ahead than the groups that have
         if (PROBS && p_mapped && lane == 0) bulk_wait_read();    // the next head's V may land on the staging area
+        if (PROBS && !p_mapped) proxy_fence();                   // (plain stores staged there come before that copy)
         tc_fence_before();
         arrive(&epi_done);
         if (RING) turn = turn == 0 ? 2 : turn - 1;
@@ -877,7 +898,7 @@ int launch_mha_head(const float *q, const float *k, const float *v, float *out, 
         rc = tma_plane_map(&maps.p, probs, B * H, S, S, 32, CU_TENSOR_MAP_SWIZZLE_128B);
         if (rc != HIPGPT_OK) return rc;
     }
-    // The ring where it is the faster order: a single query tile (three heads in flight instead of one: 27.5 -> 25.6 us at B=64 H=16
+    // The ring where it is the faster order: a single query tile (three heads in flight instead of one: 27.5 -> 26.9 us at B=64 H=16
     // S=100 unmasked), and unmasked heads whose probabilities are stored (30.8 -> 30.2 us at B=32 H=8 S=256, 52.6 -> 49.7 at B=40 H=12
     // S=200).  Unmasked without them it is the slower one (21.7 against 21.0 us): the next head's first two tiles both
     // need groups that are still busy with this head's output.

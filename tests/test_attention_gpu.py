@@ -64,6 +64,33 @@ def test_whole_head_kernel_many_heads_per_block(S, causal):
     np.testing.assert_array_equal(out, plain)
 
 
+@pytest.mark.parametrize("S", [1, 33, 64, 100, 128])
+@pytest.mark.parametrize("causal", [False, True])
+def test_whole_head_kernel_one_query_tile_repeats_every_bit(S, causal):
+    """One query tile: the groups of a block convert the next head's operands in turn, beside the head that is being worked on.  Hundreds of heads,
+    launched many times from warm and from cold memory, with and without stored probabilities: every launch gives the first one's bits."""
+    from hipgpt_b200 import launchers
+    B, H, D = 75, 12, 32
+    E = H * D
+    qkv = synth.qkv_planes(170 + S, B, S, E)
+    ref_out, ref_probs = ob.mha(qkv, B, S, E, H, causal=causal, want_probs=True)
+    d_qkv, flush = dev(qkv.reshape(3, B * S, E)), torch.empty(1 << 26, device="cuda")
+    first = None
+    for i in range(40):
+        out, probs = torch.full((B * S, E), float("nan"), device="cuda"), torch.full((B, H, S, S), float("nan"), device="cuda")
+        plain = torch.full_like(out, float("nan"))
+        if i & 1:
+            flush.zero_()
+        launchers.launch_multihead_attention(d_qkv, out, probs, B, S, E, H, causal=causal)
+        if i & 1:
+            flush.zero_()
+        launchers.launch_multihead_attention(d_qkv, plain, None, B, S, E, H, causal=causal)
+        if first is None:
+            first = out, probs
+            assert _maxerr(out.cpu().numpy(), ref_out.reshape(B * S, E)) <= TOL and _maxerr(probs.cpu().numpy().reshape(-1), ref_probs.reshape(-1)) <= TOL
+        assert torch.equal(out, first[0]) and torch.equal(probs, first[1]) and torch.equal(plain, first[0])
+
+
 @pytest.mark.parametrize("S", [40, 200, 300])
 def test_output_aligned_to_16_bytes_only(S):
     """head_dim 32: an output whose rows are not whole 32-byte sectors, probabilities that are not 16-byte aligned."""
