@@ -48,6 +48,9 @@ constexpr int kRows = 128;        // query rows per block
 constexpr int kKeys = 64;         // keys per tile
 constexpr int kWorkers = kRows;
 constexpr float kRescaleStep = 8.0f;
+// The smallest factor that P takes for a tile whose V is smaller than the block's largest.  Below 2^-39 its P, at most 2^14 without it, is zero in fp16
+// whatever the factor; the row sum is taken from P in fp32, whose exponentials are flushed below 2^-126, and the factor has to have an inverse.
+constexpr float kVrelLeast = 0x1p-64f;
 constexpr float kPShift = 6.0f;   // P carries a factor 2^6: with the lazy reference maximum it stays below 2^15
 constexpr int kBufs = 2;          // S / P buffers in TMEM
 constexpr uint32_t kColX = 0, kColO = kBufs * kKeys, kTmemCols = 256;
@@ -468,13 +471,13 @@ mha_tc16_kernel(const uint8_t *__restrict__ kimg, const uint8_t *__restrict__ vi
     const uint32_t o_addr = lane_base + kColO;
 
     float m_ref = 0.0f, l = 0.0f;                    // reference maximum (log2 domain) and row sum (of P, which carries 2^6)
-    // Lane x holds the factors of tile x of 32, powers of two: one over K's, and V's against the block's (<= 1; a tile of zeros: 1).
+    // Lane x holds the factors of tile x of 32, powers of two: one over K's, and V's against the block's, no less than kVrelLeast and no more than 1.
     // (Loaded a tile ahead and divided by in every tile, they stood between the sweeps: B=16 H=8 S=1024 head_dim 64 causal 98.7 -> 97.6 us with kv_pack_kernel's halves.)
     float kinv_of = 0.0f, vrel_of = 0.0f;
     auto factors = [&](int t0) {
         const int t = min(t0 + lane, nt - 1);
         kinv_of = inverse_of_pow2(range_scale(__ldg(tmax_k + t)));
-        vrel_of = fminf(vhs / range_scale(__ldg(tmax_v + t)), 1.0f);
+        vrel_of = fminf(fmaxf(vhs / range_scale(__ldg(tmax_v + t)), kVrelLeast), 1.0f);
     };
     factors(0);
     for (int t = 0; t < nt; ++t) {

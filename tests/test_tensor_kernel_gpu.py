@@ -199,6 +199,24 @@ def test_tiled_kernel_rescales_when_row_maxima_grow(D, want_probs):
             assert float(np.abs(probs - ref_probs).max()) <= 1e-4
 
 
+@pytest.mark.parametrize("D", [32, 64])
+@pytest.mark.parametrize("e", [-30, -64, -65, -100, -126, -127, -128, -190])
+def test_tiled_kernel_row_sum_beside_value_tiles_of_unequal_size(D, e):
+    """Every tile of V has a power of two of its own, and its probabilities carry it against the largest one; the row sum counts them without it,
+    however far apart the tiles are (the factor must stay a normal number, and the exponentials that carry it above 2^-126)."""
+    B, H, S = 2, 3, 320
+    E = H * D
+    qkv = synth.qkv_planes(370 + D, B, S, E).reshape(3, B, S, E).copy()
+    big = np.float32(2.0 ** 66)
+    qkv[2] *= big
+    for tile in (0, 3):
+        qkv[2][:, 64 * tile:64 * tile + 64] = np.ldexp(qkv[2][:, 64 * tile:64 * tile + 64], e)
+    ref_out, _ = ob.mha(qkv, B, S, E, H)
+    out, _ = gpu_mha(qkv, B, S, E, H, False, False, algo=_capi.ALGO_TENSOR, warps=_capi.TENSOR_TILED)
+    assert _status() == 0
+    assert float(np.abs(out - ref_out).max()) <= TOL * float(big) * 4         # |V| reaches about 4 big
+
+
 @pytest.mark.parametrize("causal", [False, True])
 @pytest.mark.parametrize("want_probs", [False, True])
 def test_tiled_kernel_in_several_groups_of_batches(monkeypatch, causal, want_probs):
