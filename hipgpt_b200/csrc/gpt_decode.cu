@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(32 * kSeg, 2)
 matmul_rows_kernel(const float *__restrict__ A, int lda, const float *__restrict__ ln_g, const float *__restrict__ ln_b,
                    const float *__restrict__ W, const float *__restrict__ bias, MatmulOut o, int M, int K, int N, int relu)
 {
-    extern __shared__ float a_s[];
+    extern __shared__ __align__(16) float a_s[];
     dependency_wait();
     dependents_may_start();
     matmul_rows_body<false>(blockIdx.x, blockIdx.y, a_s, A, lda, ln_g, ln_b, W, bias, o, M, K, N, relu);
@@ -473,7 +473,7 @@ __device__ __forceinline__ void attn_split_phase(const FusedArgs &a, const float
 __global__ void __launch_bounds__(32 * kSeg, 1)
 gpt_steps_kernel(const FusedArgs a)
 {
-    extern __shared__ float dsm[];                   // the matmul's rows and partial sums; the other phases' scratch
+    extern __shared__ __align__(16) float dsm[];     // the matmul's rows and partial sums; the other phases' scratch
     __shared__ int ok_s;
     const int B = a.B, E = a.E, F = a.F, V = a.V, D = a.E / a.H;
     unsigned gen = *reinterpret_cast<volatile unsigned *>(a.bar + 1);   // read before this block's first arrival: cannot move yet

@@ -22,6 +22,17 @@ def test_header_and_bindings_agree():
     assert _declared_symbols() == sorted(_capi.SIGNATURES)
 
 
+def test_dynamic_shared_memory_read_in_16_byte_words_is_declared_so():
+    """A kernel that reads its dynamic shared memory in words of 16 bytes must not depend on what the linker places before it."""
+    src = os.path.join(ROOT, "hipgpt_b200", "csrc")
+    for name in sorted(os.listdir(src)):
+        text = open(os.path.join(src, name)).read()
+        if re.search(r"\b(float4|uint4)\b", text):
+            for decl in re.findall(r"extern __shared__[^;]*;", text):
+                align = re.search(r"__align__\((\d+)\)", decl)
+                assert align and int(align.group(1)) >= 16, (name, decl)
+
+
 def test_library_exports_every_declared_symbol():
     lib = _capi.lib()
     for name in _declared_symbols():
