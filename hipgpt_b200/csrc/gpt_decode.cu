@@ -659,11 +659,14 @@ int enqueue_step(GptDecoder &g, int B, int n_prompt, int n_new)
 
 // The keys and values of prompt positions 0 ... n - 1 of all sequences, every position of a layer in the same launches: the arithmetic
 // of a step, row by row, so what follows is the same bits.  A step costs the same chain of products for one position as these launches do for
-// some hundred rows.  The default model, 8 x 15 positions: 330 us instead of 15 x 72 (the whole request of 143
-// positions 10450 -> 9760 us); E=192, four layers, 5 x 17 of 67 positions: 2200 -> 1825.  The steps are kept for fewer than kPassFrom positions.
-// The last layer ends with its keys and values, and no logits are formed.
+// some hundred rows.  The default model, 8 x 15 positions: 330 us instead of 15 x 67 (the whole request of 143
+// positions 10450 -> 9760 us); E=192, four layers, 5 x 17 of 67 positions: 2200 -> 1825.  The last layer ends with its keys and values, and no logits are formed.
+// From how many positions on (us for the prompt, with these launches against steps alone): a step of the clusters is about a third as long as a layer's
+// launches, 3 positions are a draw (the default model's 8 sequences 268 against 277, 14 sequences 303 against 275, E=192 133 against 129), 4 are ahead
+// everywhere (278 against 345, 311 against 340, 134 against 159); a step of the graph is longer than the launches for one position
+// (E=512, six layers, 8 sequences 437 against 505, one 397 against 479; the default model's 32 sequences 381 against 404; E=96, two layers 87 against 105).
 constexpr int kPassRows = 512;                       // most rows at a time (at least a position of every sequence)
-constexpr int kPassFrom = 4;
+constexpr int kPassFromClusters = 4, kPassFromGraph = 1;
 int prompt_pass(GptDecoder &g, int B, int n_prompt, int n, int ns)
 {
     const int E = g.E, F = g.F, D = g.E / g.H;
@@ -693,10 +696,10 @@ int prompt_pass(GptDecoder &g, int B, int n_prompt, int n, int ns)
 }
 
 // Positions of a prompt that prompt_pass is to take (0: none), with the memory that it needs.
-int pass_positions(GptDecoder &g, int B, int n_prompt, int ns)
+int pass_positions(GptDecoder &g, int B, int n_prompt, int ns, bool clusters)
 {
     const int n = n_prompt - 1, rows = B * std::max(1, std::min(n, kPassRows / B));
-    if (n < kPassFrom || g.H > 65535 || !decode_rows_supports(g.E / g.H, ns)) return 0;
+    if (n < (clusters ? kPassFromClusters : kPassFromGraph) || g.H > 65535 || !decode_rows_supports(g.E / g.H, ns)) return 0;
     const size_t need = (size_t)rows * (3 * g.E + g.F) * sizeof(float);
     if (g.pre_bytes < need) {
         if (g.d_pre) cudaFree(g.d_pre);
@@ -889,7 +892,7 @@ int hipgpt_gpt_generate(hipgpt_gpt *handle, const int *h_prompts, int B, int n_p
     if (!g->plan.ok) cluster = 0;
     if (!persistent && !cluster) rc = build_graph(*g, B, n_prompt, n_new);
     if (rc != HIPGPT_OK) return rc;
-    const int pre = persistent ? 0 : pass_positions(*g, B, n_prompt, ns);
+    const int pre = persistent ? 0 : pass_positions(*g, B, n_prompt, ns, cluster != 0);
     CUDA_OK(cudaMemcpyAsync(g->d_prompts, h_prompts, (size_t)B * n_prompt * sizeof(int), cudaMemcpyHostToDevice, g->stream));
     CUDA_OK(cudaMemsetAsync(g->d_pos, 0, sizeof(int), g->stream));
     for (cudaEvent_t &ev : g->ev)

@@ -228,7 +228,8 @@ def test_gpu_generation_handles_of_different_widths_side_by_side():
     (dict(V=90, S=24, E=64, L=2, H=4, F=128), 3, 5, 6),             # as few positions as are taken together; head_dim 16, one split
     (dict(V=90, S=160, E=128, L=2, H=1, F=256), 2, 150, 4),         # head_dim 128, splits of more keys than a block's lanes hold
     (dict(V=300, S=300, E=320, L=2, H=5, F=1280), 7, 80, 5),        # clusters; more rows than fit at a time
-    (dict(V=90, S=40, E=60 * 16, L=1, H=12, F=960), 1, 33, 3)])     # head_dim 80
+    (dict(V=90, S=40, E=60 * 16, L=1, H=12, F=960), 1, 33, 3),      # head_dim 80
+    (dict(V=90, S=40, E=60 * 16, L=2, H=12, F=960), 2, 2, 5)])      # the graph: a single position
 def test_gpu_generation_takes_the_positions_of_a_prompt_together(cfg, B, n_prompt, n_new):
     pytest.importorskip("torch")
     from hipgpt_b200 import generation
