@@ -297,7 +297,7 @@ gemm_tc_kernel(const uint8_t *__restrict__ aimg, const uint8_t *__restrict__ bim
     };
     // The block takes output tiles blockIdx.x, + gridDim.x, ... (column tile fastest: blocks that run side by side share
     // the rows of A).  Stages are counted through all tiles (g), accumulators alternate between two halves of TMEM, so
-    // the copies of the next tile and its products run while the four epilogue warps drain the tile before it.
+    // the copies of the next tile and its products run while the eight epilogue warps drain the tile before it.
     int rank = 0;
     if constexpr (KS > 1) asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
     const int kt0 = rank * KT / KS, kt1 = (rank + 1) * KT / KS, first = (int)blockIdx.x / KS, stride = (int)gridDim.x / KS;
@@ -602,14 +602,20 @@ int pack_a_and_multiply(const float *A, const uint8_t *bimg, const float *b_amax
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
     const long long ntiles = (long long)MT * NT;
     if (ntiles > 2147483647LL) return fail(HIPGPT_ERR_BAD_ARG, "%lld output tiles are too many", ntiles);
-    // Too few tiles: the slices of a tile on up to four SMs, two slices each at least (below that the exchange costs what it saves), and as many clusters at
+    // Too few tiles: the slices of a tile on up to four SMs, two slices each at least, and as many clusters at
     // the same time as there are tiles: one that waits for another costs the whole product again (148 SMs in clusters of four are 33 clusters, not 37:
     // 1152 x 2048 x 512, 36 tiles, 23.9 -> 17.7 us; 640 x 1024 x 896, 35 tiles, 17.7 -> 13.0).
-    // The last places are found only when the SMs come free in the right order (44 tiles in clusters of three, of which 45 fit: two waited, 7 us), so a product of
-    // few slices, which gains little by one block more, leaves a sixteenth of them: 1407 x 512 x 512 13.0 -> 10.0 us, a block of 1407 rows, E=512 81.9 -> 80.1, of 1380
-    // 80.2 -> 79.0.  With 16 slices and more the block more is worth it (leaving places there too: 80.8 and 79.2).
+    // A sixteenth of the places stays free where the block more does not pay for the last ones (us back to back):
+    //   threes of fewer than 16 slices: the last places are found only when the SMs come free in the right order, of 45 that fit 43 - 45 tiles waited
+    //     (44 tiles: 8 slices 9.8, threes 12.7; 12 slices 12.0, 14.2; a block of 1407 rows, E=512 81.9 -> 80.1 with this);
+    //   pairs of fewer than 8 slices: one block alone is the faster (72 tiles: 4 slices 7.9, pairs 8.8; 6 slices 9.5, 9.7; 8 slices 10.6, 10.3; 12 slices 13.5, 12.6).
+    // Fours leave none (33 tiles: 8 slices 10.05, threes 10.3; 31 tiles, 12 slices 12.3, 12.7).
+    // Fewer blocks per tile than this would often be faster (32 tiles of 16 slices in pairs 12.2, fours 13.0; 44 of 32 in pairs 17.9, threes 18.8; fewer than 8
+    // slices alone), but the sum that one block keeps in TMEM is then longer and its error larger: 6.2e-7 instead of 3.4e-7 of the result's norm for
+    // 6 slices alone instead of on three blocks, 1.37e-6 instead of 0.97e-6 for 32 on two.
+    auto leaves_some = [&](int n) { return (n == 3 && KT < 16) || (n == 2 && KT < 8); };
     int ks = 1;
-    while (ks < kMostSplit && ntiles * (ks + 1) <= sms && KT >= 2 * (ks + 1) && ntiles * 16 <= (KT < 16 ? 15LL : 16LL) * clusters_at_once(dev, ks + 1)) ++ks;
+    while (ks < kMostSplit && ntiles * (ks + 1) <= sms && KT >= 2 * (ks + 1) && ntiles * 16 <= (leaves_some(ks + 1) ? 15LL : 16LL) * clusters_at_once(dev, ks + 1)) ++ks;
     const unsigned grid = ks > 1 ? (unsigned)(ntiles * ks) : (unsigned)(ntiles < sms ? ntiles : sms);      // ks = 1: one block per SM, each takes tiles in turn
     const auto kern = ks == 1 ? gemm_tc_kernel<1> : ks == 2 ? gemm_tc_kernel<2> : ks == 3 ? gemm_tc_kernel<3> : gemm_tc_kernel<4>;
     e = launch_overlapped_clusters(kern, ks, dim3(grid), dim3(kGemmThreads), kGemmSmem, st, (const uint8_t *)aimg, bimg,

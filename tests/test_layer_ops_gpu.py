@@ -64,8 +64,9 @@ def test_matmul_tiles_are_bit_identical_to_the_reference_order(M, K):
 
 @pytest.mark.parametrize("M,N,K,bias", [(8192, 256, 768, True), (300, 256, 768, True), (64, 1024, 256, True), (257, 256, 1024, False), (130, 64, 5000, False),
                                         (33, 100, 20, True), (5, 7, 3, False), (1, 256, 256, True), (129, 65, 129, True),
-                                        (1407, 512, 509, True), (1407, 2048, 512, False), (700, 330, 260, True),     # slices of a tile on 3, 3 and 2 blocks
-                                        (1152, 512, 510, True), (1408, 520, 384, False)])       # 36 and 33 tiles: as many clusters of four as fit, or fewer
+                                        (1407, 512, 509, True), (1407, 2048, 512, False), (700, 330, 260, True),     # slices of a tile on 2, 3 and 3 blocks
+                                        (1152, 512, 510, True), (1408, 520, 384, False),         # 36 and 33 tiles: as many clusters of four as fit, or fewer
+                                        (4700, 520, 256, True), (4700, 260, 256, False), (4750, 520, 250, False)])    # 74 tiles: all the pairs there are, one block each; 76
 def test_tensor_core_matmul_is_fp32_grade(M, N, K, bias):
     """hipgpt_matmul_tc: the projections on the tensor pipe.  Not the reference's summation order, so not its bits: the
     bar is 1e-5 relative to the largest output against a float64 product (the exact-order kernel's own distance from
