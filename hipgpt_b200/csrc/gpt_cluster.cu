@@ -25,7 +25,7 @@
 // out too, and all meet at the barriers of the remaining steps and leave.  (A barrier whose phase has not been seen complete is not
 // opened again, and the bytes that nobody waits for stay within eight layers' worth, at most 90 KB each: an mbarrier counts 2^20.)
 //
-// Measured at the default model (E=256 L=8 H=8 V=5000), batch 8: 72 us per step (the replayed graph: 318), batch 1: 67 (256).  A
+// Measured at the default model (E=256 L=8 H=8 V=5000), batch 8: 72 us per step (the replayed graph: 184), batch 1: 66 (175).  A
 // step is 42 products of 400 - 450 ns each, attention a third of a layer.  Sizes are template parameters because the chain is
 // bound by the instructions of single warps: with sizes read from the plan a step took 143 us.
 #include "gpt_cluster.cuh"
@@ -830,9 +830,12 @@ int cluster_pack(const ClusterPlan &p, int E, const ClusterLayerWeights *layers,
 // One sequence per cluster while every cluster is resident, then two; larger batches take the launches, whose matmuls share a
 // weight among eight rows.  The ring has to hold a part (sixteen chunks at most) and more.
 // `positions` of the longest context: a cluster reads its sequences' keys and values with sixteen SMs, the launches theirs with all,
-// so where few clusters have long contexts the launches are ahead.  us per position of a whole run, cluster / launches (two layers): E = 256,
-// 2 sequences: 77 / 111 at 16384, 154 / 143 at 32768; 8: 134 / 189, 249 / 253; 14: 130 / 231, 241 / 340.  E = 128, 2: 78 / 89 at 32768,
-// 155 / 113 at 65536; 8: 131 / 150, 244 / 213.  The line lies between: positions x E x (sequences per cluster) / clusters = 3 x 2^20.
+// so where few clusters have long contexts the launches are ahead.  us per position of a whole run by steps, cluster / launches (two layers): E = 256,
+// 2 sequences: 37 / 67 at 8192, 71 / 80 at 16384, 143 / 104 at 32768; 4: 40 / 76, 70 / 101.  E = 128, 2: 39 / 69 at 16384, 71 / 80 at 32768; 8: 72 / 96,
+// 128 / 130.  E = 384, 2: 75 / 96 at 8192.  The line, positions x E x (sequences per cluster) / clusters = 3 x 2^20 (24576 positions for the first), was
+// found with a slower row kernel in the launches; by these figures both sides meet at 2 to 2.6 x 2^20, and at the line the launches are up to 15 % ahead.
+// Where a prompt's positions are taken together (prompt_pass) the steps that remain are those of the longest contexts, and the sides meet earlier: E = 256,
+// 8 sequences 129 / 133 us per step behind 8159 positions, 236 / 197 behind 16351; 14: 131 / 178, 243 / 287; E = 384, 8: 120 / 146 behind 4063, 205 / 188 behind 8159.
 int cluster_rows(const ClusterPlan &p, int B, int E, int H, int ns, int positions)
 {
     if (!p.ok) return 0;

@@ -264,10 +264,10 @@ using LayerW = ClusterLayerWeights;
 // form is 52 launches of a few microseconds each; here the same phases (the same device
 // functions, the same arithmetic; the split of a (batch, head) that finishes last merges the
 // attention partials instead of a kernel of its own) follow one another inside the kernel,
-// separated by a barrier over the grid.  Measured on B200 at the default model, batch 8: 336 us
-// per step against 318 us of the replayed graph - a barrier over 148 blocks costs about what a
-// launch inside a graph costs, and the phases themselves (a few blocks each, chains of L2 round
-// trips) are the larger part of both.  Selectable (hipgpt_gpt_set_mode), not the default.  The grid is one
+// separated by a barrier over the grid.  Measured on B200 at the default model, batch 8: 299 us
+// per step against 184 us of the replayed graph (batch 1: 286, 175).  The graph's launches are overlapped
+// ones: the next kernel's blocks are resident when the one before ends, while a barrier over 148 blocks
+// is a round trip through memory for all of them.  Selectable (hipgpt_gpt_set_mode), not the default.  The grid is one
 // block per SM, co-resident by the cooperative launch.  The barrier is a counter and a
 // generation word in global memory; its wait is bounded: when it runs out, the block raises the
 // error word, every other block sees it in its own wait, and all of them return.
@@ -581,7 +581,7 @@ struct GptDecoder {
     LayerW *d_layers = nullptr;
     unsigned *d_bar = nullptr, *d_cnt = nullptr;
     int *d_err = nullptr;
-    int mode = HIPGPT_GPT_MODE_GRAPH;                // measured: the persistent form is no faster (336 against 318 us per step)
+    int mode = HIPGPT_GPT_MODE_GRAPH;                // measured: the persistent form is slower (299 against 184 us per step)
     bool persistent_ok = false;                      // head_dim, shared memory and co-residency allow it
     int grid_blocks = 0;
     size_t fused_smem = 0;

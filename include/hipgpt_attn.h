@@ -299,8 +299,8 @@ HIPGPT_API int hipgpt_gpt_create_from_run(hipgpt_gpt **out, const char *json_pat
  *     clusters of sixteen blocks run all token positions of their sequences in one launch; elsewhere one step = 52 kernel launches captured once as a CUDA graph and replayed per token.
  *   HIPGPT_GPT_MODE_PERSISTENT (head_dim % 4 == 0 and head_dim <= 128): one cooperative launch runs all
  *     prompt positions, a second one the remaining tokens; the phases of a step follow one another inside the
- *     kernel, separated by a bounded barrier over the grid (one block per SM).  Measured no faster than the
- *     graph on B200 (336 against 318 us per step of 8 tokens; the clusters: 72).
+ *     kernel, separated by a bounded barrier over the grid (one block per SM).  Measured slower than the
+ *     graph on B200 (299 against 184 us per step of 8 tokens; the clusters: 72).
  * If a wait inside a kernel of either mode runs out, hipgpt_gpt_generate returns HIPGPT_ERR_CUDA and the handle stays usable.
  */
 #define HIPGPT_GPT_MODE_GRAPH 0

@@ -225,7 +225,8 @@ def test_gpu_generation_handles_of_different_widths_side_by_side():
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("cfg,B,n_prompt,n_new", [
-    (dict(V=90, S=24, E=64, L=2, H=4, F=128), 3, 5, 6),             # as few positions as are taken together; head_dim 16, one split
+    (dict(V=90, S=24, E=64, L=2, H=4, F=128), 3, 5, 6),             # head_dim 16, one split
+    (dict(V=90, S=24, E=128, L=2, H=4, F=512), 3, 5, 6),            # clusters: as few positions as are taken together there
     (dict(V=90, S=160, E=128, L=2, H=1, F=256), 2, 150, 4),         # head_dim 128, splits of more keys than a block's lanes hold
     (dict(V=300, S=300, E=320, L=2, H=5, F=1280), 7, 80, 5),        # clusters; more rows than fit at a time
     (dict(V=90, S=40, E=60 * 16, L=1, H=12, F=960), 1, 33, 3),      # head_dim 80
