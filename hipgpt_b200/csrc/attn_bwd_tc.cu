@@ -3,10 +3,17 @@
 //     vd_ij = g_i . V_j            w_i  = sum_j P_ij vd_ij        ds_ij = P_ij (vd_ij - w_i)
 //     dQ_i  = c sum_j ds_ij K_j    dK_j = c sum_i ds_ij Q_i       dV_j  = sum_i P_ij g_i
 //
-// Arithmetic.  An fp32 number is the sum of three bf16 numbers (8 bits each, the exponent range of fp32: no scaling, any magnitude).
-// A product of two such sums is formed from six products of the pieces, hi hi, hi mid, mid hi, mid mid, hi lo, lo hi, which the
-// tensor core multiplies exactly and adds in fp32; what is dropped (mid lo, lo mid, lo lo) is below 2^-24 of the product, the
-// rounding of an fp32 product.  P and ds, formed in fp32 in registers, are cut the same way before they become operands.
+// Arithmetic.  An fp32 number, brought near 2^14 by a power of two, is the sum of two fp16 numbers to 2^-23 of it.  A product of two
+// such sums is formed from three products of the pieces, lo hi, hi lo, hi hi, which the tensor core multiplies exactly and adds in
+// fp32 (lo lo, below 2^-22 of the product, where it comes in the same instruction).  The tensor core truncates where it adds to its
+// accumulator; what that takes on the average is given back at the end.  Before, three bf16 pieces and six products: twice the instructions and half as
+// many bytes more per operand (B=3 H=12 S=777 D=64 causal 117 -> 79 us, B=32 H=8 S=256 D=32 with stored probabilities 97 -> 89.5), and the relative error of all
+// three gradients against float64 no smaller: 2.8e-7 then and 2.1e-7 now at the first shape, 1.40e-7 and 1.28e-7 at the second (0.6 - 1.0 of what it was
+// over eleven shapes of S = 77 ... 1024; dV alone, with stored probabilities at D = 64, 0.93e-7 -> 1.09e-7).
+// Powers of two: one per 64-row tile for Q, K, V and dO, kept beside the images; for P and ds, which are formed in fp32 in registers,
+// one per thread (32 columns of a row or key of a tile).  An accumulator holds one tile and one half of its columns, and the factors leave
+// where the workers add it to the running sum; those of a tile's scores go into the multiply-adds that form P and ds.  A value
+// keeps its 22 bits down to 2^-15 of the largest of its tile, below that what the largest leaves of it: 2^-39 of that one.
 //
 // Three kernels per group of batches:
 //   bwd_pack_kernel   Q, K, V, dO -> their pieces, once per call, in the order in which shared memory holds an operand: 8 x 8 core
@@ -28,6 +35,7 @@
 #include "tc_primitives.cuh"
 #include "tma_host.cuh"
 
+#include <cuda_fp16.h>
 #include <math.h>
 #include <type_traits>
 
@@ -55,51 +63,84 @@ __device__ __noinline__ bool bwd_wait_slow(uint64_t *bar, uint32_t parity, int s
 template <int D>
 struct Img {
     static constexpr int kPiece = (D / 8) * 128;     // one piece of an 8-row block
-    static constexpr int kBlock = 3 * kPiece;        // an 8-row block
+    static constexpr int kBlock = 2 * kPiece;        // an 8-row block
     static constexpr int kTileBytes = (kTile / 8) * kBlock;     // 64 rows
 };
 
-// Two fp32 numbers -> three words of two bf16 each whose sums are the numbers (to 2^-25 of them)
-__device__ __forceinline__ void cut3(float x, float y, uint32_t &h, uint32_t &m, uint32_t &l)
+// Two fp32 numbers below 2^16 -> two words of two fp16 each whose sums are the numbers (to 2^-23 of them, 2^-25 where that is more).
+// An infinity leaves a NaN.
+__device__ __forceinline__ void cut2(float2 x, uint32_t &h, uint32_t &l)
 {
-    h = pack_bf16(x, y);
-    const float2 r = fadd2(make_float2(x, y), make_float2(-__uint_as_float(h << 16), -__uint_as_float(h & 0xffff0000u)));
-    m = pack_bf16(r.x, r.y);
-    const float2 s = fadd2(r, make_float2(-__uint_as_float(m << 16), -__uint_as_float(m & 0xffff0000u)));
-    l = pack_bf16(s.x, s.y);
+    const __half2 hh = __float22half2_rn(x);
+    const float2 back = __half22float2(hh);
+    const __half2 ll = __float22half2_rn(fadd2(x, make_float2(-back.x, -back.y)));
+    h = *reinterpret_cast<const uint32_t *>(&hh);
+    l = *reinterpret_cast<const uint32_t *>(&ll);
 }
 
+// The power of two that brings a largest magnitude into [2^14, 2^15), and one over it, from the magnitude's bits.  Magnitudes
+// below 2^-100 are treated as that; an infinite one leaves both normal numbers.
+__device__ __forceinline__ uint32_t range_exponent(uint32_t bits) { return max(bits & 0x7f800000u, 27u << 23); }
+__device__ __forceinline__ float range_up(uint32_t e) { return __uint_as_float((268u << 23) - e); }
+__device__ __forceinline__ float range_down(uint32_t e) { return __uint_as_float(e - (14u << 23)); }
+
 // ---- the pieces of the four planes ---------------------------------------------------------------------
-// A warp takes 8 rows x 32 columns: lane = (column block of 8) * 8 + row, so that it reads 8 whole lines and writes four core
-// matrices of 128 contiguous bytes per piece.  Bound by memory: 4 bytes read and 6 written per element.
+// A block takes a 64-row tile of a head in one plane, a warp 8 of its rows: lane = (column block of 8) * 8 + row, so that it reads 8 whole lines and
+// writes core matrices of 128 contiguous bytes per piece.  fac: [plane][tile], what an image is multiplied by to give the plane.  The tile's
+// largest magnitude counts finite values only: an infinity becomes NaN in its own row and the tile's other rows keep their scale.
+// Bound by memory: 4 bytes read and 4 written per element.
 template <int D>
 __global__ void __launch_bounds__(256)
 bwd_pack_kernel(const float *__restrict__ q, const float *__restrict__ k, const float *__restrict__ v, const float *__restrict__ g,
-                uint8_t *__restrict__ img, size_t img_bytes, int S, int Spad, int E, int H, int tasks)
+                uint8_t *__restrict__ img, size_t img_bytes, float *__restrict__ fac, int S, int nt, int E, int H)
 {
     constexpr int PARTS = D / 32;
+    __shared__ uint32_t red[8];
     dependency_wait();
     dependents_may_start();
-    const int task = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (task >= tasks) return;
-    const int part = task % PARTS, rb = (task / PARTS) % (Spad / 8), bh = task / PARTS / (Spad / 8);
-    const int r = lane & 7, cb = part * 4 + (lane >> 3), row = rb * 8 + r;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int t = (int)blockIdx.x % nt, bh = (int)blockIdx.x / nt;
+    const int r = lane & 7, row = t * kTile + warp * 8 + r;
     const float *src = blockIdx.y == 0 ? q : blockIdx.y == 1 ? k : blockIdx.y == 2 ? v : g;
-    float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
-    if (row < S) {
-        const float4 *p = reinterpret_cast<const float4 *>(src + ((size_t)(bh / H) * S + row) * E + (size_t)(bh % H) * D + cb * 8);
-        a = __ldg(p);
-        b = __ldg(p + 1);
+    float4 x[PARTS][2];
+    uint32_t mx = 0;
+#pragma unroll
+    for (int p = 0; p < PARTS; ++p) {
+        x[p][0] = x[p][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (row < S) {
+            const float4 *at = reinterpret_cast<const float4 *>(src + ((size_t)(bh / H) * S + row) * E + (size_t)(bh % H) * D + p * 32 + (lane >> 3) * 8);
+            x[p][0] = __ldg(at);
+            x[p][1] = __ldg(at + 1);
+        }
     }
-    uint4 h, m, l;
-    cut3(a.x, a.y, h.x, m.x, l.x);
-    cut3(a.z, a.w, h.y, m.y, l.y);
-    cut3(b.x, b.y, h.z, m.z, l.z);
-    cut3(b.z, b.w, h.w, m.w, l.w);
-    uint8_t *dst = img + blockIdx.y * img_bytes + ((size_t)bh * (Spad / 8) + rb) * Img<D>::kBlock + cb * 128 + r * 16;
-    *reinterpret_cast<uint4 *>(dst) = h;
-    *reinterpret_cast<uint4 *>(dst + Img<D>::kPiece) = m;
-    *reinterpret_cast<uint4 *>(dst + 2 * Img<D>::kPiece) = l;
+#pragma unroll
+    for (int p = 0; p < PARTS; ++p)
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const uint32_t m = __float_as_uint(reinterpret_cast<const float *>(&x[p][c])[u]) & 0x7fffffffu;
+                mx = m < 0x7f800000u ? max(mx, m) : mx;
+            }
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    if (lane == 0) red[warp] = mx;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) mx = max(mx, red[i]);
+    const uint32_t e = range_exponent(mx);
+    const float up = range_up(e);
+    if (threadIdx.x == 0) fac[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = range_down(e);
+    uint8_t *dst = img + blockIdx.y * img_bytes + (size_t)blockIdx.x * Img<D>::kTileBytes + warp * Img<D>::kBlock + (lane >> 3) * 128 + r * 16;
+#pragma unroll
+    for (int p = 0; p < PARTS; ++p) {
+        uint4 h, l;
+        cut2(make_float2(x[p][0].x * up, x[p][0].y * up), h.x, l.x);
+        cut2(make_float2(x[p][0].z * up, x[p][0].w * up), h.y, l.y);
+        cut2(make_float2(x[p][1].x * up, x[p][1].y * up), h.z, l.z);
+        cut2(make_float2(x[p][1].z * up, x[p][1].w * up), h.w, l.w);
+        *reinterpret_cast<uint4 *>(dst + p * 512) = h;
+        *reinterpret_cast<uint4 *>(dst + p * 512 + Img<D>::kPiece) = l;
+    }
 }
 
 // ---- the products, issued by one converged warp that elects the lane per instruction ---------------------
@@ -108,10 +149,10 @@ template <int D>
 __device__ __forceinline__ void issue_scores(uint32_t d_tmem, uint32_t a_smem, uint32_t b_smem)
 {
     const uint64_t a = make_desc(a_smem, 128, Img<D>::kBlock, 0), b = make_desc(b_smem, 128, Img<D>::kBlock, 0);
-    constexpr uint32_t id = idesc_bf16(kLanes, kTile, 0);
-    constexpr int PA[6] = {0, 2, 1, 1, 0, 0}, PB[6] = {2, 0, 1, 0, 1, 0};        // small terms first
+    constexpr uint32_t id = idesc_f16(kLanes, kTile);
+    constexpr int PA[3] = {1, 0, 0}, PB[3] = {0, 1, 0};      // small terms first
 #pragma unroll
-    for (int p = 0; p < 6; ++p)
+    for (int p = 0; p < 3; ++p)
 #pragma unroll
         for (int k = 0; k < D / 16; ++k) {
             const uint64_t da = a + (uint64_t)((PA[p] * (D / 8) + 2 * k) * 8), db = b + (uint64_t)((PB[p] * (D / 8) + 2 * k) * 8);
@@ -119,81 +160,97 @@ __device__ __forceinline__ void issue_scores(uint32_t d_tmem, uint32_t a_smem, u
         }
 }
 
-// acc[tmem] (128 x D) = A B over rows [16 KS0, 16 KS1) of B's image, read N-major; A: three pieces in TMEM, the piece `p` of the columns
-// [32 hf, 32 hf + 32) packed in 16 columns at a_col(p, hf).  WIDE: acc is 2 D columns, the second half collects the products with
-// B's mid and lo pieces (wider instructions, fewer of them).  The small products come first: the tensor core truncates where
-// it adds to its accumulator, so the accumulator should be small while they are added, and it starts anew for every tile (the
-// workers add the tiles up in registers).  One accumulator over all tiles was 10 times farther from float64 at S = 777.
-template <int D, bool WIDE, int KS0, int KS1, typename ACol>
-__device__ __forceinline__ void issue_accumulate(uint32_t acc, ACol a_col, uint32_t b_smem)
+// acc[tmem] (128 x D) = A B over rows [32 hf, 32 hf + 32) of B's image, read N-major; A: two pieces in TMEM, 16 columns each, hi first.
+// WIDE: acc is 2 D columns, the second half collects the products with B's lo pieces (wider instructions, fewer of them).  The
+// small products come first: the tensor core truncates where it adds to its accumulator, so the accumulator should be small
+// while they are added, and it starts anew for every tile (the workers add the tiles up in registers).  One accumulator over all
+// tiles was 10 times farther from float64 at S = 777.
+template <int D, bool WIDE>
+__device__ __forceinline__ void issue_accumulate(uint32_t acc, uint32_t a_tmem, uint32_t b_smem, int hf)
 {
-    const uint64_t b = make_desc(b_smem, Img<D>::kBlock, 128, 0);
-    constexpr uint32_t id1 = idesc_bf16(kLanes, D, 1), id2 = idesc_bf16(kLanes, 2 * D, 1);
-    auto product = [&](int pa, int pb, int d, uint32_t id, bool fresh) {
+    const uint64_t b = make_desc(b_smem, Img<D>::kBlock, 128, 0) + (uint64_t)(hf * 4 * (Img<D>::kBlock >> 4));
+    constexpr uint32_t id = idesc_f16(kLanes, WIDE ? 2 * D : D) | (1u << 16);
+    auto product = [&](int pa, int pb, bool fresh) {
 #pragma unroll
-        for (int ks = KS0; ks < KS1; ++ks) {
+        for (int ks = 0; ks < 2; ++ks) {
             const uint64_t bk = b + (uint64_t)(ks * 2 * (Img<D>::kBlock >> 4) + pb * (Img<D>::kPiece >> 4));
-            if (elect_one()) mma_h_ts(acc + d, a_col(pa, ks >> 1) + (ks & 1) * 8, bk, id, (fresh && ks == KS0) ? 0u : 1u);
+            if (elect_one()) mma_h_ts(acc, a_tmem + 16 * pa + 8 * ks, bk, id, (fresh && ks == 0) ? 0u : 1u);
         }
     };
-    if (WIDE) {
-        product(1, 0, 0, id2, true);                 // mid x [hi | mid]
-        product(2, 0, 0, id1, false);                // lo x hi
-        product(0, 2, D, id1, false);                // hi x lo
-        product(0, 0, 0, id2, false);                // hi x [hi | mid]
-    } else {
-        product(0, 2, 0, id1, true);
-        product(2, 0, 0, id1, false);
-        product(1, 1, 0, id1, false);
-        product(0, 1, 0, id1, false);
-        product(1, 0, 0, id1, false);
-        product(0, 0, 0, id1, false);
-    }
+    product(1, 0, true);                             // lo x hi (WIDE: lo x [hi | lo])
+    if (!WIDE) product(0, 1, false);                 // hi x lo
+    product(0, 0, false);                            // hi x hi (WIDE: hi x [hi | lo])
 }
 
-// 32 numbers of a row (or key) -> their three pieces at the given TMEM columns
-__device__ __forceinline__ void store_pieces(const float (&x)[32], uint32_t hi, uint32_t mid, uint32_t lo)
+// 32 numbers of a row (or key), scaled by a power of two of their own -> their two pieces in 32 TMEM columns, hi first.  Returns one
+// over the factor.
+__device__ __forceinline__ float store_pieces(const float (&x)[32], uint32_t addr)
 {
-    uint32_t h[16], m[16], l[16];
+    float m4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-    for (int c = 0; c < 16; ++c) cut3(x[2 * c], x[2 * c + 1], h[c], m[c], l[c]);
-    tmem_st16_u32(hi, h);
-    tmem_st16_u32(mid, m);
-    tmem_st16_u32(lo, l);
+    for (int c = 0; c < 32; c += 2) m4[(c >> 1) & 3] = max3(m4[(c >> 1) & 3], fabsf(x[c]), fabsf(x[c + 1]));
+    const uint32_t e = range_exponent(__float_as_uint(max3(fmaxf(m4[0], m4[1]), m4[2], m4[3])));
+    const float up = range_up(e);
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        uint32_t h[8], l[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) cut2(fmul2(make_float2(x[16 * half + 2 * c], x[16 * half + 2 * c + 1]), make_float2(up, up)), h[c], l[c]);
+        tmem_st8_u32(addr + 8 * half, h);
+        tmem_st8_u32(addr + 16 + 8 * half, l);
+    }
+    return range_down(e);
 }
 
-// Adds a tile's accumulator (this thread's D / 2 columns of its row) to the running sum
+// Adds a tile's two accumulators (one per half of its columns; this thread's D / 2 columns of its row) times their factors to the running sum
 template <int D, bool WIDE>
-__device__ __forceinline__ void add_tile(uint32_t acc, int hf, float (&o)[D / 2])
+__device__ __forceinline__ void add_tile(uint32_t acc, int hf, float f0, float f1, float (&o)[D / 2])
 {
+    constexpr int kAcc = WIDE ? 2 * D : D;
 #pragma unroll
     for (int c0 = 0; c0 < D / 2; c0 += 16) {
-        float a[16], b[16];
-        tmem_ld16(acc + hf * (D / 2) + c0, a);
-        if (WIDE) tmem_ld16(acc + D + hf * (D / 2) + c0, b);
+        float a[2][16], b[2][16];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            tmem_ld16(acc + u * kAcc + hf * (D / 2) + c0, a[u]);
+            if (WIDE) tmem_ld16(acc + u * kAcc + D + hf * (D / 2) + c0, b[u]);
+        }
         tmem_wait_ld();
 #pragma unroll
         for (int c = 0; c < 16; c += 2) {
-            float2 t = make_float2(a[c], a[c + 1]);
-            if (WIDE) t = fadd2(t, make_float2(b[c], b[c + 1]));
-            t = fadd2(make_float2(o[c0 + c], o[c0 + c + 1]), t);
+            float2 y[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                y[u] = make_float2(a[u][c], a[u][c + 1]);
+                if (WIDE) y[u] = fadd2(y[u], make_float2(b[u][c], b[u][c + 1]));
+            }
+            // (the halves first: one addition to the long sum per tile)
+            const float2 t = fadd2(make_float2(o[c0 + c], o[c0 + c + 1]), ffma2(y[1], make_float2(f1, f1), fmul2(y[0], make_float2(f0, f0))));
             o[c0 + c] = t.x;
             o[c0 + c + 1] = t.y;
         }
     }
 }
 
+// The tensor core cuts off, towards zero, what does not fit where it adds to its accumulator: results come out smaller by so much on the
+// average, whatever the sizes (measured against float64: 5.1 - 5.5e-8 behind the one product of dV, 1.2 - 1.4e-7 behind the two of dQ and dK).
+// It is given back with the last multiplication.
+constexpr float kSumLoss = 5.4e-8f, kScoreLoss = 1.3e-7f;
+
 // A warp's 32 rows x D / 2 results leave in whole lines: through shared memory (boxes of 32 x 32, 16-byte pieces permuted by the row; at head_dim
 // 32 the two warps of a quarter share one), then a row of 128 bytes per eight lanes.  A thread's own stores touched 32 lines
 // each (1.2 us at the end of a 10.7 us block of columns).  dst: the head's first column of the warp's first row.
 template <int D>
-__device__ __forceinline__ void store_out(const float (&o)[D / 2], int warp, int lane, float scale, uint8_t *stage, float *dst, int E, int nrows, bool off)
+__device__ __forceinline__ void store_out(const float (&o)[D / 2], int warp, int lane, float scale, float loss, uint8_t *stage, float *dst, int E, int nrows, bool off)
 {
     const int wq = warp & 3, hf = warp >> 2;
     uint8_t *box = stage + (D == 64 ? warp : wq) * 4096;
 #pragma unroll
-    for (int c = 0; c < D / 8; ++c)
-        *reinterpret_cast<float4 *>(box + sw128(lane, D == 64 ? c : hf * 4 + c)) = make_float4(o[4 * c] * scale, o[4 * c + 1] * scale, o[4 * c + 2] * scale, o[4 * c + 3] * scale);
+    for (int c = 0; c < D / 8; ++c) {
+        float4 x = make_float4(o[4 * c] * scale, o[4 * c + 1] * scale, o[4 * c + 2] * scale, o[4 * c + 3] * scale);
+        x.x = fmaf(x.x, loss, x.x); x.y = fmaf(x.y, loss, x.y); x.z = fmaf(x.z, loss, x.z); x.w = fmaf(x.w, loss, x.w);
+        *reinterpret_cast<float4 *>(box + sw128(lane, D == 64 ? c : hf * 4 + c)) = x;
+    }
     if (D == 64) __syncwarp();
     else asm volatile("bar.sync %0, 64;" ::"r"(2 + wq) : "memory");
     constexpr int kRows = D == 64 ? 32 : 16;
@@ -205,7 +262,7 @@ __device__ __forceinline__ void store_out(const float (&o)[D / 2], int warp, int
     }
 }
 
-// ---- rows: log-sum-exp, w, dQ --------------------------------------------------------------------------
+// ---- rows: maximum and sum, w, dQ --------------------------------------------------------------------------
 // STORED: where the probabilities come from.  0: formed again from Q and K.  1: the caller's, one tile ahead through registers
 // (rows that TMA cannot address: S not a multiple of four).  2: the caller's, by TMA into a ring of tiles: a tile of
 // the first sweep took 1.2 us, which was the latency of the loads one tile ahead; no registers and no turning are needed
@@ -216,21 +273,26 @@ using PMap = std::conditional_t<STORED == 2, CUtensorMap, int>;
 template <int D>
 constexpr int kPStages = D == 32 ? 3 : 2;
 
+// A worker writes the factor of its piece of tile i beside tile i and reads that of both halves when tile i + 1 is under way.  The other half's
+// worker may be as far as tile i + 2 then (whose scores are formed before tile i + 1 has been handed over), not i + 3.
+constexpr int kDownSlots = 4;
+
 template <int D, int STORED>
 struct RowsCfg {
-    static constexpr int kKStages = D == 32 ? 4 : (STORED ? 2 : 3);      // what 227 KB hold beside Q, dO and the probabilities
-    static constexpr int kVStages = D == 32 ? 4 : 2;
+    static constexpr int kKStages = D == 64 && STORED ? 3 : 4;           // what 227 KB hold beside Q, dO and the probabilities
+    static constexpr int kVStages = kKStages;
     static constexpr int kResident = (STORED ? 1 : 2) * 2 * Img<D>::kTileBytes;      // dO and, to form P again, Q: 128 rows each
     // 1: per warp 32 rows x 32 probabilities on their way to their rows
     static constexpr int kStage = STORED == 2 ? kPStages<D> * kPTile : STORED == 1 ? kWorkerWarps * 4096 : 0;
     static constexpr size_t kSmem = (STORED == 2 ? 1024 : 0) + (size_t)kResident + (kKStages + kVStages) * Img<D>::kTileBytes + kStage;
-    static constexpr uint32_t kColAcc = 4 * kTile;                       // after two buffers of S and dP: two accumulators of 2 D columns
+    static constexpr bool kWide = D == 32;                               // an accumulator has 64 columns
+    static constexpr uint32_t kColAcc = 4 * kTile;                       // after two buffers of S and dP: an accumulator per half tile
 };
 
 template <int D, bool CAUSAL, int STORED>
 __global__ void __launch_bounds__(kThreads, 1)
-bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *__restrict__ P, float *__restrict__ dQ,
-                float *__restrict__ lse_out, float *__restrict__ w_out, int S, int Spad, int E, int H, int nblk, float c, const __grid_constant__ PMap<STORED> p_map, int expire)
+bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *fac, const float *__restrict__ P, float *__restrict__ dQ,
+                float *__restrict__ stat, size_t nstat, int S, int Spad, int E, int H, int nblk, float c, const __grid_constant__ PMap<STORED> p_map, int expire)
 {
     using C = RowsCfg<D, STORED>;
     constexpr int TB = Img<D>::kTileBytes;
@@ -239,6 +301,7 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
     uint8_t *q_s = p_s + C::kStage, *g_s = q_s + (STORED ? 0 : 2 * TB), *k_s = g_s + 2 * TB, *v_s = k_s + C::kKStages * TB;
     __shared__ uint64_t res_full, k_full[C::kKStages], v_full[C::kVStages], sd_full[2], ready[2], acc_done[2], p_full[STORED == 2 ? kPStages<D> : 1];
     __shared__ float comb[2][STORED ? 1 : 3][kLanes];           // w and, where P is formed again, maximum and sum of each half row
+    __shared__ float down_s[kDownSlots][2][kLanes];             // a tile's factors: [half][row]
     __shared__ uint32_t tmem_base_slot;
     __shared__ volatile int abort_flag;
 
@@ -369,9 +432,8 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
                 wait(&k_full[k_slot(i)], k_phase(i), 2);
                 tc_fence_after();
                 const uint32_t s0 = tmem + (uint32_t)((i & 1) * 2 * kTile), kt = smem_u32(k_s + k_slot(i) * TB);
-                auto a_col = [&](int p, int hf) { return p == 2 ? s0 + kTile + 32 * hf : s0 + 32 * hf + 16 * p; };
-                if (first) issue_accumulate<D, true, 0, 2>(tmem + C::kColAcc, a_col, kt);
-                else issue_accumulate<D, true, 2, 4>(tmem + C::kColAcc + 2 * D, a_col, kt);
+                const int half = first ? 0 : 1;
+                issue_accumulate<D, C::kWide>(tmem + C::kColAcc + 64 * half, s0 + 32 * half, kt, half);
                 if (elect_one()) tc_commit(&acc_done[i & 1]);
             }
         }
@@ -427,21 +489,32 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         for (int ch = 0; ch < 8; ++ch) *reinterpret_cast<float4 *>(&p[ch * 4]) = *reinterpret_cast<const float4 *>(src + sw128(r0, ch));
     };
 
-    float m = -INFINITY, l = 0.0f, w = 0.0f, lse = 0.0f;
+    float m = -INFINITY, l = 0.0f, w = 0.0f, rinv = 1.0f;
     float o[D / 2];
 #pragma unroll
     for (int x = 0; x < D / 2; ++x) o[x] = 0.0f;
     auto add_dq = [&](int i) {                       // tile i of the second sweep has been accumulated
         wait_w(&acc_done[i & 1], (uint32_t)(((i - nk) >> 1) & 1), 6);
         tc_fence_after();
-        add_tile<D, true>(lane_base + C::kColAcc, hf, o);
-        add_tile<D, true>(lane_base + C::kColAcc + 2 * D, hf, o);
+        add_tile<D, C::kWide>(lane_base + C::kColAcc, hf, down_s[i % kDownSlots][0][rloc], down_s[i % kDownSlots][1][rloc], o);
     };
+    // factors: of this row's Q (with the exponent's) and dO, and of 32 tiles of K and V, one per lane
+    const size_t ntile = (size_t)nbh * (Spad / kTile), tile0 = (size_t)bh * (Spad / kTile);
+    const float q_fac = STORED ? 0.0f : cl2 * fac[tile0 + row / kTile], g_fac = fac[3 * ntile + tile0 + row / kTile];
+    float k_facs = 0.0f, v_facs = 0.0f;
     if (STORED == 1) fetch_p(0);
     for (int i = 0; i < total; ++i) {
         const uint32_t s_addr = lane_base + (uint32_t)((i & 1) * 2 * kTile) + hf * 32, dp_addr = s_addr + kTile;
-        const int j0 = (i % nk) * kTile + hf * 32;
+        const int kt = i < nk ? i : i - nk, j0 = kt * kTile + hf * 32;
         const int nvalid = min(S - j0, CAUSAL ? row - j0 + 1 : 32);      // columns of this row that count
+        if ((kt & 31) == 0) {
+            const size_t at = tile0 + min(kt + lane, Spad / kTile - 1);
+            k_facs = fac[ntile + at];
+            v_facs = fac[2 * ntile + at];
+        }
+        const float k_fac = __shfl_sync(0xffffffffu, k_facs, kt & 31), dp_fac = g_fac * __shfl_sync(0xffffffffu, v_facs, kt & 31);
+        const float s_fac = fmaxf(q_fac * k_fac, 1e-37f);        // (never zero: a hidden score is -inf, and times the factor it stays that)
+        const float2 dp2 = make_float2(dp_fac, dp_fac), s2 = make_float2(s_fac, s_fac);
         float s[32], dp[32];
         if (i == nk) {
             // the first sweep is over: join the two halves of each row
@@ -457,14 +530,16 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
                 const float a1 = ex2_approx(m - mn), a2 = ex2_approx(m2 - mn);
                 const float la = l * a1, lb = l2 * a2, wa = w * a1, wb = w2 * a2;
                 l = hf == 0 ? la + lb : lb + la;
-                w = (hf == 0 ? wa + wb : wb + wa) / fmaxf(l, 1e-30f);
-                lse = mn + log2f(fmaxf(l, 1e-30f));
+                rinv = 1.0f / fmaxf(l, 1e-30f);
+                w = (hf == 0 ? wa + wb : wb + wa) * rinv;
+                m = mn;
             }
             if (hf == 0) {                           // rows past S: a probability of 0 for every key
                 // after a wait that ran out: NaN, so that no block of columns makes a result of what the buffer held before
                 const bool lost = abort_flag;
-                if (!STORED) lse_out[(size_t)bh * Spad + row] = lost ? NAN : row < S ? lse : 1e30f;
-                w_out[(size_t)bh * Spad + row] = lost ? NAN : row < S ? w : 0.0f;
+                float *at = stat + (size_t)bh * Spad + row;
+                at[0] = lost ? NAN : row < S ? w : 0.0f;
+                if (!STORED) { at[nstat] = lost ? NAN : row < S ? m : 0.0f; at[2 * nstat] = lost ? NAN : row < S ? rinv : 0.0f; }
             }
         }
         if (STORED) {
@@ -485,7 +560,7 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
                     if (CAUSAL) { s[x] = x < nvalid ? s[x] : 0.0f; s[x + 1] = x + 1 < nvalid ? s[x + 1] : 0.0f; }
                     ws[(x >> 1) & 1] = ffma2(make_float2(s[x], s[x + 1]), make_float2(dp[x], dp[x + 1]), ws[(x >> 1) & 1]);
                 }
-                w += (ws[0].x + ws[0].y) + (ws[1].x + ws[1].y);
+                w = fmaf((ws[0].x + ws[0].y) + (ws[1].x + ws[1].y), dp_fac, w);
             } else if (nvalid > 0) {
                 float mx = -INFINITY;
                 if (nvalid < 32) {
@@ -494,36 +569,36 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
                 }
 #pragma unroll
                 for (int x = 0; x < 32; x += 2) mx = max3(mx, s[x], s[x + 1]);
-                const float mn = fmaxf(m, mx * cl2), alpha = ex2_approx(m - mn);
+                const float mn = fmaxf(m, mx * s_fac), alpha = ex2_approx(m - mn);
                 m = mn;
                 float2 ls[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)}, ws[2] = {ls[0], ls[0]};
 #pragma unroll
                 for (int x = 0; x < 32; x += 2) {
-                    const float2 t = ffma2(make_float2(s[x], s[x + 1]), make_float2(cl2, cl2), make_float2(-mn, -mn));
+                    const float2 t = ffma2(make_float2(s[x], s[x + 1]), s2, make_float2(-mn, -mn));
                     const float2 e = make_float2(ex2_approx(t.x), ex2_approx(t.y));
                     ls[(x >> 1) & 1] = fadd2(ls[(x >> 1) & 1], e);
                     ws[(x >> 1) & 1] = ffma2(e, make_float2(dp[x], dp[x + 1]), ws[(x >> 1) & 1]);
                 }
                 l = fmaf(l, alpha, (ls[0].x + ls[0].y) + (ls[1].x + ls[1].y));
-                w = fmaf(w, alpha, (ws[0].x + ws[0].y) + (ws[1].x + ws[1].y));
+                w = fmaf(w, alpha, ((ws[0].x + ws[0].y) + (ws[1].x + ws[1].y)) * dp_fac);
             }
         } else {
 #pragma unroll
             for (int x = 0; x < 32; x += 2) {
                 float2 p = make_float2(s[x], s[x + 1]);
                 if (!STORED) {
-                    p = ffma2(p, make_float2(cl2, cl2), make_float2(-lse, -lse));
+                    p = ffma2(p, s2, make_float2(-m, -m));         // (1 / l leaves with the row of dQ)
                     p = make_float2(ex2_approx(p.x), ex2_approx(p.y));
                 }
-                const float2 d = fadd2(make_float2(dp[x], dp[x + 1]), make_float2(-w, -w));
-                dp[x] = p.x * d.x;
-                dp[x + 1] = p.y * d.y;
+                const float2 d = fmul2(p, ffma2(make_float2(dp[x], dp[x + 1]), dp2, make_float2(-w, -w)));
+                dp[x] = d.x;
+                dp[x + 1] = d.y;
             }
             if (nvalid < 32) {
 #pragma unroll
                 for (int x = 0; x < 32; ++x) dp[x] = x < nvalid ? dp[x] : 0.0f;
             }
-            store_pieces(dp, s_addr, s_addr + 16, dp_addr);
+            down_s[i % kDownSlots][hf][rloc] = store_pieces(dp, s_addr) * k_fac;
             if (i > nk) add_dq(i - 1);
             tmem_wait_st();
             arrive(&ready[i & 1]);
@@ -532,7 +607,7 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
     add_dq(total - 1);
     // (through the K tiles' memory: the last product has read it)
     const int row0 = q0 + wq * 32;
-    store_out<D>(o, warp, lane, c, k_s, dQ + ((size_t)b * S + row0) * E + (size_t)h * D, E, S - row0, abort_flag);
+    store_out<D>(o, warp, lane, c * rinv, kScoreLoss, k_s, dQ + ((size_t)b * S + row0) * E + (size_t)h * D, E, S - row0, abort_flag);
     tc_fence_before();
     __syncthreads();
 }
@@ -540,30 +615,29 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
 // ---- columns: dK, dV -----------------------------------------------------------------------------------
 template <int D, int STORED>
 struct ColsCfg {
-    static constexpr int kStages = D == 32 ? 4 : 2;                      // (Q, dO) tile pairs
+    static constexpr int kStages = D == 64 && STORED ? 3 : 4;            // (Q, dO) tile pairs
     static constexpr int kResident = (STORED ? 1 : 2) * 2 * Img<D>::kTileBytes;      // V and, to form P again, K: 128 rows each
     static constexpr int kStage = STORED == 2 ? kPStages<D> * kPTile : 0;
     static constexpr size_t kSmem = (STORED == 2 ? 1024 : 0) + (size_t)kResident + kStages * 2 * Img<D>::kTileBytes + kStage;
-    static constexpr uint32_t kBuf = 3 * kTile;                          // S^T, dP^T and room: six pieces take 192 columns
-    static constexpr uint32_t kColV = 2 * kBuf, kColK = kColV + 64;
-    static constexpr bool kWide = D == 32;                               // 64 columns per accumulator
-    // w and lse by bulk copy, tiles ahead, or by the workers' loads: those stand between the scores and ds (0.3 us per tile of 1.4, 1.4 in
-    // a block's first at D = 32 with stored probabilities: 100.7 -> 97.8 us at B=32 H=8 S=256), but where the rest of a tile is short
-    // and a block has a tile or two the copy's longer way costs more (D = 32 without them, S = 64: 17.1 against 17.5 us)
-    static constexpr bool kRowsAhead = STORED != 0 || D == 64;
+    static constexpr uint32_t kBuf = 2 * kTile;                          // S^T and dP^T, then the pieces of P^T and ds^T
+    static constexpr uint32_t kColV = 2 * kBuf, kColK = kColV + 128;     // an accumulator per half tile
+    static constexpr bool kWide = D == 32;                               // an accumulator has 64 columns
+    // (a tile's w, maxima and sums come by bulk copy, tiles ahead: the workers' own loads stood between the scores and ds, 0.3 us per tile of
+    // 1.4, 1.4 in a block's first at D = 32 with stored probabilities)
 };
 
 template <int D, bool CAUSAL, int STORED>
 __global__ void __launch_bounds__(kThreads, 1)
-bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *__restrict__ P, float *__restrict__ dK, float *__restrict__ dV,
-                const float *__restrict__ lse_in, const float *__restrict__ w_in, int S, int Spad, int E, int H, int nblk, float c, const __grid_constant__ PMap<STORED> p_map, int expire)
+bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *fac, const float *__restrict__ P, float *__restrict__ dK, float *__restrict__ dV,
+                const float *__restrict__ stat, size_t nstat, int S, int Spad, int E, int H, int nblk, float c, const __grid_constant__ PMap<STORED> p_map, int expire)
 {
     using C = ColsCfg<D, STORED>;
     constexpr int TB = Img<D>::kTileBytes;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *p_s = STORED == 2 ? reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023) : smem_raw;
     uint8_t *k_s = p_s + C::kStage, *v_s = k_s + (STORED ? 0 : 2 * TB), *t_s = v_s + 2 * TB;     // t_s: [stage][Q tile | dO tile]
-    __shared__ __align__(16) float rows_s[C::kStages][2][kTile];         // w and, to form P again, lse of a tile's queries
+    __shared__ __align__(16) float rows_s[C::kStages][STORED ? 1 : 3][kTile];        // w and, to form P again, maximum and 1 / sum of a tile's queries
+    __shared__ float down_s[kDownSlots][2][2][kLanes];                   // a tile's factors: [dV, dK][half][key]
     __shared__ uint64_t res_full, full[C::kStages], w_full[C::kStages], sd_full[2], ready[2], acc_done[2], p_full[STORED == 2 ? kPStages<D> : 1];
     __shared__ uint32_t tmem_base_slot;
     __shared__ volatile int abort_flag;
@@ -588,12 +662,12 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     // No wait for the kernel before yet: the probabilities and the images are older than that one (it waited for the
-    // packing before it let this one start); who reads w and lse waits for it.
+    // packing before it let this one start); who reads the rows' statistics waits for it.
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_base_slot;
-    // site codes: 11 resident operands, 12 tile pair, 14 scores, 15 workers at a tile, 16 accumulation, 17 probabilities, 18 w and lse
+    // site codes: 11 resident operands, 12 tile pair, 14 scores, 15 workers at a tile, 16 accumulation, 17 probabilities, 18 rows' statistics
     bool seen = true;                                // what this thread waited for last has come (for who asks for copies then)
     auto wait = [&](uint64_t *bar, uint32_t parity, int site) {
         const int gone = abort_flag;                 // (before the test, and not in its way)
@@ -653,9 +727,8 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
             if (lane == 0 && i < total && seen) {
                 uint64_t *bar = &w_full[i % C::kStages];
                 const size_t at = (size_t)bh * Spad + (size_t)(t0 + i) * kTile;
-                mbar_arrive_expect_tx(bar, (STORED ? 1 : 2) * kTile * 4);
-                bulk_load(rows_s[i % C::kStages][0], w_in + at, kTile * 4, bar);
-                if (!STORED) bulk_load(rows_s[i % C::kStages][1], lse_in + at, kTile * 4, bar);
+                mbar_arrive_expect_tx(bar, (STORED ? 1 : 3) * kTile * 4);
+                for (int u = 0; u < (STORED ? 1 : 3); ++u) bulk_load(rows_s[i % C::kStages][u], stat + u * nstat + at, kTile * 4, bar);
             }
             __syncwarp();
         };
@@ -671,7 +744,7 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         wait(&res_full, 0, 11);
         tc_fence_after();
         issue_sd(0);
-        if (!first && C::kRowsAhead) {
+        if (!first) {
             dependency_wait();
             for (int i = 0; i < C::kStages; ++i) fetch_w(i);
         }
@@ -685,12 +758,10 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
             wait(&ready[i & 1], (uint32_t)((i >> 1) & 1), 15);
             tc_fence_after();
             if (STORED == 2 && first) fetch_p(i + kPStages<D>);      // the workers have read tile i of the probabilities
-            if (!first && C::kRowsAhead) fetch_w(i + C::kStages);                     // ... and its w and lse
+            if (!first) fetch_w(i + C::kStages);     // ... and its rows' statistics
             const uint32_t s0 = tmem + (uint32_t)(i & 1) * C::kBuf, t = smem_u32(t_s + (i % C::kStages) * 2 * TB);
-            auto p_col = [&](int p, int hf) { return p == 2 ? s0 + kTile + 32 * hf : s0 + 32 * hf + 16 * p; };
-            auto ds_col = [&](int p, int hf) { return p == 0 ? s0 + kTile + 32 * hf + 16 : s0 + 2 * kTile + 32 * hf + 16 * (p - 1); };
-            if (first) issue_accumulate<D, C::kWide, 0, 4>(tmem + C::kColV, p_col, t + TB);
-            else issue_accumulate<D, C::kWide, 0, 4>(tmem + C::kColK, ds_col, t);
+            for (int half = 0; half < 2; ++half)
+                issue_accumulate<D, C::kWide>(tmem + (first ? C::kColV : C::kColK) + 64 * half, s0 + (first ? 0 : kTile) + 32 * half, first ? t + TB : t, half);
             if (elect_one()) tc_commit(&acc_done[i & 1]);
         }
         __syncwarp();
@@ -731,16 +802,25 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
     auto add_dkv = [&](int i) {                      // tile i has been accumulated
         wait_w(&acc_done[i & 1], (uint32_t)((i >> 1) & 1), 16);
         tc_fence_after();
-        add_tile<D, C::kWide>(lane_base + C::kColV, hf, ov);
-        add_tile<D, C::kWide>(lane_base + C::kColK, hf, ok);
+        add_tile<D, C::kWide>(lane_base + C::kColV, hf, down_s[i % kDownSlots][0][0][rloc], down_s[i % kDownSlots][0][1][rloc], ov);
+        add_tile<D, C::kWide>(lane_base + C::kColK, hf, down_s[i % kDownSlots][1][0][rloc], down_s[i % kDownSlots][1][1][rloc], ok);
     };
+    // factors: of this key's K (with the exponent's) and V, and of 32 tiles of Q and dO, one per lane
+    const size_t ntile = (size_t)nbh * (Spad / kTile), tile0 = (size_t)bh * (Spad / kTile);
+    const float k_fac = STORED ? 0.0f : cl2 * fac[ntile + tile0 + key / kTile], v_fac = fac[2 * ntile + tile0 + key / kTile];
+    float q_facs = 0.0f, g_facs = 0.0f;
     if (STORED == 1) fetch_p(0);
-    if (!C::kRowsAhead) dependency_wait();
     for (int i = 0; i < total; ++i) {
-        const uint32_t s_addr = lane_base + (uint32_t)(i & 1) * C::kBuf + hf * 32, dp_addr = s_addr + kTile, room = s_addr + 2 * kTile;
+        const uint32_t s_addr = lane_base + (uint32_t)(i & 1) * C::kBuf + hf * 32, dp_addr = s_addr + kTile;
         const int qb = (t0 + i) * kTile + hf * 32;
-        const size_t at = (size_t)bh * Spad + qb;
-        const float *wrow = C::kRowsAhead ? rows_s[i % C::kStages][0] + hf * 32 : w_in + at, *lrow = C::kRowsAhead ? rows_s[i % C::kStages][1] + hf * 32 : lse_in + at;
+        if ((i & 31) == 0) {
+            const size_t ft = tile0 + min(t0 + i + lane, Spad / kTile - 1);
+            q_facs = fac[ft];
+            g_facs = fac[3 * ntile + ft];
+        }
+        const float q_fac = __shfl_sync(0xffffffffu, q_facs, i & 31), g_fac = __shfl_sync(0xffffffffu, g_facs, i & 31);
+        const float2 s2 = make_float2(k_fac * q_fac, k_fac * q_fac), dp2 = make_float2(v_fac * g_fac, v_fac * g_fac);
+        const float *wrow = rows_s[i % C::kStages][0] + hf * 32;
         const bool mask = CAUSAL && qb < k0 + wq * 32 + 31;              // some lane of the warp has a key after some query
         float p[32], d[32];
         if (STORED == 1) {
@@ -759,14 +839,17 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         if (!STORED) tmem_ld32(s_addr, p);
         tmem_ld32(dp_addr, d);
         tmem_wait_ld();
-        if (C::kRowsAhead) wait_w(&w_full[i % C::kStages], (uint32_t)((i / C::kStages) & 1), 18);
+        wait_w(&w_full[i % C::kStages], (uint32_t)((i / C::kStages) & 1), 18);
         if (!STORED) {
 #pragma unroll
             for (int x = 0; x < 32; x += 4) {
-                const float4 ls = *reinterpret_cast<const float4 *>(lrow + x);       // rows past S: a probability of 0
-                float2 a = ffma2(make_float2(p[x], p[x + 1]), make_float2(cl2, cl2), make_float2(-ls.x, -ls.y));
-                float2 e = ffma2(make_float2(p[x + 2], p[x + 3]), make_float2(cl2, cl2), make_float2(-ls.z, -ls.w));
-                p[x] = ex2_approx(a.x); p[x + 1] = ex2_approx(a.y); p[x + 2] = ex2_approx(e.x); p[x + 3] = ex2_approx(e.y);
+                // (the maximum and 1 / sum apart: the exponent of a probability that counts is then near zero and its rounding small)
+                const float4 mx = *reinterpret_cast<const float4 *>(wrow + kTile + x), ri = *reinterpret_cast<const float4 *>(wrow + 2 * kTile + x);
+                const float2 a = ffma2(make_float2(p[x], p[x + 1]), s2, make_float2(-mx.x, -mx.y));
+                const float2 e = ffma2(make_float2(p[x + 2], p[x + 3]), s2, make_float2(-mx.z, -mx.w));
+                const float2 pa = fmul2(make_float2(ex2_approx(a.x), ex2_approx(a.y)), make_float2(ri.x, ri.y));       // rows past S: 1 / sum is 0
+                const float2 pe = fmul2(make_float2(ex2_approx(e.x), ex2_approx(e.y)), make_float2(ri.z, ri.w));
+                p[x] = pa.x; p[x + 1] = pa.y; p[x + 2] = pe.x; p[x + 3] = pe.y;
             }
         }
         if (mask) {
@@ -776,11 +859,12 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
 #pragma unroll
         for (int x = 0; x < 32; x += 4) {
             const float4 w4 = *reinterpret_cast<const float4 *>(wrow + x);
-            d[x] = p[x] * (d[x] - w4.x); d[x + 1] = p[x + 1] * (d[x + 1] - w4.y);
-            d[x + 2] = p[x + 2] * (d[x + 2] - w4.z); d[x + 3] = p[x + 3] * (d[x + 3] - w4.w);
+            const float2 a = fmul2(make_float2(p[x], p[x + 1]), ffma2(make_float2(d[x], d[x + 1]), dp2, make_float2(-w4.x, -w4.y)));
+            const float2 e = fmul2(make_float2(p[x + 2], p[x + 3]), ffma2(make_float2(d[x + 2], d[x + 3]), dp2, make_float2(-w4.z, -w4.w)));
+            d[x] = a.x; d[x + 1] = a.y; d[x + 2] = e.x; d[x + 3] = e.y;
         }
-        store_pieces(p, s_addr, s_addr + 16, dp_addr);
-        store_pieces(d, dp_addr + 16, room, room + 16);
+        down_s[i % kDownSlots][0][hf][rloc] = store_pieces(p, s_addr) * g_fac;
+        down_s[i % kDownSlots][1][hf][rloc] = store_pieces(d, dp_addr) * q_fac;
         if (i > 0) add_dkv(i - 1);
         tmem_wait_st();
         arrive(&ready[i & 1]);
@@ -789,8 +873,8 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
     // (through the tiles' memory: the last products have read it)
     const int row0 = k0 + wq * 32;
     const size_t dst = ((size_t)b * S + row0) * E + (size_t)h * D;
-    store_out<D>(ov, warp, lane, 1.0f, t_s, dV + dst, E, S - row0, abort_flag);
-    store_out<D>(ok, warp, lane, c, t_s + TB * 2, dK + dst, E, S - row0, abort_flag);
+    store_out<D>(ov, warp, lane, 1.0f, kSumLoss, t_s, dV + dst, E, S - row0, abort_flag);
+    store_out<D>(ok, warp, lane, c, kScoreLoss, t_s + TB * 2, dK + dst, E, S - row0, abort_flag);
     tc_fence_before();
     __syncthreads();
 }
@@ -804,30 +888,31 @@ int launch_cfg(const float *g, const float *q, const float *k, const float *v, c
     auto rows = bwd_rows_kernel<D, CAUSAL, STORED>;
     auto cols = bwd_cols_kernel<D, CAUSAL, STORED>;
     constexpr size_t rows_smem = RowsCfg<D, STORED>::kSmem, cols_smem = ColsCfg<D, STORED>::kSmem;
-    static_assert(rows_smem + (STORED ? 1 : 3) * 2 * kLanes * 4 + 256 <= 232448 && cols_smem + ColsCfg<D, STORED>::kStages * 2 * kTile * 4 + 512 <= 232448, "shared memory of a block");
+    static_assert(rows_smem + ((STORED ? 1 : 3) + kDownSlots) * 2 * kLanes * 4 + 256 <= 232448 &&
+                  cols_smem + ColsCfg<D, STORED>::kStages * (STORED ? 1 : 3) * kTile * 4 + kDownSlots * 4 * kLanes * 4 + 512 <= 232448, "shared memory of a block");
     cudaError_t e = cudaFuncSetAttribute(rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(cols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cols_smem);
     if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     const int nblk = (S + kLanes - 1) / kLanes, Spad = nblk * kLanes;
-    // groups of batches whose images (6 bytes per element) stay in L2 between the kernels that write and read them
-    const size_t per_batch = (size_t)4 * H * Spad * D * 6;
-    long long gb = (long long)((96u << 20) / per_batch);
+    // groups of batches whose images (4 bytes per element) stay in L2 between the kernels that write and read them
+    const size_t per_batch = (size_t)4 * H * Spad * D * 4;
+    long long gb = (long long)((64u << 20) / per_batch);
     gb = gb < 1 ? 1 : gb > B ? B : gb;
-    while (gb > 1 && gb * H * (long long)(Spad / 8) * (D / 32) > 2000000000LL) gb /= 2;
-    const size_t img_bytes = (size_t)gb * H * Spad * D * 6, stat = (size_t)gb * H * Spad;
+    while (gb > 1 && gb * H * (long long)(Spad / kTile) > 2000000000LL) gb /= 2;
+    const size_t img_bytes = (size_t)gb * H * Spad * D * 4, nstat = (size_t)gb * H * Spad;
     StreamWorkspace::Lease ws;
-    int rc = g_bwd_ws.enter(st, 4 * img_bytes + 2 * stat * sizeof(float), &ws);
+    int rc = g_bwd_ws.enter(st, 4 * img_bytes + ((STORED ? 1 : 3) * nstat + 4 * (nstat / kTile)) * sizeof(float), &ws);
     if (rc != HIPGPT_OK) return rc;
     uint8_t *img = ws.get();
-    float *lse = reinterpret_cast<float *>(img + 4 * img_bytes), *w = lse + stat;
+    // beside the images: w and, where P is formed again, maximum and 1 / sum of the rows; the tiles' factors
+    float *stat = reinterpret_cast<float *>(img + 4 * img_bytes), *fac = stat + (STORED ? 1 : 3) * nstat;
     const float c = 1.0f / sqrtf((float)D);
     const int expire = take_expiry(600);
     for (long long b0 = 0; b0 < B; b0 += gb) {
         const int nb = (int)(B - b0 < gb ? B - b0 : gb);
         const size_t off = (size_t)b0 * S * E;
         const float *p = STORED ? probs + (size_t)b0 * H * S * S : nullptr;
-        const int tasks = nb * H * (Spad / 8) * (D / 32);
-        e = launch_overlapped(bwd_pack_kernel<D>, dim3((unsigned)((tasks + 7) / 8), 4), dim3(256), 0, st, q + off, k + off, v + off, g + off, img, img_bytes, S, Spad, E, H, tasks);
+        e = launch_overlapped(bwd_pack_kernel<D>, dim3((unsigned)(nb * H * (Spad / kTile)), 4), dim3(256), 0, st, q + off, k + off, v + off, g + off, img, img_bytes, fac, S, Spad / kTile, E, H);
         if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "bwd_pack_kernel launch: %s", cudaGetErrorString(e));
         PMap<STORED> rows_map = {}, cols_map = {};
         if constexpr (STORED == 2) {
@@ -836,10 +921,10 @@ int launch_cfg(const float *g, const float *q, const float *k, const float *v, c
             if (rc != HIPGPT_OK) return rc;
         }
         const dim3 grid((unsigned)(nb * H * nblk));
-        e = launch_overlapped(rows, grid, dim3(kThreads), rows_smem, st, (const uint8_t *)img, img_bytes, p, dq + off, lse, w, S, Spad, E, H, nblk, c, rows_map, (expire & 255) <= 10 ? expire : 0);
+        e = launch_overlapped(rows, grid, dim3(kThreads), rows_smem, st, (const uint8_t *)img, img_bytes, (const float *)fac, p, dq + off, stat, nstat, S, Spad, E, H, nblk, c, rows_map, (expire & 255) <= 10 ? expire : 0);
         if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "bwd_rows_kernel launch: %s", cudaGetErrorString(e));
-        e = launch_overlapped(cols, grid, dim3(kThreads), cols_smem, st, (const uint8_t *)img, img_bytes, p, dk + off, dv + off, (const float *)lse,
-                              (const float *)w, S, Spad, E, H, nblk, c, cols_map, (expire & 255) > 10 ? expire : 0);
+        e = launch_overlapped(cols, grid, dim3(kThreads), cols_smem, st, (const uint8_t *)img, img_bytes, (const float *)fac, p, dk + off, dv + off, (const float *)stat, nstat,
+                              S, Spad, E, H, nblk, c, cols_map, (expire & 255) > 10 ? expire : 0);
         if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "bwd_cols_kernel launch: %s", cudaGetErrorString(e));
     }
     return HIPGPT_OK;

@@ -299,6 +299,12 @@ __device__ __forceinline__ float2 fadd2(float2 a, float2 b)
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(*reinterpret_cast<const uint64_t *>(&a)), "l"(*reinterpret_cast<const uint64_t *>(&b)));
     return *reinterpret_cast<float2 *>(&d);
 }
+__device__ __forceinline__ float2 fmul2(float2 a, float2 b)
+{
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(*reinterpret_cast<const uint64_t *>(&a)), "l"(*reinterpret_cast<const uint64_t *>(&b)));
+    return *reinterpret_cast<float2 *>(&d);
+}
 __device__ __forceinline__ float max3(float a, float b, float c)
 {
     float r;

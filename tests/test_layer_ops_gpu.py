@@ -354,6 +354,39 @@ def test_attention_backward_of_any_magnitude_and_captured_into_a_graph():
         assert np.array_equal(dout.cpu().numpy().reshape(3, -1), got)
 
 
+@pytest.mark.parametrize("D,S", [(32, 130), (64, 97)])
+@pytest.mark.parametrize("stored", [False, True])
+def test_attention_backward_tiles_of_their_own_scale(D, S, stored):
+    """The operands are cut relative to the largest magnitude of a 64-row tile: tiles of zeros, tiles 2^40 apart, and an infinity, which stays
+    in its own row of dQ and leaves the tile's other rows their bits."""
+    B, H = 1, 2
+    E = H * D
+    qkv = synth.qkv_planes(850 + S, B, S, E).reshape(3, S, E)
+    g = synth.normal(851 + S, (S, E))
+    zero = np.zeros_like(qkv)
+    p_of = lambda x, causal: ob.mha(x, B, S, E, H, causal=causal, want_probs=True)[1] if stored else None
+    got = _run_backward(g, zero, p_of(zero, True), B, S, E, H, True)
+    want = ob.mha_backward(g, zero, p_of(zero, True), B, S, E, H, causal=True, fma=True)
+    assert float(np.abs(got - want).max()) <= 4e-6 * max(1.0, float(np.abs(want).max()))
+    # the second tile's V and dO 2^-40 of the first's: dP's own factor per pair of tiles, and dQ, dK of each tile to its own scale
+    qkv[2, 64:] *= np.float32(2.0 ** -40)
+    g[64:] *= np.float32(2.0 ** -40)
+    probs = p_of(qkv, True)
+    got = _run_backward(g, qkv, probs, B, S, E, H, True).reshape(3, S, E)
+    want = ob.mha_backward(g, qkv, probs, B, S, E, H, causal=True, fma=True).reshape(3, S, E)
+    for part in (slice(0, 64), slice(64, S)):
+        for plane in range(3):
+            w = want[plane, part]
+            assert float(np.abs(got[plane, part] - w).max()) <= 1e-5 * float(np.abs(w).max())
+    bad = g.copy()
+    bad[5, 3] = np.inf                                     # a row of the first tile, in head 0
+    hit = _run_backward(bad, qkv, probs, B, S, E, H, True).reshape(3, S, E)
+    same = np.ones(S, bool)
+    same[5] = False
+    assert not np.isfinite(hit[0, 5, :D]).any()
+    assert np.array_equal(hit[0, same], got[0, same]) and np.array_equal(hit[:, :, D:], got[:, :, D:])
+
+
 def test_attention_backward_reference_named_launcher():
     raw = C.CDLL(_capi.lib_path())
     fn = getattr(raw, _capi.CXX_LAUNCHERS["launch_multihead_attention_backward"])
