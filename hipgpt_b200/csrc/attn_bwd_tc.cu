@@ -322,7 +322,7 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         for (int i = 0; i < C::kKStages; ++i) mbar_init(&k_full[i], 1);
         for (int i = 0; i < C::kVStages; ++i) mbar_init(&v_full[i], 1);
         if (STORED == 2) for (int i = 0; i < kPStages<D>; ++i) mbar_init(&p_full[i], 1);
-        for (int i = 0; i < 2; ++i) { mbar_init(&sd_full[i], STORED ? 1 : 2); mbar_init(&ready[i], kWorkerWarps); mbar_init(&acc_done[i], 2); }      // (commits: one per issuing warp)
+        for (int i = 0; i < 2; ++i) { mbar_init(&sd_full[i], 2); mbar_init(&ready[i], kWorkerWarps); mbar_init(&acc_done[i], 2); }      // (commits: one per issuing warp)
     }
     if (warp == kWorkerWarps) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)), "r"(kTmemCols) : "memory");
@@ -400,8 +400,15 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         }
         auto issue_sd = [&](int i) {
             const uint32_t d = tmem + (uint32_t)((i & 1) * 2 * kTile);
+            if (first && STORED) {
+                // No product of its own, but the workers wait for this warp's word all the same: it must not fall two tiles behind them in
+                // the first sweep, where a ring of three tiles of probabilities would let them.  The phase of `ready` that it
+                // looks for would then have come and gone twice, for the tile after too, and it would wait for a third that needs its next copy.
+                if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&sd_full[i & 1])) : "memory");
+                __syncwarp();
+                return;
+            }
             if (first) {
-                if (STORED) return;
                 wait(&k_full[k_slot(i)], k_phase(i), 2);
                 tc_fence_after();
                 issue_scores<D>(d, smem_u32(q_s), smem_u32(k_s + k_slot(i) * TB));

@@ -333,6 +333,21 @@ def test_attention_backward_ring_of_stored_probabilities(shape, causal):
     assert float(np.abs(got - want).max()) <= 4e-6 * max(1.0, float(np.abs(want).max()))
 
 
+def test_attention_backward_ring_of_stored_probabilities_many_times():
+    """head_dim 32: the workers may be three tiles of probabilities ahead of the warp that fetches them.  It once could miss that a
+    tile had been read, now and then, and the block gave up after a second."""
+    B, H, S, D = 4, 8, 388, 32
+    E = H * D
+    qkv, g = torch.randn(3, B * S, E, device="cuda"), torch.randn(B * S, E, device="cuda")
+    p, out, grad = torch.empty(B, H, S, S, device="cuda"), torch.empty(B * S, E, device="cuda"), torch.empty(3, B * S, E, device="cuda")
+    _capi.check(_capi.lib().hipgpt_mha_forward_planes(qkv.data_ptr(), out.data_ptr(), p.data_ptr(), B, S, E, H, 0, _st()))
+    for _ in range(4000):
+        _capi.check(_capi.lib().hipgpt_mha_backward_planes(g.data_ptr(), qkv.data_ptr(), p.data_ptr(), grad.data_ptr(), B, S, E, H, 0, _st()))
+    st = C.c_int(-1)
+    _capi.check(_capi.lib().hipgpt_kernel_status(C.byref(st)))
+    assert st.value == 0
+
+
 def test_attention_backward_of_any_magnitude_and_captured_into_a_graph():
     B, H, S, D = 2, 2, 96, 64
     E = H * D
