@@ -31,19 +31,16 @@
 // issue side by side.  Two score buffers in TMEM: the products of tile i + 1 run while the workers are at tile i.  Every wait is bounded: on expiry the
 // block raises a flag that cuts later waits short, records a status code, skips its stores, lets what is on its way land, frees its
 // TMEM and returns.
+#include "attn_bwd_pieces.cuh"
 #include "stream_workspace.hpp"
-#include "tc_primitives.cuh"
 #include "tma_host.cuh"
 
-#include <cuda_fp16.h>
 #include <math.h>
 #include <type_traits>
 
 namespace hipgpt {
 namespace {
 
-constexpr int kLanes = 128;            // rows (or keys) per block = TMEM lanes
-constexpr int kTile = 64;              // columns per tile
 constexpr int kWorkerWarps = 8;
 constexpr int kThreads = kWorkerWarps * 32 + 64;
 constexpr uint32_t kTmemCols = 512;
@@ -58,31 +55,6 @@ __device__ __noinline__ bool bwd_wait_slow(uint64_t *bar, uint32_t parity, int s
     linger();
     return false;
 }
-
-// Sizes of an operand image, in bytes.
-template <int D>
-struct Img {
-    static constexpr int kPiece = (D / 8) * 128;     // one piece of an 8-row block
-    static constexpr int kBlock = 2 * kPiece;        // an 8-row block
-    static constexpr int kTileBytes = (kTile / 8) * kBlock;     // 64 rows
-};
-
-// Two fp32 numbers below 2^16 -> two words of two fp16 each whose sums are the numbers (to 2^-23 of them, 2^-25 where that is more).
-// An infinity leaves a NaN.
-__device__ __forceinline__ void cut2(float2 x, uint32_t &h, uint32_t &l)
-{
-    const __half2 hh = __float22half2_rn(x);
-    const float2 back = __half22float2(hh);
-    const __half2 ll = __float22half2_rn(fadd2(x, make_float2(-back.x, -back.y)));
-    h = *reinterpret_cast<const uint32_t *>(&hh);
-    l = *reinterpret_cast<const uint32_t *>(&ll);
-}
-
-// The power of two that brings a largest magnitude into [2^14, 2^15), and one over it, from the magnitude's bits.  Magnitudes
-// below 2^-100 are treated as that; an infinite one leaves both normal numbers.
-__device__ __forceinline__ uint32_t range_exponent(uint32_t bits) { return max(bits & 0x7f800000u, 27u << 23); }
-__device__ __forceinline__ float range_up(uint32_t e) { return __uint_as_float((268u << 23) - e); }
-__device__ __forceinline__ float range_down(uint32_t e) { return __uint_as_float(e - (14u << 23)); }
 
 // ---- the pieces of the four planes ---------------------------------------------------------------------
 // A block takes a 64-row tile of a head in one plane, a warp 8 of its rows: lane = (column block of 8) * 8 + row, so that it reads 8 whole lines and
@@ -954,6 +926,7 @@ bool mha_backward_tc_supports(const void *g, const void *q, const void *k, const
 int launch_mha_backward_tc(const float *g, const float *q, const float *k, const float *v, const float *probs, float *dq, float *dk, float *dv,
                            int B, int S, int E, int H, int causal, cudaStream_t st)
 {
+    if (mha_backward_head_supports(E / H, S)) return launch_mha_backward_head(g, q, k, v, probs, dq, dk, dv, B, S, E, H, causal, st);
     // probabilities whose rows TMA can address (the pointer is 16-byte aligned)
     const int stored = !probs ? 0 : (S & 3) == 0 && tma_encode_fn() != nullptr ? 2 : 1;
     auto go = [&](auto launch) { return launch(g, q, k, v, probs, dq, dk, dv, B, S, E, H, st); };

@@ -154,6 +154,11 @@ bool mha_backward_tc_supports(const void *g, const void *q, const void *k, const
 int launch_mha_backward_tc(const float *g, const float *q, const float *k, const float *v, const float *probs, float *dq, float *dk, float *dv,
                            int B, int S, int E, int H, int causal, cudaStream_t st);
 int mha_backward_tc_status_fetch(int *status);
+// a head whose operands fit shared memory, in one launch (attn_bwd_head.cu; the tensor pipe's conditions hold)
+bool mha_backward_head_supports(int D, int S);
+int launch_mha_backward_head(const float *g, const float *q, const float *k, const float *v, const float *probs, float *dq, float *dk, float *dv,
+                             int B, int S, int E, int H, int causal, cudaStream_t st);
+int mha_backward_head_status_fetch(int *status);
 void mha_backward_tc_release();
 // the launchers either side of attention (layer_ops.cu)
 int launch_matmul_exact(const float *A, const float *B, const float *bias, float *C, int M, int N, int K, cudaStream_t st);

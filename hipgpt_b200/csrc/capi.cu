@@ -162,6 +162,7 @@ static int fetch_status_words(int *status)
     int pr = 0, gm = 0, bw = 0;
     if (rc == HIPGPT_OK) rc = probe_status_fetch(&pr);
     if (rc == HIPGPT_OK) rc = mha_backward_tc_status_fetch(&bw);
+    if (rc == HIPGPT_OK && !bw) rc = mha_backward_head_status_fetch(&bw);
     if (rc == HIPGPT_OK) rc = gemm_tc_status_fetch(&gm);
     if (rc != HIPGPT_OK) return rc;
     *status = a ? a : (b ? 100 + b : (d ? 300 + d : (h ? 400 + h : (gm ? 500 + gm : (bw ? 600 + bw : (pr ? 900 + pr : 0))))));

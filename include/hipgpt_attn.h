@@ -401,7 +401,7 @@ HIPGPT_API int hipgpt_set_full_range(int on);
  *       arrives, with a limit of `limit_cycles` SM cycles (at most 2^24, a few milliseconds).  Afterwards
  *       hipgpt_kernel_status() reports 907 and d_canary[0..n) is untouched.
  *   hipgpt_debug_expire_wait  in the calling thread's next call of a tensor-core projection (code 501 ... 504) or of a tensor-core
- *       backward (601 ... 618) the wait that hipgpt_kernel_status reports with this code runs out at once in block `block` of
+ *       backward (601 ... 627) the wait that hipgpt_kernel_status reports with this code runs out at once in block `block` of
  *       each of the call's launches that has it, if it has to wait at all.
  *   hipgpt_gpt_debug_stall_barrier  makes the NEXT hipgpt_gpt_generate call give up: in the persistent mode it starts with a
  *       grid-barrier counter that cannot complete, and every block gives up at its first barrier; by clusters the first block's

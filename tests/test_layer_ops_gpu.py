@@ -333,6 +333,29 @@ def test_attention_backward_ring_of_stored_probabilities(shape, causal):
     assert float(np.abs(got - want).max()) <= 4e-6 * max(1.0, float(np.abs(want).max()))
 
 
+@pytest.mark.parametrize("B,H,S,D", [(1, 1, 1, 32), (2, 3, 3, 32), (1, 2, 66, 32), (3, 2, 191, 32), (1, 3, 192, 32), (2, 2, 255, 32), (40, 4, 256, 32), (1, 2, 1, 64), (2, 2, 68, 64), (160, 1, 127, 64)])
+@pytest.mark.parametrize("causal,stored", [(False, True), (True, True), (True, False), (False, False)])
+def test_attention_backward_of_a_whole_head(B, H, S, D, causal, stored):
+    """One block or a cluster of two per head: tiles of 64 keys and blocks of 128 rows that end inside, probabilities with and without 16-byte rows, more
+    blocks than SMs; planes on 16-byte boundaries that are not 32-byte ones give the same bits."""
+    E = H * D
+    qkv, g = synth.qkv_planes(870 + S + D, B, S, E), synth.normal(871 + S, (B * S, E))
+    probs = ob.mha(qkv, B, S, E, H, causal=causal, want_probs=True)[1] if stored else None
+    want = ob.mha_backward(g, qkv, probs, B, S, E, H, causal=causal, fma=True)
+    got = _run_backward(g, qkv, probs, B, S, E, H, causal, planes=True)
+    assert float(np.abs(got - want).max()) <= 4e-6 * max(1.0, float(np.abs(want).max()))
+    buf = torch.empty(4 + 3 * B * S * E, device="cuda")
+    shifted = buf[4:]
+    shifted.copy_(torch.from_numpy(np.ascontiguousarray(qkv).reshape(-1)))
+    dg, dp, dout = dev(g), dev(probs) if stored else None, torch.full((3 * B * S * E,), float("nan"), device="cuda")
+    _capi.check(_capi.lib().hipgpt_mha_backward_planes(dg.data_ptr(), shifted.data_ptr(), dp.data_ptr() if stored else None, dout.data_ptr(), B, S, E, H, int(causal), _st()))
+    torch.cuda.synchronize()
+    assert np.array_equal(dout.cpu().numpy().reshape(-1), got.reshape(-1))
+    st = C.c_int(-1)
+    _capi.check(_capi.lib().hipgpt_kernel_status(C.byref(st)))
+    assert st.value == 0
+
+
 def test_attention_backward_ring_of_stored_probabilities_many_times():
     """head_dim 32: the workers may be three tiles of probabilities ahead of the warp that fetches them.  It once could miss that a
     tile had been read, now and then, and the block gave up after a second."""

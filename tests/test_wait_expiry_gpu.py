@@ -183,3 +183,31 @@ def test_an_expired_wait_of_a_split_product_leaves_the_whole_tile_out(code, bloc
             assert torch.equal(got[piece], want[piece]), t
     run()
     assert torch.equal(out, want) and _status() == 0
+
+
+@pytest.mark.parametrize("D,S", [(32, 200), (64, 100)])
+@pytest.mark.parametrize("stored,code", [(s, c) for s in (True, False) for c in (621, 623, 624, 625, 626) if not s or c != 623])
+def test_an_expired_wait_of_a_whole_head_stores_none_of_its_rows(D, S, stored, code):
+    """The last block of the first head: nothing of its rows is stored, the other block of the head stores what does not depend on it or nothing, and the
+    other heads are as ever.  (Stored probabilities, 622, and g V^T, 623 with them, are there before they are waited for.)"""
+    B, H = 2, 2
+    E, block = H * D, 1 if S > 128 else 0
+    gen = torch.Generator(device="cuda").manual_seed(6)
+    qkv, g = torch.randn(3, B * S, E, generator=gen, device="cuda"), torch.randn(B * S, E, generator=gen, device="cuda")
+    p, grad, st = torch.empty(B, H, S, S, device="cuda"), torch.empty(3, B * S, E, device="cuda"), torch.cuda.current_stream().cuda_stream
+    _capi.check(_capi.lib().hipgpt_mha_forward_planes(qkv.data_ptr(), grad.data_ptr(), p.data_ptr(), B, S, E, H, 0, st))
+    run = lambda: _capi.check(_capi.lib().hipgpt_mha_backward_planes(g.data_ptr(), qkv.data_ptr(), p.data_ptr() if stored else None, grad.data_ptr(), B, S, E, H, 0, st))   # noqa: E731
+    run()
+    want = grad.clone()
+    got, = _expired(code, block, run, grad)
+    got, want4 = got.view(3, B, S, H, D), want.view(3, B, S, H, D)
+    mine = slice(128 * block, S)
+    assert bool((got[:, 0, mine, 0] == -7.0).all())
+    if block:
+        assert torch.equal(got[0, 0, :128, 0], want4[0, 0, :128, 0])         # dQ needs nothing of the other block
+        for i in (1, 2):
+            part = got[i, 0, :128, 0]
+            assert torch.equal(part, want4[i, 0, :128, 0]) or bool((part == -7.0).all())
+    assert torch.equal(got[:, :, :, 1], want4[:, :, :, 1]) and torch.equal(got[:, 1], want4[:, 1])
+    run()
+    assert torch.equal(grad, want) and _status() == 0
