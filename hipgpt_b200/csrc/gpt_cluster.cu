@@ -16,7 +16,7 @@
 //     bulk copies that run up to a layer ahead of the arithmetic; they do not depend on activations, so nothing waits for them.
 //   * Warp s owns segment s of the inner dimension (lanes: columns), so a layer norm needs no barrier either: every warp forms
 //     the row's statistics and normalises the part that it multiplies.
-//   * Keys and values of older positions are asked for before the projection of the new one is formed.
+//   * Keys and values of older positions are asked for while the projection of the new one is on its way between the blocks.
 //   * The logits are formed where an id is picked from them: not at prompt positions before the last.
 // Buffers are received into once per layer (or step); a sender can be at most one product ahead of the slowest receiver, because
 // each product needs the columns of all blocks, so a buffer is never overwritten while it is read.
@@ -25,8 +25,11 @@
 // out too, and all meet at the barriers of the remaining steps and leave.  (A barrier whose phase has not been seen complete is not
 // opened again, and the bytes that nobody waits for stay within eight layers' worth, at most 90 KB each: an mbarrier counts 2^20.)
 //
-// Measured at the default model (E=256 L=8 H=8 V=5000), batch 8: 72 us per step (the replayed graph: 184), batch 1: 66 (175).  A
-// step is 42 products of 400 - 450 ns each, attention a third of a layer.  Sizes are template parameters because the chain is
+// Measured at the default model (E=256 L=8 H=8 V=5000), batch 8: 66 us per step (the replayed graph: 184), batch 3: 59.  A layer of
+// 8 us: the hops (450 - 700 ns from the last store to the first read, five of them), attention 1.2, the two layer norms 0.35 each, a product's
+// multiply-adds 0.15 - 0.5.  Besides, the shared memory's width is in the chain wherever all warps read at once (192 KB of weights are 1536 cycles of a
+// layer): sums column by column, weights that no two lanes read twice and QKV's weights asked for before their activations took a step from 72 to 66 us
+// (B=7 E=192 L=5, 67 positions and more: 5268 -> 4723 us a request).  Sizes are template parameters because the chain is
 // bound by the instructions of single warps: with sizes read from the plan a step took 143 us.
 #include "gpt_cluster.cuh"
 #include "tc_primitives.cuh"
@@ -230,36 +233,41 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) q = __fadd_rn(q, __shfl_xor_sync(0xffffffffu, q, o));
         const float var = (E & (E - 1)) == 0 ? __fmul_rn(q, 1.0f / E) : __fdiv_rn(q, (float)E);
-        return make_float2(mean, __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(var, 1e-5f))));
+        return make_float2(mean, __frcp_rn(__fsqrt_rn(__fadd_rn(var, 1e-5f))));
     };
 
-    auto add4 = [](float4 x, float4 y) { return make_float4(__fadd_rn(x.x, y.x), __fadd_rn(x.y, y.y), __fadd_rn(x.z, y.z), __fadd_rn(x.w, y.w)); };
     // One product's multiply-adds: this warp's segment of the inner dimension, all columns of the part.  The activations: rows at
     // `src` in shared memory, normalised first where the job says so; kJobO takes this warp's own segment.  Leaves the partial sums
     // in part + flip * part_stride and ends with a barrier of the block.  Lanes: up to 16 columns: (column, row of a pair); more:
-    // columns lane, lane + 32, all rows.  Returns the part's bias for the columns that this thread finishes.
+    // columns lane, lane + 32, all rows.  kPaired (the long product of few columns): eight of the warps take two segments each, a half of the lanes a segment
+    // and all its rows, so that a warp reads each weight once; as (column, row) its weights were read once per row, the 1000 cycles that the product took
+    // to begin.  Returns the part's bias for the column that this thread finishes.
     // `arrival` waits for the activations.  Before it the weights of this lane go to registers (where there are at most 64): they
-    // have been in the ring for long, and reading them takes the shared memory's return path about as long as a hop takes.
+    // have been in the ring for long, and reading them takes the shared memory's return path about as long as a hop takes.  (With two rows the
+    // other warps wait with that until the sums before have been read: bar 9 in `finish`, 8874 -> 8779 us a request; with one row it costs as much.)
     auto product = [&](auto jn, const float *src, auto arrival) {
         constexpr int J = decltype(jn)::value;
         constexpr ClusterJob jb = cluster_job_of(J, E, 64 * 64);          // (the output projection's cut depends on V in its parts only)
         constexpr int pw = jb.width, klen = jb.klen, klp = jb.klp, sh = jb.seg_shift, nch = jb.chunks();
         constexpr int stride = J == kJobF2 ? C::fs : C::es;
-        int slot = slot0 + (warp >> sh);
+        constexpr bool kPaired = J == kJobF2 && pw <= 16 && klp <= 64;
+        static_assert(!kPaired || (sh >= 1 && (klen & 3) == 0), "two segments lie in one chunk, rows of activations are read in place");
+        const int seg = kPaired ? 2 * (warp & 7) + (lane >> 4) : warp;
+        int slot = slot0 + ((kPaired ? 2 * (warp & 7) : warp) >> sh);
         uint32_t par = slot_par;
         if (slot >= lay.slots) { slot -= lay.slots; par ^= 1u; }
         const float *chunk = reinterpret_cast<const float *>(ring + slot * C::kSlot);
-        const int in_chunk = warp & ((1 << sh) - 1);
+        const int in_chunk = seg & ((1 << sh) - 1);
         const float4 *w4 = reinterpret_cast<const float4 *>(chunk + in_chunk * (klp * pw));
         const float *as = aw;
         constexpr bool kOwn = jb.ln || J == kJobO || (klen & 3) != 0;     // the activations are (copied) in this warp's own segment
         constexpr int astride = kOwn ? C::seg : stride;
         constexpr int NC = pw <= 16 ? 1 : (pw + 31) / 32;                // columns per lane
-        constexpr bool kEarly = J != kJobQkv && J != kJobVoc && NC * klp <= 64;
+        constexpr bool kEarly = J != kJobVoc && NC * klp <= 64;
         const int wc0 = pw <= 16 ? (pw < 16 ? min(lane & 15, pw - 1) : lane & 15) : (pw < 32 ? min(lane, pw - 1) : lane);
         const float4 *wp = w4 + wc0, *wq = w4 + (pw < 64 ? min(lane + 32, pw - 1) : lane + 32);
         float4 held[kEarly ? NC * klp / 4 : 1];
-        if constexpr (kEarly) {
+        if constexpr (kEarly && !kPaired) {
             wait(&full[slot], par);
 #pragma unroll
             for (int k = 0; k < klp / 4; ++k) {
@@ -267,7 +275,7 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
                 if constexpr (NC > 1) held[NC * k + 1] = wq[k * pw];
             }
         }
-        arrival();
+        if constexpr (!kPaired) arrival();
         float2 own = make_float2(0.f, 0.f);
         if constexpr (jb.ln != 0 && R == 1) own = row_stats(src);
         if constexpr (jb.ln != 0 && R > 1) {
@@ -277,7 +285,7 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
             }
             __syncthreads();
         }
-        if constexpr (!kEarly) wait(&full[slot], par);
+        if constexpr (!kEarly && !kPaired) wait(&full[slot], par);
         if constexpr (jb.ln != 0) {
             const float *gm = chunk + jb.weight_floats() + in_chunk * klp, *bt = gm + (klp << sh);
 #pragma unroll
@@ -297,10 +305,37 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
             }
             __syncwarp();
         } else if constexpr (!kOwn) {
-            as = src + warp * klen;
+            as = src + seg * klen;
         }
-        float *dst = part + flip * C::part_stride + warp * pw;
-        if constexpr (pw <= 16) {
+        float *dst = part + flip * C::part_stride + seg * pw;
+        if constexpr (kPaired) {
+            if (warp >= 8) {
+                float4 w[klp / 4];
+                wait(&full[slot], par);
+#pragma unroll
+                for (int k = 0; k < klp / 4; ++k) w[k] = wp[k * pw];
+                arrival();
+                float acc[R];
+#pragma unroll
+                for (int r = 0; r < R; ++r) acc[r] = 0.0f;
+#pragma unroll
+                for (int k = 0; k < klp / 4; ++k) {
+#pragma unroll
+                    for (int r = 0; r < R; ++r) {
+                        const float4 x = *reinterpret_cast<const float4 *>(as + r * astride + 4 * k);
+                        acc[r] = fmaf(x.x, w[k].x, acc[r]);
+                        acc[r] = fmaf(x.y, w[k].y, acc[r]);
+                        acc[r] = fmaf(x.z, w[k].z, acc[r]);
+                        acc[r] = fmaf(x.w, w[k].w, acc[r]);
+                    }
+                }
+                if ((lane & 15) < pw)
+#pragma unroll
+                    for (int r = 0; r < R; ++r) dst[r * 16 * pw + (lane & 15)] = acc[r];
+            } else {
+                arrival();
+            }
+        } else if constexpr (pw <= 16) {
             constexpr int RH = (R + 1) / 2;          // rows of a lane: r0, r0 + 2
             const int c = lane & 15, r0 = R > 1 ? lane >> 4 : 0;
             float acc[RH];
@@ -351,12 +386,12 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
                 for (int n = 0; n < NC; ++n)
                     if (32 * (n + 1) <= pw || lane + 32 * n < pw) dst[r * 16 * pw + lane + 32 * n] = acc[n][r];
         }
-        float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
+        float bias = 0.0f;
         if constexpr (J != kJobVoc) {
             // the first chunk has landed: warp 0 waited for it; another warp may not have, and asks again
             if (tid < pw * R) {
                 wait(&full[slot0], slot_par);
-                bias = *reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(ring + slot0 * C::kSlot) + jb.weight_floats() + jb.ln_floats() + 4 * (tid / (4 * R)));
+                bias = (reinterpret_cast<const float *>(ring + slot0 * C::kSlot) + jb.weight_floats() + jb.ln_floats())[R == 1 ? tid : tid % pw];
             }
         }
         __syncthreads();                             // the partial sums are there; the chunks may be overwritten
@@ -365,34 +400,46 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
         if (slot0 >= lay.slots) { slot0 -= lay.slots; slot_par ^= 1u; }
         return bias;
     };
-    // Finishes part `pt` of a product: a thread adds up four columns of a row (partial sums in ascending order) and stores them
-    // into four of the sixteen blocks; the threads of the other receivers form the same sums, which is cheaper than handing them over.
-    auto finish = [&](auto jn, int pt, float4 bias, int layer, int p) {
+    // Finishes part `pt` of a product: a thread adds up a column of a row (partial sums in ascending order; a warp reads whole lines: as four
+    // columns per thread, with a thread per four receivers, each line was read four times, and that traffic stood in the chain); four neighbours
+    // then exchange theirs and each stores all four columns into four of the sixteen blocks.
+    auto finish = [&](auto jn, int pt, float bias, int layer, int p) {
         constexpr int J = decltype(jn)::value;
         constexpr ClusterJob jb = cluster_job_of(J, E, 64 * 64);
         constexpr int pw = jb.width, stride = J == kJobQkv ? C::qs : J == kJobF1 ? C::fs : C::es;
         constexpr int buf = J == kJobQkv ? C::qkv : J == kJobO ? C::xa : J == kJobF1 ? C::ff : C::xb;
         constexpr int res = J == kJobO ? C::xb : C::xa;
         constexpr int h = J == kJobQkv ? kQkv : J == kJobO ? kXa : J == kJobF1 ? kFf : kXb;
-        const int r = (tid >> 2) & (R - 1), g = tid / (4 * R), n = rank * jb.nc + pt * pw + 4 * g;
-        // the block's last columns may lie past its share (the last part) or past the matrix
-        if (g < pw / 4 && r < rows && pt * pw + 4 * g < jb.nc && n < jb.n) {
-            const float *ps = part + flip * C::part_stride + r * 16 * pw + 4 * g;
-            float4 v = *reinterpret_cast<const float4 *>(ps);
+        if (warp * 32 < pw * R) {                    // (whole warps)
+            const int r = R == 1 ? 0 : tid / pw, c = tid - r * pw, n = rank * jb.nc + pt * pw + c;
+            // the block's last columns may lie past its share (the last part) or past the matrix: four at a time
+            const bool mine = tid < pw * R && r < rows && pt * pw + c < jb.nc && n < jb.n;
+            float v = 0.0f;
+            if (mine) {
+                const float *ps = part + flip * C::part_stride + r * 16 * pw + c;
+                v = ps[0];
 #pragma unroll
-            for (int s = 1; s < 16; ++s) v = add4(v, *reinterpret_cast<const float4 *>(ps + s * pw));
-            v = add4(v, bias);
-            if constexpr (J == kJobF1) v = make_float4(fmaxf(0.0f, v.x), fmaxf(0.0f, v.y), fmaxf(0.0f, v.z), fmaxf(0.0f, v.w));
-            if constexpr (J == kJobO || J == kJobF2) v = add4(*reinterpret_cast<const float4 *>(sm + res + r * stride + n), v);
-            const uint32_t to = smem_u32(sm + buf + r * stride + n), bar = smem_u32(&hop[h]);
+                for (int s = 1; s < 16; ++s) v = __fadd_rn(v, ps[s * pw]);
+                v = __fadd_rn(v, bias);
+                if constexpr (J == kJobF1) v = fmaxf(0.0f, v);
+                if constexpr (J == kJobO || J == kJobF2) v = __fadd_rn(sm[res + r * stride + n], v);
+            }
+            if constexpr (R > 1) asm volatile("bar.arrive 9, 512;" ::: "memory");
+            const float4 four = make_float4(__shfl_sync(0xffffffffu, v, 0, 4), __shfl_sync(0xffffffffu, v, 1, 4), __shfl_sync(0xffffffffu, v, 2, 4), __shfl_sync(0xffffffffu, v, 3, 4));
+            if (mine) {
+                const int n0 = n & ~3;               // (shares and parts are whole fours)
+                const uint32_t to = smem_u32(sm + buf + r * stride + n0), bar = smem_u32(&hop[h]);
 #pragma unroll
-            for (int d = 0; d < 4; ++d) send4(to + peer[d], bar + peer[d], v);
-            if constexpr (J == kJobQkv) {
-                if (dq == (rank >> 2) && n >= E) {   // keys and values, for the later positions
-                    float *cache = (n < 2 * E ? a.kc : a.vc) + (size_t)layer * a.layer_stride + ((size_t)(row0 + r) * a.S + p) * E;
-                    *reinterpret_cast<float4 *>(cache + (n < 2 * E ? n - E : n - 2 * E)) = v;
+                for (int d = 0; d < 4; ++d) send4(to + peer[d], bar + peer[d], four);
+                if constexpr (J == kJobQkv) {
+                    if (dq == (rank >> 2) && n0 >= E) {          // keys and values, for the later positions
+                        float *cache = (n0 < 2 * E ? a.kc : a.vc) + (size_t)layer * a.layer_stride + ((size_t)(row0 + r) * a.S + p) * E;
+                        *reinterpret_cast<float4 *>(cache + (n0 < 2 * E ? n0 - E : n0 - 2 * E)) = four;
+                    }
                 }
             }
+        } else if constexpr (R > 1) {
+            asm volatile("bar.sync 9, 512;" ::: "memory");
         }
         flip ^= 1;
     };
@@ -541,20 +588,21 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
                 const int h = e / D, d = e % D;
                 const float *rc = rec + (r * H + h) * ns * rstride;
                 float M = -1e30f, Lsum = 0.0f, acc = 0.0f;
-                if (ns <= 8) {                       // all loads in flight at once
+                if (ns <= 8) {
+                    // all loads in flight at once; a split that is not there counts as one without keys (which adds zeros), so nothing branches
                     float2 ml[8];
                     float os[8];
 #pragma unroll
                     for (int s = 0; s < 8; ++s) {
-                        if (s >= ns) break;
-                        ml[s] = *reinterpret_cast<const float2 *>(rc + s * rstride + D);
-                        os[s] = rc[s * rstride + d];
+                        const float *at = rc + (s < ns ? s : 0) * rstride;
+                        ml[s] = *reinterpret_cast<const float2 *>(at + D);
+                        os[s] = at[d];
+                        if (s >= ns) { ml[s] = make_float2(-INFINITY, 0.0f); os[s] = 0.0f; }
                     }
 #pragma unroll
-                    for (int s = 0; s < 8; ++s) { if (s >= ns) break; M = fmaxf(M, ml[s].x); }
+                    for (int s = 0; s < 8; ++s) M = fmaxf(M, ml[s].x);
 #pragma unroll
                     for (int s = 0; s < 8; ++s) {
-                        if (s >= ns) break;
                         const float x = ex2_approx(ml[s].x - M);
                         Lsum += ml[s].y * x;
                         acc += os[s] * x;
@@ -598,10 +646,10 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
                 step = a.nsteps;
                 break;
             }
-            ask(first_unit, l, p, 0);
 #pragma unroll 1
             for (int pt = 0; pt < cluster_job_of(kJobQkv, E, 0).parts; ++pt)
                 finish(Job<kJobQkv>(), pt, product(Job<kJobQkv>(), xb, [&] { if (pt == 0 && l > 0) receive(kXb); }), l, p);
+            ask(first_unit, l, p, 0);
             receive(kQkv);
             attend(l, p);
 #pragma unroll 1
