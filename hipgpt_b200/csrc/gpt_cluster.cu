@@ -14,7 +14,9 @@
 //     is therefore one such store and one barrier inside the block: no barrier over the cluster, nothing through L2.
 //   * A block's weights are laid out once in the order in which a step reads them and arrive through a ring in shared memory by
 //     bulk copies that run up to a layer ahead of the arithmetic; they do not depend on activations, so nothing waits for them.
-//   * Warp s owns segment s of the inner dimension (lanes: columns), so a layer norm needs no barrier either: every warp forms
+//   * The feed-forward's inner row does not leave its block: a block's columns of the first matrix are a segment of the second one's inner
+//     dimension, so it multiplies them on and sends partial sums to the columns' owners.
+//   * Elsewhere warp s owns segment s of the inner dimension (lanes: columns), so a layer norm needs no barrier either: every warp forms
 //     the row's statistics and normalises the part that it multiplies.
 //   * Keys and values of older positions are asked for while the projection of the new one is on its way between the blocks.
 //   * The logits are formed where an id is picked from them: not at prompt positions before the last.
@@ -25,8 +27,8 @@
 // out too, and all meet at the barriers of the remaining steps and leave.  (A barrier whose phase has not been seen complete is not
 // opened again, and the bytes that nobody waits for stay within eight layers' worth, at most 90 KB each: an mbarrier counts 2^20.)
 //
-// Measured at the default model (E=256 L=8 H=8 V=5000), batch 8: 66 us per step (the replayed graph: 184), batch 3: 59.  A layer of
-// 8 us: the hops (450 - 700 ns from the last store to the first read, five of them), attention 1.2, the two layer norms 0.35 each, a product's
+// Measured at the default model (E=256 L=8 H=8 V=5000), batch 8: 64 us per step (the replayed graph: 184), batch 3: 57.  A layer of
+// 7.6 us: the hops (450 - 700 ns from the last store to the first read, five of them), attention 1.2, the two layer norms 0.35 each, a product's
 // multiply-adds 0.15 - 0.5.  Besides, the shared memory's width is in the chain wherever all warps read at once (192 KB of weights are 1536 cycles of a
 // layer): sums column by column, weights that no two lanes read twice and QKV's weights asked for before their activations took a step from 72 to 66 us
 // (B=7 E=192 L=5, 67 positions and more: 5268 -> 4723 us a request).  Sizes are template parameters because the chain is
@@ -88,10 +90,11 @@ struct Width { static constexpr int kE = E, kD = D, kR = R, kVW = VW; };
 // by four floats: the rows that a warp reads side by side then lie in different banks.
 template <int E, int R>
 struct Lay {
-    static constexpr int F = 4 * E;
-    static constexpr int es = E + 4, qs = 3 * E + 4, fs = F + 4;         // row strides
+    static constexpr int es = E + 4, qs = 3 * E + 4;                     // row strides
     static constexpr int seg = cluster_job_of(kJobQkv, E, 16).klp + 4;   // of a warp's own segment
-    static constexpr int xb = 0, xa = xb + R * es, qkv = xa + R * es, ff = qkv + R * qs, aw = ff + R * fs, part = aw + kWarps * R * seg;
+    static constexpr ClusterJob f2 = cluster_job_of(kJobF2, E, 16);
+    static constexpr int fs = f2.klen + 4;                               // of the block's segment of the feed-forward's inner row
+    static constexpr int xb = 0, xa = xb + R * es, qkv = xa + R * es, ff = qkv + R * qs, f2s = ff + R * fs, aw = f2s + 16 * R * f2.nc, part = aw + kWarps * R * seg;
     static constexpr int part_stride = R * 16 * 64;
     static constexpr int unit = part + 2 * part_stride, amax = unit + 8 * 4 * 16 * 8, fixed = (amax + 32 * R * 2 + 3) & ~3;
     static constexpr int slot_bytes()
@@ -123,14 +126,13 @@ __global__ void __launch_bounds__(kThreads, 1)
 cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_constant__ ClusterArgs a, const __grid_constant__ Rest lay)
 {
     using C = Lay<E, R>;
-    constexpr int F = 4 * E;
     extern __shared__ __align__(128) float sm[];
     __shared__ uint64_t full[kMostSlots];
-    __shared__ uint64_t hop[6];                      // qkv, attention records, xa, ff, xb, first maxima
+    __shared__ uint64_t hop[6];                      // qkv, attention records, xa, partial sums of the second feed-forward product, xb, first maxima
     __shared__ float2 stats[R];                      // (R > 1) a row's mean and 1 / sqrt(variance + eps)
     __shared__ int next_id[R];
     __shared__ Waits waits;
-    enum { kQkv, kRec, kXa, kFf, kXb, kAm };
+    enum { kQkv, kRec, kXa, kF2, kXb, kAm };
     static_assert(kRec == kHopRecords, "");
 
     const int tid = threadIdx.x, lane = tid & 31;
@@ -142,13 +144,14 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
     constexpr int H = E / D, rstride = D + 4;
     const int V = a.V, ns = a.ns;
 
-    float *xb = sm + C::xb, *xa = sm + C::xa, *qkv = sm + C::qkv, *ff = sm + C::ff, *rec = sm + C::fixed, *part = sm + C::part;
+    float *xb = sm + C::xb, *xa = sm + C::xa, *qkv = sm + C::qkv, *rec = sm + C::fixed, *part = sm + C::part;
     float *aw = sm + C::aw + warp * (R * C::seg);    // this warp's own segment of the activations
     uint32_t *amax = reinterpret_cast<uint32_t *>(sm + C::amax);
     uint2 *table = reinterpret_cast<uint2 *>(sm + lay.table);
     uint8_t *ring = reinterpret_cast<uint8_t *>(sm + lay.ring);
+    const int f2_own = max(0, min(C::f2.nc, E - rank * C::f2.nc));       // columns whose partial sums come to this block
     auto tx = [&](int i) {
-        return (uint32_t)(rows * (i == kQkv ? 12 * E : i == kRec ? H * ns * (D + 2) * 4 : i == kFf ? 4 * F : i == kAm ? 32 * 8 : 4 * E));
+        return (uint32_t)(rows * (i == kQkv ? 12 * E : i == kRec ? H * ns * (D + 2) * 4 : i == kF2 ? 16 * 4 * f2_own : i == kAm ? 32 * 8 : 4 * E));
     };
 
     for (int i = tid; i < lay.table; i += kThreads) sm[i] = 0.0f;         // rows that the cluster does not have stay zero
@@ -239,9 +242,7 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
     // One product's multiply-adds: this warp's segment of the inner dimension, all columns of the part.  The activations: rows at
     // `src` in shared memory, normalised first where the job says so; kJobO takes this warp's own segment.  Leaves the partial sums
     // in part + flip * part_stride and ends with a barrier of the block.  Lanes: up to 16 columns: (column, row of a pair); more:
-    // columns lane, lane + 32, all rows.  kPaired (the long product of few columns): eight of the warps take two segments each, a half of the lanes a segment
-    // and all its rows, so that a warp reads each weight once; as (column, row) its weights were read once per row, the 1000 cycles that the product took
-    // to begin.  Returns the part's bias for the column that this thread finishes.
+    // columns lane, lane + 32, all rows.  Returns the part's bias for the column that this thread finishes.
     // `arrival` waits for the activations.  Before it the weights of this lane go to registers (where there are at most 64): they
     // have been in the ring for long, and reading them takes the shared memory's return path about as long as a hop takes.  (With two rows the
     // other warps wait with that until the sums before have been read: bar 9 in `finish`, 8874 -> 8779 us a request; with one row it costs as much.)
@@ -249,15 +250,12 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
         constexpr int J = decltype(jn)::value;
         constexpr ClusterJob jb = cluster_job_of(J, E, 64 * 64);          // (the output projection's cut depends on V in its parts only)
         constexpr int pw = jb.width, klen = jb.klen, klp = jb.klp, sh = jb.seg_shift, nch = jb.chunks();
-        constexpr int stride = J == kJobF2 ? C::fs : C::es;
-        constexpr bool kPaired = J == kJobF2 && pw <= 16 && klp <= 64;
-        static_assert(!kPaired || (sh >= 1 && (klen & 3) == 0), "two segments lie in one chunk, rows of activations are read in place");
-        const int seg = kPaired ? 2 * (warp & 7) + (lane >> 4) : warp;
-        int slot = slot0 + ((kPaired ? 2 * (warp & 7) : warp) >> sh);
+        constexpr int stride = C::es;
+        int slot = slot0 + (warp >> sh);
         uint32_t par = slot_par;
         if (slot >= lay.slots) { slot -= lay.slots; par ^= 1u; }
         const float *chunk = reinterpret_cast<const float *>(ring + slot * C::kSlot);
-        const int in_chunk = seg & ((1 << sh) - 1);
+        const int in_chunk = warp & ((1 << sh) - 1);
         const float4 *w4 = reinterpret_cast<const float4 *>(chunk + in_chunk * (klp * pw));
         const float *as = aw;
         constexpr bool kOwn = jb.ln || J == kJobO || (klen & 3) != 0;     // the activations are (copied) in this warp's own segment
@@ -267,7 +265,7 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
         const int wc0 = pw <= 16 ? (pw < 16 ? min(lane & 15, pw - 1) : lane & 15) : (pw < 32 ? min(lane, pw - 1) : lane);
         const float4 *wp = w4 + wc0, *wq = w4 + (pw < 64 ? min(lane + 32, pw - 1) : lane + 32);
         float4 held[kEarly ? NC * klp / 4 : 1];
-        if constexpr (kEarly && !kPaired) {
+        if constexpr (kEarly) {
             wait(&full[slot], par);
 #pragma unroll
             for (int k = 0; k < klp / 4; ++k) {
@@ -275,7 +273,7 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
                 if constexpr (NC > 1) held[NC * k + 1] = wq[k * pw];
             }
         }
-        if constexpr (!kPaired) arrival();
+        arrival();
         float2 own = make_float2(0.f, 0.f);
         if constexpr (jb.ln != 0 && R == 1) own = row_stats(src);
         if constexpr (jb.ln != 0 && R > 1) {
@@ -285,7 +283,7 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
             }
             __syncthreads();
         }
-        if constexpr (!kEarly && !kPaired) wait(&full[slot], par);
+        if constexpr (!kEarly) wait(&full[slot], par);
         if constexpr (jb.ln != 0) {
             const float *gm = chunk + jb.weight_floats() + in_chunk * klp, *bt = gm + (klp << sh);
 #pragma unroll
@@ -305,37 +303,10 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
             }
             __syncwarp();
         } else if constexpr (!kOwn) {
-            as = src + seg * klen;
+            as = src + warp * klen;
         }
-        float *dst = part + flip * C::part_stride + seg * pw;
-        if constexpr (kPaired) {
-            if (warp >= 8) {
-                float4 w[klp / 4];
-                wait(&full[slot], par);
-#pragma unroll
-                for (int k = 0; k < klp / 4; ++k) w[k] = wp[k * pw];
-                arrival();
-                float acc[R];
-#pragma unroll
-                for (int r = 0; r < R; ++r) acc[r] = 0.0f;
-#pragma unroll
-                for (int k = 0; k < klp / 4; ++k) {
-#pragma unroll
-                    for (int r = 0; r < R; ++r) {
-                        const float4 x = *reinterpret_cast<const float4 *>(as + r * astride + 4 * k);
-                        acc[r] = fmaf(x.x, w[k].x, acc[r]);
-                        acc[r] = fmaf(x.y, w[k].y, acc[r]);
-                        acc[r] = fmaf(x.z, w[k].z, acc[r]);
-                        acc[r] = fmaf(x.w, w[k].w, acc[r]);
-                    }
-                }
-                if ((lane & 15) < pw)
-#pragma unroll
-                    for (int r = 0; r < R; ++r) dst[r * 16 * pw + (lane & 15)] = acc[r];
-            } else {
-                arrival();
-            }
-        } else if constexpr (pw <= 16) {
+        float *dst = part + flip * C::part_stride + warp * pw;
+        if constexpr (pw <= 16) {
             constexpr int RH = (R + 1) / 2;          // rows of a lane: r0, r0 + 2
             const int c = lane & 15, r0 = R > 1 ? lane >> 4 : 0;
             float acc[RH];
@@ -400,16 +371,24 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
         if (slot0 >= lay.slots) { slot0 -= lay.slots; slot_par ^= 1u; }
         return bias;
     };
+    // Four neighbouring threads' columns (where `mine`: of an existing row, within the block's share), stored by each into four of the sixteen blocks
+    auto send_four = [&](float v, bool mine, int to_floats, int h) {
+        const float4 four = make_float4(__shfl_sync(0xffffffffu, v, 0, 4), __shfl_sync(0xffffffffu, v, 1, 4), __shfl_sync(0xffffffffu, v, 2, 4), __shfl_sync(0xffffffffu, v, 3, 4));
+        if (mine) {
+            const uint32_t to = smem_u32(sm + (to_floats & ~3)), bar = smem_u32(&hop[h]);
+#pragma unroll
+            for (int d = 0; d < 4; ++d) send4(to + peer[d], bar + peer[d], four);
+        }
+        return four;
+    };
     // Finishes part `pt` of a product: a thread adds up a column of a row (partial sums in ascending order; a warp reads whole lines: as four
-    // columns per thread, with a thread per four receivers, each line was read four times, and that traffic stood in the chain); four neighbours
-    // then exchange theirs and each stores all four columns into four of the sixteen blocks.
+    // columns per thread, with a thread per four receivers, each line was read four times, and that traffic stood in the chain) and hands it over with
+    // its neighbours'.  The feed-forward's inner row stays in the block, which goes on with its segment of it.
     auto finish = [&](auto jn, int pt, float bias, int layer, int p) {
         constexpr int J = decltype(jn)::value;
         constexpr ClusterJob jb = cluster_job_of(J, E, 64 * 64);
-        constexpr int pw = jb.width, stride = J == kJobQkv ? C::qs : J == kJobF1 ? C::fs : C::es;
-        constexpr int buf = J == kJobQkv ? C::qkv : J == kJobO ? C::xa : J == kJobF1 ? C::ff : C::xb;
-        constexpr int res = J == kJobO ? C::xb : C::xa;
-        constexpr int h = J == kJobQkv ? kQkv : J == kJobO ? kXa : J == kJobF1 ? kFf : kXb;
+        constexpr int pw = jb.width, stride = J == kJobQkv ? C::qs : C::es;
+        constexpr int buf = J == kJobQkv ? C::qkv : C::xa;
         if (warp * 32 < pw * R) {                    // (whole warps)
             const int r = R == 1 ? 0 : tid / pw, c = tid - r * pw, n = rank * jb.nc + pt * pw + c;
             // the block's last columns may lie past its share (the last part) or past the matrix: four at a time
@@ -421,27 +400,100 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
 #pragma unroll
                 for (int s = 1; s < 16; ++s) v = __fadd_rn(v, ps[s * pw]);
                 v = __fadd_rn(v, bias);
-                if constexpr (J == kJobF1) v = fmaxf(0.0f, v);
-                if constexpr (J == kJobO || J == kJobF2) v = __fadd_rn(sm[res + r * stride + n], v);
+                if constexpr (J == kJobF1) sm[C::ff + r * C::fs + pt * pw + c] = fmaxf(0.0f, v);
+                if constexpr (J == kJobO) v = __fadd_rn(sm[C::xb + r * stride + n], v);
             }
-            if constexpr (R > 1) asm volatile("bar.arrive 9, 512;" ::: "memory");
-            const float4 four = make_float4(__shfl_sync(0xffffffffu, v, 0, 4), __shfl_sync(0xffffffffu, v, 1, 4), __shfl_sync(0xffffffffu, v, 2, 4), __shfl_sync(0xffffffffu, v, 3, 4));
-            if (mine) {
-                const int n0 = n & ~3;               // (shares and parts are whole fours)
-                const uint32_t to = smem_u32(sm + buf + r * stride + n0), bar = smem_u32(&hop[h]);
-#pragma unroll
-                for (int d = 0; d < 4; ++d) send4(to + peer[d], bar + peer[d], four);
+            if constexpr (J != kJobF1) {
+                if constexpr (R > 1) asm volatile("bar.arrive 9, 512;" ::: "memory");
+                const float4 four = send_four(v, mine, buf + r * stride + n, J == kJobQkv ? kQkv : kXa);
                 if constexpr (J == kJobQkv) {
-                    if (dq == (rank >> 2) && n0 >= E) {          // keys and values, for the later positions
+                    const int n0 = n & ~3;           // (shares and parts are whole fours)
+                    if (mine && dq == (rank >> 2) && n0 >= E) {  // keys and values, for the later positions
                         float *cache = (n0 < 2 * E ? a.kc : a.vc) + (size_t)layer * a.layer_stride + ((size_t)(row0 + r) * a.S + p) * E;
                         *reinterpret_cast<float4 *>(cache + (n0 < 2 * E ? n0 - E : n0 - 2 * E)) = four;
                     }
                 }
             }
-        } else if constexpr (R > 1) {
+        } else if constexpr (J != kJobF1 && R > 1) {
             asm volatile("bar.sync 9, 512;" ::: "memory");
         }
         flip ^= 1;
+    };
+    // The second product of the feed-forward: this block's columns of the first are a segment of its inner dimension, so they need no hop.  The last
+    // warps take 32 columns each, all rows, and send the partial sums to the blocks that own the columns; these add them up in order (the same
+    // order as everywhere) and hand the row out.  As a product like the others, the inner row by a hop (512 stores a block, 0.3 us to issue) and partial sums
+    // through the block: 66 us a step instead of 64 at the default model, E=320 D=64 batch 4 10956 us a request instead of 8964, E=384 batch 8 10309 instead of 9027.
+    auto second = [&]() {
+        constexpr ClusterJob jb = C::f2;
+        constexpr int G = jb.per * jb.width / 32, K4 = jb.klen / 4;      // warps at work
+        constexpr int kHeld = K4 < 8 ? K4 : 8;                           // a column's first weights are in registers before the row is there (all: spills)
+        float bias = 0.0f;
+        const int own_r = R == 1 ? 0 : tid / jb.nc, own_c = tid - own_r * jb.nc, own_n = rank * jb.nc + own_c;
+        const bool sums = warp * 32 < jb.nc * R, mine = sums && tid < jb.nc * R && own_r < rows && own_n < E;
+        if (sums) {
+            wait(&full[slot0], slot_par);
+            if (tid < jb.nc * R) bias = (reinterpret_cast<const float *>(ring + slot0 * C::kSlot) + jb.weight_floats())[own_c];
+        }
+#pragma unroll 1
+        for (int pt = 0; pt < jb.parts; ++pt) {
+            const int g = warp - (kWarps - G);
+            if (g >= 0) {
+                int slot = slot0 + g / (jb.width / 32);
+                uint32_t par = slot_par;
+                if (slot >= lay.slots) { slot -= lay.slots; par ^= 1u; }
+                const float4 *wp = reinterpret_cast<const float4 *>(ring + slot * C::kSlot) + g % (jb.width / 32) * 32 + lane;
+                wait(&full[slot], par);
+                float4 w[kHeld];
+#pragma unroll
+                for (int k = 0; k < kHeld; ++k) w[k] = wp[k * jb.width];
+                if (pt == 0) __syncthreads();        // the segment of the inner row is there
+                float acc[R];
+#pragma unroll
+                for (int r = 0; r < R; ++r) acc[r] = 0.0f;
+                auto take = [&](int k, const float4 &wk) {
+#pragma unroll
+                    for (int r = 0; r < R; ++r) {
+                        const float4 x = *reinterpret_cast<const float4 *>(sm + C::ff + r * C::fs + 4 * k);
+                        acc[r] = fmaf(x.x, wk.x, acc[r]);
+                        acc[r] = fmaf(x.y, wk.y, acc[r]);
+                        acc[r] = fmaf(x.z, wk.z, acc[r]);
+                        acc[r] = fmaf(x.w, wk.w, acc[r]);
+                    }
+                };
+#pragma unroll
+                for (int k = 0; k < kHeld; ++k) take(k, w[k]);
+#pragma unroll 8
+                for (int k = kHeld; k < K4; ++k) take(k, wp[k * jb.width]);
+                // four columns of a row in one store, a lane of four per row
+                const int n = (pt * G + g) * 32 + (lane & ~3), owner = n / jb.nc;
+                const uint32_t to = smem_u32(sm + C::f2s + (rank * R + dq) * jb.nc + n - owner * jb.nc);
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const float4 four = make_float4(__shfl_sync(0xffffffffu, acc[r], 0, 4), __shfl_sync(0xffffffffu, acc[r], 1, 4), __shfl_sync(0xffffffffu, acc[r], 2, 4), __shfl_sync(0xffffffffu, acc[r], 3, 4));
+                    if (dq == r && r < rows && n < E) send4(peer_addr(to, owner), peer_addr(smem_u32(&hop[kF2]), owner), four);
+                }
+                asm volatile("bar.sync 10, %0;" ::"n"(32 * G) : "memory");       // the chunks may be overwritten
+                if (warp == kWarps - 1) fetch(jb.per);
+            } else if (pt == 0) {
+                __syncthreads();
+            }
+            slot0 += jb.per;
+            if (slot0 >= lay.slots) { slot0 -= lay.slots; slot_par ^= 1u; }
+        }
+        // (the last warp opens the barrier's next phase; the others have nothing to wait for)
+        if (sums || warp == kWarps - 1) receive(kF2);
+        else hop_phase ^= 1u << kF2;
+        if (sums) {
+            float v = 0.0f;
+            if (mine) {
+                const float *ps = sm + C::f2s + own_r * jb.nc + own_c;
+                v = ps[0];
+#pragma unroll
+                for (int s = 1; s < 16; ++s) v = __fadd_rn(v, ps[s * R * jb.nc]);
+                v = __fadd_rn(sm[C::xa + own_r * C::es + own_n], __fadd_rn(v, bias));
+            }
+            send_four(v, mine, C::xb + own_r * C::es + own_n, kXb);
+        }
     };
 
     // ---- the attention of one position: units of (row, head, split), dealt out over the blocks' warp groups.  attn_decode.cu gives a
@@ -658,9 +710,7 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
 #pragma unroll 1
             for (int pt = 0; pt < cluster_job_of(kJobF1, E, 0).parts; ++pt)
                 finish(Job<kJobF1>(), pt, product(Job<kJobF1>(), xa, [&] { if (pt == 0) receive(kXa); }), 0, 0);
-#pragma unroll 1
-            for (int pt = 0; pt < cluster_job_of(kJobF2, E, 0).parts; ++pt)
-                finish(Job<kJobF2>(), pt, product(Job<kJobF2>(), ff, [&] { if (pt == 0) receive(kFf); }), 0, 0);
+            second();
         }
         if (step >= a.nsteps) break;
         receive(kXb);
@@ -746,6 +796,15 @@ cluster_pack_kernel(const ClusterJob j, int pt, const float *__restrict__ w, con
     const int pw = j.width, ch = blockIdx.x, owner = blockIdx.y;
     const int first = owner * j.nc + pt * pw, end = min(j.n, (owner + 1) * j.nc), segs = 1 << j.seg_shift;
     float *d = reinterpret_cast<float *>(dst + (size_t)owner * block_bytes + (size_t)ch * j.chunk_bytes());
+    if (j.per) {
+        for (int i = threadIdx.x; i < j.weight_floats(); i += blockDim.x) {
+            const int u = i & 3, c = ((pt * j.per + ch) * pw) + (i >> 2) % pw, k = 4 * ((i >> 2) / pw) + u;
+            d[i] = c < j.n ? w[(size_t)(owner * j.klen + k) * j.n + c] : 0.0f;
+        }
+        d += j.weight_floats();
+        for (int i = threadIdx.x; i < j.nc; i += blockDim.x) d[i] = owner * j.nc + i < j.n ? bias[owner * j.nc + i] : 0.0f;
+        return;
+    }
     for (int i = threadIdx.x; i < j.weight_floats(); i += blockDim.x) {
         const int u = i & 3, c = (i >> 2) % pw, k4 = (i >> 2) / pw % (j.klp >> 2), s = (i >> 2) / pw / (j.klp >> 2);
         const int k = 4 * k4 + u;

@@ -15,12 +15,15 @@ constexpr int kHopRecords = 1;                         // the attention records 
 // [klp / 4][width][4]: four consecutive inner indices of a column side by side (klp: klen rounded up to a multiple of 4; what is
 // past the matrix is zero).  After the weights a chunk carries gamma and beta of its segments (where a layer norm precedes the
 // product) and the part's bias.
+// Where the block already has a segment of the inner dimension (`per` > 0: the second matrix of the feed-forward, whose segments are the
+// blocks' columns of the first) it owns that segment for all columns: chunks of `width` columns, [klen / 4][width][4], `per` to a part, each
+// with the bias of the nc columns whose partial sums this block adds up.
 struct ClusterJob {
-    int n, nc, width, parts, klen, klp, seg_shift, ln;
-    __host__ __device__ constexpr int chunks() const { return 16 >> seg_shift; }
-    __host__ __device__ constexpr int weight_floats() const { return (klp * width) << seg_shift; }
+    int n, nc, width, parts, klen, klp, seg_shift, ln, per;
+    __host__ __device__ constexpr int chunks() const { return per ? per : 16 >> seg_shift; }
+    __host__ __device__ constexpr int weight_floats() const { return per ? klen * width : (klp * width) << seg_shift; }
     __host__ __device__ constexpr int ln_floats() const { return ln ? (2 * klp) << seg_shift : 0; }
-    __host__ __device__ constexpr int chunk_bytes() const { return 4 * (weight_floats() + ln_floats() + width); }
+    __host__ __device__ constexpr int chunk_bytes() const { return 4 * (weight_floats() + ln_floats() + (per ? nc : width)); }
 };
 enum { kJobQkv, kJobO, kJobF1, kJobF2, kJobVoc, kJobs };
 
@@ -41,9 +44,22 @@ __host__ __device__ constexpr ClusterJob cluster_job(int n, int k, int ln)
     while (j.seg_shift > 1 && j.chunk_bytes() > 18 * 1024) --j.seg_shift;
     return j;
 }
+// The same, a segment per block.  64 columns to a chunk where that is at most 16 KB; at most eight chunks to a part.
+__host__ __device__ constexpr ClusterJob cluster_job_by_segment(int n, int k)
+{
+    ClusterJob j = {};
+    j.n = n;
+    j.nc = 4 * ((n + 63) / 64);
+    j.klen = j.klp = k / 16;
+    j.width = j.klen <= 64 ? 64 : 32;
+    const int total = (n + j.width - 1) / j.width;
+    j.parts = total > 8 ? 2 : 1;
+    j.per = (total + j.parts - 1) / j.parts;
+    return j;
+}
 __host__ __device__ constexpr ClusterJob cluster_job_of(int i, int E, int V)
 {
-    return i == kJobQkv ? cluster_job(3 * E, E, 1) : i == kJobO ? cluster_job(E, E, 0) : i == kJobF1 ? cluster_job(4 * E, E, 1) : i == kJobF2 ? cluster_job(E, 4 * E, 0)
+    return i == kJobQkv ? cluster_job(3 * E, E, 1) : i == kJobO ? cluster_job(E, E, 0) : i == kJobF1 ? cluster_job(4 * E, E, 1) : i == kJobF2 ? cluster_job_by_segment(E, 4 * E)
                                                                                                                           : cluster_job(V, E, 0);
 }
 

@@ -145,6 +145,8 @@ def test_gpu_generation_forms_agree_and_a_handle_serves_many_requests():
     (dict(V=777, S=64, E=160, L=2, H=5, F=640), 3, 1, 30),          # segments of 10 inner indices: padded
     (dict(V=1000, S=300, E=256, L=1, H=4, F=1024), 9, 5, 40),       # head_dim 64, two sequences per cluster, one left over
     (dict(V=1371, S=96, E=384, L=1, H=12, F=1536), 2, 4, 24),       # products in several parts
+    (dict(V=150, S=40, E=224, L=2, H=7, F=896), 3, 2, 12),          # a chunk of the second feed-forward matrix half past its columns
+    (dict(V=150, S=40, E=288, L=2, H=9, F=1152), 9, 2, 12),         # ... and one wholly, in the second of two parts; two sequences per cluster
     (dict(V=300, S=700, E=128, L=1, H=2, F=512), 2, 300, 60),       # contexts of more rows than a lane asks for ahead
     (dict(V=200, S=2100, E=128, L=1, H=4, F=512), 2, 2060, 40),     # a long context, several rounds of a unit
     (dict(V=200, S=40, E=128, L=1, H=4, F=512), 15, 2, 10),         # a batch for the replayed graph
