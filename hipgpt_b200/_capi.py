@@ -6,6 +6,8 @@ exception is raised.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import os
 
 from . import build as _build
@@ -119,6 +121,16 @@ def lib() -> C.CDLL:
             fn.restype, fn.argtypes = res, args
         _lib = handle
     return _lib
+
+
+def native():
+    """The extension with the hot calls of launchers.py, built with the library."""
+    if not os.path.exists(_build.EXT):
+        _build.build()
+    loader = importlib.machinery.ExtensionFileLoader("hipgpt_launch", _build.EXT)
+    module = importlib.util.module_from_spec(importlib.util.spec_from_loader("hipgpt_launch", loader))
+    loader.exec_module(module)
+    return module
 
 
 def check(rc: int) -> None:

@@ -19,6 +19,7 @@ CSRC = os.path.join(PKG, "csrc")
 LIBDIR = os.path.join(PKG, "_lib")
 LIB = os.path.join(LIBDIR, "libhipgpt_attn.so")
 OBJDIR = os.path.join(LIBDIR, "obj")
+EXT = os.path.join(LIBDIR, "hipgpt_launch.so")          # the Python mirror's hot calls (csrc/launchers_py.cpp)
 
 SOURCES = ["attn_fwd_rows.cu", "attn_fwd_tc.cu", "attn_fwd_bf16.cu", "attn_fwd_tc16.cu", "attn_fwd_head.cu", "attn_fwd_generic.cu", "attn_unfused.cu", "attn_bwd.cu", "attn_bwd_tc.cu", "attn_bwd_head.cu", "layer_ops.cu", "attn_decode.cu", "gpt_decode.cu", "gpt_cluster.cu", "probe.cu", "wait_probe.cu", "capi.cu",
            "compat_launchers.cpp", "checkpoint.cpp", "sharded.cpp", "shard_push.cu", "gemm_tc.cu"]
@@ -42,10 +43,30 @@ def _deps():
 
 
 def up_to_date() -> bool:
-    if not os.path.exists(LIB):
+    if not (os.path.exists(LIB) and os.path.exists(EXT)):
         return False
-    t = os.path.getmtime(LIB)
+    t = min(os.path.getmtime(LIB), os.path.getmtime(EXT))
     return all(os.path.getmtime(p) <= t for p in _deps())
+
+
+def build_extension() -> str:
+    """The CPython extension on torch's headers, linked against the library beside it."""
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+
+    torch_lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(nvcc())))
+    inc = [*cpp_extension.include_paths(), os.path.join(cuda, "include"), sysconfig.get_paths()["include"], os.path.join(ROOT, "include")]
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *[f"-I{d}" for d in inc], os.path.join(CSRC, "launchers_py.cpp"), "-o", EXT, f"-L{torch_lib}", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda",
+           f"-L{LIBDIR}", "-l:libhipgpt_attn.so", "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{torch_lib}"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        sys.stderr.write(r.stdout + r.stderr)
+        raise RuntimeError("g++ failed on launchers_py.cpp")
+    return EXT
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -72,6 +93,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     if r.returncode != 0:
         sys.stderr.write(r.stdout + r.stderr)
         raise RuntimeError("link failed")
+    build_extension()
     return LIB
 
 

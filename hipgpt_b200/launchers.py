@@ -22,6 +22,12 @@ def _ptr(t):
     return t.data_ptr()
 
 
+def _ptr_bf16(t):
+    if not (t.is_cuda and t.dtype == torch.bfloat16 and t.is_contiguous()):
+        raise ValueError("expected a contiguous CUDA bfloat16 tensor")
+    return t.data_ptr()
+
+
 # the current stream's handle without the Stream object around it (3.2 us of host time per call)
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 _current_device = torch.cuda.current_device
@@ -33,14 +39,19 @@ def _stream():
     return _raw_stream(_current_device())
 
 
+_native = _capi.native()
+_native.bind(_ptr, _ptr_bf16)
+
+
 def launch_multihead_attention(d_qkv, d_output, d_attn_probs, B: int, S: int, E: int, H: int, *, causal: bool = False):
     """softmax(Q K^T / sqrt(E/H)) V per (batch, head).  d_qkv: three stacked [B*S, E] planes;
     d_output [B*S, E]; d_attn_probs [B, H, S, S] or None.  Not causal unless asked: the
     reference never masks (src/hip_kernels.cpp:287-319)."""
     if H <= 0 or E % H != 0:
         raise ValueError(f"Bad MHA config: E={E} H={H}")   # the reference aborts here
-    _capi.check(_capi.lib().hipgpt_mha_forward_planes(_ptr(d_qkv), _ptr(d_output), _ptr(d_attn_probs),
-                                                      B, S, E, H, int(causal), _stream()))
+    rc = _native.attention(d_qkv, d_output, d_attn_probs, B, S, E, H, int(causal))
+    if rc:
+        _capi.check(rc)
 
 
 def mha_forward(q, k, v, out, probs, B: int, S: int, E: int, H: int, *, causal: bool = False,
@@ -53,13 +64,9 @@ def mha_forward(q, k, v, out, probs, B: int, S: int, E: int, H: int, *, causal: 
 def mha_forward_bf16(d_qkv, d_output, B: int, S: int, E: int, H: int, *, causal: bool = False, variant: int = 0):
     """The launcher's contract with bf16 storage: d_qkv = three stacked [B*S, E] bf16 planes, d_output
     [B*S, E] bf16 (head_dim 64), fp32 accumulation."""
-    for t in (d_qkv, d_output):
-        if not (t.is_cuda and t.dtype == torch.bfloat16 and t.is_contiguous()):
-            raise ValueError("expected a contiguous CUDA bfloat16 tensor")
-    plane = B * S * E * 2                                   # bytes
-    p = d_qkv.data_ptr()
-    _capi.check(_capi.lib().hipgpt_mha_forward_bf16_ex(p, p + plane, p + 2 * plane, d_output.data_ptr(), B, S, E, H, int(causal),
-                                                       int(variant), _stream()))
+    rc = _native.attention_bf16(d_qkv, d_output, B, S, E, H, int(causal), int(variant))
+    if rc:
+        _capi.check(rc)
 
 
 def launch_scaled_dot_product(Q, K, scores, B: int, S: int, D: int):
@@ -80,9 +87,10 @@ def decode_scratch_bytes(B: int, H: int, D: int, ctx: int) -> int:
 
 def mha_decode(q, kcache, vcache, out, scratch, B: int, H: int, D: int, ctx: int, cap: int):
     """One query row per (batch, head) over the first ctx rows of the caches."""
-    nbytes = 0 if scratch is None else scratch.numel() * scratch.element_size()
-    _capi.check(_capi.lib().hipgpt_mha_decode(_ptr(q), _ptr(kcache), _ptr(vcache), _ptr(out), _ptr(scratch), nbytes,
-                                              B, H, D, ctx, cap, _stream()))
+    nbytes = None if scratch is None or type(scratch) is torch.Tensor else scratch.numel() * scratch.element_size()
+    rc = _native.decode(q, kcache, vcache, out, scratch, nbytes, B, H, D, ctx, cap)
+    if rc:
+        _capi.check(rc)
 
 
 def mha_forward_host(h_qkv, h_out, h_probs, B: int, S: int, E: int, H: int, *, causal: bool = False):
