@@ -54,11 +54,11 @@ def build_extension() -> str:
     import sysconfig
 
     import torch
-    from torch.utils import cpp_extension
 
-    torch_lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    torch_dir = os.path.dirname(torch.__file__)
+    torch_lib = os.path.join(torch_dir, "lib")
     cuda = os.path.dirname(os.path.dirname(os.path.realpath(nvcc())))
-    inc = [*cpp_extension.include_paths(), os.path.join(cuda, "include"), sysconfig.get_paths()["include"], os.path.join(ROOT, "include")]
+    inc = [os.path.join(torch_dir, "include"), os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"), os.path.join(cuda, "include"), sysconfig.get_paths()["include"], os.path.join(ROOT, "include")]
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
            *[f"-I{d}" for d in inc], os.path.join(CSRC, "launchers_py.cpp"), "-o", EXT, f"-L{torch_lib}", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda",
            f"-L{LIBDIR}", "-l:libhipgpt_attn.so", "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{torch_lib}"]

@@ -188,14 +188,22 @@ kv_pack_kernel(const float *__restrict__ K, const float *__restrict__ V, float *
     const float *src = (vside ? V : K) + ((size_t)b * S + kt * kKeys) * (size_t)E + (size_t)h * D + 8 * pc;
     float4 xa[NP], xc[NP];
     float mx = 0.0f;
+    // At head_dim 64 whole sectors (where the planes allow it) that leave L2 first, so that the images stay: B=4 H=8 S=2048 causal 64.6 -> 62.7 us per call,
+    // B=16 H=8 S=1024 88.9 -> 88.0, unmasked 130.5 -> 129.8.  At 32, where K and V are smaller and may be found in L2, 24.6 -> 25.3 (B=8 H=9 S=700).
+    const bool sectors = D == 64 && ((reinterpret_cast<uintptr_t>(K) | reinterpret_cast<uintptr_t>(V)) & 31) == 0;
 #pragma unroll
     for (int i = 0; i < NP; ++i) {
         const int r = r0 + i * RPT;
         const bool ok = kt * kKeys + r < S;
         const float4 *p = reinterpret_cast<const float4 *>(src + (ok ? (size_t)r * E : 0));
         const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-        xa[i] = ok ? __ldg(p) : z;
-        xc[i] = ok ? __ldg(p + 1) : z;
+        xa[i] = xc[i] = z;
+        if (ok && sectors) {
+            load_sector_once(p, xa[i], xc[i]);
+        } else if (ok) {
+            xa[i] = __ldg(p);
+            xc[i] = __ldg(p + 1);
+        }
     }
 #pragma unroll
     for (int i = 0; i < NP; ++i)
