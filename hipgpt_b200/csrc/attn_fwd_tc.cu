@@ -233,10 +233,10 @@ mha_tc_kernel(const float *__restrict__ Q, const float *__restrict__ K, const fl
         };
         fetch_tile(K, k_raw, 0);
         fetch_tile(V, v_raw, 0);
-        cp_async_wait_1();
+        cp_async_wait<1>();
         store_k();
         fetch_tile(K, k_raw, 1);
-        cp_async_wait_1();
+        cp_async_wait<1>();
         store_v(0);
         fetch_tile(V, v_raw, 1);                 // from here on: K(t+1), then V(t+1) in flight at the top of iteration t
         proxy_fence();                           // generic-proxy writes -> visible to the tensor core's reads
@@ -244,13 +244,13 @@ mha_tc_kernel(const float *__restrict__ Q, const float *__restrict__ K, const fl
         __syncthreads();
         for (int t = 0; t < ntiles; ++t) {
             wait(&mbar_s[t & 1], (uint32_t)((t >> 1) & 1), 7);     // Q K(t)^T has completed: the K buffer is free
-            cp_async_wait_1();                                  // K(t+1) has landed
+            cp_async_wait<1>();                                  // K(t+1) has landed
             if (t + 1 < ntiles) store_k();
             proxy_fence();
             arrive(&mbar_k);
             fetch_tile(K, k_raw, t + 2);
             if (t > 0) wait(&mbar_o, (uint32_t)((t - 1) & 1), 8); // P V(t-1) has completed: its V buffer is free
-            cp_async_wait_1();                                  // V(t+1) has landed
+            cp_async_wait<1>();                                  // V(t+1) has landed
             if (t + 1 < ntiles) store_v((t + 1) & 1);
             proxy_fence();
             arrive(&mbar_v[(t + 1) & 1]);

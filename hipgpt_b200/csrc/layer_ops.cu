@@ -24,8 +24,6 @@
 namespace hipgpt {
 namespace {
 
-constexpr int kBK = 16;
-
 // A tile is 8 TM x 16 TN outputs, 128 threads of TM x TN; TM and TN are chosen per call so that the tiles fill the SMs evenly
 // (launch_matmul_tiles).
 // Two bounds: the FFMA pipe, TM TN clocks per inner index and warp, and the return path of shared memory, which hands a warp 128
@@ -36,23 +34,28 @@ constexpr int kBK = 16;
 // Registers alone (the same multiply-adds without loads) reach 61 TFLOP/s; here 54 at 16384 x 512 x 1536 (one inner index after
 // another in 128 x 128 tiles, operands through registers: 47.7).  With 8192 rows: 256 -> 768 columns 80 -> 63 us, 256 -> 256 35 -> 27,
 // 256 -> 1024 105 -> 83, 1024 -> 256 125 -> 92.
-constexpr int kTileThreads = 128;
-constexpr int kTileStages = 3;
-template <int TM, int TN>
+// Small products (TN = 4) are bound by neither but by the distance from a load to its use and by what a stage costs besides: their fragments are read
+// eight inner indices of B and four of A ahead, a stage has 32 inner indices, and where few tiles have to fill many SMs a block has TY = 4 rows of
+// threads instead of 8: half as many warps at the return path.  Rows x inner x columns: 100 x 1024 x 256 21.1 -> 12.4 us, 400 x 256 x 768 9.8 -> 7.5,
+// 200 x 2048 x 512 41.3 -> 30.9, 2000 x 768 x 192 28.0 -> 19.5.  (Deeper stages for the tiles between, 5 x 8 and so on: 1407 x 512 x 2048 65 -> 66.)
+template <int TM, int TN, int TY>
 struct TileCfg {
-    static constexpr int BM = 8 * TM, BN = 16 * TN;
+    static constexpr bool kSmall = TN == 4;
+    static constexpr int kBK = kSmall ? 32 : 16, kStages = kSmall ? 5 : 3;         // inner indices of a stage
+    static constexpr int kThreads = 16 * TY, BM = TY * TM, BN = 16 * TN;
+    static constexpr int kAheadB = kSmall ? 8 : 2, kAheadA = kSmall ? 2 : 1;      // fragments in registers: of an index of B, of four of A
     static constexpr int AStride = kBK + 4;                              // floats between rows of A in shared memory
     static constexpr int kStageFloats = BM * AStride + kBK * BN;
-    static constexpr size_t kSmem = (size_t)kTileStages * kStageFloats * 4;
+    static constexpr size_t kSmem = (size_t)kStages * kStageFloats * 4;
 };
-template <int TM, int TN>
-__global__ void __launch_bounds__(kTileThreads, TM * TN > 64 ? 2 : 3)
+template <int TM, int TN, int TY>
+__global__ void __launch_bounds__(16 * TY, TM * TN > 64 ? 2 : 3)
 matmul_tile_kernel(const float *A, const float *__restrict__ B, const float *__restrict__ bias, float *C,     // A and C may be one buffer
                    int M, int N, int K, int col_tiles)
 {
-    using T = TileCfg<TM, TN>;
-    constexpr int BM = T::BM, BN = T::BN;
-    extern __shared__ __align__(16) float tile_s[];                      // [stage][A: BM rows of 16 | B: 16 rows of BN]
+    using T = TileCfg<TM, TN, TY>;
+    constexpr int BM = T::BM, BN = T::BN, kTileThreads = T::kThreads, kBK = T::kBK;
+    extern __shared__ __align__(16) float tile_s[];                      // [stage][A: BM rows of kBK | B: kBK rows of BN]
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
     // column tile fastest: blocks that run side by side share rows of A
     const int row0 = (int)(blockIdx.x / col_tiles) * BM, col0 = (int)(blockIdx.x % col_tiles) * BN;
@@ -68,13 +71,13 @@ matmul_tile_kernel(const float *A, const float *__restrict__ B, const float *__r
     const int ntiles = (N + kBK - 1) / kBK;
     auto copy = [&](int t) {
         if (t < ntiles) {
-            float *as = tile_s + (t % kTileStages) * T::kStageFloats, *bs = as + BM * T::AStride;
+            float *as = tile_s + (t % T::kStages) * T::kStageFloats, *bs = as + BM * T::AStride;
             const int k0 = t * kBK;
 #pragma unroll
-            for (int i = 0; i < (BM * 4 + kTileThreads - 1) / kTileThreads; ++i) {
-                const int f = tid + i * kTileThreads, m = f >> 2, k = (f & 3) * 4;
+            for (int i = 0; i < (BM * (kBK / 4) + kTileThreads - 1) / kTileThreads; ++i) {
+                const int f = tid + i * kTileThreads, m = f / (kBK / 4), k = f % (kBK / 4) * 4;
                 const bool in = row0 + m < M && k0 + k < N;
-                if (BM * 4 % kTileThreads == 0 || f < BM * 4) cp_async16(as + m * T::AStride + k, A + (in ? (size_t)(row0 + m) * N + k0 + k : 0), in);
+                if (BM * (kBK / 4) % kTileThreads == 0 || f < BM * (kBK / 4)) cp_async16(as + m * T::AStride + k, A + (in ? (size_t)(row0 + m) * N + k0 + k : 0), in);
             }
 #pragma unroll
             for (int i = 0; i < kBK * BN / 4 / kTileThreads; ++i) {
@@ -85,37 +88,42 @@ matmul_tile_kernel(const float *A, const float *__restrict__ B, const float *__r
         }
         cp_async_commit();
     };
-    copy(0);
-    copy(1);
+#pragma unroll
+    for (int t = 0; t + 1 < T::kStages; ++t) copy(t);
     for (int t = 0; t < ntiles; ++t) {
-        cp_async_wait_1();                                   // tile t is there (this thread's part)
+        cp_async_wait<T::kStages - 2>();                     // tile t is there (this thread's part)
         __syncthreads();                                     // everybody's part; and everybody is done with tile t - 1
-        copy(t + 2);
-        const float *as = tile_s + (t % kTileStages) * T::kStageFloats + ty * TM * T::AStride;
-        const float *bs = tile_s + (t % kTileStages) * T::kStageFloats + BM * T::AStride + tx * 4;
-        float2 b[2][TN / 2];
+        copy(t + T::kStages - 1);
+        const float *as = tile_s + (t % T::kStages) * T::kStageFloats + ty * TM * T::AStride;
+        const float *bs = tile_s + (t % T::kStages) * T::kStageFloats + BM * T::AStride + tx * 4;
+        constexpr int PB = T::kAheadB, PA = T::kAheadA;
+        float2 b[PB][TN / 2];
         auto load_b = [&](int k) {
 #pragma unroll
-            for (int j = 0; j < TN / 4; ++j) *reinterpret_cast<float4 *>(&b[k & 1][2 * j]) = *reinterpret_cast<const float4 *>(bs + k * BN + 64 * j);
+            for (int j = 0; j < TN / 4; ++j) *reinterpret_cast<float4 *>(&b[k % PB][2 * j]) = *reinterpret_cast<const float4 *>(bs + k * BN + 64 * j);
         };
-        float a[TM][4];
-        auto load_a = [&](int i, int k) { *reinterpret_cast<float4 *>(a[i]) = *reinterpret_cast<const float4 *>(as + i * T::AStride + k); };
+        float a[PA][TM][4];
+        auto load_a = [&](int i, int k) { *reinterpret_cast<float4 *>(a[k / 4 % PA][i]) = *reinterpret_cast<const float4 *>(as + i * T::AStride + k); };
 #pragma unroll
         for (int i = 0; i < TM; ++i) load_a(i, 0);
-        load_b(0);
+#pragma unroll
+        for (int k = 0; k + 1 < PB; ++k) load_b(k);
 #pragma unroll
         for (int k = 0; k < kBK; ++k) {
-            if (k + 1 < kBK) load_b(k + 1);
+            if (k + PB - 1 < kBK) load_b(k + PB - 1);
+            if (PA > 1 && (k & 3) == 0 && k + 4 < kBK)
+#pragma unroll
+                for (int i = 0; i < TM; ++i) load_a(i, k + 4);
             float2 aa[TM];
 #pragma unroll
-            for (int i = 0; i < TM; ++i) aa[i] = make_float2(a[i][k & 3], a[i][k & 3]);
-            if ((k & 3) == 3 && k + 1 < kBK)
+            for (int i = 0; i < TM; ++i) aa[i] = make_float2(a[k / 4 % PA][i][k & 3], a[k / 4 % PA][i][k & 3]);
+            if (PA == 1 && (k & 3) == 3 && k + 1 < kBK)
 #pragma unroll
                 for (int i = 0; i < TM; ++i) load_a(i, k + 1);
 #pragma unroll
             for (int j = 0; j < TN / 2; ++j)
 #pragma unroll
-                for (int i = 0; i < TM; ++i) acc[i][j] = ffma2(aa[i], b[k & 1][j], acc[i][j]);
+                for (int i = 0; i < TM; ++i) acc[i][j] = ffma2(aa[i], b[k % PB][j], acc[i][j]);
         }
     }
     float4 bb[TN / 4];
@@ -332,25 +340,26 @@ bool overlap(const void *a, size_t na, const void *b, size_t nb)
 // single block of four warps hides less latency, about a fifth), the larger tile among equals.
 struct TileChoice {
     void (*kernel)(const float *, const float *, const float *, float *, int, int, int, int);
-    int tm, tn;
+    int tm, tn, ty;
     size_t smem;
 };
-template <int TM, int TN>
-TileChoice tile_choice() { return {matmul_tile_kernel<TM, TN>, TM, TN, TileCfg<TM, TN>::kSmem}; }
+template <int TM, int TN, int TY = 8>
+TileChoice tile_choice() { return {matmul_tile_kernel<TM, TN, TY>, TM, TN, TY, TileCfg<TM, TN, TY>::kSmem}; }
 
 static int launch_matmul_tiles(const float *A, const float *B, const float *bias, float *C, int M, int N, int K, bool whole_rows, cudaStream_t st)
 {
     static const TileChoice choices[] = {tile_choice<8, 16>(), tile_choice<7, 16>(), tile_choice<6, 16>(), tile_choice<5, 16>(), tile_choice<8, 8>(), tile_choice<7, 8>(),
-                                         tile_choice<6, 8>(), tile_choice<5, 8>(), tile_choice<4, 8>(), tile_choice<3, 8>(), tile_choice<4, 4>(), tile_choice<2, 4>()};
+                                         tile_choice<6, 8>(), tile_choice<5, 8>(), tile_choice<4, 8>(), tile_choice<3, 8>(), tile_choice<4, 4>(),
+                                         tile_choice<6, 4, 4>(), tile_choice<5, 4, 4>(), tile_choice<4, 4, 4>(), tile_choice<3, 4, 4>(), tile_choice<2, 4, 4>(), tile_choice<1, 4, 4>()};
     constexpr int kSms = 148, kSmSharedBytes = 228 * 1024;
     const TileChoice *best = nullptr;
     double best_cost = 0.0;
     long long best_tiles = 0;
     for (const TileChoice &c : choices) {
         if (whole_rows && K > 16 * c.tn) continue;
-        const long long tiles = (long long)((M + 8 * c.tm - 1) / (8 * c.tm)) * ((K + 16 * c.tn - 1) / (16 * c.tn));
+        const long long tiles = (long long)((M + c.ty * c.tm - 1) / (c.ty * c.tm)) * ((K + 16 * c.tn - 1) / (16 * c.tn));
         const long long per_sm = (tiles + kSms - 1) / kSms;
-        const int fma = c.tm * c.tn, loads = 4 * (c.tm + c.tn), clocks = fma > loads ? fma : loads;
+        const int fma = c.tm * c.tn, loads = c.ty / 2 * (c.tm + c.tn), clocks = fma > loads ? fma : loads;
         const double cost = (double)per_sm * clocks * (per_sm == 1 ? 1.2 : 1.0);
         if (!best || cost < best_cost) { best = &c; best_cost = cost; best_tiles = tiles; }
     }
@@ -365,7 +374,7 @@ static int launch_matmul_tiles(const float *A, const float *B, const float *bias
     if (per_sm <= 3) smem = std::max(smem, (size_t)(((size_t)kSmSharedBytes / (size_t)(per_sm + 1) + 128) & ~(size_t)127));
     cudaError_t e = cudaFuncSetAttribute(best->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max(best->smem, (size_t)kSmSharedBytes / 2 + 128));
     if (e == cudaSuccess)
-        e = launch_overlapped(best->kernel, dim3((unsigned)best_tiles), dim3(kTileThreads), smem, st, A, B, bias, C, M, N, K, (K + 16 * best->tn - 1) / (16 * best->tn));
+        e = launch_overlapped(best->kernel, dim3((unsigned)best_tiles), dim3((unsigned)(16 * best->ty)), smem, st, A, B, bias, C, M, N, K, (K + 16 * best->tn - 1) / (16 * best->tn));
     if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "matmul_tile_kernel: %s", cudaGetErrorString(e));
     return HIPGPT_OK;
 }

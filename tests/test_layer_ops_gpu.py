@@ -62,6 +62,27 @@ def test_matmul_tiles_are_bit_identical_to_the_reference_order(M, K):
         assert np.array_equal(dA2.cpu().numpy(), want)
 
 
+@pytest.mark.parametrize("M,K", [(1002, 388), (1249, 388), (664, 388), (495, 388), (157, 388), (79, 388), (2965, 132), (2393, 20), (1795, 20), (1210, 20), (612, 20), (14, 20)])
+def test_matmul_small_tiles_are_bit_identical_to_the_reference_order(M, K):
+    """One shape for each of the tiles of small products, with rows and columns left over and several stages of an inner dimension that is no multiple of
+    one; and, where a block has whole rows, in place."""
+    lib = _capi.lib()
+    N = 300
+    A, W, b = synth.normal(14, (M, N)), synth.normal(15, (N, K), 0.1), synth.normal(16, (K,))
+    want = ob.matmul(A, W, b, M, N, K, fma=True)
+    dA, dW, db, dC = dev(A), dev(W), dev(b), torch.full((M, K), float("nan"), device="cuda")
+    _capi.check(lib.hipgpt_matmul(dA.data_ptr(), dW.data_ptr(), db.data_ptr(), dC.data_ptr(), M, N, K, _st()))
+    torch.cuda.synchronize()
+    assert np.array_equal(dC.cpu().numpy(), want)
+    if K <= 64:
+        W2, A2 = synth.normal(17, (K, K), 0.1), synth.normal(18, (M, K))
+        want = ob.matmul(A2, W2, b, M, K, K, fma=True)
+        dA2, dW2 = dev(A2), dev(W2)
+        _capi.check(lib.hipgpt_matmul(dA2.data_ptr(), dW2.data_ptr(), db.data_ptr(), dA2.data_ptr(), M, K, K, _st()))
+        torch.cuda.synchronize()
+        assert np.array_equal(dA2.cpu().numpy(), want)
+
+
 @pytest.mark.parametrize("M,N,K,bias", [(8192, 256, 768, True), (300, 256, 768, True), (64, 1024, 256, True), (257, 256, 1024, False), (130, 64, 5000, False),
                                         (33, 100, 20, True), (5, 7, 3, False), (1, 256, 256, True), (129, 65, 129, True),
                                         (1407, 512, 509, True), (1407, 2048, 512, False), (700, 330, 260, True),     # slices of a tile on 2, 3 and 3 blocks
