@@ -137,7 +137,9 @@ __device__ __forceinline__ void issue_scores(uint32_t d_tmem, uint32_t a_smem, u
 // small products come first: the tensor core truncates where it adds to its accumulator, so the accumulator should be small
 // while they are added, and it starts anew for every tile (the workers add the tiles up in registers).  One accumulator over all
 // tiles was 10 times farther from float64 at S = 777.
-template <int D, bool WIDE>
+// LOLO: lo x lo too (WIDE has it in any case), for stored probabilities, which are exact: without it dV was 1.24e-7 instead of 1.16e-7 and dQ 1.66e-7 instead of 1.60e-7 from float64 at S = 1024, D = 64, 142 us instead of 143.5;
+// probabilities formed again carry more than it takes away.
+template <int D, bool WIDE, bool LOLO>
 __device__ __forceinline__ void issue_accumulate(uint32_t acc, uint32_t a_tmem, uint32_t b_smem, int hf)
 {
     const uint64_t b = make_desc(b_smem, Img<D>::kBlock, 128, 0) + (uint64_t)(hf * 4 * (Img<D>::kBlock >> 4));
@@ -149,7 +151,8 @@ __device__ __forceinline__ void issue_accumulate(uint32_t acc, uint32_t a_tmem, 
             if (elect_one()) mma_h_ts(acc, a_tmem + 16 * pa + 8 * ks, bk, id, (fresh && ks == 0) ? 0u : 1u);
         }
     };
-    product(1, 0, true);                             // lo x hi (WIDE: lo x [hi | lo])
+    if (!WIDE && LOLO) product(1, 1, true);
+    product(1, 0, WIDE || !LOLO);                    // lo x hi (WIDE: lo x [hi | lo])
     if (!WIDE) product(0, 1, false);                 // hi x lo
     product(0, 0, false);                            // hi x hi (WIDE: hi x [hi | lo])
 }
@@ -412,7 +415,7 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
                 tc_fence_after();
                 const uint32_t s0 = tmem + (uint32_t)((i & 1) * 2 * kTile), kt = smem_u32(k_s + k_slot(i) * TB);
                 const int half = first ? 0 : 1;
-                issue_accumulate<D, C::kWide>(tmem + C::kColAcc + 64 * half, s0 + 32 * half, kt, half);
+                issue_accumulate<D, C::kWide, STORED != 0>(tmem + C::kColAcc + 64 * half, s0 + 32 * half, kt, half);
                 if (elect_one()) tc_commit(&acc_done[i & 1]);
             }
         }
@@ -740,7 +743,7 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
             if (!first) fetch_w(i + C::kStages);     // ... and its rows' statistics
             const uint32_t s0 = tmem + (uint32_t)(i & 1) * C::kBuf, t = smem_u32(t_s + (i % C::kStages) * 2 * TB);
             for (int half = 0; half < 2; ++half)
-                issue_accumulate<D, C::kWide>(tmem + (first ? C::kColV : C::kColK) + 64 * half, s0 + (first ? 0 : kTile) + 32 * half, first ? t + TB : t, half);
+                issue_accumulate<D, C::kWide, STORED != 0>(tmem + (first ? C::kColV : C::kColK) + 64 * half, s0 + (first ? 0 : kTile) + 32 * half, first ? t + TB : t, half);
             if (elect_one()) tc_commit(&acc_done[i & 1]);
         }
         __syncwarp();
