@@ -15,10 +15,10 @@
 // largest there, ds's from a bound by row (largest P |dP|, and largest P times |w|), at most twice what ds reaches.
 // The queries of the other block contribute to this block's keys: their sums come through distributed shared memory at the end.
 //
-// Measured, us, three kernels -> one: B=32 H=8 S=256 D=32 with stored probabilities 90.4 -> 63.6, causal without 78.5 -> 62.5; B=16 H=12 S=128 D=32
+// Measured, us, three kernels -> one: B=32 H=8 S=256 D=32 with stored probabilities 90.4 -> 64.1, causal without 78.5 -> 62.5; B=16 H=12 S=128 D=32
 // stored 28.9 -> 20.4; B=64 H=12 S=35 68.2 -> 53.1; D=64: B=32 H=8 S=128 stored 41.8 -> 29.6, causal without 45.8 -> 29.9; B=9 H=16 S=101 25.0 -> 14.6.
-// There is no length in its range at which the three are faster.  Relative error of the gradients against float64: 1.5e-7, 1.5e-7, 1.0e-7 (dQ, dK, dV) at the
-// first, 1.8e-7, 1.9e-7, 1.6e-7 at the second.
+// There is no length in its range at which the three are faster.  Relative error of the gradients against float64: 1.45, 1.39, 1.03e-7 (dQ, dK, dV) at the
+// first, 1.8, 1.9, 1.6e-7 at the second (with stored probabilities the products of the low pieces are formed too: without, 1.51, 1.46, 1.03e-7 and 63.5 us instead of 64.1).
 // What bounds it: a block takes 15 us at the first shape, 3.5 rounds of them.  5 until its operands are cut (224 KB come in at 64 bytes
 // per clock; the cut is bound by the instructions of conversion), 2 for w, 3 for ds and P's pieces, 2.5 for ds's, 1.5 for the last product and the other
 // block's sums, 1 for the output.  In the sweeps the conversions and the shared memory's width (512 cycles each per tile) share the time.
@@ -162,12 +162,13 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
         auto scores = [&](uint32_t d, const uint8_t *as, const uint8_t *bs) {
             const uint64_t da = make_desc(smem_u32(as), 128, Img<D>::kBlock, 0), db = make_desc(smem_u32(bs), 128, Img<D>::kBlock, 0);
             constexpr uint32_t id = idesc_f16(kLanes, kLanes);
-            constexpr int PA[3] = {1, 0, 0}, PB[3] = {0, 1, 0};          // small terms first
+            constexpr int PA[4] = {1, 1, 0, 0}, PB[4] = {1, 0, 1, 0};    // small terms first; the smallest where the probabilities, stored, are exact
 #pragma unroll
-            for (int p = 0; p < 3; ++p)
+            for (int p = STORED ? 0 : 1; p < 4; ++p)
 #pragma unroll
                 for (int ks = 0; ks < D / 16; ++ks)
-                    if (elect_one()) mma_h_ss(d, da + (uint64_t)((PA[p] * (D / 8) + 2 * ks) * 8), db + (uint64_t)((PB[p] * (D / 8) + 2 * ks) * 8), id, (p | ks) ? 1u : 0u);
+                    if (elect_one())
+                        mma_h_ss(d, da + (uint64_t)((PA[p] * (D / 8) + 2 * ks) * 8), db + (uint64_t)((PB[p] * (D / 8) + 2 * ks) * 8), id, p > (STORED ? 0 : 1) || ks > 0 ? 1u : 0u);
         };
         // acc (128 x D; WIDE: 2 D, the products with B's lo pieces apart) = A B over 64 rows of B's image, read N-major.  da: the descriptor of A's hi
         // pieces; a_step: 16 reductions on, in 16 bytes; id: A K- or M-major.  The small products first, a fresh accumulator per 64.
