@@ -7,9 +7,9 @@
 // such sums is formed from three products of the pieces, lo hi, hi lo, hi hi, which the tensor core multiplies exactly and adds in
 // fp32 (lo lo, below 2^-22 of the product, where it comes in the same instruction).  The tensor core truncates where it adds to its
 // accumulator; what that takes on the average is given back at the end.  Before, three bf16 pieces and six products: twice the instructions and half as
-// many bytes more per operand (B=3 H=12 S=777 D=64 causal 117 -> 79 us, B=32 H=8 S=256 D=32 with stored probabilities 97 -> 89.5), and the relative error of all
-// three gradients against float64 no smaller: 2.8e-7 then and 2.1e-7 now at the first shape, 1.40e-7 and 1.28e-7 at the second (0.6 - 1.0 of what it was
-// over eleven shapes of S = 77 ... 1024; dV alone, with stored probabilities at D = 64, 0.93e-7 -> 1.09e-7).
+// many bytes more per operand (B=3 H=12 S=777 D=64 causal 117 -> 79 us, B=2 H=16 S=1024 D=64 with stored probabilities 208 -> 144), and the relative error of the
+// gradients against float64 no smaller: 2.8e-7 then and 2.1e-7 now at the first shape (dQ), 1.72 and 1.60e-7 at the second.  Only dV with stored probabilities is a little
+// farther off (1.10 and 1.16e-7 there), and dK as much nearer (1.78 and 1.57e-7).
 // Powers of two: one per 64-row tile for Q, K, V and dO, kept beside the images; for P and ds, which are formed in fp32 in registers,
 // one per thread (32 columns of a row or key of a tile).  An accumulator holds one tile and one half of its columns, and the factors leave
 // where the workers add it to the running sum; those of a tile's scores go into the multiply-adds that form P and ds.  A value
