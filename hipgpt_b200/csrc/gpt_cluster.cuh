@@ -62,6 +62,14 @@ __host__ __device__ constexpr ClusterJob cluster_job_of(int i, int E, int V)
     return i == kJobQkv ? cluster_job(3 * E, E, 1) : i == kJobO ? cluster_job(E, E, 0) : i == kJobF1 ? cluster_job(4 * E, E, 1) : i == kJobF2 ? cluster_job_by_segment(E, 4 * E)
                                                                                                                           : cluster_job(V, E, 0);
 }
+// Columns of the second feed-forward product whose partial sums come to block `rank`.  Shares are whole fours, so the last blocks may have none
+// (E = 160, 224: two of them; 288, 352: one).  Such a block takes no part in that hop: a phase that expects no bytes is complete when it is
+// opened, and who tests for it after the next one has been opened sees neither.
+__host__ __device__ constexpr int cluster_f2_columns(int E, int rank)
+{
+    const int nc = cluster_job_of(kJobF2, E, 16).nc, left = E - rank * nc;
+    return left < 0 ? 0 : left < nc ? left : nc;
+}
 
 struct ClusterPlan {
     ClusterJob voc;

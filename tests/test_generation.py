@@ -1,5 +1,8 @@
 """Greedy KV-cache generation: the CPU oracle against plain numpy on a tiny model (CPU), and the
 GPU driver against the oracle: token ids must be identical, logits within 1e-4."""
+import os
+import subprocess
+
 import numpy as np
 import pytest
 
@@ -160,6 +163,71 @@ def test_gpu_generation_by_clusters_at_its_edges(cfg, B, n_prompt, n_new):
     dec = generation.GptDecoder(w, **cfg, max_batch=B)
     for _ in range(2):
         ids, logits, _, _ = dec.generate(prompts, n_new)
+        assert np.array_equal(ids, ref_ids)
+        assert float(np.abs(logits - ref_logits).max()) <= 1e-4
+    dec.close()
+
+
+_F2_HOP = r"""
+#include "gpt_cluster.cuh"
+#include <cstdio>
+using namespace hipgpt;
+// A barrier of one arrival: the phase it is in, complete once it has been opened and the bytes it expects have come.
+struct Barrier {
+    int phase = 0, bytes = 0;
+    bool opened = false;
+    void open(int expect) { opened = true; bytes += expect; settle(); }
+    void come(int n) { bytes -= n; settle(); }
+    void settle() { if (opened && bytes == 0) { ++phase; opened = false; } }
+    bool test(int parity) const { return (phase & 1) != parity; }
+};
+int main()
+{
+    int bad = 0;
+    for (int E = 128; E <= 384; E += 32)
+        for (int rank = 0; rank < kClusterBlocks; ++rank) {
+            const int own = cluster_f2_columns(E, rank);
+            const bool waits = HIPGPT_TEST_WAITS;
+            Barrier b;
+            if (waits) b.open(64 * own);
+            for (int layer = 0; layer < 6 && waits; ++layer) {
+                b.come(64 * own);                    // the sixteen blocks' partial sums
+                // the last warp comes first: it sees its phase and opens the next one
+                bad += !b.test(layer & 1);
+                b.open(64 * own);
+                bad += !b.test(layer & 1);           // a warp that adds up, after it
+            }
+            if (!waits && own) ++bad;
+        }
+    std::printf("%d\n", bad);
+}
+"""
+
+
+@pytest.mark.parametrize("waits,ok", [("own > 0", True), ("true", False)])
+def test_generation_by_clusters_no_block_waits_for_sums_that_nobody_sends(tmp_path, waits, ok):
+    """The second feed-forward product's hop with the last warp ahead of those that add up: blocks with columns see their phase whatever the order; a
+    block without would look for one that has come and gone (which is why it stays out of the hop)."""
+    from hipgpt_b200 import build
+    src, exe = tmp_path / "hop.cu", tmp_path / "hop"
+    src.write_text(_F2_HOP)
+    subprocess.run([build.nvcc(), *build.ARCH, "-std=c++17", f"-DHIPGPT_TEST_WAITS=({waits})", "-I", build.CSRC, "-I", os.path.join(build.ROOT, "include"), str(src), "-o", str(exe)], check=True)
+    assert (int(subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout) == 0) is ok
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("E,B", [(160, 1), (160, 9), (224, 9), (288, 1), (352, 2), (352, 9)])
+def test_gpu_generation_by_clusters_with_blocks_that_own_no_columns(E, B):
+    """Widths whose last blocks have no column of the second feed-forward product, one sequence per cluster and two, many layers and positions."""
+    pytest.importorskip("torch")
+    from hipgpt_b200 import generation
+    cfg = dict(V=200, S=72, E=E, L=5, H=E // 32, F=4 * E)
+    w = synth.gpt_weights(41, **cfg, std=0.05)
+    prompts = synth.token_ids(42, (B, 3), cfg["V"])
+    ref_ids, ref_logits = ob.gpt_generate(w, **cfg, prompts=prompts, n_new=64, fma=True)
+    dec = generation.GptDecoder(w, **cfg, max_batch=B)
+    for _ in range(4):
+        ids, logits, _, _ = dec.generate(prompts, 64)
         assert np.array_equal(ids, ref_ids)
         assert float(np.abs(logits - ref_logits).max()) <= 1e-4
     dec.close()
