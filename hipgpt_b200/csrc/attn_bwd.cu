@@ -235,12 +235,12 @@ int launch_bwd_cfg(const float *g, const float *q, const float *k, const float *
 size_t mha_backward_scratch_bytes(int B, int H, int S) { return (size_t)2 * B * H * S * sizeof(float); }
 
 int launch_mha_backward(const float *g, const float *q, const float *k, const float *v, const float *probs,
-                        float *dq, float *dk, float *dv, float *scratch, int B, int S, int E, int H, int causal, cudaStream_t st)
+                        float *dq, float *dk, float *dv, float *scratch, int B, int S, int E, int H, int causal, bool tensor, cudaStream_t st)
 {
     const int D = E / H;
     if (D > kBwdMaxD) return fail(HIPGPT_ERR_UNSUPPORTED, "attention backward: head_dim %d exceeds %d", D, kBwdMaxD);
     if (B == 0 || S == 0) return HIPGPT_OK;
-    if (mha_backward_tc_supports(g, q, k, v, probs, dq, dk, dv, B, S, E, H))
+    if (tensor)
         return launch_mha_backward_tc(g, q, k, v, probs, dq, dk, dv, B, S, E, H, causal, st);
 #define HIPGPT_BWD(DP) (causal ? launch_bwd_cfg<DP, true>(g, q, k, v, probs, dq, dk, dv, scratch, B, S, E, H, st) \
                                : launch_bwd_cfg<DP, false>(g, q, k, v, probs, dq, dk, dv, scratch, B, S, E, H, st))

@@ -11,8 +11,9 @@
 //   dP = g V^T     256 columns of TMEM, formed once.  ds takes their place in fp32, and when the pieces of P have been read, ds's
 //                  pieces take theirs, where they serve both products: read K-major for dQ = ds K, M-major for dK = ds^T Q.
 // so that the sweeps of the workers (w; ds and P's pieces; ds's pieces) run over whole rows with no product to wait for inside.
-// The pieces of P and ds are cut by one power of two per 64 queries (the reduction of dV and dK runs over queries): P's from its
-// largest there, ds's from a bound by row (largest P |dP|, and largest P times |w|), at most twice what ds reaches.
+// The pieces of P and ds are cut by one power of two per tile of 64 queries x 64 keys, which can leave with a row of dQ's sums (kept per tile of keys) and with
+// one of dV's and dK's (kept per 64 queries): P's from its largest there, ds's from an upper bound by row (largest P |dP|, and largest P times |w|).
+// The bound is no estimate: where a row has all its weight on one key it is 2 |w| and ds near zero.  The pieces' range (attn_bwd_pieces.cuh) is what covers that.
 // The queries of the other block contribute to this block's keys: their sums come through distributed shared memory at the end.
 //
 // Measured, us, three kernels -> one: B=32 H=8 S=256 D=32 with stored probabilities 90.4 -> 64.1, causal without 78.5 -> 62.5; B=16 H=12 S=128 D=32
@@ -93,7 +94,7 @@ struct HeadSmall {
     uint64_t p_full[2 * NB], scores, asked, cut[2], p_read[NB], p_ready[NB], v_done[NB], d_ready[NB], k_done[NB];
     alignas(16) uint32_t largest[4 + 4 * NB][8];                // of a tile's rows that a warp has
     float fac[4 + 4 * NB];
-    uint32_t group_p[4], group_d[4];                 // per lane quarter: P's largest, ds's bound
+    uint32_t group_p[2 * NB][2], group_d[2 * NB][2]; // of a tile of 64 queries (second index) x 64 keys: P's largest, ds's bound
     uint32_t tmem_base;
     volatile int abort_flag, peer_gone;
 };
@@ -123,6 +124,7 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
     if (tid == 0) {
         sh.abort_flag = 0;
         sh.peer_gone = 0;
+        for (int t = 0; t < 2 * NB; ++t) sh.group_p[t][0] = sh.group_p[t][1] = sh.group_d[t][0] = sh.group_d[t][1] = 0;
         for (int i = 0; i < 2 * NB; ++i) mbar_init(&sh.p_full[i], 1);
         mbar_init(&sh.scores, 2);                    // (commits: one per issuing warp)
         for (int i = 0; i < 2; ++i) mbar_init(&sh.cut[i], kWorkerWarps);
@@ -167,23 +169,30 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
             for (int p = STORED ? 0 : 1; p < 4; ++p)
 #pragma unroll
                 for (int ks = 0; ks < D / 16; ++ks)
-                    if (elect_one())
-                        mma_h_ss(d, da + (uint64_t)((PA[p] * (D / 8) + 2 * ks) * 8), db + (uint64_t)((PB[p] * (D / 8) + 2 * ks) * 8), id, p > (STORED ? 0 : 1) || ks > 0 ? 1u : 0u);
+                    if (elect_one()) {
+                        const uint64_t ak = da + (uint64_t)((PA[p] * (D / 8) + 2 * ks) * 8), bk = db + (uint64_t)((PB[p] * (D / 8) + 2 * ks) * 8);
+                        if (ks == 0 && (p == 3 || (STORED && p == 1))) mma_h_ss_down<kLowShift>(d, ak, bk, id);
+                        else mma_h_ss(d, ak, bk, id, p > (STORED ? 0 : 1) || ks > 0 ? 1u : 0u);
+                    }
         };
         // acc (128 x D; WIDE: 2 D, the products with B's lo pieces apart) = A B over 64 rows of B's image, read N-major.  da: the descriptor of A's hi
         // pieces; a_step: 16 reductions on, in 16 bytes; id: A K- or M-major.  The small products first, a fresh accumulator per 64.
         auto sums = [&](uint32_t acc, uint64_t da, int a_step, uint32_t id, const uint8_t *bs) {
             const uint64_t db = make_desc(smem_u32(bs), Img<D>::kBlock, 128, 0);
-            auto product = [&](int pa, int pb, bool fresh) {
+            enum { kFresh, kDown, kMore };           // how a product finds the accumulator
+            auto product = [&](int pa, int pb, int start) {
 #pragma unroll
                 for (int ks = 0; ks < 4; ++ks)
-                    if (elect_one()) mma_h_ss(acc, da + (uint64_t)(pa * (kPiecePart >> 4) + ks * a_step), db + (uint64_t)(ks * 2 * (Img<D>::kBlock >> 4) + pb * (Img<D>::kPiece >> 4)), id,
-                                              fresh && ks == 0 ? 0u : 1u);
+                    if (elect_one()) {
+                        const uint64_t ak = da + (uint64_t)(pa * (kPiecePart >> 4) + ks * a_step), bk = db + (uint64_t)(ks * 2 * (Img<D>::kBlock >> 4) + pb * (Img<D>::kPiece >> 4));
+                        if (start == kDown && ks == 0) mma_h_ss_down<kLowShift>(acc, ak, bk, id);
+                        else mma_h_ss(acc, ak, bk, id, start == kFresh && ks == 0 ? 0u : 1u);
+                    }
             };
-            if (!C::kWide && STORED) product(1, 1, true);        // (WIDE has it in any case.  Formed probabilities carry more than it takes away)
-            product(1, 0, C::kWide || !STORED);
-            if (!C::kWide) product(0, 1, false);
-            product(0, 0, false);
+            if (!C::kWide && STORED) product(1, 1, kFresh);      // (WIDE has it in any case.  Formed probabilities carry more than it takes away)
+            product(1, 0, C::kWide || !STORED ? kFresh : kDown);
+            if (!C::kWide) product(0, 1, kMore);
+            product(0, 0, kDown);
         };
         constexpr uint32_t id_sums = idesc_f16(kLanes, C::kWide ? 2 * D : D) | (1u << 16);
         // the M-major image of 128 keys: A of dV and dK
@@ -362,11 +371,11 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
     tc_fence_after();
 
     // First sweep: maximum and sum of the exponentials (where P is formed here), w, and the largest P and P |dP| of the row
-    float m = -INFINITY, l = 0.0f, w = 0.0f, rinv = 1.0f, most_p = 0.0f, most_d = 0.0f;
+    float m = -INFINITY, l = 0.0f, w = 0.0f, rinv = 1.0f, most_p[C::kTiles], most_d[C::kTiles];
     if (!STORED) {
         for (int t = 0; t < ntile; ++t) {
             const int nvalid = count(t);
-            const float s_fac = fmaxf(q_fac * sh.fac[C::tK + t], 1e-37f);        // (never zero: a hidden score is -inf, and times the factor it stays that)
+            const float s_fac = fminf(fmaxf(q_fac * sh.fac[C::tK + t], 1e-37f), kFacMost);        // (never zero: a hidden score is -inf, and times the factor it stays that)
             float s[kCols];
             tmem_ld16(my_tile + C::kColAcc + t * kTile, s);
             tmem_wait_ld();
@@ -380,9 +389,12 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
         meet();
         m = fmaxf(fmaxf(fmaxf(comb[0][0][rloc], comb[0][1][rloc]), fmaxf(comb[0][2][rloc], comb[0][3][rloc])), -1e30f);
     }
-    for (int t = 0; t < ntile; ++t) {
+#pragma unroll
+    for (int t = 0; t < C::kTiles; ++t) {
+        most_p[t] = most_d[t] = 0.0f;
+        if (t >= ntile) continue;
         const int nvalid = count(t);
-        const float dp_fac = g_fac * sh.fac[C::tV + t];
+        const float dp_fac = fminf(g_fac * sh.fac[C::tV + t], kFacMost);
         float p[kCols], dp[kCols];
         if (STORED && by_tma) wait(&sh.p_full[t], 0, 22);
         if (STORED) read_p(t, p);
@@ -394,7 +406,7 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
         if (STORED) {
             mask(p, nvalid, 0.0f);
         } else {
-            const float s_fac = fmaxf(q_fac * sh.fac[C::tK + t], 1e-37f);
+            const float s_fac = fminf(fmaxf(q_fac * sh.fac[C::tK + t], 1e-37f), kFacMost);
             mask(p, nvalid, -INFINITY);
 #pragma unroll
             for (int i = 0; i < kCols; i += 2) {
@@ -417,35 +429,33 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
             md[z] = max3(md[z], fabsf(pd.x), fabsf(pd.y));
         }
         w = fmaf((ws[0].x + ws[0].y) + (ws[1].x + ws[1].y), dp_fac, w);
-        most_p = max3(most_p, mp[0], mp[1]);
-        most_d = fmaxf(most_d, fmaxf(md[0], md[1]) * dp_fac);
+        most_p[t] = fmaxf(mp[0], mp[1]);
+        most_d[t] = fmaxf(md[0], md[1]) * dp_fac;
     }
     {
         comb[1][cf][rloc] = w;
-        comb[2][cf][rloc] = most_p;
-        comb[3][cf][rloc] = most_d;
-        if (!STORED) comb[4][cf][rloc] = l;
+        if (!STORED) comb[2][cf][rloc] = l;
         meet();
         w = (comb[1][0][rloc] + comb[1][1][rloc]) + (comb[1][2][rloc] + comb[1][3][rloc]);
         if (!STORED) {
-            rinv = 1.0f / fmaxf((comb[4][0][rloc] + comb[4][1][rloc]) + (comb[4][2][rloc] + comb[4][3][rloc]), 1e-30f);
+            rinv = 1.0f / fmaxf((comb[2][0][rloc] + comb[2][1][rloc]) + (comb[2][2][rloc] + comb[2][3][rloc]), 1e-30f);
             w *= rinv;
         }
-        if (cf == 0) {
-            // (finite ones only; whatever is in a row with an infinity or a NaN stays in it)
-            most_p = fmaxf(fmaxf(most_p, comb[2][1][rloc]), fmaxf(comb[2][2][rloc], comb[2][3][rloc])) * rinv;
-            most_d = fmaxf(fmaxf(most_d, comb[3][1][rloc]), fmaxf(comb[3][2][rloc], comb[3][3][rloc])) * rinv;
-            uint32_t bp = __float_as_uint(most_p), bd = __float_as_uint(fmaf(most_p, fabsf(w), most_d));
+        // (finite ones only; whatever is in a row with an infinity or a NaN stays in it)
+#pragma unroll
+        for (int t = 0; t < C::kTiles; ++t) {
+            if (t >= ntile) break;
+            uint32_t bp = __float_as_uint(most_p[t] * rinv), bd = __float_as_uint(fmaf(most_p[t], fabsf(w), most_d[t]) * rinv);
             bp = __reduce_max_sync(0xffffffffu, bp < 0x7f800000u ? bp : 0u);
             bd = __reduce_max_sync(0xffffffffu, bd < 0x7f800000u ? bd : 0u);
-            if (lane == 0) { sh.group_p[wq] = bp; sh.group_d[wq] = bd; }
+            if (lane == 0) { atomicMax(&sh.group_p[t][u], bp); atomicMax(&sh.group_d[t][u], bd); }
         }
         meet();
     }
     if (NB > 1) cluster_arrive();                    // V's image is this block's no longer: the other one's sums may come
-    const uint32_t e_p[2] = {range_exponent(max(sh.group_p[0], sh.group_p[1])), range_exponent(max(sh.group_p[2], sh.group_p[3]))};
-    const uint32_t e_d[2] = {range_exponent(max(sh.group_d[0], sh.group_d[1])), range_exponent(max(sh.group_d[2], sh.group_d[3]))};
-    const float up_p = range_up(u ? e_p[1] : e_p[0]), up_d = range_up(u ? e_d[1] : e_d[0]);
+    // exponents of a tile: of its probabilities and of its ds (at most 2^100 below the probabilities': the ratio of the factors stays a number)
+    auto e_p = [&](int t, int y) { return range_exponent(sh.group_p[t][y]); };
+    auto e_d = [&](int t, int y) { const uint32_t p = e_p(t, y), d = range_exponent(sh.group_d[t][y]); return p > d + (100u << 23) ? p - (100u << 23) : d; };
 
     // Second sweep: ds, scaled, in fp32 in dP's place; P's pieces in P's.  A block of keys' probabilities are read first: eight warps share the memory
     // that each of them then writes its pieces to (a meeting per tile, between reading and writing it, kept them all in the same step: 1300 cycles per tile).
@@ -470,14 +480,15 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
         arrive(&sh.p_read[i]);
     };
     read_block(0);
-    const float up_row = STORED ? up_p : rinv * up_p, ratio = up_d * range_down(u ? e_p[1] : e_p[0]), w_up = w * ratio;
     for (int i = 0; i < nkb; ++i) {
         const int kb = block_at(i);
 #pragma unroll
         for (int y = 0; y < 2; ++y) {
             const int t = 2 * kb + y;
             if (t >= ntile) break;
-            const float dp_up = g_fac * sh.fac[C::tV + t] * ratio;
+            const uint32_t ep = e_p(t, u);
+            const float up_row = STORED ? range_up(ep) : rinv * range_up(ep), ratio = range_up(e_d(t, u)) * range_down(ep);
+            const float dp_up = fminf(g_fac * sh.fac[C::tV + t], kFacMost) * ratio, w_up = w * ratio;
             float dp[kCols];
             tmem_ld16(my_tile + t * kTile, dp);
             if (STORED) mask(p[y], count(t), 0.0f);
@@ -506,7 +517,7 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
         if constexpr (OC == 8) tmem_ld8(at, x);
         else tmem_ld16(at, x);
     };
-    // sums over the two 64's of queries: accumulators times their factors
+    // sums over the two 64's of queries: accumulators times their factors (this thread's key is in tile 2 kb + u)
     auto key_sums = [&](uint32_t acc, float f0, float f1, float (&o)[OC]) {
         float a[2][OC], z[2][OC];
 #pragma unroll
@@ -517,7 +528,7 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
         tmem_wait_ld();
 #pragma unroll
         for (int x = 0; x < OC; ++x) {
-            if (C::kWide) { a[0][x] += z[0][x]; a[1][x] += z[1][x]; }
+            if (C::kWide) { a[0][x] = fmaf(z[0][x], kLowDown, a[0][x]); a[1][x] = fmaf(z[1][x], kLowDown, a[1][x]); }
             o[x] = fmaf(a[1][x], f1, a[0][x] * f0);
         }
     };
@@ -548,7 +559,7 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
             tmem_wait_ld();
             store_pieces(t, d, [] {});
         }
-        key_sums(lane_base + C::kColAcc + kb * 128, range_down(e_p[0]) * sh.fac[C::tG], range_down(e_p[1]) * sh.fac[C::tG + 1], ov);
+        key_sums(lane_base + C::kColAcc + kb * 128, range_down(e_p(2 * kb + u, 0)) * sh.fac[C::tG], range_down(e_p(2 * kb + u, 1)) * sh.fac[C::tG + 1], ov);
         proxy_fence();
         tc_fence_before();
         arrive(&sh.d_ready[i]);
@@ -559,14 +570,13 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
         }
     }
     // dK; dQ from the tiles' sums, a block of keys after the other
-    const float d_down = range_down(u ? e_d[1] : e_d[0]);
 #pragma unroll
     for (int x = 0; x < OC; ++x) oq[x] = 0.0f;
     for (int i = 0; i < nkb; ++i) {
         const int kb = block_at(i);
         wait(&sh.k_done[i], 0, 26);
         tc_fence_after();
-        key_sums(lane_base + C::kColAcc + C::kColK + kb * 128, range_down(e_d[0]) * sh.fac[C::tQ], range_down(e_d[1]) * sh.fac[C::tQ + 1], ok);
+        key_sums(lane_base + C::kColAcc + C::kColK + kb * 128, range_down(e_d(2 * kb + u, 0)) * sh.fac[C::tQ], range_down(e_d(2 * kb + u, 1)) * sh.fac[C::tQ + 1], ok);
         if (NB > 1 && i == 0) {                      // (every block takes both steps of the cluster's barrier twice)
             if (!joined) cluster_wait();
             if (kb != blk) {
@@ -590,9 +600,9 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
 #pragma unroll
         for (int y = 0; y < 2; ++y) {
             if (2 * kb + y >= ntile) break;
-            const float f = d_down * sh.fac[C::tK + 2 * kb + y];
+            const float f = range_down(e_d(2 * kb + y, u)) * sh.fac[C::tK + 2 * kb + y];
 #pragma unroll
-            for (int x = 0; x < OC; ++x) oq[x] = fmaf(C::kWide ? a[y][x] + z[y][x] : a[y][x], f, oq[x]);
+            for (int x = 0; x < OC; ++x) oq[x] = fmaf(C::kWide ? fmaf(z[y][x], kLowDown, a[y][x]) : a[y][x], f, oq[x]);
         }
     }
     // 32 rows x 32 columns leave in whole lines: through shared memory (16-byte pieces permuted by the row), then a row of 128 bytes per eight lanes

@@ -19,13 +19,17 @@ struct Img {
     static constexpr int kTileBytes = (kTile / 8) * kBlock;     // 64 rows
 };
 
-// Two fp32 numbers below 2^16 -> two words of two fp16 each whose sums are the numbers (to 2^-23 of them, 2^-25 where that is more).
+// Two fp32 numbers up to 2^15 -> two words of two fp16 each, hi and 2^12 times what hi leaves: hi + 2^-12 lo is the number to 2^-23 of it
+// down to 2^-14, to 2^-37 below.  (Without the factor the low piece ran into fp16's smallest numbers at 2^-2 already.)  The products with one low piece are 2^12
+// times too large then, that of two 2^24: the tensor core brings the accumulator down where the next larger products start.
 // An infinity leaves a NaN.
+constexpr int kLowShift = 12;
+constexpr float kLowUp = 4096.0f, kLowDown = 1.0f / 4096.0f;
 __device__ __forceinline__ void cut2(float2 x, uint32_t &h, uint32_t &l)
 {
     const __half2 hh = __float22half2_rn(x);
     const float2 back = __half22float2(hh);
-    const __half2 ll = __float22half2_rn(ffma2(back, make_float2(-1.0f, -1.0f), x));
+    const __half2 ll = __float22half2_rn(fmul2(ffma2(back, make_float2(-1.0f, -1.0f), x), make_float2(kLowUp, kLowUp)));
     h = *reinterpret_cast<const uint32_t *>(&hh);
     l = *reinterpret_cast<const uint32_t *>(&ll);
 }
@@ -35,6 +39,8 @@ __device__ __forceinline__ void cut2(float2 x, uint32_t &h, uint32_t &l)
 __device__ __forceinline__ uint32_t range_exponent(uint32_t bits) { return max(bits & 0x7f800000u, 27u << 23); }
 __device__ __forceinline__ float range_up(uint32_t e) { return __uint_as_float((268u << 23) - e); }
 __device__ __forceinline__ float range_down(uint32_t e) { return __uint_as_float(e - (14u << 23)); }
+// The most that two such factors make together: not infinite, so that a row of zeros stays one beside rows whose scores leave fp32
+constexpr float kFacMost = 1e38f;
 
 }  // namespace
 }  // namespace hipgpt

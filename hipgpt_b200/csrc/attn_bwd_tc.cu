@@ -1,5 +1,5 @@
 // Attention backward on the Blackwell tensor pipe (tcgen05 + TMEM), head_dim 32 or 64, any sequence length, with the accuracy of
-// fp32 products.  Same contract as attn_bwd.cu (HipGPT src/hip_kernels.cpp:1162-1272), which keeps every other head_dim:
+// fp32 sums over the range that is stated below.  Same contract as attn_bwd.cu (HipGPT src/hip_kernels.cpp:1162-1272), which keeps every other head_dim:
 //     vd_ij = g_i . V_j            w_i  = sum_j P_ij vd_ij        ds_ij = P_ij (vd_ij - w_i)
 //     dQ_i  = c sum_j ds_ij K_j    dK_j = c sum_i ds_ij Q_i       dV_j  = sum_i P_ij g_i
 //
@@ -12,8 +12,10 @@
 // farther off (1.10 and 1.16e-7 there), and dK as much nearer (1.78 and 1.57e-7).
 // Powers of two: one per 64-row tile for Q, K, V and dO, kept beside the images; for P and ds, which are formed in fp32 in registers,
 // one per thread (32 columns of a row or key of a tile).  An accumulator holds one tile and one half of its columns, and the factors leave
-// where the workers add it to the running sum; those of a tile's scores go into the multiply-adds that form P and ds.  A value
-// keeps its 22 bits down to 2^-15 of the largest of its tile, below that what the largest leaves of it: 2^-39 of that one.
+// where the workers add it to the running sum; those of a tile's scores go into the multiply-adds that form P and ds.  The low piece is kept 2^12 times too
+// large (the tensor core brings the accumulator down by as much between the products), so that a value keeps its 23 bits down to 2^-29 of the largest of its
+// tile, and below that what the largest leaves of it: 2^-52 of that one.  (With both pieces at one scale: 2^-15 and 2^-39; a row of dO 2^-30 below its
+// neighbours gave nine bits of dQ.  The times are the same: B=3 H=12 S=777 D=64 causal 79.0 -> 79.6 us.)
 //
 // Three kernels per group of batches:
 //   bwd_pack_kernel   Q, K, V, dO -> their pieces, once per call, in the order in which shared memory holds an operand: 8 x 8 core
@@ -128,12 +130,15 @@ __device__ __forceinline__ void issue_scores(uint32_t d_tmem, uint32_t a_smem, u
 #pragma unroll
         for (int k = 0; k < D / 16; ++k) {
             const uint64_t da = a + (uint64_t)((PA[p] * (D / 8) + 2 * k) * 8), db = b + (uint64_t)((PB[p] * (D / 8) + 2 * k) * 8);
-            if (elect_one()) mma_h_ss(d_tmem, da, db, id, (p | k) ? 1u : 0u);
+            if (elect_one()) {
+                if (p == 2 && k == 0) mma_h_ss_down<kLowShift>(d_tmem, da, db, id);
+                else mma_h_ss(d_tmem, da, db, id, (p | k) ? 1u : 0u);
+            }
         }
 }
 
 // acc[tmem] (128 x D) = A B over rows [32 hf, 32 hf + 32) of B's image, read N-major; A: two pieces in TMEM, 16 columns each, hi first.
-// WIDE: acc is 2 D columns, the second half collects the products with B's lo pieces (wider instructions, fewer of them).  The
+// WIDE: acc is 2 D columns, the second half collects the products with B's lo pieces, 2^12 times (wider instructions, fewer of them).  The
 // small products come first: the tensor core truncates where it adds to its accumulator, so the accumulator should be small
 // while they are added, and it starts anew for every tile (the workers add the tiles up in registers).  One accumulator over all
 // tiles was 10 times farther from float64 at S = 777.
@@ -144,17 +149,22 @@ __device__ __forceinline__ void issue_accumulate(uint32_t acc, uint32_t a_tmem, 
 {
     const uint64_t b = make_desc(b_smem, Img<D>::kBlock, 128, 0) + (uint64_t)(hf * 4 * (Img<D>::kBlock >> 4));
     constexpr uint32_t id = idesc_f16(kLanes, WIDE ? 2 * D : D) | (1u << 16);
-    auto product = [&](int pa, int pb, bool fresh) {
+    enum { kFresh, kDown, kMore };                   // how a product finds the accumulator
+    auto product = [&](int pa, int pb, int start) {
 #pragma unroll
         for (int ks = 0; ks < 2; ++ks) {
             const uint64_t bk = b + (uint64_t)(ks * 2 * (Img<D>::kBlock >> 4) + pb * (Img<D>::kPiece >> 4));
-            if (elect_one()) mma_h_ts(acc, a_tmem + 16 * pa + 8 * ks, bk, id, (fresh && ks == 0) ? 0u : 1u);
+            const uint32_t ak = a_tmem + 16 * pa + 8 * ks;
+            if (elect_one()) {
+                if (start == kDown && ks == 0) mma_h_ts_down<kLowShift>(acc, ak, bk, id);
+                else mma_h_ts(acc, ak, bk, id, (start == kFresh && ks == 0) ? 0u : 1u);
+            }
         }
     };
-    if (!WIDE && LOLO) product(1, 1, true);
-    product(1, 0, WIDE || !LOLO);                    // lo x hi (WIDE: lo x [hi | lo])
-    if (!WIDE) product(0, 1, false);                 // hi x lo
-    product(0, 0, false);                            // hi x hi (WIDE: hi x [hi | lo])
+    if (!WIDE && LOLO) product(1, 1, kFresh);
+    product(1, 0, WIDE || !LOLO ? kFresh : kDown);   // lo x hi (WIDE: lo x [hi | lo])
+    if (!WIDE) product(0, 1, kMore);                 // hi x lo
+    product(0, 0, kDown);                            // hi x hi (WIDE: hi x [hi | lo])
 }
 
 // 32 numbers of a row (or key), scaled by a power of two of their own -> their two pieces in 32 TMEM columns, hi first.  Returns one
@@ -197,7 +207,7 @@ __device__ __forceinline__ void add_tile(uint32_t acc, int hf, float f0, float f
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
                 y[u] = make_float2(a[u][c], a[u][c + 1]);
-                if (WIDE) y[u] = fadd2(y[u], make_float2(b[u][c], b[u][c + 1]));
+                if (WIDE) y[u] = ffma2(make_float2(b[u][c], b[u][c + 1]), make_float2(kLowDown, kLowDown), y[u]);
             }
             // (the halves first: one addition to the long sum per tile)
             const float2 t = fadd2(make_float2(o[c0 + c], o[c0 + c + 1]), ffma2(y[1], make_float2(f1, f1), fmul2(y[0], make_float2(f0, f0))));
@@ -494,8 +504,8 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
             k_facs = fac[ntile + at];
             v_facs = fac[2 * ntile + at];
         }
-        const float k_fac = __shfl_sync(0xffffffffu, k_facs, kt & 31), dp_fac = g_fac * __shfl_sync(0xffffffffu, v_facs, kt & 31);
-        const float s_fac = fmaxf(q_fac * k_fac, 1e-37f);        // (never zero: a hidden score is -inf, and times the factor it stays that)
+        const float k_fac = __shfl_sync(0xffffffffu, k_facs, kt & 31), dp_fac = fminf(g_fac * __shfl_sync(0xffffffffu, v_facs, kt & 31), kFacMost);
+        const float s_fac = fminf(fmaxf(q_fac * k_fac, 1e-37f), kFacMost);        // (never zero: a hidden score is -inf, and times the factor it stays that)
         const float2 dp2 = make_float2(dp_fac, dp_fac), s2 = make_float2(s_fac, s_fac);
         float s[32], dp[32];
         if (i == nk) {
@@ -801,7 +811,8 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
             g_facs = fac[3 * ntile + ft];
         }
         const float q_fac = __shfl_sync(0xffffffffu, q_facs, i & 31), g_fac = __shfl_sync(0xffffffffu, g_facs, i & 31);
-        const float2 s2 = make_float2(k_fac * q_fac, k_fac * q_fac), dp2 = make_float2(v_fac * g_fac, v_fac * g_fac);
+        const float s_fac = fminf(k_fac * q_fac, kFacMost), dp_fac = fminf(v_fac * g_fac, kFacMost);
+        const float2 s2 = make_float2(s_fac, s_fac), dp2 = make_float2(dp_fac, dp_fac);
         const float *wrow = rows_s[i % C::kStages][0] + hf * 32;
         const bool mask = CAUSAL && qb < k0 + wq * 32 + 31;              // some lane of the warp has a key after some query
         float p[32], d[32];

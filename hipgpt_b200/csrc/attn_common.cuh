@@ -148,7 +148,7 @@ int bf16_status_fetch(int *status);
 // attention backward (attn_bwd.cu): scratch = 2 B H S floats (row sums w_i, then log-sum-exp of the rows)
 size_t mha_backward_scratch_bytes(int B, int H, int S);
 int launch_mha_backward(const float *g, const float *q, const float *k, const float *v, const float *probs,
-                        float *dq, float *dk, float *dv, float *scratch, int B, int S, int E, int H, int causal, cudaStream_t st);
+                        float *dq, float *dk, float *dv, float *scratch, int B, int S, int E, int H, int causal, bool tensor, cudaStream_t st);
 // the same on the tensor pipe, head_dim 32 / 64 (attn_bwd_tc.cu)
 bool mha_backward_tc_supports(const void *g, const void *q, const void *k, const void *v, const void *probs, const void *dq, const void *dk,
                               const void *dv, int B, int S, int E, int H);

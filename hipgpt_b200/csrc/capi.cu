@@ -412,7 +412,8 @@ int hipgpt_mha_backward(const float *d_grad_out, const float *d_q, const float *
     const size_t need = mha_backward_scratch_bytes(B, H, S);
     if (!d_scratch || scratch_bytes < need)
         return fail(HIPGPT_ERR_SCRATCH, "scratch of %zu bytes needed, %zu given", need, d_scratch ? scratch_bytes : (size_t)0);
-    return launch_mha_backward(d_grad_out, d_q, d_k, d_v, d_probs, d_grad_q, d_grad_k, d_grad_v, d_scratch, B, S, E, H, causal,
+    const bool tensor = !full_range() && mha_backward_tc_supports(d_grad_out, d_q, d_k, d_v, d_probs, d_grad_q, d_grad_k, d_grad_v, B, S, E, H);
+    return launch_mha_backward(d_grad_out, d_q, d_k, d_v, d_probs, d_grad_q, d_grad_k, d_grad_v, d_scratch, B, S, E, H, causal, tensor,
                                static_cast<cudaStream_t>(stream));
 }
 
@@ -430,11 +431,12 @@ int hipgpt_mha_backward_planes(const float *d_grad_out, const float *d_qkv, cons
     float *dk = d_grad_qkv + plane, *dv = dk + plane;
     const cudaStream_t st = static_cast<cudaStream_t>(stream);
     StreamWorkspace::Lease scratch;
-    if (!mha_backward_tc_supports(d_grad_out, d_qkv, k, v, d_probs, d_grad_qkv, dk, dv, B, S, E, H)) {
+    const bool tensor = !full_range() && mha_backward_tc_supports(d_grad_out, d_qkv, k, v, d_probs, d_grad_qkv, dk, dv, B, S, E, H);    // (asked once: the setting may change)
+    if (!tensor) {
         const int rc = g_bwd_rows_ws.enter(st, mha_backward_scratch_bytes(B, H, S), &scratch);
         if (rc != HIPGPT_OK) return rc;
     }
-    return launch_mha_backward(d_grad_out, d_qkv, k, v, d_probs, d_grad_qkv, dk, dv, reinterpret_cast<float *>(scratch.get()), B, S, E, H, causal, st);
+    return launch_mha_backward(d_grad_out, d_qkv, k, v, d_probs, d_grad_qkv, dk, dv, reinterpret_cast<float *>(scratch.get()), B, S, E, H, causal, tensor, st);
 }
 
 int hipgpt_shard_range(int B, int world, int rank, int *b_begin, int *b_end)

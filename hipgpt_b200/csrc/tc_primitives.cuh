@@ -270,6 +270,26 @@ __device__ __forceinline__ void mma_h_ts(uint32_t d_tmem, uint32_t a_tmem, uint6
         ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
 
+// The same, adding to the accumulator times 2^-SHIFT
+template <int SHIFT>
+__device__ __forceinline__ void mma_h_ss_down(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, 1, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p, %4;\n\t}"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "n"(SHIFT) : "memory");
+}
+template <int SHIFT>
+__device__ __forceinline__ void mma_h_ts_down(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, 1, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p, %4;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "n"(SHIFT) : "memory");
+}
+
 // fp32 accumulator, bf16 A and B, A K-major, B K- or N-major
 __host__ __device__ constexpr uint32_t idesc_bf16(int m, int n, int b_n_major)
 {

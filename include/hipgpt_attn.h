@@ -148,11 +148,17 @@ HIPGPT_API int hipgpt_attention_weighted_sum(const float *d_softmax, const float
  *                  written them at all
  *   d_grad_q/k/v   [B*S][E], fully overwritten
  *   d_scratch      hipgpt_mha_backward_scratch_bytes(B, H, S) bytes (2 B H S floats)
- * No atomics: a key row's gradients add its queries in ascending order, so results are reproducible run to
- * run (the reference's atomicAdd order is not); they agree with the reference's arithmetic to rounding.
- * head_dim 32 and 64 run on the tensor pipe with fp32 accuracy over the whole fp32 range (every operand as the sum of three
- * bf16 numbers, six products per product); the operands' images live in a buffer of the library (per device and stream,
- * at most eight; hipgpt_release_workspace() frees them; a captured call gets a buffer of its graph).
+ * No atomics: the order of every sum is fixed, so results are reproducible run to run (the reference's atomicAdd order is
+ * not); they agree with the reference's arithmetic to rounding.  (Each head_dim and length has its own order: tiles of 64
+ * queries or keys, their sums in ascending order; where a head is taken in one piece by two blocks, each block's own queries
+ * last.)
+ * head_dim 32 and 64 run on the tensor pipe: an operand is the sum of two fp16 numbers under one power of two per 64 rows of a
+ * head (probabilities and their gradients: per 64 x 64 of them at most), that is 2^-23 of a value down to 2^-29 of the largest
+ * of its 64 rows, 2^-52 of that one below: rows beside each other may be nine decimal orders apart.  Error against float64
+ * 1 - 2.6e-7 on unit normals.  Wider ranges than that: hipgpt_set_full_range(1) takes the kernels of the other head dimensions, exact
+ * fp32 throughout.  Contexts that do not fit one block (head_dim 32: more than 256 rows, 64: more than 128) keep the operands'
+ * images in a buffer of the library (per device and stream, at most eight; hipgpt_release_workspace() frees them; a captured
+ * call gets a buffer of its graph).
  * hipgpt_mha_backward_planes is the launcher's own view (three stacked planes in d_qkv and d_grad_qkv): the scratch, which
  * only the kernels of the other head dimensions use, comes from a buffer of the library of the same kind.
  */
@@ -388,7 +394,7 @@ HIPGPT_API int hipgpt_kernel_status(int *status);
  * 1e-5-grade.  Waits for the device, then reads and clears the flag.
  * hipgpt_set_full_range(1) (or the environment variable HIPGPT_FULL_RANGE=1, read at the first call)
  * makes every entry point, the reference-named launchers included, use the kernels whose accuracy does
- * not depend on magnitude (split-TF32; exact FFMA when the probabilities are stored).
+ * not depend on magnitude (split-TF32; exact FFMA when the probabilities are stored, and for the backward).
  */
 HIPGPT_API int hipgpt_accuracy_notice(int *notice);
 HIPGPT_API int hipgpt_set_full_range(int on);

@@ -446,6 +446,139 @@ def test_attention_backward_tiles_of_their_own_scale(D, S, stored):
     assert np.array_equal(hit[0, same], got[0, same]) and np.array_equal(hit[:, :, D:], got[:, :, D:])
 
 
+def _backward_in_64_bits(g, qkv, probs, B, S, E, H, causal):
+    """The three gradients [plane][B*S][E] in float64, and for each element the sum of its terms' magnitudes."""
+    D, c = E // H, 1.0 / (E // H) ** 0.5
+    heads = lambda x: torch.as_tensor(x, device="cuda").double().reshape(B, S, H, D).transpose(1, 2)      # noqa: E731
+    back = lambda x: x.transpose(1, 2).reshape(B * S, E)      # noqa: E731
+    q, k, v, g = *(heads(x) for x in torch.as_tensor(qkv).reshape(3, B * S, E)), heads(g)
+    most = 0.0
+    if probs is not None:
+        p = torch.as_tensor(probs, device="cuda").double().reshape(B, H, S, S)
+    else:
+        s = c * q @ k.transpose(-1, -2)
+        most = float(s.abs().max())
+        p = (s.masked_fill(torch.ones(S, S, dtype=torch.bool, device="cuda").triu(1), float("-inf")) if causal else s).softmax(-1)
+    vd, a = g @ v.transpose(-1, -2), g.abs() @ v.abs().transpose(-1, -2)
+    ds, da = p * (vd - (p * vd).sum(-1, keepdim=True)), p.abs() * (a + (p.abs() * a).sum(-1, keepdim=True))
+    t = lambda x: x.transpose(-1, -2)      # noqa: E731
+    want = torch.stack([back(x) for x in (c * ds @ k, c * t(ds) @ q, t(p) @ g)])
+    terms = torch.stack([back(x) for x in (c * da @ k.abs(), c * t(da) @ q.abs(), t(p).abs() @ g.abs())])
+    return want, terms, most
+
+
+def _assert_rows_are_near(got, want, terms, most):
+    """Row by row of a head: within 5e-6 of the row's largest sum of magnitudes.  (Three factors to 2^-22 each, up to thirty truncations and roundings of
+    2^-24 on the way through the two products, the sums of a row and of the tiles: below 40 x 2^-23.)  Where probabilities are formed again, their
+    exponent's rounding too: 2^-21 of the largest score."""
+    got, D = torch.as_tensor(got).cuda().double().reshape(want.shape), 32
+    err, bound = ((x.reshape(*x.shape[:2], -1, D).amax(-1)) for x in ((got - want).abs(), terms))
+    tol = 5e-6 + 2.0 ** -21 * most
+    worst = float((err / bound.clamp_min(1e-300)).max())
+    assert bool(torch.isfinite(got).all()) and worst <= tol, (worst, tol)
+
+
+@pytest.mark.parametrize("D,S", [(32, 130), (64, 97), (32, 300), (64, 200)])
+@pytest.mark.parametrize("stored", [False, True])
+@pytest.mark.parametrize("plane", ["dO", "V", "K"])
+def test_attention_backward_rows_of_a_tile_far_apart(D, S, stored, plane):
+    """Rows of one 64-row tile down to 2^-28 of its largest, in any order, each output row to its own scale: with the mask a key of the last rows is
+    seen by few queries, and those may all be small."""
+    B, H = 1, 2
+    E = H * D
+    rng = np.random.default_rng(S)
+    scale = (2.0 ** -rng.integers(0, 29, (S, 1))).astype(np.float32)
+    qkv, g = synth.qkv_planes(890 + S, B, S, E).reshape(3, S, E).copy(), synth.normal(891 + S, (S, E))
+    if plane == "dO":
+        g = g * scale
+    else:
+        qkv[2 if plane == "V" else 1] *= scale
+    for causal in (True, False):
+        probs = ob.mha(qkv, B, S, E, H, causal=causal, want_probs=True)[1] if stored else None
+        got = _run_backward(g, qkv, probs, B, S, E, H, causal)
+        _assert_rows_are_near(got, *_backward_in_64_bits(g, qkv, probs, B, S, E, H, causal))
+
+
+@pytest.mark.parametrize("D,S", [(32, 130), (32, 256), (64, 128), (32, 300), (64, 200)])
+@pytest.mark.parametrize("stored", [False, True])
+def test_attention_backward_of_keys_that_get_little_probability(D, S, stored):
+    """Keys whose probabilities go down to e^-18 for every query: their rows of dK and dV to their own scale."""
+    B, H = 1, 2
+    E = H * D
+    rng = np.random.default_rng(S + 1)
+    qkv, g = synth.qkv_planes(892 + S, B, S, E).reshape(3, S, H, D) * np.float32(0.25), synth.normal(893 + S, (S, E))
+    qkv[0, :, :, 0] = D ** 0.5
+    qkv[1, :, :, 0] = -18.0 * rng.random((S, 1))
+    qkv[1, 7, :, 0] = 0.0
+    qkv = np.ascontiguousarray(qkv, dtype=np.float32).reshape(3, S, E)
+    probs = ob.mha(qkv, B, S, E, H, want_probs=True)[1] if stored else None
+    got = _run_backward(g, qkv, probs, B, S, E, H, False)
+    _assert_rows_are_near(got, *_backward_in_64_bits(g, qkv, probs, B, S, E, H, False))
+
+
+@pytest.mark.parametrize("D,S,B,H", [(32, 300, 1, 2), (64, 200, 1, 2), (32, 2200, 1, 1), (64, 384, 24, 8)])
+@pytest.mark.parametrize("causal,stored", [(False, True), (True, False)])
+def test_attention_backward_long_contexts_each_tile_of_its_own_scale(D, S, B, H, causal, stored):
+    """The kernels of the longer contexts: a power of two of its own for each 64-row tile of Q, K, V and dO, more tiles than factors are read at a time
+    (2200 rows), and more than one group of batches (24 x 8 heads of 384 rows)."""
+    E = H * D
+    tile = np.arange(S) // 64
+    power = lambda n, lo: (2.0 ** -((tile * n) % 7 * lo)).astype(np.float32)[None, :, None]      # noqa: E731
+    gen = torch.Generator(device="cuda").manual_seed(S)
+    qkv = torch.randn(3, B, S, E, generator=gen, device="cuda")
+    g = torch.randn(B, S, E, generator=gen, device="cuda") * torch.from_numpy(power(3, 5)).cuda()
+    for i, (n, lo) in enumerate(((1, 1), (2, 1), (4, 6))):
+        qkv[i] *= torch.from_numpy(power(n, lo)).cuda()
+    p = torch.empty(B, H, S, S, device="cuda") if stored else None
+    out, grad = torch.empty(B * S, E, device="cuda"), torch.full((3, B * S, E), float("nan"), device="cuda")
+    if stored:
+        _capi.check(_capi.lib().hipgpt_mha_forward_planes(qkv.data_ptr(), out.data_ptr(), p.data_ptr(), B, S, E, H, int(causal), _st()))
+    _capi.check(_capi.lib().hipgpt_mha_backward_planes(g.data_ptr(), qkv.data_ptr(), p.data_ptr() if stored else None, grad.data_ptr(), B, S, E, H, int(causal), _st()))
+    torch.cuda.synchronize()
+    for b in range(0, B, 8):                               # (the comparison in parts: float64 scores take room)
+        rows, n = slice(b * S, (b + 8) * S), min(8, B - b)
+        args = (g[b:b + 8], qkv[:, b:b + 8], p[b:b + 8] if stored else None)
+        _assert_rows_are_near(grad[:, rows], *_backward_in_64_bits(*args, n, S, E, H, causal))
+
+
+@pytest.mark.parametrize("D,S", [(32, 300), (64, 200)])
+def test_attention_backward_long_contexts_an_infinity_stays_in_its_row(D, S):
+    """An infinity of dO becomes NaN in its own row of dQ and leaves the other rows, and the other head, their bits."""
+    B, H = 1, 2
+    E = H * D
+    qkv, g = synth.qkv_planes(894 + S, B, S, E).reshape(3, S, E), synth.normal(895 + S, (S, E))
+    for stored in (False, True):
+        probs = ob.mha(qkv, B, S, E, H, causal=True, want_probs=True)[1] if stored else None
+        want = _run_backward(g, qkv, probs, B, S, E, H, True).reshape(3, S, E)
+        bad = g.copy()
+        bad[70, 3] = np.inf
+        got = _run_backward(bad, qkv, probs, B, S, E, H, True).reshape(3, S, E)
+        same = np.arange(S) != 70
+        assert not np.isfinite(got[0, 70, :D]).any()
+        assert np.array_equal(got[0, same], want[0, same]) and np.array_equal(got[:, :, D:], want[:, :, D:])
+
+
+@pytest.mark.parametrize("D,S", [(32, 130), (64, 200)])
+@pytest.mark.parametrize("stored", [False, True])
+def test_attention_backward_with_the_full_range_asked_for(D, S, stored):
+    """hipgpt_set_full_range: rows 2^-60 apart inside a tile, each to its own scale, through both entry points; and afterwards the tensor pipe's bits again."""
+    B, H, lib = 1, 2, _capi.lib()
+    E = H * D
+    rng = np.random.default_rng(S + 2)
+    qkv, g0 = synth.qkv_planes(896 + S, B, S, E).reshape(3, S, E), synth.normal(897 + S, (S, E))
+    g = g0 * (2.0 ** -rng.integers(0, 61, (S, 1))).astype(np.float32)
+    probs = ob.mha(qkv, B, S, E, H, causal=True, want_probs=True)[1] if stored else None
+    before = _run_backward(g0, qkv, probs, B, S, E, H, True)
+    _capi.check(lib.hipgpt_set_full_range(1))
+    try:
+        got = [_run_backward(g, qkv, probs, B, S, E, H, True, planes=planes) for planes in (False, True)]
+    finally:
+        _capi.check(lib.hipgpt_set_full_range(0))
+    assert np.array_equal(got[0], got[1])
+    _assert_rows_are_near(got[0], *_backward_in_64_bits(g, qkv, probs, B, S, E, H, True))
+    assert np.array_equal(_run_backward(g0, qkv, probs, B, S, E, H, True), before)
+
+
 def test_attention_backward_reference_named_launcher():
     raw = C.CDLL(_capi.lib_path())
     fn = getattr(raw, _capi.CXX_LAUNCHERS["launch_multihead_attention_backward"])
