@@ -7,24 +7,27 @@
 // shared memory one kernel does it all: 128 queries per block, all keys of the head, the two blocks of a head of more
 // than 128 rows as a cluster.  Everything a block needs is on the SM at once:
 //   operands       as pieces (attn_bwd_pieces.cuh), cut by the workers on the way from memory: g and Q of the block's rows, K and V of the head
-//   P              128 x 256 fp32 (from memory, by TMA; or formed here), 128 KB.  A probability's two pieces take the place it had.
-//   dP = g V^T     256 columns of TMEM, formed once.  ds takes their place in fp32, and when the pieces of P have been read, ds's
-//                  pieces take theirs, where they serve both products: read K-major for dQ = ds K, M-major for dK = ds^T Q.
+//   P              128 x 256 fp32 (from memory, by TMA; or formed here), 128 KB
+//   dP = g V^T     256 columns of TMEM, formed once
+//   ds             as pieces in P's place, where they serve both products: read K-major for dQ = ds K, M-major for dK = ds^T Q
+//   dV             formed probabilities: their two pieces take P's place first, and ds waits in dP's in fp32 until they have been read.
+//                  Stored ones, which are exact: as in attn_bwd_tc.cu, from three bf16 pieces, when all else has been done: the block's keys, all queries.
 // so that the sweeps of the workers (w; ds and P's pieces; ds's pieces) run over whole rows with no product to wait for inside.
 // The pieces of P and ds are cut by one power of two per tile of 64 queries x 64 keys, which can leave with a row of dQ's sums (kept per tile of keys) and with
 // one of dV's and dK's (kept per 64 queries): P's from its largest there, ds's from an upper bound by row (largest P |dP|, and largest P times |w|).
 // The bound is no estimate: where a row has all its weight on one key it is 2 |w| and ds near zero.  The pieces' range (attn_bwd_pieces.cuh) is what covers that.
 // The queries of the other block contribute to this block's keys: their sums come through distributed shared memory at the end.
 //
-// Measured, us, three kernels -> one: B=32 H=8 S=256 D=32 with stored probabilities 90.4 -> 64.1, causal without 78.5 -> 62.5; B=16 H=12 S=128 D=32
-// stored 28.9 -> 20.4; B=64 H=12 S=35 68.2 -> 53.1; D=64: B=32 H=8 S=128 stored 41.8 -> 29.6, causal without 45.8 -> 29.9; B=9 H=16 S=101 25.0 -> 14.6.
-// There is no length in its range at which the three are faster.  Relative error of the gradients against float64: 1.45, 1.39, 1.03e-7 (dQ, dK, dV) at the
-// first, 1.8, 1.9, 1.6e-7 at the second (with stored probabilities the products of the low pieces are formed too: without, 1.51, 1.46, 1.03e-7 and 63.5 us instead of 64.1).
-// What bounds it: a block takes 15 us at the first shape, 3.5 rounds of them.  5 until its operands are cut (224 KB come in at 64 bytes
-// per clock; the cut is bound by the instructions of conversion), 2 for w, 3 for ds and P's pieces, 2.5 for ds's, 1.5 for the last product and the other
-// block's sums, 1 for the output.  In the sweeps the conversions and the shared memory's width (512 cycles each per tile) share the time.
+// Measured, us, three kernels -> one: B=32 H=8 S=256 D=32 with stored probabilities 94.9 -> 77.3, causal without 80.9 -> 70.1; S=161 (probabilities that TMA cannot
+// address) 84.7 -> 86.1, causal without 69.1 -> 59.8; B=16 H=12 S=128 D=32 stored 31.2 -> 24.9; B=64 H=12 S=35 82.0 -> 60.2; D=64: B=32 H=8 S=128 stored 46.2 -> 35.4, causal
+// without 46.2 -> 32.7; B=9 H=16 S=101 27.2 -> 19.5.  But for odd lengths just above 128 at D=32, where both are the same, the one is faster throughout.
+// Relative error of the gradients against float64: 1.45, 1.40, 0.90e-7 (dQ, dK, dV) at the first, 1.42, 1.40, 0.83e-7 at B=8 H=8 S=128 D=64 stored; three bf16
+// pieces and six products throughout: 1.47, 1.68, 0.94e-7 and 1.41, 1.63, 0.83e-7.  (dV of two fp16 pieces: 1.03 and 0.95e-7; 69.0 us at the first.)
+// What bounds it: a block takes 33200 cycles at the first shape, 3.5 rounds of them.  9700 until its operands are cut and g V^T is there (224 KB come in at
+// 64 bytes per clock; the cut is bound by the instructions of conversion), 4500 for w and the scales, 5300 for ds and its pieces, 4300 for the products with
+// them and the other block's sums, 6800 for dV (900 dO's pieces, 1000 per tile of probabilities, 1400 the last product), 1900 for the output.
 // Steps, B=32 H=8 S=256 D=32 stored: eight worker warps 76.7, sixteen 72.9; operands as whole sectors, two issuing warps, no stall between the reading of a tile's
-// probabilities and the writing of its pieces 64.3.
+// probabilities and the writing of its pieces 64.3; scales per 64 x 64 instead of per 64 x 256, for keys of little probability, 69.0; dV exact 77.3.
 #include "attn_bwd_pieces.cuh"
 #include "tma_host.cuh"
 
@@ -85,13 +88,17 @@ struct HeadCfg {
     // columns of TMEM: dP (ds, dQ's sums of a tile); scores, then the sums of dV and dK, [block of keys][64 queries]
     static constexpr int kColAcc = 256, kColK = D == 32 ? 0 : 128;
     // tiles of 64 rows of the planes
+    // dV of stored probabilities: g's image as three bf16 pieces, in V's and K's place (behind what the other block sends); pieces of P in TMEM, 96 columns per 64 queries, then sums
+    static constexpr int kExactG = kV + (NB > 1 ? 16384 : 0), kCols3 = 96;
+    static constexpr uint32_t kCol3 = kTiles * kCols3;
+    static_assert(kExactG + NB * 16 * kBlock3<D> <= kSmall && kCol3 + kTiles * D <= kTmemCols, "");
     static constexpr int tG = 0, tV = 2, tQ = 2 + kTiles, tK = 4 + kTiles, kAll = 4 + 2 * kTiles;
 };
 
 // The small things behind the operands
 template <int NB>
 struct HeadSmall {
-    uint64_t p_full[2 * NB], scores, asked, cut[2], p_read[NB], p_ready[NB], v_done[NB], d_ready[NB], k_done[NB];
+    uint64_t p_full[2 * NB], p3_full[NB], p3_ready[2 * NB], v3_done, scores, asked, cut[2], p_read[NB], p_ready[NB], v_done[NB], d_ready[NB], k_done[NB];
     alignas(16) uint32_t largest[4 + 4 * NB][8];                // of a tile's rows that a warp has
     float fac[4 + 4 * NB];
     uint32_t group_p[2 * NB][2], group_d[2 * NB][2]; // of a tile of 64 queries (second index) x 64 keys: P's largest, ds's bound
@@ -119,13 +126,18 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
     const int b = bh / H, h = bh % H, q0 = blk * kLanes, next = (int)blockIdx.x + ahead;
     const int nkb = CAUSAL ? blk + 1 : NB;           // blocks of 128 keys that these queries see
     const int ntile = (min(S, nkb * kLanes) + kTile - 1) / kTile;
+    const int qb0 = CAUSAL ? blk : 0, nqb = (S + kLanes - 1) / kLanes, nq = (S + kTile - 1) / kTile;      // blocks and tiles of queries that see these keys: from qb0, 2 qb0 on
     auto block_at = [&](int i) { return nkb == 1 ? 0 : i == 0 ? blk ^ 1 : blk; };         // the other block's keys first: their sums have a way to go
+    // the block of keys whose place the probabilities of query block j take later on
+    auto place = [&](int j) { return nkb == 1 ? j - qb0 : block_at(j - qb0); };
 
     if (tid == 0) {
         sh.abort_flag = 0;
         sh.peer_gone = 0;
         for (int t = 0; t < 2 * NB; ++t) sh.group_p[t][0] = sh.group_p[t][1] = sh.group_d[t][0] = sh.group_d[t][1] = 0;
-        for (int i = 0; i < 2 * NB; ++i) mbar_init(&sh.p_full[i], 1);
+        for (int i = 0; i < 2 * NB; ++i) { mbar_init(&sh.p_full[i], 1); mbar_init(&sh.p3_ready[i], kWorkerWarps); }
+        for (int i = 0; i < NB; ++i) mbar_init(&sh.p3_full[i], 1);
+        mbar_init(&sh.v3_done, 2);
         mbar_init(&sh.scores, 2);                    // (commits: one per issuing warp)
         for (int i = 0; i < 2; ++i) mbar_init(&sh.cut[i], kWorkerWarps);
         mbar_init(&sh.asked, kWorkerWarps);
@@ -210,7 +222,7 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
         if (elect_one()) tc_commit(&sh.scores);
         if (STORED) wait(&sh.cut[1], 0, 21);
         if (NB > 1) cluster_arrive();
-        for (int i = 0; i < nkb; ++i) {
+        for (int i = 0; i < (STORED ? 0 : nkb); ++i) {
             const int kb = block_at(i);
             wait(&sh.p_ready[i], 0, 24);
             tc_fence_after();
@@ -226,13 +238,35 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
             if (t < ntile) sums(tmem + t * kTile, make_desc(smem_u32(p_s + t * 2 * kGroup), kKeys8, 128, 0), 2 * kKeys8 >> 4, id_sums, k_s + t * TB);
             if (elect_one()) tc_commit(&sh.k_done[i]);
         }
-        __syncwarp();
-        if (sh.abort_flag) linger();
-        if (NB > 1) {
+        if (NB > 1) {                                // (before the workers are needed again: theirs wait for these arrivals too)
             cluster_wait();
             cluster_arrive();
-            cluster_wait();
         }
+        if constexpr (STORED) {
+            for (int i = 0; i < nkb; ++i) {          // a block of keys' pieces have been read: a block of queries' probabilities take their place
+                wait(&sh.k_done[i], 0, 26);
+                if (by_tma && mine == 0 && lane == 0 && !sh.abort_flag)
+                    for (int j = qb0 + i; j < (i + 1 < nkb ? min(qb0 + i + 1, nqb) : nqb); ++j) {
+                        mbar_arrive_expect_tx(&sh.p3_full[j], 4 * kGroup);
+                        for (int x = 0; x < 4; ++x) tma_load_3d(p_s + (4 * place(j) + x) * kGroup, &p_map, q0 + 32 * x, j * kLanes, bh, &sh.p3_full[j]);
+                    }
+                __syncwarp();
+            }
+            for (int t = 2 * qb0 + mine; t < nq; t += 2) {
+                wait(&sh.p3_ready[t], 0, 24);
+                tc_fence_after();
+                const uint64_t db = make_desc(smem_u32(sm + C::kExactG + t * 8 * kBlock3<D>), kBlock3<D>, 128, 0);
+#pragma unroll
+                for (int p = 0; p < 6; ++p)
+#pragma unroll
+                    for (int ks = 0; ks < 4; ++ks)
+                        if (elect_one()) mma_h_ts(tmem + C::kCol3 + t * D, tmem + t * C::kCols3 + kExactA[p] * 32 + ks * 8, db + (uint64_t)(ks * 2 * (kBlock3<D> >> 4) + kExactB[p] * (Img<D>::kPiece >> 4)), idesc_bf16(kLanes, D, 1), p + ks > 0 ? 1u : 0u);
+            }
+            if (elect_one()) tc_commit(&sh.v3_done);
+        }
+        __syncwarp();
+        if (sh.abort_flag) linger();
+        if (NB > 1) cluster_wait();
         tc_fence_before();
         __syncthreads();
         if (mine == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
@@ -446,16 +480,17 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
         for (int t = 0; t < C::kTiles; ++t) {
             if (t >= ntile) break;
             uint32_t bp = __float_as_uint(most_p[t] * rinv), bd = __float_as_uint(fmaf(most_p[t], fabsf(w), most_d[t]) * rinv);
-            bp = __reduce_max_sync(0xffffffffu, bp < 0x7f800000u ? bp : 0u);
+            if (!STORED) bp = __reduce_max_sync(0xffffffffu, bp < 0x7f800000u ? bp : 0u);
             bd = __reduce_max_sync(0xffffffffu, bd < 0x7f800000u ? bd : 0u);
-            if (lane == 0) { atomicMax(&sh.group_p[t][u], bp); atomicMax(&sh.group_d[t][u], bd); }
+            if (lane == 0 && !STORED) atomicMax(&sh.group_p[t][u], bp);
+            if (lane == 0) atomicMax(&sh.group_d[t][u], bd);
         }
         meet();
     }
     if (NB > 1) cluster_arrive();                    // V's image is this block's no longer: the other one's sums may come
-    // exponents of a tile: of its probabilities and of its ds (at most 2^100 below the probabilities': the ratio of the factors stays a number)
+    // exponents of a tile: of its probabilities (those that are formed: at most 1) and of its ds
     auto e_p = [&](int t, int y) { return range_exponent(sh.group_p[t][y]); };
-    auto e_d = [&](int t, int y) { const uint32_t p = e_p(t, y), d = range_exponent(sh.group_d[t][y]); return p > d + (100u << 23) ? p - (100u << 23) : d; };
+    auto e_d = [&](int t, int y) { return range_exponent(sh.group_d[t][y]); };
 
     // Second sweep: ds, scaled, in fp32 in dP's place; P's pieces in P's.  A block of keys' probabilities are read first: eight warps share the memory
     // that each of them then writes its pieces to (a meeting per tile, between reading and writing it, kept them all in the same step: 1300 cycles per tile).
@@ -486,29 +521,31 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
         for (int y = 0; y < 2; ++y) {
             const int t = 2 * kb + y;
             if (t >= ntile) break;
-            const uint32_t ep = e_p(t, u);
-            const float up_row = STORED ? range_up(ep) : rinv * range_up(ep), ratio = range_up(e_d(t, u)) * range_down(ep);
+            const uint32_t ep = STORED ? 0u : e_p(t, u);
+            const float up_d = range_up(e_d(t, u)), up_row = rinv * range_up(ep), ratio = STORED ? 1.0f : up_d * range_down(ep);
             const float dp_up = fminf(g_fac * sh.fac[C::tV + t], kFacMost) * ratio, w_up = w * ratio;
             float dp[kCols];
             tmem_ld16(my_tile + t * kTile, dp);
             if (STORED) mask(p[y], count(t), 0.0f);
+            if (!STORED)
 #pragma unroll
-            for (int x = 0; x < kCols; x += 2) { const float2 z = fmul2(make_float2(p[y][x], p[y][x + 1]), make_float2(up_row, up_row)); p[y][x] = z.x; p[y][x + 1] = z.y; }
+                for (int x = 0; x < kCols; x += 2) { const float2 z = fmul2(make_float2(p[y][x], p[y][x + 1]), make_float2(up_row, up_row)); p[y][x] = z.x; p[y][x + 1] = z.y; }
             tmem_wait_ld();
 #pragma unroll
             for (int x = 0; x < kCols; x += 2) {
-                const float2 d = fmul2(make_float2(p[y][x], p[y][x + 1]), ffma2(make_float2(dp[x], dp[x + 1]), make_float2(dp_up, dp_up), make_float2(-w_up, -w_up)));
+                float2 d = fmul2(make_float2(p[y][x], p[y][x + 1]), ffma2(make_float2(dp[x], dp[x + 1]), make_float2(dp_up, dp_up), make_float2(-w_up, -w_up)));
+                if (STORED) d = fmul2(d, make_float2(up_d, up_d));       // (last: whatever the probabilities are, this is at most 2^15)
                 dp[x] = d.x;
                 dp[x + 1] = d.y;
             }
-            tmem_st16(my_tile + t * kTile, dp);
-            store_pieces(t, p[y], [&] { if (y == 0) wait(&sh.p_read[i], 0, 27); });
+            if (!STORED) tmem_st16(my_tile + t * kTile, dp);
+            store_pieces(t, STORED ? dp : p[y], [&] { if (y == 0) wait(&sh.p_read[i], 0, 27); });
         }
         if (i + 1 < nkb) read_block(i + 1);
-        tmem_wait_st();
+        if (!STORED) tmem_wait_st();
         proxy_fence();
         tc_fence_before();
-        arrive(&sh.p_ready[i]);
+        arrive(STORED ? &sh.d_ready[i] : &sh.p_ready[i]);
     }
 
     // Third sweep: ds's pieces in the place of P's.  Between: this thread's columns of its key's row of dV
@@ -548,8 +585,10 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
         }
     };
     float ov[OC], ok[OC], oq[OC];
+#pragma unroll
+    for (int x = 0; x < OC; ++x) ov[x] = 0.0f;
     bool joined = NB == 1;                           // the other block has said that its V is free
-    for (int i = 0; i < nkb; ++i) {
+    for (int i = 0; i < (STORED ? 0 : nkb); ++i) {
         const int kb = block_at(i);
         wait(&sh.v_done[i], 0, 25);
         tc_fence_after();
@@ -580,7 +619,7 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
         if (NB > 1 && i == 0) {                      // (every block takes both steps of the cluster's barrier twice)
             if (!joined) cluster_wait();
             if (kb != blk) {
-                send(ok, 1);
+                send(ok, STORED ? 0 : 1);
                 // a warp that has seen a wait run out, its own or one that its sums depend on, says so
                 if (lane == 0 && sh.abort_flag) {
                     const uint32_t gone = peer_of(smem_u32(const_cast<int *>(&sh.peer_gone)), blk ^ 1);
@@ -612,7 +651,7 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
 #pragma unroll
         for (int i = 0; i < OC / 4; ++i) {
             float4 x = make_float4(o[4 * i] * scale, o[4 * i + 1] * scale, o[4 * i + 2] * scale, o[4 * i + 3] * scale);
-            x.x = fmaf(x.x, loss, x.x); x.y = fmaf(x.y, loss, x.y); x.z = fmaf(x.z, loss, x.z); x.w = fmaf(x.w, loss, x.w);
+            if (loss != 0.0f) { x.x = fmaf(x.x, loss, x.x); x.y = fmaf(x.y, loss, x.y); x.z = fmaf(x.z, loss, x.z); x.w = fmaf(x.w, loss, x.w); }
             *reinterpret_cast<float4 *>(box + sw128(lane, D == 64 ? (cf & 1) * 4 + i : cf * 2 + i)) = x;
         }
         if (D == 64) asm volatile("bar.sync %0, 64;" ::"r"(4 + wq * 2 + (cf >> 1)) : "memory");
@@ -625,16 +664,92 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
             if (row0 + r < S && !off) *reinterpret_cast<float4 *>(dst + ((size_t)b * S + row0 + r) * E + (size_t)h * D + (D == 64 ? (cf >> 1) * 32 : 0) + (lane & 7) * 4) = x;
         }
     };
+    tc_fence_before();
     meet();                                          // the products have been waited for by all: their operands' memory is free
+    tc_fence_after();
+    // dV of stored probabilities, which are exact, as dO is: three bf16 pieces hold all 24 bits of both, and nothing depends on their magnitudes.  The block's
+    // keys, all queries; the probabilities come a second time (from L2), turned: lane = key, 16 queries of a tile.
+    if constexpr (STORED) {
+        constexpr int PARTS = D / 32;
+        float4 x3[NB][PARTS][2];
+#pragma unroll
+        for (int i = 0; i < NB; ++i) {
+            const int at = i * kLanes + warp * 8 + (lane & 7);
+            const float4 *g4 = reinterpret_cast<const float4 *>(g + ((size_t)b * S + at) * E + (size_t)h * D + (lane >> 3) * 8);
+#pragma unroll
+            for (int y = 0; y < PARTS; ++y) {
+                x3[i][y][0] = x3[i][y][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (i >= qb0 && at < S) { x3[i][y][0] = g4[8 * y]; x3[i][y][1] = g4[8 * y + 1]; }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < NB; ++i)
+#pragma unroll
+            for (int y = 0; y < PARTS; ++y) {
+                uint8_t *at = sm + C::kExactG + (i * 16 + warp) * kBlock3<D> + (lane >> 3) * 128 + (lane & 7) * 16 + y * 512;
+                uint4 pc[3];
+                cut3(make_float2(x3[i][y][0].x, x3[i][y][0].y), pc[0].x, pc[1].x, pc[2].x);
+                cut3(make_float2(x3[i][y][0].z, x3[i][y][0].w), pc[0].y, pc[1].y, pc[2].y);
+                cut3(make_float2(x3[i][y][1].x, x3[i][y][1].y), pc[0].z, pc[1].z, pc[2].z);
+                cut3(make_float2(x3[i][y][1].z, x3[i][y][1].w), pc[0].w, pc[1].w, pc[2].w);
+#pragma unroll
+                for (int z = 0; z < 3; ++z) *reinterpret_cast<uint4 *>(at + z * Img<D>::kPiece) = pc[z];
+            }
+        proxy_fence();
+#pragma unroll
+        for (int t = 0; t < C::kTiles; ++t) {
+            if (t < 2 * qb0 || t >= nq) continue;
+            const int q16 = t * kTile + cf * 16;     // this thread's first query
+            float pt[16];
+            if (by_tma) {
+                wait(&sh.p3_full[t >> 1], 0, 22);
+                const uint8_t *src = p_s + (4 * place(t >> 1) + wq) * kGroup + (lane & 3) * 4;
+#pragma unroll
+                for (int i = 0; i < 16; ++i) pt[i] = *reinterpret_cast<const float *>(src + sw128((t & 1) * kTile + cf * 16 + i, lane >> 2));
+            } else {
+                // (a lane past S reads its neighbour's key: its results go nowhere)
+                const float *src = P + ((size_t)bh * S + q16) * S + min(row, S - 1);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) pt[i] = q16 + i < S ? src[(size_t)i * S] : 0.0f;
+            }
+            if (CAUSAL) {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) pt[i] = row <= q16 + i ? pt[i] : 0.0f;
+            }
+            uint32_t pc[3][8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) cut3(make_float2(pt[2 * i], pt[2 * i + 1]), pc[0][i], pc[1][i], pc[2][i]);
+#pragma unroll
+            for (int z = 0; z < 3; ++z) tmem_st8_u32(lane_base + t * C::kCols3 + 32 * z + 8 * cf, pc[z]);
+            tmem_wait_st();
+            tc_fence_before();
+            arrive(&sh.p3_ready[t]);
+        }
+        wait(&sh.v3_done, 0, 25);
+        tc_fence_after();
+#pragma unroll
+        for (int t = 0; t < C::kTiles; ++t) {
+            if (t < 2 * qb0 || t >= nq) continue;
+            float a[OC];
+            load_acc(lane_base + C::kCol3 + t * D + cf * OC, a);
+            tmem_wait_ld();
+#pragma unroll
+            for (int i = 0; i < OC; ++i) ov[i] += a[i];
+        }
+        meet();                                      // (who has not seen a wait run out: the last word on it)
+    }
     bool off = sh.abort_flag;
     store_rows(oq, c, kScoreLoss, q_s, dQ, off);
     if (NB > 1) {
         cluster_wait();
-        if (!CAUSAL || blk == 0) { receive(ov, 0); receive(ok, 1); }
+        if (!CAUSAL || blk == 0) {
+            if (!STORED) receive(ov, 0);
+            receive(ok, STORED ? 0 : 1);
+        }
         off = off || sh.peer_gone;
     }
-    store_rows(ov, 1.0f, kSumLoss, g_s, dV, off);
-    store_rows(ok, c, kScoreLoss, k_s, dK, off);
+    store_rows(ov, 1.0f, STORED ? 0.0f : kSumLoss, STORED ? p_s : g_s, dV, off);
+    store_rows(ok, c, kScoreLoss, STORED ? g_s : k_s, dK, off);
     tc_fence_before();
     __syncthreads();
 }

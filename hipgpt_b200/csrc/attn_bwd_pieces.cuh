@@ -19,6 +19,13 @@ struct Img {
     static constexpr int kTileBytes = (kTile / 8) * kBlock;     // 64 rows
 };
 
+// The same of an operand as three bf16 pieces; the six products of such pieces that count, small ones first
+template <int D>
+constexpr int kBlock3 = 3 * Img<D>::kPiece;
+template <int D>
+constexpr int kTileBytes3 = (kTile / 8) * kBlock3<D>;
+__device__ constexpr int kExactA[6] = {0, 2, 1, 0, 1, 0}, kExactB[6] = {2, 0, 1, 1, 0, 0};
+
 // Two fp32 numbers up to 2^15 -> two words of two fp16 each, hi and 2^12 times what hi leaves: hi + 2^-12 lo is the number to 2^-23 of it
 // down to 2^-14, to 2^-37 below.  (Without the factor the low piece ran into fp16's smallest numbers at 2^-2 already.)  The products with one low piece are 2^12
 // times too large then, that of two 2^24: the tensor core brings the accumulator down where the next larger products start.
@@ -32,6 +39,16 @@ __device__ __forceinline__ void cut2(float2 x, uint32_t &h, uint32_t &l)
     const __half2 ll = __float22half2_rn(fmul2(ffma2(back, make_float2(-1.0f, -1.0f), x), make_float2(kLowUp, kLowUp)));
     h = *reinterpret_cast<const uint32_t *>(&hh);
     l = *reinterpret_cast<const uint32_t *>(&ll);
+}
+
+// Two fp32 numbers -> three words of two bf16 each whose sums are the numbers (to 2^-25 of them, whatever their magnitude)
+__device__ __forceinline__ void cut3(float2 x, uint32_t &h, uint32_t &m, uint32_t &l)
+{
+    h = pack_bf16(x.x, x.y);
+    const float2 r = fadd2(x, make_float2(-__uint_as_float(h << 16), -__uint_as_float(h & 0xffff0000u)));
+    m = pack_bf16(r.x, r.y);
+    const float2 s = fadd2(r, make_float2(-__uint_as_float(m << 16), -__uint_as_float(m & 0xffff0000u)));
+    l = pack_bf16(s.x, s.y);
 }
 
 // The power of two that brings a largest magnitude into [2^14, 2^15), and one over it, from the magnitude's bits.  Magnitudes

@@ -7,9 +7,10 @@
 // such sums is formed from three products of the pieces, lo hi, hi lo, hi hi, which the tensor core multiplies exactly and adds in
 // fp32 (lo lo, below 2^-22 of the product, where it comes in the same instruction).  The tensor core truncates where it adds to its
 // accumulator; what that takes on the average is given back at the end.  Before, three bf16 pieces and six products: twice the instructions and half as
-// many bytes more per operand (B=3 H=12 S=777 D=64 causal 117 -> 79 us, B=2 H=16 S=1024 D=64 with stored probabilities 208 -> 144), and the relative error of the
-// gradients against float64 no smaller: 2.8e-7 then and 2.1e-7 now at the first shape (dQ), 1.72 and 1.60e-7 at the second.  Only dV with stored probabilities is a little
-// farther off (1.10 and 1.16e-7 there), and dK as much nearer (1.78 and 1.57e-7).
+// many bytes more per operand (B=3 H=12 S=777 D=64 causal 117 -> 79 us), and the relative error of the gradients against float64 no smaller where P is formed here:
+// 2.8, 3.1, 2.6e-7 then and 2.1, 2.3, 1.9e-7 now (dQ, dK, dV).  Stored probabilities are exact, and so is dO: there two pieces' 23 bits
+// showed in dV (1.11 -> 1.17e-7 at B=2 H=16 S=1024 D=64, 0.90 -> 0.97e-7 at S=200), so that this one product keeps three bf16 pieces and six products
+// (1.11 and 0.90e-7; 143 -> 165 us and 28.2 -> 29.5).  dQ and dK are 1.60 and 1.57e-7 there, 1.73 and 1.78e-7 with six products throughout (208 us).
 // Powers of two: one per 64-row tile for Q, K, V and dO, kept beside the images; for P and ds, which are formed in fp32 in registers,
 // one per thread (32 columns of a row or key of a tile).  An accumulator holds one tile and one half of its columns, and the factors leave
 // where the workers add it to the running sum; those of a tile's scores go into the multiply-adds that form P and ds.  The low piece is kept 2^12 times too
@@ -62,11 +63,11 @@ __device__ __noinline__ bool bwd_wait_slow(uint64_t *bar, uint32_t parity, int s
 // A block takes a 64-row tile of a head in one plane, a warp 8 of its rows: lane = (column block of 8) * 8 + row, so that it reads 8 whole lines and
 // writes core matrices of 128 contiguous bytes per piece.  fac: [plane][tile], what an image is multiplied by to give the plane.  The tile's
 // largest magnitude counts finite values only: an infinity becomes NaN in its own row and the tile's other rows keep their scale.
-// Bound by memory: 4 bytes read and 4 written per element.
+// exact_g: where dO's three bf16 pieces go, for dV of stored probabilities.  Bound by memory: 4 bytes read and 4 written per element (dO's: 10).
 template <int D>
 __global__ void __launch_bounds__(256)
 bwd_pack_kernel(const float *__restrict__ q, const float *__restrict__ k, const float *__restrict__ v, const float *__restrict__ g,
-                uint8_t *__restrict__ img, size_t img_bytes, float *__restrict__ fac, int S, int nt, int E, int H)
+                uint8_t *__restrict__ img, size_t img_bytes, float *__restrict__ fac, uint8_t *__restrict__ exact_g, int S, int nt, int E, int H)
 {
     constexpr int PARTS = D / 32;
     __shared__ uint32_t red[8];
@@ -115,6 +116,19 @@ bwd_pack_kernel(const float *__restrict__ q, const float *__restrict__ k, const 
         *reinterpret_cast<uint4 *>(dst + p * 512) = h;
         *reinterpret_cast<uint4 *>(dst + p * 512 + Img<D>::kPiece) = l;
     }
+    if (exact_g && blockIdx.y == 3) {
+        dst = exact_g + (size_t)blockIdx.x * kTileBytes3<D> + warp * kBlock3<D> + (lane >> 3) * 128 + r * 16;
+#pragma unroll
+        for (int p = 0; p < PARTS; ++p) {
+            uint4 pc[3];
+            cut3(make_float2(x[p][0].x, x[p][0].y), pc[0].x, pc[1].x, pc[2].x);
+            cut3(make_float2(x[p][0].z, x[p][0].w), pc[0].y, pc[1].y, pc[2].y);
+            cut3(make_float2(x[p][1].x, x[p][1].y), pc[0].z, pc[1].z, pc[2].z);
+            cut3(make_float2(x[p][1].z, x[p][1].w), pc[0].w, pc[1].w, pc[2].w);
+#pragma unroll
+            for (int z = 0; z < 3; ++z) *reinterpret_cast<uint4 *>(dst + p * 512 + z * Img<D>::kPiece) = pc[z];
+        }
+    }
 }
 
 // ---- the products, issued by one converged warp that elects the lane per instruction ---------------------
@@ -142,7 +156,7 @@ __device__ __forceinline__ void issue_scores(uint32_t d_tmem, uint32_t a_smem, u
 // small products come first: the tensor core truncates where it adds to its accumulator, so the accumulator should be small
 // while they are added, and it starts anew for every tile (the workers add the tiles up in registers).  One accumulator over all
 // tiles was 10 times farther from float64 at S = 777.
-// LOLO: lo x lo too (WIDE has it in any case), for stored probabilities, which are exact: without it dV was 1.24e-7 instead of 1.16e-7 and dQ 1.66e-7 instead of 1.60e-7 from float64 at S = 1024, D = 64, 142 us instead of 143.5;
+// LOLO: lo x lo too (WIDE has it in any case), for stored probabilities, which are exact: without it dQ was 1.66e-7 instead of 1.60e-7 from float64 at S = 1024, D = 64, about 1 us less of 165;
 // probabilities formed again carry more than it takes away.
 template <int D, bool WIDE, bool LOLO>
 __device__ __forceinline__ void issue_accumulate(uint32_t acc, uint32_t a_tmem, uint32_t b_smem, int hf)
@@ -167,6 +181,19 @@ __device__ __forceinline__ void issue_accumulate(uint32_t acc, uint32_t a_tmem, 
     product(0, 0, kDown);                            // hi x hi (WIDE: hi x [hi | lo])
 }
 
+// acc[tmem] (128 x D) = A B over the 64 rows of B's image of three pieces, read N-major; A: three pieces in TMEM, 32 columns each
+template <int D>
+__device__ __forceinline__ void issue_exact(uint32_t acc, uint32_t a_tmem, uint32_t b_smem)
+{
+    const uint64_t b = make_desc(b_smem, kBlock3<D>, 128, 0);
+#pragma unroll
+    for (int p = 0; p < 6; ++p)
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks)
+            if (elect_one())
+                mma_h_ts(acc, a_tmem + 32 * kExactA[p] + 8 * ks, b + (uint64_t)(ks * 2 * (kBlock3<D> >> 4) + kExactB[p] * (Img<D>::kPiece >> 4)), idesc_bf16(kLanes, D, 1), p + ks > 0 ? 1u : 0u);
+}
+
 // 32 numbers of a row (or key), scaled by a power of two of their own -> their two pieces in 32 TMEM columns, hi first.  Returns one
 // over the factor.
 __device__ __forceinline__ float store_pieces(const float (&x)[32], uint32_t addr)
@@ -185,6 +212,32 @@ __device__ __forceinline__ float store_pieces(const float (&x)[32], uint32_t add
         tmem_st8_u32(addr + 16 + 8 * half, l);
     }
     return range_down(e);
+}
+
+// 32 probabilities of a key (half of a tile's queries) -> their three pieces, 32 TMEM columns apart, 16 columns each
+__device__ __forceinline__ void store_exact(const float (&x)[32], uint32_t addr)
+{
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        uint32_t pc[3][8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) cut3(make_float2(x[16 * half + 2 * c], x[16 * half + 2 * c + 1]), pc[0][c], pc[1][c], pc[2][c]);
+#pragma unroll
+        for (int z = 0; z < 3; ++z) tmem_st8_u32(addr + 32 * z + 8 * half, pc[z]);
+    }
+}
+// Adds a tile's accumulator of the exact products (this thread's D / 2 columns of its key) to the running sum
+template <int D>
+__device__ __forceinline__ void add_exact(uint32_t acc, int hf, float (&o)[D / 2])
+{
+#pragma unroll
+    for (int c0 = 0; c0 < D / 2; c0 += 16) {
+        float a[16];
+        tmem_ld16(acc + hf * (D / 2) + c0, a);
+        tmem_wait_ld();
+#pragma unroll
+        for (int c = 0; c < 16; ++c) o[c0 + c] += a[c];
+    }
 }
 
 // Adds a tile's two accumulators (one per half of its columns; this thread's D / 2 columns of its row) times their factors to the running sum
@@ -233,7 +286,7 @@ __device__ __forceinline__ void store_out(const float (&o)[D / 2], int warp, int
 #pragma unroll
     for (int c = 0; c < D / 8; ++c) {
         float4 x = make_float4(o[4 * c] * scale, o[4 * c + 1] * scale, o[4 * c + 2] * scale, o[4 * c + 3] * scale);
-        x.x = fmaf(x.x, loss, x.x); x.y = fmaf(x.y, loss, x.y); x.z = fmaf(x.z, loss, x.z); x.w = fmaf(x.w, loss, x.w);
+        if (loss != 0.0f) { x.x = fmaf(x.x, loss, x.x); x.y = fmaf(x.y, loss, x.y); x.z = fmaf(x.z, loss, x.z); x.w = fmaf(x.w, loss, x.w); }
         *reinterpret_cast<float4 *>(box + sw128(lane, D == 64 ? c : hf * 4 + c)) = x;
     }
     if (D == 64) __syncwarp();
@@ -607,12 +660,15 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
 // ---- columns: dK, dV -----------------------------------------------------------------------------------
 template <int D, int STORED>
 struct ColsCfg {
-    static constexpr int kStages = D == 64 && STORED ? 3 : 4;            // (Q, dO) tile pairs
+    // dV of stored probabilities, which are exact, as dO is: three bf16 pieces hold all 24 bits of both (two fp16 ones hold 23: dV was 0.97e-7 instead of
+    // 0.90e-7 from float64 at S = 200 D = 64).  A tile pair then comes with dO's three pieces too, and P^T's take 96 columns.
+    static constexpr int kStages = !STORED ? 4 : D == 64 ? 2 : 3;        // (Q, dO) tile pairs
+    static constexpr int kPair = 2 * Img<D>::kTileBytes + (STORED ? kTileBytes3<D> : 0);
     static constexpr int kResident = (STORED ? 1 : 2) * 2 * Img<D>::kTileBytes;      // V and, to form P again, K: 128 rows each
     static constexpr int kStage = STORED == 2 ? kPStages<D> * kPTile : 0;
-    static constexpr size_t kSmem = (STORED == 2 ? 1024 : 0) + (size_t)kResident + kStages * 2 * Img<D>::kTileBytes + kStage;
-    static constexpr uint32_t kBuf = 2 * kTile;                          // S^T and dP^T, then the pieces of P^T and ds^T
-    static constexpr uint32_t kColV = 2 * kBuf, kColK = kColV + 128;     // an accumulator per half tile
+    static constexpr size_t kSmem = (STORED == 2 ? 1024 : 0) + (size_t)kResident + kStages * kPair + kStage;
+    static constexpr uint32_t kColD = STORED ? 96 : kTile, kBuf = kColD + kTile;      // S^T and, from kColD on, dP^T, then the pieces of P^T and ds^T
+    static constexpr uint32_t kColV = 2 * kBuf, kColK = kColV + (STORED ? 64 : 128);  // an accumulator per half tile; one per tile for the exact products
     static constexpr bool kWide = D == 32;                               // an accumulator has 64 columns
     // (a tile's w, maxima and sums come by bulk copy, tiles ahead: the workers' own loads stood between the scores and ds, 0.3 us per tile of
     // 1.4, 1.4 in a block's first at D = 32 with stored probabilities)
@@ -627,7 +683,7 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
     constexpr int TB = Img<D>::kTileBytes;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *p_s = STORED == 2 ? reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023) : smem_raw;
-    uint8_t *k_s = p_s + C::kStage, *v_s = k_s + (STORED ? 0 : 2 * TB), *t_s = v_s + 2 * TB;     // t_s: [stage][Q tile | dO tile]
+    uint8_t *k_s = p_s + C::kStage, *v_s = k_s + (STORED ? 0 : 2 * TB), *t_s = v_s + 2 * TB;     // t_s: [stage][Q tile | dO tile | its three pieces]
     __shared__ __align__(16) float rows_s[C::kStages][STORED ? 1 : 3][kTile];        // w and, to form P again, maximum and 1 / sum of a tile's queries
     __shared__ float down_s[kDownSlots][2][2][kLanes];                   // a tile's factors: [dV, dK][half][key]
     __shared__ uint64_t res_full, full[C::kStages], w_full[C::kStages], sd_full[2], ready[2], acc_done[2], p_full[STORED == 2 ? kPStages<D> : 1];
@@ -679,13 +735,15 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         const bool first = warp == kWorkerWarps;
         const uint8_t *q_img = img + (size_t)bh * Spad * (Img<D>::kBlock / 8);
         const uint8_t *k_img = q_img + img_bytes + (size_t)k0 * (Img<D>::kBlock / 8), *v_img = k_img + img_bytes, *g_img = q_img + 3 * img_bytes;
+        const uint8_t *g3_img = img + 4 * img_bytes + (size_t)bh * (Spad / kTile) * kTileBytes3<D>;
         auto fetch = [&](int i) {
             if (lane == 0 && i < total && seen) {
                 uint64_t *bar = &full[i % C::kStages];
-                uint8_t *dst = t_s + (i % C::kStages) * 2 * TB;
-                mbar_arrive_expect_tx(bar, 2 * TB);
+                uint8_t *dst = t_s + (i % C::kStages) * C::kPair;
+                mbar_arrive_expect_tx(bar, C::kPair);
                 bulk_load(dst, q_img + (size_t)(t0 + i) * TB, TB, bar);
                 bulk_load(dst + TB, g_img + (size_t)(t0 + i) * TB, TB, bar);
+                if (STORED) bulk_load(dst + 2 * TB, g3_img + (size_t)(t0 + i) * kTileBytes3<D>, kTileBytes3<D>, bar);
             }
             __syncwarp();
         };
@@ -726,11 +784,11 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         };
         auto issue_sd = [&](int i) {
             if (STORED && first) return;
-            const uint32_t d = tmem + (uint32_t)(i & 1) * C::kBuf, t = smem_u32(t_s + (i % C::kStages) * 2 * TB);
+            const uint32_t d = tmem + (uint32_t)(i & 1) * C::kBuf, t = smem_u32(t_s + (i % C::kStages) * C::kPair);
             wait(&full[i % C::kStages], (uint32_t)((i / C::kStages) & 1), 12);
             tc_fence_after();
             if (first) issue_scores<D>(d, smem_u32(k_s), t);
-            else issue_scores<D>(d + kTile, smem_u32(v_s), t + TB);
+            else issue_scores<D>(d + C::kColD, smem_u32(v_s), t + TB);
             if (elect_one()) tc_commit(&sd_full[i & 1]);
         };
         wait(&res_full, 0, 11);
@@ -751,9 +809,12 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
             tc_fence_after();
             if (STORED == 2 && first) fetch_p(i + kPStages<D>);      // the workers have read tile i of the probabilities
             if (!first) fetch_w(i + C::kStages);     // ... and its rows' statistics
-            const uint32_t s0 = tmem + (uint32_t)(i & 1) * C::kBuf, t = smem_u32(t_s + (i % C::kStages) * 2 * TB);
-            for (int half = 0; half < 2; ++half)
-                issue_accumulate<D, C::kWide, STORED != 0>(tmem + (first ? C::kColV : C::kColK) + 64 * half, s0 + (first ? 0 : kTile) + 32 * half, first ? t + TB : t, half);
+            const uint32_t s0 = tmem + (uint32_t)(i & 1) * C::kBuf, t = smem_u32(t_s + (i % C::kStages) * C::kPair);
+            if (STORED && first)
+                issue_exact<D>(tmem + C::kColV, s0, t + 2 * TB);
+            else
+                for (int half = 0; half < 2; ++half)
+                    issue_accumulate<D, C::kWide, STORED != 0>(tmem + (first ? C::kColV : C::kColK) + 64 * half, s0 + (first ? 0 : C::kColD) + 32 * half, first ? t + TB : t, half);
             if (elect_one()) tc_commit(&acc_done[i & 1]);
         }
         __syncwarp();
@@ -794,7 +855,8 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
     auto add_dkv = [&](int i) {                      // tile i has been accumulated
         wait_w(&acc_done[i & 1], (uint32_t)((i >> 1) & 1), 16);
         tc_fence_after();
-        add_tile<D, C::kWide>(lane_base + C::kColV, hf, down_s[i % kDownSlots][0][0][rloc], down_s[i % kDownSlots][0][1][rloc], ov);
+        if (STORED) add_exact<D>(lane_base + C::kColV, hf, ov);
+        else add_tile<D, C::kWide>(lane_base + C::kColV, hf, down_s[i % kDownSlots][0][0][rloc], down_s[i % kDownSlots][0][1][rloc], ov);
         add_tile<D, C::kWide>(lane_base + C::kColK, hf, down_s[i % kDownSlots][1][0][rloc], down_s[i % kDownSlots][1][1][rloc], ok);
     };
     // factors: of this key's K (with the exponent's) and V, and of 32 tiles of Q and dO, one per lane
@@ -803,7 +865,7 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
     float q_facs = 0.0f, g_facs = 0.0f;
     if (STORED == 1) fetch_p(0);
     for (int i = 0; i < total; ++i) {
-        const uint32_t s_addr = lane_base + (uint32_t)(i & 1) * C::kBuf + hf * 32, dp_addr = s_addr + kTile;
+        const uint32_t s_addr = lane_base + (uint32_t)(i & 1) * C::kBuf + hf * 32, dp_addr = s_addr + C::kColD;
         const int qb = (t0 + i) * kTile + hf * 32;
         if ((i & 31) == 0) {
             const size_t ft = tile0 + min(t0 + i + lane, Spad / kTile - 1);
@@ -856,7 +918,8 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
             const float2 e = fmul2(make_float2(p[x + 2], p[x + 3]), ffma2(make_float2(d[x + 2], d[x + 3]), dp2, make_float2(-w4.z, -w4.w)));
             d[x] = a.x; d[x + 1] = a.y; d[x + 2] = e.x; d[x + 3] = e.y;
         }
-        down_s[i % kDownSlots][0][hf][rloc] = store_pieces(p, s_addr) * g_fac;
+        if (STORED) store_exact(p, s_addr - hf * 16);
+        else down_s[i % kDownSlots][0][hf][rloc] = store_pieces(p, s_addr) * g_fac;
         down_s[i % kDownSlots][1][hf][rloc] = store_pieces(d, dp_addr) * q_fac;
         if (i > 0) add_dkv(i - 1);
         tmem_wait_st();
@@ -866,7 +929,7 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
     // (through the tiles' memory: the last products have read it)
     const int row0 = k0 + wq * 32;
     const size_t dst = ((size_t)b * S + row0) * E + (size_t)h * D;
-    store_out<D>(ov, warp, lane, 1.0f, kSumLoss, t_s, dV + dst, E, S - row0, abort_flag);
+    store_out<D>(ov, warp, lane, 1.0f, STORED ? 0.0f : kSumLoss, t_s, dV + dst, E, S - row0, abort_flag);
     store_out<D>(ok, warp, lane, c, kScoreLoss, t_s + TB * 2, dK + dst, E, S - row0, abort_flag);
     tc_fence_before();
     __syncthreads();
@@ -882,30 +945,30 @@ int launch_cfg(const float *g, const float *q, const float *k, const float *v, c
     auto cols = bwd_cols_kernel<D, CAUSAL, STORED>;
     constexpr size_t rows_smem = RowsCfg<D, STORED>::kSmem, cols_smem = ColsCfg<D, STORED>::kSmem;
     static_assert(rows_smem + ((STORED ? 1 : 3) + kDownSlots) * 2 * kLanes * 4 + 256 <= 232448 &&
-                  cols_smem + ColsCfg<D, STORED>::kStages * (STORED ? 1 : 3) * kTile * 4 + kDownSlots * 4 * kLanes * 4 + 512 <= 232448, "shared memory of a block");
+                  cols_smem + ColsCfg<D, STORED>::kStages * (STORED ? 1 : 3) * kTile * 4 + kDownSlots * 4 * kLanes * 4 + 512 <= 232448 && ColsCfg<D, STORED>::kColK + 128 <= kTmemCols, "shared memory of a block");
     cudaError_t e = cudaFuncSetAttribute(rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(cols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cols_smem);
     if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     const int nblk = (S + kLanes - 1) / kLanes, Spad = nblk * kLanes;
-    // groups of batches whose images (4 bytes per element) stay in L2 between the kernels that write and read them
-    const size_t per_batch = (size_t)4 * H * Spad * D * 4;
+    // groups of batches whose images (4 bytes per element, 6 more for dO's three pieces) stay in L2 between the kernels that write and read them
+    const size_t per_batch = (size_t)H * Spad * D * (STORED ? 22 : 16);
     long long gb = (long long)((64u << 20) / per_batch);
     gb = gb < 1 ? 1 : gb > B ? B : gb;
     while (gb > 1 && gb * H * (long long)(Spad / kTile) > 2000000000LL) gb /= 2;
-    const size_t img_bytes = (size_t)gb * H * Spad * D * 4, nstat = (size_t)gb * H * Spad;
+    const size_t img_bytes = (size_t)gb * H * Spad * D * 4, exact_bytes = STORED ? img_bytes / 2 * 3 : 0, nstat = (size_t)gb * H * Spad;
     StreamWorkspace::Lease ws;
-    int rc = g_bwd_ws.enter(st, 4 * img_bytes + ((STORED ? 1 : 3) * nstat + 4 * (nstat / kTile)) * sizeof(float), &ws);
+    int rc = g_bwd_ws.enter(st, 4 * img_bytes + exact_bytes + ((STORED ? 1 : 3) * nstat + 4 * (nstat / kTile)) * sizeof(float), &ws);
     if (rc != HIPGPT_OK) return rc;
     uint8_t *img = ws.get();
     // beside the images: w and, where P is formed again, maximum and 1 / sum of the rows; the tiles' factors
-    float *stat = reinterpret_cast<float *>(img + 4 * img_bytes), *fac = stat + (STORED ? 1 : 3) * nstat;
+    float *stat = reinterpret_cast<float *>(img + 4 * img_bytes + exact_bytes), *fac = stat + (STORED ? 1 : 3) * nstat;
     const float c = 1.0f / sqrtf((float)D);
     const int expire = take_expiry(600);
     for (long long b0 = 0; b0 < B; b0 += gb) {
         const int nb = (int)(B - b0 < gb ? B - b0 : gb);
         const size_t off = (size_t)b0 * S * E;
         const float *p = STORED ? probs + (size_t)b0 * H * S * S : nullptr;
-        e = launch_overlapped(bwd_pack_kernel<D>, dim3((unsigned)(nb * H * (Spad / kTile)), 4), dim3(256), 0, st, q + off, k + off, v + off, g + off, img, img_bytes, fac, S, Spad / kTile, E, H);
+        e = launch_overlapped(bwd_pack_kernel<D>, dim3((unsigned)(nb * H * (Spad / kTile)), 4), dim3(256), 0, st, q + off, k + off, v + off, g + off, img, img_bytes, fac, STORED ? img + 4 * img_bytes : (uint8_t *)nullptr, S, Spad / kTile, E, H);
         if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "bwd_pack_kernel launch: %s", cudaGetErrorString(e));
         PMap<STORED> rows_map = {}, cols_map = {};
         if constexpr (STORED == 2) {

@@ -579,6 +579,42 @@ def test_attention_backward_with_the_full_range_asked_for(D, S, stored):
     assert np.array_equal(_run_backward(g0, qkv, probs, B, S, E, H, True), before)
 
 
+@pytest.mark.parametrize("D,S", [(32, 5), (32, 128), (32, 201), (32, 256), (64, 66), (64, 128), (32, 388), (32, 301), (64, 200), (64, 387)])
+def test_attention_backward_moves_rows_of_one_probability_unchanged(D, S):
+    """Stored probabilities of one key each, a permutation: dV is dO's rows bit for bit, whatever their magnitudes (powers of two over 2^100)."""
+    B, H = 2, 2
+    E = H * D
+    rng = np.random.default_rng(S)
+    qkv, g = synth.qkv_planes(880 + S, B, S, E), synth.normal(881 + S, (B, S, H, D)) * (2.0 ** rng.integers(-50, 51, (B, S, H, 1))).astype(np.float32)
+    keys = np.stack([rng.permutation(S) for _ in range(B * H)]).reshape(B, H, S)
+    probs = np.zeros((B, H, S, S), np.float32)
+    np.put_along_axis(probs, keys[..., None], 1.0, axis=-1)
+    dv = _run_backward(g.reshape(B * S, E), qkv, probs, B, S, E, H, False, planes=True).reshape(3, B, S, H, D)[2]
+    for b in range(B):
+        for h in range(H):
+            assert np.array_equal(dv[b, keys[b, h], h], g[b, :, h])
+
+
+@pytest.mark.parametrize("shape", [(8, 8, 256, 32), (8, 8, 128, 64), (4, 8, 700, 32), (2, 12, 777, 64)])
+@pytest.mark.parametrize("causal,stored", [(False, True), (False, False), (True, False)])
+def test_attention_backward_is_not_smaller_or_larger_than_it_should_be_on_the_average(shape, causal, stored):
+    """The tensor core truncates where it adds; what that takes on the average, on unit normals, is given back: what is left is below a unit in the last
+    place (2^-23) of the gradients as a whole."""
+    B, H, S, D = shape
+    E = H * D
+    gen = torch.Generator(device="cuda").manual_seed(S + D)
+    qkv, g = torch.randn(3, B * S, E, generator=gen, device="cuda"), torch.randn(B * S, E, generator=gen, device="cuda")
+    p = torch.empty(B, H, S, S, device="cuda") if stored else None
+    out, grad = torch.empty(B * S, E, device="cuda"), torch.empty(3, B * S, E, device="cuda")
+    if stored:
+        _capi.check(_capi.lib().hipgpt_mha_forward_planes(qkv.data_ptr(), out.data_ptr(), p.data_ptr(), B, S, E, H, int(causal), _st()))
+    _capi.check(_capi.lib().hipgpt_mha_backward_planes(g.data_ptr(), qkv.data_ptr(), p.data_ptr() if stored else None, grad.data_ptr(), B, S, E, H, int(causal), _st()))
+    want = _backward_in_64_bits(g, qkv, p, B, S, E, H, causal)[0]
+    for plane in range(3):
+        off = float(((grad[plane].double() - want[plane]) * want[plane]).sum() / (want[plane] ** 2).sum())
+        assert abs(off) <= 2.0 ** -23, (plane, off)
+
+
 def test_attention_backward_reference_named_launcher():
     raw = C.CDLL(_capi.lib_path())
     fn = getattr(raw, _capi.CXX_LAUNCHERS["launch_multihead_attention_backward"])
