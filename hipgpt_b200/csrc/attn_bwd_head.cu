@@ -19,9 +19,9 @@
 // The queries of the other block contribute to this block's keys: their sums come through distributed shared memory at the end.
 //
 // Measured, us, three kernels -> one: B=32 H=8 S=256 D=32 with stored probabilities 94.9 -> 77.3, causal without 80.9 -> 70.1; S=161 (probabilities that TMA cannot
-// address) 84.7 -> 86.1, causal without 69.1 -> 59.8; B=16 H=12 S=128 D=32 stored 31.2 -> 24.9; B=64 H=12 S=35 82.0 -> 60.2; D=64: B=32 H=8 S=128 stored 46.2 -> 35.4, causal
-// without 46.2 -> 32.7; B=9 H=16 S=101 27.2 -> 19.5.  But for odd lengths just above 128 at D=32, where both are the same, the one is faster throughout.
-// Relative error of the gradients against float64: 1.45, 1.40, 0.90e-7 (dQ, dK, dV) at the first, 1.42, 1.40, 0.83e-7 at B=8 H=8 S=128 D=64 stored; three bf16
+// address) 84.7 -> 86.1, causal without 69.1 -> 59.8; B=16 H=12 S=128 D=32 stored 31.2 -> 25.2; B=64 H=12 S=35 82.0 -> 61.9; D=64: B=32 H=8 S=128 stored 46.2 -> 36.1, causal
+// without 46.2 -> 32.7; B=9 H=16 S=101 27.2 -> 19.6.  But for odd lengths just above 128 at D=32, where both are the same, the one is faster throughout.
+// Relative error of the gradients against float64: 1.45, 1.40, 0.90e-7 (dQ, dK, dV) at the first, 1.37, 1.40, 0.83e-7 at B=8 H=8 S=128 D=64 stored; three bf16
 // pieces and six products throughout: 1.47, 1.68, 0.94e-7 and 1.41, 1.63, 0.83e-7.  (dV of two fp16 pieces: 1.03 and 0.95e-7; 69.0 us at the first.)
 // What bounds it: a block takes 33200 cycles at the first shape, 3.5 rounds of them.  9700 until its operands are cut and g V^T is there (224 KB come in at
 // 64 bytes per clock; the cut is bound by the instructions of conversion), 4500 for w and the scales, 5300 for ds and its pieces, 4300 for the products with
@@ -41,7 +41,7 @@ constexpr int kThreads = kWorkerWarps * 32 + 64;
 constexpr int kCols = 16;                // of a tile's 64 columns, per thread
 constexpr uint32_t kTmemCols = 512;
 // What the tensor core's truncation takes from the results on the average (attn_bwd_tc.cu), given back with the last multiplication
-constexpr float kSumLoss = 7.3e-8f, kScoreLoss = 1.65e-7f;
+constexpr float kSumLoss = 7.3e-8f, kScoreLoss = 1.65e-7f, kScoreLoss32 = 1.3e-7f;      // the last: accumulators of 32
 
 __device__ int g_bwd_head_status = 0;
 
@@ -86,7 +86,7 @@ struct HeadCfg {
     static constexpr bool kWide = D == 32;                               // products with [hi | lo] at once, accumulators of 64 columns either way
     static constexpr int kTiles = 2 * NB;                                // of 64 keys
     // columns of TMEM: dP (ds, dQ's sums of a tile); scores, then the sums of dV and dK, [block of keys][64 queries]
-    static constexpr int kColAcc = 256, kColK = D == 32 ? 0 : 128;
+    static constexpr int kColAcc = 256, kColK = D == 32 ? 0 : 128, kColQ2 = 384;
     // tiles of 64 rows of the planes
     // dV of stored probabilities: g's image as three bf16 pieces, in V's and K's place (behind what the other block sends); pieces of P in TMEM, 96 columns per 64 queries, then sums
     static constexpr int kExactG = kV + (NB > 1 ? 16384 : 0), kCols3 = 96;
@@ -112,6 +112,10 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
                 int S, int E, int H, float c, int by_tma, int ahead, const __grid_constant__ CUtensorMap p_map, int expire)
 {
     using C = HeadCfg<D, NB>;
+    // One block per head and stored probabilities, whose dV takes no columns yet: a tile's dQ from two accumulators of 32 keys, so that less is truncated
+    // (B=8 H=8: dQ 1.42 -> 1.37e-7 at S = 128 D = 64, 1.39 -> 1.36e-7 at S = 64 D = 32, where three bf16 pieces gave 1.41 and 1.38; 35.4 -> 36.1 us at B=32 H=8 S=128 D=64)
+    constexpr bool kHalves = STORED && NB == 1;
+    constexpr int kColK = STORED ? 0 : C::kColK;
     constexpr int TB = C::TB;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *sm = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -189,16 +193,16 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
         };
         // acc (128 x D; WIDE: 2 D, the products with B's lo pieces apart) = A B over 64 rows of B's image, read N-major.  da: the descriptor of A's hi
         // pieces; a_step: 16 reductions on, in 16 bytes; id: A K- or M-major.  The small products first, a fresh accumulator per 64.
-        auto sums = [&](uint32_t acc, uint64_t da, int a_step, uint32_t id, const uint8_t *bs) {
+        auto sums = [&](uint32_t acc, uint64_t da, int a_step, uint32_t id, const uint8_t *bs, int from = 0, int to = 4) {
             const uint64_t db = make_desc(smem_u32(bs), Img<D>::kBlock, 128, 0);
             enum { kFresh, kDown, kMore };           // how a product finds the accumulator
             auto product = [&](int pa, int pb, int start) {
 #pragma unroll
                 for (int ks = 0; ks < 4; ++ks)
-                    if (elect_one()) {
+                    if (ks >= from && ks < to && elect_one()) {
                         const uint64_t ak = da + (uint64_t)(pa * (kPiecePart >> 4) + ks * a_step), bk = db + (uint64_t)(ks * 2 * (Img<D>::kBlock >> 4) + pb * (Img<D>::kPiece >> 4));
-                        if (start == kDown && ks == 0) mma_h_ss_down<kLowShift>(acc, ak, bk, id);
-                        else mma_h_ss(acc, ak, bk, id, start == kFresh && ks == 0 ? 0u : 1u);
+                        if (start == kDown && ks == from) mma_h_ss_down<kLowShift>(acc, ak, bk, id);
+                        else mma_h_ss(acc, ak, bk, id, start == kFresh && ks == from ? 0u : 1u);
                     }
             };
             if (!C::kWide && STORED) product(1, 1, kFresh);      // (WIDE has it in any case.  Formed probabilities carry more than it takes away)
@@ -233,9 +237,13 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
             const int kb = block_at(i);
             wait(&sh.d_ready[i], 0, 24);
             tc_fence_after();
-            sums(tmem + C::kColAcc + C::kColK + kb * 128 + 64 * mine, keys_desc(kb, mine), 256 >> 4, id_sums | (1u << 15), q_s + mine * TB);
+            sums(tmem + C::kColAcc + kColK + kb * 128 + 64 * mine, keys_desc(kb, mine), 256 >> 4, id_sums | (1u << 15), q_s + mine * TB);
             const int t = 2 * kb + mine;
-            if (t < ntile) sums(tmem + t * kTile, make_desc(smem_u32(p_s + t * 2 * kGroup), kKeys8, 128, 0), 2 * kKeys8 >> 4, id_sums, k_s + t * TB);
+            if (t < ntile) {
+                const uint64_t da = make_desc(smem_u32(p_s + t * 2 * kGroup), kKeys8, 128, 0);
+                sums(tmem + t * kTile, da, 2 * kKeys8 >> 4, id_sums, k_s + t * TB, 0, kHalves ? 2 : 4);
+                if (kHalves) sums(tmem + C::kColQ2 + t * kTile, da, 2 * kKeys8 >> 4, id_sums, k_s + t * TB, 2, 4);
+            }
             if (elect_one()) tc_commit(&sh.k_done[i]);
         }
         if (NB > 1) {                                // (before the workers are needed again: theirs wait for these arrivals too)
@@ -615,7 +623,7 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
         const int kb = block_at(i);
         wait(&sh.k_done[i], 0, 26);
         tc_fence_after();
-        key_sums(lane_base + C::kColAcc + C::kColK + kb * 128, range_down(e_d(2 * kb + u, 0)) * sh.fac[C::tQ], range_down(e_d(2 * kb + u, 1)) * sh.fac[C::tQ + 1], ok);
+        key_sums(lane_base + C::kColAcc + kColK + kb * 128, range_down(e_d(2 * kb + u, 0)) * sh.fac[C::tQ], range_down(e_d(2 * kb + u, 1)) * sh.fac[C::tQ + 1], ok);
         if (NB > 1 && i == 0) {                      // (every block takes both steps of the cluster's barrier twice)
             if (!joined) cluster_wait();
             if (kb != blk) {
@@ -629,19 +637,32 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
             cluster_arrive();
         }
         float a[2][OC], z[2][OC];
+        auto load_q = [&](uint32_t col) {
 #pragma unroll
-        for (int y = 0; y < 2; ++y) {
-            if (2 * kb + y >= ntile) break;
-            load_acc(lane_base + (2 * kb + y) * kTile + cf * OC, a[y]);
-            if (C::kWide) load_acc(lane_base + (2 * kb + y) * kTile + D + cf * OC, z[y]);
-        }
-        tmem_wait_ld();
+            for (int y = 0; y < 2; ++y) {
+                if (2 * kb + y >= ntile) break;
+                load_acc(lane_base + col + (2 * kb + y) * kTile + cf * OC, a[y]);
+                if (C::kWide) load_acc(lane_base + col + (2 * kb + y) * kTile + D + cf * OC, z[y]);
+            }
+            tmem_wait_ld();
+        };
+        load_q(0);
 #pragma unroll
         for (int y = 0; y < 2; ++y) {
             if (2 * kb + y >= ntile) break;
             const float f = range_down(e_d(2 * kb + y, u)) * sh.fac[C::tK + 2 * kb + y];
 #pragma unroll
             for (int x = 0; x < OC; ++x) oq[x] = fmaf(C::kWide ? fmaf(z[y][x], kLowDown, a[y][x]) : a[y][x], f, oq[x]);
+        }
+        if (kHalves) {
+            load_q(C::kColQ2);
+#pragma unroll
+            for (int y = 0; y < 2; ++y) {
+                if (2 * kb + y >= ntile) break;
+                const float f = range_down(e_d(2 * kb + y, u)) * sh.fac[C::tK + 2 * kb + y];
+#pragma unroll
+                for (int x = 0; x < OC; ++x) oq[x] = fmaf(C::kWide ? fmaf(z[y][x], kLowDown, a[y][x]) : a[y][x], f, oq[x]);
+            }
         }
     }
     // 32 rows x 32 columns leave in whole lines: through shared memory (16-byte pieces permuted by the row), then a row of 128 bytes per eight lanes
@@ -739,7 +760,7 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
         meet();                                      // (who has not seen a wait run out: the last word on it)
     }
     bool off = sh.abort_flag;
-    store_rows(oq, c, kScoreLoss, q_s, dQ, off);
+    store_rows(oq, c, kHalves ? kScoreLoss32 : kScoreLoss, q_s, dQ, off);
     if (NB > 1) {
         cluster_wait();
         if (!CAUSAL || blk == 0) {
