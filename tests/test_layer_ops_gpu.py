@@ -615,6 +615,28 @@ def test_attention_backward_is_not_smaller_or_larger_than_it_should_be_on_the_av
         assert abs(off) <= 2.0 ** -23, (plane, off)
 
 
+@pytest.mark.parametrize("D,S", [(32, 300), (64, 200)])
+@pytest.mark.parametrize("stored", [False, True])
+def test_attention_backward_long_contexts_of_any_magnitude_and_captured_into_a_graph(D, S, stored):
+    B, H = 2, 2
+    E = H * D
+    qkv = synth.qkv_planes(832 + S, B, S, E).reshape(3, B * S, E)
+    qkv[0] *= np.float32(1e-6); qkv[1] *= np.float32(1e6); qkv[2] *= np.float32(3e8)
+    g = synth.normal(833 + S, (B * S, E)) * np.float32(2e-9)
+    probs = ob.mha(qkv, B, S, E, H, want_probs=True)[1] if stored else None
+    got = _run_backward(g, qkv, probs, B, S, E, H, False)
+    _assert_rows_are_near(got, *_backward_in_64_bits(g, qkv, probs, B, S, E, H, False))
+    dg, dq, dp, dout = dev(g), dev(qkv), dev(probs) if stored else None, torch.full((3, B * S, E), float("nan"), device="cuda")
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        _capi.check(_capi.lib().hipgpt_mha_backward_planes(dg.data_ptr(), dq.data_ptr(), dp.data_ptr() if stored else None, dout.data_ptr(), B, S, E, H, 0, _st()))
+    for _ in range(2):
+        dout.fill_(float("nan"))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert np.array_equal(dout.cpu().numpy().reshape(-1), got)
+
+
 def test_attention_backward_reference_named_launcher():
     raw = C.CDLL(_capi.lib_path())
     fn = getattr(raw, _capi.CXX_LAUNCHERS["launch_multihead_attention_backward"])
