@@ -124,10 +124,12 @@ def lib() -> C.CDLL:
 
 
 def native():
-    """The extension with the hot calls of launchers.py, built with the library."""
-    if not os.path.exists(_build.EXT):
-        _build.build()
-    loader = importlib.machinery.ExtensionFileLoader("hipgpt_launch", _build.EXT)
+    """The extension with the hot calls of launchers.py, built first if there is none for this Python and torch (needs g++)."""
+    lib()
+    path = _build.extension_path()
+    if not os.path.exists(path):
+        _build.build_extension()
+    loader = importlib.machinery.ExtensionFileLoader("hipgpt_launch", path)
     module = importlib.util.module_from_spec(importlib.util.spec_from_loader("hipgpt_launch", loader))
     loader.exec_module(module)
     return module

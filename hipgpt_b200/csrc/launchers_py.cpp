@@ -13,7 +13,8 @@
 
 namespace {
 
-PyObject *g_any_ptr = nullptr, *g_any_bf16 = nullptr;        // launchers._ptr and _ptr_bf16: for what is not exactly a tensor
+// launchers._ptr and _ptr_bf16, for what is not exactly a tensor; _int, for what is not an int
+PyObject *g_any_ptr = nullptr, *g_any_bf16 = nullptr, *g_any_int = nullptr;
 
 // A contiguous CUDA tensor of `type` (for float32 also None or an address) -> its address; false with an exception set
 bool address_of(PyObject *o, at::ScalarType type, void **out)
@@ -38,11 +39,14 @@ bool address_of(PyObject *o, at::ScalarType type, void **out)
 bool ints(PyObject *const *args, int n, int *out)
 {
     for (int i = 0; i < n; ++i) {
-        if (!PyLong_Check(args[i])) {
-            PyErr_Format(PyExc_TypeError, "int expected instead of %s instance", Py_TYPE(args[i])->tp_name);
-            return false;
+        if (PyLong_Check(args[i])) {
+            out[i] = static_cast<int>(PyLong_AsUnsignedLongMask(args[i]));
+            continue;
         }
-        out[i] = static_cast<int>(PyLong_AsUnsignedLongMask(args[i]));
+        PyObject *x = PyObject_CallOneArg(g_any_int, args[i]);
+        if (!x) return false;
+        out[i] = static_cast<int>(PyLong_AsUnsignedLongMask(x));
+        Py_DECREF(x);
     }
     return !PyErr_Occurred();
 }
@@ -118,7 +122,8 @@ PyObject *decode(PyObject *, PyObject *const *a, Py_ssize_t n)
 
 PyObject *bind(PyObject *, PyObject *const *a, Py_ssize_t n)
 {
-    if (!count(n, 2)) return nullptr;
+    if (!count(n, 3)) return nullptr;
+    Py_XSETREF(g_any_int, Py_NewRef(a[2]));
     Py_XSETREF(g_any_ptr, Py_NewRef(a[0]));
     Py_XSETREF(g_any_bf16, Py_NewRef(a[1]));
     Py_RETURN_NONE;

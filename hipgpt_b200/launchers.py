@@ -6,6 +6,9 @@ streams only; every kernel is the library's own.
 """
 from __future__ import annotations
 
+import ctypes
+import warnings
+
 import torch
 
 from . import _capi
@@ -39,8 +42,58 @@ def _stream():
     return _raw_stream(_current_device())
 
 
-_native = _capi.native()
-_native.bind(_ptr, _ptr_bf16)
+class ArgumentError(ctypes.ArgumentError, TypeError):
+    """A size that is no integer."""
+
+
+def _int(x):
+    """What ctypes takes for an int: an int, a c_int, or what stands for one."""
+    if isinstance(x, int):
+        return x
+    if isinstance(x, ctypes.c_int):
+        return x.value
+    if hasattr(x, "_as_parameter_"):
+        return _int(x._as_parameter_)
+    raise ArgumentError(f"int expected instead of {type(x).__name__} instance")
+
+
+class _ThroughCtypes:
+    """The extension's calls without it."""
+
+    @staticmethod
+    def attention(d_qkv, d_output, d_attn_probs, B, S, E, H, causal):
+        return _capi.lib().hipgpt_mha_forward_planes(_ptr(d_qkv), _ptr(d_output), _ptr(d_attn_probs), _int(B), _int(S), _int(E), _int(H), causal, _stream())
+
+    @staticmethod
+    def attention_bf16(d_qkv, d_output, B, S, E, H, causal, variant):
+        p, out = _ptr_bf16(d_qkv), _ptr_bf16(d_output)
+        plane = B * S * E * 2                               # bytes
+        return _capi.lib().hipgpt_mha_forward_bf16_ex(p, p + plane, p + 2 * plane, out, B, S, E, H, causal, variant, _stream())
+
+    @staticmethod
+    def decode(q, kcache, vcache, out, scratch, nbytes, B, H, D, ctx, cap):
+        p = [_ptr(t) for t in (q, kcache, vcache, out, scratch)]
+        if nbytes is None:
+            nbytes = 0 if scratch is None else scratch.numel() * scratch.element_size()
+        return _capi.lib().hipgpt_mha_decode(*p, nbytes, _int(B), _int(H), _int(D), _int(ctx), _int(cap), _stream())
+
+
+class _AtFirstCall:
+    """Stands for the extension until it is needed: importing this module builds and loads nothing."""
+
+    def __getattr__(self, name):
+        global _native
+        try:
+            native = _capi.native()
+            native.bind(_ptr, _ptr_bf16, _int)
+        except (RuntimeError, ImportError, OSError) as e:       # no g++, no headers: the same library through ctypes
+            warnings.warn(f"the extension of the hot calls cannot be built or loaded, they go through ctypes (a few microseconds more each): {e}", RuntimeWarning, stacklevel=3)
+            native = _ThroughCtypes
+        _native = native
+        return getattr(native, name)
+
+
+_native = _AtFirstCall()
 
 
 def launch_multihead_attention(d_qkv, d_output, d_attn_probs, B: int, S: int, E: int, H: int, *, causal: bool = False):
