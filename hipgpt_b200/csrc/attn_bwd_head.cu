@@ -67,12 +67,6 @@ __device__ __forceinline__ void peer_store4(uint32_t addr, float a, float b, flo
     asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }
 
-// 32 bytes, aligned
-__device__ __forceinline__ void load_sector(const float4 *src, float4 (&x)[2])
-{
-    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];" : "=f"(x[0].x), "=f"(x[0].y), "=f"(x[0].z), "=f"(x[0].w), "=f"(x[1].x), "=f"(x[1].y), "=f"(x[1].z), "=f"(x[1].w) : "l"(src));
-}
-
 // The pieces of P and of ds, [8 keys][piece][8 queries] core matrices of 128 bytes: 16 of them along the queries.
 constexpr int kPiecePart = 16 * 128, kKeys8 = 2 * kPiecePart, kGroup = 4 * kKeys8;          // a piece of 8 keys, 8 keys, 32 keys
 
@@ -310,7 +304,7 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
             for (int p = 0; p < PARTS; ++p) {
                 x[t][p][0] = x[t][p][1] = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (here && sectors) {
-                    load_sector(p4 + 8 * p, x[t][p]);
+                    load_sector(p4 + 8 * p, x[t][p][0], x[t][p][1]);
                 } else if (here) {
                     x[t][p][0] = p4[8 * p];
                     x[t][p][1] = p4[8 * p + 1];

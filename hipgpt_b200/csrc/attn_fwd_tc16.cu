@@ -188,8 +188,9 @@ kv_pack_kernel(const float *__restrict__ K, const float *__restrict__ V, float *
     const float *src = (vside ? V : K) + ((size_t)b * S + kt * kKeys) * (size_t)E + (size_t)h * D + 8 * pc;
     float4 xa[NP], xc[NP];
     float mx = 0.0f;
-    // At head_dim 64 whole sectors (where the planes allow it) that leave L2 first, so that the images stay: B=4 H=8 S=2048 causal 64.6 -> 62.7 us per call,
-    // B=16 H=8 S=1024 88.9 -> 88.0, unmasked 130.5 -> 129.8.  At 32, where K and V are smaller and may be found in L2, 24.6 -> 25.3 (B=8 H=9 S=700).
+    // At head_dim 64 whole sectors, where the planes allow it: B=4 H=8 S=2048 causal 62.5 -> 61.1 us per call, B=16 H=8 S=1024 91.3 -> 86.9 - 88.9, S=400 17.9 -> 17.7.
+    // (Marked to leave L2 first they were no faster, 60.7 - 61.0, 85.9 - 92.5 and 18.0, and a backward that reads the planes again lost by it: B=3 H=12 S=777, forward and
+    // backward, 105.9 us without the mark and 106.8 with it.)  At 32, where K and V are smaller and may be found in L2, 24.6 -> 25.3 (B=8 H=9 S=700).
     const bool sectors = D == 64 && ((reinterpret_cast<uintptr_t>(K) | reinterpret_cast<uintptr_t>(V)) & 31) == 0;
 #pragma unroll
     for (int i = 0; i < NP; ++i) {
@@ -199,7 +200,7 @@ kv_pack_kernel(const float *__restrict__ K, const float *__restrict__ V, float *
         const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
         xa[i] = xc[i] = z;
         if (ok && sectors) {
-            load_sector_once(p, xa[i], xc[i]);
+            load_sector(p, xa[i], xc[i]);
         } else if (ok) {
             xa[i] = __ldg(p);
             xc[i] = __ldg(p + 1);

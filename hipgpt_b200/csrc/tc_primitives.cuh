@@ -100,10 +100,10 @@ __device__ __forceinline__ void tma_prefetch_3d(const void *tensor_map, int c0, 
                  ::"l"(reinterpret_cast<uint64_t>(tensor_map)), "r"(c0), "r"(c1), "r"(c2) : "memory");
 }
 
-// One whole 32-byte sector (src 32-byte aligned) that is read this once: it leaves L2 first.
-__device__ __forceinline__ void load_sector_once(const float4 *src, float4 &a, float4 &b)
+// One whole 32-byte sector (src 32-byte aligned).
+__device__ __forceinline__ void load_sector(const float4 *src, float4 &a, float4 &b)
 {
-    asm volatile("ld.global.L1::no_allocate.L2::evict_first.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                  : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w) : "l"(src));
 }
 
