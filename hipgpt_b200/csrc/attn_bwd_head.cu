@@ -56,12 +56,6 @@ __device__ __noinline__ bool head_wait_slow(uint64_t *bar, uint32_t parity, int 
 
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-__device__ __forceinline__ uint32_t peer_of(uint32_t addr, int rank)
-{
-    uint32_t r;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-    return r;
-}
 __device__ __forceinline__ void peer_store4(uint32_t addr, float a, float b, float c, float d)
 {
     asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
@@ -574,7 +568,7 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
     const int recv = cf * 2 * kLanes * 16 + rloc * 16;                   // [dV, dK][quarter][16 bytes][key]
     auto send = [&](const float (&o)[OC], int what) {
         if constexpr (NB > 1) {
-            const uint32_t to = peer_of(smem_u32(v_s) + recv + what * 16384, blk ^ 1);
+            const uint32_t to = peer_addr(smem_u32(v_s) + recv + what * 16384, blk ^ 1);
 #pragma unroll
             for (int x = 0; x < 2; ++x) peer_store4(to + x * (kLanes * 16), o[4 * x], o[4 * x + 1], o[4 * x + 2], o[4 * x + 3]);
         }
@@ -624,7 +618,7 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
                 send(ok, STORED ? 0 : 1);
                 // a warp that has seen a wait run out, its own or one that its sums depend on, says so
                 if (lane == 0 && sh.abort_flag) {
-                    const uint32_t gone = peer_of(smem_u32(const_cast<int *>(&sh.peer_gone)), blk ^ 1);
+                    const uint32_t gone = peer_addr(smem_u32(const_cast<int *>(&sh.peer_gone)), blk ^ 1);
                     asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(gone), "r"(1) : "memory");
                 }
             }

@@ -48,12 +48,6 @@ constexpr int kSmemMost = 232448 - 1024;
 constexpr int kLayersChecked = 4;                // layers between two looks at whether a wait has run out
 constexpr int kAhead = 4;                        // key / value rows per lane asked for ahead of the projection
 
-__device__ __forceinline__ uint32_t peer_addr(uint32_t addr, int rank)
-{
-    uint32_t r;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-    return r;
-}
 // 16 or 8 bytes into a block of the cluster, counted on the mbarrier there
 __device__ __forceinline__ void send4(uint32_t addr, uint32_t bar, float4 v)
 {

@@ -76,6 +76,13 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t *bar, uint32_t by
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
 
+__device__ __forceinline__ uint32_t peer_addr(uint32_t addr, int rank)
+{
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+
 // TMA: one box of a rank-3 tensor map (this GPU's own memory; no multicast) into shared memory; the
 // bytes count towards `bar`.  c0 is the innermost coordinate: c0 * element size must be a multiple
 // of 16 bytes.
