@@ -36,11 +36,12 @@ namespace {
 // 256 -> 1024 105 -> 83, 1024 -> 256 125 -> 92.
 // Small products (TN = 4) are bound by neither but by the distance from a load to its use and by what a stage costs besides: their fragments are read
 // eight inner indices of B and four of A ahead, a stage has 32 inner indices, and where few tiles have to fill many SMs a block has TY = 4 rows of
-// threads instead of 8: half as many warps at the return path.  Rows x inner x columns: 100 x 1024 x 256 21.1 -> 12.4 us, 400 x 256 x 768 9.8 -> 7.5,
+// threads instead of 8: half as many warps at the return path.  (Not where each SM has many tiles and each few inner indices: three short stages then, which take little
+// memory, so that many blocks share an SM.)  Rows x inner x columns: 100 x 1024 x 256 21.1 -> 12.4 us, 400 x 256 x 768 9.8 -> 7.5,
 // 200 x 2048 x 512 41.3 -> 30.9, 2000 x 768 x 192 28.0 -> 19.5.  (Deeper stages for the tiles between, 5 x 8 and so on: 1407 x 512 x 2048 65 -> 66.)
-template <int TM, int TN, int TY>
+template <int TM, int TN, int TY, bool DEEP>
 struct TileCfg {
-    static constexpr bool kSmall = TN == 4;
+    static constexpr bool kSmall = DEEP;
     static constexpr int kBK = kSmall ? 32 : 16, kStages = kSmall ? 5 : 3;         // inner indices of a stage
     static constexpr int kThreads = 16 * TY, BM = TY * TM, BN = 16 * TN;
     static constexpr int kAheadB = kSmall ? 8 : 2, kAheadA = kSmall ? 2 : 1;      // fragments in registers: of an index of B, of four of A
@@ -48,12 +49,12 @@ struct TileCfg {
     static constexpr int kStageFloats = BM * AStride + kBK * BN;
     static constexpr size_t kSmem = (size_t)kStages * kStageFloats * 4;
 };
-template <int TM, int TN, int TY>
+template <int TM, int TN, int TY, bool DEEP>
 __global__ void __launch_bounds__(16 * TY, TM * TN > 64 ? 2 : 3)
 matmul_tile_kernel(const float *A, const float *__restrict__ B, const float *__restrict__ bias, float *C,     // A and C may be one buffer
                    int M, int N, int K, int col_tiles)
 {
-    using T = TileCfg<TM, TN, TY>;
+    using T = TileCfg<TM, TN, TY, DEEP>;
     constexpr int BM = T::BM, BN = T::BN, kTileThreads = T::kThreads, kBK = T::kBK;
     extern __shared__ __align__(16) float tile_s[];                      // [stage][A: BM rows of kBK | B: kBK rows of BN]
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
@@ -336,21 +337,26 @@ bool overlap(const void *a, size_t na, const void *b, size_t nb)
 
 }  // namespace
 
-// The tile of a product.  In place (C over A) a block must own whole rows: it stores after its last read.  Cost: clocks per inner index of the SM with the most tiles (a tile's own bound, see above; an SM with a
-// single block of four warps hides less latency, about a fifth), the larger tile among equals.
+// The tile of a product.  In place (C over A) a block must own whole rows: it stores after its last read.  Cost: clocks of the SM with the most tiles: a tile's own
+// bound (see above) times the inner indices, whole stages of them, and what a block costs besides; an SM with a single block of four warps hides less latency,
+// about a fifth; of blocks of two warps with five stages only three to five fit an SM, a tenth where there are more; the wide tiles stay 30 % off
+// their bound, the tiles of 64 columns within 10 %.  The larger tile among equals.
+// Fitted to the times of all nineteen tiles at eighty shapes (30 - 120000 rows, 8 - 400 inner, 8 - 400 columns and a few beyond): 1.1 % above the best
+// tile in the geometric mean, 14 % at most.  By the bound alone, and without the tiles of three short stages: 6.8 % and 62 %, worst where a short inner
+// dimension meets many rows (rows x inner x columns 40114 x 48 x 8 16.1 us, now 10; 61815 x 36 x 12 23.9, now 18; 29618 x 104 x 52 19.4, now 15).
 struct TileChoice {
     void (*kernel)(const float *, const float *, const float *, float *, int, int, int, int);
-    int tm, tn, ty;
+    int tm, tn, ty, bk;
     size_t smem;
 };
-template <int TM, int TN, int TY = 8>
-TileChoice tile_choice() { return {matmul_tile_kernel<TM, TN, TY>, TM, TN, TY, TileCfg<TM, TN, TY>::kSmem}; }
+template <int TM, int TN, int TY = 8, bool DEEP = TN == 4>
+TileChoice tile_choice() { return {matmul_tile_kernel<TM, TN, TY, DEEP>, TM, TN, TY, TileCfg<TM, TN, TY, DEEP>::kBK, TileCfg<TM, TN, TY, DEEP>::kSmem}; }
 
 static int launch_matmul_tiles(const float *A, const float *B, const float *bias, float *C, int M, int N, int K, bool whole_rows, cudaStream_t st)
 {
     static const TileChoice choices[] = {tile_choice<8, 16>(), tile_choice<7, 16>(), tile_choice<6, 16>(), tile_choice<5, 16>(), tile_choice<8, 8>(), tile_choice<7, 8>(),
                                          tile_choice<6, 8>(), tile_choice<5, 8>(), tile_choice<4, 8>(), tile_choice<3, 8>(), tile_choice<4, 4>(),
-                                         tile_choice<6, 4, 4>(), tile_choice<5, 4, 4>(), tile_choice<4, 4, 4>(), tile_choice<3, 4, 4>(), tile_choice<2, 4, 4>(), tile_choice<1, 4, 4>()};
+                                         tile_choice<6, 4, 4>(), tile_choice<5, 4, 4>(), tile_choice<4, 4, 4>(), tile_choice<3, 4, 4>(), tile_choice<2, 4, 4>(), tile_choice<1, 4, 4>(), tile_choice<4, 4, 8, false>(), tile_choice<2, 4, 8, false>()};
     constexpr int kSms = 148, kSmSharedBytes = 228 * 1024;
     const TileChoice *best = nullptr;
     double best_cost = 0.0;
@@ -360,7 +366,8 @@ static int launch_matmul_tiles(const float *A, const float *B, const float *bias
         const long long tiles = (long long)((M + c.ty * c.tm - 1) / (c.ty * c.tm)) * ((K + 16 * c.tn - 1) / (16 * c.tn));
         const long long per_sm = (tiles + kSms - 1) / kSms;
         const int fma = c.tm * c.tn, loads = c.ty / 2 * (c.tm + c.tn), clocks = fma > loads ? fma : loads;
-        const double cost = (double)per_sm * clocks * (per_sm == 1 ? 1.2 : 1.0);
+        const double inner = (double)((N + c.bk - 1) & -c.bk), fixed = c.tn == 16 ? 1300.0 : c.tn == 8 ? 900.0 : c.ty == 4 ? 300.0 : 0.0, off = c.tn > 4 ? 1.3 : c.ty == 4 && per_sm >= 3 ? 1.1 : 1.0;
+        const double cost = (double)per_sm * (clocks * inner * off + fixed) * (per_sm == 1 ? 1.2 : 1.0);
         if (!best || cost < best_cost) { best = &c; best_cost = cost; best_tiles = tiles; }
     }
     if (best_tiles > 2147483647LL) return fail(HIPGPT_ERR_BAD_ARG, "matmul: %lld tiles are too many", best_tiles);

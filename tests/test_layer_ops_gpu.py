@@ -83,6 +83,22 @@ def test_matmul_small_tiles_are_bit_identical_to_the_reference_order(M, K):
         assert np.array_equal(dA2.cpu().numpy(), want)
 
 
+@pytest.mark.parametrize("M,N,K", [(2400, 52, 132), (1800, 44, 20), (1249, 300, 388), (16353, 52, 28), (40114, 48, 8), (9000, 16, 16)])
+def test_matmul_of_many_rows_and_few_inner_indices_is_bit_identical_to_the_reference_order(M, N, K):
+    """The tiles of short stages, with inner dimensions of less than the stages hold and with rows and columns left over; the last in place too."""
+    lib = _capi.lib()
+    A, W, b = synth.normal(24, (M, N)), synth.normal(25, (N, K), 0.1), synth.normal(26, (K,))
+    want = ob.matmul(A, W, b, M, N, K, fma=True)
+    dA, dW, db, dC = dev(A), dev(W), dev(b), torch.full((M, K), float("nan"), device="cuda")
+    _capi.check(lib.hipgpt_matmul(dA.data_ptr(), dW.data_ptr(), db.data_ptr(), dC.data_ptr(), M, N, K, _st()))
+    torch.cuda.synchronize()
+    assert np.array_equal(dC.cpu().numpy(), want)
+    if N == K:
+        _capi.check(lib.hipgpt_matmul(dA.data_ptr(), dW.data_ptr(), db.data_ptr(), dA.data_ptr(), M, N, K, _st()))
+        torch.cuda.synchronize()
+        assert np.array_equal(dA.cpu().numpy(), want)
+
+
 @pytest.mark.parametrize("M,N,K,bias", [(8192, 256, 768, True), (300, 256, 768, True), (64, 1024, 256, True), (257, 256, 1024, False), (130, 64, 5000, False),
                                         (33, 100, 20, True), (5, 7, 3, False), (1, 256, 256, True), (129, 65, 129, True),
                                         (1407, 512, 509, True), (1407, 2048, 512, False), (700, 330, 260, True),     # slices of a tile on 2, 3 and 3 blocks
