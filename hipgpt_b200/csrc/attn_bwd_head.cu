@@ -18,16 +18,17 @@
 // The bound is no estimate: where a row has all its weight on one key it is 2 |w| and ds near zero.  The pieces' range (attn_bwd_pieces.cuh) is what covers that.
 // The queries of the other block contribute to this block's keys: their sums come through distributed shared memory at the end.
 //
-// Measured, us, three kernels -> one: B=32 H=8 S=256 D=32 with stored probabilities 94.9 -> 77.3, causal without 80.9 -> 70.1; S=161 (probabilities that TMA cannot
-// address) 84.7 -> 86.1, causal without 69.1 -> 59.8; B=16 H=12 S=128 D=32 stored 31.2 -> 25.2; B=64 H=12 S=35 82.0 -> 61.9; D=64: B=32 H=8 S=128 stored 46.2 -> 36.1, causal
-// without 46.2 -> 32.7; B=9 H=16 S=101 27.2 -> 19.6.  But for odd lengths just above 128 at D=32, where both are the same, the one is faster throughout.
-// Relative error of the gradients against float64: 1.45, 1.40, 0.90e-7 (dQ, dK, dV) at the first, 1.37, 1.40, 0.83e-7 at B=8 H=8 S=128 D=64 stored; three bf16
+// Measured, us, three kernels -> one: B=32 H=8 S=256 D=32 with stored probabilities 94.9 -> 74.9, causal without 80.9 -> 69.8; S=161 (probabilities that TMA cannot
+// address) 84.7 -> 85.4, causal without 69.1 -> 59.8; B=16 H=12 S=128 D=32 stored 31.2 -> 25.4; B=64 H=12 S=35 82.0 -> 61.9; D=64: B=32 H=8 S=128 stored 46.2 -> 36.3, causal
+// without 46.2 -> 33.0; B=9 H=16 S=101 27.2 -> 19.9.  But for odd lengths just above 128 at D=32, where both are the same, the one is faster throughout.
+// Relative error of the gradients against float64: 1.45, 1.40, 0.90e-7 (dQ, dK, dV) at the first, 1.34, 1.40, 0.83e-7 at B=8 H=8 S=128 D=64 stored; three bf16
 // pieces and six products throughout: 1.47, 1.68, 0.94e-7 and 1.41, 1.63, 0.83e-7.  (dV of two fp16 pieces: 1.03 and 0.95e-7; 69.0 us at the first.)
-// What bounds it: a block takes 33200 cycles at the first shape, 3.5 rounds of them.  9700 until its operands are cut and g V^T is there (224 KB come in at
+// What bounds it: a block takes about 32000 cycles at the first shape, 3.5 rounds of them.  9700 until its operands are cut and g V^T is there (224 KB come in at
 // 64 bytes per clock; the cut is bound by the instructions of conversion), 4500 for w and the scales, 5300 for ds and its pieces, 4300 for the products with
-// them and the other block's sums, 6800 for dV (900 dO's pieces, 1000 per tile of probabilities, 1400 the last product), 1900 for the output.
+// them and the other block's sums, 6000 for dV (900 dO's pieces, 900 per tile of probabilities, the last product), 1700 for the output.
 // Steps, B=32 H=8 S=256 D=32 stored: eight worker warps 76.7, sixteen 72.9; operands as whole sectors, two issuing warps, no stall between the reading of a tile's
-// probabilities and the writing of its pieces 64.3; scales per 64 x 64 instead of per 64 x 256, for keys of little probability, 69.0; dV exact 77.3.
+// probabilities and the writing of its pieces 64.3; scales per 64 x 64 instead of per 64 x 256, for keys of little probability, 69.0; dV exact 77.3; its
+// probabilities' next tile read while the pieces of one are on their way, the other gradients got ready during its last products, a tile's exponents read at once 74.9.
 #include "attn_bwd_pieces.cuh"
 #include "tma_host.cuh"
 
@@ -89,7 +90,7 @@ struct HeadSmall {
     uint64_t p_full[2 * NB], p3_full[NB], p3_ready[2 * NB], v3_done, scores, asked, cut[2], p_read[NB], p_ready[NB], v_done[NB], d_ready[NB], k_done[NB];
     alignas(16) uint32_t largest[4 + 4 * NB][8];                // of a tile's rows that a warp has
     float fac[4 + 4 * NB];
-    uint32_t group_p[2 * NB][2], group_d[2 * NB][2]; // of a tile of 64 queries (second index) x 64 keys: P's largest, ds's bound
+    alignas(16) uint32_t group_p[2][4], group_d[2][4];          // of a tile of 64 queries (first index) x 64 keys: P's largest, ds's bound
     uint32_t tmem_base;
     volatile int abort_flag, peer_gone;
 };
@@ -101,7 +102,7 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
 {
     using C = HeadCfg<D, NB>;
     // One block per head and stored probabilities, whose dV takes no columns yet: a tile's dQ from two accumulators of 32 keys, so that less is truncated
-    // (B=8 H=8: dQ 1.42 -> 1.37e-7 at S = 128 D = 64, 1.39 -> 1.36e-7 at S = 64 D = 32, where three bf16 pieces gave 1.41 and 1.38; 35.4 -> 36.1 us at B=32 H=8 S=128 D=64)
+    // (B=8 H=8: dQ 1.42 -> 1.34e-7 at S = 128 D = 64, 1.39 -> 1.28e-7 at S = 64 D = 32, where three bf16 pieces gave 1.41 and 1.38; 35.4 -> 36.1 us at B=32 H=8 S=128 D=64)
     constexpr bool kHalves = STORED && NB == 1;
     constexpr int kColK = STORED ? 0 : C::kColK;
     constexpr int TB = C::TB;
@@ -126,7 +127,7 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
     if (tid == 0) {
         sh.abort_flag = 0;
         sh.peer_gone = 0;
-        for (int t = 0; t < 2 * NB; ++t) sh.group_p[t][0] = sh.group_p[t][1] = sh.group_d[t][0] = sh.group_d[t][1] = 0;
+        for (int t = 0; t < 2 * NB; ++t) sh.group_p[0][t] = sh.group_p[1][t] = sh.group_d[0][t] = sh.group_d[1][t] = 0;
         for (int i = 0; i < 2 * NB; ++i) { mbar_init(&sh.p_full[i], 1); mbar_init(&sh.p3_ready[i], kWorkerWarps); }
         for (int i = 0; i < NB; ++i) mbar_init(&sh.p3_full[i], 1);
         mbar_init(&sh.v3_done, 2);
@@ -478,15 +479,15 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
             uint32_t bp = __float_as_uint(most_p[t] * rinv), bd = __float_as_uint(fmaf(most_p[t], fabsf(w), most_d[t]) * rinv);
             if (!STORED) bp = __reduce_max_sync(0xffffffffu, bp < 0x7f800000u ? bp : 0u);
             bd = __reduce_max_sync(0xffffffffu, bd < 0x7f800000u ? bd : 0u);
-            if (lane == 0 && !STORED) atomicMax(&sh.group_p[t][u], bp);
-            if (lane == 0) atomicMax(&sh.group_d[t][u], bd);
+            if (lane == 0 && !STORED) atomicMax(&sh.group_p[u][t], bp);
+            if (lane == 0) atomicMax(&sh.group_d[u][t], bd);
         }
         meet();
     }
     if (NB > 1) cluster_arrive();                    // V's image is this block's no longer: the other one's sums may come
     // exponents of a tile: of its probabilities (those that are formed: at most 1) and of its ds
-    auto e_p = [&](int t, int y) { return range_exponent(sh.group_p[t][y]); };
-    auto e_d = [&](int t, int y) { return range_exponent(sh.group_d[t][y]); };
+    auto e_p = [&](int t, int y) { return range_exponent(sh.group_p[y][t]); };
+    auto e_d = [&](int t, int y) { return range_exponent(sh.group_d[y][t]); };
 
     // Second sweep: ds, scaled, in fp32 in dP's place; P's pieces in P's.  A block of keys' probabilities are read first: eight warps share the memory
     // that each of them then writes its pieces to (a meeting per tile, between reading and writing it, kept them all in the same step: 1300 cycles per tile).
@@ -503,6 +504,8 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
             *reinterpret_cast<uint4 *>(at + i * kKeys8 + kPiecePart) = make_uint4(lo[4 * i], lo[4 * i + 1], lo[4 * i + 2], lo[4 * i + 3]);
         }
     };
+    const uint4 all_p = STORED ? make_uint4(0, 0, 0, 0) : *reinterpret_cast<const uint4 *>(sh.group_p[u]), all_d = *reinterpret_cast<const uint4 *>(sh.group_d[u]);
+    auto of_tile = [](const uint4 &v, int kb, int y) { return range_exponent(NB == 1 || kb == 0 ? (y ? v.y : v.x) : (y ? v.w : v.z)); };
     float p[2][kCols];
     auto read_block = [&](int i) {
         const int t = 2 * block_at(i);
@@ -517,8 +520,8 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
         for (int y = 0; y < 2; ++y) {
             const int t = 2 * kb + y;
             if (t >= ntile) break;
-            const uint32_t ep = STORED ? 0u : e_p(t, u);
-            const float up_d = range_up(e_d(t, u)), up_row = rinv * range_up(ep), ratio = STORED ? 1.0f : up_d * range_down(ep);
+            const uint32_t ep = STORED ? 0u : of_tile(all_p, kb, y);
+            const float up_d = range_up(of_tile(all_d, kb, y)), up_row = rinv * range_up(ep), ratio = STORED ? 1.0f : up_d * range_down(ep);
             const float dp_up = fminf(g_fac * sh.fac[C::tV + t], kFacMost) * ratio, w_up = w * ratio;
             float dp[kCols];
             tmem_ld16(my_tile + t * kTile, dp);
@@ -655,7 +658,7 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
     }
     // 32 rows x 32 columns leave in whole lines: through shared memory (16-byte pieces permuted by the row), then a row of 128 bytes per eight lanes
     const int row0 = q0 + wq * 32;
-    auto store_rows = [&](const float (&o)[OC], float scale, float loss, uint8_t *stage, float *dst, bool off) {
+    auto stage_rows = [&](const float (&o)[OC], float scale, float loss, uint8_t *stage) {
         uint8_t *box = stage + (D == 64 ? wq * 2 + (cf >> 1) : wq) * 4096;
 #pragma unroll
         for (int i = 0; i < OC / 4; ++i) {
@@ -663,6 +666,9 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
             if (loss != 0.0f) { x.x = fmaf(x.x, loss, x.x); x.y = fmaf(x.y, loss, x.y); x.z = fmaf(x.z, loss, x.z); x.w = fmaf(x.w, loss, x.w); }
             *reinterpret_cast<float4 *>(box + sw128(lane, D == 64 ? (cf & 1) * 4 + i : cf * 2 + i)) = x;
         }
+    };
+    auto store_rows = [&](const uint8_t *stage, float *dst, bool off) {
+        const uint8_t *box = stage + (D == 64 ? wq * 2 + (cf >> 1) : wq) * 4096;
         if (D == 64) asm volatile("bar.sync %0, 64;" ::"r"(4 + wq * 2 + (cf >> 1)) : "memory");
         else asm volatile("bar.sync %0, 128;" ::"r"(4 + wq) : "memory");
         constexpr int kRows = D == 64 ? 16 : 8;
@@ -705,13 +711,11 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
                 for (int z = 0; z < 3; ++z) *reinterpret_cast<uint4 *>(at + z * Img<D>::kPiece) = pc[z];
             }
         proxy_fence();
-#pragma unroll
-        for (int t = 0; t < C::kTiles; ++t) {
-            if (t < 2 * qb0 || t >= nq) continue;
-            const int q16 = t * kTile + cf * 16;     // this thread's first query
-            float pt[16];
+        float pt[16];
+        auto fetch = [&](int t) {                    // this thread's 16 queries of tile t
+            const int q16 = t * kTile + cf * 16;
             if (by_tma) {
-                wait(&sh.p3_full[t >> 1], 0, 22);
+                if ((t & 1) == 0) wait(&sh.p3_full[t >> 1], 0, 22);
                 const uint8_t *src = p_s + (4 * place(t >> 1) + wq) * kGroup + (lane & 3) * 4;
 #pragma unroll
                 for (int i = 0; i < 16; ++i) pt[i] = *reinterpret_cast<const float *>(src + sw128((t & 1) * kTile + cf * 16 + i, lane >> 2));
@@ -721,19 +725,33 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
 #pragma unroll
                 for (int i = 0; i < 16; ++i) pt[i] = q16 + i < S ? src[(size_t)i * S] : 0.0f;
             }
+        };
+        fetch(2 * qb0);
+#pragma unroll
+        for (int n = 0; n < C::kTiles; ++n) {
+            const int t = 2 * qb0 + n;
+            if (t >= nq) break;
             if (CAUSAL) {
 #pragma unroll
-                for (int i = 0; i < 16; ++i) pt[i] = row <= q16 + i ? pt[i] : 0.0f;
+                for (int i = 0; i < 16; ++i) pt[i] = row <= t * kTile + cf * 16 + i ? pt[i] : 0.0f;
             }
             uint32_t pc[3][8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) cut3(make_float2(pt[2 * i], pt[2 * i + 1]), pc[0][i], pc[1][i], pc[2][i]);
 #pragma unroll
             for (int z = 0; z < 3; ++z) tmem_st8_u32(lane_base + t * C::kCols3 + 32 * z + 8 * cf, pc[z]);
+            if (t + 1 < nq) fetch(t + 1);            // (while the pieces are on their way)
             tmem_wait_st();
             tc_fence_before();
             arrive(&sh.p3_ready[t]);
         }
+        // (while the last products run: the other gradients are got ready.  Nothing is stored before it is known that no wait has run out)
+        stage_rows(oq, c, kHalves ? kScoreLoss32 : kScoreLoss, q_s);
+        if (NB > 1) {
+            cluster_wait();
+            if (!CAUSAL || blk == 0) receive(ok, 0);
+        }
+        stage_rows(ok, c, kScoreLoss, g_s);
         wait(&sh.v3_done, 0, 25);
         tc_fence_after();
 #pragma unroll
@@ -748,17 +766,24 @@ bwd_head_kernel(const float *q, const float *k, const float *v, const float *g, 
         meet();                                      // (who has not seen a wait run out: the last word on it)
     }
     bool off = sh.abort_flag;
-    store_rows(oq, c, kHalves ? kScoreLoss32 : kScoreLoss, q_s, dQ, off);
-    if (NB > 1) {
-        cluster_wait();
-        if (!CAUSAL || blk == 0) {
-            if (!STORED) receive(ov, 0);
-            receive(ok, STORED ? 0 : 1);
+    if constexpr (STORED) {
+        store_rows(q_s, dQ, off);
+        store_rows(g_s, dK, off || sh.peer_gone);
+        stage_rows(ov, 1.0f, 0.0f, p_s);
+        store_rows(p_s, dV, off);
+    } else {
+        stage_rows(oq, c, kScoreLoss, q_s);
+        store_rows(q_s, dQ, off);
+        if (NB > 1) {
+            cluster_wait();
+            if (!CAUSAL || blk == 0) { receive(ov, 0); receive(ok, 1); }
+            off = off || sh.peer_gone;
         }
-        off = off || sh.peer_gone;
+        stage_rows(ov, 1.0f, kSumLoss, g_s);
+        store_rows(g_s, dV, off);
+        stage_rows(ok, c, kScoreLoss, k_s);
+        store_rows(k_s, dK, off);
     }
-    store_rows(ov, 1.0f, STORED ? 0.0f : kSumLoss, STORED ? p_s : g_s, dV, off);
-    store_rows(ok, c, kScoreLoss, STORED ? g_s : k_s, dK, off);
     tc_fence_before();
     __syncthreads();
 }
