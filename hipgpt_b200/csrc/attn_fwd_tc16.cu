@@ -170,7 +170,7 @@ __device__ __forceinline__ float log2_of_pow2(float p) { return (float)((int)((_
 template <int D>
 __global__ void __launch_bounds__(kPackThreads)
 kv_pack_kernel(const float *__restrict__ K, const float *__restrict__ V, float *__restrict__ tmax,
-               uint8_t *__restrict__ kimg, uint8_t *__restrict__ vimg, int S, int E, int H, int ntk, int ntiles)
+               uint8_t *__restrict__ kimg, uint8_t *__restrict__ vimg, int S, int E, int H, int ntk, int ntiles, int once)
 {
     using C = Tc16Cfg<D>;
     constexpr int kSide = kPackThreads / 2;
@@ -189,8 +189,10 @@ kv_pack_kernel(const float *__restrict__ K, const float *__restrict__ V, float *
     float4 xa[NP], xc[NP];
     float mx = 0.0f;
     // At head_dim 64 whole sectors, where the planes allow it: B=4 H=8 S=2048 causal 62.5 -> 61.1 us per call, B=16 H=8 S=1024 91.3 -> 86.9 - 88.9, S=400 17.9 -> 17.7.
-    // (Marked to leave L2 first they were no faster, 60.7 - 61.0, 85.9 - 92.5 and 18.0, and a backward that reads the planes again lost by it: B=3 H=12 S=777, forward and
-    // backward, 105.9 us without the mark and 106.8 with it.)  At 32, where K and V are smaller and may be found in L2, 24.6 -> 25.3 (B=8 H=9 S=700).
+    // At 32, where K and V are smaller and may be found in L2, 24.6 -> 25.3 (B=8 H=9 S=700).
+    // `once`: the call's planes are larger than L2, so that whoever reads K and V next will not find them there: they leave it first and the images stay (B=16 H=8
+    // S=1024, a long run: 101.4 -> 99.6 us).  Of smaller planes the mark takes them from the backward that reads them next (B=3 H=12 S=777, forward and backward,
+    // 105.9 us without the mark and 106.8 with it) and gives the forward nothing (B=4 H=8 S=2048 61.1 and 60.9, S=400 17.7 and 17.9).
     const bool sectors = D == 64 && ((reinterpret_cast<uintptr_t>(K) | reinterpret_cast<uintptr_t>(V)) & 31) == 0;
 #pragma unroll
     for (int i = 0; i < NP; ++i) {
@@ -200,7 +202,8 @@ kv_pack_kernel(const float *__restrict__ K, const float *__restrict__ V, float *
         const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
         xa[i] = xc[i] = z;
         if (ok && sectors) {
-            load_sector(p, xa[i], xc[i]);
+            if (once) load_sector_once(p, xa[i], xc[i]);
+            else load_sector(p, xa[i], xc[i]);
         } else if (ok) {
             xa[i] = __ldg(p);
             xc[i] = __ldg(p + 1);
@@ -750,12 +753,13 @@ int launch_tc16_cfg(const float *q, const float *k, const float *v, float *out, 
             if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "event hand-off: %s", cudaGetErrorString(e));
         }
         const dim3 pgrid((unsigned)ntk, (unsigned)(nb * H));
+        const int once = (size_t)4 * B * S * E * sizeof(float) > (size_t)126 << 20;          // Q, K, V and the output against L2
         if (overlap) {                               // on the second stream, behind an event
-            kv_pack_kernel<D><<<pgrid, kPackThreads, 0, ps>>>(k + off, v + off, tmax, buf, buf + kbytes, S, E, H, ntk, ntiles);
+            kv_pack_kernel<D><<<pgrid, kPackThreads, 0, ps>>>(k + off, v + off, tmax, buf, buf + kbytes, S, E, H, ntk, ntiles, once);
             rc = check_launch("kv_pack_kernel");
             if (rc != HIPGPT_OK) return rc;
         } else {
-            e = launch_overlapped(kv_pack_kernel<D>, pgrid, dim3(kPackThreads), 0, ps, k + off, v + off, tmax, buf, buf + kbytes, S, E, H, ntk, ntiles);
+            e = launch_overlapped(kv_pack_kernel<D>, pgrid, dim3(kPackThreads), 0, ps, k + off, v + off, tmax, buf, buf + kbytes, S, E, H, ntk, ntiles, once);
             if (e != cudaSuccess) return fail(HIPGPT_ERR_CUDA, "kv_pack_kernel launch: %s", cudaGetErrorString(e));
         }
         if (overlap) {

@@ -114,6 +114,13 @@ __device__ __forceinline__ void load_sector(const float4 *src, float4 &a, float4
                  : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w) : "l"(src));
 }
 
+// The same, of a line that leaves L2 first.
+__device__ __forceinline__ void load_sector_once(const float4 *src, float4 &a, float4 &b)
+{
+    asm volatile("ld.global.L1::no_allocate.L2::evict_first.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w) : "l"(src));
+}
+
 // One whole 32-byte sector (dst 32-byte aligned).
 __device__ __forceinline__ void store_sector(float *dst, float a, float b, float c, float d, float e, float f, float g, float h)
 {

@@ -235,3 +235,19 @@ def test_tiled_kernel_in_several_groups_of_batches(monkeypatch, causal, want_pro
         assert float(np.abs(out - ref_out).max()) <= TOL
         if want_probs:
             assert float(np.abs(probs - ref_probs).max()) <= TOL
+
+
+def test_tiled_kernel_with_planes_larger_than_l2_gives_the_bits_of_each_half():
+    """head_dim 64: K and V are read with another cache hint where the call's planes are larger than L2; on 16-byte boundaries without either."""
+    B, H, S, D = 18, 8, 1000, 64
+    E, st = H * D, torch.cuda.current_stream().cuda_stream
+    buf = torch.randn(3 * B * S * E + 4, generator=torch.Generator(device="cuda").manual_seed(3), device="cuda")
+    for shift in (0, 4):
+        q, k, v = buf[shift:shift + 3 * B * S * E].view(3, B, S, E)
+        out, part = torch.empty(B, S, E, device="cuda"), torch.empty(B // 2, S, E, device="cuda")
+        ptr = lambda *t: [x.data_ptr() for x in t]               # noqa: E731
+        _capi.check(_capi.lib().hipgpt_mha_forward(*ptr(q, k, v, out), None, B, S, E, H, 1, st))
+        for rows in (slice(0, B // 2), slice(B // 2, B)):
+            _capi.check(_capi.lib().hipgpt_mha_forward(*ptr(q[rows], k[rows], v[rows], part), None, B // 2, S, E, H, 1, st))
+            assert torch.equal(out[rows], part)
+    assert _status() == 0
