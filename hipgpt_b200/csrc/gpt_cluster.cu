@@ -144,6 +144,7 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
     uint2 *table = reinterpret_cast<uint2 *>(sm + lay.table);
     uint8_t *ring = reinterpret_cast<uint8_t *>(sm + lay.ring);
     const int f2_own = cluster_f2_columns(E, rank);
+    const bool f2_here = cluster_f2_columns(E, kClusterBlocks - 1) > 0 || f2_own > 0;
     auto tx = [&](int i) {
         return (uint32_t)(rows * (i == kQkv ? 12 * E : i == kRec ? H * ns * (D + 2) * 4 : i == kF2 ? 16 * 4 * f2_own : i == kAm ? 32 * 8 : 4 * E));
     };
@@ -158,7 +159,7 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
         for (int i = 0; i < lay.slots; ++i) mbar_init(&full[i], 1);
         for (int i = 0; i < 6; ++i) {
             mbar_init(&hop[i], 1);
-            if (i != kF2 || f2_own > 0) mbar_arrive_expect_tx(&hop[i], tx(i));
+            if (i != kF2 || f2_here) mbar_arrive_expect_tx(&hop[i], tx(i));
         }
     }
     __syncthreads();
@@ -426,7 +427,7 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
         constexpr int kHeld = K4 < 8 ? K4 : 8;                           // a column's first weights are in registers before the row is there (all: spills)
         float bias = 0.0f;
         const int own_r = R == 1 ? 0 : tid / jb.nc, own_c = tid - own_r * jb.nc, own_n = rank * jb.nc + own_c;
-        const bool sums = f2_own > 0 && warp * 32 < jb.nc * R, mine = sums && tid < jb.nc * R && own_r < rows && own_n < E;
+        const bool sums = f2_here && warp * 32 < jb.nc * R, mine = sums && tid < jb.nc * R && own_r < rows && own_n < E;
         if (sums) {
             wait(&full[slot0], slot_par);
             if (tid < jb.nc * R) bias = (reinterpret_cast<const float *>(ring + slot0 * C::kSlot) + jb.weight_floats())[own_c];
@@ -478,7 +479,7 @@ cluster_steps_kernel(const __grid_constant__ ClusterPlan plan, const __grid_cons
             if (slot0 >= lay.slots) { slot0 -= lay.slots; slot_par ^= 1u; }
         }
         // (the last warp opens the barrier's next phase, where there is one; the others have nothing to wait for)
-        if (sums || (f2_own > 0 && warp == kWarps - 1)) receive(kF2);
+        if (sums || (f2_here && warp == kWarps - 1)) receive(kF2);
         else hop_phase ^= 1u << kF2;
         if (sums) {
             float v = 0.0f;
