@@ -380,12 +380,6 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         seen = !gone;
         if (!gone && !done) seen = bwd_wait_slow(bar, parity, site, &abort_flag, expire);
     };
-    // the workers' wait: without stored probabilities they are short of registers (B=3 H=12 S=777 D=64 causal: 114.4 us with the wait above)
-    auto wait_w = [&](uint64_t *bar, uint32_t parity, int site) {
-        if (STORED) return wait(bar, parity, site);
-        if (abort_flag || mbar_test(bar, parity)) return;
-        bwd_wait_slow(bar, parity, site, &abort_flag, expire);
-    };
 
     if (warp >= kWorkerWarps) {
         // the first issuing warp has K: S = Q K^T and half of the accumulation; the second V: dP = dO V^T and the other half
@@ -520,7 +514,7 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         const uint8_t *src = p_s + (i % kPStages<D>) * kPTile + hf * (kPTile / 2);
         int r0 = rloc;
         if (STORED == 2) {
-            wait_w(&p_full[i % kPStages<D>], (uint32_t)((i / kPStages<D>) & 1), 7);
+            wait(&p_full[i % kPStages<D>], (uint32_t)((i / kPStages<D>) & 1), 7);
         } else {
             uint8_t *turn = p_s + warp * 4096;
             __syncwarp();
@@ -539,7 +533,7 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
 #pragma unroll
     for (int x = 0; x < D / 2; ++x) o[x] = 0.0f;
     auto add_dq = [&](int i) {                       // tile i of the second sweep has been accumulated
-        wait_w(&acc_done[i & 1], (uint32_t)(((i - nk) >> 1) & 1), 6);
+        wait(&acc_done[i & 1], (uint32_t)(((i - nk) >> 1) & 1), 6);
         tc_fence_after();
         add_tile<D, C::kWide>(lane_base + C::kColAcc, hf, down_s[i % kDownSlots][0][rloc], down_s[i % kDownSlots][1][rloc], o);
     };
@@ -591,7 +585,7 @@ bwd_rows_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
             take_p(i, s);
             if (STORED == 1 && i + 1 < total) fetch_p(i + 1);       // in flight during this tile
         }
-        wait_w(&sd_full[i & 1], (uint32_t)((i >> 1) & 1), 4);
+        wait(&sd_full[i & 1], (uint32_t)((i >> 1) & 1), 4);
         tc_fence_after();
         if (!STORED) tmem_ld32(s_addr, s);
         tmem_ld32(dp_addr, dp);
@@ -723,12 +717,6 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
         seen = !gone;
         if (!gone && !done) seen = bwd_wait_slow(bar, parity, site, &abort_flag, expire);
     };
-    // the workers' wait: without stored probabilities they are short of registers (B=3 H=12 S=777 D=64 causal: 114.4 us with the wait above)
-    auto wait_w = [&](uint64_t *bar, uint32_t parity, int site) {
-        if (STORED) return wait(bar, parity, site);
-        if (abort_flag || mbar_test(bar, parity)) return;
-        bwd_wait_slow(bar, parity, site, &abort_flag, expire);
-    };
 
     if (warp >= kWorkerWarps) {
         // the first issuing warp: S^T = K Q^T and dV; the second: dP^T = V dO^T and dK
@@ -853,7 +841,7 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
 #pragma unroll
     for (int x = 0; x < D / 2; ++x) ok[x] = ov[x] = 0.0f;
     auto add_dkv = [&](int i) {                      // tile i has been accumulated
-        wait_w(&acc_done[i & 1], (uint32_t)((i >> 1) & 1), 16);
+        wait(&acc_done[i & 1], (uint32_t)((i >> 1) & 1), 16);
         tc_fence_after();
         if (STORED) add_exact<D>(lane_base + C::kColV, hf, ov);
         else add_tile<D, C::kWide>(lane_base + C::kColV, hf, down_s[i % kDownSlots][0][0][rloc], down_s[i % kDownSlots][0][1][rloc], ov);
@@ -884,17 +872,17 @@ bwd_cols_kernel(const uint8_t *__restrict__ img, size_t img_bytes, const float *
             if (i + 1 < total) fetch_p(i + 1);       // in flight during this tile
         }
         if (STORED == 2) {
-            wait_w(&p_full[i % kPStages<D>], (uint32_t)((i / kPStages<D>) & 1), 17);
+            wait(&p_full[i % kPStages<D>], (uint32_t)((i / kPStages<D>) & 1), 17);
             const uint8_t *src = p_s + (i % kPStages<D>) * kPTile + wq * (kPTile / 4) + (lane & 3) * 4;
 #pragma unroll
             for (int x = 0; x < 32; ++x) p[x] = *reinterpret_cast<const float *>(src + sw128(hf * 32 + x, lane >> 2));
         }
-        wait_w(&sd_full[i & 1], (uint32_t)((i >> 1) & 1), 14);
+        wait(&sd_full[i & 1], (uint32_t)((i >> 1) & 1), 14);
         tc_fence_after();
         if (!STORED) tmem_ld32(s_addr, p);
         tmem_ld32(dp_addr, d);
         tmem_wait_ld();
-        wait_w(&w_full[i % C::kStages], (uint32_t)((i / C::kStages) & 1), 18);
+        wait(&w_full[i % C::kStages], (uint32_t)((i / C::kStages) & 1), 18);
         if (!STORED) {
 #pragma unroll
             for (int x = 0; x < 32; x += 4) {
