@@ -155,7 +155,7 @@ HIPGPT_API int hipgpt_attention_weighted_sum(const float *d_softmax, const float
  * head_dim 32 and 64 run on the tensor pipe: an operand is the sum of two fp16 numbers under one power of two per 64 rows of a
  * head (probabilities and their gradients: per 64 x 64 of them at most), that is 2^-23 of a value down to 2^-29 of the largest
  * of its 64 rows, 2^-52 of that one below: rows beside each other may be nine decimal orders apart.  Error against float64
- * 1 - 2.6e-7 on unit normals.  Wider ranges than that: hipgpt_set_full_range(1) takes the kernels of the other head dimensions, exact
+ * 1 - 2.6e-7 on unit normals.  Wider ranges than that (no notice is raised for them): hipgpt_set_full_range(1) takes the kernels of the other head dimensions, exact
  * fp32 throughout.  Contexts that do not fit one block (head_dim 32: more than 256 rows, 64: more than 128) keep the operands'
  * images in a buffer of the library (per device and stream, at most eight; hipgpt_release_workspace() frees them; a captured
  * call gets a buffer of its graph).

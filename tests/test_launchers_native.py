@@ -140,6 +140,7 @@ def test_without_the_extension_the_same_is_refused(without_extension):
     test_what_is_not_a_cuda_tensor_is_refused()
 
 
+@pytest.mark.filterwarnings("ignore:the extension of the hot calls")
 @pytest.mark.parametrize("native", [True, False])
 def test_sizes_are_what_ctypes_takes(native, request):
     """As through ctypes: an int or a c_int; what is neither is ctypes.ArgumentError, and a TypeError, before anything is called."""
@@ -153,6 +154,7 @@ def test_sizes_are_what_ctypes_takes(native, request):
 
 
 @pytest.mark.gpu
+@pytest.mark.filterwarnings("ignore:the extension of the hot calls")
 @pytest.mark.parametrize("native", [True, False])
 def test_c_ints_are_taken(native, request):
     if not native:
