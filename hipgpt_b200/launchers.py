@@ -7,6 +7,7 @@ streams only; every kernel is the library's own.
 from __future__ import annotations
 
 import ctypes
+import threading
 import warnings
 
 import torch
@@ -79,18 +80,22 @@ class _ThroughCtypes:
 
 
 class _AtFirstCall:
-    """Stands for the extension until it is needed: importing this module builds and loads nothing."""
+    """Stands for the extension until it is needed, by the first of however many threads: importing this module builds and loads nothing."""
+
+    _lock = threading.Lock()
 
     def __getattr__(self, name):
         global _native
-        try:
-            native = _capi.native()
-            native.bind(_ptr, _ptr_bf16, _int)
-        except (RuntimeError, ImportError, OSError) as e:       # no g++, no headers: the same library through ctypes
-            warnings.warn(f"the extension of the hot calls cannot be built or loaded, they go through ctypes (a few microseconds more each): {e}", RuntimeWarning, stacklevel=3)
-            native = _ThroughCtypes
-        _native = native
-        return getattr(native, name)
+        with self._lock:
+            if _native is self:
+                try:
+                    native = _capi.native()
+                    native.bind(_ptr, _ptr_bf16, _int)
+                except (RuntimeError, ImportError, OSError) as e:       # no g++, no headers: the same library through ctypes
+                    warnings.warn(f"the extension of the hot calls cannot be built or loaded, they go through ctypes (a few microseconds more each): {e}", RuntimeWarning, stacklevel=3)
+                    native = _ThroughCtypes
+                _native = native
+        return getattr(_native, name)
 
 
 _native = _AtFirstCall()

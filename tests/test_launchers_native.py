@@ -5,6 +5,8 @@ import ctypes
 import os
 import subprocess
 import sys
+import threading
+import time
 
 import pytest
 
@@ -124,6 +126,31 @@ def test_an_extension_belongs_to_one_torch_and_appears_when_it_is_whole(tmp_path
     assert os.listdir(tmp_path) == []
     Done.returncode = 0
     assert build.build_extension() == out and os.listdir(tmp_path) == [os.path.basename(out)]
+
+
+def test_threads_that_call_first_together_load_one_extension(monkeypatch):
+    loaded, real, start = [], _capi.native, threading.Barrier(8)
+
+    def native():
+        loaded.append(threading.get_ident())
+        time.sleep(0.2)
+        return real()
+    monkeypatch.setattr(_capi, "native", native)
+    monkeypatch.setattr(launchers, "_native", launchers._AtFirstCall())
+    refused = []
+
+    def call():
+        start.wait()
+        try:
+            launchers.mha_decode(torch.zeros(4), None, None, None, None, 1, 1, 32, 1, 1)
+        except ValueError:
+            refused.append(1)
+    threads = [threading.Thread(target=call) for _ in range(8)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert len(loaded) == 1 and len(refused) == 8
 
 
 @pytest.fixture
